@@ -1,318 +1,361 @@
-// Causal flash attention forward for sm_100a on the packed (B, T, 3, NH, HS) QKV layout; head sizes 64..128
-// (multiples of 8; sizes above 64 run as a 128-wide head whose missing channels TMA fills with zeros).
+// Causal flash attention forward for sm_100a on the packed (B, T, 3, NH, HS) QKV layout, head sizes 72..128 (multiples of 8; a
+// narrower head runs as a 128-wide one whose missing channels TMA fills with zeros, with the products cut to whole 16-channel steps).
 //
-// Persistent: one CTA per SM walks a heavy-first list of (batch, head, 128-row query tile) work items; Q is double
-// buffered so the next item's loads and first MMA run under the current item's tail.  Roles inside a CTA (576 threads):
-//   warp 0      TMA producer: Q once, then K and V tiles (double buffered), read in place from the
-//               packed QKV tensor through a 4-D tensor map.
-//   warp 1      MMA issuer: S = Q K^T into TMEM columns [0,128), PV = P V into one of two 64-column
-//               TMEM buffers.  S(j+1) is issued as soon as the softmax threads hold S(j) in registers.
-//   warps 2-17  softmax: thread = query row x 32-column quarter.  One TMEM load of its 32 scores, row
-//               maximum exchanged between the four quarters through shared memory, exp2 on the SFU,
-//               bf16 P written to 128-byte-swizzled shared memory (A operand of the PV MMA, double
-//               buffered); each thread owns 16 of the 64 output columns in registers and folds in the
-//               previous tile's PV while the tensor core works on the current one.
-// Statistics are written as natural-log LSE per (b, h, t), the layout cuDNN's SDPA uses in the
-// reference (llmc/cudnn_att.cpp:105-113).  Tiles above the diagonal are skipped.
+// The scheme of the 64-wide kernel (attention_fwd1.cu): a CTA works on TWO adjacent 128-row query tiles (slots A = 2p, B = 2p + 1) of
+// one head and streams the key / value tiles 0..2p+1 past both; one softmax thread owns a whole row of 128 scores in registers; P goes
+// back to tensor memory as bf16 and is the A operand of O += P V; O stays in tensor memory and is rescaled only when the running
+// maximum has moved by more than 2^8.  What 128 channels change:
+//   * S and O of both slots take all 512 TMEM columns, so P_X(t) overwrites the scores S_X(t) it came from, and S_X(t+1) is issued
+//     directly behind O_X += P_X(t) V (program order keeps it from overwriting P).  A slot therefore alternates between its softmax
+//     and its products; the other slot's products fill the tensor pipe meanwhile.
+//   * K and V tiles (32 KB each) share one three-stage ring, and the Q tiles are single-buffered, each released by its slot's last
+//     score product: the next item's Q tile arrives while that slot finishes its last softmax and its epilogue.
+// Bound by the softmax of the two slots (1024 exponential cycles per 128 x 128 tile each) with the tensor pipe right behind (2 x 1024
+// cycles per key tile).  Measured, with the kernel this one replaces (16 softmax warps exchanging row statistics, P through shared
+// memory) in brackets: B=16 T=2048 NH=8 HS=128 169 us (256), B=2 T=4096 NH=32 HS=128 271 us (420), B=3 T=1000 NH=32 HS=80 44 us (68).
+// Handing P over in two halves, so that the product starts under the second half's exponentials, was slower (174 / 281 us).
 //
-// Capability parity: attention_forward_cudnn (llmc/cudnn_att.cpp:222-254) and the unfused
-// attention_forward of llmc/attention.cuh in the reference.
+// Items are dealt to the persistent CTAs heaviest first in alternating direction, which evens out their decreasing lengths.
+//
+// TMEM columns: S_A [0,128)  S_B [128,256)  O_A [256,384)  O_B [384,512);  P_X: the first 64 columns of S_X (128 bf16 per row)
+//
+// Statistics are written as natural-log LSE per (b, h, t), the layout cuDNN's SDPA uses in the reference (llmc/cudnn_att.cpp:105-113).
+// Capability parity: attention_forward_cudnn (llmc/cudnn_att.cpp:222-254) and attention_forward of llmc/attention.cuh.
 #include "common.cuh"
 
 namespace {
 
-constexpr int BQ = 128, BKV = 128;
-constexpr int CHUNK_BYTES = 128 * 64 * 2;          // 16 KB: 128 rows x 64 channels of bf16, one 128-byte-swizzled TMA box
-constexpr int P_BYTES = BQ * BKV * 2;              // 32 KB
-constexpr int XCH_BYTES = (2 * 4 * 128 + 4 * 128) * 4;     // row-max exchange (double buffered) + final row sums
-constexpr int FWD_THREADS = 576;                   // TMA warp + MMA warp + 16 softmax warps
+constexpr int BT = 128;
+constexpr int CHUNK_BYTES = BT * 64 * 2;            // 16 KB: 128 rows x 64 channels, one 128-byte-swizzled TMA box
+constexpr int TILE_BYTES = 2 * CHUNK_BYTES;
+constexpr int RING = 3;                             // K_0 V_0 K_1 V_1 ... tiles in flight
+constexpr int THREADS = 384;                        // TMA warp, issuer warp, two idle warps, 2 x 4 softmax warps
+constexpr int TMEM_COLS = 512;
+constexpr int SMEM = 2 * TILE_BYTES + RING * TILE_BYTES + 2 * TILE_BYTES + 256;     // Q, K/V ring, two output tiles
+static_assert(SMEM <= 232448, "shared memory of one CTA");
+constexpr long long SKEW_CYCLES = 1200;
+constexpr float RESCALE_LOG2 = 8.0f;                // the running maximum may lag by this much (in log2 units of the scaled scores)
 
-// NC = number of 64-channel chunks of the (zero-padded) head: 1 -> head size 64, 2 -> head sizes 72..128.
-// The wider variant trades buffering for capacity (single Q / P buffers, two K/V stages) to stay within shared memory.
-template <int NC> struct FwdCfg {
-    static constexpr int HSP = 64 * NC;
-    static constexpr int TILE_BYTES = NC * CHUNK_BYTES;
-    static constexpr int QBUF = NC == 1 ? 2 : 1;
-    static constexpr int KVSTAGES = NC == 1 ? 3 : 2;
-    static constexpr int PBUF = NC == 1 ? 2 : 1;
-    static constexpr int SMEM = QBUF * TILE_BYTES + 2 * KVSTAGES * TILE_BYTES + PBUF * P_BYTES + XCH_BYTES + 256;
-    static constexpr int TMEM_COLS = NC == 1 ? 256 : 512;      // S (128) + two O buffers of HSP columns
-};
-
-struct FwdArgs {
-    bf16* out;         // (B, T, NH, HS)
+struct Args {
     float* lse;        // (B, NH, T)
-    int B, T, NH, hs;
+    int T, NH, BH;
+    int ks;            // 16-channel steps of the head: ceil(hs / 16)
     float scale_log2e; // (1/sqrt(HS)) * log2(e)
     float scale;
     unsigned int* status;
 };
 
-DEVINL void quarter_barrier(int q) { asm volatile("bar.sync %0, 128;" ::"r"(1 + q) : "memory"); }
+DEVINL void tmem_st16(uint32_t taddr, const uint32_t* r) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
+        "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
+        ::"r"(taddr),
+          "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
+          "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+        : "memory");
+}
 
-template <int NC>
-__global__ void __launch_bounds__(FWD_THREADS, 1)
-attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const FwdArgs a) {
-    using Cfg = FwdCfg<NC>;
-    constexpr int HSP = Cfg::HSP, TILE_BYTES = Cfg::TILE_BYTES, QBUF = Cfg::QBUF, KVSTAGES = Cfg::KVSTAGES, PBUF = Cfg::PBUF;
+// The items of one CTA: query-tile pair p of a head, late (heavy) pairs first.
+struct Items {
+    int round, cta, grid, total, BH, np, NH, nq;
+    int w, p, b, h;
+    DEVINL void start(int cta_, int grid_, int BH_, int nq_, int NH_) {
+        cta = cta_; grid = grid_; BH = BH_; nq = nq_; np = (nq_ + 1) >> 1; NH = NH_; total = BH * np; round = 0;
+        p = b = h = 0;
+        w = cta;
+        if (w < total) item();
+    }
+    DEVINL bool valid() const { return w < total; }
+    DEVINL void item() { const int rank = w / BH, bh = w - rank * BH; p = np - 1 - rank; b = bh / NH; h = bh - b * NH; }
+    DEVINL void next() {
+        round++;
+        w = round * grid + ((round & 1) ? grid - 1 - cta : cta);
+        if (w < total) item();
+    }
+    DEVINL bool has_b() const { return 2 * p + 1 < nq; }
+    DEVINL int tiles(int x) const { return x == 0 ? 2 * p + 1 : (has_b() ? 2 * p + 2 : 0); }      // key tiles of slot x
+    DEVINL int kv_tiles() const { return has_b() ? 2 * p + 2 : 2 * p + 1; }
+};
+
+__global__ void __launch_bounds__(THREADS, 1)
+attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant__ CUtensorMap tmOut, const Args a) {
     extern __shared__ __align__(1024) uint8_t smem[];
-    uint8_t* sQ = smem;                        // QBUF buffers (current / next work item)
-    uint8_t* sK = sQ + QBUF * TILE_BYTES;      // KVSTAGES stages
-    uint8_t* sV = sK + KVSTAGES * TILE_BYTES;  // KVSTAGES stages
-    uint8_t* sP = sV + KVSTAGES * TILE_BYTES;  // PBUF buffers
-    float* xmax = reinterpret_cast<float*>(sP + PBUF * P_BYTES);   // [2][4][128]
-    float* xsum = xmax + 2 * 4 * 128;                              // [4][128]
-    uint64_t* bars = reinterpret_cast<uint64_t*>(reinterpret_cast<uint8_t*>(xmax) + XCH_BYTES);
-    uint64_t* q_full = bars + 0;     // [2]
-    uint64_t* q_empty = bars + 2;    // [2]
-    uint64_t* k_full = bars + 4;     // [KVSTAGES]
-    uint64_t* k_empty = bars + 8;    // [KVSTAGES]
-    uint64_t* v_full = bars + 12;    // [KVSTAGES]
-    uint64_t* v_empty = bars + 16;   // [KVSTAGES]
-    uint64_t* s_full = bars + 20;
-    uint64_t* s_empty = bars + 21;
-    uint64_t* p_full = bars + 22;
-    uint64_t* o_full = bars + 23;    // [2]
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 25);
+    uint8_t* sQ = smem;                                   // [A, B]
+    uint8_t* sKV = sQ + 2 * TILE_BYTES;                   // [RING]
+    uint8_t* sO = sKV + RING * TILE_BYTES;                // [A, B] output tiles on their way out
+    uint64_t* bars = reinterpret_cast<uint64_t*>(sO + 2 * TILE_BYTES);
+    uint64_t* q_full = bars + 0;      // [2 slots]
+    uint64_t* q_empty = bars + 2;     // [2] the slot's last S of the item is complete          (1 commit)
+    uint64_t* kv_full = bars + 4;     // [3]
+    uint64_t* kv_empty = bars + 7;    // [3]
+    uint64_t* s_full = bars + 10;     // [2] S_X(t) complete, and with it every earlier product (1 commit)
+    uint64_t* p_ready = bars + 12;    // [2] P_X(t) is in TMEM (and O_X rescaled if needed)     (4 arrivals)
+    uint64_t* o_full = bars + 14;     // [2] the item's O_X is complete                         (1 commit)
+    uint64_t* o_free = bars + 16;     // [2] the slot's warps have read O_X                     (4 arrivals)
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 18);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int nq = CEIL_DIV(a.T, BQ);
-    const int BH = a.B * a.NH;
-    const int total = BH * nq;
-    // persistent: work item w -> (query tile, batch, head); late (heavy) query tiles first
-    auto decode = [&](int w, int& qi, int& b, int& h) {
-        const int rank = w / BH, bh = w - rank * BH;
-        qi = nq - 1 - rank;
-        b = bh / a.NH; h = bh - b * a.NH;
-    };
+    const int nq = CEIL_DIV(a.T, BT);
 
     if (threadIdx.x == 0) {
-        if ((smem_u32(smem) & 1023u) != 0) record_error(a.status, ST_BAD_ARG, 0x10);
-        for (int i = 0; i < 2; i++) { mbar_init(&q_full[i], 1); mbar_init(&q_empty[i], 1); mbar_init(&o_full[i], 1); }
-        for (int i = 0; i < KVSTAGES; i++) { mbar_init(&k_full[i], 1); mbar_init(&k_empty[i], 1); mbar_init(&v_full[i], 1); mbar_init(&v_empty[i], 1); }
-        mbar_init(s_full, 1); mbar_init(s_empty, 16); mbar_init(p_full, 16);
+        if ((smem_u32(smem) & 1023u) != 0) record_error(a.status, ST_BAD_ARG, 0x18);
+        for (int i = 0; i < 2; i++) {
+            mbar_init(&q_full[i], 1); mbar_init(&q_empty[i], 1);
+            mbar_init(&s_full[i], 1); mbar_init(&p_ready[i], 4); mbar_init(&o_full[i], 1); mbar_init(&o_free[i], 4);
+        }
+        for (int i = 0; i < RING; i++) { mbar_init(&kv_full[i], 1); mbar_init(&kv_empty[i], 1); }
         *abort_flag = 0;
         mbar_fence_init();
-        tma_prefetch_desc(&tmQKV);
+        tma_prefetch_desc(&tmQKV); tma_prefetch_desc(&tmOut);
     }
-    if (warp == 1) { tmem_alloc(tmem_slot, Cfg::TMEM_COLS); tmem_relinquish(); }
+    if (warp == 1) { tmem_alloc(tmem_slot, TMEM_COLS); tmem_relinquish(); }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
-    const uint32_t tS = tmem_base, tO = tmem_base + 128;       // O partial products: two buffers of HSP columns
+
+    Items im;
+    im.start(blockIdx.x, gridDim.x, a.BH, nq, a.NH);
 
     if (warp == 0) {
+        // ---------------------------------------------------------------- TMA producer
         if (lane == 0) {
-            int kst = 0; uint32_t kph = 0;
-            int it = 0;
-            for (int w = blockIdx.x; w < total; w += gridDim.x, it++) {
-                int qi, b, h; decode(w, qi, b, h);
-                const int qb = it % QBUF;
-                if (!mbar_wait(&q_empty[qb], ((it / QBUF) & 1) ^ 1, abort_flag, a.status, 0x502)) break;
-                mbar_expect_tx(&q_full[qb], TILE_BYTES);
-                #pragma unroll
-                for (int c = 0; c < NC; c++) tma_load_4d(sQ + qb * TILE_BYTES + c * CHUNK_BYTES, &tmQKV, &q_full[qb], c * 64, h, qi * BQ, b);
-                bool fail = false;
-                for (int j = 0; j <= qi; j++) {
-                    const int st = kst;
-                    const uint32_t ph = kph ^ 1;
-                    if (++kst == KVSTAGES) { kst = 0; kph ^= 1; }
-                    if (!mbar_wait(&k_empty[st], ph, abort_flag, a.status, 0x500)) { fail = true; break; }
-                    mbar_expect_tx(&k_full[st], TILE_BYTES);
-                    #pragma unroll
-                    for (int c = 0; c < NC; c++) tma_load_4d(sK + st * TILE_BYTES + c * CHUNK_BYTES, &tmQKV, &k_full[st], c * 64, a.NH + h, j * BKV, b);
-                    if (!mbar_wait(&v_empty[st], ph, abort_flag, a.status, 0x501)) { fail = true; break; }
-                    mbar_expect_tx(&v_full[st], TILE_BYTES);
-                    #pragma unroll
-                    for (int c = 0; c < NC; c++) tma_load_4d(sV + st * TILE_BYTES + c * CHUNK_BYTES, &tmQKV, &v_full[st], c * 64, 2 * a.NH + h, j * BKV, b);
+            auto load = [&](uint8_t* dst, uint64_t* bar, int head, int tile, int b) {
+                mbar_expect_tx(bar, TILE_BYTES);
+                tma_load_4d(dst, &tmQKV, bar, 0, head, tile * BT, b);
+                tma_load_4d(dst + CHUNK_BYTES, &tmQKV, bar, 64, head, tile * BT, b);
+            };
+            uint32_t n = 0;                    // ring tiles so far
+            uint32_t nx[2] = {0, 0};           // items of each slot so far
+            bool fail = false;
+            for (; im.valid() && !fail; im.next()) {
+                const int nkv = im.kv_tiles();
+                for (int j = 0; j < nkv && !fail; j++) {
+                    if (j == 0) {
+                        for (int x = 0; x < (im.has_b() ? 2 : 1) && !fail; x++) {
+                            if (!mbar_wait_relaxed(&q_empty[x], (nx[x] & 1) ^ 1, abort_flag, a.status, 0x502)) { fail = true; break; }
+                            load(sQ + x * TILE_BYTES, &q_full[x], im.h, 2 * im.p + x, im.b);
+                            nx[x]++;
+                        }
+                    }
+                    for (int kv = 0; kv < 2 && !fail; kv++, n++) {
+                        const uint32_t st = n % RING;
+                        if (!mbar_wait_relaxed(&kv_empty[st], ((n / RING) & 1) ^ 1, abort_flag, a.status, 0x500)) { fail = true; break; }
+                        load(sKV + st * TILE_BYTES, &kv_full[st], (kv + 1) * a.NH + im.h, j, im.b);
+                    }
                 }
-                if (fail) break;
             }
         }
     } else if (warp == 1) {
-        // The whole warp runs the issuing code in uniform control flow and one elected lane executes the tcgen05 instructions: a
-        // single lane inside a divergent branch has to move every descriptor from its registers to uniform registers, which costs
-        // it about 90 cycles per product (measured), more than a 128 x 64 x 16 product runs.  Wait results go through a warp vote
-        // so that the compiler knows the branches on them to be uniform; descriptors are built once and advanced by addition.
-        {
-            const bool leader = elect_one();
-#define WAIT_ALL(bar, parity, code) (__all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, a.status, code)) != 0)
-            constexpr uint32_t idesc_s = umma_idesc_bf16(BQ, BKV, 0, 0);     // Q (K-major) x K (K-major)
-            constexpr uint32_t idesc_o = umma_idesc_bf16(BQ, HSP, 0, 1);     // P (K-major) x V (N-major)
-            constexpr uint32_t TILE_UNITS = TILE_BYTES / 16, P_UNITS = P_BYTES / 16;
-            const uint64_t dQ0 = umma_desc_sw128(smem_u32(sQ), 16, 1024), dK0 = umma_desc_sw128(smem_u32(sK), 16, 1024);
-            const uint64_t dP0 = umma_desc_sw128(smem_u32(sP), 16, 1024), dV0 = umma_desc_sw128(smem_u32(sV), CHUNK_BYTES, 1024);
-            auto issue_s = [&](int st, int qb, bool last_of_item) {
-                const uint64_t q = dQ0 + (uint32_t)qb * TILE_UNITS, k = dK0 + (uint32_t)st * TILE_UNITS;
-                if (leader) {
-                    #pragma unroll
-                    for (int kk = 0; kk < HSP / 16; kk++) {      // 64-channel chunks are 16 KB apart, 16 channels = 32 bytes inside a chunk
-                        const uint32_t off = ((kk >> 2) * CHUNK_BYTES + (kk & 3) * 32) / 16;
-                        umma_ss(tS, q + off, k + off, idesc_s, kk > 0);
-                    }
-                    umma_commit(s_full);
-                    umma_commit(&k_empty[st]);
-                    if (last_of_item) umma_commit(&q_empty[qb]);
-                }
-            };
-            uint32_t t = 0;
-            int cst = 0; uint32_t cph = 0;        // K/V ring position of tile t
-            int it = 0;
-            bool ok = true;
-            if ((int)blockIdx.x < total) {
-                int qi, b, h; decode(blockIdx.x, qi, b, h);
-                ok = WAIT_ALL(&q_full[0], 0, 0x510) && WAIT_ALL(&k_full[0], 0, 0x511);
-                tc_fence_after();
-                if (ok) issue_s(0, 0, qi == 0);
-            }
-            for (int w = blockIdx.x; w < total && ok; w += gridDim.x, it++) {
-                int qi, b, h; decode(w, qi, b, h);
-                for (int j = 0; j <= qi && ok; j++, t++) {
-                    // S of the next tile (possibly the first tile of the next work item) as soon as S(t) sits in registers
-                    bool have_next = true, new_item = false; int nqi = qi, nj = j + 1;
-                    if (nj > qi) {
-                        if (w + (int)gridDim.x < total) { int b2, h2; decode(w + gridDim.x, nqi, b2, h2); nj = 0; new_item = true; }
-                        else have_next = false;
-                    }
-                    if (have_next) {
-                        const int nit = it + (new_item ? 1 : 0);
-                        if (new_item) ok = ok && WAIT_ALL(&q_full[nit % QBUF], (nit / QBUF) & 1, 0x516);
-                        int nst = cst + 1; uint32_t nph = cph;
-                        if (nst == KVSTAGES) { nst = 0; nph ^= 1; }
-                        ok = ok && WAIT_ALL(&k_full[nst], nph, 0x512);
-                        ok = ok && WAIT_ALL(s_empty, t & 1, 0x513);
-                        if (!ok) break;
-                        tc_fence_after();
-                        issue_s(nst, nit % QBUF, nj == nqi);
-                    }
-                    ok = ok && WAIT_ALL(p_full, t & 1, 0x514);
-                    ok = ok && WAIT_ALL(&v_full[cst], cph, 0x515);
-                    if (!ok) break;
-                    tc_fence_after();
-                    const uint64_t p = dP0 + (uint32_t)(t % PBUF) * P_UNITS, v = dV0 + (uint32_t)cst * TILE_UNITS;
-                    if (leader) {
-                        #pragma unroll
-                        for (int kk = 0; kk < BKV / 16; kk++) {
-                            // P: two 64-column swizzled chunks of 16 KB; V: 128 kv rows of 128 B, 16 rows per K step
-                            umma_ss(tO + (t & 1) * HSP, p + ((kk >> 2) * (BQ * 128) + (kk & 3) * 32) / 16, v + kk * 128, idesc_o, kk > 0);
-                        }
-                        umma_commit(&o_full[t & 1]);
-                        umma_commit(&v_empty[cst]);
-                    }
-                    if (++cst == KVSTAGES) { cst = 0; cph ^= 1; }
-                }
-            }
-#undef WAIT_ALL
-        }
-    } else {
-        // softmax: thread = query row r x 32-column quarter cq of the S tile; it also owns 16 of the 64 output columns.
-        // These warps meet at named barriers, so they never leave the loops early (abandoned waits return at once).
-        const int q = warp & 3;
-        const int cq = (warp - 2) >> 2;
-        const int r = q * 32 + lane;
-        const uint32_t lane_off = (uint32_t)(q * 32) << 16;
+        // ---------------------------------------------------------------- issuer: per item  S_A(0) S_B(0), then for every key tile j
+        // O_A += P_A(j) V_j, S_A(j+1), O_B += P_B(j) V_j, S_B(j+1); slot B's last two steps have the next item's S_A(0) between them
+        const bool leader = elect_one();
+#define WAIT_ALL(bar, parity, code) (__all_sync(0xffffffffu, mbar_wait_relaxed(bar, parity, abort_flag, a.status, code)) != 0)
+        constexpr uint32_t idesc_s = umma_idesc_bf16(BT, BT, 0, 0);                             // Q (K-major) x K (K-major)
+        const uint32_t idesc_o = umma_idesc_bf16(BT, 0, 0, 1) | ((uint32_t)(a.ks * 2) << 17);   // P (TMEM) x V (N-major), N = 16 ks
+        constexpr uint32_t TILE_UNITS = TILE_BYTES / 16, CHUNK_UNITS = CHUNK_BYTES / 16;
+        const uint64_t dQ0 = umma_desc_sw128(smem_u32(sQ), 16, 1024), dK0 = umma_desc_sw128(smem_u32(sKV), 16, 1024);
+        const uint64_t dV0 = umma_desc_sw128(smem_u32(sKV), CHUNK_BYTES, 1024);
+        const int ks = a.ks;
+        uint32_t tp[2] = {0, 0};          // P V products issued per slot
+        uint32_t qn[2] = {0, 0};          // Q tiles (items) whose first S has been issued per slot
+        uint32_t on[2] = {0, 0};          // items whose first P V has been issued per slot
+        uint32_t kabs = 0;                // key tiles of earlier items: K_j sits at ring position 2 (kabs + j), V_j behind it
         bool ok = true;
-        uint32_t t = 0;
-        for (int w = blockIdx.x; w < total; w += gridDim.x) {
-            int qi, b, h; decode(w, qi, b, h);
-            float m = -INFINITY, l = 0.f;
-            float O[16 * NC];                  // columns c*64 + cq*16 .. +15 of every 64-channel chunk c
-            #pragma unroll
-            for (int d = 0; d < 16 * NC; d++) O[d] = 0.f;
-            // adds the finished P V of tile `tt` to the running output (optionally rescaled afterwards)
-            auto fold = [&](uint32_t tt, float rescale) {
-                ok = mbar_wait(&o_full[tt & 1], (tt >> 1) & 1, abort_flag, a.status, 0x521) && ok;
-                tc_fence_after();
+        auto kv_wait = [&](uint32_t pos, uint32_t code) { return WAIT_ALL(&kv_full[pos % RING], (pos / RING) & 1, code); };
+        // S_x of the key tile at ring position pos; first: the slot's Q tile is new; the slot that reads a K tile last releases it
+        auto issue_s = [&](int x, uint32_t pos, bool first, bool release_k, bool last) {
+            bool good = true;
+            if (first) good = WAIT_ALL(&q_full[x], qn[x]++ & 1, 0x510);
+            good = good && kv_wait(pos, 0x511);
+            if (!good) return false;
+            tc_fence_after();
+            const uint64_t q = dQ0 + (uint32_t)x * TILE_UNITS, k = dK0 + (pos % RING) * TILE_UNITS;
+            if (leader) {
                 #pragma unroll
-                for (int c = 0; c < NC; c++) {
-                    uint32_t ov[16];
-                    tmem_ld16(tO + (tt & 1) * HSP + c * 64 + lane_off + cq * 16, ov);
-                    tmem_ld_wait();
-                    #pragma unroll
-                    for (int d = 0; d < 16; d++) O[c * 16 + d] = (O[c * 16 + d] + __uint_as_float(ov[d])) * rescale;
+                for (int kk = 0; kk < 8; kk++)
+                    if (kk < ks)
+                        umma_ss(tmem_base + x * 128, q + (kk >> 2) * CHUNK_UNITS + (kk & 3) * 2, k + (kk >> 2) * CHUNK_UNITS + (kk & 3) * 2, idesc_s, kk > 0);
+                umma_commit(&s_full[x]);
+                if (release_k) umma_commit(&kv_empty[pos % RING]);
+                if (last) umma_commit(&q_empty[x]);
+            }
+            return true;
+        };
+        // O_x += P_x V: A = P_x in TMEM (16 keys = 8 columns per step), B = V N-major (16 rows = 2048 bytes per step)
+        auto issue_pv = [&](int x, uint32_t pos, bool first, bool release_v, bool last) {
+            bool good = kv_wait(pos, 0x515) && WAIT_ALL(&p_ready[x], tp[x] & 1, 0x514);
+            if (good && first && on[x] > 0) good = WAIT_ALL(&o_free[x], (on[x] - 1) & 1, 0x517);
+            if (!good) return false;
+            tc_fence_after();
+            const uint64_t v = dV0 + (pos % RING) * TILE_UNITS;
+            if (leader) {
+                #pragma unroll
+                for (int kk = 0; kk < BT / 16; kk++) umma_ts(tmem_base + 256 + x * 128, tmem_base + x * 128 + kk * 8, v + 128 * kk, idesc_o, !first || kk > 0);
+                if (release_v) umma_commit(&kv_empty[pos % RING]);
+                if (last) umma_commit(&o_full[x]);
+            }
+            tp[x]++;
+            if (first) on[x]++;
+            return true;
+        };
+        // S_x(0) of an item whose key tiles start at kabs_
+        auto issue_first = [&](const Items& it, int x, uint32_t kabs_) {
+            const bool reads_last = it.has_b() ? x == 1 : x == 0;
+            return issue_s(x, 2 * kabs_, true, reads_last, it.tiles(x) == 1);
+        };
+        if (im.valid()) {
+            ok = issue_first(im, 0, 0);
+            if (ok && im.has_b()) ok = issue_first(im, 1, 0);
+        }
+        while (im.valid() && ok) {
+            Items nx = im; nx.next();
+            const int nA = im.tiles(0), nB = im.tiles(1), nkv = im.kv_tiles();
+            for (int j = 0; j < nkv && ok; j++) {
+                const uint32_t kpos = 2 * (kabs + j);
+                if (j < nA) {
+                    ok = issue_pv(0, kpos + 1, j == 0, nB == 0, j == nA - 1);
+                    if (ok && j + 1 < nA) ok = issue_s(0, kpos + 2, false, nB == 0, j + 1 == nA - 1);
                 }
-                tc_fence_before();
-            };
-            for (int j = 0; j <= qi; j++, t++) {
-                ok = mbar_wait(s_full, t & 1, abort_flag, a.status, 0x520) && ok;
+                // the next item's first S of slot A: its K tile is behind this item's tiles in the ring
+                if (ok && j == nkv - 1 && nx.valid()) ok = issue_first(nx, 0, kabs + nkv);
+                if (ok && j < nB) {
+                    ok = issue_pv(1, kpos + 1, j == 0, true, j == nB - 1);
+                    if (ok && j + 1 < nB) ok = issue_s(1, kpos + 2, false, true, j + 1 == nB - 1);
+                }
+            }
+            kabs += nkv;
+            if (ok && nx.valid() && nx.has_b()) ok = issue_first(nx, 1, kabs);
+            im = nx;
+        }
+#undef WAIT_ALL
+    }
+    else if (warp >= 4) {
+        // ---------------------------------------------------------------- softmax of slot x: thread = query row r of the slot's tile
+        const int x = (warp - 4) >> 2;
+        const int q4 = warp & 3;
+        const int r = q4 * 32 + lane;
+        const uint32_t lane_off = (uint32_t)(q4 * 32) << 16;
+        const uint32_t tS = tmem_base + x * 128 + lane_off, tO = tmem_base + 256 + x * 128 + lane_off;
+        const bool issuer = q4 == 0 && lane == 0;          // the thread of the slot that issues its output stores
+        const float c = a.scale_log2e;
+        bool ok = true;
+        bool staged = false;
+        uint32_t t = 0;                                    // tiles of this slot so far
+        uint32_t it = 0;                                   // items of this slot so far
+        for (; im.valid(); im.next()) {
+            const int nj = im.tiles(x);
+            if (nj == 0) continue;                         // (uniform for the slot) no second tile in this item
+            float m = -INFINITY, l = 0.f;                  // reference maximum (raw score units) and row sum relative to it
+            for (int j = 0; j < nj; j++, t++) {
+                ok = mbar_wait(&s_full[x], t & 1, abort_flag, a.status, 0x520 + x) && ok;
+                // The first S products of both slots complete together: the slots would compete for the special-function unit and then leave
+                // it idle together.  Slot B starts half a tile late; from then on the order of the products keeps the two apart.
+                if (x == 1 && t == 0) { const long long t0 = clock64(); while (clock64() - t0 < SKEW_CYCLES) { } }
                 tc_fence_after();
-                uint32_t v[32];
-                tmem_ld32(tS + lane_off + cq * 32, v);
+                uint32_t sv[128];
+                tmem_ld32(tS, sv);
+                tmem_ld32(tS + 32, sv + 32);
+                tmem_ld32(tS + 64, sv + 64);
+                tmem_ld32(tS + 96, sv + 96);
                 tmem_ld_wait();
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(s_empty);
-                float mx = -INFINITY;
-                if (j == qi) {
+                if (j == nj - 1) {
                     #pragma unroll
-                    for (int e = 0; e < 32; e++) {
-                        if (cq * 32 + e > r) v[e] = 0xff800000u;      // -inf: above the diagonal
-                        mx = fmaxf(mx, __uint_as_float(v[e]));
-                    }
-                } else {
-                    #pragma unroll
-                    for (int e = 0; e < 32; e++) mx = fmaxf(mx, __uint_as_float(v[e]));
+                    for (int e = 0; e < 128; e++) if (e > r) sv[e] = 0xff800000u;      // -inf above the diagonal
                 }
-                // row maximum over the four column quarters
-                float* xm = xmax + (t & 1) * 512;
-                xm[cq * 128 + r] = mx;
-                quarter_barrier(q);
-                mx = fmaxf(fmaxf(xm[r], xm[128 + r]), fmaxf(xm[256 + r], xm[384 + r]));
-                const float m_new = fmaxf(m, mx);
-                const float alpha = ex2_fast((m - m_new) * a.scale_log2e);      // m = -inf on the first tile -> 0
-                m = m_new;
-                const float moff = m * a.scale_log2e;
-                float rs = 0.f;
-                uint32_t pk[16];
+                float mx0 = -INFINITY, mx1 = -INFINITY, mx2 = -INFINITY, mx3 = -INFINITY;
                 #pragma unroll
-                for (int e = 0; e < 32; e += 2) {
-                    const float p0 = ex2_fast(fmaf(__uint_as_float(v[e]), a.scale_log2e, -moff));
-                    const float p1 = ex2_fast(fmaf(__uint_as_float(v[e + 1]), a.scale_log2e, -moff));
-                    rs += p0 + p1;
+                for (int e = 0; e < 128; e += 4) {
+                    mx0 = fmaxf(mx0, __uint_as_float(sv[e])); mx1 = fmaxf(mx1, __uint_as_float(sv[e + 1]));
+                    mx2 = fmaxf(mx2, __uint_as_float(sv[e + 2])); mx3 = fmaxf(mx3, __uint_as_float(sv[e + 3]));
+                }
+                const float mx = fmaxf(fmaxf(mx0, mx1), fmaxf(mx2, mx3));
+                // move the reference maximum only when it lags by more than 2^RESCALE_LOG2 (decided per warp, so that the
+                // TMEM accesses stay warp-wide); a moved maximum rescales the row sum now and the row of O_X below
+                const bool grow = (mx - m) * c > RESCALE_LOG2 || j == 0;
+                const bool moved = __any_sync(0xffffffffu, grow) != 0;
+                float alpha = 1.0f;
+                if (moved) {
+                    const float m_new = fmaxf(m, mx);
+                    alpha = ex2_fast((m - m_new) * c);      // 0 on the first tile (m = -inf)
+                    l *= alpha;
+                    m = m_new;
+                }
+                const float moff = m * c;
+                float rs0 = 0.f, rs1 = 0.f;
+                uint32_t pk[64];
+                #pragma unroll
+                for (int e = 0; e < 128; e += 2) {
+                    const float p0 = ex2_fast(fmaf(__uint_as_float(sv[e]), c, -moff));
+                    const float p1 = ex2_fast(fmaf(__uint_as_float(sv[e + 1]), c, -moff));
+                    rs0 += p0; rs1 += p1;
                     pk[e >> 1] = pack_bf16x2(p0, p1);
                 }
-                l = l * alpha + rs;
-                if (PBUF == 1 && j > 0) fold(t - 1, alpha);      // single P buffer: the previous P V must have consumed it
-                uint8_t* prow = sP + (t % PBUF) * P_BYTES + (cq >> 1) * (BQ * 128) + r * 128;
-                #pragma unroll
-                for (int u = 0; u < 4; u++) {
-                    const int pos = ((((cq & 1) * 4) + u) ^ (r & 7)) * 16;
-                    *reinterpret_cast<uint4*>(prow + pos) = make_uint4(pk[u * 4], pk[u * 4 + 1], pk[u * 4 + 2], pk[u * 4 + 3]);
-                }
-                fence_async_smem();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(p_full);
-                // fold in the previous tile's P V (rescaled to the new maximum together with the running output)
-                if (PBUF != 1 && j > 0) fold(t - 1, alpha);
-            }
-            fold(t - 1, 1.0f);      // last tile of the item
-            // total row sum over the four quarters
-            xsum[cq * 128 + r] = l;
-            quarter_barrier(q);
-            l = xsum[r] + xsum[128 + r] + xsum[256 + r] + xsum[384 + r];
-            const int trow = qi * BQ + r;
-            if (trow < a.T && ok) {
-                const float inv = 1.0f / l;
-                bf16* op = a.out + (((size_t)b * a.T + trow) * a.NH + h) * a.hs;
-                #pragma unroll
-                for (int c = 0; c < NC; c++) {
+                l += rs0 + rs1;
+                tmem_st16(tS, pk);                          // over this row's own scores
+                tmem_st16(tS + 16, pk + 16);
+                tmem_st16(tS + 32, pk + 32);
+                tmem_st16(tS + 48, pk + 48);
+                if (moved && j > 0) {                       // O_X(t-1) is complete: its product was issued ahead of S_X(t)
                     #pragma unroll
-                    for (int d = 0; d < 16; d += 8) {
-                        const int col = c * 64 + cq * 16 + d;
-                        if (col < a.hs) {          // head sizes are multiples of 8: whole 16-byte groups
-                            const float* Oc = O + c * 16 + d;
-                            uint4 o;
-                            o.x = pack_bf16x2(Oc[0] * inv, Oc[1] * inv); o.y = pack_bf16x2(Oc[2] * inv, Oc[3] * inv);
-                            o.z = pack_bf16x2(Oc[4] * inv, Oc[5] * inv); o.w = pack_bf16x2(Oc[6] * inv, Oc[7] * inv);
-                            *reinterpret_cast<uint4*>(op + col) = o;
+                    for (int cc = 0; cc < 4; cc++) {
+                        if (cc * 2 < a.ks) {
+                            uint32_t ov[32];
+                            tmem_ld32(tO + cc * 32, ov);
+                            tmem_ld_wait();
+                            #pragma unroll
+                            for (int e = 0; e < 32; e++) ov[e] = __float_as_uint(__uint_as_float(ov[e]) * alpha);
+                            tmem_st16(tO + cc * 32, ov);
+                            tmem_st16(tO + cc * 32 + 16, ov + 16);
                         }
                     }
                 }
-                if (cq == 0) a.lse[((size_t)b * a.NH + h) * a.T + trow] = m * a.scale + logf(l);
+                tmem_st_wait();
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&p_ready[x]);
             }
+            // ---- item epilogue: O_X / l -> bf16 tile in the layout of two 128-byte-swizzled TMA boxes -> bulk stores
+            ok = mbar_wait(&o_full[x], it & 1, abort_flag, a.status, 0x528 + x) && ok;
+            it++;
+            tc_fence_after();
+            if (staged) { if (issuer) tma_store_wait_read<0>(); asm volatile("bar.sync %0, 128;" ::"r"(1 + x) : "memory"); }
+            const float inv = 1.0f / l;
+            #pragma unroll
+            for (int cc = 0; cc < 4; cc++) {
+                if (cc * 2 < a.ks) {
+                    uint32_t ov[32];
+                    tmem_ld32(tO + cc * 32, ov);
+                    tmem_ld_wait();
+                    uint8_t* orow = sO + x * TILE_BYTES + (cc >> 1) * CHUNK_BYTES + r * 128;
+                    #pragma unroll
+                    for (int u = 0; u < 4; u++) {
+                        uint4 o;
+                        o.x = pack_bf16x2(__uint_as_float(ov[8 * u]) * inv, __uint_as_float(ov[8 * u + 1]) * inv);
+                        o.y = pack_bf16x2(__uint_as_float(ov[8 * u + 2]) * inv, __uint_as_float(ov[8 * u + 3]) * inv);
+                        o.z = pack_bf16x2(__uint_as_float(ov[8 * u + 4]) * inv, __uint_as_float(ov[8 * u + 5]) * inv);
+                        o.w = pack_bf16x2(__uint_as_float(ov[8 * u + 6]) * inv, __uint_as_float(ov[8 * u + 7]) * inv);
+                        *reinterpret_cast<uint4*>(orow + ((((cc & 1) * 4 + u) ^ (r & 7)) * 16)) = o;
+                    }
+                }
+            }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&o_free[x]);            // O_X may be overwritten by the next item's first product
+            fence_async_smem();
+            asm volatile("bar.sync %0, 128;" ::"r"(1 + x) : "memory");
+            const int qi = 2 * im.p + x;
+            if (issuer && ok) {
+                tma_store_4d(&tmOut, sO + x * TILE_BYTES, 0, im.h, qi * BT, im.b);
+                tma_store_4d(&tmOut, sO + x * TILE_BYTES + CHUNK_BYTES, 64, im.h, qi * BT, im.b);
+                tma_store_commit();
+            }
+            staged = true;
+            const int trow = qi * BT + r;
+            if (trow < a.T && ok) a.lse[((size_t)im.b * a.NH + im.h) * a.T + trow] = m * a.scale + logf(l);
         }
+        if (issuer) tma_store_wait<0>();
     }
     tc_fence_before();
     __syncthreads();
@@ -322,7 +365,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const FwdArgs a) {
         while (clock64() - t0 < 2000000ll) { __nanosleep(1000); }
         __syncthreads();
     }
-    if (warp == 1) tmem_dealloc(tmem_base, Cfg::TMEM_COLS);
+    if (warp == 1) tmem_dealloc(tmem_base, TMEM_COLS);
 }
 
 }  // namespace
@@ -335,32 +378,34 @@ int llmc_attn_qkv_map(CUtensorMap* tm, const bf16* qkv, int B, int T, int NH, in
     return llmc_get_tensormap(tm, qkv, 2, 4, dims, strides, box, 3);
 }
 
-template <int NC>
-int launch_fwd(const CUtensorMap& tm, const FwdArgs& a, int grid, cudaStream_t stream) {
-    static bool configured = false;
-    if (!configured) {
-        CUDA_CHECK(cudaFuncSetAttribute(attn_fwd_kernel<NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, FwdCfg<NC>::SMEM));
-        configured = true;
-    }
-    attn_fwd_kernel<NC><<<grid, FWD_THREADS, FwdCfg<NC>::SMEM, stream>>>(tm, a);
-    CUDA_CHECK(cudaGetLastError());
-    return 0;
-}
-
-// out (B,T,NH,HS) = causal softmax(Q K^T / sqrt(HS)) V ; lse (B,NH,T) fp32.  Head sizes: multiples of 8 up to 128.
+// out (B,T,NH,HS) = causal softmax(Q K^T / sqrt(HS)) V ; lse (B,NH,T) fp32.  Head sizes: multiples of 8, 72..128.
 // The entry point llmc_attention_fwd (attention_fwd1.cu) sends every head size but 64 here.
 int llmc_attention_fwd_general(bf16* out, float* lse, const bf16* qkv, int B, int T, int NH, int hs, cudaStream_t stream) {
-    if (hs < 64 || hs > 128 || (hs % 8)) { fprintf(stderr, "[llmc_b200] attention: head size %d not supported (multiples of 8 from 64 to 128)\n", hs); return -1; }
-    CUtensorMap tm;
-    int rc = llmc_attn_qkv_map(&tm, qkv, B, T, NH, hs);
+    if (hs <= 64 || hs > 128 || (hs % 8)) { fprintf(stderr, "[llmc_b200] attention: head size %d not supported (multiples of 8 from 64 to 128)\n", hs); return -1; }
+    CUtensorMap tmQKV, tmOut;
+    int rc = llmc_attn_qkv_map(&tmQKV, qkv, B, T, NH, hs);
     if (rc) return rc;
-    FwdArgs a;
-    a.out = out; a.lse = lse; a.B = B; a.T = T; a.NH = NH; a.hs = hs;
+    {
+        uint64_t dims[4] = {(uint64_t)hs, (uint64_t)NH, (uint64_t)T, (uint64_t)B};
+        uint64_t strides[4] = {2, (uint64_t)hs * 2, (uint64_t)NH * hs * 2, (uint64_t)T * NH * hs * 2};
+        uint32_t box[4] = {64, 1, 128, 1};
+        if ((rc = llmc_get_tensormap(&tmOut, out, 2, 4, dims, strides, box, 3))) return rc;
+    }
+    Args a;
+    a.lse = lse; a.T = T; a.NH = NH; a.BH = B * NH;
+    a.ks = CEIL_DIV(hs, 16);
     a.scale = 1.0f / sqrtf((float)hs);
     a.scale_log2e = a.scale * 1.4426950408889634f;
     a.status = llmc_status_ptr();
-    const int nq = CEIL_DIV(T, BQ);
+    const int total = B * NH * ((CEIL_DIV(T, BT) + 1) / 2);
     int sms = llmc_device_sm_count(); if (sms <= 0) sms = 148;
-    const int grid = B * NH * nq < sms ? B * NH * nq : sms;
-    return hs <= 64 ? launch_fwd<1>(tm, a, grid, stream) : launch_fwd<2>(tm, a, grid, stream);
+    const int grid = total < sms ? total : sms;
+    static bool configured = false;
+    if (!configured) {
+        CUDA_CHECK(cudaFuncSetAttribute(attn_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM));
+        configured = true;
+    }
+    attn_fwd_kernel<<<grid, THREADS, SMEM, stream>>>(tmQKV, tmOut, a);
+    CUDA_CHECK(cudaGetLastError());
+    return 0;
 }
