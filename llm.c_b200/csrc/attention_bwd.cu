@@ -1,27 +1,40 @@
-// Causal flash attention backward for sm_100a on the packed (B, T, 3, NH, HS) layout; head sizes 64..128
-// (multiples of 8; sizes above 64 run as a 128-wide head whose missing channels TMA fills with zeros).
+// Causal flash attention backward for sm_100a on the packed (B, T, 3, NH, HS) layout, head sizes 72..128 (multiples of 8; a
+// narrower head runs as a 128-wide one whose missing channels TMA fills with zeros, with the products cut to whole 16-channel steps).
 //
-// Deterministic by construction: no atomics, every output element has one writer and a fixed
-// summation order.  Three launches:
+// Deterministic by construction: no atomics, every output element has one writer and a fixed summation order.  Three launches:
 //   1. delta[b,h,t] = sum_d O[b,t,h,d] * dO[b,t,h,d]
-//   2. "dK/dV" kernel: one CTA per (b, h, 128-row key/value tile).  K_j and V_j stay resident in
-//      shared memory while the query tiles i >= j stream through a 2-stage TMA ring.  Per query tile
-//      S = Q K^T and dP = dO V^T are formed in TMEM, the 512 softmax threads turn them into
-//      P = exp(S*scale - LSE) and dS = P (dP - delta) scale (bf16, swizzled shared memory), and
-//      dV += P^T dO, dK += dS^T Q accumulate in TMEM over the whole loop (MN-major A operands).
-//   3. "dQ" kernel: one CTA per (b, h, query tile); K_j, V_j stream; dQ += dS K accumulates in TMEM.
-// S and dP are recomputed in (3) instead of exchanging dQ partials through atomics; that costs two
-// extra MMAs per tile and buys bit-reproducible gradients, which the reference also demands of
-// cuDNN (llmc/cudnn_att.cpp:186-191).
+//   2. dK / dV: the key tile (K_j, V_j) stays in shared memory, the query tiles i >= j stream past it.  The score tiles are formed
+//      TRANSPOSED (keys on the TMEM lanes): S^T = K Q^T, dP^T = V dO^T, so that P^T and dS^T, written back to tensor memory as
+//      bf16 over the scores they came from, are the A operands of dV += P^T dO and dK += dS^T Q.
+//   3. dQ: the query tile (Q_i, dO_i) stays, the key tiles j <= i stream; S = Q K^T, dP = dO V^T, dQ += dS K_j with dS in TMEM.
 //
-// Both MMA kernels are persistent (one CTA per SM walks a heavy-first list of work items; resident tiles and
-// TMEM accumulators are double buffered across items).  A CTA has 608 threads: warp 0 TMA producer, warp 1 issuer of the score
-// products (S, dP), warps 2..17 softmax/epilogue (thread = one row x one 32-column quarter), warp 18 issuer of the accumulating
-// products (dV, dK or dQ).  The softmax threads pull S/dP into registers and release the TMEM tiles at once, so the next
-// tile's S/dP MMAs run underneath the exponentials.
+// Why two passes with S and dP formed twice and not one: with 128 channels a tile pair's dQ contribution is 64 KB of fp32.  Summing
+// these in a fixed order through memory (what attention_bwd1.cu does at 64 channels) would write and read them at the rate of
+// HBM, which takes longer than the two extra products; and dV, dK, dQ and both score tiles together do not fit 512 TMEM columns.
 //
-// Capability parity: attention_backward_cudnn (llmc/cudnn_att.cpp:256-288) and attention_backward
-// of llmc/attention.cuh in the reference.
+// Both passes are bound by the softmax warps (16 exponentials per clock and SM: 1024 cycles for a 128 x 128 tile, plus the TMEM
+// loads and stores around them) with the tensor pipe close behind (2048 / 1536 cycles a pair).  So nothing but that is left to the
+// softmax warps: no operand goes through shared memory (the kernel this one replaces staged P and dS there, with one stage of
+// streamed tiles), S of the next pair is issued before dS of this one is finished, the outputs leave through four warps of
+// their own.  All three launches, the kernels before these in brackets: B=16 T=2048 NH=8 HS=128 521 us (978), B=2 T=4096 NH=32 HS=128
+// 880 us (1723), B=3 T=1000 NH=32 HS=80 113 us (235).
+//
+// Work items are one fixed tile of one head, heaviest first, dealt to the persistent CTAs in alternating direction (CTA c gets items
+// c, 2G-1-c, 2G+c, ...), which evens out the decreasing sizes; a plain round-robin gives CTA 0 the longest item of every round.
+//
+// Roles inside a CTA (512 threads):
+//   warp 0       TMA producer (fixed tiles single-buffered, each of the two released by the last product that reads it, one pair
+//                before the item ends; X0, which a pair needs from its first product to its last, in a ring of three, X1, which is
+//                free again by the middle of its pair, in one buffer: with both in a two-stage ring S waited for loads)
+//   warp 1       issuer of the products; program order keeps a score tile from overwriting the bf16 operand that aliases it
+//   warps 4-11   softmax: thread = row of the score tile x 64-column half
+//   warps 12-15  drain: accumulators -> bf16 -> shared memory -> TMA store; in the dK / dV pass also the per-query statistics table
+//
+// TMEM columns: S [0,128) (P^T bf16 in the first 32 columns of each half)   dP [128,256) (dS bf16 likewise)
+//               dK/dV pass: dV [256,384) dK [384,512)      dQ pass: dQ [256,384), second S buffer [384,512)
+//
+// Capability parity: attention_backward_cudnn (llmc/cudnn_att.cpp:256-288) and attention_backward of llmc/attention.cuh in the
+// reference, which also demands reproducible gradients of cuDNN (llmc/cudnn_att.cpp:186-191).
 #include "common.cuh"
 
 int llmc_attn_qkv_map(CUtensorMap* tm, const bf16* qkv, int B, int T, int NH, int hs);   // attention_fwd.cu
@@ -29,29 +42,20 @@ int llmc_attn_qkv_map(CUtensorMap* tm, const bf16* qkv, int B, int T, int NH, in
 namespace {
 
 constexpr int BT = 128;                             // tile rows (queries and keys)
-constexpr int CHUNK_BYTES = 128 * 64 * 2;           // 16 KB: 128 rows x 64 channels, one 128-byte-swizzled TMA box
-constexpr int PS_BYTES = BT * BT * 2;               // 32 KB
-constexpr int BWD_THREADS = 608;                    // TMA warp + score-product issuer + 16 softmax warps + accumulate-product issuer
-constexpr int BWD_TMEM_COLS = 512;
+constexpr int CHUNK_BYTES = BT * 64 * 2;            // 16 KB: 128 rows x 64 channels, one 128-byte-swizzled TMA box
+constexpr int TILE_BYTES = 2 * CHUNK_BYTES;
+constexpr int X0STAGES = 3;                         // ring of the streamed tiles X0; X1 has one buffer
+constexpr int THREADS = 512;
+constexpr int TMEM_COLS = 512;
+constexpr int STAT_BYTES = 2 * 2 * BT * 4;          // [2 buffers][lse, delta][128 queries]
+constexpr int SMEM = 2 * TILE_BYTES + (X0STAGES + 1) * TILE_BYTES + TILE_BYTES + STAT_BYTES + 256;
+static_assert(SMEM <= 232448, "shared memory of one CTA");
 
-// NC = number of 64-channel chunks of the (zero-padded) head: 1 -> head size 64, 2 -> head sizes 72..128.
-// With two chunks a tile pair is 64 KB and an accumulator pair fills the rest of TMEM, so that variant runs without
-// double buffering (one resident buffer, one stream stage, one accumulator set).
-template <int NC> struct BwdCfg {
-    static constexpr int HSP = 64 * NC;
-    static constexpr int TILE_BYTES = NC * CHUNK_BYTES;
-    static constexpr int PAIR_BYTES = 2 * TILE_BYTES;
-    static constexpr int RB = NC == 1 ? 2 : 1;          // resident pair buffers
-    static constexpr int XSTAGES = NC == 1 ? 3 : 1;     // ring of streamed tile pairs
-    static constexpr int ACCBUF = NC == 1 ? 2 : 1;      // TMEM accumulator sets (each 2 * HSP columns)
-    static constexpr int SMEM = RB * PAIR_BYTES + XSTAGES * PAIR_BYTES + 2 * PS_BYTES + 256;
-};
-
-struct BwdArgs {
-    bf16* dqkv;          // (B, T, 3, NH, HS)
+struct Args {
     const float* lse;    // (B, NH, T)
     const float* delta;  // (B, NH, T)
-    int B, T, NH, hs;
+    int T, NH, BH;
+    int ks;              // 16-channel steps of the head: ceil(hs / 16)
     float scale, scale_log2e;
     unsigned int* status;
 };
@@ -81,316 +85,388 @@ __global__ void delta_kernel(float* __restrict__ delta, const bf16* __restrict__
     }
 }
 
-// DKV = true : resident (K_j, V_j), streamed (Q_i, dO_i), outputs dK_j, dV_j
-// DKV = false: resident (Q_i, dO_i), streamed (K_j, V_j), output dQ_i
-// Persistent: gridDim.x CTAs (one per SM) take work items w = blockIdx.x, blockIdx.x + gridDim.x, ...; the item list is
-// ordered heavy first.  The resident pair and the TMEM accumulators are double buffered so that the loads and the first
-// MMAs of the next item run underneath the epilogue of the current one.
-template <bool DKV, int NC>
-__global__ void __launch_bounds__(BWD_THREADS, 1)
-attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant__ CUtensorMap tmDO, const BwdArgs a) {
-    using Cfg = BwdCfg<NC>;
-    constexpr int HSP = Cfg::HSP, TILE_BYTES = Cfg::TILE_BYTES, PAIR_BYTES = Cfg::PAIR_BYTES;
-    constexpr int RB = Cfg::RB, XSTAGES = Cfg::XSTAGES, ACCBUF = Cfg::ACCBUF;
+DEVINL void tmem_st16(uint32_t taddr, const uint32_t* r) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
+        "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
+        ::"r"(taddr),
+          "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
+          "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+        : "memory");
+}
+DEVINL void tmem_st8(uint32_t taddr, const uint32_t* r) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+        ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]) : "memory");
+}
+
+// The sequence of tile pairs of one CTA.  f: the item's fixed tile (key tile in the dK / dV pass, query tile in the dQ pass),
+// x: the streamed tile, x0..x1 its range.
+template <bool DKV>
+struct Walk {
+    int round, cta, grid, total, BH, nt, NH;
+    int w, bh, b, h, f, x, x0, x1;
+    DEVINL void start(int cta_, int grid_, int BH_, int nt_, int NH_) {
+        cta = cta_; grid = grid_; BH = BH_; nt = nt_; NH = NH_; total = BH_ * nt_; round = 0;
+        bh = b = h = f = x = x0 = x1 = 0;
+        w = cta;
+        if (w < total) item();
+    }
+    DEVINL bool valid() const { return w < total; }
+    DEVINL void item() {
+        const int rank = w / BH;
+        bh = w - rank * BH; b = bh / NH; h = bh - b * NH;
+        if (DKV) { f = rank; x0 = f; x1 = nt - 1; }
+        else { f = nt - 1 - rank; x0 = 0; x1 = f; }
+        x = x0;
+    }
+    DEVINL bool first() const { return x == x0; }
+    DEVINL bool last() const { return x == x1; }
+    DEVINL void next() {                      // valid() turns false past the last pair
+        if (++x <= x1) return;
+        round++;
+        w = round * grid + ((round & 1) ? grid - 1 - cta : cta);
+        if (w < total) item();
+    }
+};
+
+template <bool DKV>
+__global__ void __launch_bounds__(THREADS, 1)
+attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant__ CUtensorMap tmDO,
+                const __grid_constant__ CUtensorMap tmDQKV, const Args a) {
     extern __shared__ __align__(1024) uint8_t smem[];
-    uint8_t* sRes = smem;                              // [RB][2 tiles]
-    uint8_t* sStr = sRes + RB * PAIR_BYTES;            // [XSTAGES][2 tiles]
-    uint8_t* sP = sStr + XSTAGES * PAIR_BYTES;
-    uint8_t* sdS = sP + PS_BYTES;
-    uint64_t* bars = reinterpret_cast<uint64_t*>(sdS + PS_BYTES);
-    uint64_t* res_full = bars + 0;    // [2]
-    uint64_t* res_empty = bars + 2;   // [2]
-    uint64_t* x_full = bars + 4;      // [XSTAGES]
-    uint64_t* x_empty = bars + 8;     // [XSTAGES]
-    uint64_t* sdp_full = bars + 12;
-    uint64_t* sdp_empty = bars + 13;
-    uint64_t* pds_full = bars + 14;
-    uint64_t* pds_empty = bars + 15;
-    uint64_t* acc_full = bars + 16;   // [2]
-    uint64_t* acc_empty = bars + 18;  // [2]
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 20);
+    uint8_t* sF = smem;                                // fixed tiles F0 (K_j / Q_i), F1 (V_j / dO_i)
+    uint8_t* sX0 = sF + 2 * TILE_BYTES;                // [X0STAGES] streamed tiles X0 (Q_i / K_j)
+    uint8_t* sX1 = sX0 + X0STAGES * TILE_BYTES;        // streamed tile X1 (dO_i / V_j)
+    uint8_t* sOut = sX1 + TILE_BYTES;                  // an accumulator tile on its way out (two TMA boxes)
+    float* sStat = reinterpret_cast<float*>(sOut + TILE_BYTES);     // [2][2][128]
+    uint64_t* bars = reinterpret_cast<uint64_t*>(reinterpret_cast<uint8_t*>(sStat) + STAT_BYTES);
+    uint64_t* f_full = bars + 0;      // [F0, F1]
+    uint64_t* f_empty = bars + 2;     // [F0, F1]
+    uint64_t* x0_full = bars + 21;    // [3]
+    uint64_t* x0_empty = bars + 24;   // [3]
+    uint64_t* x1_full = bars + 4;
+    uint64_t* x1_empty = bars + 5;
+    uint64_t* s_full = bars + 8;      // [2] S(t) complete, t & 1                           (1 commit)
+    uint64_t* dp_full = bars + 10;    // dP(t) complete                                     (1 commit)
+    uint64_t* p_ready = bars + 11;    // P^T(t) is in TMEM                                  (8 arrivals)
+    uint64_t* ds_ready = bars + 12;   // dS(t) is in TMEM, S(t) has been read               (8 arrivals)
+    uint64_t* acc_full = bars + 13;   // [2] accumulator of the item complete               (1 commit)
+    uint64_t* acc_empty = bars + 15;  // [2] the drain warps have read it                   (4 arrivals)
+    uint64_t* st_full = bars + 17;    // [2] statistics table of a pair written             (4 arrivals)
+    uint64_t* st_empty = bars + 19;   // [2] ... and read by every softmax warp             (8 arrivals)
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 27);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int nt = CEIL_DIV(a.T, BT);
-    const int BH = a.B * a.NH;
-    const int total = BH * nt;
-    // work item -> (fixed tile, batch, head, number of streamed tiles); heavy items first:
-    // key tile 0 sees every query tile; query tile nt-1 sees every key tile
-    auto decode = [&](int w, int& fixed, int& b, int& h, int& cnt) {
-        const int rank = w / BH, bh = w - rank * BH;
-        fixed = DKV ? rank : (nt - 1 - rank);
-        cnt = DKV ? (nt - fixed) : (fixed + 1);
-        b = bh / a.NH; h = bh - b * a.NH;
-    };
 
     if (threadIdx.x == 0) {
-        if ((smem_u32(smem) & 1023u) != 0) record_error(a.status, ST_BAD_ARG, 0x20);
+        if ((smem_u32(smem) & 1023u) != 0) record_error(a.status, ST_BAD_ARG, 0x28);
         for (int i = 0; i < 2; i++) {
-            mbar_init(&res_full[i], 1); mbar_init(&res_empty[i], 1);
-            mbar_init(&acc_full[i], 1); mbar_init(&acc_empty[i], 16);
+            mbar_init(&f_full[i], 1); mbar_init(&f_empty[i], 1); mbar_init(&s_full[i], 1);
+            mbar_init(&acc_full[i], 1); mbar_init(&acc_empty[i], 4); mbar_init(&st_full[i], 4); mbar_init(&st_empty[i], 8);
         }
-        for (int i = 0; i < XSTAGES; i++) { mbar_init(&x_full[i], 1); mbar_init(&x_empty[i], 1); }
-        mbar_init(sdp_full, 1); mbar_init(sdp_empty, 16); mbar_init(pds_full, 16); mbar_init(pds_empty, 1);
+        for (int i = 0; i < X0STAGES; i++) { mbar_init(&x0_full[i], 1); mbar_init(&x0_empty[i], 1); }
+        mbar_init(x1_full, 1); mbar_init(x1_empty, 1); mbar_init(dp_full, 1); mbar_init(p_ready, 8); mbar_init(ds_ready, 8);
         *abort_flag = 0;
         mbar_fence_init();
-        tma_prefetch_desc(&tmQKV); tma_prefetch_desc(&tmDO);
+        tma_prefetch_desc(&tmQKV); tma_prefetch_desc(&tmDO); tma_prefetch_desc(&tmDQKV);
     }
-    if (warp == 1) { tmem_alloc(tmem_slot, BWD_TMEM_COLS); tmem_relinquish(); }
+    if (warp == 1) { tmem_alloc(tmem_slot, TMEM_COLS); tmem_relinquish(); }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
-    const uint32_t tS = tmem_base, tdP = tmem_base + 128, tAcc = tmem_base + 256;     // ACCBUF accumulator sets of 2 * HSP columns
+    const uint32_t tS = tmem_base, tdP = tmem_base + 128, tAcc0 = tmem_base + 256, tAcc1 = tmem_base + 384;
+    constexpr uint32_t S_BUF = DKV ? 0 : 384;           // distance of the second S buffer (the dK / dV pass has one)
 
-    // one 128-row tile = NC boxes of 64 channels
-    auto load_tile = [&](uint8_t* dst, const CUtensorMap* tm, uint64_t* bar, int slot, int row0, int b) {
-        #pragma unroll
-        for (int c = 0; c < NC; c++) tma_load_4d(dst + c * CHUNK_BYTES, tm, bar, c * 64, slot, row0, b);
-    };
+    Walk<DKV> wk;
+    wk.start(blockIdx.x, gridDim.x, a.BH, nt, a.NH);
 
     if (warp == 0) {
+        // ---------------------------------------------------------------- TMA producer
         if (lane == 0) {
-            int xst = 0; uint32_t xph = 0;                    // stream ring position of the next tile to load
-            int it = 0;
-            for (int w = blockIdx.x; w < total; w += gridDim.x, it++) {
-                int fixed, b, h, cnt; decode(w, fixed, b, h, cnt);
-                const int rb = it % RB;
-                if (!mbar_wait(&res_empty[rb], ((it / RB) & 1) ^ 1, abort_flag, a.status, 0x601)) break;
-                uint8_t* rdst = sRes + rb * PAIR_BYTES;
-                mbar_expect_tx(&res_full[rb], PAIR_BYTES);
-                if (DKV) {
-                    load_tile(rdst, &tmQKV, &res_full[rb], a.NH + h, fixed * BT, b);                   // K_j
-                    load_tile(rdst + TILE_BYTES, &tmQKV, &res_full[rb], 2 * a.NH + h, fixed * BT, b);  // V_j
-                } else {
-                    load_tile(rdst, &tmQKV, &res_full[rb], h, fixed * BT, b);                          // Q_i
-                    load_tile(rdst + TILE_BYTES, &tmDO, &res_full[rb], h, fixed * BT, b);              // dO_i
+            auto load = [&](uint8_t* dst, const CUtensorMap* tm, uint64_t* bar, int head, int tile, int b) {
+                tma_load_4d(dst, tm, bar, 0, head, tile * BT, b);
+                tma_load_4d(dst + CHUNK_BYTES, tm, bar, 64, head, tile * BT, b);
+            };
+            uint32_t t = 0;
+            int item = 0;
+            for (; wk.valid(); wk.next(), t++) {
+                if (wk.first()) {
+                    if (!mbar_wait_relaxed(&f_empty[0], (item & 1) ^ 1, abort_flag, a.status, 0x681)) break;
+                    mbar_expect_tx(&f_full[0], TILE_BYTES);
+                    load(sF, &tmQKV, &f_full[0], DKV ? a.NH + wk.h : wk.h, wk.f, wk.b);
+                    if (!mbar_wait_relaxed(&f_empty[1], (item & 1) ^ 1, abort_flag, a.status, 0x682)) break;
+                    mbar_expect_tx(&f_full[1], TILE_BYTES);
+                    load(sF + TILE_BYTES, DKV ? &tmQKV : &tmDO, &f_full[1], DKV ? 2 * a.NH + wk.h : wk.h, wk.f, wk.b);
+                    item++;
                 }
-                bool fail = false;
-                for (int n = 0; n < cnt; n++) {
-                    const int st = xst;
-                    if (!mbar_wait(&x_empty[st], xph ^ 1, abort_flag, a.status, 0x600)) { fail = true; break; }
-                    if (++xst == XSTAGES) { xst = 0; xph ^= 1; }
-                    uint8_t* dst = sStr + st * PAIR_BYTES;
-                    mbar_expect_tx(&x_full[st], PAIR_BYTES);
-                    if (DKV) {
-                        const int i = fixed + n;
-                        load_tile(dst, &tmQKV, &x_full[st], h, i * BT, b);                        // Q_i
-                        load_tile(dst + TILE_BYTES, &tmDO, &x_full[st], h, i * BT, b);            // dO_i
-                    } else {
-                        load_tile(dst, &tmQKV, &x_full[st], a.NH + h, n * BT, b);                 // K_j
-                        load_tile(dst + TILE_BYTES, &tmQKV, &x_full[st], 2 * a.NH + h, n * BT, b);// V_j
-                    }
-                }
-                if (fail) break;
+                const uint32_t st = t % X0STAGES;
+                if (!mbar_wait_relaxed(&x0_empty[st], ((t / X0STAGES) & 1) ^ 1, abort_flag, a.status, 0x680)) break;
+                mbar_expect_tx(&x0_full[st], TILE_BYTES);
+                load(sX0 + st * TILE_BYTES, &tmQKV, &x0_full[st], DKV ? wk.h : a.NH + wk.h, wk.x, wk.b);
+                if (!mbar_wait_relaxed(x1_empty, (t & 1) ^ 1, abort_flag, a.status, 0x683)) break;
+                mbar_expect_tx(x1_full, TILE_BYTES);
+                load(sX1, DKV ? &tmDO : &tmQKV, x1_full, DKV ? wk.h : 2 * a.NH + wk.h, wk.x, wk.b);
             }
         }
     } else if (warp == 1) {
-        // ---- issuer of the score products S = Q K^T and dP = dO V^T.  Tile g + 1 is issued as soon as the softmax threads hold
-        //      tile g in registers, so it runs underneath their exponentials.
-        if (lane == 0) {
-            constexpr uint32_t idesc_s = umma_idesc_bf16(BT, BT, 0, 0);
+        // ---------------------------------------------------------------- issuer: the whole warp in uniform control flow, one elected
+        // lane executes the tcgen05 instructions; wait results go through a warp vote so that the branches on them are uniform
+        if (wk.valid()) {
+            const bool leader = elect_one();
+#define WAIT_ALL(bar, parity, code) (__all_sync(0xffffffffu, mbar_wait_relaxed(bar, parity, abort_flag, a.status, code)) != 0)
+            constexpr uint32_t idesc_s = umma_idesc_bf16(BT, BT, 0, 0);                // both operands K-major
+            const uint32_t idesc_acc = umma_idesc_bf16(BT, 0, 0, 1) | ((uint32_t)(a.ks * 2) << 17);      // A from TMEM, B N-major, N = 16 ks
+            constexpr uint32_t TILE_UNITS = TILE_BYTES / 16, CHUNK_UNITS = CHUNK_BYTES / 16;
+            const uint64_t dF0 = umma_desc_sw128(smem_u32(sF), 16, 1024), dF1 = umma_desc_sw128(smem_u32(sF + TILE_BYTES), 16, 1024);
+            const uint64_t dX0 = umma_desc_sw128(smem_u32(sX0), 16, 1024), dX1 = umma_desc_sw128(smem_u32(sX1), 16, 1024);
+            const uint64_t nX0 = umma_desc_sw128(smem_u32(sX0), CHUNK_BYTES, 1024), nX1 = umma_desc_sw128(smem_u32(sX1), CHUNK_BYTES, 1024);
+            const int ks = a.ks;
+            // score product: 16 channels = 32 bytes = 2 address units per step, 4 steps per 64-channel chunk
+            auto issue_score = [&](uint32_t d, uint64_t f, uint64_t x, uint64_t* bar) {
+                if (leader) {
+                    #pragma unroll
+                    for (int kk = 0; kk < 8; kk++)
+                        if (kk < ks) umma_ss(d, f + (kk >> 2) * CHUNK_UNITS + (kk & 3) * 2, x + (kk >> 2) * CHUNK_UNITS + (kk & 3) * 2, idesc_s, kk > 0);
+                    umma_commit(bar);
+                }
+            };
+            // accumulating product: A = bf16 operand over its score tile (16 rows of B = 8 columns per step, each 64-row half at its own half
+            // of the tile), B = streamed tile N-major (16 rows = 2048 bytes = 128 units per step)
+            auto issue_acc = [&](uint32_t d, uint32_t ta, uint64_t x, uint32_t acc) {
+                if (leader) {
+                    #pragma unroll
+                    for (int kk = 0; kk < BT / 16; kk++) umma_ts(d, ta + (kk >> 2) * 64 + (kk & 3) * 8, x + 128 * kk, idesc_acc, acc | (kk > 0));
+                }
+            };
             uint32_t t = 0;
-            int st = 0; uint32_t ph = 0;                      // stream ring position of tile t
-            int it = 0;
-            bool ok = true;
-            for (int w = blockIdx.x; w < total && ok; w += gridDim.x, it++) {
-                int fixed, b, h, cnt; decode(w, fixed, b, h, cnt);
-                const int rb = it % RB;
-                ok = mbar_wait(&res_full[rb], (it / RB) & 1, abort_flag, a.status, 0x610);
-                for (int n = 0; n < cnt && ok; n++, t++) {
-                    ok = ok && mbar_wait(&x_full[st], ph, abort_flag, a.status, 0x612);
-                    if (t > 0) ok = ok && mbar_wait(sdp_empty, (t - 1) & 1, abort_flag, a.status, 0x613);
+            int item = 0;              // item of pair t
+            bool ok = WAIT_ALL(&f_full[0], 0, 0x690) && WAIT_ALL(&x0_full[0], 0, 0x691);
+            tc_fence_after();
+            if (ok) { issue_score(tS, dF0, dX0, &s_full[0]); if (leader && wk.last()) umma_commit(&f_empty[0]); }
+            ok = ok && WAIT_ALL(&f_full[1], 0, 0x692) && WAIT_ALL(x1_full, 0, 0x692);
+            tc_fence_after();
+            if (ok) {
+                issue_score(tdP, dF1, dX1, dp_full);
+                if (leader && !DKV) umma_commit(x1_empty);
+                if (leader && wk.last()) umma_commit(&f_empty[1]);
+            }
+            while (ok) {
+                Walk<DKV> nx = wk; nx.next();
+                const bool have_next = nx.valid();
+                const uint32_t st = t % X0STAGES, nst = (t + 1) % X0STAGES, sb = (t + 1) & 1;
+                const uint64_t xo = (uint64_t)(st * TILE_UNITS), nxo = (uint64_t)(nst * TILE_UNITS);
+                const int nitem = have_next && nx.first() ? item + 1 : item;
+                const uint32_t acc = wk.first() ? 0u : 1u;
+                if (DKV) {
+                    // ---- dV(t) += P^T dO_i
+                    ok = WAIT_ALL(p_ready, t & 1, 0x693);
+                    if (ok && wk.first() && item > 0) ok = WAIT_ALL(&acc_empty[0], (item - 1) & 1, 0x694);
                     if (!ok) break;
                     tc_fence_after();
-                    const uint32_t xs = smem_u32(sStr + st * PAIR_BYTES), rs = smem_u32(sRes + rb * PAIR_BYTES);
-                    const uint32_t q = DKV ? xs : rs, dO = (DKV ? xs : rs) + TILE_BYTES;
-                    const uint32_t k = DKV ? rs : xs, v = (DKV ? rs : xs) + TILE_BYTES;
-                    #pragma unroll
-                    for (int kk = 0; kk < HSP / 16; kk++) {      // 64-channel chunks are 16 KB apart, 16 channels = 32 bytes inside a chunk
-                        const uint32_t off = (kk >> 2) * CHUNK_BYTES + (kk & 3) * 32;
-                        umma_ss(tS, umma_desc_sw128(q + off, 16, 1024), umma_desc_sw128(k + off, 16, 1024), idesc_s, kk > 0);
+                    issue_acc(tAcc0, tS, nX1, acc);
+                    if (leader) {
+                        umma_commit(x1_empty);
+                        if (wk.last()) umma_commit(&acc_full[0]);
                     }
-                    #pragma unroll
-                    for (int kk = 0; kk < HSP / 16; kk++) {
-                        const uint32_t off = (kk >> 2) * CHUNK_BYTES + (kk & 3) * 32;
-                        umma_ss(tdP, umma_desc_sw128(dO + off, 16, 1024), umma_desc_sw128(v + off, 16, 1024), idesc_s, kk > 0);
-                    }
-                    umma_commit(sdp_full);
-                    if (n == cnt - 1) umma_commit(&res_empty[rb]);     // the resident pair is only read by these two products
-                    if (++st == XSTAGES) { st = 0; ph ^= 1; }
                 }
-            }
-        }
-    } else if (warp == BWD_THREADS / 32 - 1) {
-        // ---- issuer of the accumulating products (dV += P^T dO, dK += dS^T Q, or dQ += dS K).  A second issuing thread: a
-        //      tcgen05.mma costs its issuer about a hundred cycles whatever its shape, and the two streams of products depend on
-        //      different events, so two threads keep the tensor pipe fed where one could not.
-        if (lane == 0) {
-            constexpr uint32_t idesc_acc = DKV ? umma_idesc_bf16(BT, HSP, 1, 1) : umma_idesc_bf16(BT, HSP, 0, 1);
-            uint32_t t = 0;
-            int cst = 0;
-            int it = 0;
-            bool ok = true;
-            for (int w = blockIdx.x; w < total && ok; w += gridDim.x, it++) {
-                int fixed, b, h, cnt; decode(w, fixed, b, h, cnt);
-                const int ab = it % ACCBUF;
-                const uint32_t acc0 = tAcc + ab * (2 * HSP), acc1 = acc0 + HSP;
-                ok = mbar_wait(&acc_empty[ab], ((it / ACCBUF) & 1) ^ 1, abort_flag, a.status, 0x616);
-                for (int n = 0; n < cnt && ok; n++, t++) {
-                    ok = mbar_wait(pds_full, t & 1, abort_flag, a.status, 0x614);
+                // ---- S(t+1): into the tile P^T(t) was read from just before (dK / dV pass), or into the other S buffer, which the
+                //      softmax warps have read before they announced dS(t-1)
+                if (have_next) {
+                    if (nx.first()) ok = WAIT_ALL(&f_full[0], nitem & 1, 0x695);
+                    ok = ok && WAIT_ALL(&x0_full[nst], ((t + 1) / X0STAGES) & 1, 0x696);
                     if (!ok) break;
                     tc_fence_after();
-                    const uint32_t xs = smem_u32(sStr + cst * PAIR_BYTES);
-                    const uint32_t p = smem_u32(sP), ds = smem_u32(sdS);
-                    if (DKV) {
-                        // dV += P^T dO ; dK += dS^T Q : A is MN-major (two 64-wide groups 16 KB apart), K = 128 query rows;
-                        // B = dO / Q tile as an N-major operand (NC groups of 64 channels, 16 KB apart)
-                        #pragma unroll
-                        for (int kk = 0; kk < BT / 16; kk++)
-                            umma_ss(acc0, umma_desc_sw128(p + kk * 2048, BT * 128, 1024), umma_desc_sw128(xs + TILE_BYTES + kk * 2048, CHUNK_BYTES, 1024),
-                                    idesc_acc, (n > 0 || kk > 0));
-                        #pragma unroll
-                        for (int kk = 0; kk < BT / 16; kk++)
-                            umma_ss(acc1, umma_desc_sw128(ds + kk * 2048, BT * 128, 1024), umma_desc_sw128(xs + kk * 2048, CHUNK_BYTES, 1024),
-                                    idesc_acc, (n > 0 || kk > 0));
-                    } else {
-                        // dQ += dS K : A K-major (two 64-column chunks), B = K_j as an N-major operand
-                        #pragma unroll
-                        for (int kk = 0; kk < BT / 16; kk++)
-                            umma_ss(acc0, umma_desc_sw128(ds + (kk >> 2) * (BT * 128) + (kk & 3) * 32, 16, 1024),
-                                    umma_desc_sw128(xs + kk * 2048, CHUNK_BYTES, 1024), idesc_acc, (n > 0 || kk > 0));
-                    }
-                    umma_commit(&x_empty[cst]);
-                    umma_commit(pds_empty);
-                    if (n == cnt - 1) umma_commit(&acc_full[ab]);
-                    if (++cst == XSTAGES) cst = 0;
+                    issue_score(tS + sb * S_BUF, dF0, dX0 + nxo, &s_full[sb]);
+                    if (leader && nx.last()) umma_commit(&f_empty[0]);
                 }
+                // ---- dK(t) += dS^T Q_i   or   dQ(t) += dS K_j
+                ok = WAIT_ALL(ds_ready, t & 1, 0x697);
+                if (ok && wk.first() && item > 0) ok = WAIT_ALL(&acc_empty[DKV ? 1 : 0], (item - 1) & 1, 0x698);
+                if (!ok) break;
+                tc_fence_after();
+                issue_acc(DKV ? tAcc1 : tAcc0, tdP, nX0 + xo, acc);
+                if (leader) {
+                    umma_commit(&x0_empty[st]);
+                    if (wk.last()) umma_commit(&acc_full[DKV ? 1 : 0]);
+                }
+                // ---- dP(t+1): after the product above in program order, so it cannot overwrite dS(t) early
+                if (have_next) {
+                    if (nx.first()) ok = WAIT_ALL(&f_full[1], nitem & 1, 0x699);
+                    ok = ok && WAIT_ALL(x1_full, (t + 1) & 1, 0x69a);
+                    if (!ok) break;
+                    tc_fence_after();
+                    issue_score(tdP, dF1, dX1, dp_full);
+                    if (leader) {
+                        if (!DKV) umma_commit(x1_empty);
+                        if (nx.last()) umma_commit(&f_empty[1]);
+                    }
+                }
+                if (!have_next) break;
+                wk = nx; item = nitem; t++;
             }
+#undef WAIT_ALL
         }
-    } else {
-        // softmax / epilogue: thread = one row x one 32-column quarter of the 128 x 128 tile.
-        // These warps never leave their loops early: after an abandoned wait every later wait returns at once.
+    } else if (warp >= 4 && warp < 12) {
+        // ---------------------------------------------------------------- softmax: thread = row r of the score tile x column half hf
         const int q = warp & 3;                        // TMEM lane quarter
-        const int cq = (warp - 2) >> 2;                // column quarter handled by this thread
-        const int r = q * 32 + lane;                   // row of the tile (a query row in S / dP)
+        const int hf = (warp - 4) >> 2;
+        const int r = q * 32 + lane;
         const uint32_t lane_off = (uint32_t)(q * 32) << 16;
         const float log2e = 1.4426950408889634f;
         bool ok = true;
         uint32_t t = 0;
-        int it = 0;
-        for (int w = blockIdx.x; w < total; w += gridDim.x, it++) {
-            int fixed, b, h, cnt; decode(w, fixed, b, h, cnt);
-            const size_t stat_base = ((size_t)b * a.NH + h) * a.T;
-            float lse_l2 = 0.f, dlt_s = 0.f;           // LSE in log2 units; delta pre-multiplied by the softmax scale
-            bool row_ok;
-            {
-                const int t0 = fixed * BT + r;
-                row_ok = t0 < a.T;
-                if (row_ok) { lse_l2 = a.lse[stat_base + t0] * log2e; dlt_s = a.delta[stat_base + t0] * a.scale; }
+        float row_lse = 0.f, row_delta = 0.f;          // dQ pass: statistics of this thread's query row
+        for (; wk.valid(); wk.next(), t++) {
+            const bool diag = wk.x == wk.f;
+            const float* stat = sStat + (t & 1) * (2 * BT) + hf * 64;       // dK / dV pass: lse * log2(e) of this half's queries; delta * scale 128 floats further
+            if (!DKV && wk.first()) {
+                const int tq = wk.f * BT + r;
+                row_lse = INFINITY; row_delta = 0.f;
+                if (tq < a.T) { row_lse = a.lse[(size_t)wk.bh * a.T + tq] * log2e; row_delta = a.delta[(size_t)wk.bh * a.T + tq] * a.scale; }
             }
-            for (int n = 0; n < cnt; n++, t++) {
-                const int qi = DKV ? fixed + n : fixed;    // query tile index
-                const int kj = DKV ? fixed : n;            // key tile index
-                // prefetch the next query tile's statistics (only the dK/dV kernel changes rows between tiles)
-                float nxt_lse = 0.f, nxt_dlt = 0.f; bool nxt_ok = row_ok;
-                const bool fetch_next = DKV && n + 1 < cnt;
-                if (fetch_next) {
-                    const int tn = (qi + 1) * BT + r;
-                    nxt_ok = tn < a.T;
-                    if (nxt_ok) { nxt_lse = a.lse[stat_base + tn]; nxt_dlt = a.delta[stat_base + tn]; } else { nxt_lse = 0.f; nxt_dlt = 0.f; }     // raw: converted below, after the loads had a whole tile to land
-                }
-                ok = mbar_wait(sdp_full, t & 1, abort_flag, a.status, 0x620) && ok;
-                tc_fence_after();
-                uint32_t sv[32], dv[32];
-                tmem_ld32(tS + lane_off + cq * 32, sv);
-                tmem_ld32(tdP + lane_off + cq * 32, dv);
+            ok = mbar_wait(&s_full[t & 1], (t >> 1) & 1, abort_flag, a.status, 0x6a0) && ok;
+            if (DKV) ok = mbar_wait(&st_full[t & 1], (t >> 1) & 1, abort_flag, a.status, 0x6a1) && ok;
+            tc_fence_after();
+            // ---- P = exp2(S * scale * log2(e) - LSE * log2(e)), causal, in two passes of 32 columns (with all 64 scores next to the 64
+            //      results the register file is so full that every exponential waits for its predecessor)
+            const uint32_t tSt = tS + (DKV ? 0u : (t & 1) * S_BUF) + lane_off + hf * 64;
+            float p[64];
+            #pragma unroll
+            for (int h2 = 0; h2 < 2; h2++) {
+                uint32_t sv[32];
+                tmem_ld32(tSt + h2 * 32, sv);
                 tmem_ld_wait();
+                #pragma unroll
+                for (int e4 = 0; e4 < 8; e4++) {
+                    float4 l4 = make_float4(row_lse, row_lse, row_lse, row_lse);
+                    if (DKV) l4 = *reinterpret_cast<const float4*>(stat + h2 * 32 + e4 * 4);
+                    p[h2 * 32 + e4 * 4 + 0] = ex2_fast(fmaf(__uint_as_float(sv[e4 * 4 + 0]), a.scale_log2e, -l4.x));
+                    p[h2 * 32 + e4 * 4 + 1] = ex2_fast(fmaf(__uint_as_float(sv[e4 * 4 + 1]), a.scale_log2e, -l4.y));
+                    p[h2 * 32 + e4 * 4 + 2] = ex2_fast(fmaf(__uint_as_float(sv[e4 * 4 + 2]), a.scale_log2e, -l4.z));
+                    p[h2 * 32 + e4 * 4 + 3] = ex2_fast(fmaf(__uint_as_float(sv[e4 * 4 + 3]), a.scale_log2e, -l4.w));
+                }
+            }
+            // only the diagonal tile needs a mask (query >= key).  Rows and columns past T need none beyond it: queries past T have
+            // LSE = +inf, and a key past T is seen by no query before T.
+            if (diag) {
+                #pragma unroll
+                for (int e = 0; e < 64; e++) if (DKV ? hf * 64 + e < r : hf * 64 + e > r) p[e] = 0.f;
+            }
+            if (DKV) {
+                uint32_t pk[32];
+                #pragma unroll
+                for (int e = 0; e < 32; e++) pk[e] = pack_bf16x2(p[2 * e], p[2 * e + 1]);
+                tmem_st16(tSt, pk);
+                tmem_st16(tSt + 16, pk + 16);
+                tmem_st_wait();
                 tc_fence_before();
                 __syncwarp();
-                if (lane == 0) mbar_arrive(sdp_empty);      // S / dP may be overwritten by the next tile
-                uint32_t pp[16], dd[16];
-                if (qi == kj || !row_ok) {
-                    // diagonal tile (or rows past the end of the sequence): mask above the diagonal
-                    #pragma unroll
-                    for (int e = 0; e < 32; e += 2) {
-                        const int c0 = cq * 32 + e;
-                        float p0 = ex2_fast(fmaf(__uint_as_float(sv[e]), a.scale_log2e, -lse_l2));
-                        float p1 = ex2_fast(fmaf(__uint_as_float(sv[e + 1]), a.scale_log2e, -lse_l2));
-                        if (!row_ok || c0 > r) p0 = 0.f;
-                        if (!row_ok || c0 + 1 > r) p1 = 0.f;
-                        const float d0 = p0 * fmaf(__uint_as_float(dv[e]), a.scale, -dlt_s);
-                        const float d1 = p1 * fmaf(__uint_as_float(dv[e + 1]), a.scale, -dlt_s);
-                        pp[e >> 1] = pack_bf16x2(p0, p1);
-                        dd[e >> 1] = pack_bf16x2(d0, d1);
-                    }
-                } else {
-                    #pragma unroll
-                    for (int e = 0; e < 32; e += 2) {
-                        const float p0 = ex2_fast(fmaf(__uint_as_float(sv[e]), a.scale_log2e, -lse_l2));
-                        const float p1 = ex2_fast(fmaf(__uint_as_float(sv[e + 1]), a.scale_log2e, -lse_l2));
-                        const float d0 = p0 * fmaf(__uint_as_float(dv[e]), a.scale, -dlt_s);
-                        const float d1 = p1 * fmaf(__uint_as_float(dv[e + 1]), a.scale, -dlt_s);
-                        pp[e >> 1] = pack_bf16x2(p0, p1);
-                        dd[e >> 1] = pack_bf16x2(d0, d1);
-                    }
-                }
-                if (t > 0) ok = mbar_wait(pds_empty, (t - 1) & 1, abort_flag, a.status, 0x621) && ok;   // previous tile's MMAs have read P / dS
-                // 64-column chunk (cq >> 1), 16-byte units (cq & 1) * 4 .. +3 of this row, 128-byte swizzle
-                uint8_t* prow = sP + (cq >> 1) * (BT * 128) + r * 128;
-                uint8_t* drow = sdS + (cq >> 1) * (BT * 128) + r * 128;
-                #pragma unroll
-                for (int u = 0; u < 4; u++) {
-                    const int pos = ((((cq & 1) * 4) + u) ^ (r & 7)) * 16;
-                    if (DKV) *reinterpret_cast<uint4*>(prow + pos) = make_uint4(pp[u * 4], pp[u * 4 + 1], pp[u * 4 + 2], pp[u * 4 + 3]);
-                    *reinterpret_cast<uint4*>(drow + pos) = make_uint4(dd[u * 4], dd[u * 4 + 1], dd[u * 4 + 2], dd[u * 4 + 3]);
-                }
-                fence_async_smem();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(pds_full);
-                if (fetch_next) { lse_l2 = nxt_lse * log2e; dlt_s = nxt_dlt * a.scale; row_ok = nxt_ok; }
+                if (lane == 0) mbar_arrive(p_ready);
             }
-            // ---- item epilogue: accumulators -> global; the issuing warps are already working on the next item
-            const int ab = it % ACCBUF;
-            ok = mbar_wait(&acc_full[ab], (it / ACCBUF) & 1, abort_flag, a.status, 0x622) && ok;
+            // ---- dS = P * (dP * scale - delta * scale), in four chunks of 16 columns: bf16 inside this half's own columns of the dP tile
+            //      (a chunk's bf16 lands on fp32 columns that are already in registers)
+            ok = mbar_wait(dp_full, t & 1, abort_flag, a.status, 0x6a3) && ok;
             tc_fence_after();
-            uint32_t v0[16 * NC], v1[16 * NC];
             #pragma unroll
-            for (int c = 0; c < NC; c++) {
-                tmem_ld16(tAcc + ab * (2 * HSP) + c * 64 + lane_off + cq * 16, v0 + c * 16);
-                if (DKV) tmem_ld16(tAcc + ab * (2 * HSP) + HSP + c * 64 + lane_off + cq * 16, v1 + c * 16);
+            for (int c = 0; c < 4; c++) {
+                uint32_t dv[16];
+                tmem_ld16(tdP + lane_off + hf * 64 + c * 16, dv);
+                tmem_ld_wait();
+                uint32_t dd[8];
+                #pragma unroll
+                for (int e4 = 0; e4 < 4; e4++) {
+                    float4 d4 = make_float4(row_delta, row_delta, row_delta, row_delta);
+                    if (DKV) d4 = *reinterpret_cast<const float4*>(stat + BT + c * 16 + e4 * 4);
+                    const float dl[4] = {d4.x, d4.y, d4.z, d4.w};
+                    float ds[4];
+                    #pragma unroll
+                    for (int k = 0; k < 4; k++) ds[k] = p[c * 16 + e4 * 4 + k] * fmaf(__uint_as_float(dv[e4 * 4 + k]), a.scale, -dl[k]);
+                    dd[e4 * 2] = pack_bf16x2(ds[0], ds[1]);
+                    dd[e4 * 2 + 1] = pack_bf16x2(ds[2], ds[3]);
+                }
+                tmem_st8(tdP + lane_off + hf * 64 + c * 8, dd);
             }
-            tmem_ld_wait();
+            tmem_st_wait();
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(&acc_empty[ab]);
-            const int trow = fixed * BT + r;
-            if (trow < a.T && ok) {
-                // DKV: acc0 = dV (slot 2), acc1 = dK (slot 1); else acc0 = dQ (slot 0)
-                bf16* dst0 = a.dqkv + (((size_t)b * a.T + trow) * 3 + (DKV ? 2 : 0)) * a.NH * a.hs + (size_t)h * a.hs;
-                bf16* dst1 = a.dqkv + (((size_t)b * a.T + trow) * 3 + 1) * a.NH * a.hs + (size_t)h * a.hs;
-                #pragma unroll
-                for (int c = 0; c < NC; c++) {
+            if (lane == 0) { mbar_arrive(ds_ready); if (DKV) mbar_arrive(&st_empty[t & 1]); }
+        }
+    } else if (warp >= 12) {
+        // ---------------------------------------------------------------- drain warps (128 threads): thread = row rr of a tile
+        const int q = warp & 3;
+        const int rr = q * 32 + lane;
+        const uint32_t lane_off = (uint32_t)(q * 32) << 16;
+        const float log2e = 1.4426950408889634f;
+        const bool issuer = warp == 12 && lane == 0;
+        bool ok = true;
+        bool staged = false;
+        uint32_t t = 0;
+        int item = 0;
+        // dK / dV pass: statistics of query rr of a pair's query tile -> table (tt & 1): LSE in log2 units, delta times the scale;
+        // queries past the end of the sequence get LSE = +inf, so that their P^T column is zero
+        auto put_stats = [&](const Walk<DKV>& pr, uint32_t tt) {
+            const int tq = pr.x * BT + rr;
+            float l = INFINITY, d = 0.f;
+            if (tq < a.T) { l = a.lse[(size_t)pr.bh * a.T + tq] * log2e; d = a.delta[(size_t)pr.bh * a.T + tq] * a.scale; }
+            ok = mbar_wait_relaxed(&st_empty[tt & 1], ((tt >> 1) & 1) ^ 1, abort_flag, a.status, 0x6b0) && ok;
+            float* tab = sStat + (tt & 1) * (2 * BT);
+            tab[rr] = l; tab[BT + rr] = d;
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&st_full[tt & 1]);
+        };
+        // accumulator tile -> bf16 in the layout of two 128-byte-swizzled TMA boxes -> bulk stores (rows past T and channels past the
+        // head are clipped by TMA); warps writing rows themselves would touch 32 cache lines per instruction
+        auto drain = [&](int which, uint32_t tAcc, int head, int f, int b) {
+            ok = mbar_wait_relaxed(&acc_full[which], item & 1, abort_flag, a.status, 0x6b2) && ok;
+            tc_fence_after();
+            if (staged) { if (issuer) tma_store_wait_read<0>(); asm volatile("bar.sync 1, 128;" ::: "memory"); }
+            #pragma unroll
+            for (int c = 0; c < 4; c++) {
+                if (c * 2 < a.ks) {
+                    uint32_t v[32];
+                    tmem_ld32(tAcc + lane_off + c * 32, v);
+                    tmem_ld_wait();
+                    uint8_t* orow = sOut + (c >> 1) * CHUNK_BYTES + rr * 128;
                     #pragma unroll
-                    for (int e = 0; e < 16; e += 8) {
-                        const int col = c * 64 + cq * 16 + e;
-                        if (col < a.hs) {
-                            const uint32_t* x0 = v0 + c * 16 + e;
-                            uint4 o;
-                            o.x = pack_bf16x2(__uint_as_float(x0[0]), __uint_as_float(x0[1])); o.y = pack_bf16x2(__uint_as_float(x0[2]), __uint_as_float(x0[3]));
-                            o.z = pack_bf16x2(__uint_as_float(x0[4]), __uint_as_float(x0[5])); o.w = pack_bf16x2(__uint_as_float(x0[6]), __uint_as_float(x0[7]));
-                            *reinterpret_cast<uint4*>(dst0 + col) = o;
-                            if (DKV) {
-                                const uint32_t* x1 = v1 + c * 16 + e;
-                                o.x = pack_bf16x2(__uint_as_float(x1[0]), __uint_as_float(x1[1])); o.y = pack_bf16x2(__uint_as_float(x1[2]), __uint_as_float(x1[3]));
-                                o.z = pack_bf16x2(__uint_as_float(x1[4]), __uint_as_float(x1[5])); o.w = pack_bf16x2(__uint_as_float(x1[6]), __uint_as_float(x1[7]));
-                                *reinterpret_cast<uint4*>(dst1 + col) = o;
-                            }
-                        }
+                    for (int u = 0; u < 4; u++) {
+                        uint4 o;
+                        o.x = pack_bf16x2(__uint_as_float(v[8 * u]), __uint_as_float(v[8 * u + 1]));
+                        o.y = pack_bf16x2(__uint_as_float(v[8 * u + 2]), __uint_as_float(v[8 * u + 3]));
+                        o.z = pack_bf16x2(__uint_as_float(v[8 * u + 4]), __uint_as_float(v[8 * u + 5]));
+                        o.w = pack_bf16x2(__uint_as_float(v[8 * u + 6]), __uint_as_float(v[8 * u + 7]));
+                        *reinterpret_cast<uint4*>(orow + ((((c & 1) * 4 + u) ^ (rr & 7)) * 16)) = o;
                     }
                 }
             }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&acc_empty[which]);
+            fence_async_smem();
+            asm volatile("bar.sync 1, 128;" ::: "memory");
+            if (issuer && ok) {
+                tma_store_4d(&tmDQKV, sOut, 0, head, f * BT, b);
+                tma_store_4d(&tmDQKV, sOut + CHUNK_BYTES, 64, head, f * BT, b);
+                tma_store_commit();
+            }
+            staged = true;
+        };
+        if (DKV && wk.valid()) put_stats(wk, 0);
+        for (; wk.valid(); t++) {
+            const int b = wk.b, h = wk.h, f = wk.f;
+            const bool last = wk.last();
+            wk.next();
+            if (DKV && wk.valid()) put_stats(wk, t + 1);        // the next pair's table, one pair ahead
+            if (last) {
+                drain(0, tAcc0, DKV ? 2 * a.NH + h : h, f, b);
+                if (DKV) drain(1, tAcc1, a.NH + h, f, b);
+                item++;
+            }
         }
+        if (issuer) tma_store_wait<0>();
     }
     tc_fence_before();
     __syncthreads();
@@ -400,25 +476,10 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
         while (clock64() - t0 < 2000000ll) { __nanosleep(1000); }
         __syncthreads();
     }
-    if (warp == 1) tmem_dealloc(tmem_base, BWD_TMEM_COLS);
+    if (warp == 1) tmem_dealloc(tmem_base, TMEM_COLS);
 }
 
 }  // namespace
-
-template <int NC>
-int launch_bwd(const CUtensorMap& tmQKV, const CUtensorMap& tmDO, const BwdArgs& a, int grid, cudaStream_t stream) {
-    static bool configured = false;
-    if (!configured) {
-        CUDA_CHECK(cudaFuncSetAttribute(attn_bwd_kernel<true, NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, BwdCfg<NC>::SMEM));
-        CUDA_CHECK(cudaFuncSetAttribute(attn_bwd_kernel<false, NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, BwdCfg<NC>::SMEM));
-        configured = true;
-    }
-    attn_bwd_kernel<true, NC><<<grid, BWD_THREADS, BwdCfg<NC>::SMEM, stream>>>(tmQKV, tmDO, a);
-    CUDA_CHECK(cudaGetLastError());
-    attn_bwd_kernel<false, NC><<<grid, BWD_THREADS, BwdCfg<NC>::SMEM, stream>>>(tmQKV, tmDO, a);
-    CUDA_CHECK(cudaGetLastError());
-    return 0;
-}
 
 // delta[b,h,t] = sum_d O[b,t,h,d] * dO[b,t,h,d] (shared with the single-pass kernel of attention_bwd1.cu)
 int llmc_attention_delta(float* delta, const bf16* out, const bf16* dout, int B, int T, int NH, int hs, cudaStream_t stream) {
@@ -428,12 +489,12 @@ int llmc_attention_delta(float* delta, const bf16* out, const bf16* dout, int B,
     return 0;
 }
 
-// dqkv (B,T,3,NH,HS) = gradient of causal attention; delta: scratch of B*NH*T floats.  Head sizes: multiples of 8, 64..128.
+// dqkv (B,T,3,NH,HS) = gradient of causal attention; delta: scratch of B*NH*T floats.  Head sizes: multiples of 8, 72..128.
 // The entry point llmc_attention_bwd (attention_bwd1.cu) sends every head size but 64 here.
 int llmc_attention_bwd_two_pass(bf16* dqkv, float* delta, const bf16* dout, const bf16* qkv, const bf16* out, const float* lse,
                                 int B, int T, int NH, int hs, cudaStream_t stream) {
-    if (hs < 64 || hs > 128 || (hs % 8)) { fprintf(stderr, "[llmc_b200] attention backward: head size %d not supported (multiples of 8 from 64 to 128)\n", hs); return -1; }
-    CUtensorMap tmQKV, tmDO;
+    if (hs <= 64 || hs > 128 || (hs % 8)) { fprintf(stderr, "[llmc_b200] attention backward: head size %d not supported (multiples of 8 from 64 to 128)\n", hs); return -1; }
+    CUtensorMap tmQKV, tmDO, tmDQKV;
     int rc = llmc_attn_qkv_map(&tmQKV, qkv, B, T, NH, hs);
     if (rc) return rc;
     {
@@ -442,14 +503,26 @@ int llmc_attention_bwd_two_pass(bf16* dqkv, float* delta, const bf16* dout, cons
         uint32_t box[4] = {64, 1, 128, 1};
         if ((rc = llmc_get_tensormap(&tmDO, dout, 2, 4, dims, strides, box, 3))) return rc;
     }
+    if ((rc = llmc_attn_qkv_map(&tmDQKV, dqkv, B, T, NH, hs))) return rc;
     if ((rc = llmc_attention_delta(delta, out, dout, B, T, NH, hs, stream))) return rc;
-    BwdArgs a;
-    a.dqkv = dqkv; a.lse = lse; a.delta = delta; a.B = B; a.T = T; a.NH = NH; a.hs = hs;
+    Args a;
+    a.lse = lse; a.delta = delta; a.T = T; a.NH = NH; a.BH = B * NH;
+    a.ks = CEIL_DIV(hs, 16);
     a.scale = 1.0f / sqrtf((float)hs);
     a.scale_log2e = a.scale * 1.4426950408889634f;
     a.status = llmc_status_ptr();
     const int nt = CEIL_DIV(T, BT);
     int sms = llmc_device_sm_count(); if (sms <= 0) sms = 148;
     const int grid = B * NH * nt < sms ? B * NH * nt : sms;
-    return hs <= 64 ? launch_bwd<1>(tmQKV, tmDO, a, grid, stream) : launch_bwd<2>(tmQKV, tmDO, a, grid, stream);
+    static bool configured = false;
+    if (!configured) {
+        CUDA_CHECK(cudaFuncSetAttribute(attn_bwd_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM));
+        CUDA_CHECK(cudaFuncSetAttribute(attn_bwd_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM));
+        configured = true;
+    }
+    attn_bwd_kernel<true><<<grid, THREADS, SMEM, stream>>>(tmQKV, tmDO, tmDQKV, a);
+    CUDA_CHECK(cudaGetLastError());
+    attn_bwd_kernel<false><<<grid, THREADS, SMEM, stream>>>(tmQKV, tmDO, tmDQKV, a);
+    CUDA_CHECK(cudaGetLastError());
+    return 0;
 }
