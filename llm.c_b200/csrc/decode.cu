@@ -1,6 +1,6 @@
 // Incremental decoding with a key / value cache (the inference path of the reference's LLaMA script,
 // train_llama3.py:167-190 and :476-556: keys and values of earlier positions are kept, only the new tokens run through
-// the network).  Two kernels; both are memory-bound and small, so they use plain loads, no tensor cores:
+// the network).  The kernels are memory-bound and small; the products of the step are in stream_gemm.cu:
 //
 //   rope_cache      raw (N, (NH + 2 NKV) * HS), N = B * Tq new tokens at positions start_pos .. start_pos + Tq - 1
 //                     -> q (N, NH, HS) rotated queries
@@ -12,6 +12,7 @@
 // replayed with the position advanced on the device.  A device position that would leave the cache or the rotary table makes
 // the kernel record ST_BAD_ARG in the status word and return without touching memory.
 #include "common.cuh"
+#include "pdl.cuh"
 
 namespace {
 
@@ -32,6 +33,8 @@ __global__ void __launch_bounds__(256)
 rope_cache_kernel(bf16* __restrict__ q, bf16* __restrict__ kcache, bf16* __restrict__ vcache, const bf16* __restrict__ raw,
                   const float2* __restrict__ freqs, long long N, int Tq, int Tmax, int start_pos, int NH, int NKV, int HS,
                   const int* __restrict__ pos_ptr, int freqs_len, unsigned int* status) {
+    pdl_wait();
+    pdl_trigger();
     if (pos_ptr) {
         start_pos = *pos_ptr;
         if (start_pos < 0 || start_pos + Tq > Tmax || start_pos + Tq > freqs_len) {
@@ -151,23 +154,26 @@ cached_attention_kernel(bf16* __restrict__ out, const bf16* __restrict__ q, cons
 
 // ---------------------------------------------------------------------------------------------------------------
 // Decoding attention, fast path (head width 64 or 128, at most 8 query rows per cached head: the decoding step itself).
-// The general kernel above gives a thread a whole key row straight from global memory (32 rows per load instruction, one
-// cache line each) and runs once per QUERY head, so grouped queries re-read their keys; it is bound by instruction issue at
-// a fifth of the memory rate.  Here
-//   * a CTA serves ONE cached head of one batch row for ALL its R = (NH / NKV) * Tq query rows and a slice of the keys
-//     (grid: key slices x cached heads x batch rows, sized to fill the GPU at any batch size);
-//   * each of its 4 warps walks tiles of 32 keys.  The K tile comes in with cp.async (16 lanes read one 256-byte row:
-//     coalesced), double buffered, into shared memory with the 16-byte chunks of row j XOR-swizzled by j & 7; then lane j
-//     owns key j and reads its row without bank conflicts: whole dot products per lane, no butterflies, one exponential
-//     per key and query row;
-//   * the probabilities go through a small shared tile; for the weighted sum of V every lane owns HS / 32 channels and the
-//     V rows are read from global memory as the 32 lanes' contiguous 8- or 4-byte pieces, eight rows in flight;
-//   * running (max, sum, accumulator) per warp, merged over the warps, then over the key slices in a small fp32 workspace
-//     that a second kernel folds in slice order (deterministic).
+// Reading the cache once is all the work there is, so
+//   * a CTA serves ONE cached head of one batch row for ALL its (NH / NKV) * Tq query rows and a slice of the keys;
+//   * each of its 4 warps walks tiles of 16 keys whose K and V rows arrive by cp.async through a ring of its own (two tiles in
+//     flight per warp, 16-byte chunks of row j XOR-swizzled by j & 7), so that about 100 KB per SM are on the way at any time;
+//   * the products run on warp-level MMAs: S = Q K^T with the query rows as the 16-row operand (8 of them used), O += P V with the
+//     probabilities taken from the score registers.  fp32 FMAs with one key per lane (the kernel before this one) were bound by the
+//     shared-memory reads of the queries and the probabilities (187 us for the case below).
+//   * probabilities keep about 16 bits: P = hi + lo, both bf16, hi in rows 0..7 of the MMA operand and lo in the otherwise idle rows
+//     8..15, and the two halves of the accumulator are added at the end.  Queries, keys and values are bf16 as stored.
+//   * running (max, sum, accumulator) per warp, merged over the warps through shared memory, then over the key slices in slice
+//     order: through distributed shared memory when the slices of a head form one cluster (at most 8), else through a small fp32
+//     workspace and a second kernel.
+// 32 rows at position 4095, 32 heads on 8 cached heads of 128: 109 us (4.9 TB/s); 4 rows at position 160: 10 us against 25.
 constexpr int CA_WARPS = 4;
 constexpr int CA_THREADS = CA_WARPS * 32;
 constexpr int CA_MAX_R = 8;
-constexpr int CA_MIN_KEYS = 256;      // a slice is at least this long (unless the cache is shorter)
+constexpr int CA_TILE = 16;           // keys per tile of a warp
+constexpr int CA_STAGES = 3;
+constexpr int CA_MIN_KEYS = 128;      // a slice is at least this long (unless the cache is shorter)
+constexpr int CA_MAX_CLUSTER = 8;
 constexpr float CA_LOG2E = 1.4426950408889634f;
 
 DEVINL void cp_async16(void* smem_dst, const void* gsrc) {
@@ -175,278 +181,241 @@ DEVINL void cp_async16(void* smem_dst, const void* gsrc) {
 }
 DEVINL void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N> DEVINL void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
-
-template <int HS_, int R> constexpr int ca_smem_bytes() {
-    return R * HS_ * 4 + CA_WARPS * (2 * 32 * HS_ * 2 + 32 * R * 4);
+DEVINL void ldmatrix4(uint32_t (&r)[4], uint32_t addr) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+DEVINL void ldmatrix4_trans(uint32_t (&r)[4], uint32_t addr) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+DEVINL void mma_16x8x16(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+                 : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+// float4 of this CTA's shared memory at byte address `addr`, in CTA `rank` of the cluster
+DEVINL float ld_peer(uint32_t addr, uint32_t rank) {
+    uint32_t ra; float v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(addr), "r"(rank));
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(ra) : "memory");
+    return v;
+}
+DEVINL void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
-template <int HS_, int R>
+template <int HS_> __host__ __device__ constexpr int ca_ring_bytes() { return CA_STAGES * 2 * CA_TILE * HS_ * 2; }                     // of one warp
+template <int HS_> __host__ __device__ constexpr int ca_part_floats() { return CA_MAX_R * (HS_ + 2); }                                 // acc, max, sum of 8 rows
+template <int HS_> __host__ __device__ constexpr int ca_smem_bytes() { return CA_WARPS * ca_ring_bytes<HS_>() + ca_part_floats<HS_>() * 4; }
+
+// CLUSTER: the gridDim.x slices of a head are one cluster and `out` receives the result; otherwise the slice's partial goes to ws.
+template <int HS_, bool CLUSTER>
 __global__ void __launch_bounds__(CA_THREADS)
-cached_attention_split_kernel(float* __restrict__ ws, const bf16* __restrict__ q, const bf16* __restrict__ kcache,
+cached_attention_split_kernel(bf16* __restrict__ out, float* __restrict__ ws, const bf16* __restrict__ q, const bf16* __restrict__ kcache,
                               const bf16* __restrict__ vcache, int Tq, int Tmax, int start_pos, int NH, int NKV, float scale,
                               const int* __restrict__ pos_ptr, unsigned int* status, int keys_per_slice, int rows) {
+    pdl_wait();
+    pdl_trigger();
     if (pos_ptr) {
         start_pos = *pos_ptr;
-        if (start_pos < 0 || start_pos + Tq > Tmax) {
+        if (start_pos < 0 || start_pos + Tq > Tmax) {           // the same for every CTA of a cluster
             if (threadIdx.x == 0 && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0) record_error(status, ST_BAD_ARG, 0x32);
             return;
         }
     }
     constexpr int ROWB = HS_ * 2;              // bytes of a key row
     constexpr int CHUNKS = HS_ / 8;            // 16-byte chunks of a row
-    constexpr int CPL = HS_ / 32;              // channels of V and of the output per lane
+    constexpr int KS = HS_ / 16;               // 16-channel steps
+    constexpr int STAGE = 2 * CA_TILE * ROWB;  // K tile, V tile
+    constexpr int PART = ca_part_floats<HS_>();
     extern __shared__ __align__(16) uint8_t ca_smem[];
-    float* qs = reinterpret_cast<float*>(ca_smem);                                   // [R][HS_], scaled by scale * log2(e)
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    uint8_t* kbuf = ca_smem + R * HS_ * 4 + warp * (2 * 32 * ROWB + 32 * R * 4);      // [2][32 rows][ROWB], swizzled
-    float* ptile = reinterpret_cast<float*>(kbuf + 2 * 32 * ROWB);                   // [32 keys][R]
+    const int gq = lane >> 2, tq4 = lane & 3;                  // MMA fragment coordinates: row gq, column pair tq4
+    uint8_t* ring = ca_smem + warp * ca_ring_bytes<HS_>();
+    float* part = reinterpret_cast<float*>(ca_smem + CA_WARPS * ca_ring_bytes<HS_>());      // this CTA's merged partial: [8][HS_], max[8], sum[8]
     const int slice = blockIdx.x, g = blockIdx.y, nslices = gridDim.x;
     const long long b = blockIdx.z;
     const int G = NH / NKV;
     const int nkeys = start_pos + Tq;                          // keys visible to the last new token
-    const int k0 = slice * keys_per_slice, k1 = min(nkeys, k0 + keys_per_slice);
+    const int k0 = min(nkeys, slice * keys_per_slice), k1 = min(nkeys, k0 + keys_per_slice);
 
-    // query rows: r -> token r / G, head g * G + r % G; rows past `rows` repeat row 0 and are dropped at the end
-    for (int i = threadIdx.x; i < R * HS_; i += CA_THREADS) {
-        const int r = i / HS_, c = i - r * HS_;
-        const int rr = r < rows ? r : 0;
-        const int t = rr / G, hq = g * G + rr % G;
-        qs[i] = __bfloat162float(q[((b * Tq + t) * NH + hq) * HS_ + c]) * (scale * CA_LOG2E);
-    }
-    int limit[R];                                              // keys [0, limit) are visible to row r
-    #pragma unroll
-    for (int r = 0; r < R; r++) limit[r] = min(k1, start_pos + (r < rows ? r : 0) / G + 1);
-    __syncthreads();
-
-    float m[R], l[R], acc[R][CPL];
-    #pragma unroll
-    for (int r = 0; r < R; r++) {
-        m[r] = -INFINITY; l[r] = 0.f;
-        #pragma unroll
-        for (int c = 0; c < CPL; c++) acc[r][c] = 0.f;
-    }
     const long long row_stride = (long long)NKV * HS_;
     const bf16* kbase = kcache + ((b * Tmax) * NKV + g) * HS_;
-    const bf16* vbase = vcache + ((b * Tmax) * NKV + g) * HS_ + lane * CPL;
-    // copy of the K tile that starts at key kt into buffer `which` (rows past k1 are not copied and never used)
-    auto fetch = [&](int kt, int which) {
-        uint8_t* dst = kbuf + which * 32 * ROWB;
-        #pragma unroll
-        for (int i = 0; i < CHUNKS; i++) {
-            const int qid = i * 32 + lane, row = qid / CHUNKS, c = qid % CHUNKS;
-            if (kt + row < k1) cp_async16(dst + row * ROWB + ((c ^ (row & 7)) * 16), kbase + (kt + row) * row_stride + c * 8);
+    const bf16* vbase = vcache + ((b * Tmax) * NKV + g) * HS_;
+    // K and V rows kt .. kt + 15 -> stage st; rows past the slice repeat its last row (their probabilities are zero, their values finite)
+    auto fetch = [&](int kt, int st) {
+        if (kt < k1) {
+            uint8_t* dst = ring + st * STAGE;
+            #pragma unroll
+            for (int i = 0; i < CA_TILE * CHUNKS / 32; i++) {
+                const int id = i * 32 + lane, row = id / CHUNKS, c = id % CHUNKS;
+                const long long src = min(kt + row, k1 - 1) * row_stride + c * 8;
+                const int off = row * ROWB + ((c ^ (row & 7)) * 16);
+                cp_async16(dst + off, kbase + src);
+                cp_async16(dst + CA_TILE * ROWB + off, vbase + src);
+            }
         }
-        cp_async_commit();
+        cp_async_commit();                                     // possibly empty: the group count per tile stays one
     };
-    constexpr int TSTEP = CA_WARPS * 32;
-    const int kt0 = k0 + warp * 32;
-    if (kt0 < k1) fetch(kt0, 0);
-    int buf = 0;
-    for (int kt = kt0; kt < k1; kt += TSTEP, buf ^= 1) {
-        if (kt + TSTEP < k1) { fetch(kt + TSTEP, buf ^ 1); cp_async_wait<1>(); } else { cp_async_wait<0>(); }
-        __syncwarp();
-        // ---- scores: lane j owns key kt + j
-        const uint8_t* krow = kbuf + buf * 32 * ROWB + lane * ROWB;
-        float s[R];
-        #pragma unroll
-        for (int r = 0; r < R; r++) s[r] = 0.f;
-        #pragma unroll 4
-        for (int c = 0; c < CHUNKS; c++) {
-            const uint4 kq = *reinterpret_cast<const uint4*>(krow + ((c ^ (lane & 7)) * 16));
-            const uint32_t ku[4] = {kq.x, kq.y, kq.z, kq.w};
-            float kf[8];
-            #pragma unroll
-            for (int e = 0; e < 4; e++) { kf[2 * e] = __uint_as_float(ku[e] << 16); kf[2 * e + 1] = __uint_as_float(ku[e] & 0xffff0000u); }
-            #pragma unroll
-            for (int r = 0; r < R; r++) {
-                const float4 qa = *reinterpret_cast<const float4*>(qs + r * HS_ + c * 8), qb = *reinterpret_cast<const float4*>(qs + r * HS_ + c * 8 + 4);
-                s[r] = fmaf(qa.x, kf[0], s[r]); s[r] = fmaf(qa.y, kf[1], s[r]); s[r] = fmaf(qa.z, kf[2], s[r]); s[r] = fmaf(qa.w, kf[3], s[r]);
-                s[r] = fmaf(qb.x, kf[4], s[r]); s[r] = fmaf(qb.y, kf[5], s[r]); s[r] = fmaf(qb.z, kf[6], s[r]); s[r] = fmaf(qb.w, kf[7], s[r]);
-            }
-        }
-        // ---- running softmax of the tile (base 2: the queries carry log2(e))
-        #pragma unroll
-        for (int r = 0; r < R; r++) {
-            const float sv = (kt + lane < limit[r]) ? s[r] : -INFINITY;
-            const float mn = fmaxf(m[r], warp_max(sv));
-            const float pj = (sv == -INFINITY) ? 0.f : ex2_fast(sv - mn);
-            const float corr = (m[r] == -INFINITY) ? 0.f : ex2_fast(m[r] - mn);     // mn is finite whenever any key was visible
-            if (mn != -INFINITY) {
-                l[r] = l[r] * corr + warp_sum(pj);
-                #pragma unroll
-                for (int c = 0; c < CPL; c++) acc[r][c] *= corr;
-                m[r] = mn;
-            }
-            ptile[lane * R + r] = pj;
-        }
-        __syncwarp();
-        // ---- weighted sum of the V rows: lane owns channels lane * CPL .. + CPL - 1; eight rows in flight
-        const int nv = min(32, k1 - kt);
-        for (int i0 = 0; i0 < nv; i0 += 8) {
-            uint32_t vr[8][CPL / 2];
-            #pragma unroll
-            for (int u = 0; u < 8; u++) {
-                const int i = i0 + u;
-                #pragma unroll
-                for (int w = 0; w < CPL / 2; w++) vr[u][w] = 0u;
-                if (i < nv) {
-                    const bf16* vp = vbase + (long long)(kt + i) * row_stride;
-                    if (CPL == 4) { const uint2 t2 = __ldcs(reinterpret_cast<const uint2*>(vp)); vr[u][0] = t2.x; vr[u][CPL / 2 - 1] = t2.y; }
-                    else vr[u][0] = __ldcs(reinterpret_cast<const unsigned int*>(vp));
-                }
-            }
-            #pragma unroll
-            for (int u = 0; u < 8; u++) {
-                const int i = i0 + u;
-                if (i < nv) {                                   // uniform over the warp
-                    float vf[CPL];
-                    #pragma unroll
-                    for (int w = 0; w < CPL / 2; w++) { vf[2 * w] = __uint_as_float(vr[u][w] << 16); vf[2 * w + 1] = __uint_as_float(vr[u][w] & 0xffff0000u); }
-                    #pragma unroll
-                    for (int r = 0; r < R; r++) {
-                        const float pr = ptile[i * R + r];
-                        #pragma unroll
-                        for (int c = 0; c < CPL; c++) acc[r][c] = fmaf(pr, vf[c], acc[r][c]);
-                    }
-                }
-            }
-        }
-        __syncwarp();                                           // the probability tile is rewritten by the next tile
-    }
-    // ---- merge the warps (the K buffers are free now): partial of this slice -> ws[((b, g), slice)][r][HS + 2]
-    __syncthreads();
-    float* sm_m = reinterpret_cast<float*>(ca_smem + R * HS_ * 4);                   // [CA_WARPS][R]
-    float* sm_l = sm_m + CA_WARPS * R;
-    float* sm_acc = sm_l + CA_WARPS * R;                                             // [CA_WARPS][R][HS_]
+    constexpr int TSTEP = CA_WARPS * CA_TILE;
+    const int kt0 = k0 + warp * CA_TILE;
     #pragma unroll
-    for (int r = 0; r < R; r++) {
-        if (lane == 0) { sm_m[warp * R + r] = m[r]; sm_l[warp * R + r] = l[r]; }
+    for (int s = 0; s < CA_STAGES - 1; s++) fetch(kt0 + s * TSTEP, s);
+
+    // query rows r -> token r / G, head g * G + r % G; the A operand of S: lane holds channels 2 tq4, 2 tq4 + 1 and + 8, + 9 of row gq.
+    // Rows past `rows` are zero and dropped at the end.
+    uint32_t qa[KS][2];
+    {
+        const int r = gq < rows ? gq : 0;
+        const bf16* qr = q + ((b * Tq + r / G) * NH + g * G + r % G) * HS_ + 2 * tq4;
         #pragma unroll
-        for (int c = 0; c < CPL; c++) sm_acc[(warp * R + r) * HS_ + lane * CPL + c] = acc[r][c];
+        for (int kk = 0; kk < KS; kk++) {
+            qa[kk][0] = gq < rows ? *reinterpret_cast<const uint32_t*>(qr + kk * 16) : 0u;
+            qa[kk][1] = gq < rows ? *reinterpret_cast<const uint32_t*>(qr + kk * 16 + 8) : 0u;
+        }
     }
+    const int limit = min(k1, start_pos + (gq < rows ? gq : 0) / G + 1);      // keys [0, limit) are visible to this lane's row
+    const float sl2 = scale * CA_LOG2E;
+    float m = -INFINITY, l = 0.f;                              // of row gq; l: this lane's keys only
+    float acc[HS_ / 8][4];                                     // columns 2 tq4, + 1 of channel group n: [0,1] from P hi, [2,3] from P lo
+    #pragma unroll
+    for (int n = 0; n < HS_ / 8; n++) { acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.f; }
+    // ldmatrix: lane supplies the row address of matrix lane / 8, row lane % 8
+    const int mrow = lane & 7, mid = lane >> 3;
+    int st = 0;
+    for (int kt = kt0; kt < k1; kt += TSTEP) {
+        fetch(kt + (CA_STAGES - 1) * TSTEP, st == 0 ? CA_STAGES - 1 : st - 1);
+        cp_async_wait<CA_STAGES - 1>();
+        __syncwarp();
+        const uint32_t kb = smem_u32(ring + st * STAGE), vb = kb + CA_TILE * ROWB;
+        // ---- S (row gq, keys 2 tq4 + {0,1} of each group of 8 keys)
+        float s[2][4];
+        #pragma unroll
+        for (int h = 0; h < 2; h++) { s[h][0] = s[h][1] = s[h][2] = s[h][3] = 0.f; }
+        #pragma unroll
+        for (int kk = 0; kk < KS; kk++) {
+            uint32_t kf[4];     // matrices: keys 0-7 channels 0-7 / 8-15 of the step, keys 8-15 likewise
+            const int row = (mid >> 1) * 8 + mrow, c = kk * 2 + (mid & 1);
+            ldmatrix4(kf, kb + row * ROWB + ((c ^ (row & 7)) * 16));
+            mma_16x8x16(s[0], qa[kk][0], 0u, qa[kk][1], 0u, kf[0], kf[1]);
+            mma_16x8x16(s[1], qa[kk][0], 0u, qa[kk][1], 0u, kf[2], kf[3]);
+        }
+        // ---- running softmax of row gq (base 2); the four lanes of a row hold its 16 keys
+        float sv[4];
+        #pragma unroll
+        for (int e = 0; e < 4; e++) {
+            const int key = kt + (e >> 1) * 8 + 2 * tq4 + (e & 1);
+            sv[e] = key < limit ? s[e >> 1][e & 1] * sl2 : -INFINITY;
+        }
+        float mn = fmaxf(fmaxf(sv[0], sv[1]), fmaxf(sv[2], sv[3]));
+        mn = fmaxf(mn, __shfl_xor_sync(0xffffffffu, mn, 1));
+        mn = fmaxf(mn, __shfl_xor_sync(0xffffffffu, mn, 2));
+        mn = fmaxf(mn, m);
+        const float mref = mn == -INFINITY ? 0.f : mn;         // no key seen yet: every probability below is 2^-inf = 0
+        const float corr = ex2_fast(m - mref);
+        float p[4];
+        #pragma unroll
+        for (int e = 0; e < 4; e++) p[e] = ex2_fast(sv[e] - mref);
+        l = l * corr + ((p[0] + p[1]) + (p[2] + p[3]));
+        m = mn;
+        if (__any_sync(0xffffffffu, corr != 1.0f)) {
+            #pragma unroll
+            for (int n = 0; n < HS_ / 8; n++) { acc[n][0] *= corr; acc[n][1] *= corr; acc[n][2] *= corr; acc[n][3] *= corr; }
+        }
+        uint32_t hi[2], lo[2];
+        #pragma unroll
+        for (int h = 0; h < 2; h++) {
+            hi[h] = pack_bf16x2(p[2 * h], p[2 * h + 1]);
+            const float2 hf = unpack_bf16x2(hi[h]);
+            lo[h] = pack_bf16x2(p[2 * h] - hf.x, p[2 * h + 1] - hf.y);
+        }
+        // ---- O += P V: 16 keys, 16 channels per ldmatrix
+        #pragma unroll
+        for (int n2 = 0; n2 < HS_ / 16; n2++) {
+            uint32_t vf[4];     // matrices: keys 0-7 / 8-15 of channels 0-7 of the pair of groups, then of channels 8-15
+            const int row = (mid & 1) * 8 + mrow, c = n2 * 2 + (mid >> 1);
+            ldmatrix4_trans(vf, vb + row * ROWB + ((c ^ (row & 7)) * 16));
+            mma_16x8x16(acc[2 * n2], hi[0], lo[0], hi[1], lo[1], vf[0], vf[1]);
+            mma_16x8x16(acc[2 * n2 + 1], hi[0], lo[0], hi[1], lo[1], vf[2], vf[3]);
+        }
+        __syncwarp();                                          // the stage may be refilled
+        st = st + 1 == CA_STAGES ? 0 : st + 1;
+    }
+    cp_async_wait<0>();
+    l += __shfl_xor_sync(0xffffffffu, l, 1);
+    l += __shfl_xor_sync(0xffffffffu, l, 2);
+    // ---- merge the warps in warp order (the rings are free now)
     __syncthreads();
-    float* dst = ws + (((size_t)(b * NKV + g) * nslices + slice) * R) * (HS_ + 2);
-    for (int i = threadIdx.x; i < R * HS_; i += CA_THREADS) {
-        const int r = i / HS_, c = i - r * HS_;
+    float* wp = reinterpret_cast<float*>(ca_smem) + warp * PART;
+    #pragma unroll
+    for (int n = 0; n < HS_ / 8; n++) {
+        wp[gq * HS_ + n * 8 + 2 * tq4] = acc[n][0] + acc[n][2];
+        wp[gq * HS_ + n * 8 + 2 * tq4 + 1] = acc[n][1] + acc[n][3];
+    }
+    if (tq4 == 0) { wp[CA_MAX_R * HS_ + gq] = m; wp[CA_MAX_R * HS_ + CA_MAX_R + gq] = l; }
+    __syncthreads();
+    const float* w0 = reinterpret_cast<const float*>(ca_smem);
+    float* dst = CLUSTER ? part : ws + ((size_t)(b * NKV + g) * nslices + slice) * PART;
+    for (int i = threadIdx.x; i < rows * HS_; i += CA_THREADS) {
+        const int r = i / HS_;
         float mn = -INFINITY;
         #pragma unroll
-        for (int w = 0; w < CA_WARPS; w++) mn = fmaxf(mn, sm_m[w * R + r]);
+        for (int w = 0; w < CA_WARPS; w++) mn = fmaxf(mn, w0[w * PART + CA_MAX_R * HS_ + r]);
         float a = 0.f, ls = 0.f;
         #pragma unroll
         for (int w = 0; w < CA_WARPS; w++) {
-            const float mw = sm_m[w * R + r];
+            const float mw = w0[w * PART + CA_MAX_R * HS_ + r];
             const float cw = (mw == -INFINITY) ? 0.f : ex2_fast(mw - mn);
-            a += sm_acc[(w * R + r) * HS_ + c] * cw;
-            ls += sm_l[w * R + r] * cw;
+            a += w0[w * PART + i] * cw;
+            ls += w0[w * PART + CA_MAX_R * HS_ + CA_MAX_R + r] * cw;
         }
-        dst[r * (HS_ + 2) + c] = a;
-        if (c == 0) { dst[r * (HS_ + 2) + HS_] = mn; dst[r * (HS_ + 2) + HS_ + 1] = ls; }
+        dst[i] = a;
+        if (i - r * HS_ == 0) { dst[CA_MAX_R * HS_ + r] = mn; dst[CA_MAX_R * HS_ + CA_MAX_R + r] = ls; }
+    }
+    if (CLUSTER) {
+        __syncwarp();
+        cluster_sync();                                        // the partials of all slices are in place
+        const uint32_t base = smem_u32(part);
+        for (int i = slice * CA_THREADS + threadIdx.x; i < rows * HS_; i += nslices * CA_THREADS) {
+            const int r = i / HS_, c = i - r * HS_;
+            float mn = -INFINITY;
+            for (int s2 = 0; s2 < nslices; s2++) mn = fmaxf(mn, ld_peer(base + (CA_MAX_R * HS_ + r) * 4, s2));
+            float a = 0.f, ls = 0.f;
+            for (int s2 = 0; s2 < nslices; s2++) {
+                const float ms = ld_peer(base + (CA_MAX_R * HS_ + r) * 4, s2);
+                const float cw = (ms == -INFINITY) ? 0.f : ex2_fast(ms - mn);
+                a += ld_peer(base + i * 4, s2) * cw;
+                ls += ld_peer(base + (CA_MAX_R * HS_ + CA_MAX_R + r) * 4, s2) * cw;
+            }
+            out[((b * Tq + r / G) * NH + g * G + r % G) * HS_ + c] = __float2bfloat16_rn(a / ls);
+        }
+        __syncwarp();
+        cluster_sync();                                        // no CTA leaves while a peer may still read its shared memory
     }
 }
 
-// out[row r of (b, g)] = sum over slices of acc_s * exp(m_s - M) / sum over slices of l_s * exp(m_s - M), slices in order
+// out[row r of (b, g)] = sum over slices of acc_s * 2^(m_s - M) / sum over slices of l_s * 2^(m_s - M), slices in order
 template <int HS_>
-__global__ void cached_attention_combine_kernel(bf16* __restrict__ out, const float* __restrict__ ws, int Tq, int NH, int NKV,
-                                                int nslices, int R, int rows) {
+__global__ void cached_attention_combine_kernel(bf16* __restrict__ out, const float* __restrict__ ws, int Tq, int NH, int NKV, int nslices) {
+    pdl_wait();
+    pdl_trigger();
+    constexpr int PART = ca_part_floats<HS_>();
     const int r = blockIdx.x, g = blockIdx.y;
     const long long b = blockIdx.z;
     const int c = threadIdx.x;
-    if (r >= rows || c >= HS_) return;
-    const float* src = ws + ((size_t)(b * NKV + g) * nslices * R + r) * (HS_ + 2);
-    const size_t sstride = (size_t)R * (HS_ + 2);
+    const float* src = ws + (size_t)(b * NKV + g) * nslices * PART;
     float mn = -INFINITY;
-    for (int s = 0; s < nslices; s++) mn = fmaxf(mn, src[s * sstride + HS_]);
+    for (int s = 0; s < nslices; s++) mn = fmaxf(mn, src[(size_t)s * PART + CA_MAX_R * HS_ + r]);
     float a = 0.f, ls = 0.f;
     for (int s = 0; s < nslices; s++) {
-        const float ms = src[s * sstride + HS_];
+        const float ms = src[(size_t)s * PART + CA_MAX_R * HS_ + r];
         const float cw = (ms == -INFINITY) ? 0.f : ex2_fast(ms - mn);        // the maxima are in base-2 units
-        a += src[s * sstride + c] * cw;
-        ls += src[s * sstride + HS_ + 1] * cw;
+        a += src[(size_t)s * PART + r * HS_ + c] * cw;
+        ls += src[(size_t)s * PART + CA_MAX_R * HS_ + CA_MAX_R + r] * cw;
     }
     const int G = NH / NKV;
     const int t = r / G, hq = g * G + r % G;
     out[((b * Tq + t) * NH + hq) * HS_ + c] = __float2bfloat16_rn(a / ls);
-}
-
-// ---------------------------------------------------------------------------------------------------------------
-// Skinny product for decoding steps: out (M, N) = x (M, K) . w (N, K)^T with M <= 8 rows.  A 128-row tcgen05 tile would
-// spend its time on padding and, worse, leave most SMs without a tile (N / 128 tiles for 148 SMs), while the step is bound by
-// streaming the weights once.  Here a CTA owns 16 output columns and its 8 warps split K; a warp feeds warp-level
-// m16n8k16 MMAs with the weights as the 16-row operand and the (at most 8) activation rows as the 8-column operand, so that
-// the arithmetic costs two instructions per KB of weights and the loop is nothing but 128-bit streaming loads.  A lane
-// loads 8 consecutive K elements of weight rows g and g + 8 and of activation row g (g = lane / 4) and uses them as the
-// K slots of two MMAs; the dot product does not care that this permutes K, as long as both operands agree.
-constexpr int SK_WARPS = 8;
-constexpr int SK_THREADS = SK_WARPS * 32;
-constexpr int SK_COLS = 16;
-constexpr int SK_UNROLL = 4;
-constexpr int SK_MAX_M = 8;
-
-DEVINL void mma_16x8x16(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-                 : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-
-__global__ void __launch_bounds__(SK_THREADS)
-skinny_gemm_kernel(bf16* __restrict__ out, const bf16* __restrict__ x, const bf16* __restrict__ w, int M, int N, int K,
-                   int ldx, int ldw, int ldo) {
-    __shared__ float red[SK_WARPS][4][32];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int g = lane >> 2, t = lane & 3;
-    const int n0 = blockIdx.x * SK_COLS;
-    const bf16* w0 = w + (size_t)min(n0 + g, N - 1) * ldw;          // a clamped row is computed, not stored
-    const bf16* w1 = w + (size_t)min(n0 + g + 8, N - 1) * ldw;
-    const bool xvalid = g < M;
-    const bf16* xr = x + (size_t)min(g, M - 1) * ldx;
-    const int nchunks = (K + 31) >> 5;                               // 32 K elements per chunk: 8 per lane of a quad
-    const int per_warp = (nchunks + SK_WARPS - 1) / SK_WARPS;
-    const int c_begin = warp * per_warp, c_end = min(c_begin + per_warp, nchunks);
-    float c[4] = {0.f, 0.f, 0.f, 0.f};
-    const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
-    // whole groups of SK_UNROLL full chunks: every load is issued before the first MMA, nothing is predicated
-    const int full_end = min(c_end, K >> 5);
-    int ch = c_begin;
-    for (; ch + SK_UNROLL <= full_end; ch += SK_UNROLL) {
-        uint4 a0[SK_UNROLL], a1[SK_UNROLL], b[SK_UNROLL];
-        #pragma unroll
-        for (int u = 0; u < SK_UNROLL; u++) {
-            const int k = ((ch + u) << 5) + t * 8;
-            a0[u] = __ldcs(reinterpret_cast<const uint4*>(w0 + k));
-            a1[u] = __ldcs(reinterpret_cast<const uint4*>(w1 + k));
-            b[u] = *reinterpret_cast<const uint4*>(xr + k);
-        }
-        #pragma unroll
-        for (int u = 0; u < SK_UNROLL; u++) {
-            if (!xvalid) b[u] = zero;
-            mma_16x8x16(c, a0[u].x, a1[u].x, a0[u].y, a1[u].y, b[u].x, b[u].y);
-            mma_16x8x16(c, a0[u].z, a1[u].z, a0[u].w, a1[u].w, b[u].z, b[u].w);
-        }
-    }
-    // the rest, one chunk at a time; the last chunk of K may be partial
-    for (; ch < c_end; ch++) {
-        const int k = (ch << 5) + t * 8;
-        const bool ok = k < K;
-        const uint4 a0 = ok ? __ldcs(reinterpret_cast<const uint4*>(w0 + k)) : zero;
-        const uint4 a1 = ok ? __ldcs(reinterpret_cast<const uint4*>(w1 + k)) : zero;
-        const uint4 b = (ok && xvalid) ? *reinterpret_cast<const uint4*>(xr + k) : zero;
-        mma_16x8x16(c, a0.x, a1.x, a0.y, a1.y, b.x, b.y);
-        mma_16x8x16(c, a0.z, a1.z, a0.w, a1.w, b.z, b.w);
-    }
-    #pragma unroll
-    for (int i = 0; i < 4; i++) red[warp][i][lane] = c[i];
-    __syncthreads();
-    if (warp == 0) {
-        // accumulator layout: c[2 i + j] = out[row 2 t + j][column n0 + g + 8 i]
-        #pragma unroll
-        for (int i = 0; i < 4; i++) {
-            float v = 0.f;
-            #pragma unroll
-            for (int ww = 0; ww < SK_WARPS; ww++) v += red[ww][i][lane];
-            const int m = 2 * t + (i & 1), n = n0 + g + 8 * (i >> 1);
-            if (m < M && n < N) out[(size_t)m * ldo + n] = __float2bfloat16_rn(v);
-        }
-    }
 }
 
 int decode_check(int B, int Tq, int Tmax, int start_pos, int NH, int NKV, int HS, bool device_pos) {
@@ -468,78 +437,70 @@ extern "C" int llmc_rope_cache(bf16* q, bf16* kcache, bf16* vcache, const bf16* 
     if (!pos_ptr && start_pos + Tq > freqs_len) return -4;
     const long long N = (long long)B * Tq;
     const long long total = N * (NH + 2 * NKV) * (HS / 8);
-    rope_cache_kernel<<<(unsigned)CEIL_DIV(total, 256), 256, 0, stream>>>(q, kcache, vcache, raw, reinterpret_cast<const float2*>(freqs),
-                                                                          N, Tq, Tmax, start_pos, NH, NKV, HS, pos_ptr, freqs_len,
-                                                                          llmc_status_ptr());
-    CUDA_CHECK(cudaGetLastError());
+    CUDA_CHECK(launch_pdl(rope_cache_kernel, dim3((unsigned)CEIL_DIV(total, 256)), dim3(256), 0, stream, 0, q, kcache, vcache, raw,
+                          reinterpret_cast<const float2*>(freqs), N, Tq, Tmax, start_pos, NH, NKV, HS, pos_ptr, freqs_len, llmc_status_ptr()));
     return 0;
 }
 
 namespace {
-// Key slices of the fast path: whole multiples of the 128 keys a CTA covers per trip, at least CA_MIN_KEYS, and short enough
-// for about sixteen CTAs per SM (three are resident at a time: many short CTAs keep the last wave small).  The cache's
-// capacity decides, not the current length, because the position may live on the device.
+// Key slices of the fast path: whole multiples of the 64 keys a CTA covers per trip, at least CA_MIN_KEYS, and about as many CTAs as
+// are resident at once (two per SM); one cluster per head as long as eight slices do, since a second launch costs more than the SMs
+// it leaves idle, except where a slice would get longer than 1024 keys.  The cache's capacity decides, not the current length,
+// because the position may live on the device.
 int ca_keys_per_slice(int B, int Tmax, int NKV) {
     int sms = llmc_device_sm_count(); if (sms <= 0) sms = 148;
-    const int want = CEIL_DIV(16 * sms, B * NKV);
-    int kps = CEIL_DIV(CEIL_DIV(Tmax, want), CA_WARPS * 32) * (CA_WARPS * 32);
+    int want = (2 * sms) / (B * NKV);
+    if (want < 1) want = 1;
+    if (want > CA_MAX_CLUSTER && CEIL_DIV(Tmax, CA_MAX_CLUSTER) <= 1024) want = CA_MAX_CLUSTER;
+    const int trip = CA_WARPS * CA_TILE;
+    const int kps = CEIL_DIV(CEIL_DIV(Tmax, want), trip) * trip;
     return kps < CA_MIN_KEYS ? CA_MIN_KEYS : kps;
 }
 int ca_slices(int B, int Tmax, int NKV) { return CEIL_DIV(Tmax, ca_keys_per_slice(B, Tmax, NKV)); }
-int ca_rows_padded(int rows) { return rows <= 1 ? 1 : rows <= 2 ? 2 : rows <= 4 ? 4 : 8; }
 bool ca_fast(int Tq, int NH, int NKV, int HS) { return (HS == 64 || HS == 128) && (NH / NKV) * Tq <= CA_MAX_R; }
 
-template <int HS_, int R>
+template <int HS_, bool CLUSTER>
 int ca_launch(bf16* out, float* ws, const bf16* q, const bf16* kcache, const bf16* vcache, int B, int Tq, int Tmax, int start_pos, int NH,
               int NKV, const int* pos_ptr, cudaStream_t stream) {
     const int rows = (NH / NKV) * Tq, slices = ca_slices(B, Tmax, NKV);
-    const int keys_per_slice = ca_keys_per_slice(B, Tmax, NKV);
-    constexpr int smem = ca_smem_bytes<HS_, R>();
+    constexpr int smem = ca_smem_bytes<HS_>();
     static bool configured = false;
     if (!configured) {
-        CUDA_CHECK(cudaFuncSetAttribute(cached_attention_split_kernel<HS_, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        CUDA_CHECK(cudaFuncSetAttribute(cached_attention_split_kernel<HS_, CLUSTER>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
         configured = true;
     }
-    cached_attention_split_kernel<HS_, R><<<dim3(slices, NKV, B), CA_THREADS, smem, stream>>>(ws, q, kcache, vcache, Tq, Tmax, start_pos, NH, NKV,
-                                                                                           rsqrtf((float)HS_), pos_ptr, llmc_status_ptr(),
-                                                                                           keys_per_slice, rows);
-    CUDA_CHECK(cudaGetLastError());
-    cached_attention_combine_kernel<HS_><<<dim3(rows, NKV, B), HS_, 0, stream>>>(out, ws, Tq, NH, NKV, slices, R, rows);
-    CUDA_CHECK(cudaGetLastError());
+    CUDA_CHECK(launch_pdl(cached_attention_split_kernel<HS_, CLUSTER>, dim3(slices, NKV, B), dim3(CA_THREADS), smem, stream, CLUSTER ? slices : 0,
+                          out, ws, q, kcache, vcache, Tq, Tmax, start_pos, NH, NKV, rsqrtf((float)HS_), pos_ptr, llmc_status_ptr(),
+                          ca_keys_per_slice(B, Tmax, NKV), rows));
+    if (!CLUSTER)
+        CUDA_CHECK(launch_pdl(cached_attention_combine_kernel<HS_>, dim3(rows, NKV, B), dim3(HS_), 0, stream, 0, out, (const float*)ws, Tq, NH, NKV, slices));
     return 0;
 }
 }  // namespace
 
-// fp32 words of workspace llmc_cached_attention needs for this problem (0: the general kernel runs, which needs none)
+// fp32 words of workspace llmc_cached_attention needs for this problem (0: it runs without one)
 extern "C" long long llmc_cached_attention_workspace(int B, int Tq, int Tmax, int NH, int NKV, int HS) {
     if (NKV <= 0 || NH % NKV || !ca_fast(Tq, NH, NKV, HS)) return 0;
-    return (long long)B * NKV * ca_slices(B, Tmax, NKV) * ca_rows_padded((NH / NKV) * Tq) * (HS + 2);
+    const int slices = ca_slices(B, Tmax, NKV);
+    return slices <= CA_MAX_CLUSTER ? 0 : (long long)B * NKV * slices * CA_MAX_R * (HS + 2);
 }
 
 extern "C" int llmc_cached_attention(bf16* out, const bf16* q, const bf16* kcache, const bf16* vcache, int B, int Tq, int Tmax,
                                      int start_pos, int NH, int NKV, int HS, const int* pos_ptr, float* ws, cudaStream_t stream) {
     const int rc = decode_check(B, Tq, Tmax, start_pos, NH, NKV, HS, pos_ptr != nullptr);
     if (rc) return rc;
-    if (ws != nullptr && ca_fast(Tq, NH, NKV, HS)) {
+    const bool cluster = ca_fast(Tq, NH, NKV, HS) && ca_slices(B, Tmax, NKV) <= CA_MAX_CLUSTER;
+    if (ca_fast(Tq, NH, NKV, HS) && (cluster || ws != nullptr)) {
         if ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(kcache) | reinterpret_cast<uintptr_t>(vcache)) & 15) return -5;
-        const int R = ca_rows_padded((NH / NKV) * Tq);
-#define CA_GO(H, RR) return ca_launch<H, RR>(out, ws, q, kcache, vcache, B, Tq, Tmax, start_pos, NH, NKV, pos_ptr, stream)
-        if (HS == 64) { if (R == 1) CA_GO(64, 1); if (R == 2) CA_GO(64, 2); if (R == 4) CA_GO(64, 4); CA_GO(64, 8); }
-        else { if (R == 1) CA_GO(128, 1); if (R == 2) CA_GO(128, 2); if (R == 4) CA_GO(128, 4); CA_GO(128, 8); }
+#define CA_GO(H, CL) return ca_launch<H, CL>(out, ws, q, kcache, vcache, B, Tq, Tmax, start_pos, NH, NKV, pos_ptr, stream)
+        if (HS == 64) { if (cluster) CA_GO(64, true); CA_GO(64, false); }
+        if (cluster) CA_GO(128, true);
+        CA_GO(128, false);
 #undef CA_GO
     }
     const dim3 grid(NH, Tq, B);
     cached_attention_kernel<<<grid, DEC_THREADS, 0, stream>>>(out, q, kcache, vcache, Tq, Tmax, start_pos, NH, NKV, HS, rsqrtf((float)HS),
                                                               pos_ptr, llmc_status_ptr());
-    CUDA_CHECK(cudaGetLastError());
-    return 0;
-}
-
-// out (M, N) = x (M, K) . w (N, K)^T for M <= 8; K and the row strides of x and w are multiples of 8 elements.
-extern "C" int llmc_skinny_gemm(bf16* out, const bf16* x, const bf16* w, int M, int N, int K, int ldx, int ldw, int ldo, cudaStream_t stream) {
-    if (M <= 0 || M > SK_MAX_M || N <= 0 || K <= 0 || (K % 8) || (ldx % 8) || (ldw % 8)) return -1;
-    if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w)) & 15) return -1;
-    skinny_gemm_kernel<<<(unsigned)CEIL_DIV(N, SK_COLS), SK_THREADS, 0, stream>>>(out, x, w, M, N, K, ldx, ldw, ldo);
     CUDA_CHECK(cudaGetLastError());
     return 0;
 }

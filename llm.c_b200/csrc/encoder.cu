@@ -10,11 +10,14 @@
 //
 // Capability parity: llmc/encoder.cuh (encoder_forward, encoder_backward) of the reference.
 #include "common.cuh"
+#include "pdl.cuh"
 
 namespace {
 
 __global__ void encoder_fwd_kernel(bf16* __restrict__ out, const int* __restrict__ tokens, const bf16* __restrict__ wte,
                                    const bf16* __restrict__ wpe, int B, int T, int C, int V) {
+    pdl_wait();
+    pdl_trigger();
     const int cp = C >> 3;
     const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= (long long)B * T * cp) return;
@@ -201,8 +204,7 @@ wte_bwd_kernel(bf16* __restrict__ dwte, const bf16* __restrict__ dout, const int
 extern "C" int llmc_encoder_fwd(bf16* out, const int* tokens, const bf16* wte, const bf16* wpe, int B, int T, int C, int V, cudaStream_t stream) {
     if (C % 8) return -1;
     long long total = (long long)B * T * (C / 8);
-    encoder_fwd_kernel<<<(unsigned)CEIL_DIV(total, 256), 256, 0, stream>>>(out, tokens, wte, wpe, B, T, C, V);
-    CUDA_CHECK(cudaGetLastError());
+    CUDA_CHECK(launch_pdl(encoder_fwd_kernel, dim3((unsigned)CEIL_DIV(total, 256)), dim3(256), 0, stream, 0, out, tokens, wte, wpe, B, T, C, V));
     return 0;
 }
 

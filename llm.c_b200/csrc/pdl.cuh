@@ -1,0 +1,24 @@
+// Programmatic dependent launch: a kernel launched through launch_pdl may start while the kernel before it in its stream is still
+// running, as soon as every CTA of that one has called pdl_trigger() or exited.  Such a kernel calls pdl_wait() before it touches
+// anything another kernel may have written or may still read; pdl_wait() returns when the preceding kernel has completed and its
+// writes are visible.  A kernel calls pdl_trigger() only after its own pdl_wait(), so "the preceding kernel has completed" covers all
+// kernels before it too.  Behind a kernel that never triggers (or a copy) the launch is an ordinary one.  Works the same inside a
+// captured graph.
+#pragma once
+#include "common.cuh"
+
+DEVINL void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+DEVINL void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+template <typename... P, typename... A>
+cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, int cluster_x, A... args) {
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = cluster_x; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = stream;
+    cfg.attrs = attr; cfg.numAttrs = cluster_x > 0 ? 2 : 1;
+    return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}

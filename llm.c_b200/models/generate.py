@@ -35,7 +35,11 @@ class CachedDecoder:
         # prompts of at least this many tokens per row, starting at position 0, run through the training attention kernel
         self.dense_prefill_from = 128
         # steps of at most this many rows use the weight-streaming product instead of a padded tensor-core tile (0: never)
-        self.skinny_rows = 8 if (model.device.type == "cuda" and model.dtype == torch.bfloat16) else 0
+        kernels = model.device.type == "cuda" and model.dtype == torch.bfloat16
+        self.skinny_rows = 8 if kernels else 0
+        # steps of at most this many rows run their products on exactly their rows (split-K weight streaming, csrc/stream_gemm.cu), the
+        # MLP's up-projections with the activation in the same launch; longer ones on rows padded to whole 128-row tiles
+        self.stream_rows = 128 if kernels else 0
 
     def cache_bytes(self):
         return 2 * self.kcache.numel() * self.kcache.element_size()
@@ -75,6 +79,8 @@ class CachedDecoder:
         def mm(out, inp, weight, n):
             if n <= self.skinny_rows:
                 ops.matmul_skinny(out[:n], inp[:n], weight)
+            elif n <= self.stream_rows:
+                ops.matmul_forward(out[:n], inp[:n], weight, None)
             elif padded:
                 ops.matmul_forward(out, inp, weight, None)          # whole 128-row tiles; the rows beyond n are never read
             else:
@@ -104,13 +110,19 @@ class CachedDecoder:
                 ops.cached_attention(a["atty"][:N], a["q"][:N], self.kcache[l], self.vcache[l], Tq, start_pos, NH, NKV, pos)
             mm(a["proj"], a["atty"], p["attprojw"][l], N)
             ops.rmsnorm_fused_residual_forward(a["res"][:N], ln[:N], rstd[:N], x[:N], a["proj"][:N], p["ln2w"][l], eps)
-            mm(a["fc12"], ln, p["fc12w"][l], N)
-            ops.swiglu_forward(a["h"][:N], a["fc12"][:N])
+            if N <= self.stream_rows and cfg.hidden_dim % 64 == 0:
+                ops.matmul_swiglu(a["h"][:N], ln[:N], p["fc12w"][l])
+            else:
+                mm(a["fc12"], ln, p["fc12w"][l], N)
+                ops.swiglu_forward(a["h"][:N], a["fc12"][:N])
             mm(a["proj"], a["h"], p["fcprojw"][l], N)
             w = p["ln1w"][l + 1] if l + 1 < L else p["lnfw"]
             ops.rmsnorm_fused_residual_forward(x[:N], ln[:N], rstd[:N], a["res"][:N], a["proj"][:N], w, eps)
-        a["last"][:B].copy_(ln[:N].view(B, Tq, C)[:, -1])
-        mm(a["logits"], a["last"], p["lmhead"], B)
+        last = ln                                       # one token per row: the last positions are the rows themselves
+        if Tq > 1:
+            last = a["last"]
+            last[:B].copy_(ln[:N].view(B, Tq, C)[:, -1])
+        mm(a["logits"], last, p["lmhead"], B)
         return a["logits"][:B, :cfg.vocab_size].float()
 
 

@@ -13,6 +13,9 @@ _launches = 0   # number of kernel-library launches issued (bench.py reports it)
 # forward / dgrad GEMMs with at least this many 256 x 256 tiles run on the two-SM kernel (gemm2.cu); 0 disables it
 TWO_SM_MIN_TILES = int(os.environ.get("LLMC_GEMM_2SM_MIN_TILES", "74"))
 
+# forward products of at most this many rows stream the weights through split-K clusters (stream_gemm.cu)
+STREAM_MAX_ROWS = 128
+
 
 def launch_count():
     return _launches
@@ -59,6 +62,11 @@ def gemm(a, b, d, M, N, K, lda, ldb, ldd, a_mn, b_mn, mode, bias=None, aux=None,
     global _launches
     lib = _lib.cuda()
     _launches += 1
+    if M <= STREAM_MAX_ROWS and mode == MODE_STORE and not a_mn and not b_mn:
+        if ready is not None:
+            ready.wait()
+        check(lib.llmc_stream_gemm(_p(d), _p(a), _p(b), _p(bias), M, N, K, lda, ldb, ldd, _stream()), "llmc_stream_gemm")
+        return
     tiles256 = ((M + 255) // 256) * ((N + 255) // 256)
     if mode == MODE_ACCUM:
         two_sm = TWO_SM_MIN_TILES > 0 and a_mn and b_mn and tiles256 >= 8
@@ -336,13 +344,24 @@ def cached_attention(out, q, kcache, vcache, Tq, start_pos, NH, NKV, pos=None):
 
 
 def matmul_skinny(out, inp, weight):
-    """out[M,OC] = inp[M,C] @ weight[OC,C]^T for at most 8 rows: the weight-streaming kernel of decoding steps (csrc/decode.cu)."""
+    """out[M,OC] = inp[M,C] @ weight[OC,C]^T for at most 8 rows: the weight-streaming kernel of decoding steps (csrc/stream_gemm.cu)."""
     global _launches
     M, C = inp.shape
     OC = weight.shape[0]
     _launches += 1
     check(_lib.cuda().llmc_skinny_gemm(_p(out), _p(inp), _p(weight), M, OC, C, inp.stride(0), weight.stride(0), out.stride(0), _stream()),
           "llmc_skinny_gemm")
+
+
+def matmul_swiglu(h, inp, weight12):
+    """h[M,H] = (inp @ w1^T) * silu(inp @ w2^T) with weight12 = [w1; w2] (2H, C), at most 128 rows, H a multiple of 64: the
+    up-projections of a decoding step and their activation in one launch (csrc/stream_gemm.cu)."""
+    global _launches
+    M, C = inp.shape
+    H = weight12.shape[0] // 2
+    _launches += 1
+    check(_lib.cuda().llmc_stream_gemm_swiglu(_p(h), _p(inp), _p(weight12), M, H, C, inp.stride(0), weight12.stride(0), h.stride(0), _stream()),
+          "llmc_stream_gemm_swiglu")
 
 
 def make_table(views):

@@ -377,6 +377,12 @@ def swiglu_forward(h, x12):
     h.copy_(x[:, :H] * torch.nn.functional.silu(x[:, H:]))
 
 
+def matmul_swiglu(h, inp, weight12):
+    H = h.shape[1]
+    x = _f(inp) @ _f(weight12).t()
+    h.copy_(x[:, :H] * torch.nn.functional.silu(x[:, H:]))
+
+
 def swiglu_backward(dx12, dh, x12):
     H = dh.shape[1]
     x, dy = _f(x12), _f(dh)
