@@ -16,8 +16,8 @@
 // loads and stores around them) with the tensor pipe close behind (2048 / 1536 cycles a pair).  So nothing but that is left to the
 // softmax warps: no operand goes through shared memory (the kernel this one replaces staged P and dS there, with one stage of
 // streamed tiles), S of the next pair is issued before dS of this one is finished, the outputs leave through four warps of
-// their own.  All three launches, the kernels before these in brackets: B=16 T=2048 NH=8 HS=128 521 us (978), B=2 T=4096 NH=32 HS=128
-// 880 us (1723), B=3 T=1000 NH=32 HS=80 113 us (235).
+// their own.  All three launches, the kernels before these in brackets: B=16 T=2048 NH=8 HS=128 509 us (978), B=2 T=4096 NH=32 HS=128
+// 855 us (1723), B=3 T=1000 NH=32 HS=80 112 us (235); 521 / 880 / 113 with scalar instead of paired fp32 arithmetic in the softmax.
 //
 // Work items are one fixed tile of one head, heaviest first, dealt to the persistent CTAs in alternating direction (CTA c gets items
 // c, 2G-1-c, 2G+c, ...), which evens out the decreasing sizes; a plain round-robin gives CTA 0 the longest item of every round.
@@ -319,14 +319,15 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
         const float log2e = 1.4426950408889634f;
         bool ok = true;
         uint32_t t = 0;
-        float row_lse = 0.f, row_delta = 0.f;          // dQ pass: statistics of this thread's query row
+        float row_lse = 0.f, row_delta = 0.f;          // dQ pass: statistics of this thread's query row, negated like those of the table
+        const uint64_t sl2 = f2_pack(a.scale_log2e, a.scale_log2e), sc2 = f2_pack(a.scale, a.scale);
         for (; wk.valid(); wk.next(), t++) {
             const bool diag = wk.x == wk.f;
-            const float* stat = sStat + (t & 1) * (2 * BT) + hf * 64;       // dK / dV pass: lse * log2(e) of this half's queries; delta * scale 128 floats further
+            const float* stat = sStat + (t & 1) * (2 * BT) + hf * 64;       // dK / dV pass: -lse * log2(e) of this half's queries; -delta * scale 128 floats further
             if (!DKV && wk.first()) {
                 const int tq = wk.f * BT + r;
-                row_lse = INFINITY; row_delta = 0.f;
-                if (tq < a.T) { row_lse = a.lse[(size_t)wk.bh * a.T + tq] * log2e; row_delta = a.delta[(size_t)wk.bh * a.T + tq] * a.scale; }
+                row_lse = -INFINITY; row_delta = 0.f;
+                if (tq < a.T) { row_lse = -(a.lse[(size_t)wk.bh * a.T + tq] * log2e); row_delta = -(a.delta[(size_t)wk.bh * a.T + tq] * a.scale); }
             }
             ok = mbar_wait(&s_full[t & 1], (t >> 1) & 1, abort_flag, a.status, 0x6a0) && ok;
             if (DKV) ok = mbar_wait(&st_full[t & 1], (t >> 1) & 1, abort_flag, a.status, 0x6a1) && ok;
@@ -344,10 +345,10 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
                 for (int e4 = 0; e4 < 8; e4++) {
                     float4 l4 = make_float4(row_lse, row_lse, row_lse, row_lse);
                     if (DKV) l4 = *reinterpret_cast<const float4*>(stat + h2 * 32 + e4 * 4);
-                    p[h2 * 32 + e4 * 4 + 0] = ex2_fast(fmaf(__uint_as_float(sv[e4 * 4 + 0]), a.scale_log2e, -l4.x));
-                    p[h2 * 32 + e4 * 4 + 1] = ex2_fast(fmaf(__uint_as_float(sv[e4 * 4 + 1]), a.scale_log2e, -l4.y));
-                    p[h2 * 32 + e4 * 4 + 2] = ex2_fast(fmaf(__uint_as_float(sv[e4 * 4 + 2]), a.scale_log2e, -l4.z));
-                    p[h2 * 32 + e4 * 4 + 3] = ex2_fast(fmaf(__uint_as_float(sv[e4 * 4 + 3]), a.scale_log2e, -l4.w));
+                    const float2 x0 = f2_unpack(f2_fma(f2_pack_u(sv[e4 * 4 + 0], sv[e4 * 4 + 1]), sl2, f2_pack(l4.x, l4.y)));
+                    const float2 x1 = f2_unpack(f2_fma(f2_pack_u(sv[e4 * 4 + 2], sv[e4 * 4 + 3]), sl2, f2_pack(l4.z, l4.w)));
+                    p[h2 * 32 + e4 * 4 + 0] = ex2_fast(x0.x); p[h2 * 32 + e4 * 4 + 1] = ex2_fast(x0.y);
+                    p[h2 * 32 + e4 * 4 + 2] = ex2_fast(x1.x); p[h2 * 32 + e4 * 4 + 3] = ex2_fast(x1.y);
                 }
             }
             // only the diagonal tile needs a mask (query >= key).  Rows and columns past T need none beyond it: queries past T have
@@ -381,12 +382,11 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
                 for (int e4 = 0; e4 < 4; e4++) {
                     float4 d4 = make_float4(row_delta, row_delta, row_delta, row_delta);
                     if (DKV) d4 = *reinterpret_cast<const float4*>(stat + BT + c * 16 + e4 * 4);
-                    const float dl[4] = {d4.x, d4.y, d4.z, d4.w};
-                    float ds[4];
-                    #pragma unroll
-                    for (int k = 0; k < 4; k++) ds[k] = p[c * 16 + e4 * 4 + k] * fmaf(__uint_as_float(dv[e4 * 4 + k]), a.scale, -dl[k]);
-                    dd[e4 * 2] = pack_bf16x2(ds[0], ds[1]);
-                    dd[e4 * 2 + 1] = pack_bf16x2(ds[2], ds[3]);
+                    const float* pe = p + c * 16 + e4 * 4;
+                    const float2 s0 = f2_unpack(f2_mul(f2_pack(pe[0], pe[1]), f2_fma(f2_pack_u(dv[e4 * 4 + 0], dv[e4 * 4 + 1]), sc2, f2_pack(d4.x, d4.y))));
+                    const float2 s1 = f2_unpack(f2_mul(f2_pack(pe[2], pe[3]), f2_fma(f2_pack_u(dv[e4 * 4 + 2], dv[e4 * 4 + 3]), sc2, f2_pack(d4.z, d4.w))));
+                    dd[e4 * 2] = pack_bf16x2(s0.x, s0.y);
+                    dd[e4 * 2 + 1] = pack_bf16x2(s1.x, s1.y);
                 }
                 tmem_st8(tdP + lane_off + hf * 64 + c * 8, dd);
             }
@@ -414,7 +414,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
             if (tq < a.T) { l = a.lse[(size_t)pr.bh * a.T + tq] * log2e; d = a.delta[(size_t)pr.bh * a.T + tq] * a.scale; }
             ok = mbar_wait_relaxed(&st_empty[tt & 1], ((tt >> 1) & 1) ^ 1, abort_flag, a.status, 0x6b0) && ok;
             float* tab = sStat + (tt & 1) * (2 * BT);
-            tab[rr] = l; tab[BT + rr] = d;
+            tab[rr] = -l; tab[BT + rr] = -d;
             __syncwarp();
             if (lane == 0) mbar_arrive(&st_full[tt & 1]);
         };
