@@ -179,17 +179,6 @@ DEVINL float gelu_tanh_grad(float x) {
 // 2^x on the special-function unit (inputs here are <= 0 up to rounding, so no range handling is needed)
 DEVINL float ex2_fast(float x) { float y; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
 DEVINL float tanh_fast(float x) { float y; asm("tanh.approx.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
-DEVINL float gelu_fast(float x) {
-    const float k = 0.7978845608028654f;
-    return 0.5f * x * (1.0f + tanh_fast(k * (x + 0.044715f * x * x * x)));
-}
-DEVINL float gelu_grad_fast(float x) {
-    const float k = 0.7978845608028654f;
-    const float x2 = x * x;
-    const float t = tanh_fast(k * x * (1.0f + 0.044715f * x2));
-    return 0.5f * (1.0f + t) + 0.5f * x * (1.0f - t * t) * k * (1.0f + 3.0f * 0.044715f * x2);
-}
-
 // Two fp32 operations in one instruction (each half rounds like the scalar operation, so results do not change): for loops that are bound by
 // the issue of their arithmetic.  The forward attention kernels and the 64-wide backward, measured with it, are not (no change).
 DEVINL uint64_t f2_pack(float lo, float hi) { uint64_t r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi)); return r; }
@@ -198,6 +187,37 @@ DEVINL float2 f2_unpack(uint64_t v) { float2 r; asm("mov.b64 {%0, %1}, %2;" : "=
 DEVINL uint64_t f2_fma(uint64_t a, uint64_t b, uint64_t c) { uint64_t r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c)); return r; }
 DEVINL uint64_t f2_mul(uint64_t a, uint64_t b) { uint64_t r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
 DEVINL uint64_t f2_add(uint64_t a, uint64_t b) { uint64_t r; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
+
+// GELU with the tanh approximation, 0.5 x (1 + tanh(k (x + 0.044715 x^3))), and its derivative, scalar and in pairs.  Both forms evaluate
+// the same operations in the same order, so an element gives the same bits through either.  In the GEMM epilogues, which sit behind a
+// main loop of only 12 k-blocks at K = 768, the pairs took dgrad + dGELU (M=16384 N=3072 K=768) from 95 to 89 us and GELU from 86 to 85.
+constexpr float GELU_K1 = 0.7978845608028654f;                    // k = sqrt(2 / pi)
+constexpr float GELU_K2 = 0.7978845608028654f * 0.044715f;
+DEVINL float gelu_fast(float x) {
+    const float t = tanh_fast(x * fmaf(x * x, GELU_K2, GELU_K1)), h = 0.5f * x;
+    return fmaf(h, t, h);
+}
+DEVINL float gelu_grad_fast(float x) {
+    const float u = x * x;
+    const float t = tanh_fast(x * fmaf(u, GELU_K2, GELU_K1));
+    const float r = x * fmaf(u, 1.5f * GELU_K2, 0.5f * GELU_K1);   // 0.5 x d/dx of the tanh argument
+    return fmaf(r, fmaf(-t, t, 1.0f), fmaf(0.5f, t, 0.5f));
+}
+DEVINL uint64_t gelu_fast2(float2 v) {
+    const uint64_t x = f2_pack(v.x, v.y);
+    const float2 w = f2_unpack(f2_mul(x, f2_fma(f2_mul(x, x), f2_pack(GELU_K2, GELU_K2), f2_pack(GELU_K1, GELU_K1))));
+    const uint64_t h = f2_mul(f2_pack(0.5f, 0.5f), x);
+    return f2_fma(h, f2_pack(tanh_fast(w.x), tanh_fast(w.y)), h);
+}
+DEVINL uint64_t gelu_grad_fast2(float2 v) {
+    const uint64_t x = f2_pack(v.x, v.y), u = f2_mul(x, x);
+    const float2 w = f2_unpack(f2_mul(x, f2_fma(u, f2_pack(GELU_K2, GELU_K2), f2_pack(GELU_K1, GELU_K1))));
+    const float tx = tanh_fast(w.x), ty = tanh_fast(w.y);
+    const uint64_t t = f2_pack(tx, ty), nt = f2_pack(-tx, -ty);
+    const uint64_t r = f2_mul(x, f2_fma(u, f2_pack(1.5f * GELU_K2, 1.5f * GELU_K2), f2_pack(0.5f * GELU_K1, 0.5f * GELU_K1)));
+    return f2_fma(r, f2_fma(nt, t, f2_pack(1.0f, 1.0f)), f2_fma(f2_pack(0.5f, 0.5f), t, f2_pack(0.5f, 0.5f)));
+}
+DEVINL uint32_t pack_bf16x2(uint64_t v) { const float2 f = f2_unpack(v); return pack_bf16x2(f.x, f.y); }
 
 // ----------------------------------------------------------------------------
 // bounded waits

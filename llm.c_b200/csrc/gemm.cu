@@ -71,6 +71,9 @@ DEVINL bool epi_any(int pred) {
     return r != 0;
 }
 
+DEVINL void mul2(float* f, uint64_t g) { const float2 r = f2_unpack(f2_mul(f2_pack(f[0], f[1]), g)); f[0] = r.x; f[1] = r.y; }
+DEVINL void add2(float* f, float x, float y) { const float2 r = f2_unpack(f2_add(f2_pack(f[0], f[1]), f2_pack(x, y))); f[0] = r.x; f[1] = r.y; }
+
 template <int A_MN, int B_MN, int MODE>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
@@ -235,7 +238,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
                             if (col0 + j < g.N) {   // N is a multiple of 8
                                 bf16x8 b = ld128(g.bias + col0 + j);
                                 #pragma unroll
-                                for (int e = 0; e < 8; e++) f[j + e] += __bfloat162float(b[e]);
+                                for (int e = 0; e < 8; e += 2) add2(f + j + e, __bfloat162float(b[e]), __bfloat162float(b[e + 1]));
                             }
                         }
                     }
@@ -253,10 +256,10 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
                         for (int j = 0; j < 4; j++) {
                             const uint4 a = *reinterpret_cast<const uint4*>(rowB + ((j ^ swz) * 16));
                             const float2 a0 = unpack_bf16x2(a.x), a1 = unpack_bf16x2(a.y), a2 = unpack_bf16x2(a.z), a3 = unpack_bf16x2(a.w);
-                            f[j*8+0] *= gelu_grad_fast(a0.x); f[j*8+1] *= gelu_grad_fast(a0.y);
-                            f[j*8+2] *= gelu_grad_fast(a1.x); f[j*8+3] *= gelu_grad_fast(a1.y);
-                            f[j*8+4] *= gelu_grad_fast(a2.x); f[j*8+5] *= gelu_grad_fast(a2.y);
-                            f[j*8+6] *= gelu_grad_fast(a3.x); f[j*8+7] *= gelu_grad_fast(a3.y);
+                            mul2(f + j * 8 + 0, gelu_grad_fast2(a0));
+                            mul2(f + j * 8 + 2, gelu_grad_fast2(a1));
+                            mul2(f + j * 8 + 4, gelu_grad_fast2(a2));
+                            mul2(f + j * 8 + 6, gelu_grad_fast2(a3));
                         }
                     }
                     group_barrier(grp);      // output buffer is free; (DGELU) everybody has read the pre-activation chunk
@@ -272,8 +275,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
                             pre.z = pack_bf16x2(f[j*8+4], f[j*8+5]); pre.w = pack_bf16x2(f[j*8+6], f[j*8+7]);
                             // GELU of the bf16-rounded pre-activation: a later recompute from the stored value gives the same bits
                             const float2 r0 = unpack_bf16x2(pre.x), r1 = unpack_bf16x2(pre.y), r2 = unpack_bf16x2(pre.z), r3 = unpack_bf16x2(pre.w);
-                            post.x = pack_bf16x2(gelu_fast(r0.x), gelu_fast(r0.y)); post.y = pack_bf16x2(gelu_fast(r1.x), gelu_fast(r1.y));
-                            post.z = pack_bf16x2(gelu_fast(r2.x), gelu_fast(r2.y)); post.w = pack_bf16x2(gelu_fast(r3.x), gelu_fast(r3.y));
+                            post.x = pack_bf16x2(gelu_fast2(r0)); post.y = pack_bf16x2(gelu_fast2(r1));
+                            post.z = pack_bf16x2(gelu_fast2(r2)); post.w = pack_bf16x2(gelu_fast2(r3));
                             *reinterpret_cast<uint4*>(rowB + ((j ^ swz) * 16)) = pre;
                             *reinterpret_cast<uint4*>(rowA + ((j ^ swz) * 16)) = post;
                         }

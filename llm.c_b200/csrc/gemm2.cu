@@ -100,6 +100,9 @@ DEVINL void umma_commit_2sm(uint64_t* bar) {
                  ::"r"(smem_u32(bar)), "h"((uint16_t)3) : "memory");
 }
 
+DEVINL void mul2(float* f, uint64_t g) { const float2 r = f2_unpack(f2_mul(f2_pack(f[0], f[1]), g)); f[0] = r.x; f[1] = r.y; }
+DEVINL void add2(float* f, float x, float y) { const float2 r = f2_unpack(f2_add(f2_pack(f[0], f[1]), f2_pack(x, y))); f[0] = r.x; f[1] = r.y; }
+
 template <int A_MN, int B_MN, int MODE>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
 gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
@@ -366,7 +369,7 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
                         if (col0 + j < g.N) {
                             bf16x8 b = ld128(g.bias + col0 + j);
                             #pragma unroll
-                            for (int e = 0; e < 8; e++) f[j + e] += __bfloat162float(b[e]);
+                            for (int e = 0; e < 8; e += 2) add2(f + j + e, __bfloat162float(b[e]), __bfloat162float(b[e + 1]));
                         }
                     }
                 }
@@ -381,10 +384,10 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
                     for (int j = 0; j < 4; j++) {
                         const uint4 a = *reinterpret_cast<const uint4*>(aux_row + ((j ^ swz) * 16));
                         const float2 a0 = unpack_bf16x2(a.x), a1 = unpack_bf16x2(a.y), a2 = unpack_bf16x2(a.z), a3 = unpack_bf16x2(a.w);
-                        f[j*8+0] *= gelu_grad_fast(a0.x); f[j*8+1] *= gelu_grad_fast(a0.y);
-                        f[j*8+2] *= gelu_grad_fast(a1.x); f[j*8+3] *= gelu_grad_fast(a1.y);
-                        f[j*8+4] *= gelu_grad_fast(a2.x); f[j*8+5] *= gelu_grad_fast(a2.y);
-                        f[j*8+6] *= gelu_grad_fast(a3.x); f[j*8+7] *= gelu_grad_fast(a3.y);
+                        mul2(f + j * 8 + 0, gelu_grad_fast2(a0));
+                        mul2(f + j * 8 + 2, gelu_grad_fast2(a1));
+                        mul2(f + j * 8 + 4, gelu_grad_fast2(a2));
+                        mul2(f + j * 8 + 6, gelu_grad_fast2(a3));
                     }
                     __syncwarp();            // every lane has read its row of the pre-activation box
                     if (lane == 0) {
@@ -413,8 +416,8 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
                         // the activation is computed from the rounded pre-activation, so a later recomputation from the stored
                         // tensor gives the same bits
                         const float2 r0 = unpack_bf16x2(pre_q[j].x), r1 = unpack_bf16x2(pre_q[j].y), r2 = unpack_bf16x2(pre_q[j].z), r3 = unpack_bf16x2(pre_q[j].w);
-                        out_q[j].x = pack_bf16x2(gelu_fast(r0.x), gelu_fast(r0.y)); out_q[j].y = pack_bf16x2(gelu_fast(r1.x), gelu_fast(r1.y));
-                        out_q[j].z = pack_bf16x2(gelu_fast(r2.x), gelu_fast(r2.y)); out_q[j].w = pack_bf16x2(gelu_fast(r3.x), gelu_fast(r3.y));
+                        out_q[j].x = pack_bf16x2(gelu_fast2(r0)); out_q[j].y = pack_bf16x2(gelu_fast2(r1));
+                        out_q[j].z = pack_bf16x2(gelu_fast2(r2)); out_q[j].w = pack_bf16x2(gelu_fast2(r3));
                     }
                     if (lane == 0) tma_store_wait_read<1>();
                     __syncwarp();
