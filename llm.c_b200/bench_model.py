@@ -112,6 +112,7 @@ def main(argv=None):
 
     if a.ops:
         records = []
+        m.use_graphs = False                 # every operator call has to pass through its wrapper
         saved = _instrument(records)
         try:
             for i in range(2):

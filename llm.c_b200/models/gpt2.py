@@ -20,6 +20,7 @@ from dataclasses import dataclass
 import torch
 
 from .. import ops
+from .step_graphs import StepGraphs
 
 
 class _Range:
@@ -146,6 +147,8 @@ class GPT:
         self.mean_loss = None          # device scalar after a backward with targets
         self.grad_hook = None
         # set by a communication backend whose all-gather may still be in flight when forward starts (parallel/p2p.py)
+        self.step_graphs = StepGraphs()
+        self.use_graphs = True          # replay small micro-steps from CUDA graphs (off: launch every kernel, for per-operator measurements)
         self.param_sync = None          # called as grad_hook(layer or -1 for the embeddings/final LN) on the last micro-step
 
     # ------------------------------------------------------------------ parameters
@@ -215,6 +218,7 @@ class GPT:
         self.targets = torch.zeros(B, T, dtype=torch.int32, device=dev)
         self.mean_loss = torch.zeros(1, dtype=f32, device=dev)
         self.act_shape = (B, T)
+        self.step_graphs.clear()
 
     def activation_bytes(self):
         return sum(t.numel() * t.element_size() for t in self.acts.values()) if self.acts else 0
@@ -224,15 +228,26 @@ class GPT:
         """Runs the network on tokens (B, T) int32.  With targets, the per-token losses are accumulated into
         ``acts['losses']`` and (if write_dlogits) the logits buffer is turned into dlogits scaled by
         1/(B*T*grad_accum_steps), ready for ``backward``.  Returns nothing; see ``loss()``."""
-        cfg, p = self.cfg, self.params
+        cfg = self.cfg
         B, T = tokens.shape
         if T > cfg.max_seq_len:
             raise ValueError("sequence length %d exceeds the model's maximum %d" % (T, cfg.max_seq_len))
         self.allocate_activations(B, T)
-        a = self.acts
-        L, C, NH = cfg.num_layers, cfg.channels, cfg.num_heads
         if tokens.data_ptr() != self.inputs.data_ptr():
             self.inputs.copy_(tokens, non_blocking=True)
+        if targets is not None and targets.data_ptr() != self.targets.data_ptr():
+            self.targets.copy_(targets, non_blocking=True)
+        dloss = None if targets is None else 1.0 / (B * T * grad_accum_steps)
+        launch = lambda: self._forward(B, T, dloss, micro_step > 0, write_dlogits)
+        if self.param_sync is not None:
+            launch()
+        else:
+            self.step_graphs.run(self, B * T, ("forward", self.recompute, dloss, micro_step > 0, write_dlogits), launch)
+
+    def _forward(self, B, T, dloss, accumulate_loss, write_dlogits):
+        """The launches of ``forward``, on the model's own buffers only."""
+        cfg, p, a = self.cfg, self.params, self.acts
+        L, C, NH = cfg.num_layers, cfg.channels, cfg.num_heads
         nvtx = self.device.type == "cuda"
         ps = self.param_sync
         if ps is not None:
@@ -259,12 +274,9 @@ class GPT:
                 ops.fused_residual_forward(a["residual3"][l], a["lnf"], a["lnf_mean"], a["lnf_rstd"], a["residual2"][l],
                                            a["scratch_btc"], p["lnfw"], p["lnfb"])
         ops.matmul_forward(a["logits"], a["lnf"], p["wte"], None)
-        if targets is not None:
-            if targets.data_ptr() != self.targets.data_ptr():
-                self.targets.copy_(targets, non_blocking=True)
-            dloss = 1.0 / (B * T * grad_accum_steps)
+        if dloss is not None:
             ops.fused_classifier(a["logits"], a["losses"], self.targets.view(-1), dloss, cfg.vocab_size,
-                                 write_dlogits=write_dlogits, accumulate_loss=(micro_step > 0))
+                                 write_dlogits=write_dlogits, accumulate_loss=accumulate_loss)
 
     def loss(self, grad_accum_steps=1):
         """Mean loss over the micro-steps accumulated so far, as a device scalar tensor (no synchronisation)."""
@@ -282,13 +294,21 @@ class GPT:
         """Backward pass of the last ``forward(tokens, targets)``.  Gradients are overwritten when micro_step == 0
         and added to otherwise.  On the last micro-step ``grad_hook(l)`` fires as soon as layer l's gradients are
         final (the ZeRO / data-parallel layer starts its reduction there, overlapping the rest of backward)."""
-        cfg, p = self.cfg, self.params
         self.allocate_grads()
-        g, a = self.grads, self.acts
         B, T = self.act_shape
+        hook = self.grad_hook if last_micro_step else None
+        launch = lambda: self._backward(B, T, micro_step, hook)
+        if hook is not None:
+            launch()                    # the hook runs on the host between the launches
+        else:
+            self.step_graphs.run(self, B * T, ("backward", self.recompute, micro_step), launch)
+
+    def _backward(self, B, T, micro_step, hook):
+        """The launches of ``backward``, on the model's own buffers only."""
+        cfg, p = self.cfg, self.params
+        g, a = self.grads, self.acts
         L, C, NH = cfg.num_layers, cfg.channels, cfg.num_heads
         acc = micro_step > 0
-        hook = self.grad_hook if last_micro_step else None
         dres, dl_btc, dl_bt4c, dqkv = a["dresidual"], a["scratch_btc"], a["scratch_bt4c"], a["dqkv"]
         dlogits = a["logits"]
 

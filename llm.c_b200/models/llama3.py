@@ -22,6 +22,7 @@ import torch
 
 from .. import ops
 from .gpt2 import _Range
+from .step_graphs import StepGraphs
 
 PARAM_NAMES = ["wte", "ln1w", "qkvw", "attprojw", "ln2w", "fc12w", "fcprojw", "lnfw", "lmhead"]
 # tensors that receive weight decay: everything two-dimensional (train_llama3.py:444-456 of the reference)
@@ -171,6 +172,8 @@ class Llama:
         self.grad_hook = None
         # set by a communication backend whose all-gather may still be in flight when forward starts (parallel/p2p.py)
         self.param_sync = None
+        self.step_graphs = StepGraphs()
+        self.use_graphs = True          # replay small micro-steps from CUDA graphs (off: launch every kernel, for per-operator measurements)
         self.freqs = rope_table(cfg).to(self.device)
 
     # ------------------------------------------------------------------ parameters
@@ -244,6 +247,7 @@ class Llama:
         self.targets = torch.zeros(B, T, dtype=torch.int32, device=dev)
         self.mean_loss = torch.zeros(1, dtype=f32, device=dev)
         self.act_shape = (B, T)
+        self.step_graphs.clear()
 
     def activation_bytes(self):
         return sum(t.numel() * t.element_size() for t in self.acts.values()) if self.acts else 0
@@ -252,15 +256,26 @@ class Llama:
     def forward(self, tokens, targets=None, grad_accum_steps=1, micro_step=0, write_dlogits=True):
         """Same contract as ``GPT.forward``: with targets the per-token losses are accumulated into ``acts['losses']`` and the
         logits buffer is turned into dlogits scaled by 1/(B*T*grad_accum_steps)."""
-        cfg, p = self.cfg, self.params
+        cfg = self.cfg
         B, T = tokens.shape
         if T > cfg.max_seq_len:
             raise ValueError("sequence length %d exceeds the model's maximum %d" % (T, cfg.max_seq_len))
         self.allocate_activations(B, T)
-        a = self.acts
-        L, NH, NKV, eps = cfg.num_layers, cfg.num_heads, cfg.num_kv_heads, cfg.norm_eps
         if tokens.data_ptr() != self.inputs.data_ptr():
             self.inputs.copy_(tokens, non_blocking=True)
+        if targets is not None and targets.data_ptr() != self.targets.data_ptr():
+            self.targets.copy_(targets, non_blocking=True)
+        dloss = None if targets is None else 1.0 / (B * T * grad_accum_steps)
+        launch = lambda: self._forward(B, T, dloss, micro_step > 0, write_dlogits)
+        if self.param_sync is not None:
+            launch()
+        else:
+            self.step_graphs.run(self, B * T, ("forward", self.recompute, dloss, micro_step > 0, write_dlogits), launch)
+
+    def _forward(self, B, T, dloss, accumulate_loss, write_dlogits):
+        """The launches of ``forward``, on the model's own buffers only."""
+        cfg, p, a = self.cfg, self.params, self.acts
+        L, NH, NKV, eps = cfg.num_layers, cfg.num_heads, cfg.num_kv_heads, cfg.norm_eps
         nvtx = self.device.type == "cuda"
         ps = self.param_sync
         if ps is not None:
@@ -289,12 +304,9 @@ class Llama:
                 ops.rmsnorm_fused_residual_forward(a["residual3"][l], a["lnf"], a["lnf_rstd"], a["residual2"][l], a["scratch_btc"],
                                                    p["lnfw"], eps)
         ops.matmul_forward(a["logits"], a["lnf"], p["lmhead"], None)
-        if targets is not None:
-            if targets.data_ptr() != self.targets.data_ptr():
-                self.targets.copy_(targets, non_blocking=True)
-            dloss = 1.0 / (B * T * grad_accum_steps)
+        if dloss is not None:
             ops.fused_classifier(a["logits"], a["losses"], self.targets.view(-1), dloss, cfg.vocab_size,
-                                 write_dlogits=write_dlogits, accumulate_loss=(micro_step > 0))
+                                 write_dlogits=write_dlogits, accumulate_loss=accumulate_loss)
 
     def loss(self, grad_accum_steps=1):
         B, T = self.act_shape
@@ -309,13 +321,21 @@ class Llama:
     # ------------------------------------------------------------------ backward
     def backward(self, micro_step=0, last_micro_step=True):
         """Backward pass of the last ``forward(tokens, targets)``; same contract as ``GPT.backward``."""
-        cfg, p = self.cfg, self.params
         self.allocate_grads()
-        g, a = self.grads, self.acts
         B, T = self.act_shape
+        hook = self.grad_hook if last_micro_step else None
+        launch = lambda: self._backward(B, T, micro_step, hook)
+        if hook is not None:
+            launch()                    # the hook runs on the host between the launches
+        else:
+            self.step_graphs.run(self, B * T, ("backward", self.recompute, micro_step), launch)
+
+    def _backward(self, B, T, micro_step, hook):
+        """The launches of ``backward``, on the model's own buffers only."""
+        cfg, p = self.cfg, self.params
+        g, a = self.grads, self.acts
         L, C, NH, NKV, eps = cfg.num_layers, cfg.channels, cfg.num_heads, cfg.num_kv_heads, cfg.norm_eps
         acc = micro_step > 0
-        hook = self.grad_hook if last_micro_step else None
         dres, dl_btc, dh, dfc12, dqkv, dqkv_raw = a["dresidual"], a["scratch_btc"], a["dh"], a["dfc12"], a["dqkv"], a["qkv_raw"]
         dlogits = a["logits"]
 

@@ -21,6 +21,12 @@ def launch_count():
     return _launches
 
 
+def count_launches(n):
+    """Adds launches issued without a launcher call (a replayed graph)."""
+    global _launches
+    _launches += n
+
+
 def _stream():
     return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
 
@@ -45,6 +51,13 @@ class _Scratch:
 
 
 _scratch = _Scratch()
+
+
+def scratch_buffers():
+    """The scratch buffers in use now; whoever holds their addresses beyond a call keeps the tensors too."""
+    return list(_scratch.bufs.values())
+
+
 _sm_count = {}
 
 

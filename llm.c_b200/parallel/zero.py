@@ -174,7 +174,8 @@ class ShardedAdamW:
             for l in range(L):
                 key = l if L > 1 else -1
                 self.layer_slices.setdefault(key, []).append((off + l * per, per))
-        model.grad_hook = self.on_layer_grads_ready
+        if self.N > 1:
+            model.grad_hook = self.on_layer_grads_ready
 
     # ---- gradient reduction, overlapped with backward
     def on_layer_grads_ready(self, layer):
