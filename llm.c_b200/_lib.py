@@ -78,7 +78,7 @@ def cuda():
         "llmc_swiglu_bwd": (I, [P, P, P, L, I, S]),
         "llmc_rope_cache": (I, [P, P, P, P, P, I, I, I, I, I, I, I, I, P, S]),
         "llmc_skinny_gemm": (I, [P, P, P, I, I, I, I, I, I, S]),
-        "llmc_stream_gemm": (I, [P, P, P, P, I, I, I, I, I, I, S]),
+        "llmc_stream_gemm": (I, [P, P, P, P, I, I, I, I, I, I, I, S]),
         "llmc_stream_gemm_swiglu": (I, [P, P, P, I, I, I, I, I, I, S]),
         "llmc_cached_attention": (I, [P, P, P, P, I, I, I, I, I, I, I, P, P, S]),
         "llmc_cached_attention_workspace": (L, [I, I, I, I, I, I]),

@@ -1,7 +1,8 @@
-// Products with few rows: out (M, N) = x (M, K) . w (N, K)^T (+ bias), M <= 128, and the same with SwiGLU on top.  These are the
-// products of decoding steps and short prompts.  They are bound by streaming the weights once, so the roles of the tcgen05 operands
-// are swapped: 128 weight rows are the M side of the MMA and the activation rows, padded to a multiple of 16, its N side (a 128-row
-// activation tile would be padding, and 256 weight rows per tile leave most SMs without work: 16 tiles for N = 4096).
+// Products with few tiles: out (M, N) = x (M, K) . w (N, K)^T (+ bias), x . w (K, N), and the first with SwiGLU on top.  These are the products
+// of decoding steps, short prompts and small training batches.
+// The roles of the tcgen05 operands are swapped: 128 weight rows are the M side of the MMA and up to 256 activation rows, padded to a
+// multiple of 16, its N side.  A product of at most 128 rows then has no padded rows, and weight tiles of 128 instead of 256 columns
+// leave fewer SMs without work.
 //
 // K is split over the CTAs of a cluster (1, 2, 4 or 8 of them), so that a product with few weight tiles still has enough CTAs in
 // flight to reach the memory rate.  Every CTA accumulates its K slice in TMEM, puts the fp32 partial tile into its own shared memory,
@@ -14,7 +15,8 @@
 // Alone, after an L2 flush, the 128 x 256 tiles of the training GEMM in brackets: 32 x 4096 x 14336 (M x N x K) 36 us (101),
 // 32 x 6144 x 4096 23 us (38), 32 x 28672 x 4096 58 us (69), 100 x 2048 x 7168 23 us (52).  Inside a replayed decoding step (4 rows, 4 layers
 // of 2048 channels, LM head of 128256 rows) this kernel takes the step to 277 us; a weight-streaming kernel on warp-level MMAs with the same
-// early launch and prefetch, used for the products of at most 8 rows, left it at 290 us.
+// early launch and prefetch, used for the products of at most 8 rows, left it at 290 us.  More rows: 256 x 768 x 50304 (an input gradient)
+// 60 us (291), 777 x 2048 x 7168 37 us (53), 256 x 768 x 3072 18 us (27).
 //
 // Warps of a CTA: 0 TMA producer, 1 MMA issuer, 2-5 epilogue.  Two CTAs fit an SM.
 #include "common.cuh"
@@ -22,23 +24,27 @@
 
 namespace {
 
-constexpr int WR = 128;                       // weight rows per tile
+constexpr int WR = 128;                       // weight rows (output columns) per tile
 constexpr int BK = 64;                        // K elements per stage: one 128-byte swizzled row
 constexpr int W_BYTES = WR * BK * 2;          // 16 KB
+constexpr int MAX_NB = 256;                   // activation rows per tile
 constexpr int MAX_STAGES = 6;
-constexpr int SMEM_BUDGET = 112 * 1024;       // two CTAs per SM
+constexpr int SMEM_TWO = 112 * 1024;          // two CTAs per SM (at most 128 activation rows: 16 to 32 KB per stage)
+constexpr int SMEM_ONE = 224 * 1024;          // one CTA per SM (up to 48 KB per stage)
 constexpr int THREADS = 192;
 constexpr int PREFETCH_BYTES = 1024;          // of each weight row: 296 resident CTAs x 128 KB stay well inside L2
-constexpr int MAX_M = 128;
+constexpr int MAX_SPLIT = 8;
+
+enum Mode : int { STORE = 0, SWIGLU = 1 };
 
 struct Args {
     bf16* out;
-    const bf16* bias;          // N entries or null
+    const bf16* bias;          // N entries or null (STORE)
     const bf16* w;             // for the prefetch
     int M, N, K, ldo, ldw;
-    int nb;                    // activation rows of a tile: M rounded up to 16
+    int nb;                    // activation rows of a tile, a multiple of 16
     int stages, num_kb, kb_per_split;
-    int vec_out;               // out rows start on 4-byte boundaries
+    int vec_out;               // rows of out start on 8-byte boundaries
     unsigned int* status;
 };
 
@@ -48,19 +54,29 @@ DEVINL void cluster_sync() {
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
-DEVINL float2 ld_peer2(uint32_t addr, uint32_t rank) {
-    uint32_t ra; float2 v;
+DEVINL float4 ld_peer4(uint32_t addr, uint32_t rank) {
+    uint32_t ra; float4 v;
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(addr), "r"(rank));
-    asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(ra) : "memory");
+    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(ra) : "memory");
     return v;
+}
+// sum over the cluster's partial tiles in slice order; all loads are on their way before the first is added
+DEVINL void sum_peers(float (&f)[4], uint32_t addr, uint32_t S) {
+    float4 p[MAX_SPLIT];
+    #pragma unroll
+    for (uint32_t s = 0; s < MAX_SPLIT; s++) if (s < S) p[s] = ld_peer4(addr, s);
+    f[0] = p[0].x; f[1] = p[0].y; f[2] = p[0].z; f[3] = p[0].w;
+    #pragma unroll
+    for (uint32_t s = 1; s < MAX_SPLIT; s++) if (s < S) { f[0] += p[s].x; f[1] += p[s].y; f[2] += p[s].z; f[3] += p[s].w; }
 }
 DEVINL void prefetch_l2(const void* p, uint32_t bytes) {
     asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
 }
 
+// W_MN: the weights are stored (K, N) (an input gradient); otherwise (N, K).
 // SWIGLU: w holds 2 N rows; tile t covers rows 64 t .. of the first half and the same rows of the second half, and
-// out = first * silu(second).  Otherwise tile t covers rows 128 t ..
-template <bool SWIGLU>
+// out = first * silu(second).  Otherwise tile t covers output columns 128 t ..
+template <int MODE, bool W_MN>
 __global__ void __launch_bounds__(THREADS, 2)
 stream_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX, const Args g) {
     extern __shared__ uint8_t smem_raw[];
@@ -75,10 +91,11 @@ stream_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t S = cluster_size(), rank = cluster_rank();
     const int tile = blockIdx.x / S;
-    constexpr int ROWS = SWIGLU ? WR / 2 : WR;   // output columns of a tile
-    const int n0 = tile * ROWS;
+    constexpr int COLS = MODE == SWIGLU ? WR / 2 : WR;   // output columns of a tile
+    const int n0 = tile * COLS;
+    const int m0 = blockIdx.y * g.nb;
     const int kb0 = rank * g.kb_per_split, kb1 = min(g.num_kb, kb0 + g.kb_per_split);
-    const uint32_t tmem_cols = g.nb <= 32 ? 32 : g.nb <= 64 ? 64 : 128;
+    const uint32_t tmem_cols = g.nb <= 32 ? 32 : g.nb <= 64 ? 64 : g.nb <= 128 ? 128 : 256;
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < g.stages; s++) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
@@ -88,12 +105,21 @@ stream_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
         tma_prefetch_desc(&tmW); tma_prefetch_desc(&tmX);
     }
     if (warp == 1) { tmem_alloc(tmem_slot, tmem_cols); tmem_relinquish(); }
-    if (warp >= 2 && kb0 < kb1) {
+    if (warp >= 2 && kb0 < kb1 && blockIdx.y == 0) {
         const int r = threadIdx.x - 64;
-        const int row = SWIGLU ? (r < 64 ? n0 + r : g.N + n0 + r - 64) : n0 + r;
-        const bool in = SWIGLU ? n0 + (r & 63) < g.N : row < g.N;
-        const int bytes = min(min(kb1 * BK, g.K) - kb0 * BK, PREFETCH_BYTES / 2) * 2;      // K is a multiple of 8: whole 16-byte units
-        if (in) prefetch_l2(g.w + (size_t)row * g.ldw + kb0 * BK, bytes);
+        if (W_MN) {
+            // rows of w are K: the tile's columns of the slice's first rows
+            const uint32_t bytes = 2 * min(WR, g.N - n0);      // N is a multiple of 8: whole 16-byte units
+            for (int i = 0; i < PREFETCH_BYTES / (2 * WR); i++) {
+                const int k = kb0 * BK + i * 128 + r;
+                if (k < min(kb1 * BK, g.K)) prefetch_l2(g.w + (size_t)k * g.ldw + n0, bytes);
+            }
+        } else {
+            const int row = MODE == SWIGLU ? (r < 64 ? n0 + r : g.N + n0 + r - 64) : n0 + r;
+            const bool in = MODE == SWIGLU ? n0 + (r & 63) < g.N : row < g.N;
+            const int bytes = min(min(kb1 * BK, g.K) - kb0 * BK, PREFETCH_BYTES / 2) * 2;      // K is a multiple of 8: whole 16-byte units
+            if (in) prefetch_l2(g.w + (size_t)row * g.ldw + kb0 * BK, bytes);
+        }
     }
     tc_fence_before();
     __syncthreads();
@@ -109,29 +135,33 @@ stream_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
                 if (!mbar_wait_relaxed(&empty[st], ((it / g.stages) & 1) ^ 1, abort_flag, g.status, 0x900)) break;
                 uint8_t* dst = smem + st * stage_bytes;
                 mbar_expect_tx(&full[st], stage_bytes);
-                if (SWIGLU) {
+                if (W_MN) {
+                    tma_load_2d(dst, &tmW, &full[st], n0, kb * BK);                                   // boxes {64 n, 64 k}
+                    tma_load_2d(dst + W_BYTES / 2, &tmW, &full[st], n0 + 64, kb * BK);
+                } else if (MODE == SWIGLU) {
                     tma_load_2d(dst, &tmW, &full[st], kb * BK, n0);                                   // boxes {64 k, 64 rows}
                     tma_load_2d(dst + W_BYTES / 2, &tmW, &full[st], kb * BK, g.N + n0);
                 } else {
                     tma_load_2d(dst, &tmW, &full[st], kb * BK, n0);                                   // box {64 k, 128 rows}
                 }
-                tma_load_2d(dst + W_BYTES, &tmX, &full[st], kb * BK, 0);                              // box {64 k, nb rows}
+                tma_load_2d(dst + W_BYTES, &tmX, &full[st], kb * BK, m0);                             // box {64 k, nb rows}
             }
         }
     } else if (warp == 1) {
         const bool leader = elect_one();
-        const uint32_t idesc = umma_idesc_bf16(WR, 0, 0, 0) | ((uint32_t)(g.nb >> 3) << 17);
+        const uint32_t idesc = umma_idesc_bf16(WR, 0, W_MN, 0) | ((uint32_t)(g.nb >> 3) << 17);
         bool ok = true;
         for (int kb = kb0; kb < kb1 && ok; kb++) {
             const int it = kb - kb0, st = it % g.stages;
             ok = __all_sync(0xffffffffu, mbar_wait_relaxed(&full[st], (it / g.stages) & 1, abort_flag, g.status, 0x910)) != 0;
             if (!ok) break;
             tc_fence_after();
-            const uint64_t dw = umma_desc_sw128(smem_u32(smem + st * stage_bytes), 16, 1024);
+            const uint64_t dw = umma_desc_sw128(smem_u32(smem + st * stage_bytes), W_MN ? BK * 128 : 16, 1024);
             const uint64_t dx = umma_desc_sw128(smem_u32(smem + st * stage_bytes + W_BYTES), 16, 1024);
             if (leader) {
+                // 16 K elements: 32 bytes along a K-major row, 16 rows of 128 bytes of an N-major tile
                 #pragma unroll
-                for (int kk = 0; kk < BK / 16; kk++) umma_ss(tmem_base, dw + 2 * kk, dx + 2 * kk, idesc, (it | kk) > 0);
+                for (int kk = 0; kk < BK / 16; kk++) umma_ss(tmem_base, dw + (W_MN ? 128 : 2) * kk, dx + 2 * kk, idesc, (it | kk) > 0);
                 umma_commit(&empty[st]);
                 if (kb == kb1 - 1) umma_commit(acc_full);
             }
@@ -158,36 +188,37 @@ stream_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
     __syncwarp();
     cluster_sync();                                           // every partial tile of the cluster is in place
     if (warp >= 2) {
-        constexpr int PAIRS = ROWS / 2, GROUPS = 128 / PAIRS;           // column pairs of a tile; rows handled side by side
+        // four adjacent columns per thread; the rows are dealt to the CTAs of the cluster
+        constexpr int QUADS = COLS / 4, GROUPS = 128 / QUADS;
         const int tid = threadIdx.x - 64;
-        const int pi = tid % PAIRS, grp = tid / PAIRS;
-        const int n = n0 + 2 * pi;
-        const uint32_t base = smem_u32(smem) + pi * 8;
-        float b0 = 0.f, b1 = 0.f;
-        if (!SWIGLU && g.bias != nullptr) {
-            if (n < g.N) b0 = __bfloat162float(g.bias[n]);
-            if (n + 1 < g.N) b1 = __bfloat162float(g.bias[n + 1]);
+        const int qd = tid % QUADS, grp = tid / QUADS;
+        const int n = n0 + 4 * qd;
+        const uint32_t base = smem_u32(smem) + qd * 16;
+        const int rows = min(g.nb, g.M - m0);
+        float bias[4] = {0.f, 0.f, 0.f, 0.f};
+        if (MODE == STORE && g.bias != nullptr) {
+            #pragma unroll
+            for (int e = 0; e < 4; e++) if (n + e < g.N) bias[e] = __bfloat162float(g.bias[n + e]);
         }
-        for (int m = (int)rank * GROUPS + grp; m < g.M; m += (int)S * GROUPS) {
-            float2 v = make_float2(0.f, 0.f), u = make_float2(0.f, 0.f);
-            for (uint32_t s = 0; s < S; s++) {
-                const float2 p = ld_peer2(base + m * (WR * 4), s);
-                v.x += p.x; v.y += p.y;
-                if (SWIGLU) {
-                    const float2 p2 = ld_peer2(base + m * (WR * 4) + (WR / 2) * 4, s);
-                    u.x += p2.x; u.y += p2.y;
-                }
-            }
-            if (SWIGLU) {
-                v.x *= u.x / (1.0f + __expf(-u.x));
-                v.y *= u.y / (1.0f + __expf(-u.y));
-            } else { v.x += b0; v.y += b1; }
-            bf16* o = g.out + (size_t)m * g.ldo + n;
-            if (n + 1 < g.N && g.vec_out) {
-                *reinterpret_cast<uint32_t*>(o) = pack_bf16x2(v.x, v.y);
+        const bool vec = g.vec_out && n + 3 < g.N;
+        for (int m = (int)rank * GROUPS + grp; m < rows; m += (int)S * GROUPS) {
+            const size_t at = (size_t)(m0 + m) * g.ldo + n;
+            float f[4];
+            sum_peers(f, base + m * (WR * 4), S);
+            if (MODE == SWIGLU) {
+                float u[4];
+                sum_peers(u, base + m * (WR * 4) + (WR / 2) * 4, S);
+                #pragma unroll
+                for (int e = 0; e < 4; e++) f[e] *= u[e] / (1.0f + __expf(-u[e]));
             } else {
-                if (n < g.N) o[0] = __float2bfloat16_rn(v.x);
-                if (n + 1 < g.N) o[1] = __float2bfloat16_rn(v.y);
+                #pragma unroll
+                for (int e = 0; e < 4; e++) f[e] += bias[e];
+            }
+            if (vec) {
+                *reinterpret_cast<uint2*>(g.out + at) = make_uint2(pack_bf16x2(f[0], f[1]), pack_bf16x2(f[2], f[3]));
+            } else {
+                #pragma unroll
+                for (int e = 0; e < 4; e++) if (n + e < g.N) g.out[at + e] = __float2bfloat16_rn(f[e]);
             }
         }
     }
@@ -197,30 +228,37 @@ stream_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
     if (warp == 1) tmem_dealloc(tmem_base, tmem_cols);
 }
 
-// CTAs per weight tile: as many as keep all of them resident at once (two per SM) and leave each at least four K blocks
-int pick_split(int tiles, int num_kb, int sms) {
+// CTAs per weight tile: as many as are resident at once and have some K blocks each; the wider the tile, the more blocks a slice must have to
+// be worth its share of the reduction.  A cluster lives in one GPC, so an eighth of the SMs is not counted on: 36 clusters of 4 on 148 SMs ran
+// in two waves.
+int pick_split(int tiles, int num_kb, int nb, int sms) {
+    const int slots = (nb <= 128 ? 2 : 1) * (sms * 7 / 8), min_kb = nb <= 128 ? 4 : 8;
     int s = 1;
-    while (s < 8 && tiles * s * 2 <= 2 * sms && num_kb >= s * 2 * 4) s *= 2;
+    while (s < MAX_SPLIT && tiles * s * 2 <= slots && num_kb >= s * 2 * min_kb) s *= 2;
     return s;
 }
 
-template <bool SWIGLU>
+template <int MODE, bool W_MN>
 int launch_stream(bf16* out, const bf16* x, const bf16* w, const bf16* bias, int M, int N, int K, int ldx, int ldw, int ldo, cudaStream_t stream) {
-    if (M <= 0 || M > MAX_M || N <= 0 || K <= 0 || (K % 8) || (ldx % 8) || (ldw % 8) || ldx < K || ldw < K || ldo < N) return -1;
+    if (M <= 0 || N <= 0 || K <= 0 || (K % 8) || (ldx % 8) || (ldw % 8) || ldx < K || ldw < (W_MN ? N : K) || ldo < N) return -1;
+    if (W_MN && (N % 8)) return -1;
     Args g;
     g.out = out; g.bias = bias; g.w = w; g.M = M; g.N = N; g.K = K; g.ldo = ldo; g.ldw = ldw;
-    g.nb = (M + 15) & ~15;
+    const int mtiles = CEIL_DIV(M, MAX_NB);
+    g.nb = (CEIL_DIV(M, mtiles) + 15) & ~15;             // M spread evenly over its tiles
     g.num_kb = CEIL_DIV(K, BK);
     const int stage_bytes = W_BYTES + g.nb * (BK * 2);
-    g.stages = (SMEM_BUDGET - 2048) / stage_bytes;
+    const bool two = g.nb <= 128;
+    g.stages = ((two ? SMEM_TWO : SMEM_ONE) - 2048) / stage_bytes;
     if (g.stages > MAX_STAGES) g.stages = MAX_STAGES;
-    g.vec_out = (ldo % 2 == 0) && (reinterpret_cast<uintptr_t>(out) & 3) == 0;
+    g.vec_out = (ldo % 4 == 0) && (reinterpret_cast<uintptr_t>(out) & 7) == 0;
     g.status = llmc_status_ptr();
     CUtensorMap tmW, tmX;
     {
-        uint64_t dims[2] = {(uint64_t)K, (uint64_t)(SWIGLU ? 2 * (uint64_t)N : (uint64_t)N)};
+        uint64_t dims[2] = {(uint64_t)K, (uint64_t)(MODE == SWIGLU ? 2 * (uint64_t)N : (uint64_t)N)};
+        uint32_t box[2] = {BK, MODE == SWIGLU ? WR / 2 : WR};
+        if (W_MN) { dims[0] = (uint64_t)N; dims[1] = (uint64_t)K; box[0] = 64; box[1] = BK; }
         uint64_t strides[2] = {2, (uint64_t)ldw * 2};
-        uint32_t box[2] = {BK, SWIGLU ? WR / 2 : WR};
         int rc = llmc_get_tensormap(&tmW, w, 2, 2, dims, strides, box, 3);
         if (rc) return rc;
         uint64_t dimx[2] = {(uint64_t)K, (uint64_t)M};
@@ -230,35 +268,36 @@ int launch_stream(bf16* out, const bf16* x, const bf16* w, const bf16* bias, int
         if (rc) return rc;
     }
     int sms = llmc_device_sm_count(); if (sms <= 0) sms = 148;
-    const int tiles = CEIL_DIV(N, SWIGLU ? WR / 2 : WR);
-    const int S = pick_split(tiles, g.num_kb, sms);
+    const int tiles = CEIL_DIV(N, MODE == SWIGLU ? WR / 2 : WR);
+    const int S = pick_split(tiles * mtiles, g.num_kb, g.nb, sms);
     g.kb_per_split = CEIL_DIV(g.num_kb, S);
     const int smem = g.stages * stage_bytes + 1024 + 256;
     static bool configured = false;
     if (!configured) {
-        CUDA_CHECK(cudaFuncSetAttribute(stream_gemm_kernel<SWIGLU>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BUDGET));
+        CUDA_CHECK(cudaFuncSetAttribute(stream_gemm_kernel<MODE, W_MN>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_ONE));
         configured = true;
     }
-    CUDA_CHECK(launch_pdl(stream_gemm_kernel<SWIGLU>, dim3(tiles * S), dim3(THREADS), smem, stream, S, tmW, tmX, g));
+    CUDA_CHECK(launch_pdl(stream_gemm_kernel<MODE, W_MN>, dim3(tiles * S, mtiles), dim3(THREADS), smem, stream, S, tmW, tmX, g));
     return 0;
 }
 
 }  // namespace
 
-// out (M, N) = x (M, K) . w (N, K)^T (+ bias) for M <= 128; K and the row strides of x and w are multiples of 8 elements.
-extern "C" int llmc_stream_gemm(bf16* out, const bf16* x, const bf16* w, const bf16* bias, int M, int N, int K, int ldx, int ldw, int ldo,
+// out (M, N) = x (M, K) . w (N, K)^T (+ bias), or x . w (K, N) with w_mn.  K, the row strides of x and w and, with w_mn, N are multiples of 8.
+extern "C" int llmc_stream_gemm(bf16* out, const bf16* x, const bf16* w, const bf16* bias, int M, int N, int K, int ldx, int ldw, int ldo, int w_mn,
                                 cudaStream_t stream) {
-    return launch_stream<false>(out, x, w, bias, M, N, K, ldx, ldw, ldo, stream);
+    if (w_mn) return launch_stream<STORE, true>(out, x, w, bias, M, N, K, ldx, ldw, ldo, stream);
+    return launch_stream<STORE, false>(out, x, w, bias, M, N, K, ldx, ldw, ldo, stream);
 }
 
 // out (M, N) = (x . w1^T) * silu(x . w2^T) with w = [w1; w2] of 2 N rows, M <= 128; N a multiple of 64
 extern "C" int llmc_stream_gemm_swiglu(bf16* out, const bf16* x, const bf16* w, int M, int N, int K, int ldx, int ldw, int ldo, cudaStream_t stream) {
-    if (N % 64) return -1;
-    return launch_stream<true>(out, x, w, nullptr, M, N, K, ldx, ldw, ldo, stream);
+    if (N % 64 || M > 128) return -1;
+    return launch_stream<SWIGLU, false>(out, x, w, nullptr, M, N, K, ldx, ldw, ldo, stream);
 }
 
-// The same product for the at most 8 rows of a decoding step
+// The plain product for the at most 8 rows of a decoding step
 extern "C" int llmc_skinny_gemm(bf16* out, const bf16* x, const bf16* w, int M, int N, int K, int ldx, int ldw, int ldo, cudaStream_t stream) {
     if (M > 8) return -1;
-    return launch_stream<false>(out, x, w, nullptr, M, N, K, ldx, ldw, ldo, stream);
+    return launch_stream<STORE, false>(out, x, w, nullptr, M, N, K, ldx, ldw, ldo, stream);
 }

@@ -13,7 +13,7 @@ _launches = 0   # number of kernel-library launches issued (bench.py reports it)
 # forward / dgrad GEMMs with at least this many 256 x 256 tiles run on the two-SM kernel (gemm2.cu); 0 disables it
 TWO_SM_MIN_TILES = int(os.environ.get("LLMC_GEMM_2SM_MIN_TILES", "74"))
 
-# forward products of at most this many rows stream the weights through split-K clusters (stream_gemm.cu)
+# products of at most this many rows may stream the weights through split-K clusters whatever their depth (_few_rows)
 STREAM_MAX_ROWS = 128
 
 
@@ -68,17 +68,35 @@ def sm_count(device):
     return _sm_count[idx]
 
 
+def _few_rows(M, N, K, mode, b_mn, device):
+    """Whether a plain product goes to the split-K kernel with 128 x 256 tiles of csrc/stream_gemm.cu.  The lines are where it overtakes the other
+    two kernels (M from 100 to 2048, fourteen pairs of N and K, us): deep products whose tiles leave at least half of the SMs idle
+    (K = 3072: 24 tiles 21 against 27, 36 tiles 33 against 27; K = 7168: 64 tiles 37 to 43 against 53, 96 tiles 61 against 55), and
+    at most 128 rows, unless there are so many tiles that the overlap of tiles on a persistent CTA counts (100 x 50304 x 768:
+    39 against 31) or the product is a shallow input gradient (100 x 768 x 768: 16 against 14)."""
+    if mode != MODE_STORE:
+        return False
+    wtiles = (N + 127) // 128
+    tiles = (M + 255) // 256 * wtiles
+    if (K >= 6144 and tiles <= 64) or (K >= 3072 and tiles <= 32):
+        return True
+    if b_mn:
+        return M <= STREAM_MAX_ROWS and K >= 2048 and wtiles <= 2 * sm_count(device)
+    return M <= 64 or (M <= STREAM_MAX_ROWS and wtiles <= 2 * sm_count(device))
+
+
 def gemm(a, b, d, M, N, K, lda, ldb, ldd, a_mn, b_mn, mode, bias=None, aux=None, accumulate=False, splits=1, max_ctas=0, ready=None):
-    """Dispatches to the two-SM kernel (256 x 256 tiles on CTA pairs) for problems with enough tiles, else to the single-CTA one.
+    """Dispatches to the split-K kernel for plain products with few tiles (``_few_rows``), to the two-SM kernel (256 x 256 tiles on
+    CTA pairs) for problems with enough tiles, else to the single-CTA one.
     ``ready`` (an object with flags_ptr, n, seq and wait()) marks the B operand as the target of an all-gather in flight: the
     two-SM kernel polls the peers' flags itself before its first load; the single-CTA kernel runs after ``ready.wait()``."""
     global _launches
     lib = _lib.cuda()
     _launches += 1
-    if M <= STREAM_MAX_ROWS and mode == MODE_STORE and not a_mn and not b_mn:
+    if not a_mn and _few_rows(M, N, K, mode, b_mn, d.device):
         if ready is not None:
             ready.wait()
-        check(lib.llmc_stream_gemm(_p(d), _p(a), _p(b), _p(bias), M, N, K, lda, ldb, ldd, _stream()), "llmc_stream_gemm")
+        check(lib.llmc_stream_gemm(_p(d), _p(a), _p(b), _p(bias), M, N, K, lda, ldb, ldd, int(b_mn), _stream()), "llmc_stream_gemm")
         return
     tiles256 = ((M + 255) // 256) * ((N + 255) // 256)
     if mode == MODE_ACCUM:
