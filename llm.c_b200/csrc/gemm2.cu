@@ -11,7 +11,7 @@
 // Supported: forward (A, B K-major; STORE + bias, GELU + pre-activation), dgrad (B MN-major; STORE, DGELU) and wgrad
 // (A, B MN-major; bf16 accumulate with deterministic split-K).  Small problems use the single-CTA kernel (gemm.cu).
 // Epilogue: sixteen warps per CTA in four groups of four, each group owning 64 columns of the CTA's 128 x 256 half tile
-// (64-byte-swizzled staging, TMA stores).
+// (staging in shared memory, TMA stores).
 #include "common.cuh"
 
 namespace {
@@ -27,9 +27,7 @@ constexpr int EPI_GROUPS = 4;          // epilogue groups of four warps, each ow
 constexpr int GROUP_COLS = BN / EPI_GROUPS;
 constexpr int EPI_COLS = 32;
 constexpr int EPI_BUF_BYTES = BM * EPI_COLS * 2;      // 8 KB
-// Staging: 64 KB next to five pipeline stages, split evenly over the sixteen epilogue warps (two 2 KB buffers each).  STORE
-// alternates between a warp's two buffers; the epilogues with two tensors per chunk (GELU: activation + pre-activation out;
-// dGELU: pre-activation in + gradient out) use one each.
+// Staging: 64 KB next to five pipeline stages, split evenly over the sixteen epilogue warps.
 __host__ __device__ constexpr int stages_for(int mode) { return 5; }
 __host__ __device__ constexpr int epi_bufs_for(int mode) { return 2 * EPI_GROUPS; }
 __host__ __device__ constexpr int smem_for(int mode) { return stages_for(mode) * STAGE_BYTES + epi_bufs_for(mode) * EPI_BUF_BYTES + 1024 + 512; }
@@ -44,7 +42,7 @@ struct Gemm2Args {
     int num_m_tiles, num_n_tiles, num_kb;     // 256 x 256 tiles
     int splits, kb_per_split;                 // EPI_ACCUM: split-K
     const bf16* bias;
-    bf16* D; int ldd;                         // EPI_ACCUM writes D directly
+    bf16* D; int ldd;                         // of the fold kernel
     float* workspace;                         // [half tile][split][128 * 256] fp32 partials
     unsigned int* counters;                   // unused (kept in the argument list of the entry points)
     int accumulate;
@@ -134,7 +132,7 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
     }
     if (warp == 0 && lane == 0) {
         tma_prefetch_desc(&tmA); tma_prefetch_desc(&tmB);
-        if (MODE != EPI_ACCUM) tma_prefetch_desc(&tmD);
+        tma_prefetch_desc(&tmD);
         if (MODE == EPI_GELU || MODE == EPI_DGELU) tma_prefetch_desc(&tmAux);
     }
     cluster_sync_all();                                   // both CTAs' barriers exist before anyone signals them
@@ -255,31 +253,37 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
         const int grp = ew >> 2;
         const int q = warp & 3;
         const int row = q * 32 + lane;
-        // Every epilogue warp is its own pipeline over its 32 rows x GROUP_COLS columns: TMEM -> registers -> its own two
-        // 2 KB staging buffers (64-byte swizzle) -> its own TMA stores.  Warps never wait for one another, so the TMEM
+        // Every epilogue warp is its own pipeline over its 32 rows x GROUP_COLS columns: TMEM -> registers -> its own 4 KB staging
+        // buffer -> its own TMA stores.  Warps never wait for one another, so the TMEM
         // load, shared-memory fence and store-drain latencies of one warp are covered by the other three of its scheduler.
-        //   STORE: the two buffers alternate;  GELU: buffer 0 = activation, buffer 1 = pre-activation;
-        //   DGELU: buffer 0 = output, buffer 1 = this warp's 32 x 32 box of the stored pre-activation (TMA load).
-        constexpr int WARP_BUF_BYTES = 32 * EPI_COLS * 2;           // 2 KB
-        static_assert(2 * WARP_BUF_BYTES * 4 * EPI_GROUPS == NUM_EPI_BUFS * EPI_BUF_BYTES, "staging space is split evenly over the epilogue warps");
-        uint8_t* wbuf = epi_smem + ew * 2 * WARP_BUF_BYTES;
+        //   GELU: the pre-activation, then the activation;  DGELU: the stored pre-activation comes in through the buffer (its box in L2
+        //   since the tile before), the gradient leaves through it;  ACCUM without split: the old values of D likewise.  (Reading and writing
+        //   D row by row from the registers touched 32 cache lines per instruction.)
+        // The epilogues with two tensors move the whole piece in one go, in 128-byte rows: half as many TMA requests, and a store or load has
+        // a tile's time to complete instead of half a chunk's (M=65536 N=3072 K=768: GELU 302 -> 265 us, dGELU at M=16384 94 -> 82 us;
+        // in 32-column chunks the dGELU loads of 2 KB per warp were all that was on its way).  STORE keeps the 32-column chunks through two
+        // halves in turn: 222 us against 226.
+        constexpr int WARP_BUF_BYTES = 32 * GROUP_COLS * 2;         // 4 KB
+        static_assert(WARP_BUF_BYTES * 4 * EPI_GROUPS == NUM_EPI_BUFS * EPI_BUF_BYTES, "staging space is split evenly over the epilogue warps");
+        uint8_t* wbuf = epi_smem + ew * WARP_BUF_BYTES;
         constexpr int CHUNKS = GROUP_COLS / EPI_COLS;
-        const int swz = (lane >> 1) & 3;
-        uint32_t kctr = 0;
-        // pre-activation box of chunk c_ of work item w_ -> this warp's second buffer; chunk k completes phase k & 1 of its barrier
-        auto aux_load = [&](int w_, int c_) {
+        // pre-activation (or old gradient) box of work item w_ -> this warp's buffer (item i of the warp completes phase i & 1), or only into L2
+        auto aux_load = [&](int w_) {
             int mt_, nt_, sp_; decode(w_, mt_, nt_, sp_);
             uint64_t* bar = &aux_full[ew];
             mbar_expect_tx(bar, WARP_BUF_BYTES);
-            tma_load_2d(wbuf + WARP_BUF_BYTES, &tmAux, bar, nt_ * BN + grp * GROUP_COLS + c_ * EPI_COLS, mt_ * 256 + (int)rank * BM + q * 32);
+            tma_load_2d(wbuf, &tmAux, bar, nt_ * BN + grp * GROUP_COLS, mt_ * 256 + (int)rank * BM + q * 32);
         };
-        // (work item, chunk) that follows (w_, c_) in this warp's sequence; false at the end
-        auto next_chunk = [&](int& w_, int& c_) {
-            if (c_ + 1 < CHUNKS) { c_++; return true; }
-            if (w_ + npairs < total_work) { w_ += npairs; c_ = 0; return true; }
-            return false;
+        auto aux_prefetch = [&](int w_) {
+            int mt_, nt_, sp_; decode(w_, mt_, nt_, sp_);
+            asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global [%0, {%1, %2}];"
+                         ::"l"(reinterpret_cast<uint64_t>(&tmAux)), "r"(nt_ * BN + grp * GROUP_COLS), "r"(mt_ * 256 + (int)rank * BM + q * 32) : "memory");
         };
-        if (MODE == EPI_DGELU && lane == 0 && pair < total_work) aux_load(pair, 0);
+        const bool use_aux = MODE == EPI_DGELU || (MODE == EPI_ACCUM && g.accumulate && g.splits == 1);
+        if (use_aux && lane == 0 && pair < total_work) {
+            aux_load(pair);
+            if (pair + npairs < total_work) aux_prefetch(pair + npairs);
+        }
         const uint32_t lead_acc_empty0 = map_to_cta(smem_u32(&acc_empty[0]), 0);
         const uint32_t lead_acc_empty1 = map_to_cta(smem_u32(&acc_empty[1]), 0);
         int it = 0;
@@ -290,153 +294,68 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
             bool ok = mbar_wait(&acc_full[buf], use & 1, abort_flag, g.status, 0xC00 + buf);
             tc_fence_after();
             const int m0 = mt * 256 + (int)rank * BM, n0 = nt * BN + grp * GROUP_COLS;
-            const int grow = m0 + row;
             const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16) + buf * BN + grp * GROUP_COLS;
             const uint32_t lead_acc_empty = buf ? lead_acc_empty1 : lead_acc_empty0;
-            if (MODE == EPI_ACCUM) {
-                // ---- EPI_ACCUM: direct global read-modify-write, optional split-K ----
+            if (MODE == EPI_ACCUM && g.splits > 1) {
+                // ---- split-K
                 const int tile = (mt * g.num_n_tiles + nt) * 2 + (int)rank;      // this CTA's half of the 256 x 256 tile
-                if (g.splits == 1) {
-                    #pragma unroll 1
-                    for (int c = 0; c < CHUNKS; c++) {
-                        const int col0 = n0 + c * 32;
-                        if (col0 >= g.N) break;
-                        uint32_t v[32];
-                        tmem_ld32(t_row + c * 32, v);
-                        tmem_ld_wait();
-                        float* f = reinterpret_cast<float*>(v);
-                        if (grow < g.M && ok) {
-                            #pragma unroll
-                            for (int j = 0; j < 32; j += 8) {
-                                if (col0 + j < g.N) {
-                                    bf16* dp = g.D + (size_t)grow * g.ldd + col0 + j;
-                                    bf16x8 o;
-                                    if (g.accumulate) {
-                                        bf16x8 old = ld128(dp);
-                                        #pragma unroll
-                                        for (int e = 0; e < 8; e++) o[e] = __float2bfloat16_rn(f[j + e] + __bfloat162float(old[e]));
-                                    } else {
-                                        #pragma unroll
-                                        for (int e = 0; e < 8; e++) o[e] = __float2bfloat16_rn(f[j + e]);
-                                    }
-                                    st128(dp, o);
-                                }
-                            }
-                        }
+                // partial tile -> workspace, laid out [col/4][row][4] so that a warp writes 512 contiguous bytes
+                float* wsp = g.workspace + ((size_t)tile * g.splits + sp) * (BM * BN);
+                const int cbase = grp * GROUP_COLS;
+                #pragma unroll 1
+                for (int c = 0; c < CHUNKS; c++) {
+                    uint32_t v[32];
+                    tmem_ld32(t_row + c * 32, v);
+                    tmem_ld_wait();
+                    #pragma unroll
+                    for (int j = 0; j < 32; j += 4) {
+                        float4 o = make_float4(__uint_as_float(v[j]), __uint_as_float(v[j+1]), __uint_as_float(v[j+2]), __uint_as_float(v[j+3]));
+                        __stcg(reinterpret_cast<float4*>(wsp + ((size_t)((cbase + c * 32 + j) >> 2) * BM + row) * 4), o);
                     }
-                    tc_fence_before();
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive_cluster(lead_acc_empty);
-                } else {
-                    // partial tile -> workspace, laid out [col/4][row][4] so that a warp writes 512 contiguous bytes
-                    float* wsp = g.workspace + ((size_t)tile * g.splits + sp) * (BM * BN);
-                    const int cbase = grp * GROUP_COLS;
-                    #pragma unroll 1
-                    for (int c = 0; c < CHUNKS; c++) {
-                        uint32_t v[32];
-                        tmem_ld32(t_row + c * 32, v);
-                        tmem_ld_wait();
-                        #pragma unroll
-                        for (int j = 0; j < 32; j += 4) {
-                            float4 o = make_float4(__uint_as_float(v[j]), __uint_as_float(v[j+1]), __uint_as_float(v[j+2]), __uint_as_float(v[j+3]));
-                            __stcg(reinterpret_cast<float4*>(wsp + ((size_t)((cbase + c * 32 + j) >> 2) * BM + row) * 4), o);
-                        }
-                    }
-                    tc_fence_before();
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive_cluster(lead_acc_empty);
-                    // the partial sums of a tile are added, in split order, by gemm2_fold_kernel after this kernel
                 }
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive_cluster(lead_acc_empty);
+                // the partial sums of a tile are added, in split order, by gemm2_fold_kernel after this kernel
                 if (epi_any(*abort_flag)) break;
                 continue;
             }
-            #pragma unroll 1
-            for (int c = 0; c < CHUNKS; c++) {
-                const int col0 = n0 + c * EPI_COLS;
-                uint32_t v[32];
-                tmem_ld32(t_row + c * EPI_COLS, v);
-                tmem_ld_wait();
-                if (c == CHUNKS - 1) {
-                    // this warp holds the last of its part of the accumulator: tell the leader CTA's MMA thread
-                    tc_fence_before();
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive_cluster(lead_acc_empty);
-                }
-                float* f = reinterpret_cast<float*>(v);
-                if ((MODE == EPI_STORE || MODE == EPI_GELU) && g.bias != nullptr) {
-                    #pragma unroll
-                    for (int j = 0; j < 32; j += 8) {
-                        if (col0 + j < g.N) {
-                            bf16x8 b = ld128(g.bias + col0 + j);
-                            #pragma unroll
-                            for (int e = 0; e < 8; e += 2) add2(f + j + e, __bfloat162float(b[e]), __bfloat162float(b[e + 1]));
+            if (MODE == EPI_STORE) {
+                // ---- one tensor out: chunks of 32 columns through the two halves of the buffer in turn
+                #pragma unroll 1
+                for (int c = 0; c < CHUNKS; c++) {
+                    const int col0 = n0 + c * EPI_COLS;
+                    uint32_t v[EPI_COLS];
+                    tmem_ld32(t_row + c * EPI_COLS, v);
+                    tmem_ld_wait();
+                    if (c == CHUNKS - 1) {
+                        // this warp holds the last of its part of the accumulator: tell the leader CTA's MMA thread
+                        tc_fence_before();
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive_cluster(lead_acc_empty);
+                    }
+                    float* f = reinterpret_cast<float*>(v);
+                    if (g.bias != nullptr) {
+                        #pragma unroll
+                        for (int j = 0; j < EPI_COLS; j += 8) {
+                            if (col0 + j < g.N) {
+                                bf16x8 b = ld128(g.bias + col0 + j);
+                                #pragma unroll
+                                for (int e = 0; e < 8; e += 2) add2(f + j + e, __bfloat162float(b[e]), __bfloat162float(b[e + 1]));
+                            }
                         }
                     }
-                }
-                uint8_t* out_buf = wbuf + ((MODE == EPI_STORE) ? (kctr & 1) * WARP_BUF_BYTES : 0);
-                uint8_t* aux_buf = wbuf + WARP_BUF_BYTES;
-                uint8_t* out_row = out_buf + lane * 64;
-                uint8_t* aux_row = aux_buf + lane * 64;
-                uint4 pre_q[4], out_q[4];
-                if (MODE == EPI_DGELU) {
-                    ok = mbar_wait(&aux_full[ew], kctr & 1, abort_flag, g.status, 0xC40 + ew) && ok;
-                    #pragma unroll
-                    for (int j = 0; j < 4; j++) {
-                        const uint4 a = *reinterpret_cast<const uint4*>(aux_row + ((j ^ swz) * 16));
-                        const float2 a0 = unpack_bf16x2(a.x), a1 = unpack_bf16x2(a.y), a2 = unpack_bf16x2(a.z), a3 = unpack_bf16x2(a.w);
-                        mul2(f + j * 8 + 0, gelu_grad_fast2(a0));
-                        mul2(f + j * 8 + 2, gelu_grad_fast2(a1));
-                        mul2(f + j * 8 + 4, gelu_grad_fast2(a2));
-                        mul2(f + j * 8 + 6, gelu_grad_fast2(a3));
-                    }
-                    __syncwarp();            // every lane has read its row of the pre-activation box
-                    if (lane == 0) {
-                        int w_ = w, c_ = c;
-                        if (next_chunk(w_, c_)) aux_load(w_, c_);
-                    }
-                }
-                if (MODE == EPI_GELU) {
-                    // Two stores per chunk, each from its own buffer and in its own bulk group, issued half a chunk apart:
-                    // when a buffer is needed again the only younger group is the other tensor's, so each store has a full
-                    // chunk of work to drain underneath (the same slack the alternating buffers give plain STORE).
-                    #pragma unroll
-                    for (int j = 0; j < 4; j++) {
-                        pre_q[j].x = pack_bf16x2(f[j*8+0], f[j*8+1]); pre_q[j].y = pack_bf16x2(f[j*8+2], f[j*8+3]);
-                        pre_q[j].z = pack_bf16x2(f[j*8+4], f[j*8+5]); pre_q[j].w = pack_bf16x2(f[j*8+6], f[j*8+7]);
-                    }
-                    if (lane == 0) tma_store_wait_read<1>();
-                    __syncwarp();
-                    #pragma unroll
-                    for (int j = 0; j < 4; j++) *reinterpret_cast<uint4*>(aux_row + ((j ^ swz) * 16)) = pre_q[j];
-                    fence_async_smem();
-                    __syncwarp();
-                    if (lane == 0 && ok && col0 < g.N) { tma_store_2d(&tmAux, aux_buf, col0, m0 + q * 32); tma_store_commit(); }
-                    #pragma unroll
-                    for (int j = 0; j < 4; j++) {
-                        // the activation is computed from the rounded pre-activation, so a later recomputation from the stored
-                        // tensor gives the same bits
-                        const float2 r0 = unpack_bf16x2(pre_q[j].x), r1 = unpack_bf16x2(pre_q[j].y), r2 = unpack_bf16x2(pre_q[j].z), r3 = unpack_bf16x2(pre_q[j].w);
-                        out_q[j].x = pack_bf16x2(gelu_fast2(r0)); out_q[j].y = pack_bf16x2(gelu_fast2(r1));
-                        out_q[j].z = pack_bf16x2(gelu_fast2(r2)); out_q[j].w = pack_bf16x2(gelu_fast2(r3));
-                    }
-                    if (lane == 0) tma_store_wait_read<1>();
-                    __syncwarp();
-                    #pragma unroll
-                    for (int j = 0; j < 4; j++) *reinterpret_cast<uint4*>(out_row + ((j ^ swz) * 16)) = out_q[j];
-                    fence_async_smem();
-                    __syncwarp();
-                    if (lane == 0 && ok && col0 < g.N) { tma_store_2d(&tmD, out_buf, col0, m0 + q * 32); tma_store_commit(); }
-                } else {
                     // all arithmetic happens before the wait for the staging buffer, so the drain of the previous store hides under it
+                    uint4 out_q[4];
                     #pragma unroll
                     for (int j = 0; j < 4; j++) {
                         out_q[j].x = pack_bf16x2(f[j*8+0], f[j*8+1]); out_q[j].y = pack_bf16x2(f[j*8+2], f[j*8+3]);
                         out_q[j].z = pack_bf16x2(f[j*8+4], f[j*8+5]); out_q[j].w = pack_bf16x2(f[j*8+6], f[j*8+7]);
                     }
-                    if (lane == 0) {
-                        if (MODE == EPI_STORE) tma_store_wait_read<1>();      // the store issued two chunks ago has read this buffer
-                        else tma_store_wait_read<0>();
-                    }
+                    uint8_t* out_buf = wbuf + (c & 1) * (WARP_BUF_BYTES / 2);
+                    uint8_t* out_row = out_buf + lane * 64;
+                    const int swz = (lane >> 1) & 3;
+                    if (lane == 0) tma_store_wait_read<1>();      // the store issued two chunks ago has read this half
                     __syncwarp();
                     #pragma unroll
                     for (int j = 0; j < 4; j++) *reinterpret_cast<uint4*>(out_row + ((j ^ swz) * 16)) = out_q[j];
@@ -444,9 +363,81 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
                     __syncwarp();
                     if (lane == 0 && ok && col0 < g.N) { tma_store_2d(&tmD, out_buf, col0, m0 + q * 32); tma_store_commit(); }
                 }
-                kctr++;
+                if (epi_any(*abort_flag)) break;
+                continue;
             }
-            if (epi_any(*abort_flag)) break;
+            // ---- a second tensor comes in or goes out: the warp's whole 32 x 64 piece at once
+            uint32_t v[GROUP_COLS];
+            tmem_ld32(t_row, v);
+            tmem_ld32(t_row + 32, v + 32);
+            tmem_ld_wait();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_cluster(lead_acc_empty);      // the leader CTA's MMA thread may refill the accumulator
+            float* f = reinterpret_cast<float*>(v);
+            if (MODE == EPI_GELU && g.bias != nullptr) {
+                #pragma unroll
+                for (int j = 0; j < GROUP_COLS; j += 8) {
+                    if (n0 + j < g.N) {
+                        bf16x8 b = ld128(g.bias + n0 + j);
+                        #pragma unroll
+                        for (int e = 0; e < 8; e += 2) add2(f + j + e, __bfloat162float(b[e]), __bfloat162float(b[e + 1]));
+                    }
+                }
+            }
+            uint8_t* srow = wbuf + lane * 128;
+            const int swz = lane & 7;
+            auto store = [&](const CUtensorMap* tm) {
+                fence_async_smem();
+                __syncwarp();
+                if (lane == 0 && ok && n0 < g.N) { tma_store_2d(tm, wbuf, n0, m0 + q * 32); tma_store_commit(); }
+            };
+            auto buffer_free = [&] {
+                if (lane == 0) tma_store_wait_read<0>();
+                __syncwarp();
+            };
+            uint32_t pk[GROUP_COLS / 2];
+            if (MODE == EPI_ACCUM && use_aux) {
+                ok = mbar_wait(&aux_full[ew], (uint32_t)it & 1, abort_flag, g.status, 0xC40 + ew) && ok;
+                #pragma unroll
+                for (int j = 0; j < 8; j++) {
+                    const uint4 x = *reinterpret_cast<const uint4*>(srow + ((j ^ swz) * 16));
+                    const float2 x0 = unpack_bf16x2(x.x), x1 = unpack_bf16x2(x.y), x2 = unpack_bf16x2(x.z), x3 = unpack_bf16x2(x.w);
+                    add2(f + j * 8 + 0, x0.x, x0.y); add2(f + j * 8 + 2, x1.x, x1.y); add2(f + j * 8 + 4, x2.x, x2.y); add2(f + j * 8 + 6, x3.x, x3.y);
+                }
+            }
+            if (MODE == EPI_DGELU) {
+                ok = mbar_wait(&aux_full[ew], (uint32_t)it & 1, abort_flag, g.status, 0xC40 + ew) && ok;
+                #pragma unroll
+                for (int j = 0; j < 8; j++) {
+                    const uint4 x = *reinterpret_cast<const uint4*>(srow + ((j ^ swz) * 16));
+                    mul2(f + j * 8 + 0, gelu_grad_fast2(unpack_bf16x2(x.x))); mul2(f + j * 8 + 2, gelu_grad_fast2(unpack_bf16x2(x.y)));
+                    mul2(f + j * 8 + 4, gelu_grad_fast2(unpack_bf16x2(x.z))); mul2(f + j * 8 + 6, gelu_grad_fast2(unpack_bf16x2(x.w)));
+                }
+            }
+            #pragma unroll
+            for (int j = 0; j < GROUP_COLS / 2; j++) pk[j] = pack_bf16x2(f[2 * j], f[2 * j + 1]);
+            if (!use_aux) buffer_free();                           // the previous tile's store has had a whole tile's time
+            else __syncwarp();                                     // every lane has read its row of the tensor that came in
+            #pragma unroll
+            for (int j = 0; j < 8; j++) *reinterpret_cast<uint4*>(srow + ((j ^ swz) * 16)) = make_uint4(pk[4 * j], pk[4 * j + 1], pk[4 * j + 2], pk[4 * j + 3]);
+            store(MODE == EPI_GELU ? &tmAux : &tmD);
+            if (MODE == EPI_GELU) {
+                // the activation is computed from the rounded pre-activation, so a later recomputation from the stored tensor gives the
+                // same bits; it follows through the same buffer
+                #pragma unroll
+                for (int j = 0; j < GROUP_COLS / 2; j++) pk[j] = pack_bf16x2(gelu_fast2(unpack_bf16x2(pk[j])));
+                buffer_free();
+                #pragma unroll
+                for (int j = 0; j < 8; j++) *reinterpret_cast<uint4*>(srow + ((j ^ swz) * 16)) = make_uint4(pk[4 * j], pk[4 * j + 1], pk[4 * j + 2], pk[4 * j + 3]);
+                store(&tmD);
+            }
+            if (use_aux && lane == 0 && w + npairs < total_work) {
+                tma_store_wait_read<0>();
+                aux_load(w + npairs);
+                if (w + 2 * npairs < total_work) aux_prefetch(w + 2 * npairs);
+            }
+            if (__any_sync(0xffffffffu, *abort_flag)) break;       // warps are independent: no barrier joins them
         }
         if (lane == 0) tma_store_wait<0>();
     }
@@ -617,10 +608,11 @@ static int gemm2_impl(const bf16* A, const bf16* B, bf16* D, const bf16* bias, b
     }
     {
         uint64_t dims[2] = {(uint64_t)N, (uint64_t)M}, strides[2] = {2, (uint64_t)ldd * 2};
-        uint32_t box[2] = {EPI_COLS, 32};        // one epilogue warp's rows
-        if ((rc = llmc_get_tensormap(&tmD, D, 2, 2, dims, strides, box, 2))) return rc;
+        uint32_t box[2] = {GROUP_COLS, 32};      // one epilogue warp's piece (STORE: half of it)
+        if (mode == EPI_STORE) box[0] = EPI_COLS;
+        if ((rc = llmc_get_tensormap(&tmD, D, 2, 2, dims, strides, box, mode == EPI_STORE ? 2 : 3))) return rc;
         tmAux = tmD;
-        if (mode == EPI_GELU || mode == EPI_DGELU) { if ((rc = llmc_get_tensormap(&tmAux, aux, 2, 2, dims, strides, box, 2))) return rc; }
+        if (mode == EPI_GELU || mode == EPI_DGELU) { if ((rc = llmc_get_tensormap(&tmAux, aux, 2, 2, dims, strides, box, 3))) return rc; }
     }
     int sms = llmc_device_sm_count(); if (sms <= 0) sms = 148;
     int pairs = sms / 2;
