@@ -8,6 +8,7 @@
 //
 // Capability parity: llmc/fused_classifier.cuh (fused_classifier) of the reference.
 #include "common.cuh"
+#include "pdl.cuh"
 
 namespace {
 
@@ -17,6 +18,8 @@ template <bool WRITE_DLOGITS>
 __global__ void __launch_bounds__(CLS_THREADS)
 classifier_kernel(bf16* __restrict__ logits, float* __restrict__ losses, const int* __restrict__ targets,
                   float dloss, int V, int Vp, int accumulate_loss) {
+    pdl_wait();
+    pdl_trigger();
     __shared__ float red[32];
     constexpr float LOG2E = 1.4426950408889634f, LN2 = 0.6931471805599453f;
     // rows are processed back to front so that the rows the LM-head GEMM wrote last (still in L2) go first
@@ -85,8 +88,7 @@ classifier_kernel(bf16* __restrict__ logits, float* __restrict__ losses, const i
 extern "C" int llmc_fused_classifier(bf16* logits, float* losses, const int* targets, float dloss, int N, int V, int Vp,
                                      int write_dlogits, int accumulate_loss, cudaStream_t stream) {
     if (Vp % 8) return -1;
-    if (write_dlogits) classifier_kernel<true><<<N, CLS_THREADS, 0, stream>>>(logits, losses, targets, dloss, V, Vp, accumulate_loss);
-    else classifier_kernel<false><<<N, CLS_THREADS, 0, stream>>>(logits, losses, targets, dloss, V, Vp, accumulate_loss);
-    CUDA_CHECK(cudaGetLastError());
+    if (write_dlogits) CUDA_CHECK(launch_pdl(classifier_kernel<true>, dim3(N), dim3(CLS_THREADS), 0, stream, 0, logits, losses, targets, dloss, V, Vp, accumulate_loss));
+    else CUDA_CHECK(launch_pdl(classifier_kernel<false>, dim3(N), dim3(CLS_THREADS), 0, stream, 0, logits, losses, targets, dloss, V, Vp, accumulate_loss));
     return 0;
 }

@@ -9,10 +9,13 @@
 // Capability parity: llmc/gelu.cuh and matmul_backward_bias_kernel9 / reduce_add_sum_kernel of
 // llmc/matmul.cuh in the reference.
 #include "common.cuh"
+#include "pdl.cuh"
 
 namespace {
 
 __global__ void gelu_fwd_kernel(bf16* __restrict__ out, const bf16* __restrict__ inp, long long npack) {
+    pdl_wait();
+    pdl_trigger();
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= npack) return;
     bf16x8 a = ld128cs(inp + i * 8), o;
@@ -22,6 +25,8 @@ __global__ void gelu_fwd_kernel(bf16* __restrict__ out, const bf16* __restrict__
 }
 
 __global__ void gelu_bwd_kernel(bf16* __restrict__ d_inout, const bf16* __restrict__ inp, long long npack) {
+    pdl_wait();
+    pdl_trigger();
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= npack) return;
     bf16x8 a = ld128cs(inp + i * 8), d = ld128(d_inout + i * 8), o;
@@ -31,6 +36,8 @@ __global__ void gelu_bwd_kernel(bf16* __restrict__ d_inout, const bf16* __restri
 }
 
 __global__ void residual_add_kernel(bf16* __restrict__ out, const bf16* __restrict__ a, const bf16* __restrict__ b, long long npack) {
+    pdl_wait();
+    pdl_trigger();
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= npack) return;
     bf16x8 x = ld128cs(a + i * 8), y = ld128cs(b + i * 8), o;
@@ -43,6 +50,8 @@ constexpr int BG_WARPS = 8;
 // grid (ceil(OC/256), strips). partials[strip][OC]
 __global__ void __launch_bounds__(BG_WARPS * 32)
 bias_grad_kernel(float* __restrict__ partials, const bf16* __restrict__ dout, int rows, int OC, int rows_per_strip) {
+    pdl_wait();
+    pdl_trigger();
     __shared__ float sh[BG_WARPS][256];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int col = blockIdx.x * 256 + lane * 8;
@@ -68,6 +77,8 @@ bias_grad_kernel(float* __restrict__ partials, const bf16* __restrict__ dout, in
 }
 
 __global__ void bias_grad_fold_kernel(bf16* __restrict__ dbias, const float* __restrict__ partials, int strips, int OC, int accumulate) {
+    pdl_wait();
+    pdl_trigger();
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= OC) return;
     float s = 0.f;
@@ -89,20 +100,17 @@ int bg_strips(int rows, int OC) {
 
 extern "C" int llmc_gelu_fwd(bf16* out, const bf16* inp, long long n, cudaStream_t stream) {
     if (n % 8) return -1;
-    gelu_fwd_kernel<<<(unsigned)CEIL_DIV(n / 8, 256), 256, 0, stream>>>(out, inp, n / 8);
-    CUDA_CHECK(cudaGetLastError());
+    CUDA_CHECK(launch_pdl(gelu_fwd_kernel, dim3((unsigned)CEIL_DIV(n / 8, 256)), dim3(256), 0, stream, 0, out, inp, n / 8));
     return 0;
 }
 extern "C" int llmc_gelu_bwd_inplace(bf16* d_inout, const bf16* inp, long long n, cudaStream_t stream) {
     if (n % 8) return -1;
-    gelu_bwd_kernel<<<(unsigned)CEIL_DIV(n / 8, 256), 256, 0, stream>>>(d_inout, inp, n / 8);
-    CUDA_CHECK(cudaGetLastError());
+    CUDA_CHECK(launch_pdl(gelu_bwd_kernel, dim3((unsigned)CEIL_DIV(n / 8, 256)), dim3(256), 0, stream, 0, d_inout, inp, n / 8));
     return 0;
 }
 extern "C" int llmc_residual_add(bf16* out, const bf16* a, const bf16* b, long long n, cudaStream_t stream) {
     if (n % 8) return -1;
-    residual_add_kernel<<<(unsigned)CEIL_DIV(n / 8, 256), 256, 0, stream>>>(out, a, b, n / 8);
-    CUDA_CHECK(cudaGetLastError());
+    CUDA_CHECK(launch_pdl(residual_add_kernel, dim3((unsigned)CEIL_DIV(n / 8, 256)), dim3(256), 0, stream, 0, out, a, b, n / 8));
     return 0;
 }
 extern "C" long long llmc_bias_grad_scratch(int rows, int OC) { return (long long)bg_strips(rows, OC) * OC; }
@@ -111,9 +119,7 @@ extern "C" int llmc_bias_grad(bf16* dbias, float* scratch, const bf16* dout, int
     if (OC % 8) return -1;
     const int strips = bg_strips(rows, OC);
     const int rps = CEIL_DIV(rows, strips);
-    bias_grad_kernel<<<dim3(CEIL_DIV(OC, 256), strips), BG_WARPS * 32, 0, stream>>>(scratch, dout, rows, OC, rps);
-    CUDA_CHECK(cudaGetLastError());
-    bias_grad_fold_kernel<<<CEIL_DIV(OC, 128), 128, 0, stream>>>(dbias, scratch, strips, OC, accumulate);
-    CUDA_CHECK(cudaGetLastError());
+    CUDA_CHECK(launch_pdl(bias_grad_kernel, dim3(CEIL_DIV(OC, 256), strips), dim3(BG_WARPS * 32), 0, stream, 0, scratch, dout, rows, OC, rps));
+    CUDA_CHECK(launch_pdl(bias_grad_fold_kernel, dim3(CEIL_DIV(OC, 128)), dim3(128), 0, stream, 0, dbias, scratch, strips, OC, accumulate));
     return 0;
 }

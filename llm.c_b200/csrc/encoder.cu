@@ -41,6 +41,8 @@ __global__ void encoder_fwd_kernel(bf16* __restrict__ out, const int* __restrict
 // dwpe[t, c] (+)= sum_b dout[b, t, c]
 __global__ void wpe_bwd_kernel(bf16* __restrict__ dwpe, const bf16* __restrict__ dout, int B, int T, int C,
                                int accumulate, unsigned int seed) {
+    pdl_wait();
+    pdl_trigger();
     const int cp = C >> 3;
     const int idx = blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= T * cp) return;
@@ -76,6 +78,8 @@ static_assert(WTE_SCAN * (WTE_THREADS / 32) == 32, "the scan of the hit counts i
 __global__ void __launch_bounds__(WTE_THREADS)
 wte_bwd_kernel(bf16* __restrict__ dwte, const bf16* __restrict__ dout, const int* __restrict__ tokens,
                int N, int C, int V, int accumulate, unsigned int seed) {
+    pdl_wait();
+    pdl_trigger();
     __shared__ int list_pos[LIST_CAP];
     __shared__ unsigned char list_id[LIST_CAP];
     __shared__ int warp_counts[WTE_SCAN * (WTE_THREADS / 32)];
@@ -214,10 +218,8 @@ extern "C" int llmc_encoder_bwd(bf16* dwte, bf16* dwpe, const bf16* dout, const 
                                 int accumulate_wte, int accumulate_wpe, unsigned int seed, cudaStream_t stream) {
     if (C % 8) return -1;
     if (dwpe != nullptr) {
-        wpe_bwd_kernel<<<CEIL_DIV(T * (C / 8), 256), 256, 0, stream>>>(dwpe, dout, B, T, C, accumulate_wpe, seed);
-        CUDA_CHECK(cudaGetLastError());
+        CUDA_CHECK(launch_pdl(wpe_bwd_kernel, dim3(CEIL_DIV(T * (C / 8), 256)), dim3(256), 0, stream, 0, dwpe, dout, B, T, C, accumulate_wpe, seed));
     }
-    wte_bwd_kernel<<<CEIL_DIV(V, IDS_PER_CTA), WTE_THREADS, 0, stream>>>(dwte, dout, tokens, B * T, C, V, accumulate_wte, seed + 1);
-    CUDA_CHECK(cudaGetLastError());
+    CUDA_CHECK(launch_pdl(wte_bwd_kernel, dim3(CEIL_DIV(V, IDS_PER_CTA)), dim3(WTE_THREADS), 0, stream, 0, dwte, dout, tokens, B * T, C, V, accumulate_wte, seed + 1));
     return 0;
 }

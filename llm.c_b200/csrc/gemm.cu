@@ -21,6 +21,7 @@
 //               tile's MMAs overlap.
 // No TMA load uses cluster multicast. All waits are bounded (see common.cuh).
 #include "common.cuh"
+#include "pdl.cuh"
 
 namespace {
 
@@ -110,6 +111,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    pdl_wait();
+    pdl_trigger();
 
     // work item -> (m tile, n tile, split); m tiles are visited in groups so that concurrently
     // running CTAs share both A and B tiles in L2
@@ -449,8 +452,7 @@ int launch(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tm
         CUDA_CHECK(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
         configured = true;
     }
-    kfn<<<grid, NUM_THREADS, SMEM_BYTES, stream>>>(tmA, tmB, tmD, tmAux, g);
-    CUDA_CHECK(cudaGetLastError());
+    CUDA_CHECK(launch_pdl(kfn, dim3(grid), dim3(NUM_THREADS), SMEM_BYTES, stream, 0, tmA, tmB, tmD, tmAux, g));
     return 0;
 }
 

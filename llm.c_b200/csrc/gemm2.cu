@@ -13,6 +13,7 @@
 // Epilogue: sixteen warps per CTA in four groups of four, each group owning 64 columns of the CTA's 128 x 256 half tile
 // (staging in shared memory, TMA stores).
 #include "common.cuh"
+#include "pdl.cuh"
 
 namespace {
 
@@ -141,6 +142,8 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    pdl_wait();
+    pdl_trigger();
 
     auto decode = [&](int w, int& mt, int& nt, int& sp) {
         // split-K: units that run at the same time (consecutive w) cover all tiles of the same K range, so the operand strips of
@@ -461,6 +464,8 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
 // the last CTA pair of a tile took 16 dependent round trips to L2 per thread (about 30 us per launch, measured).
 __global__ void __launch_bounds__(256)
 gemm2_fold_kernel(bf16* __restrict__ D, const float* __restrict__ ws, int M, int N, int ldd, int num_n_tiles, int splits, int accumulate) {
+    pdl_wait();
+    pdl_trigger();
     __shared__ __align__(16) bf16 tile[BM][64 + 8];
     const int chunk = blockIdx.x & 3, half = blockIdx.x >> 2;
     const int rank = half & 1, t2 = half >> 1;
@@ -530,11 +535,9 @@ int launch2(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& t
         CUDA_CHECK(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_for(MODE)));
         configured = true;
     }
-    kfn<<<grid, NUM_THREADS, smem_for(MODE), stream>>>(tmA, tmB, tmD, tmAux, g);
-    CUDA_CHECK(cudaGetLastError());
+    CUDA_CHECK(launch_pdl(kfn, dim3(grid), dim3(NUM_THREADS), smem_for(MODE), stream, 0, tmA, tmB, tmD, tmAux, g));
     if (MODE == EPI_ACCUM && g.splits > 1) {
-        gemm2_fold_kernel<<<g.num_m_tiles * g.num_n_tiles * 2 * 4, 256, 0, stream>>>(g.D, g.workspace, g.M, g.N, g.ldd, g.num_n_tiles, g.splits, g.accumulate);
-        CUDA_CHECK(cudaGetLastError());
+        CUDA_CHECK(launch_pdl(gemm2_fold_kernel, dim3(g.num_m_tiles * g.num_n_tiles * 2 * 4), dim3(256), 0, stream, 0, g.D, g.workspace, g.M, g.N, g.ldd, g.num_n_tiles, g.splits, g.accumulate));
     }
     return 0;
 }

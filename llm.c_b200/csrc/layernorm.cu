@@ -10,6 +10,7 @@
 // Capability parity: llmc/layernorm.cuh (layernorm_forward, fused_residual_forward5,
 // layernorm_backward) of the reference.
 #include "common.cuh"
+#include "pdl.cuh"
 
 namespace {
 
@@ -26,6 +27,8 @@ __global__ void __launch_bounds__(256)
 ln_fwd_kernel(bf16* __restrict__ out, float* __restrict__ mean_out, float* __restrict__ rstd_out,
               bf16* __restrict__ residual_out, const bf16* __restrict__ inp1, const bf16* __restrict__ inp2,
               const bf16* __restrict__ weight, const bf16* __restrict__ bias, int N, int C) {
+    pdl_wait();
+    pdl_trigger();
     const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (row >= N) return;
     const int lane = threadIdx.x & 31;
@@ -157,6 +160,8 @@ __global__ void __launch_bounds__(LNB_MAX_THREADS)
 ln_bwd_col_kernel(bf16* __restrict__ dinp, float* __restrict__ partials, const bf16* __restrict__ dout,
                   const bf16* __restrict__ inp, const bf16* __restrict__ weight,
                   const float* __restrict__ mean, const float* __restrict__ rstd, int N, int C, int rows_per_cta) {
+    pdl_wait();
+    pdl_trigger();
     __shared__ float2 red[2][LNB_MAX_THREADS / 32];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5, nthr = blockDim.x;
     const int npack = C >> 3;
@@ -297,6 +302,8 @@ DEVINL void add4(float4& a, const float4& b) { a.x += b.x; a.y += b.y; a.z += b.
 __global__ void __launch_bounds__(4 * LNB_FOLD_SLICES)
 ln_bwd_fold_kernel(bf16* __restrict__ dweight, bf16* __restrict__ dbias, bf16* __restrict__ dcolsum,
                    const float* __restrict__ partials, int num_ctas, int C, int accumulate, int accumulate_col) {
+    pdl_wait();
+    pdl_trigger();
     __shared__ float4 sh[3][LNB_FOLD_SLICES][4];
     const int x = threadIdx.x & 3, y = threadIdx.x >> 2;
     const int c = blockIdx.x * 16 + x * 4;
@@ -339,7 +346,7 @@ int ln_fwd(bf16* out, float* mean, float* rstd, bf16* residual, const bf16* inp1
     if (C % 8) return -1;
     const int packs = CEIL_DIV(C / 8, 32);
     const dim3 grid(CEIL_DIV(N, 8));
-#define LNF_GO(MP) ln_fwd_kernel<FUSED, MP><<<grid, 256, 0, stream>>>(out, mean, rstd, residual, inp1, inp2, weight, bias, N, C)
+#define LNF_GO(MP) CUDA_CHECK(launch_pdl(ln_fwd_kernel<FUSED, MP>, dim3(grid), dim3(256), 0, stream, 0, out, mean, rstd, residual, inp1, inp2, weight, bias, N, C))
     if (packs <= 2) LNF_GO(2);
     else if (packs <= 3) LNF_GO(3);
     else if (packs <= LNF_MAX_PACKS) LNF_GO(4);
@@ -373,10 +380,11 @@ struct LnbLaunch { int threads, ctas, rows_per_cta; };
 template <bool ACC, int MAXP, bool COL>
 int lnb_launch(bf16* dinp, float* scratch, const bf16* dout, const bf16* inp, const bf16* weight, const float* mean, const float* rstd,
                int N, int C, int threads, int* ctas_out, cudaStream_t stream) {
+    constexpr bool CACHE = MAXP <= 2;
     static int occ_cache[LNB_MAX_THREADS / 32 + 1] = {0};
     int& occ = occ_cache[threads / 32];
     if (occ == 0) {
-        CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, ln_bwd_col_kernel<ACC, MAXP, COL, (MAXP <= 2)>, threads, 0));
+        CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, ln_bwd_col_kernel<ACC, MAXP, COL, CACHE>, threads, 0));
         if (occ < 1) occ = 1;
         if (occ > LNB_MAX_CTAS_PER_SM) occ = LNB_MAX_CTAS_PER_SM;
     }
@@ -384,8 +392,7 @@ int lnb_launch(bf16* dinp, float* scratch, const bf16* dout, const bf16* inp, co
     int ctas = occ * sms;
     int rows_per_cta = CEIL_DIV(N, ctas);
     ctas = CEIL_DIV(N, rows_per_cta);
-    ln_bwd_col_kernel<ACC, MAXP, COL, (MAXP <= 2)><<<ctas, threads, 0, stream>>>(dinp, scratch, dout, inp, weight, mean, rstd, N, C, rows_per_cta);
-    CUDA_CHECK(cudaGetLastError());
+    CUDA_CHECK(launch_pdl(ln_bwd_col_kernel<ACC, MAXP, COL, CACHE>, dim3(ctas), dim3(threads), 0, stream, 0, dinp, scratch, dout, inp, weight, mean, rstd, N, C, rows_per_cta));
     *ctas_out = ctas;
     return 0;
 }
@@ -417,7 +424,6 @@ extern "C" int llmc_layernorm_bwd(bf16* dinp, bf16* dweight, bf16* dbias, float*
     else if (packs <= 4) rc = lnb_dispatch<4>(acc, col, dinp, scratch, dout, inp, weight, mean, rstd, N, C, threads, &ctas, stream);
     else rc = lnb_dispatch<8>(acc, col, dinp, scratch, dout, inp, weight, mean, rstd, N, C, threads, &ctas, stream);
     if (rc) return rc;
-    ln_bwd_fold_kernel<<<CEIL_DIV(C, 16), 4 * LNB_FOLD_SLICES, 0, stream>>>(dweight, dbias, dcolsum, scratch, ctas, C, accumulate_dwdb, accumulate_dcol);
-    CUDA_CHECK(cudaGetLastError());
+    CUDA_CHECK(launch_pdl(ln_bwd_fold_kernel, dim3(CEIL_DIV(C, 16)), dim3(4 * LNB_FOLD_SLICES), 0, stream, 0, dweight, dbias, dcolsum, scratch, ctas, C, accumulate_dwdb, accumulate_dcol));
     return 0;
 }

@@ -139,6 +139,8 @@ __global__ void __launch_bounds__(RMSB_THREADS)
 rms_bwd_kernel(bf16* __restrict__ dinp, float* __restrict__ partials, const bf16* __restrict__ dout,
                const bf16* __restrict__ inp, const bf16* __restrict__ weight, const float* __restrict__ rstd,
                int N, int C, int rows_per_cta) {
+    pdl_wait();
+    pdl_trigger();
     __shared__ float red[2][RMSB_THREADS / 32];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int npack = C >> 3;
@@ -222,6 +224,8 @@ rms_bwd_kernel(bf16* __restrict__ dinp, float* __restrict__ partials, const bf16
 constexpr int RMS_FOLD_SLICES = 64;
 __global__ void __launch_bounds__(4 * RMS_FOLD_SLICES)
 rms_bwd_fold_kernel(bf16* __restrict__ dweight, const float* __restrict__ partials, int num_ctas, int C, int accumulate) {
+    pdl_wait();
+    pdl_trigger();
     __shared__ float4 sh[RMS_FOLD_SLICES][4];
     const int x = threadIdx.x & 3, y = threadIdx.x >> 2;
     const int c = blockIdx.x * 16 + x * 4;
@@ -276,6 +280,8 @@ constexpr int ROPE_THREADS = 256;
 template <int REP>
 __global__ void __launch_bounds__(ROPE_THREADS)
 rope_fwd_kernel(bf16* __restrict__ packed, const bf16* __restrict__ raw, const float2* __restrict__ freqs, int T, int NH, int NKV, int HS) {
+    pdl_wait();
+    pdl_trigger();
     const int hp = HS >> 3, heads = NH + 2 * NKV, items = heads * hp, rep = REP ? REP : NH / NKV;
     const long long n = blockIdx.x;
     const float4* frow = reinterpret_cast<const float4*>(freqs + (size_t)(blockIdx.x % (unsigned)T) * (HS >> 1));
@@ -302,6 +308,8 @@ rope_fwd_kernel(bf16* __restrict__ packed, const bf16* __restrict__ raw, const f
 template <int REP>
 __global__ void __launch_bounds__(ROPE_THREADS)
 rope_bwd_kernel(bf16* __restrict__ draw, const bf16* __restrict__ dpacked, const float2* __restrict__ freqs, int T, int NH, int NKV, int HS) {
+    pdl_wait();
+    pdl_trigger();
     const int hp = HS >> 3, heads = NH + 2 * NKV, items = heads * hp, rep = REP ? REP : NH / NKV;
     const long long n = blockIdx.x;
     const float4* frow = reinterpret_cast<const float4*>(freqs + (size_t)(blockIdx.x % (unsigned)T) * (HS >> 1));
@@ -365,6 +373,8 @@ DEVINL float sigmoid_fast(float x) { return __fdividef(1.0f, 1.0f + __expf(-x));
 
 __global__ void __launch_bounds__(256)
 swiglu_fwd_kernel(bf16* __restrict__ h, const bf16* __restrict__ x12, long long N, int H) {
+    pdl_wait();
+    pdl_trigger();
     const int hp = H >> 3;
     const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= N * hp) return;
@@ -382,6 +392,8 @@ swiglu_fwd_kernel(bf16* __restrict__ h, const bf16* __restrict__ x12, long long 
 
 __global__ void __launch_bounds__(256)
 swiglu_bwd_kernel(bf16* __restrict__ dx12, const bf16* __restrict__ dh, const bf16* __restrict__ x12, long long N, int H) {
+    pdl_wait();
+    pdl_trigger();
     const int hp = H >> 3;
     const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= N * hp) return;
@@ -450,7 +462,7 @@ extern "C" int llmc_rmsnorm_bwd(bf16* dinp, bf16* dweight, float* scratch, const
     int rows_per_cta = CEIL_DIV(N, ctas);
     ctas = CEIL_DIV(N, rows_per_cta);
     const int packs = CEIL_DIV(C / 8, RMSB_THREADS);
-#define RMSB_LAUNCH(ACC, MP) rms_bwd_kernel<ACC, MP><<<ctas, RMSB_THREADS, 0, stream>>>(dinp, scratch, dout, inp, weight, rstd, N, C, rows_per_cta)
+#define RMSB_LAUNCH(ACC, MP) CUDA_CHECK(launch_pdl(rms_bwd_kernel<ACC, MP>, dim3(ctas), dim3(RMSB_THREADS), 0, stream, 0, dinp, scratch, dout, inp, weight, rstd, N, C, rows_per_cta))
 #define RMSB_PICK(MP) do { if (accumulate_dinp) RMSB_LAUNCH(true, MP); else RMSB_LAUNCH(false, MP); } while (0)
     if (packs <= 1) RMSB_PICK(1);
     else if (packs <= 2) RMSB_PICK(2);
@@ -459,8 +471,7 @@ extern "C" int llmc_rmsnorm_bwd(bf16* dinp, bf16* dweight, float* scratch, const
 #undef RMSB_PICK
 #undef RMSB_LAUNCH
     CUDA_CHECK(cudaGetLastError());
-    rms_bwd_fold_kernel<<<CEIL_DIV(C, 16), 4 * RMS_FOLD_SLICES, 0, stream>>>(dweight, scratch, ctas, C, accumulate_dw);
-    CUDA_CHECK(cudaGetLastError());
+    CUDA_CHECK(launch_pdl(rms_bwd_fold_kernel, dim3(CEIL_DIV(C, 16)), dim3(4 * RMS_FOLD_SLICES), 0, stream, 0, dweight, scratch, ctas, C, accumulate_dw));
     return 0;
 }
 
@@ -469,7 +480,7 @@ static int rope_check(int NH, int NKV, int HS) { return (HS % 8 || NKV <= 0 || N
 extern "C" int llmc_rope_fwd(bf16* packed, const bf16* raw, const float* freqs, long long N, int T, int NH, int NKV, int HS, cudaStream_t stream) {
     if (rope_check(NH, NKV, HS)) return -1;
     if (N <= 0) return 0;
-#define ROPE_GO(R) rope_fwd_kernel<R><<<(unsigned)N, ROPE_THREADS, 0, stream>>>(packed, raw, reinterpret_cast<const float2*>(freqs), T, NH, NKV, HS)
+#define ROPE_GO(R) CUDA_CHECK(launch_pdl(rope_fwd_kernel<R>, dim3((unsigned)N), dim3(ROPE_THREADS), 0, stream, 0, packed, raw, reinterpret_cast<const float2*>(freqs), T, NH, NKV, HS))
     const int rep = NH / NKV;
     if (rep == 1) ROPE_GO(1);
     else if (rep == 2) ROPE_GO(2);
@@ -483,7 +494,7 @@ extern "C" int llmc_rope_fwd(bf16* packed, const bf16* raw, const float* freqs, 
 extern "C" int llmc_rope_bwd(bf16* draw, const bf16* dpacked, const float* freqs, long long N, int T, int NH, int NKV, int HS, cudaStream_t stream) {
     if (rope_check(NH, NKV, HS)) return -1;
     if (N <= 0) return 0;
-#define ROPE_GO(R) rope_bwd_kernel<R><<<(unsigned)N, ROPE_THREADS, 0, stream>>>(draw, dpacked, reinterpret_cast<const float2*>(freqs), T, NH, NKV, HS)
+#define ROPE_GO(R) CUDA_CHECK(launch_pdl(rope_bwd_kernel<R>, dim3((unsigned)N), dim3(ROPE_THREADS), 0, stream, 0, draw, dpacked, reinterpret_cast<const float2*>(freqs), T, NH, NKV, HS))
     const int rep = NH / NKV;
     if (rep == 1) ROPE_GO(1);
     else if (rep == 2) ROPE_GO(2);
@@ -496,14 +507,12 @@ extern "C" int llmc_rope_bwd(bf16* draw, const bf16* dpacked, const float* freqs
 
 extern "C" int llmc_swiglu_fwd(bf16* h, const bf16* x12, long long N, int H, cudaStream_t stream) {
     if (H % 8) return -1;
-    swiglu_fwd_kernel<<<(unsigned)CEIL_DIV(N * (H / 8), 256), 256, 0, stream>>>(h, x12, N, H);
-    CUDA_CHECK(cudaGetLastError());
+    CUDA_CHECK(launch_pdl(swiglu_fwd_kernel, dim3((unsigned)CEIL_DIV(N * (H / 8), 256)), dim3(256), 0, stream, 0, h, x12, N, H));
     return 0;
 }
 
 extern "C" int llmc_swiglu_bwd(bf16* dx12, const bf16* dh, const bf16* x12, long long N, int H, cudaStream_t stream) {
     if (H % 8) return -1;
-    swiglu_bwd_kernel<<<(unsigned)CEIL_DIV(N * (H / 8), 256), 256, 0, stream>>>(dx12, dh, x12, N, H);
-    CUDA_CHECK(cudaGetLastError());
+    CUDA_CHECK(launch_pdl(swiglu_bwd_kernel, dim3((unsigned)CEIL_DIV(N * (H / 8), 256)), dim3(256), 0, stream, 0, dx12, dh, x12, N, H));
     return 0;
 }
