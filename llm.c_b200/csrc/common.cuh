@@ -194,8 +194,8 @@ DEVINL uint64_t f2_add(uint64_t a, uint64_t b) { uint64_t r; asm("add.rn.f32x2 %
 constexpr float GELU_K1 = 0.7978845608028654f;                    // k = sqrt(2 / pi)
 constexpr float GELU_K2 = 0.7978845608028654f * 0.044715f;
 DEVINL float gelu_fast(float x) {
-    const float t = tanh_fast(x * fmaf(x * x, GELU_K2, GELU_K1)), h = 0.5f * x;
-    return fmaf(h, t, h);
+    const float t = tanh_fast(GELU_K1 * fmaf(0.044715f * x * x, x, x));
+    return 0.5f * x * (1.0f + t);
 }
 DEVINL float gelu_grad_fast(float x) {
     const float u = x * x;
@@ -205,9 +205,9 @@ DEVINL float gelu_grad_fast(float x) {
 }
 DEVINL uint64_t gelu_fast2(float2 v) {
     const uint64_t x = f2_pack(v.x, v.y);
-    const float2 w = f2_unpack(f2_mul(x, f2_fma(f2_mul(x, x), f2_pack(GELU_K2, GELU_K2), f2_pack(GELU_K1, GELU_K1))));
-    const uint64_t h = f2_mul(f2_pack(0.5f, 0.5f), x);
-    return f2_fma(h, f2_pack(tanh_fast(w.x), tanh_fast(w.y)), h);
+    const uint64_t c = f2_mul(f2_mul(f2_pack(0.044715f, 0.044715f), x), x);
+    const float2 w = f2_unpack(f2_mul(f2_pack(GELU_K1, GELU_K1), f2_fma(c, x, x)));
+    return f2_mul(f2_mul(f2_pack(0.5f, 0.5f), x), f2_add(f2_pack(1.0f, 1.0f), f2_pack(tanh_fast(w.x), tanh_fast(w.y))));
 }
 DEVINL uint64_t gelu_grad_fast2(float2 v) {
     const uint64_t x = f2_pack(v.x, v.y), u = f2_mul(x, x);

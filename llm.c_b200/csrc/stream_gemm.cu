@@ -15,7 +15,8 @@
 // Alone, after an L2 flush, the 128 x 256 tiles of the training GEMM in brackets: 32 x 4096 x 14336 (M x N x K) 36 us (101),
 // 32 x 6144 x 4096 23 us (38), 32 x 28672 x 4096 58 us (69), 100 x 2048 x 7168 23 us (52).  Inside a replayed decoding step (4 rows, 4 layers
 // of 2048 channels, LM head of 128256 rows) this kernel takes the step to 277 us; a weight-streaming kernel on warp-level MMAs with the same
-// early launch and prefetch, used for the products of at most 8 rows, left it at 290 us.  More rows: 256 x 768 x 50304 (an input gradient)
+// early launch and prefetch, used for the products of at most 8 rows, left it at 290 us (at 284 us for the LM head alone), although launched
+// by itself it took wide ones faster (4 x 28672 x 4096 50 us against 59).  More rows: 256 x 768 x 50304 (an input gradient)
 // 60 us (291), 777 x 2048 x 7168 37 us (53), 256 x 768 x 3072 18 us (27).
 //
 // Warps of a CTA: 0 TMA producer, 1 MMA issuer, 2-5 epilogue.  Two CTAs fit an SM.

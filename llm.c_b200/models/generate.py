@@ -7,7 +7,8 @@ sampling is nucleus (top-p) at a temperature, or greedy at temperature 0.
 
 The decoder works on the parameter tensors of a ``models.llama3.Llama`` (it never copies them), with its own small activation
 set and the caches ``(L, max_batch, max_len, NKV, HS)``.  On a GPU every step is a chain of this library's kernels: the GEMMs
-of training for prompts (rows padded to one 128-row tile) or a weight-streaming product for steps of at most 8 rows, RMSNorm / SwiGLU, and the two decoding kernels of csrc/decode.cu (rotary
+of training for prompts (rows padded to whole 128-row tiles) or split-K weight streaming for steps of at most 128 rows (csrc/stream_gemm.cu,
+SwiGLU in its epilogue), RMSNorm, and the two decoding kernels of csrc/decode.cu (rotary
 embedding written straight into the cache; attention of the new queries over the cached keys with grouped heads read in
 place).  A one-token step issues about nine small launches per layer and is bound by launch latency, so on a GPU it is
 captured once in a CUDA graph and replayed (``GraphStep``): the position lives in device memory, the graph advances it itself,

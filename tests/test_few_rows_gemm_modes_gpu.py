@@ -51,7 +51,7 @@ def test_input_gradient(M, N, K):
 
 # one size on either side of each line of the rule: rows, tiles at both depths, depth of an input gradient
 @pytest.mark.parametrize("M,N,K,forward,gradient", [(64, 256, 64, True, False), (65, 128 * 297, 64, False, False), (129, 256, 64, False, False),
-                                                    (128, 256, 2048, True, True), (1024, 1024, 3072, True, True), (1025, 1024, 3072, False, False),
+                                                    (128, 256, 2048, True, True), (1024, 1024, 3072, False, True), (1025, 1024, 3072, False, False),
                                                     (512, 4096, 6144, True, True), (513, 4096, 6144, False, False)])
 def test_dispatch(M, N, K, forward, gradient):
     dev = torch.device(DEV, 0)
