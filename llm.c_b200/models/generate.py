@@ -20,6 +20,11 @@ import torch
 from .. import ops
 
 
+def _whole_tiles(n):
+    """n rows padded to whole 128-row tiles."""
+    return (n + 127) // 128 * 128
+
+
 class CachedDecoder:
     def __init__(self, model, max_batch, max_len):
         cfg = model.cfg
@@ -30,11 +35,13 @@ class CachedDecoder:
         L, NKV, HS = cfg.num_layers, cfg.num_kv_heads, cfg.head_size
         self.kcache = torch.zeros(L, max_batch, max_len, NKV, HS, dtype=model.dtype, device=model.device)
         self.vcache = torch.zeros_like(self.kcache)
-        self._rows = 0
-        self._bufs = None
+        self._rows = self._last_rows = 0
+        self._bufs = {}
         self._dense = None
         # prompts of at least this many tokens per row, starting at position 0, run through the training attention kernel
         self.dense_prefill_from = 128
+        # products run on rows padded to whole 128-row tiles
+        self.whole_tiles = model.device.type == "cuda"
         # steps of at most this many rows use the weight-streaming product instead of a padded tensor-core tile (0: never)
         kernels = model.device.type == "cuda" and model.dtype == torch.bfloat16
         self.skinny_rows = 8 if kernels else 0
@@ -47,17 +54,19 @@ class CachedDecoder:
 
     def _buffers(self, N, B):
         """Activation rows are padded to a multiple of 128 so that every product is made of whole tiles; the rows beyond N
-        stay zero and are never read back."""
-        rows = (max(N, B) + 127) // 128 * 128
+        stay zero and are never read back.  The rows of the last positions (``last``, ``logits``) grow with the batch on their own."""
+        rows, last_rows = _whole_tiles(max(N, B)), _whole_tiles(B)
+        m, cfg = self.model, self.model.cfg
+        C, H, Vp = cfg.channels, cfg.hidden_dim, cfg.padded_vocab_size
+        z = lambda *s, dtype=m.dtype: torch.zeros(*s, dtype=dtype, device=m.device)
         if rows > self._rows:
-            m, cfg = self.model, self.model.cfg
-            C, H, Vp = cfg.channels, cfg.hidden_dim, cfg.padded_vocab_size
             QR = (cfg.num_heads + 2 * cfg.num_kv_heads) * cfg.head_size
-            z = lambda *s, dtype=m.dtype: torch.zeros(*s, dtype=dtype, device=m.device)
-            self._bufs = dict(x=z(rows, C), ln=z(rows, C), rstd=z(rows, dtype=torch.float32), raw=z(rows, QR), q=z(rows, C), atty=z(rows, C),
-                              proj=z(rows, C), res=z(rows, C), fc12=z(rows, 2 * H), h=z(rows, H), last=z(128 * ((B + 127) // 128), C),
-                              logits=z(128 * ((B + 127) // 128), Vp))
+            self._bufs = dict(self._bufs, x=z(rows, C), ln=z(rows, C), rstd=z(rows, dtype=torch.float32), raw=z(rows, QR), q=z(rows, C),
+                              atty=z(rows, C), proj=z(rows, C), res=z(rows, C), fc12=z(rows, 2 * H), h=z(rows, H))
             self._rows = rows
+        if last_rows > self._last_rows:
+            self._bufs = dict(self._bufs, last=z(last_rows, C), logits=z(last_rows, Vp))
+            self._last_rows = last_rows
         return self._bufs, rows
 
     def forward(self, tokens, start_pos, pos=None):
@@ -75,15 +84,15 @@ class CachedDecoder:
         a, rows = self._buffers(N, B)
         L, NH, NKV, eps, C = cfg.num_layers, cfg.num_heads, cfg.num_kv_heads, cfg.norm_eps, cfg.channels
         x, ln, rstd = a["x"], a["ln"], a["rstd"]
-        padded = m.device.type == "cuda"
 
         def mm(out, inp, weight, n):
             if n <= self.skinny_rows:
                 ops.matmul_skinny(out[:n], inp[:n], weight)
             elif n <= self.stream_rows:
                 ops.matmul_forward(out[:n], inp[:n], weight, None)
-            elif padded:
-                ops.matmul_forward(out, inp, weight, None)          # whole 128-row tiles; the rows beyond n are never read
+            elif self.whole_tiles:
+                r = _whole_tiles(n)                                 # of both operands: either may have more rows than this product
+                ops.matmul_forward(out[:r], inp[:r], weight, None)  # the rows beyond n are never read
             else:
                 ops.matmul_forward(out[:n], inp[:n], weight, None)
 

@@ -110,3 +110,27 @@ def test_sample_top_p():
     a = G.generate(m, [[4, 5, 6]], 8, temperature=0.8, top_p=0.9, generator=g1)
     b = G.generate(m, [[4, 5, 6]], 8, temperature=0.8, top_p=0.9, generator=g2)
     assert a == b
+
+
+def test_products_stay_inside_their_outputs(monkeypatch):
+    """Whole-tile products of a batch of more than one tile: as many rows of the output as of the input, whatever was run before."""
+    m = small_model("llama3:l=1,c=64,h=4,kv=2,t=64,v=97,m=32,f=1.0")
+    shapes = []
+    product = G.ops.matmul_forward
+
+    def spy(out, inp, weight, bias):
+        shapes.append((out.shape[0], inp.shape[0]))
+        product(out, inp, weight, bias)
+
+    monkeypatch.setattr(G.ops, "matmul_forward", spy)
+    g = torch.Generator().manual_seed(0)
+    dec, plain = G.CachedDecoder(m, 200, 16), G.CachedDecoder(m, 200, 16)
+    dec.whole_tiles = True
+    # a batch of several tiles after a longer prompt, and a batch that grows from call to call
+    for B, T in ((129, 10), (129, 1), (3, 2), (200, 1), (200, 3), (130, 1)):
+        tok = torch.randint(0, m.cfg.vocab_size, (B, T), generator=g, dtype=torch.int32)
+        shapes.clear()
+        got = dec.forward(tok, 0)
+        rows, last = (B * T + 127) // 128 * 128, (B + 127) // 128 * 128
+        assert shapes == [(rows, rows)] * 4 + [(last, last)]
+        assert torch.allclose(got, plain.forward(tok, 0), atol=1e-4, rtol=1e-4)

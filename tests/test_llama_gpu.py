@@ -315,3 +315,29 @@ def test_trainer_samples_with_the_cache_during_training(tmp_path, capsys):
     t.close()
     out = capsys.readouterr().out
     assert out.count("generating:") >= 2 and "val loss" in out
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_decoding_more_rows_than_one_tile(dtype):
+    """200 rows after a prompt of several tokens (more activation rows than logits rows), eager and, in bf16, replayed, against the CPU decoder."""
+    from llmc_b200.models import generate as G
+    cfg = llama3.config_from_descriptor("llama3:l=2,c=256,h=4,kv=2,t=64,v=500,m=64,f=1.0")
+    m = llama3.Llama(cfg, DEV, dtype, recompute=1)
+    m.init_random(3)
+    for n in ("qkvw", "attprojw", "fc12w", "fcprojw"):
+        m.params[n].mul_(3.0)
+    c = llama3.Llama(cfg, "cpu", torch.float32, recompute=0)
+    c.params_flat.copy_(m.params_flat.float().cpu())
+    g = torch.Generator().manual_seed(0)
+    tok = torch.randint(0, cfg.vocab_size, (200, 9), generator=g, dtype=torch.int32)
+    dm, dg, dc = G.CachedDecoder(m, 200, 16), G.CachedDecoder(m, 200, 16), G.CachedDecoder(c, 200, 16)
+    for d, t in ((dm, tok.to(DEV)), (dg, tok.to(DEV)), (dc, tok)):
+        d.forward(t[:2, :3].contiguous(), 0)                   # a small batch first: the logits rows have to grow
+        d.forward(t[:, :6].contiguous(), 0)
+    step = G.GraphStep(dg, 200, 6) if dtype == torch.bfloat16 else None
+    for t in range(6, 9):
+        got, want = dm.forward(tok[:, t:t + 1].contiguous().to(DEV), t), dc.forward(tok[:, t:t + 1].contiguous(), t)
+        close(got, want, 3e-2, 3e-2, "decode logits")
+        if step is not None:
+            assert torch.equal(step.step(tok[:, t:t + 1].to(DEV)), got)
+    assert dm._bufs["logits"].shape[0] == 256
