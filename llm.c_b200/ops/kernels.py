@@ -132,11 +132,19 @@ def gemm(a, b, d, M, N, K, lda, ldb, ldd, a_mn, b_mn, mode, bias=None, aux=None,
                         int(accumulate), splits, _p(ws), _p(cnt), max_ctas, _stream()), "llmc_gemm")
 
 
+def _check_sizes(op, *need):
+    """The launchers take the sizes of a product from two of its operands; the others have to be at least that large."""
+    for what, t, n in need:
+        if t is not None and t.numel() < n:
+            raise ValueError("%s: %s of shape %s, but the product needs %d elements of it" % (op, what, tuple(t.shape), n))
+
+
 def matmul_forward(out, inp, weight, bias=None, pre_gelu=None, ready=None):
     """out[M,OC] = inp[M,C] @ weight[OC,C]^T (+ bias).  With ``pre_gelu`` the pre-activation is stored there and
     ``out`` receives its tanh-GELU (reference: matmul_forward_cublaslt, llmc/matmul.cuh:230-242)."""
     M, C = inp.shape
     OC = weight.shape[0]
+    _check_sizes("matmul_forward", ("out", out, M * OC), ("weight", weight, OC * C), ("bias", bias, OC), ("pre_gelu", pre_gelu, M * OC))
     mode = MODE_GELU if pre_gelu is not None else MODE_STORE
     gemm(inp, weight, out, M, OC, C, C, C, OC, 0, 0, mode, bias=bias, aux=pre_gelu, ready=ready)
 
@@ -146,6 +154,7 @@ def matmul_dgrad(dinp, dout, weight, pre_gelu=None):
     (reference: matmul_backward dgrad with the DGELU epilogue, llmc/matmul.cuh:279-285)."""
     M, OC = dout.shape
     C = weight.shape[1]
+    _check_sizes("matmul_dgrad", ("dinp", dinp, M * C), ("weight", weight, OC * C), ("pre_gelu", pre_gelu, M * C))
     mode = MODE_DGELU if pre_gelu is not None else MODE_STORE
     gemm(dout, weight, dinp, M, C, OC, OC, C, C, 0, 1, mode, aux=pre_gelu)
 
@@ -154,6 +163,7 @@ def matmul_wgrad(dweight, dout, inp, accumulate=True):
     """dweight[OC,C] (+)= dout[M,OC]^T @ inp[M,C] with split-K sized to fill the SMs."""
     M, OC = dout.shape
     C = inp.shape[1]
+    _check_sizes("matmul_wgrad", ("dweight", dweight, OC * C), ("inp", inp, M * C))
     splits = _lib.cuda().llmc_gemm_pick_splits(OC, C, M, sm_count(dout.device))
     gemm(dout, inp, dweight, OC, C, M, OC, C, C, 1, 1, MODE_ACCUM, accumulate=accumulate, splits=splits)
 
@@ -375,11 +385,19 @@ def cached_attention(out, q, kcache, vcache, Tq, start_pos, NH, NKV, pos=None):
           "llmc_cached_attention")
 
 
+def _check_strided(op, *need):
+    """``_check_sizes`` for products that take row strides: rows and columns of every other operand."""
+    for what, t, rows, cols in need:
+        if t.shape[0] < rows or t.numel() < cols * t.shape[0]:
+            raise ValueError("%s: %s of shape %s, but the product needs (%d, %d)" % (op, what, tuple(t.shape), rows, cols))
+
+
 def matmul_skinny(out, inp, weight):
     """out[M,OC] = inp[M,C] @ weight[OC,C]^T for at most 8 rows: the weight-streaming kernel of decoding steps (csrc/stream_gemm.cu)."""
     global _launches
     M, C = inp.shape
     OC = weight.shape[0]
+    _check_strided("matmul_skinny", ("out", out, M, OC), ("weight", weight, OC, C))
     _launches += 1
     check(_lib.cuda().llmc_skinny_gemm(_p(out), _p(inp), _p(weight), M, OC, C, inp.stride(0), weight.stride(0), out.stride(0), _stream()),
           "llmc_skinny_gemm")
@@ -391,6 +409,7 @@ def matmul_swiglu(h, inp, weight12):
     global _launches
     M, C = inp.shape
     H = weight12.shape[0] // 2
+    _check_strided("matmul_swiglu", ("h", h, M, H), ("weight12", weight12, 2 * H, C))
     _launches += 1
     check(_lib.cuda().llmc_stream_gemm_swiglu(_p(h), _p(inp), _p(weight12), M, H, C, inp.stride(0), weight12.stride(0), h.stride(0), _stream()),
           "llmc_stream_gemm_swiglu")

@@ -1,10 +1,12 @@
 """Generation with a key / value cache on the CPU path: cached logits against the training forward pass, batched prompts of
 different lengths, stop tokens, echo, nucleus sampling (behaviour of LLaMA.generate / sample_top_p in the reference's
 train_llama3.py:476-576)."""
+import pytest
 import torch
 
 from llmc_b200.models import generate as G
 from llmc_b200.models import llama3
+from llmc_b200.ops import kernels as KN
 
 DESC = "llama3:l=2,c=64,h=4,kv=2,t=48,v=97,m=32,f=1.0"
 
@@ -134,3 +136,21 @@ def test_products_stay_inside_their_outputs(monkeypatch):
         rows, last = (B * T + 127) // 128 * 128, (B + 127) // 128 * 128
         assert shapes == [(rows, rows)] * 4 + [(last, last)]
         assert torch.allclose(got, plain.forward(tok, 0), atol=1e-4, rtol=1e-4)
+
+
+@pytest.mark.parametrize("op,shapes", [
+    ("matmul_forward", [(255, 64), (256, 32), (64, 32)]), ("matmul_forward", [(256, 56), (256, 32), (64, 32)]),
+    ("matmul_forward", [(256, 64), (256, 32), (64, 24)]), ("matmul_forward", [(256, 64), (256, 32), (64, 32), (56,)]),
+    ("matmul_forward", [(256, 64), (256, 32), (64, 32), (64,), (255, 64)]),
+    ("matmul_dgrad", [(255, 32), (256, 64), (64, 32)]), ("matmul_dgrad", [(256, 32), (256, 64), (56, 32)]),
+    ("matmul_dgrad", [(256, 32), (256, 64), (64, 32), (255, 32)]),
+    ("matmul_wgrad", [(56, 32), (256, 64), (256, 32)]), ("matmul_wgrad", [(64, 32), (256, 64), (255, 32)]),
+    ("matmul_skinny", [(7, 64), (8, 32), (64, 32)]), ("matmul_skinny", [(8, 56), (8, 32), (64, 32)]), ("matmul_skinny", [(8, 64), (8, 32), (64, 24)]),
+    ("matmul_swiglu", [(7, 64), (8, 32), (128, 32)]), ("matmul_swiglu", [(8, 56), (8, 32), (128, 32)]), ("matmul_swiglu", [(8, 64), (8, 32), (128, 24)])])
+def test_device_products_refuse_operands_that_are_too_small(monkeypatch, op, shapes):
+    """The launchers raise before anything is launched."""
+    def library():
+        raise AssertionError("launched")
+    monkeypatch.setattr(KN._lib, "cuda", library)
+    with pytest.raises(ValueError):
+        getattr(KN, op)(*[torch.zeros(*s, dtype=torch.bfloat16) for s in shapes])
