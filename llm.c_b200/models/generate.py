@@ -18,6 +18,7 @@ the fp32 restatement of the operators.
 import torch
 
 from .. import ops
+from ..ops import kernels
 
 
 def _whole_tiles(n):
@@ -43,11 +44,11 @@ class CachedDecoder:
         # products run on rows padded to whole 128-row tiles
         self.whole_tiles = model.device.type == "cuda"
         # steps of at most this many rows use the weight-streaming product instead of a padded tensor-core tile (0: never)
-        kernels = model.device.type == "cuda" and model.dtype == torch.bfloat16
-        self.skinny_rows = 8 if kernels else 0
+        own = model.device.type == "cuda" and model.dtype == torch.bfloat16
+        self.skinny_rows = 8 if own else 0
         # steps of at most this many rows run their products on exactly their rows (split-K weight streaming, csrc/stream_gemm.cu), the
         # MLP's up-projections with the activation in the same launch; longer ones on rows padded to whole 128-row tiles
-        self.stream_rows = 128 if kernels else 0
+        self.stream_rows = 128 if own else 0
 
     def cache_bytes(self):
         return 2 * self.kcache.numel() * self.kcache.element_size()
@@ -152,9 +153,11 @@ class GraphStep:
             decoder.forward(self.tokens, 0, pos=self.pos)      # buffers, tensor maps and kernel attributes exist before the capture;
         torch.cuda.current_stream(dev).wait_stream(side)       # what it wrote at start_pos is overwritten by the first real step
         self.graph = torch.cuda.CUDAGraph()
-        with torch.cuda.graph(self.graph):
+        with kernels.scratch_taken() as scratch, torch.cuda.graph(self.graph):
             self.logits = decoder.forward(self.tokens, 0, pos=self.pos)
             self.pos.add_(1)
+        # the graph holds addresses: a longer prompt replaces the decoder's activation buffers, another caller the scratch buffers
+        self._held = (scratch, decoder._bufs, decoder.kcache, decoder.vcache, decoder.model.freqs)
 
     def step(self, tokens):
         self.tokens.copy_(tokens.view_as(self.tokens), non_blocking=True)

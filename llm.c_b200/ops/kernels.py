@@ -1,6 +1,8 @@
 """Thin launchers of the sm_100a kernels: tensors in, C entry points out (see csrc/*.cu)."""
+import contextlib
 import ctypes
 import os
+import threading
 
 import torch
 
@@ -40,6 +42,7 @@ class _Scratch:
 
     def __init__(self):
         self.bufs = {}
+        self.taken = threading.local()       # .by: list that collects what this thread's calls take (scratch_taken)
 
     def get(self, key, numel, dtype, device, zero=False):
         k = (key, device.index, dtype)
@@ -47,10 +50,27 @@ class _Scratch:
         if t is None or t.numel() < numel:
             t = (torch.zeros if zero else torch.empty)(max(int(numel), 1), dtype=dtype, device=device)
             self.bufs[k] = t
+        by = getattr(self.taken, "by", None)
+        if by is not None:
+            by.append(t)
         return t
 
 
 _scratch = _Scratch()
+
+
+@contextlib.contextmanager
+def scratch_taken():
+    """A list of the scratch buffers that this thread's calls take inside the block.  A later call that needs a larger one replaces a buffer, so
+    a CUDA graph captured in the block has to keep the list."""
+    outer = getattr(_scratch.taken, "by", None)
+    _scratch.taken.by = by = []
+    try:
+        yield by
+    finally:
+        _scratch.taken.by = outer
+        if outer is not None:
+            outer += by
 
 
 def scratch_buffers():
@@ -376,8 +396,8 @@ def cached_attention(out, q, kcache, vcache, Tq, start_pos, NH, NKV, pos=None):
     N = q.shape[0]
     HS = kcache.shape[-1]
     B, Tmax = N // Tq, kcache.shape[1]
-    # decoding steps (few query rows per cached head, head width 64 or 128) take the split-key kernel and its workspace; the
-    # buffer is kept per device, so a step captured in a CUDA graph replays on the same addresses
+    # decoding steps (few query rows per cached head, head width 64 or 128) take the split-key kernel; a workspace only for more key
+    # slices than a cluster holds
     words = lib.llmc_cached_attention_workspace(B, Tq, Tmax, NH, NKV, HS)
     ws = _scratch.get("cached_attention", words, torch.float32, q.device) if words > 0 else None
     _launches += 2 if words > 0 else 1

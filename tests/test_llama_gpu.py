@@ -341,3 +341,29 @@ def test_decoding_more_rows_than_one_tile(dtype):
         if step is not None:
             assert torch.equal(step.step(tok[:, t:t + 1].to(DEV)), got)
     assert dm._bufs["logits"].shape[0] == 256
+
+
+def test_replayed_decoding_keeps_its_buffers():
+    """A cache of more key slices than a cluster holds, so that the step works in a shared scratch buffer.  Between two replays that buffer and the
+    decoder's activation buffers are outgrown and the memory they would leave behind is filled with NaN."""
+    from llmc_b200.models import generate as G
+    cfg = llama3.config_from_descriptor("llama3:l=2,c=128,h=2,kv=1,t=9100,v=500,m=64,f=1.0")
+    m = llama3.Llama(cfg, DEV, torch.bfloat16, recompute=1)
+    m.init_random(5)
+    g = torch.Generator().manual_seed(0)
+    tok = torch.randint(0, cfg.vocab_size, (1, 24), generator=g, dtype=torch.int32).to(DEV)
+    eager, graphed = G.CachedDecoder(m, 1, 9100), G.CachedDecoder(m, 1, 9100)
+    for d in (eager, graphed):
+        d.forward(tok[:, :10].contiguous(), 0)
+    gs = G.GraphStep(graphed, 1, 10)
+    assert len(gs._held[0]) > 0
+    sizes = [t.numel() * t.element_size() for t in (*gs._held[0], *graphed._bufs.values())]
+    for t in range(10, 24):
+        want = eager.forward(tok[:, t:t + 1].contiguous(), t)
+        if t == 15:
+            graphed.forward(torch.zeros(1, 300, dtype=torch.int32, device=DEV), 100)          # positions that no later step sees
+            big = torch.zeros(4, 9100, 1, 64, dtype=torch.bfloat16, device=DEV)
+            KN.cached_attention(torch.empty(4, 128, dtype=torch.bfloat16, device=DEV), torch.zeros(4, 128, dtype=torch.bfloat16, device=DEV), big, big, 1, 50, 2, 1)
+            poison = [torch.full((n // 4,), float("nan"), device=DEV) for n in sizes for _ in range(2)]
+        assert torch.equal(gs.step(tok[:, t:t + 1]), want), "position %d" % t
+    assert all(p.isnan().all() for p in poison)
