@@ -5,7 +5,7 @@ launcher takes longer than the kernel (forward + backward of 4 x 64 tokens of GP
 a launch sequence eagerly the first two times it sees its key and from the third time on replays a graph of it.
 
 What makes a replay equal to the eager call: the sequence only reads and writes buffers that the model owns (inputs are copied into them
-before), all scalar arguments are part of the key, and so are the addresses of every parameter, gradient and activation buffer.  The scratch buffers
+before), all scalar arguments are part of the key, and so are the addresses of every parameter, gradient and activation buffer and of the rotary table.  The scratch buffers
 of the operators are shared by all callers and replaced when one needs a larger one, so a graph keeps those it was captured with.
 """
 import torch
@@ -31,6 +31,8 @@ class StepGraphs:
                 or torch.cuda.is_current_stream_capturing():
             return fn()
         buffers = [model.params_flat, *model.params.values(), model.inputs, model.targets, *model.acts.values()]
+        if getattr(model, "freqs", None) is not None:
+            buffers.append(model.freqs)                        # rotary table
         if model.grads is not None:
             buffers += [model.grads_flat, *model.grads.values()]
         addresses = tuple(t.data_ptr() for t in buffers)
