@@ -6,7 +6,7 @@ a launch sequence eagerly the first two times it sees its key and from the third
 
 What makes a replay equal to the eager call: the sequence only reads and writes buffers that the model owns (inputs are copied into them
 before), all scalar arguments are part of the key, and so are the addresses of every parameter, gradient and activation buffer and of the rotary table.  The scratch buffers
-of the operators are shared by all callers and replaced when one needs a larger one, so a graph keeps those it was captured with.
+of the operators are shared by all callers and replaced when one needs a larger one, so a graph keeps those that its own operators took.
 """
 import torch
 
@@ -53,7 +53,7 @@ class StepGraphs:
     def _capture(model, e, fn):
         graph, side = torch.cuda.CUDAGraph(), torch.cuda.Stream(device=model.device)
         before = kernels.launch_count()
-        with torch.cuda.stream(side):
+        with torch.cuda.stream(side), kernels.scratch_taken() as scratch:
             # other threads (watchdog, data loader) may use the device meanwhile
             graph.capture_begin(capture_error_mode="thread_local")
             try:
@@ -62,5 +62,5 @@ class StepGraphs:
                 graph.capture_end()
         e["launches"] = kernels.launch_count() - before
         kernels.count_launches(-e["launches"])                 # captured, not launched
-        e["scratch"] = kernels.scratch_buffers()
+        e["scratch"] = scratch
         e["graph"] = graph

@@ -73,11 +73,6 @@ def scratch_taken():
             outer += by
 
 
-def scratch_buffers():
-    """The scratch buffers in use now; whoever holds their addresses beyond a call keeps the tensors too."""
-    return list(_scratch.bufs.values())
-
-
 _sm_count = {}
 
 

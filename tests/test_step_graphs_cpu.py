@@ -5,6 +5,7 @@ import pytest
 import torch
 
 from llmc_b200.models import step_graphs
+from llmc_b200.ops import kernels as KN
 
 
 def fake_model():
@@ -29,3 +30,19 @@ def test_a_replaced_buffer_is_launched_and_captured_again(monkeypatch, name):
         g.run(m, 64, ("forward",), lambda: calls.append("launch"))
     assert calls == ["launch", "launch", "replay"]
 
+
+def test_a_capture_holds_the_scratch_buffers_it_took_and_no_others():
+    dev = torch.device("cpu")
+    try:
+        other = KN._scratch.get("test_other", 1000, torch.float32, dev)
+        with KN.scratch_taken() as outer:
+            a = KN._scratch.get("test_a", 10, torch.float32, dev)
+            with KN.scratch_taken() as inner:
+                b = KN._scratch.get("test_a", 20, torch.float32, dev)          # outgrown inside: both are part of the capture
+            assert len(inner) == 1 and inner[0] is b
+        assert [id(t) for t in outer] == [id(a), id(b)]
+        KN._scratch.get("test_a", 30, torch.float32, dev)
+        assert len(outer) == 2 and all(t is not other for t in outer)
+    finally:
+        for k in [k for k in KN._scratch.bufs if k[0].startswith("test_")]:
+            del KN._scratch.bufs[k]

@@ -45,8 +45,11 @@ def train(family, use_graphs):
 
 @pytest.mark.parametrize("family", ["gpt2", "llama3"])
 def test_replayed_steps_equal_launched_steps(family):
+    other = KN._scratch.get("another_caller", 1000, torch.float32, DEV)
     want, launches, _ = train(family, False)
     got, counted, m = train(family, True)
     assert all(torch.equal(a, b) for a, b in zip(got, want))
     assert counted == launches
-    assert any(e["graph"] is not None for e in m.step_graphs._entries.values())
+    graphs = [e for e in m.step_graphs._entries.values() if e["graph"] is not None]
+    assert graphs
+    assert all(len(e["scratch"]) > 0 and not any(t is other for t in e["scratch"]) for k, e in m.step_graphs._entries.items() if k[0] == "backward" and e["graph"])
