@@ -287,6 +287,7 @@ int launch_stream(bf16* out, const bf16* x, const bf16* w, const bf16* bias, int
 // out (M, N) = x (M, K) . w (N, K)^T (+ bias), or x . w (K, N) with w_mn.  K, the row strides of x and w and, with w_mn, N are multiples of 8.
 extern "C" int llmc_stream_gemm(bf16* out, const bf16* x, const bf16* w, const bf16* bias, int M, int N, int K, int ldx, int ldw, int ldo, int w_mn,
                                 cudaStream_t stream) {
+    if (M <= 0 || N <= 0 || K <= 0) return 0;        // an empty product leaves out as it is, like the other two kernels'
     if (w_mn) return launch_stream<STORE, true>(out, x, w, bias, M, N, K, ldx, ldw, ldo, stream);
     return launch_stream<STORE, false>(out, x, w, bias, M, N, K, ldx, ldw, ldo, stream);
 }

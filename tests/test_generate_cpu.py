@@ -154,3 +154,12 @@ def test_device_products_refuse_operands_that_are_too_small(monkeypatch, op, sha
     monkeypatch.setattr(KN._lib, "cuda", library)
     with pytest.raises(ValueError):
         getattr(KN, op)(*[torch.zeros(*s, dtype=torch.bfloat16) for s in shapes])
+
+
+@pytest.mark.parametrize("M,N,K", [(0, 64, 64), (4, 0, 64), (4, 64, 0)])
+def test_an_empty_product_of_few_rows_is_no_error(M, N, K):
+    """All three product kernels return without a launch (no GPU is needed for that)."""
+    lib = KN._lib.cuda()
+    assert lib.llmc_stream_gemm(None, None, None, None, M, N, K, 64, 64, 64, 0, None) == 0
+    assert lib.llmc_gemm(None, None, None, None, None, M, N, K, 64, 64, 64, 0, 0, KN.MODE_STORE, 0, 1, None, None, 0, None) == 0
+    assert lib.llmc_gemm2(None, None, None, None, None, M, N, K, 64, 64, 64, 0, 0, KN.MODE_STORE, 0, 1, None, None, None) == 0
