@@ -223,6 +223,11 @@ stream_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
             }
         }
     }
+    // after an abandoned wait copies may still be on their way into this CTA's shared memory: give them time to land before it is freed
+    if (*abort_flag) {
+        const long long t0 = clock64();
+        while (clock64() - t0 < 2000000ll) { __nanosleep(1000); }
+    }
     __syncwarp();
     cluster_sync();                                           // no CTA leaves while a peer may still read its shared memory
     tc_fence_after();
