@@ -161,8 +161,9 @@ cached_attention_kernel(bf16* __restrict__ out, const bf16* __restrict__ q, cons
 //   * the products run on warp-level MMAs: S = Q K^T with the query rows as the 16-row operand (8 of them used), O += P V with the
 //     probabilities taken from the score registers.  fp32 FMAs with one key per lane (the kernel before this one) were bound by the
 //     shared-memory reads of the queries and the probabilities (187 us for the case below).
-//   * probabilities keep about 16 bits: P = hi + lo, both bf16, hi in rows 0..7 of the MMA operand and lo in the otherwise idle rows
-//     8..15, and the two halves of the accumulator are added at the end.  Queries, keys and values are bf16 as stored.
+//   * probabilities keep all 24 bits: P = hi + mid + lo, each the next 8 bits as a bf16.  hi in rows 0..7 of the MMA operand and mid in the
+//     otherwise idle rows 8..15, lo through a second MMA; the two halves of the accumulator are added at the end.  Queries, keys and values
+//     are bf16 as stored.
 //   * running (max, sum, accumulator) per warp, merged over the warps through shared memory, then over the key slices in slice
 //     order: through distributed shared memory when the slices of a head form one cluster (at most 8), else through a small fp32
 //     workspace and a second kernel.
@@ -192,7 +193,9 @@ DEVINL void mma_16x8x16(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, ui
                  : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
                  : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
-// float4 of this CTA's shared memory at byte address `addr`, in CTA `rank` of the cluster
+// the upper 16 bits of two floats: bf16 without rounding
+DEVINL uint32_t top_bf16x2(float lo, float hi) { return __byte_perm(__float_as_uint(lo), __float_as_uint(hi), 0x7632); }
+// float of this CTA's shared memory at byte address `addr`, in CTA `rank` of the cluster
 DEVINL float ld_peer(uint32_t addr, uint32_t rank) {
     uint32_t ra; float v;
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(addr), "r"(rank));
@@ -277,7 +280,7 @@ cached_attention_split_kernel(bf16* __restrict__ out, float* __restrict__ ws, co
     const int limit = min(k1, start_pos + (gq < rows ? gq : 0) / G + 1);      // keys [0, limit) are visible to this lane's row
     const float sl2 = scale * CA_LOG2E;
     float m = -INFINITY, l = 0.f;                              // of row gq; l: this lane's keys only
-    float acc[HS_ / 8][4];                                     // columns 2 tq4, + 1 of channel group n: [0,1] from P hi, [2,3] from P lo
+    float acc[HS_ / 8][4];                                     // columns 2 tq4, + 1 of channel group n: [0,1] from P hi and lo, [2,3] from P mid
     #pragma unroll
     for (int n = 0; n < HS_ / 8; n++) { acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.f; }
     // ldmatrix: lane supplies the row address of matrix lane / 8, row lane % 8
@@ -322,12 +325,15 @@ cached_attention_split_kernel(bf16* __restrict__ out, float* __restrict__ ws, co
             #pragma unroll
             for (int n = 0; n < HS_ / 8; n++) { acc[n][0] *= corr; acc[n][1] *= corr; acc[n][2] *= corr; acc[n][3] *= corr; }
         }
-        uint32_t hi[2], lo[2];
+        uint32_t hi[2], md[2], lo[2];                          // 8 bits each, cut off: the differences are exact and not negative
         #pragma unroll
         for (int h = 0; h < 2; h++) {
-            hi[h] = pack_bf16x2(p[2 * h], p[2 * h + 1]);
+            hi[h] = top_bf16x2(p[2 * h], p[2 * h + 1]);
             const float2 hf = unpack_bf16x2(hi[h]);
-            lo[h] = pack_bf16x2(p[2 * h] - hf.x, p[2 * h + 1] - hf.y);
+            const float r0 = p[2 * h] - hf.x, r1 = p[2 * h + 1] - hf.y;
+            md[h] = top_bf16x2(r0, r1);
+            const float2 mf = unpack_bf16x2(md[h]);
+            lo[h] = top_bf16x2(r0 - mf.x, r1 - mf.y);
         }
         // ---- O += P V: 16 keys, 16 channels per ldmatrix
         #pragma unroll
@@ -335,8 +341,10 @@ cached_attention_split_kernel(bf16* __restrict__ out, float* __restrict__ ws, co
             uint32_t vf[4];     // matrices: keys 0-7 / 8-15 of channels 0-7 of the pair of groups, then of channels 8-15
             const int row = (mid & 1) * 8 + mrow, c = n2 * 2 + (mid >> 1);
             ldmatrix4_trans(vf, vb + row * ROWB + ((c ^ (row & 7)) * 16));
-            mma_16x8x16(acc[2 * n2], hi[0], lo[0], hi[1], lo[1], vf[0], vf[1]);
-            mma_16x8x16(acc[2 * n2 + 1], hi[0], lo[0], hi[1], lo[1], vf[2], vf[3]);
+            mma_16x8x16(acc[2 * n2], hi[0], md[0], hi[1], md[1], vf[0], vf[1]);
+            mma_16x8x16(acc[2 * n2 + 1], hi[0], md[0], hi[1], md[1], vf[2], vf[3]);
+            mma_16x8x16(acc[2 * n2], lo[0], 0u, lo[1], 0u, vf[0], vf[1]);
+            mma_16x8x16(acc[2 * n2 + 1], lo[0], 0u, lo[1], 0u, vf[2], vf[3]);
         }
         __syncwarp();                                          // the stage may be refilled
         st = st + 1 == CA_STAGES ? 0 : st + 1;

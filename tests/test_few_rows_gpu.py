@@ -59,7 +59,34 @@ def test_cached_attention(B, Tq, start, Tmax, NH, NKV, HS):
     R.cached_attention(ref, q, kc, vc, Tq, start, NH, NKV)
     out = torch.empty(B * Tq, NH * HS, dtype=torch.bfloat16, device=DEV)
     KN.cached_attention(out, q.to(DEV), kc.to(DEV), vc.to(DEV), Tq, start, NH, NKV)
-    close(out, ref, 4e-3, 8e-3)                                # one rounding to bf16 (2^-9), probabilities carry 16 bits
+    close(out, ref, 4e-3, 8e-3)                                # one rounding to bf16 (2^-9)
+
+
+@pytest.mark.parametrize("HS,start,Tmax", [(64, 159, 192), (128, 999, 1000)])
+def test_cached_attention_keeps_fp32_probabilities(HS, start, Tmax):
+    """Values chosen so that the weighted sum cancels to about 2^-18 of its terms.  Probabilities in fp32 (the exponential and its argument
+    are good to 2^-22) leave an error of 2^-8 of the result, next to its rounding to bf16 (2^-9); with 16 bits it would be 2^-5 and 2^-4."""
+    B, NH = 4, 8
+    g = torch.Generator().manual_seed(start)
+    q, kc = rnd(B, NH * HS), rnd(B, Tmax, NH, HS, seed=1)
+    n = start + 1
+    p = torch.softmax(torch.einsum("bhd,bshd->bhs", q.view(B, NH, HS).double(), kc[:, :n].double()) / HS ** 0.5, -1)
+    v = torch.randn(B, NH, n, HS, generator=g).bfloat16().double()
+    want = torch.randn(B, NH, HS, generator=g).double() * 2.0 ** -18
+    top = p.topk(2, -1)
+    for i in range(2):                                         # the two largest probabilities take up what is left
+        at = top.indices[..., i, None, None].expand(B, NH, 1, HS)
+        if i == 0:
+            v.scatter_(2, top.indices[..., None].expand(B, NH, 2, HS), 0.0)
+        left = want - torch.einsum("bhs,bhsd->bhd", p, v)
+        v.scatter_(2, at, (left / top.values[..., i, None]).bfloat16().double()[:, :, None])
+    exact = torch.einsum("bhs,bhsd->bhd", p, v).view(B, NH * HS)
+    vc = torch.zeros(B, Tmax, NH, HS, dtype=torch.bfloat16)
+    vc[:, :n] = v.transpose(1, 2).bfloat16()
+    out = torch.empty(B, NH * HS, dtype=torch.bfloat16, device=DEV)
+    KN.cached_attention(out, q.to(DEV), kc.to(DEV), vc.to(DEV), 1, start, NH, NH)
+    err = (out.cpu().double() - exact).norm() / exact.norm()
+    assert err < 2.0 ** -6, float(err)
 
 
 @pytest.mark.parametrize("N,C", [(1, 8), (3, 264), (5, 2048), (1024, 512), (1025, 512), (4, 2056), (2, 8192), (2, 16384), (2, 16392)])
