@@ -177,8 +177,8 @@ constexpr int CA_MIN_KEYS = 128;      // a slice is at least this long (unless t
 constexpr int CA_MAX_CLUSTER = 8;
 constexpr float CA_LOG2E = 1.4426950408889634f;
 
-DEVINL void cp_async16(void* smem_dst, const void* gsrc) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(smem_dst)), "l"(gsrc) : "memory");
+DEVINL void cp_async16_or_zero(void* smem_dst, const void* gsrc, bool in) {     // gsrc is a readable address either way
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(smem_dst)), "l"(gsrc), "r"(in ? 16 : 0) : "memory");
 }
 DEVINL void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N> DEVINL void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
@@ -195,6 +195,8 @@ DEVINL void mma_16x8x16(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, ui
 }
 // the upper 16 bits of two floats: bf16 without rounding
 DEVINL uint32_t top_bf16x2(float lo, float hi) { return __byte_perm(__float_as_uint(lo), __float_as_uint(hi), 0x7632); }
+// a lower bound for the parts of probability p: half of it is still a positive bf16
+DEVINL float least_part(float p) { return p > 0.f ? fmaxf(p * 0x1p-32f, 0x1p-132f) : 0.f; }
 // float of this CTA's shared memory at byte address `addr`, in CTA `rank` of the cluster
 DEVINL float ld_peer(uint32_t addr, uint32_t rank) {
     uint32_t ra; float v;
@@ -245,7 +247,7 @@ cached_attention_split_kernel(bf16* __restrict__ out, float* __restrict__ ws, co
     const long long row_stride = (long long)NKV * HS_;
     const bf16* kbase = kcache + ((b * Tmax) * NKV + g) * HS_;
     const bf16* vbase = vcache + ((b * Tmax) * NKV + g) * HS_;
-    // K and V rows kt .. kt + 15 -> stage st; rows past the slice repeat its last row (their probabilities are zero, their values finite)
+    // K and V rows kt .. kt + 15 -> stage st; rows past the slice are zero, and so are their probabilities
     auto fetch = [&](int kt, int st) {
         if (kt < k1) {
             uint8_t* dst = ring + st * STAGE;
@@ -254,8 +256,8 @@ cached_attention_split_kernel(bf16* __restrict__ out, float* __restrict__ ws, co
                 const int id = i * 32 + lane, row = id / CHUNKS, c = id % CHUNKS;
                 const long long src = min(kt + row, k1 - 1) * row_stride + c * 8;
                 const int off = row * ROWB + ((c ^ (row & 7)) * 16);
-                cp_async16(dst + off, kbase + src);
-                cp_async16(dst + CA_TILE * ROWB + off, vbase + src);
+                cp_async16_or_zero(dst + off, kbase + src, kt + row < k1);
+                cp_async16_or_zero(dst + CA_TILE * ROWB + off, vbase + src, kt + row < k1);
             }
         }
         cp_async_commit();                                     // possibly empty: the group count per tile stays one
@@ -325,15 +327,19 @@ cached_attention_split_kernel(bf16* __restrict__ out, float* __restrict__ ws, co
             #pragma unroll
             for (int n = 0; n < HS_ / 8; n++) { acc[n][0] *= corr; acc[n][1] *= corr; acc[n][2] *= corr; acc[n][3] *= corr; }
         }
-        uint32_t hi[2], md[2], lo[2];                          // 8 bits each, cut off: the differences are exact and not negative
+        // 8 bits each, cut off: the differences are exact and not negative.  No part of a positive probability is zero (which changes it by at
+        // most 2^-31 of its value, or of the smallest normal number), so that its product with an infinite value is that infinity in
+        // all three parts; lo goes through both halves of the operand for the same reason.
+        uint32_t hi[2], md[2], lo[2];
         #pragma unroll
         for (int h = 0; h < 2; h++) {
             hi[h] = top_bf16x2(p[2 * h], p[2 * h + 1]);
             const float2 hf = unpack_bf16x2(hi[h]);
-            const float r0 = p[2 * h] - hf.x, r1 = p[2 * h + 1] - hf.y;
+            const float e0 = least_part(p[2 * h]), e1 = least_part(p[2 * h + 1]);
+            const float r0 = fmaxf(p[2 * h] - hf.x, e0), r1 = fmaxf(p[2 * h + 1] - hf.y, e1);
             md[h] = top_bf16x2(r0, r1);
             const float2 mf = unpack_bf16x2(md[h]);
-            lo[h] = top_bf16x2(r0 - mf.x, r1 - mf.y);
+            lo[h] = top_bf16x2(0.5f * fmaxf(r0 - mf.x, e0), 0.5f * fmaxf(r1 - mf.y, e1));
         }
         // ---- O += P V: 16 keys, 16 channels per ldmatrix
         #pragma unroll
@@ -343,8 +349,8 @@ cached_attention_split_kernel(bf16* __restrict__ out, float* __restrict__ ws, co
             ldmatrix4_trans(vf, vb + row * ROWB + ((c ^ (row & 7)) * 16));
             mma_16x8x16(acc[2 * n2], hi[0], md[0], hi[1], md[1], vf[0], vf[1]);
             mma_16x8x16(acc[2 * n2 + 1], hi[0], md[0], hi[1], md[1], vf[2], vf[3]);
-            mma_16x8x16(acc[2 * n2], lo[0], 0u, lo[1], 0u, vf[0], vf[1]);
-            mma_16x8x16(acc[2 * n2 + 1], lo[0], 0u, lo[1], 0u, vf[2], vf[3]);
+            mma_16x8x16(acc[2 * n2], lo[0], lo[0], lo[1], lo[1], vf[0], vf[1]);
+            mma_16x8x16(acc[2 * n2 + 1], lo[0], lo[0], lo[1], lo[1], vf[2], vf[3]);
         }
         __syncwarp();                                          // the stage may be refilled
         st = st + 1 == CA_STAGES ? 0 : st + 1;

@@ -89,6 +89,25 @@ def test_cached_attention_keeps_fp32_probabilities(HS, start, Tmax):
     assert err < 2.0 ** -6, float(err)
 
 
+@pytest.mark.parametrize("start,Tmax", [(0, 8), (14, 192), (77, 1024), (2000, 2100)])
+@pytest.mark.parametrize("HS", [64, 128])
+def test_cached_attention_with_infinite_values(HS, start, Tmax):
+    """An infinite value gives that infinity in its channel whatever its probability (also one with a single bit), and nothing elsewhere."""
+    B, NH, NKV = 2, 8, 2
+    q, kc, vc = rnd(B, NH * HS), rnd(B, Tmax, NKV, HS, seed=1), rnd(B, Tmax, NKV, HS, seed=2)
+    kc[0] = 0.0                                                # equal scores: every probability of a tile is exactly 1
+    vc[:, start, :, 3], vc[:, start // 2, :, 9] = float("inf"), float("-inf")
+    vc[:, start + 1:] = float("nan")
+    ref = torch.empty(B, NH * HS)
+    R.cached_attention(ref, q, kc, vc, 1, start, NH, NKV)
+    assert ref.isinf().sum() == 2 * B * NH and not ref.isnan().any()
+    out = torch.empty(B, NH * HS, dtype=torch.bfloat16, device=DEV)
+    KN.cached_attention(out, q.to(DEV), kc.to(DEV), vc.to(DEV), 1, start, NH, NKV)
+    got, inf = out.float().cpu(), ref.isinf()
+    assert torch.equal(got[inf], ref[inf])
+    close(got[~inf], ref[~inf], 4e-3, 8e-3)
+
+
 @pytest.mark.parametrize("N,C", [(1, 8), (3, 264), (5, 2048), (1024, 512), (1025, 512), (4, 2056), (2, 8192), (2, 16384), (2, 16392)])
 def test_rmsnorm_forward(N, C):
     a, b, w = rnd(N, C), rnd(N, C, seed=3), rnd(C) + 1.0
