@@ -3,8 +3,8 @@
 //
 // The scheme of the 64-wide kernel (attention_fwd1.cu): a CTA works on TWO adjacent 128-row query tiles (slots A = 2p, B = 2p + 1) of
 // one head and streams the key / value tiles 0..2p+1 past both; one softmax thread owns a whole row of 128 scores in registers; P goes
-// back to tensor memory as bf16 and is the A operand of O += P V; O stays in tensor memory and is rescaled only when the running
-// maximum has moved by more than 2^8.  What 128 channels change:
+// back to tensor memory as bf16 and is the A operand of O += P V; O stays in tensor memory and is rescaled when the running maximum of a
+// row of the warp has moved.  What 128 channels change:
 //   * S and O of both slots take all 512 TMEM columns, so P_X(t) overwrites the scores S_X(t) it came from, and S_X(t+1) is issued
 //     directly behind O_X += P_X(t) V (program order keeps it from overwriting P).  A slot therefore alternates between its softmax
 //     and its products; the other slot's products fill the tensor pipe meanwhile.
@@ -12,7 +12,9 @@
 //     score product: the next item's Q tile arrives while that slot finishes its last softmax and its epilogue.
 // Bound by the softmax of the two slots (1024 exponential cycles per 128 x 128 tile each) with the tensor pipe right behind (2 x 1024
 // cycles per key tile).  Measured, with the kernel this one replaces (16 softmax warps exchanging row statistics, P through shared
-// memory) in brackets: B=16 T=2048 NH=8 HS=128 169 us (256), B=2 T=4096 NH=32 HS=128 271 us (420), B=3 T=1000 NH=32 HS=80 44 us (68).
+// memory) in brackets: B=16 T=2048 NH=8 HS=128 178 us (256), B=2 T=4096 NH=32 HS=128 296 us (422), B=3 T=1000 NH=32 HS=80 47 us (68).
+// Letting the maximum lag by up to 2^8, as the 64-wide kernel does, takes 167 / 274 / 44 us, but then the largest probability of a row is not 1
+// and is rounded to bf16 like the others: the error against 64 bits grows by 1 % (0.00200 -> 0.00204 on the last case).
 // Handing P over in two halves, so that the product starts under the second half's exponentials, was slower (174 / 281 us).
 //
 // Items are dealt to the persistent CTAs heaviest first in alternating direction, which evens out their decreasing lengths.
@@ -34,7 +36,6 @@ constexpr int TMEM_COLS = 512;
 constexpr int SMEM = 2 * TILE_BYTES + RING * TILE_BYTES + 2 * TILE_BYTES + 256;     // Q, K/V ring, two output tiles
 static_assert(SMEM <= 232448, "shared memory of one CTA");
 constexpr long long SKEW_CYCLES = 1200;
-constexpr float RESCALE_LOG2 = 8.0f;                // the running maximum may lag by this much (in log2 units of the scaled scores)
 
 struct Args {
     float* lse;        // (B, NH, T)
@@ -271,10 +272,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
                     mx2 = fmaxf(mx2, __uint_as_float(sv[e + 2])); mx3 = fmaxf(mx3, __uint_as_float(sv[e + 3]));
                 }
                 const float mx = fmaxf(fmaxf(mx0, mx1), fmaxf(mx2, mx3));
-                // move the reference maximum only when it lags by more than 2^RESCALE_LOG2 (decided per warp, so that the
-                // TMEM accesses stay warp-wide); a moved maximum rescales the row sum now and the row of O_X below
-                const bool grow = (mx - m) * c > RESCALE_LOG2 || j == 0;
-                const bool moved = __any_sync(0xffffffffu, grow) != 0;
+                // a moved maximum rescales the row sum now and the row of O_X below (decided per warp, so that the TMEM accesses stay
+                // warp-wide)
+                const bool moved = __any_sync(0xffffffffu, mx > m || j == 0) != 0;
                 float alpha = 1.0f;
                 if (moved) {
                     const float m_new = fmaxf(m, mx);
@@ -283,16 +283,16 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
                     m = m_new;
                 }
                 const float moff = m * c;
-                float rs0 = 0.f, rs1 = 0.f;
+                float rs[4] = {0.f, 0.f, 0.f, 0.f};
                 uint32_t pk[64];
                 #pragma unroll
                 for (int e = 0; e < 128; e += 2) {
                     const float p0 = ex2_fast(fmaf(__uint_as_float(sv[e]), c, -moff));
                     const float p1 = ex2_fast(fmaf(__uint_as_float(sv[e + 1]), c, -moff));
-                    rs0 += p0; rs1 += p1;
+                    rs[(e >> 1) & 3] += p0 + p1;
                     pk[e >> 1] = pack_bf16x2(p0, p1);
                 }
-                l += rs0 + rs1;
+                l += (rs[0] + rs[1]) + (rs[2] + rs[3]);
                 tmem_st16(tS, pk);                          // over this row's own scores
                 tmem_st16(tS + 16, pk + 16);
                 tmem_st16(tS + 32, pk + 32);

@@ -52,3 +52,27 @@ def test_backward(B, T, NH, hs):
     assert torch.equal(got[0], got[1])
     # delta uses the bf16 output: its rounding (2^-9 of |O| |dO| over hs channels) times P stays below 2e-2 beside the bf16 results
     close(got[0].view(B, T, -1), rd, 4e-2, 3e-2)
+
+
+@pytest.mark.parametrize("HS", [80, 128])
+def test_the_largest_probability_of_a_row_is_exact(HS):
+    """Rows whose largest score (4 to 5.5 above an earlier key's) comes with their second key tile and makes up nearly all of the sum: with the
+    probability of that key exactly 1, the error is little more than that of rounding the result to bf16."""
+    B, T, NH, lo = 1, 256, 2, 128
+    g = torch.Generator().manual_seed(HS)
+    q, k = torch.zeros(B, T, NH, HS), torch.zeros(B, T, NH, HS)
+    v = torch.randn(B, T, NH, HS, generator=g)
+    q[:, lo:, :, 0] = torch.linspace(4.0, 5.5, T - lo)[:, None] * HS ** 0.5
+    q[..., 1] = HS ** 0.5
+    k[..., 1] = -20.0
+    k[:, 0, :, 1] = k[:, lo, :, 1] = 0.0
+    k[:, lo, :, 0] = 1.0
+    qkv = torch.stack([q, k, v], 2).bfloat16()
+    qd, kd, vd = qkv.double().unbind(2)
+    s = (torch.einsum("bthd,bshd->bhts", qd, kd) / HS ** 0.5).masked_fill(torch.ones(T, T, dtype=torch.bool).triu(1), -float("inf"))
+    exact = torch.einsum("bhts,bshd->bthd", torch.softmax(s, -1), vd)[:, lo:]
+    out = torch.empty(B, T, NH * HS, dtype=torch.bfloat16, device="cuda")
+    lse = torch.empty(B, NH, T, device="cuda")
+    KN.attention_forward(out, lse, qkv.view(B, T, 3 * NH * HS).cuda(), B, T, NH)
+    err = (out.cpu().view(B, T, NH, HS)[:, lo:].double() - exact).norm()
+    assert err < 1.1 * (exact.bfloat16().double() - exact).norm()
