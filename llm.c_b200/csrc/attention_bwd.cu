@@ -351,11 +351,15 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
                     p[h2 * 32 + e4 * 4 + 2] = ex2_fast(x1.x); p[h2 * 32 + e4 * 4 + 3] = ex2_fast(x1.y);
                 }
             }
-            // only the diagonal tile needs a mask (query >= key).  Rows and columns past T need none beyond it: queries past T have
-            // LSE = +inf, and a key past T is seen by no query before T.
+            // the diagonal tile needs a mask (query >= key).  Keys past T need none beyond it, as no query before T sees them.  Queries past T
+            // have LSE = +inf, which leaves 0 except where an infinite key made their zero rows' score NaN.
             if (diag) {
                 #pragma unroll
                 for (int e = 0; e < 64; e++) if (DKV ? hf * 64 + e < r : hf * 64 + e > r) p[e] = 0.f;
+            }
+            if (DKV && (wk.x + 1) * BT > a.T) {
+                #pragma unroll
+                for (int e = 0; e < 64; e++) if (wk.x * BT + hf * 64 + e >= a.T) p[e] = 0.f;
             }
             if (DKV) {
                 uint32_t pk[32];

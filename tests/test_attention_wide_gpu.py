@@ -76,3 +76,24 @@ def test_the_largest_probability_of_a_row_is_exact(HS):
     KN.attention_forward(out, lse, qkv.view(B, T, 3 * NH * HS).cuda(), B, T, NH)
     err = (out.cpu().view(B, T, NH, HS)[:, lo:].double() - exact).norm()
     assert err < 1.1 * (exact.bfloat16().double() - exact).norm()
+
+
+@pytest.mark.parametrize("T,HS", [(100, 80), (333, 128)])
+def test_backward_with_a_key_of_score_minus_infinity(T, HS):
+    """A key that no query gives any weight: the gradients of keys and values do not depend on whether its scores are -inf or very negative, also
+    where the last query tile is ragged."""
+    B, NH, at = 2, 2, 40
+    g = torch.Generator().manual_seed(T)
+    qkv = torch.randn(B, T, 3, NH, HS, generator=g)
+    qkv[:, :, 0, :, 0] = qkv[:, :, 0, :, 0].abs() + 0.5
+    dout = torch.randn(B, T, NH * HS, generator=g).bfloat16().cuda()
+    grads = []
+    for low in (-1e30, -float("inf")):
+        qkv[:, at, 1, :, 0] = low
+        x = qkv.bfloat16().view(B, T, 3 * NH * HS).cuda()
+        out, lse, dqkv = torch.empty_like(dout), torch.empty(B, NH, T, device=DEV), torch.empty_like(x)
+        KN.attention_forward(out, lse, x, B, T, NH)
+        KN.attention_backward(dqkv, dout, x, out, lse, B, T, NH)
+        assert out.isfinite().all() and lse.isfinite().all()
+        grads.append(dqkv.view(B, T, 3, NH, HS)[:, :, 1:].clone())
+    assert grads[1].isfinite().all() and torch.equal(*grads)
