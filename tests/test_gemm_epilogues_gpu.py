@@ -51,3 +51,19 @@ def test_weight_gradient_without_split(rows, OC, C, accumulate):
     R.matmul_wgrad(ref, dy, x, accumulate=accumulate)
     close(buf[:OC], ref, 5e-2, 1.5e-2)
     assert (buf[OC:] == 7.0).all()
+
+
+@pytest.mark.parametrize("two_sm", [False, True])
+def test_gelu_gradient_of_large_inputs(two_sm, monkeypatch):
+    """Far from zero the derivative is exactly 0 or 1, up to the largest x whose square is finite: stand-alone and in both GEMM epilogues."""
+    monkeypatch.setattr(KN, "TWO_SM_MIN_TILES", 1 if two_sm else 0)
+    x = torch.tensor([s * m * 10.0 ** e for e in range(1, 19) for m in (1.0, 3.0) for s in (1.0, -1.0)]).bfloat16()
+    want = (x > 0).float()
+    d = torch.ones_like(x).to(DEV)
+    KN.gelu_backward_inplace(d, x.to(DEV))
+    assert torch.equal(d.float().cpu(), want)
+    M, N = 256, x.numel()
+    pre, dy, w = x.expand(M, N).contiguous(), torch.ones(M, 8), torch.full((8, N), 0.125)
+    out = torch.empty(M, N, dtype=torch.bfloat16, device=DEV)
+    KN.matmul_dgrad(out, dy.bfloat16().to(DEV), w.bfloat16().to(DEV), pre_gelu=pre.to(DEV))
+    assert torch.equal(out.float().cpu(), want.expand(M, N))
