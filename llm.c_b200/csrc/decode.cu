@@ -432,6 +432,82 @@ __global__ void cached_attention_combine_kernel(bf16* __restrict__ out, const fl
     out[((b * Tq + t) * NH + hq) * HS_ + c] = __float2bfloat16_rn(a / ls);
 }
 
+// ---------------------------------------------------------------------------------------------------------------
+// Skinny product, launched by itself: out (M, N) = x (M, K) . w (N, K)^T with M <= 8 rows.  It is bound by streaming the weights once.
+// stream_gemm.cu does the same product faster inside a replayed step, where it starts and prefetches under its predecessor, but slower
+// alone (us, this kernel first): 4 x 28672 x 4096 50 / 59, 4 x 49152 x 4096 76 / 90, 4 x 6144 x 4096 16 / 20, 1 x 768 x 768 8 / 10; 4 x 2048 x 7168
+// is the exception at 18 / 16.  Here a CTA owns 16 output columns and its 8 warps split K; a warp feeds warp-level
+// m16n8k16 MMAs with the weights as the 16-row operand and the (at most 8) activation rows as the 8-column operand, so that
+// the arithmetic costs two instructions per KB of weights and the loop is nothing but 128-bit streaming loads.  A lane
+// loads 8 consecutive K elements of weight rows g and g + 8 and of activation row g (g = lane / 4) and uses them as the
+// K slots of two MMAs; the dot product does not care that this permutes K, as long as both operands agree.
+constexpr int SK_WARPS = 8;
+constexpr int SK_THREADS = SK_WARPS * 32;
+constexpr int SK_COLS = 16;
+constexpr int SK_UNROLL = 4;
+constexpr int SK_MAX_M = 8;
+
+__global__ void __launch_bounds__(SK_THREADS)
+skinny_gemm_kernel(bf16* __restrict__ out, const bf16* __restrict__ x, const bf16* __restrict__ w, int M, int N, int K,
+                   int ldx, int ldw, int ldo) {
+    __shared__ float red[SK_WARPS][4][32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int g = lane >> 2, t = lane & 3;
+    const int n0 = blockIdx.x * SK_COLS;
+    const bf16* w0 = w + (size_t)min(n0 + g, N - 1) * ldw;          // a clamped row is computed, not stored
+    const bf16* w1 = w + (size_t)min(n0 + g + 8, N - 1) * ldw;
+    const bool xvalid = g < M;
+    const bf16* xr = x + (size_t)min(g, M - 1) * ldx;
+    const int nchunks = (K + 31) >> 5;                               // 32 K elements per chunk: 8 per lane of a quad
+    const int per_warp = (nchunks + SK_WARPS - 1) / SK_WARPS;
+    const int c_begin = warp * per_warp, c_end = min(c_begin + per_warp, nchunks);
+    float c[4] = {0.f, 0.f, 0.f, 0.f};
+    const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+    // whole groups of SK_UNROLL full chunks: every load is issued before the first MMA, nothing is predicated
+    const int full_end = min(c_end, K >> 5);
+    int ch = c_begin;
+    for (; ch + SK_UNROLL <= full_end; ch += SK_UNROLL) {
+        uint4 a0[SK_UNROLL], a1[SK_UNROLL], b[SK_UNROLL];
+        #pragma unroll
+        for (int u = 0; u < SK_UNROLL; u++) {
+            const int k = ((ch + u) << 5) + t * 8;
+            a0[u] = __ldcs(reinterpret_cast<const uint4*>(w0 + k));
+            a1[u] = __ldcs(reinterpret_cast<const uint4*>(w1 + k));
+            b[u] = *reinterpret_cast<const uint4*>(xr + k);
+        }
+        #pragma unroll
+        for (int u = 0; u < SK_UNROLL; u++) {
+            if (!xvalid) b[u] = zero;
+            mma_16x8x16(c, a0[u].x, a1[u].x, a0[u].y, a1[u].y, b[u].x, b[u].y);
+            mma_16x8x16(c, a0[u].z, a1[u].z, a0[u].w, a1[u].w, b[u].z, b[u].w);
+        }
+    }
+    // the rest, one chunk at a time; the last chunk of K may be partial
+    for (; ch < c_end; ch++) {
+        const int k = (ch << 5) + t * 8;
+        const bool ok = k < K;
+        const uint4 a0 = ok ? __ldcs(reinterpret_cast<const uint4*>(w0 + k)) : zero;
+        const uint4 a1 = ok ? __ldcs(reinterpret_cast<const uint4*>(w1 + k)) : zero;
+        const uint4 b = (ok && xvalid) ? *reinterpret_cast<const uint4*>(xr + k) : zero;
+        mma_16x8x16(c, a0.x, a1.x, a0.y, a1.y, b.x, b.y);
+        mma_16x8x16(c, a0.z, a1.z, a0.w, a1.w, b.z, b.w);
+    }
+    #pragma unroll
+    for (int i = 0; i < 4; i++) red[warp][i][lane] = c[i];
+    __syncthreads();
+    if (warp == 0) {
+        // accumulator layout: c[2 i + j] = out[row 2 t + j][column n0 + g + 8 i]
+        #pragma unroll
+        for (int i = 0; i < 4; i++) {
+            float v = 0.f;
+            #pragma unroll
+            for (int ww = 0; ww < SK_WARPS; ww++) v += red[ww][i][lane];
+            const int m = 2 * t + (i & 1), n = n0 + g + 8 * (i >> 1);
+            if (m < M && n < N) out[(size_t)m * ldo + n] = __float2bfloat16_rn(v);
+        }
+    }
+}
+
 int decode_check(int B, int Tq, int Tmax, int start_pos, int NH, int NKV, int HS, bool device_pos) {
     if (HS % 8 || HS > DEC_MAX_HS || HS < 16 || NKV <= 0 || NH % NKV) return -1;
     if (B <= 0 || Tq <= 0 || Tq > Tmax) return -2;
@@ -515,6 +591,15 @@ extern "C" int llmc_cached_attention(bf16* out, const bf16* q, const bf16* kcach
     const dim3 grid(NH, Tq, B);
     cached_attention_kernel<<<grid, DEC_THREADS, 0, stream>>>(out, q, kcache, vcache, Tq, Tmax, start_pos, NH, NKV, HS, rsqrtf((float)HS),
                                                               pos_ptr, llmc_status_ptr());
+    CUDA_CHECK(cudaGetLastError());
+    return 0;
+}
+
+// out (M, N) = x (M, K) . w (N, K)^T for M <= 8; K and the row strides of x and w are multiples of 8 elements.
+extern "C" int llmc_skinny_gemm(bf16* out, const bf16* x, const bf16* w, int M, int N, int K, int ldx, int ldw, int ldo, cudaStream_t stream) {
+    if (M <= 0 || M > SK_MAX_M || N <= 0 || K <= 0 || (K % 8) || (ldx % 8) || (ldw % 8)) return -1;
+    if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w)) & 15) return -1;
+    skinny_gemm_kernel<<<(unsigned)CEIL_DIV(N, SK_COLS), SK_THREADS, 0, stream>>>(out, x, w, M, N, K, ldx, ldw, ldo);
     CUDA_CHECK(cudaGetLastError());
     return 0;
 }

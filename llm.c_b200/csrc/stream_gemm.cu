@@ -16,7 +16,7 @@
 // 32 x 6144 x 4096 23 us (38), 32 x 28672 x 4096 58 us (69), 100 x 2048 x 7168 23 us (52).  Inside a replayed decoding step (4 rows, 4 layers
 // of 2048 channels, LM head of 128256 rows) this kernel takes the step to 277 us; a weight-streaming kernel on warp-level MMAs with the same
 // early launch and prefetch, used for the products of at most 8 rows, left it at 290 us (at 284 us for the LM head alone), although launched
-// by itself it took wide ones faster (4 x 28672 x 4096 50 us against 59).  More rows: 256 x 768 x 50304 (an input gradient)
+// by itself it is faster (4 x 28672 x 4096 50 us against 59; skinny_gemm_kernel in decode.cu).  More rows: 256 x 768 x 50304 (an input gradient)
 // 60 us (291), 777 x 2048 x 7168 37 us (53), 256 x 768 x 3072 18 us (27).
 //
 // Warps of a CTA: 0 TMA producer, 1 MMA issuer, 2-5 epilogue.  Two CTAs fit an SM.
@@ -301,10 +301,4 @@ extern "C" int llmc_stream_gemm(bf16* out, const bf16* x, const bf16* w, const b
 extern "C" int llmc_stream_gemm_swiglu(bf16* out, const bf16* x, const bf16* w, int M, int N, int K, int ldx, int ldw, int ldo, cudaStream_t stream) {
     if (N % 64 || M > 128) return -1;
     return launch_stream<SWIGLU, false>(out, x, w, nullptr, M, N, K, ldx, ldw, ldo, stream);
-}
-
-// The plain product for the at most 8 rows of a decoding step
-extern "C" int llmc_skinny_gemm(bf16* out, const bf16* x, const bf16* w, int M, int N, int K, int ldx, int ldw, int ldo, cudaStream_t stream) {
-    if (M > 8) return -1;
-    return launch_stream<STORE, false>(out, x, w, nullptr, M, N, K, ldx, ldw, ldo, stream);
 }

@@ -43,12 +43,9 @@ class CachedDecoder:
         self.dense_prefill_from = 128
         # products run on rows padded to whole 128-row tiles
         self.whole_tiles = model.device.type == "cuda"
-        # steps of at most this many rows use the weight-streaming product instead of a padded tensor-core tile (0: never)
-        own = model.device.type == "cuda" and model.dtype == torch.bfloat16
-        self.skinny_rows = 8 if own else 0
-        # steps of at most this many rows run their products on exactly their rows (split-K weight streaming, csrc/stream_gemm.cu), the
-        # MLP's up-projections with the activation in the same launch; longer ones on rows padded to whole 128-row tiles
-        self.stream_rows = 128 if own else 0
+        # steps of at most this many rows run their products on exactly their rows (split-K weight streaming, csrc/stream_gemm.cu), the MLP's
+        # up-projections with the activation in the same launch, instead of on rows padded to whole 128-row tiles (0: never)
+        self.skinny_rows = 128 if model.device.type == "cuda" and model.dtype == torch.bfloat16 else 0
 
     def cache_bytes(self):
         return 2 * self.kcache.numel() * self.kcache.element_size()
@@ -87,11 +84,7 @@ class CachedDecoder:
         x, ln, rstd = a["x"], a["ln"], a["rstd"]
 
         def mm(out, inp, weight, n):
-            if n <= self.skinny_rows:
-                ops.matmul_skinny(out[:n], inp[:n], weight)
-            elif n <= self.stream_rows:
-                ops.matmul_forward(out[:n], inp[:n], weight, None)
-            elif self.whole_tiles:
+            if self.whole_tiles and n > self.skinny_rows:
                 r = _whole_tiles(n)                                 # of both operands: either may have more rows than this product
                 ops.matmul_forward(out[:r], inp[:r], weight, None)  # the rows beyond n are never read
             else:
@@ -121,7 +114,7 @@ class CachedDecoder:
                 ops.cached_attention(a["atty"][:N], a["q"][:N], self.kcache[l], self.vcache[l], Tq, start_pos, NH, NKV, pos)
             mm(a["proj"], a["atty"], p["attprojw"][l], N)
             ops.rmsnorm_fused_residual_forward(a["res"][:N], ln[:N], rstd[:N], x[:N], a["proj"][:N], p["ln2w"][l], eps)
-            if N <= self.stream_rows and cfg.hidden_dim % 64 == 0:
+            if N <= min(self.skinny_rows, 128) and cfg.hidden_dim % 64 == 0:
                 ops.matmul_swiglu(a["h"][:N], ln[:N], p["fc12w"][l])
             else:
                 mm(a["fc12"], ln, p["fc12w"][l], N)

@@ -408,7 +408,8 @@ def _check_strided(op, *need):
 
 
 def matmul_skinny(out, inp, weight):
-    """out[M,OC] = inp[M,C] @ weight[OC,C]^T for at most 8 rows: the weight-streaming kernel of decoding steps (csrc/stream_gemm.cu)."""
+    """out[M,OC] = inp[M,C] @ weight[OC,C]^T for at most 8 rows on warp-level MMAs (csrc/decode.cu); ``matmul_forward`` takes such products too, faster
+    behind another kernel of this library and slower alone."""
     global _launches
     M, C = inp.shape
     OC = weight.shape[0]

@@ -224,7 +224,7 @@ def test_cached_decoder_and_generate():
     a = G.generate(m, prompts, max_gen_len=12, temperature=0.0, echo=True, decoder=d1)
     b = G.generate(m, prompts, max_gen_len=12, temperature=0.0, echo=True, use_kv=False, decoder=d2)
     assert a == b
-    assert len(G.generate(m, prompts, max_gen_len=12, temperature=0.0)[0]) == 12          # default path: skinny product + graph
+    assert len(G.generate(m, prompts, max_gen_len=12, temperature=0.0)[0]) == 12          # default path: exact rows + graph
     for p, out in zip(prompts, a):
         assert out[:len(p)] == p and len(out) == len(p) + 12
 
@@ -367,3 +367,14 @@ def test_replayed_decoding_keeps_its_buffers():
             poison = [torch.full((n // 4,), float("nan"), device=DEV) for n in sizes for _ in range(2)]
         assert torch.equal(gs.step(tok[:, t:t + 1]), want), "position %d" % t
     assert all(p.isnan().all() for p in poison)
+
+
+def test_skinny_product_of_a_repeated_row():
+    """Rows that are one row of memory (stride 0), or whose stride is shorter than a row."""
+    x, w = rnd(5 * 8 + 512), rnd(264, 512, scale=0.05, seed=1)
+    for inp in (x[:512].expand(4, 512), x.as_strided((5, 512), (8, 1))):
+        out = torch.empty(inp.shape[0], 264, dtype=torch.bfloat16, device=DEV)
+        KN.matmul_skinny(out, x.to(DEV).as_strided(inp.shape, inp.stride()), w.to(DEV))
+        ref = torch.empty(inp.shape[0], 264)
+        R.matmul_skinny(ref, inp, w)
+        close(out, ref, 2e-2, 1e-2, "matmul_skinny")
