@@ -85,10 +85,9 @@ class CachedDecoder:
 
         def mm(out, inp, weight, n):
             if self.whole_tiles and n > self.skinny_rows:
-                r = _whole_tiles(n)                                 # of both operands: either may have more rows than this product
-                ops.matmul_forward(out[:r], inp[:r], weight, None)  # the rows beyond n are never read
-            else:
-                ops.matmul_forward(out[:n], inp[:n], weight, None)
+                n = _whole_tiles(n)                             # the rows beyond n are never read
+            # of both operands: either may have more rows than this product
+            ops.matmul_forward(out if out.shape[0] == n else out[:n], inp if inp.shape[0] == n else inp[:n], weight, None)
 
         ops.encoder_forward(x[:N].view(B, Tq, C), tokens, p["wte"], None)
         ops.rmsnorm_forward(ln[:N], rstd[:N], x[:N], p["ln1w"][0], eps)

@@ -37,12 +37,16 @@ def _p(t):
     return ctypes.c_void_p(t.data_ptr()) if t is not None else ctypes.c_void_p(0)
 
 
+class _Taken(threading.local):
+    by = None                                # list that collects what this thread's calls take (scratch_taken)
+
+
 class _Scratch:
     """Per-device scratch buffers that grow to the largest request and are then reused."""
 
     def __init__(self):
         self.bufs = {}
-        self.taken = threading.local()       # .by: list that collects what this thread's calls take (scratch_taken)
+        self.taken = _Taken()
 
     def get(self, key, numel, dtype, device, zero=False):
         k = (key, device.index, dtype)
@@ -50,9 +54,8 @@ class _Scratch:
         if t is None or t.numel() < numel:
             t = (torch.zeros if zero else torch.empty)(max(int(numel), 1), dtype=dtype, device=device)
             self.bufs[k] = t
-        by = getattr(self.taken, "by", None)
-        if by is not None:
-            by.append(t)
+        if self.taken.by is not None:
+            self.taken.by.append(t)
         return t
 
 
@@ -63,7 +66,7 @@ _scratch = _Scratch()
 def scratch_taken():
     """A list of the scratch buffers that this thread's calls take inside the block.  A later call that needs a larger one replaces a buffer, so
     a CUDA graph captured in the block has to keep the list."""
-    outer = getattr(_scratch.taken, "by", None)
+    outer = _scratch.taken.by
     _scratch.taken.by = by = []
     try:
         yield by
@@ -147,11 +150,9 @@ def gemm(a, b, d, M, N, K, lda, ldb, ldd, a_mn, b_mn, mode, bias=None, aux=None,
                         int(accumulate), splits, _p(ws), _p(cnt), max_ctas, _stream()), "llmc_gemm")
 
 
-def _check_sizes(op, *need):
+def _too_small(op, **tensors):
     """The launchers take the sizes of a product from two of its operands; the others have to be at least that large."""
-    for what, t, n in need:
-        if t is not None and t.numel() < n:
-            raise ValueError("%s: %s of shape %s, but the product needs %d elements of it" % (op, what, tuple(t.shape), n))
+    return ValueError("%s: operands of shapes %s do not fit one product" % (op, {n: tuple(t.shape) for n, t in tensors.items() if t is not None}))
 
 
 def matmul_forward(out, inp, weight, bias=None, pre_gelu=None, ready=None):
@@ -159,7 +160,9 @@ def matmul_forward(out, inp, weight, bias=None, pre_gelu=None, ready=None):
     ``out`` receives its tanh-GELU (reference: matmul_forward_cublaslt, llmc/matmul.cuh:230-242)."""
     M, C = inp.shape
     OC = weight.shape[0]
-    _check_sizes("matmul_forward", ("out", out, M * OC), ("weight", weight, OC * C), ("bias", bias, OC), ("pre_gelu", pre_gelu, M * OC))
+    n = M * OC
+    if out.numel() < n or weight.numel() < OC * C or (bias is not None and bias.numel() < OC) or (pre_gelu is not None and pre_gelu.numel() < n):
+        raise _too_small("matmul_forward", out=out, inp=inp, weight=weight, bias=bias, pre_gelu=pre_gelu)
     mode = MODE_GELU if pre_gelu is not None else MODE_STORE
     gemm(inp, weight, out, M, OC, C, C, C, OC, 0, 0, mode, bias=bias, aux=pre_gelu, ready=ready)
 
@@ -169,7 +172,9 @@ def matmul_dgrad(dinp, dout, weight, pre_gelu=None):
     (reference: matmul_backward dgrad with the DGELU epilogue, llmc/matmul.cuh:279-285)."""
     M, OC = dout.shape
     C = weight.shape[1]
-    _check_sizes("matmul_dgrad", ("dinp", dinp, M * C), ("weight", weight, OC * C), ("pre_gelu", pre_gelu, M * C))
+    n = M * C
+    if dinp.numel() < n or weight.shape[0] < OC or (pre_gelu is not None and pre_gelu.numel() < n):
+        raise _too_small("matmul_dgrad", dinp=dinp, dout=dout, weight=weight, pre_gelu=pre_gelu)
     mode = MODE_DGELU if pre_gelu is not None else MODE_STORE
     gemm(dout, weight, dinp, M, C, OC, OC, C, C, 0, 1, mode, aux=pre_gelu)
 
@@ -178,7 +183,8 @@ def matmul_wgrad(dweight, dout, inp, accumulate=True):
     """dweight[OC,C] (+)= dout[M,OC]^T @ inp[M,C] with split-K sized to fill the SMs."""
     M, OC = dout.shape
     C = inp.shape[1]
-    _check_sizes("matmul_wgrad", ("dweight", dweight, OC * C), ("inp", inp, M * C))
+    if dweight.numel() < OC * C or inp.shape[0] < M:
+        raise _too_small("matmul_wgrad", dweight=dweight, dout=dout, inp=inp)
     splits = _lib.cuda().llmc_gemm_pick_splits(OC, C, M, sm_count(dout.device))
     gemm(dout, inp, dweight, OC, C, M, OC, C, C, 1, 1, MODE_ACCUM, accumulate=accumulate, splits=splits)
 
@@ -400,20 +406,14 @@ def cached_attention(out, q, kcache, vcache, Tq, start_pos, NH, NKV, pos=None):
           "llmc_cached_attention")
 
 
-def _check_strided(op, *need):
-    """``_check_sizes`` for products that take row strides: rows and columns of every other operand."""
-    for what, t, rows, cols in need:
-        if t.shape[0] < rows or t.numel() < cols * t.shape[0]:
-            raise ValueError("%s: %s of shape %s, but the product needs (%d, %d)" % (op, what, tuple(t.shape), rows, cols))
-
-
 def matmul_skinny(out, inp, weight):
     """out[M,OC] = inp[M,C] @ weight[OC,C]^T for at most 8 rows on warp-level MMAs (csrc/decode.cu); ``matmul_forward`` takes such products too, faster
     behind another kernel of this library and slower alone."""
     global _launches
     M, C = inp.shape
     OC = weight.shape[0]
-    _check_strided("matmul_skinny", ("out", out, M, OC), ("weight", weight, OC, C))
+    if out.shape[0] < M or out.shape[-1] < OC or weight.shape[1] < C:
+        raise _too_small("matmul_skinny", out=out, inp=inp, weight=weight)
     _launches += 1
     check(_lib.cuda().llmc_skinny_gemm(_p(out), _p(inp), _p(weight), M, OC, C, inp.stride(0), weight.stride(0), out.stride(0), _stream()),
           "llmc_skinny_gemm")
@@ -425,7 +425,8 @@ def matmul_swiglu(h, inp, weight12):
     global _launches
     M, C = inp.shape
     H = weight12.shape[0] // 2
-    _check_strided("matmul_swiglu", ("h", h, M, H), ("weight12", weight12, 2 * H, C))
+    if h.shape[0] < M or h.shape[-1] < H or weight12.shape[1] < C:
+        raise _too_small("matmul_swiglu", h=h, inp=inp, weight12=weight12)
     _launches += 1
     check(_lib.cuda().llmc_stream_gemm_swiglu(_p(h), _p(inp), _p(weight12), M, H, C, inp.stride(0), weight12.stride(0), h.stride(0), _stream()),
           "llmc_stream_gemm_swiglu")
