@@ -72,7 +72,8 @@ def main(argv=None):
     def hook(layer):
         if recording["on"]:
             mark("bwd_end[%d]" % layer)
-        orig_hook(layer)
+        if orig_hook is not None:               # one process: nothing to reduce
+            orig_hook(layer)
         if recording["on"] and hasattr(be, "stream") and be.stream is not None:
             mark("reduce_end[%d]" % layer, be.stream)
     m.grad_hook = hook

@@ -1,5 +1,6 @@
 """The bf16 sm_100a path against the fp32 CPU path of the same model code (the scheme of the reference's test_gpt2.cu:
 logits, loss, per-tensor gradients with bf16 tolerances, a few optimizer steps, and bit-exact determinism)."""
+import json
 import math
 
 import pytest
@@ -151,3 +152,11 @@ def test_optimizer_state_in_managed_memory_trains_identically(monkeypatch):
         del opt, m
     for a, b in zip(runs[0], runs[1]):
         assert torch.equal(a, b)
+
+
+def test_step_timeline_tool_on_one_gpu(capsys):
+    from llmc_b200 import bench_step_timeline
+    bench_step_timeline.main(["--model", "d6", "-b", "2", "-t", "64", "--total-batch", "256", "--steps", "4"])
+    out = capsys.readouterr().out
+    times = json.loads(out[out.index("{"):out.rindex("}") + 1])["ms_since_start_of_last_micro_step (max over ranks)"]
+    assert times["forward end"] < times["backward of layer 5 end"] < times["backward of layer 0 end"] < times["all parameters published"]
