@@ -22,6 +22,9 @@ class StepGraphs:
     def __init__(self):
         self._entries = {}
 
+    def __reduce__(self):
+        return StepGraphs, ()              # a copied or unpickled model captures graphs of its own buffers
+
     def clear(self):
         self._entries.clear()
 

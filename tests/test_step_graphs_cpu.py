@@ -1,10 +1,12 @@
 """When a micro-step may be replayed: every buffer that its launches read or write is the one they were captured with."""
+import copy
+import pickle
 from types import SimpleNamespace
 
 import pytest
 import torch
 
-from llmc_b200.models import step_graphs
+from llmc_b200.models import gpt2, step_graphs
 from llmc_b200.ops import kernels as KN
 
 
@@ -46,3 +48,15 @@ def test_a_capture_holds_the_scratch_buffers_it_took_and_no_others():
     finally:
         for k in [k for k in KN._scratch.bufs if k[0].startswith("test_")]:
             del KN._scratch.bufs[k]
+
+
+def test_a_model_with_captured_steps_can_be_copied_and_pickled():
+    m = gpt2.GPT(gpt2.GPTConfig(32, 100, 128, 1, 2, 64), "cpu", torch.float32)
+    m.init_random(1)
+    m.step_graphs._entries["forward"] = {"graph": (i for i in ())}             # like a CUDA graph, it can be neither copied nor pickled
+    for c in (copy.deepcopy(m), pickle.loads(pickle.dumps(m))):
+        assert torch.equal(c.params_flat, m.params_flat) and not c.step_graphs._entries
+        tok = torch.arange(32, dtype=torch.int32).view(1, 32)
+        c.forward(tok, tok)
+        m.forward(tok, tok)
+        assert torch.equal(c.loss(), m.loss())
