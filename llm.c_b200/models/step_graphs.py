@@ -1,12 +1,12 @@
 """CUDA graphs of a model's forward and backward launches.
 
 A micro-step of a small batch is bound by the host: a 12-layer GPT-2 issues about 260 kernel launches of a few microseconds each, and the
-launcher takes longer than the kernel (forward + backward of 4 x 64 tokens of GPT-2 124M: 4.46 ms launched, 3.01 ms replayed, 2.9 of them kernels).  ``StepGraphs.run`` executes
-a launch sequence eagerly the first two times it sees its key and from the third time on replays a graph of it.
+launcher takes longer than the kernel (forward + backward of 4 x 64 tokens of GPT-2 124M: 4.5 ms launched, 2.4 ms replayed).
+``StepGraphs.run`` executes a launch sequence eagerly the first two times it sees its key and from the third time on replays a graph of it.
 
 What makes a replay equal to the eager call: the sequence only reads and writes buffers that the model owns (inputs are copied into them
-before), all scalar arguments are part of the key, and so are the addresses of every parameter, gradient and activation buffer and of the rotary table.  The scratch buffers
-of the operators are shared by all callers and replaced when one needs a larger one, so a graph keeps those that its own operators took.
+before), all scalar arguments are part of the key, and the addresses of every parameter, gradient and activation buffer and of the rotary
+table are compared.  The scratch buffers of the operators are shared by all callers and replaced when one needs a larger one, so a graph keeps those that its own operators took.
 """
 import torch
 

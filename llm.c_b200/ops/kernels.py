@@ -91,8 +91,9 @@ def _few_rows(M, N, K, mode, b_mn, device):
     two kernels (M from 100 to 2048, fourteen pairs of N and K, us): deep products whose tiles leave at least half of the SMs idle
     (K = 3072: 24 tiles 21 against 27, 36 tiles 33 against 27; K = 7168: 64 tiles 37 to 43 against 53, 96 tiles 61 against 55), and
     at most 128 rows, unless there are so many tiles that the overlap of tiles on a persistent CTA counts (100 x 50304 x 768:
-    39 against 31) or the product is a shallow input gradient (100 x 768 x 768: 16 against 14).  Forward products below a depth of 6144
-    keep their one sum over K: at 8 us each (256 x 768 x 3072: 18 against 27) they are not worth another order of summation in the loss."""
+    39 against 31) or the product is a shallow input gradient (100 x 768 x 768: 16 against 14).  Forward products of more than 128 rows
+    below a depth of 6144 keep their one sum over K: at 8 us each (256 x 768 x 3072: 18 against 27) they are not worth another order of
+    summation in the loss.  At most 128 rows are summed in slices from K = 512 on, in fp32 and in slice order."""
     if mode != MODE_STORE:
         return False
     wtiles = (N + 127) // 128

@@ -53,15 +53,15 @@ def case(op):
         a, w, b = _bf(Ms, Ks), _bf(Ns, Ks, scale=0.02), _bf(Ns)
         out = torch.empty(Ms, Ns, device=DEV, dtype=torch.bfloat16)
         return (lambda: K.matmul_forward(out, a, w, b)), 2.0 * (Ms * Ks + Ns * Ks + Ms * Ns), 2.0 * Ms * Ns * Ks
-    if op in ("attn_fwd", "attn_bwd"):
-        B, T, NH = 16, 1024, 12
-        qkv, dout = _bf(B, T, 3 * NH * 64), _bf(B, T, NH * 64)
-        out = torch.empty(B, T, NH * 64, device=DEV, dtype=torch.bfloat16)
+    if op in ("attn_fwd", "attn_bwd", "attn_fwd_wide", "attn_bwd_wide"):
+        B, T, NH, HS = (16, 2048, 8, 128) if op.endswith("wide") else (16, 1024, 12, 64)
+        qkv, dout = _bf(B, T, 3 * NH * HS), _bf(B, T, NH * HS)
+        out = torch.empty(B, T, NH * HS, device=DEV, dtype=torch.bfloat16)
         lse = torch.empty(B, NH, T, device=DEV)
         dqkv = torch.empty_like(qkv)
         K.attention_forward(out, lse, qkv, B, T, NH)
-        causal = 4.0 * B * NH * T * T * 64 / 2
-        if op == "attn_fwd":
+        causal = 4.0 * B * NH * T * T * HS / 2
+        if op.startswith("attn_fwd"):
             return (lambda: K.attention_forward(out, lse, qkv, B, T, NH)), 2.0 * (qkv.numel() + out.numel()), causal
         return (lambda: K.attention_backward(dqkv, dout, qkv, out, lse, B, T, NH)), 2.0 * (2 * qkv.numel() + 2 * out.numel()), 2.5 * causal      # five products per tile pair
     if op in ("ln_fwd", "fused_residual", "ln_bwd", "ln_bwd_colsum"):
@@ -140,12 +140,13 @@ def case(op):
         if op == "swiglu_fwd":
             return (lambda: K.swiglu_forward(h, x12)), 2.0 * 3 * N * H, 0.0
         return (lambda: K.swiglu_backward(dx12, dh, x12)), 2.0 * 5 * N * H, 0.0
-    if op in ("skinny_gemm", "skinny_gemm_wide"):
+    if op in ("skinny_gemm", "skinny_gemm_wide", "stream_gemm"):
         # a decoding step of LLaMA-3 8B: 4 rows against the fused MLP up-projection (235 MB of weights) or the QKV projection
-        Mr, Kd, Nw = 4, 4096, (28672 if op == "skinny_gemm" else 6144 * 8)
+        Mr, Kd, Nw = 4, 4096, (6144 * 8 if op == "skinny_gemm_wide" else 28672)
         x, w = _bf(Mr, Kd), _bf(Nw, Kd, scale=0.02)
         out = torch.empty(Mr, Nw, device=DEV, dtype=torch.bfloat16)
-        return (lambda: K.matmul_skinny(out, x, w)), 2.0 * (Nw * Kd + Mr * Kd + Mr * Nw), 2.0 * Mr * Nw * Kd
+        product = (lambda: K.matmul_forward(out, x, w, None)) if op == "stream_gemm" else (lambda: K.matmul_skinny(out, x, w))
+        return product, 2.0 * (Nw * Kd + Mr * Kd + Mr * Nw), 2.0 * Mr * Nw * Kd
     if op == "cached_attention":
         # 32 rows decoding at position 4095 with 32 query heads over 8 cached heads of width 128 (537 MB of cache read)
         B, Tmax, NH, NKV, HS = 32, 4096, 32, 8, 128
@@ -155,9 +156,9 @@ def case(op):
     raise SystemExit("unknown operator %r" % op)
 
 
-OPS = ["gemm_fwd", "gemm_gelu", "gemm_dgrad", "gemm_dgelu", "gemm_wgrad", "attn_fwd", "attn_bwd", "ln_fwd", "fused_residual", "ln_bwd", "ln_bwd_colsum",
+OPS = ["gemm_fwd", "gemm_gelu", "gemm_dgrad", "gemm_dgelu", "gemm_wgrad", "attn_fwd", "attn_bwd", "attn_fwd_wide", "attn_bwd_wide", "ln_fwd", "fused_residual", "ln_bwd", "ln_bwd_colsum",
        "classifier", "encoder_fwd", "encoder_bwd", "adamw", "norm", "bias_grad", "gelu", "rms_fwd", "rms_fused_residual", "rms_bwd", "rope_fwd",
-       "rope_bwd", "swiglu_fwd", "swiglu_bwd", "gemm_tf32", "gemm_fwd_1cta", "skinny_gemm", "skinny_gemm_wide", "cached_attention"]
+       "rope_bwd", "swiglu_fwd", "swiglu_bwd", "gemm_tf32", "gemm_fwd_1cta", "skinny_gemm", "skinny_gemm_wide", "stream_gemm", "cached_attention"]
 
 
 def main(argv):
