@@ -8,7 +8,6 @@
 //
 // Capability parity: llmc/fused_classifier.cuh (fused_classifier) of the reference.
 #include "common.cuh"
-#include "pdl.cuh"
 
 namespace {
 
@@ -18,8 +17,6 @@ template <bool WRITE_DLOGITS>
 __global__ void __launch_bounds__(CLS_THREADS)
 classifier_kernel(bf16* __restrict__ logits, float* __restrict__ losses, const int* __restrict__ targets,
                   float dloss, int V, int Vp, int accumulate_loss) {
-    pdl_wait();
-    pdl_trigger();
     __shared__ float red[32];
     constexpr float LOG2E = 1.4426950408889634f, LN2 = 0.6931471805599453f;
     // rows are processed back to front so that the rows the LM-head GEMM wrote last (still in L2) go first
@@ -88,7 +85,10 @@ classifier_kernel(bf16* __restrict__ logits, float* __restrict__ losses, const i
 extern "C" int llmc_fused_classifier(bf16* logits, float* losses, const int* targets, float dloss, int N, int V, int Vp,
                                      int write_dlogits, int accumulate_loss, cudaStream_t stream) {
     if (Vp % 8) return -1;
-    if (write_dlogits) CUDA_CHECK(launch_pdl(classifier_kernel<true>, dim3(N), dim3(CLS_THREADS), 0, stream, 0, logits, losses, targets, dloss, V, Vp, accumulate_loss));
-    else CUDA_CHECK(launch_pdl(classifier_kernel<false>, dim3(N), dim3(CLS_THREADS), 0, stream, 0, logits, losses, targets, dloss, V, Vp, accumulate_loss));
+    // launched plainly, without an early start of its own or of the kernel behind it (pdl.cuh): with both, its blocks share the SMs with the
+    // products before and after it, and LM head + classifier + both gradients take 3950 us instead of 3884 at 16384 rows, 120 instead of 116 at 256
+    if (write_dlogits) classifier_kernel<true><<<N, CLS_THREADS, 0, stream>>>(logits, losses, targets, dloss, V, Vp, accumulate_loss);
+    else classifier_kernel<false><<<N, CLS_THREADS, 0, stream>>>(logits, losses, targets, dloss, V, Vp, accumulate_loss);
+    CUDA_CHECK(cudaGetLastError());
     return 0;
 }

@@ -6,8 +6,8 @@
 // captured graph.  The kernels of the GPT-2 and LLaMA paths are launched this way: their setup (barriers, tensor memory, tensor maps) and the
 // launch itself run under the tail of the kernel before.  The same kernels launched without the attribute in brackets: forward + backward of 4 x 64
 // tokens of GPT-2 124M 2.39 ms (2.58), a decoding step of 4 rows 280 us (312), a prefill of 777 tokens 740 us (819), residual + LayerNorm forward
-// and backward at 65536 x 768 153 us (157).  The training attention kernels are launched plainly: 64 x 1024 x 12 x 64 forward and backward took
-// 986 us with the attribute and 938 without, on one GPU in turn.
+// and backward at 65536 x 768 153 us (157).  The training attention kernels and the classifier are launched plainly and trigger nothing: attention
+// at 64 x 1024 x 12 x 64 forward and backward took 986 us with the attribute and 938 without, on one GPU in turn; the classifier's figures stand with it.
 #pragma once
 #include "common.cuh"
 
