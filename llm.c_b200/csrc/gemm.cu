@@ -294,10 +294,12 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
                     }
                     fence_async_smem();
                     group_barrier(grp);
-                    if (leader && ok && col0 < g.N) {
-                        tma_store_2d(&tmD, out_buf, col0, m0);
-                        if (MODE == EPI_GELU) tma_store_2d(&tmAux, bufB, col0, m0);
-                        tma_store_commit();
+                    if (leader) {
+                        if (ok && col0 < g.N) {
+                            tma_store_2d(&tmD, out_buf, col0, m0);
+                            if (MODE == EPI_GELU) tma_store_2d(&tmAux, bufB, col0, m0);
+                        }
+                        tma_store_commit();          // one group per chunk, also an empty one past N: the wait above counts chunks
                     }
                     kctr++;
                 }

@@ -363,7 +363,10 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
                     for (int j = 0; j < 4; j++) *reinterpret_cast<uint4*>(out_row + ((j ^ swz) * 16)) = out_q[j];
                     fence_async_smem();
                     __syncwarp();
-                    if (lane == 0 && ok && col0 < g.N) { tma_store_2d(&tmD, out_buf, col0, m0 + q * 32); tma_store_commit(); }
+                    if (lane == 0) {
+                        if (ok && col0 < g.N) tma_store_2d(&tmD, out_buf, col0, m0 + q * 32);
+                        tma_store_commit();          // one group per chunk, also an empty one past N: the wait above counts chunks
+                    }
                 }
                 if (epi_any(*abort_flag)) break;
                 continue;
