@@ -172,8 +172,8 @@ def generate(model, prompt_tokens, max_gen_len, temperature=0.6, top_p=0.9, echo
              generator=None, use_kv=True, decoder=None, use_graph=None):
     """prompt_tokens: list of token-id lists.  Returns the list of generated id lists (with the prompt in front if ``echo``),
     each cut at its first stop token.  ``use_kv=False`` recomputes the whole prefix at every step through the same decoder
-    (the slow path the cache replaces; it exists to check the cache against).  ``use_graph`` (default: on for a CUDA model)
-    replays the one-token steps from a CUDA graph."""
+    (the slow path the cache replaces; it exists to check the cache against).  ``use_graph`` (default: on for a bf16 CUDA model,
+    which alone has it) replays the one-token steps from a CUDA graph."""
     cfg = model.cfg
     bsz = len(prompt_tokens)
     lens = [len(t) for t in prompt_tokens]
@@ -185,9 +185,9 @@ def generate(model, prompt_tokens, max_gen_len, temperature=0.6, top_p=0.9, echo
     if decoder is None:
         decoder = CachedDecoder(model, bsz, total_len)
     dev = model.device
-    if use_graph is None:
-        use_graph = dev.type == "cuda"
-    use_graph = bool(use_graph) and use_kv and dev.type == "cuda"
+    # (the operators of an fp32 model read the position on the host, which a capture does not allow)
+    graphs = dev.type == "cuda" and model.dtype == torch.bfloat16
+    use_graph = graphs and use_kv and (use_graph is None or bool(use_graph))
     graph_step = None
     tokens = torch.full((bsz, total_len), pad_id, dtype=torch.int64)
     for i, t in enumerate(prompt_tokens):

@@ -378,3 +378,14 @@ def test_skinny_product_of_a_repeated_row():
         ref = torch.empty(inp.shape[0], 264)
         R.matmul_skinny(ref, inp, w)
         close(out, ref, 2e-2, 1e-2, "matmul_skinny")
+
+
+def test_generation_of_an_fp32_model_launches_its_steps():
+    from llmc_b200.models import generate as G
+    cfg = llama3.config_from_descriptor("llama3:l=1,c=128,h=2,kv=1,t=64,v=300,m=32,f=1.0")
+    m = llama3.Llama(cfg, DEV, torch.float32, recompute=1)
+    m.init_random(5)
+    prompts = [[5, 9, 11, 3], [7, 2]]
+    out = G.generate(m, prompts, 8, temperature=0.0)
+    assert out == G.generate(m, prompts, 8, temperature=0.0, use_graph=True) == G.generate(m, prompts, 8, temperature=0.0, use_kv=False)
+    assert [len(o) for o in out] == [8, 8]
