@@ -9,12 +9,12 @@
 // BIAS / GELU_AUX_BIAS / DGELU, beta=1 accumulation) with hand-written tcgen05 code.
 //
 // Structure of a CTA (320 threads, one CTA per SM, tiles taken round-robin):
-//   warp 0      TMA producer: fills a 4-stage ring of 128x64 (A) and 256x64 (B) bf16 tiles,
+//   warp 0      TMA producer: fills a ring of 128x64 (A) and BNx64 (B) bf16 tiles,
 //               128-byte swizzled, signalling `full[stage]` through complete_tx.
-//   warp 1      MMA issuer: one thread issues tcgen05.mma 128x256x16 four times per stage into one
-//               of two 256-column TMEM accumulators and commits to `empty[stage]`; after the last
+//   warp 1      MMA issuer: one thread issues tcgen05.mma 128xBNx16 four times per stage into one
+//               of two TMEM accumulators and commits to `empty[stage]`; after the last
 //               k-block it commits to `acc_full[buf]`.
-//   warps 2..9  epilogue, two groups of four warps, each group owning one 128-column half of the tile:
+//   warps 2..9  epilogue, two groups of four warps, each group owning one half of the tile's columns:
 //               tcgen05.ld the accumulator (a warp may touch 32 TMEM lanes = 32 rows), apply the epilogue
 //               (the pre-activation of dGELU arrives by TMA), stage bf16 through 64-byte-swizzled shared
 //               memory, write with TMA stores, then release the accumulator (`acc_empty[buf]`) so the next
@@ -25,17 +25,17 @@
 
 namespace {
 
-constexpr int BM = 128, BN = 256, BK = 64, STAGES = 4;
+constexpr int BM = 128, BK = 64;
 constexpr int UMMA_K = 16;
 constexpr int A_STAGE_BYTES = BM * BK * 2;            // 16 KB
-constexpr int B_STAGE_BYTES = BN * BK * 2;            // 32 KB
-constexpr int STAGE_BYTES = A_STAGE_BYTES + B_STAGE_BYTES;
+// tile widths BN: 256, or 128 / 64 where 256-wide tiles would leave SMs idle (pick_bn)
+__host__ __device__ constexpr int stage_bytes_for(int bn) { return A_STAGE_BYTES + bn * BK * 2; }
+__host__ __device__ constexpr int stages_for(int bn) { return bn == 256 ? 4 : bn == 128 ? 6 : 8; }
 constexpr int EPI_COLS = 32;                          // columns per epilogue chunk (64 B of bf16)
 constexpr int EPI_BUF_BYTES = BM * EPI_COLS * 2;      // 8 KB
 constexpr int NUM_EPI_BUFS = 4;                       // two per epilogue group
-constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + NUM_EPI_BUFS * EPI_BUF_BYTES + 1024 /*align*/ + 256 /*barriers*/;
+__host__ __device__ constexpr int smem_for(int bn) { return stages_for(bn) * stage_bytes_for(bn) + NUM_EPI_BUFS * EPI_BUF_BYTES + 1024 /*align*/ + 256 /*barriers*/; }
 constexpr int NUM_THREADS = 320;
-constexpr int TMEM_COLS = 512;
 constexpr int RASTER_GROUP = 16;
 constexpr int MAX_SPLIT_GROUP = 8;
 
@@ -75,10 +75,11 @@ DEVINL bool epi_any(int pred) {
 DEVINL void mul2(float* f, uint64_t g) { const float2 r = f2_unpack(f2_mul(f2_pack(f[0], f[1]), g)); f[0] = r.x; f[1] = r.y; }
 DEVINL void add2(float* f, float x, float y) { const float2 r = f2_unpack(f2_add(f2_pack(f[0], f[1]), f2_pack(x, y))); f[0] = r.x; f[1] = r.y; }
 
-template <int A_MN, int B_MN, int MODE>
+template <int BN, int A_MN, int B_MN, int MODE>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
             const __grid_constant__ CUtensorMap tmD, const __grid_constant__ CUtensorMap tmAux, const GemmArgs g) {
+    constexpr int STAGES = stages_for(BN), STAGE_BYTES = stage_bytes_for(BN), TMEM_COLS = 2 * BN;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint8_t* epi_smem = smem + STAGES * STAGE_BYTES;
@@ -445,31 +446,45 @@ int make_operand_map(CUtensorMap* tm, const bf16* ptr, int mn_major, int mn_exte
     return llmc_get_tensormap(tm, ptr, 2, 2, dims, strides, box, 3);
 }
 
-template <int A_MN, int B_MN, int MODE>
+template <int BN, int A_MN, int B_MN, int MODE>
 int launch(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmD, const CUtensorMap& tmAux,
            const GemmArgs& g, int grid, cudaStream_t stream) {
     static bool configured = false;
-    auto kfn = gemm_kernel<A_MN, B_MN, MODE>;
+    auto kfn = gemm_kernel<BN, A_MN, B_MN, MODE>;
     if (!configured) {
-        CUDA_CHECK(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
+        CUDA_CHECK(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_for(BN)));
         configured = true;
     }
-    CUDA_CHECK(launch_pdl(kfn, dim3(grid), dim3(NUM_THREADS), SMEM_BYTES, stream, 0, tmA, tmB, tmD, tmAux, g));
+    CUDA_CHECK(launch_pdl(kfn, dim3(grid), dim3(NUM_THREADS), smem_for(BN), stream, 0, tmA, tmB, tmD, tmAux, g));
     return 0;
+}
+
+// Width of the tiles of a product without split-K: the one whose tiles take the SMs the least time, in cycles of a k-block (what a tile's rows take to
+// arrive: 128 + BN of them) and of an epilogue.  Measured, us per launch with 256 / 128 / 64 columns (M x N x K): 256 x 2304 x 768 8.8 / 7.5 / 6.8,
+// 256 x 3072 x 768 with GELU 11.5 / 9.0 / 7.8, with dGELU 10.6 / 8.2 / 7.3, 256 x 768 x 3072 19.0 / 17.0 / 16.5, 1024 x 2304 x 768 10.0 / 8.3 / 11.0,
+// 896 x 3072 x 2048 18.2 / 23.2 / 31.3; weight gradients 768 x 768 x 256 8.8 / 5.8 / 4.7, 2304 x 768 x 256 8.9 / 5.9 / 6.7.
+int pick_bn(int m_tiles, int N, int num_kb, int sms, int mode) {
+    int best = 256; long long best_cost = -1;
+    for (int bn = 256; bn >= 64; bn >>= 1) {
+        const long long waves = CEIL_DIV(m_tiles * CEIL_DIV(N, bn), sms);
+        const long long cost = waves * (num_kb * (bn == 256 ? 560 : bn == 128 ? 370 : 290) + (mode == EPI_ACCUM ? 18 : 6) * bn + 600);
+        if (best_cost < 0 || cost < best_cost) { best = bn; best_cost = cost; }
+    }
+    return best;
 }
 
 }  // namespace
 
 // Number of fp32 workspace elements and counters llmc_gemm needs for a given problem
 extern "C" void llmc_gemm_workspace(int M, int N, int splits, long long* ws_floats, int* num_counters) {
-    int tiles = CEIL_DIV(M, BM) * CEIL_DIV(N, BN);
-    *ws_floats = splits > 1 ? (long long)tiles * splits * BM * BN : 0;
+    int tiles = CEIL_DIV(M, BM) * CEIL_DIV(N, 256);
+    *ws_floats = splits > 1 ? (long long)tiles * splits * BM * 256 : 0;
     *num_counters = tiles;
 }
 
 // Pick a split-K factor that fills the machine for a wgrad-shaped problem
 extern "C" int llmc_gemm_pick_splits(int M, int N, int K, int sm_count) {
-    int tiles = CEIL_DIV(M, BM) * CEIL_DIV(N, BN);
+    int tiles = CEIL_DIV(M, BM) * CEIL_DIV(N, 256);
     int num_kb = CEIL_DIV(K, BK);
     if (tiles >= sm_count || num_kb < 16) return 1;
     int best = 1; double best_eff = 0.0;
@@ -487,22 +502,29 @@ extern "C" int llmc_gemm_pick_splits(int M, int N, int K, int sm_count) {
 //   a_mn_major = 0: A is stored [M][K] (lda = row stride);  1: stored [K][M]
 //   b_mn_major = 0: B is stored [N][K] (ldb = row stride);  1: stored [K][N]
 // All leading dimensions in elements and multiples of 8; pointers 16-byte aligned.
-extern "C" int llmc_gemm(const bf16* A, const bf16* B, bf16* D, const bf16* bias, bf16* aux,
-                         int M, int N, int K, int lda, int ldb, int ldd,
-                         int a_mn_major, int b_mn_major, int mode, int accumulate,
-                         int splits, float* workspace, unsigned int* counters,
-                         int max_ctas, cudaStream_t stream) {
+// bn: width of the tiles, 256, 128 or 64 (0: pick_bn); split-K takes 256.
+extern "C" int llmc_gemm_tiled(const bf16* A, const bf16* B, bf16* D, const bf16* bias, bf16* aux,
+                               int M, int N, int K, int lda, int ldb, int ldd,
+                               int a_mn_major, int b_mn_major, int mode, int accumulate,
+                               int splits, float* workspace, unsigned int* counters,
+                               int max_ctas, int bn, cudaStream_t stream) {
     if (M <= 0 || N <= 0 || K <= 0) return 0;
     if ((N % 8) || (lda % 8) || (ldb % 8) || (ldd % 8)) { fprintf(stderr, "[llmc_b200] gemm: N and leading dimensions must be multiples of 8\n"); return -1; }
     GemmArgs g;
     g.M = M; g.N = N; g.K = K;
-    g.num_m_tiles = CEIL_DIV(M, BM); g.num_n_tiles = CEIL_DIV(N, BN);
+    g.num_m_tiles = CEIL_DIV(M, BM);
     g.num_kb = CEIL_DIV(K, BK);
     if (mode != EPI_ACCUM || splits < 1) splits = 1;
     if (splits > g.num_kb) splits = g.num_kb;
     g.kb_per_split = CEIL_DIV(g.num_kb, splits);
     splits = CEIL_DIV(g.num_kb, g.kb_per_split);      // no empty split
     g.splits = splits;
+    int sms = llmc_device_sm_count(); if (sms <= 0) sms = 148;
+    if (max_ctas > 0 && max_ctas < sms) sms = max_ctas;
+    if (splits > 1) bn = 256;
+    if (bn == 0) bn = pick_bn(g.num_m_tiles, N, g.num_kb, sms, mode);
+    if (bn != 64 && bn != 128 && bn != 256) return -1;
+    g.num_n_tiles = CEIL_DIV(N, bn);
     if (splits > 1 && (workspace == nullptr || counters == nullptr)) { fprintf(stderr, "[llmc_b200] gemm: split-K needs workspace\n"); return -1; }
     g.D = D; g.ldd = ldd; g.bias = bias; g.aux = aux; g.workspace = workspace; g.counters = counters;
     g.accumulate = accumulate;
@@ -511,7 +533,7 @@ extern "C" int llmc_gemm(const bf16* A, const bf16* B, bf16* D, const bf16* bias
     CUtensorMap tmA, tmB, tmD, tmAux;
     int rc;
     if ((rc = make_operand_map(&tmA, A, a_mn_major, M, K, lda, BM))) return rc;
-    if ((rc = make_operand_map(&tmB, B, b_mn_major, N, K, ldb, BN))) return rc;
+    if ((rc = make_operand_map(&tmB, B, b_mn_major, N, K, ldb, bn))) return rc;
     {
         uint64_t dims[2] = {(uint64_t)N, (uint64_t)M}, strides[2] = {2, (uint64_t)ldd * 2};
         uint32_t box[2] = {EPI_COLS, BM};
@@ -519,13 +541,13 @@ extern "C" int llmc_gemm(const bf16* A, const bf16* B, bf16* D, const bf16* bias
         tmAux = tmD;
         if (mode == EPI_GELU || mode == EPI_DGELU) { if ((rc = llmc_get_tensormap(&tmAux, aux, 2, 2, dims, strides, box, 2))) return rc; }
     }
-    int sms = llmc_device_sm_count();
-    if (max_ctas > 0 && max_ctas < sms) sms = max_ctas;
     int total = g.num_m_tiles * g.num_n_tiles * g.splits;
     int grid = total < sms ? total : sms;
     if (grid < 1) grid = 1;
 
-#define LAUNCH(AM, BMj, MD) return launch<AM, BMj, MD>(tmA, tmB, tmD, tmAux, g, grid, stream)
+#define LAUNCH(AM, BMj, MD) return bn == 256 ? launch<256, AM, BMj, MD>(tmA, tmB, tmD, tmAux, g, grid, stream) \
+                                 : bn == 128 ? launch<128, AM, BMj, MD>(tmA, tmB, tmD, tmAux, g, grid, stream) \
+                                             : launch<64, AM, BMj, MD>(tmA, tmB, tmD, tmAux, g, grid, stream)
     if (a_mn_major == 0 && b_mn_major == 0) {
         if (mode == EPI_STORE) LAUNCH(0, 0, EPI_STORE);
         if (mode == EPI_GELU) LAUNCH(0, 0, EPI_GELU);
@@ -540,4 +562,12 @@ extern "C" int llmc_gemm(const bf16* A, const bf16* B, bf16* D, const bf16* bias
 #undef LAUNCH
     fprintf(stderr, "[llmc_b200] gemm: unsupported layout/mode combination (%d,%d,%d)\n", a_mn_major, b_mn_major, mode);
     return -1;
+}
+
+extern "C" int llmc_gemm(const bf16* A, const bf16* B, bf16* D, const bf16* bias, bf16* aux,
+                         int M, int N, int K, int lda, int ldb, int ldd,
+                         int a_mn_major, int b_mn_major, int mode, int accumulate,
+                         int splits, float* workspace, unsigned int* counters,
+                         int max_ctas, cudaStream_t stream) {
+    return llmc_gemm_tiled(A, B, D, bias, aux, M, N, K, lda, ldb, ldd, a_mn_major, b_mn_major, mode, accumulate, splits, workspace, counters, max_ctas, 0, stream);
 }
