@@ -87,6 +87,40 @@ __global__ void bias_grad_fold_kernel(bf16* __restrict__ dbias, const float* __r
     dbias[c] = __float2bfloat16_rn(s);
 }
 
+// Few rows: one launch, a CTA sums all rows of 32 columns (4 lanes of 16 bytes per row, 64 rows at a time, then the 64 sums of a column).
+constexpr int BGF_SLOTS = 64;
+__global__ void __launch_bounds__(4 * BGF_SLOTS)
+bias_grad_few_kernel(bf16* __restrict__ dbias, const bf16* __restrict__ dout, int rows, int OC, int accumulate) {
+    pdl_wait();
+    pdl_trigger();
+    __shared__ float sh[BGF_SLOTS][33];
+    const int x = threadIdx.x & 3, y = threadIdx.x >> 2;
+    const int col = blockIdx.x * 32 + x * 8;
+    float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    if (col < OC) {
+        #pragma unroll 8
+        for (int r = y; r < rows; r += BGF_SLOTS) {
+            bf16x8 d = ld128(dout + (size_t)r * OC + col);
+            #pragma unroll
+            for (int e = 0; e < 8; e++) acc[e] += __bfloat162float(d[e]);
+        }
+    }
+    #pragma unroll
+    for (int e = 0; e < 8; e++) sh[y][x * 8 + e] = acc[e];
+    __syncthreads();
+    // column c = warp * 4 + lane / 8: 8 lanes add 8 slots each, then one another's sums in a fixed tree
+    const int lane = threadIdx.x & 31, c = (threadIdx.x >> 5) * 4 + (lane >> 3), part = lane & 7;
+    float s = 0.f;
+    #pragma unroll
+    for (int i = 0; i < BGF_SLOTS / 8; i++) s += sh[part * (BGF_SLOTS / 8) + i][c];
+    s += __shfl_xor_sync(0xffffffffu, s, 1);
+    s += __shfl_xor_sync(0xffffffffu, s, 2);
+    s += __shfl_xor_sync(0xffffffffu, s, 4);
+    const int oc = blockIdx.x * 32 + c;
+    if (part == 0 && oc < OC) dbias[oc] = __float2bfloat16_rn(accumulate ? s + __bfloat162float(dbias[oc]) : s);
+}
+constexpr int BG_FEW_ROWS = 1024;
+
 int bg_strips(int rows, int OC) {
     int sms = llmc_device_sm_count(); if (sms <= 0) sms = 148;
     int colgroups = CEIL_DIV(OC, 256);
@@ -113,10 +147,14 @@ extern "C" int llmc_residual_add(bf16* out, const bf16* a, const bf16* b, long l
     CUDA_CHECK(launch_pdl(residual_add_kernel, dim3((unsigned)CEIL_DIV(n / 8, 256)), dim3(256), 0, stream, 0, out, a, b, n / 8));
     return 0;
 }
-extern "C" long long llmc_bias_grad_scratch(int rows, int OC) { return (long long)bg_strips(rows, OC) * OC; }
-// dbias[c] (+)= sum_r dout[r, c]; scratch: llmc_bias_grad_scratch floats
+extern "C" long long llmc_bias_grad_scratch(int rows, int OC) { return rows <= BG_FEW_ROWS ? 0 : (long long)bg_strips(rows, OC) * OC; }
+// dbias[c] (+)= sum_r dout[r, c]; scratch: llmc_bias_grad_scratch floats (none for few rows)
 extern "C" int llmc_bias_grad(bf16* dbias, float* scratch, const bf16* dout, int rows, int OC, int accumulate, cudaStream_t stream) {
     if (OC % 8) return -1;
+    if (rows <= BG_FEW_ROWS) {
+        CUDA_CHECK(launch_pdl(bias_grad_few_kernel, dim3(CEIL_DIV(OC, 32)), dim3(4 * BGF_SLOTS), 0, stream, 0, dbias, dout, rows, OC, accumulate));
+        return 0;
+    }
     const int strips = bg_strips(rows, OC);
     const int rps = CEIL_DIV(rows, strips);
     CUDA_CHECK(launch_pdl(bias_grad_kernel, dim3(CEIL_DIV(OC, 256), strips), dim3(BG_WARPS * 32), 0, stream, 0, scratch, dout, rows, OC, rps));

@@ -379,7 +379,7 @@ struct LnbLaunch { int threads, ctas, rows_per_cta; };
 
 template <bool ACC, int MAXP, bool COL>
 int lnb_launch(bf16* dinp, float* scratch, const bf16* dout, const bf16* inp, const bf16* weight, const float* mean, const float* rstd,
-               int N, int C, int threads, int* ctas_out, cudaStream_t stream) {
+               int N, int C, int threads, bool rows, int* ctas_out, cudaStream_t stream) {
     constexpr bool CACHE = MAXP <= 2;
     static int occ_cache[LNB_MAX_THREADS / 32 + 1] = {0};
     int& occ = occ_cache[threads / 32];
@@ -392,38 +392,47 @@ int lnb_launch(bf16* dinp, float* scratch, const bf16* dout, const bf16* inp, co
     int ctas = occ * sms;
     int rows_per_cta = CEIL_DIV(N, ctas);
     ctas = CEIL_DIV(N, rows_per_cta);
-    CUDA_CHECK(launch_pdl(ln_bwd_col_kernel<ACC, MAXP, COL, CACHE>, dim3(ctas), dim3(threads), 0, stream, 0, dinp, scratch, dout, inp, weight, mean, rstd, N, C, rows_per_cta));
+    if (rows) CUDA_CHECK(launch_pdl(ln_bwd_col_kernel<ACC, MAXP, COL, CACHE>, dim3(ctas), dim3(threads), 0, stream, 0, dinp, scratch, dout, inp, weight, mean, rstd, N, C, rows_per_cta));
     *ctas_out = ctas;
     return 0;
 }
 
 template <int MAXP>
 int lnb_dispatch(bool acc, bool col, bf16* dinp, float* scratch, const bf16* dout, const bf16* inp, const bf16* weight,
-                 const float* mean, const float* rstd, int N, int C, int threads, int* ctas_out, cudaStream_t stream) {
-    if (acc) return col ? lnb_launch<true, MAXP, true>(dinp, scratch, dout, inp, weight, mean, rstd, N, C, threads, ctas_out, stream)
-                        : lnb_launch<true, MAXP, false>(dinp, scratch, dout, inp, weight, mean, rstd, N, C, threads, ctas_out, stream);
-    return col ? lnb_launch<false, MAXP, true>(dinp, scratch, dout, inp, weight, mean, rstd, N, C, threads, ctas_out, stream)
-               : lnb_launch<false, MAXP, false>(dinp, scratch, dout, inp, weight, mean, rstd, N, C, threads, ctas_out, stream);
+                 const float* mean, const float* rstd, int N, int C, int threads, bool rows, int* ctas_out, cudaStream_t stream) {
+    if (acc) return col ? lnb_launch<true, MAXP, true>(dinp, scratch, dout, inp, weight, mean, rstd, N, C, threads, rows, ctas_out, stream)
+                        : lnb_launch<true, MAXP, false>(dinp, scratch, dout, inp, weight, mean, rstd, N, C, threads, rows, ctas_out, stream);
+    return col ? lnb_launch<false, MAXP, true>(dinp, scratch, dout, inp, weight, mean, rstd, N, C, threads, rows, ctas_out, stream)
+               : lnb_launch<false, MAXP, false>(dinp, scratch, dout, inp, weight, mean, rstd, N, C, threads, rows, ctas_out, stream);
 }
 }  // namespace
 
 // dinp (+)= dLN ; dweight, dbias (+)= column sums.  `scratch` holds llmc_layernorm_bwd_scratch floats.
 // If dcolsum is given it receives (+)= the column sums of the final dinp: when dinp is the residual-stream gradient, that
 // is the bias gradient of the projection that wrote into the residual stream, obtained without another pass.  C <= 16384.
-extern "C" int llmc_layernorm_bwd(bf16* dinp, bf16* dweight, bf16* dbias, float* scratch, const bf16* dout, const bf16* inp,
+// parts: 1 the kernel over the rows, 2 the sums over its CTAs (dweight, dbias, dcolsum), which nothing of a backward pass reads: they may follow in
+// another stream; 3 both.
+extern "C" int llmc_layernorm_bwd_parts(bf16* dinp, bf16* dweight, bf16* dbias, float* scratch, const bf16* dout, const bf16* inp,
                                   const bf16* weight, const float* mean, const float* rstd, int N, int C,
-                                  int accumulate_dinp, int accumulate_dwdb, bf16* dcolsum, int accumulate_dcol, cudaStream_t stream) {
+                                  int accumulate_dinp, int accumulate_dwdb, bf16* dcolsum, int accumulate_dcol, int parts, cudaStream_t stream) {
     if (C % 8 || C > LNB_MAX_THREADS * 8 * 8) return -1;
     const int npack = C / 8;
     const int threads = npack <= LNB_MAX_THREADS ? CEIL_DIV(npack, 32) * 32 : LNB_MAX_THREADS;
     const int packs = CEIL_DIV(npack, threads);
     const bool acc = accumulate_dinp != 0, col = dcolsum != nullptr;
     int ctas = 0, rc;
-    if (packs <= 1) rc = lnb_dispatch<1>(acc, col, dinp, scratch, dout, inp, weight, mean, rstd, N, C, threads, &ctas, stream);
-    else if (packs <= 2) rc = lnb_dispatch<2>(acc, col, dinp, scratch, dout, inp, weight, mean, rstd, N, C, threads, &ctas, stream);
-    else if (packs <= 4) rc = lnb_dispatch<4>(acc, col, dinp, scratch, dout, inp, weight, mean, rstd, N, C, threads, &ctas, stream);
-    else rc = lnb_dispatch<8>(acc, col, dinp, scratch, dout, inp, weight, mean, rstd, N, C, threads, &ctas, stream);
+    if (packs <= 1) rc = lnb_dispatch<1>(acc, col, dinp, scratch, dout, inp, weight, mean, rstd, N, C, threads, parts & 1, &ctas, stream);
+    else if (packs <= 2) rc = lnb_dispatch<2>(acc, col, dinp, scratch, dout, inp, weight, mean, rstd, N, C, threads, parts & 1, &ctas, stream);
+    else if (packs <= 4) rc = lnb_dispatch<4>(acc, col, dinp, scratch, dout, inp, weight, mean, rstd, N, C, threads, parts & 1, &ctas, stream);
+    else rc = lnb_dispatch<8>(acc, col, dinp, scratch, dout, inp, weight, mean, rstd, N, C, threads, parts & 1, &ctas, stream);
     if (rc) return rc;
-    CUDA_CHECK(launch_pdl(ln_bwd_fold_kernel, dim3(CEIL_DIV(C, 16)), dim3(4 * LNB_FOLD_SLICES), 0, stream, 0, dweight, dbias, dcolsum, scratch, ctas, C, accumulate_dwdb, accumulate_dcol));
+    if (parts & 2) CUDA_CHECK(launch_pdl(ln_bwd_fold_kernel, dim3(CEIL_DIV(C, 16)), dim3(4 * LNB_FOLD_SLICES), 0, stream, 0, dweight, dbias, dcolsum, scratch, ctas, C, accumulate_dwdb, accumulate_dcol));
     return 0;
+}
+
+extern "C" int llmc_layernorm_bwd(bf16* dinp, bf16* dweight, bf16* dbias, float* scratch, const bf16* dout, const bf16* inp,
+                                  const bf16* weight, const float* mean, const float* rstd, int N, int C,
+                                  int accumulate_dinp, int accumulate_dwdb, bf16* dcolsum, int accumulate_dcol, cudaStream_t stream) {
+    return llmc_layernorm_bwd_parts(dinp, dweight, dbias, scratch, dout, inp, weight, mean, rstd, N, C, accumulate_dinp, accumulate_dwdb, dcolsum,
+                                    accumulate_dcol, 3, stream);
 }

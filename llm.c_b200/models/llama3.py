@@ -338,9 +338,11 @@ class Llama:
         acc = micro_step > 0
         dres, dl_btc, dh, dfc12, dqkv, dqkv_raw = a["dresidual"], a["scratch_btc"], a["dh"], a["dfc12"], a["dqkv"], a["qkv_raw"]
         dlogits = a["logits"]
+        side = self.step_graphs.side            # weight gradients beside the chain of input gradients, as in models/gpt2.py
 
+        with side.fork():
+            ops.matmul_wgrad(g["lmhead"], dlogits, a["lnf"], accumulate=acc)
         ops.matmul_dgrad(dl_btc, dlogits, p["lmhead"])
-        ops.matmul_wgrad(g["lmhead"], dlogits, a["lnf"], accumulate=acc)
         ops.rmsnorm_backward(dres, g["lnfw"], dl_btc, a["residual3"][L - 1], p["lnfw"], a["lnf_rstd"], accumulate_dinp=False,
                              accumulate_dw=acc)
         nvtx = self.device.type == "cuda"
@@ -351,25 +353,34 @@ class Llama:
             lg = 0 if self.recompute >= 1 else l
             if self.recompute >= 1:
                 ops.swiglu_forward(a["h"][lg], a["fc12"][l])
+            with side.fork():
+                ops.matmul_wgrad(g["fcprojw"][l], dres, a["h"][lg], accumulate=acc)
+            dres_read = side.mark()
             ops.matmul_dgrad(dh, dres, p["fcprojw"][l])
-            ops.matmul_wgrad(g["fcprojw"][l], dres, a["h"][lg], accumulate=acc)
             ops.swiglu_backward(dfc12, dh, a["fc12"][l])
             if self.recompute >= 2:
                 ops.rmsnorm_forward(a["ln2"][lln], None, a["residual2"][l], p["ln2w"][l], eps)
+            with side.fork():
+                ops.matmul_wgrad(g["fc12w"][l], dfc12, a["ln2"][lln], accumulate=acc)
             ops.matmul_dgrad(dl_btc, dfc12, p["fc12w"][l])
-            ops.matmul_wgrad(g["fc12w"][l], dfc12, a["ln2"][lln], accumulate=acc)
+            side.join(dres_read)
             ops.rmsnorm_backward(dres, g["ln2w"][l], dl_btc, a["residual2"][l], p["ln2w"][l], a["ln2_rstd"][l], accumulate_dinp=True,
                                  accumulate_dw=acc)
+            with side.fork():
+                ops.matmul_wgrad(g["attprojw"][l], dres, a["atty"][l], accumulate=acc)
+            dres_read = side.mark()
             ops.matmul_dgrad(dl_btc, dres, p["attprojw"][l])
-            ops.matmul_wgrad(g["attprojw"][l], dres, a["atty"][l], accumulate=acc)
             ops.attention_backward(dqkv, dl_btc, a["qkv"][l], a["atty"][l], a["lse"][l], B, T, NH)
             ops.rope_backward(dqkv_raw, dqkv, self.freqs, T, NH, NKV)
             if self.recompute >= 2:
                 ops.rmsnorm_forward(a["ln1"][lln], None, residual, p["ln1w"][l], eps)
+            with side.fork():
+                ops.matmul_wgrad(g["qkvw"][l], dqkv_raw, a["ln1"][lln], accumulate=acc)
             ops.matmul_dgrad(dl_btc, dqkv_raw, p["qkvw"][l])
-            ops.matmul_wgrad(g["qkvw"][l], dqkv_raw, a["ln1"][lln], accumulate=acc)
+            side.join(dres_read)
             ops.rmsnorm_backward(dres, g["ln1w"][l], dl_btc, residual, p["ln1w"][l], a["ln1_rstd"][l], accumulate_dinp=True,
                                  accumulate_dw=acc)
+            side.join()
             if hook is not None:
                 hook(l)
         ops.encoder_backward(g["wte"], None, dres.view(B, T, C), self.inputs, accumulate_wte=acc, accumulate_wpe=False,

@@ -8,9 +8,51 @@ What makes a replay equal to the eager call: the sequence only reads and writes 
 before), all scalar arguments are part of the key, and the addresses of every parameter, gradient and activation buffer and of the rotary
 table are compared.  The scratch buffers of the operators are shared by all callers and replaced when one needs a larger one, so a graph keeps those that its own operators took.
 """
+import contextlib
+
 import torch
 
 from ..ops import kernels
+
+
+class Inline:
+    """Launches outside a capture: everything in one stream, in the order of the calls."""
+
+    def fork(self):
+        return contextlib.nullcontext()
+
+    refork = fork
+
+    def mark(self):
+        return None
+
+    def join(self, mark=None):
+        pass
+
+
+class Side:
+    """A second branch of the graph that is being captured, for launches whose results the chain of the backward pass does not read (gradients of
+    weights and biases).  A small batch leaves most SMs idle in every kernel of that chain.  ``fork()``: the launches inside the block follow
+    all launches of the main branch so far; ``join(mark())``: the launches of the main branch from here on follow what the side branch had
+    been given up to the mark."""
+
+    def __init__(self, stream):
+        self.stream = stream
+
+    def fork(self):
+        self.stream.wait_event(torch.cuda.current_stream().record_event())
+        return torch.cuda.stream(self.stream)
+
+    def refork(self):
+        """``join()``, then ``fork()``."""
+        self.join()
+        return self.fork()
+
+    def mark(self):
+        return self.stream.record_event()
+
+    def join(self, mark=None):
+        torch.cuda.current_stream().wait_event(self.mark() if mark is None else mark)
 
 
 class StepGraphs:
@@ -21,6 +63,7 @@ class StepGraphs:
 
     def __init__(self):
         self._entries = {}
+        self.side = Inline()               # where the launches beside the main chain go
 
     def __reduce__(self):
         return StepGraphs, ()              # a copied or unpickled model captures graphs of its own buffers
@@ -59,9 +102,11 @@ class StepGraphs:
         with torch.cuda.stream(side), kernels.scratch_taken() as scratch:
             # other threads (watchdog, data loader) may use the device meanwhile
             graph.capture_begin(capture_error_mode="thread_local")
+            model.step_graphs.side = Side(torch.cuda.Stream(device=model.device))
             try:
                 fn()
             finally:
+                model.step_graphs.side = Inline()
                 graph.capture_end()
         e["launches"] = kernels.launch_count() - before
         kernels.count_launches(-e["launches"])                 # captured, not launched

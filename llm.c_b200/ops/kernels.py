@@ -216,8 +216,9 @@ def bias_grad(dbias, dout, accumulate=True):
     global _launches
     lib = _lib.cuda()
     M, OC = dout.shape
-    s = _scratch.get("bias_grad", lib.llmc_bias_grad_scratch(M, OC), torch.float32, dout.device)
-    _launches += 2
+    words = lib.llmc_bias_grad_scratch(M, OC)
+    s = _scratch.get("bias_grad", words, torch.float32, dout.device)
+    _launches += 2 if words else 1
     check(lib.llmc_bias_grad(_p(dbias), _p(s), _p(dout), M, OC, int(accumulate), _stream()), "llmc_bias_grad")
 
 
@@ -259,17 +260,23 @@ def fused_residual_forward(residual, normed, mean, rstd, inp1, inp2, weight, bia
 
 
 def layernorm_backward(dinp, dweight, dbias, dout, inp, weight, mean, rstd, accumulate_dinp=True, accumulate_dwdb=True,
-                       dcolsum=None, accumulate_dcol=True):
+                       dcolsum=None, accumulate_dcol=True, sums_in=None):
     """dinp (+)= dLN(dout); dweight/dbias (+)= their gradients.  ``dcolsum`` (+)= column sums of the final dinp: the bias
-    gradient of the projection that wrote into the residual stream, at no extra pass over memory."""
+    gradient of the projection that wrote into the residual stream, at no extra pass over memory.  ``sums_in()`` may give a
+    context (another stream) in which the three column sums are finished; the next call has to follow them."""
     global _launches
     lib = _lib.cuda()
     N, C = inp.shape
     s = _scratch.get("ln_bwd", lib.llmc_layernorm_bwd_scratch(N, C), torch.float32, inp.device)
     _launches += 2
-    check(lib.llmc_layernorm_bwd(_p(dinp), _p(dweight), _p(dbias), _p(s), _p(dout), _p(inp), _p(weight), _p(mean), _p(rstd),
-                                 N, C, int(accumulate_dinp), int(accumulate_dwdb), _p(dcolsum), int(accumulate_dcol), _stream()),
-          "llmc_layernorm_bwd")
+    args = (_p(dinp), _p(dweight), _p(dbias), _p(s), _p(dout), _p(inp), _p(weight), _p(mean), _p(rstd),
+            N, C, int(accumulate_dinp), int(accumulate_dwdb), _p(dcolsum), int(accumulate_dcol))
+    if sums_in is None:
+        check(lib.llmc_layernorm_bwd(*args, _stream()), "llmc_layernorm_bwd")
+        return
+    check(lib.llmc_layernorm_bwd_parts(*args, 1, _stream()), "llmc_layernorm_bwd_parts")
+    with sums_in():
+        check(lib.llmc_layernorm_bwd_parts(*args, 2, _stream()), "llmc_layernorm_bwd_parts")
 
 
 def attention_forward(out, lse, qkv, B, T, NH):

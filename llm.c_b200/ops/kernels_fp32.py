@@ -79,7 +79,7 @@ def fused_residual_forward(residual, normed, mean, rstd, inp1, inp2, weight, bia
 
 
 def layernorm_backward(dinp, dweight, dbias, dout, inp, weight, mean, rstd, accumulate_dinp=True, accumulate_dwdb=True,
-                       dcolsum=None, accumulate_dcol=True):
+                       dcolsum=None, accumulate_dcol=True, sums_in=None):
     lib = _lib_()
     C = inp.shape[-1]
     rows = inp.numel() // C

@@ -130,7 +130,7 @@ def fused_residual_forward(residual, normed, mean, rstd, inp1, inp2, weight, bia
 
 
 def layernorm_backward(dinp, dweight, dbias, dout, inp, weight, mean, rstd, accumulate_dinp=True, accumulate_dwdb=True,
-                       dcolsum=None, accumulate_dcol=True):
+                       dcolsum=None, accumulate_dcol=True, sums_in=None):
     dy, x, w = _f(dout), _f(inp), _f(weight)
     norm = (x - mean.unsqueeze(-1)) * rstd.unsqueeze(-1)
     dnorm = dy * w
