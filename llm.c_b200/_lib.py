@@ -74,6 +74,7 @@ def cuda():
         "llmc_rmsnorm_fused_residual_fwd": (I, [P, P, P, P, P, P, I, I, F, S]),
         "llmc_rmsnorm_bwd_scratch": (L, [I, I]),
         "llmc_rmsnorm_bwd": (I, [P, P, P, P, P, P, P, I, I, I, I, S]),
+        "llmc_rope_fwd_cache": (I, [P, P, P, P, P, I, L, I, I, I, I, S]),
         "llmc_rope_fwd": (I, [P, P, P, L, I, I, I, I, S]),
         "llmc_rope_bwd": (I, [P, P, P, L, I, I, I, I, S]),
         "llmc_swiglu_fwd": (I, [P, P, L, I, S]),

@@ -279,7 +279,8 @@ constexpr int ROPE_THREADS = 256;
 
 template <int REP>
 __global__ void __launch_bounds__(ROPE_THREADS)
-rope_fwd_kernel(bf16* __restrict__ packed, const bf16* __restrict__ raw, const float2* __restrict__ freqs, int T, int NH, int NKV, int HS) {
+rope_fwd_kernel(bf16* __restrict__ packed, const bf16* __restrict__ raw, const float2* __restrict__ freqs, bf16* __restrict__ kcache,
+                bf16* __restrict__ vcache, int cache_len, int T, int NH, int NKV, int HS) {
     pdl_wait();
     pdl_trigger();
     const int hp = HS >> 3, heads = NH + 2 * NKV, items = heads * hp, rep = REP ? REP : NH / NKV;
@@ -301,6 +302,10 @@ rope_fwd_kernel(bf16* __restrict__ packed, const bf16* __restrict__ raw, const f
             #pragma unroll
             for (int r = 0; r < (REP ? REP : 1); r++) st128(d + r * HS, a);
             if (REP == 0) for (int r = 1; r < rep; r++) st128(d + r * HS, a);
+            if (kcache != nullptr) {
+                const size_t at = (((size_t)(blockIdx.x / (unsigned)T) * cache_len + blockIdx.x % (unsigned)T) * NKV + hk) * HS + p * 8;
+                st128((which == 1 ? kcache : vcache) + at, a);
+            }
         }
     }
 }
@@ -477,10 +482,13 @@ extern "C" int llmc_rmsnorm_bwd(bf16* dinp, bf16* dweight, float* scratch, const
 
 static int rope_check(int NH, int NKV, int HS) { return (HS % 8 || NKV <= 0 || NH % NKV) ? -1 : 0; }
 
-extern "C" int llmc_rope_fwd(bf16* packed, const bf16* raw, const float* freqs, long long N, int T, int NH, int NKV, int HS, cudaStream_t stream) {
+// kcache, vcache (both or neither): (batch, cache_len, NKV, HS); the rotated keys and the values of position t of sequence b also go to their entries
+// (b, t).  Copied out of the packed tensor afterwards they take two launches more.
+extern "C" int llmc_rope_fwd_cache(bf16* packed, const bf16* raw, const float* freqs, bf16* kcache, bf16* vcache, int cache_len, long long N, int T, int NH,
+                                   int NKV, int HS, cudaStream_t stream) {
     if (rope_check(NH, NKV, HS)) return -1;
     if (N <= 0) return 0;
-#define ROPE_GO(R) CUDA_CHECK(launch_pdl(rope_fwd_kernel<R>, dim3((unsigned)N), dim3(ROPE_THREADS), 0, stream, 0, packed, raw, reinterpret_cast<const float2*>(freqs), T, NH, NKV, HS))
+#define ROPE_GO(R) CUDA_CHECK(launch_pdl(rope_fwd_kernel<R>, dim3((unsigned)N), dim3(ROPE_THREADS), 0, stream, 0, packed, raw, reinterpret_cast<const float2*>(freqs), kcache, vcache, cache_len, T, NH, NKV, HS))
     const int rep = NH / NKV;
     if (rep == 1) ROPE_GO(1);
     else if (rep == 2) ROPE_GO(2);
@@ -489,6 +497,10 @@ extern "C" int llmc_rope_fwd(bf16* packed, const bf16* raw, const float* freqs, 
 #undef ROPE_GO
     CUDA_CHECK(cudaGetLastError());
     return 0;
+}
+
+extern "C" int llmc_rope_fwd(bf16* packed, const bf16* raw, const float* freqs, long long N, int T, int NH, int NKV, int HS, cudaStream_t stream) {
+    return llmc_rope_fwd_cache(packed, raw, freqs, nullptr, nullptr, 0, N, T, NH, NKV, HS, stream);
 }
 
 extern "C" int llmc_rope_bwd(bf16* draw, const bf16* dpacked, const float* freqs, long long N, int T, int NH, int NKV, int HS, cudaStream_t stream) {

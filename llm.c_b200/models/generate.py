@@ -92,10 +92,9 @@ class CachedDecoder:
         ops.encoder_forward(x[:N].view(B, Tq, C), tokens, p["wte"], None)
         ops.rmsnorm_forward(ln[:N], rstd[:N], x[:N], p["ln1w"][0], eps)
         # a long prompt from position 0 is the training forward pass: its attention kernel (tensor cores, one pass over the
-        # keys per 128 queries) replaces the per-query scan of the cache, and keys / values are copied into the cache afterwards
+        # keys per 128 queries) replaces the per-query scan of the cache, and the rotary kernel writes keys / values to the cache too
         dense = pos is None and start_pos == 0 and Tq >= self.dense_prefill_from
         if dense:
-            rep, HS = NH // NKV, cfg.head_size
             if self._dense is None or self._dense[0].shape[0] < N or self._dense[1].numel() < B * NH * Tq:
                 self._dense = (torch.zeros(rows, 3 * C, dtype=m.dtype, device=m.device),
                                torch.zeros(B * NH * Tq, dtype=torch.float32, device=m.device))
@@ -103,11 +102,8 @@ class CachedDecoder:
         for l in range(L):
             mm(a["raw"], ln, p["qkvw"][l], N)
             if dense:
-                ops.rope_forward(packed, a["raw"][:N], m.freqs, Tq, NH, NKV)
+                ops.rope_forward(packed, a["raw"][:N], m.freqs, Tq, NH, NKV, self.kcache[l], self.vcache[l])
                 ops.attention_forward(a["atty"][:N], lse, packed, B, Tq, NH)
-                kv = packed.view(B, Tq, 3, NKV, rep, HS)
-                self.kcache[l][:B, :Tq].copy_(kv[:, :, 1, :, 0])
-                self.vcache[l][:B, :Tq].copy_(kv[:, :, 2, :, 0])
             else:
                 ops.rope_cache(a["q"][:N], self.kcache[l], self.vcache[l], a["raw"][:N], m.freqs, Tq, start_pos, NH, NKV, pos)
                 ops.cached_attention(a["atty"][:N], a["q"][:N], self.kcache[l], self.vcache[l], Tq, start_pos, NH, NKV, pos)

@@ -354,13 +354,22 @@ def rmsnorm_backward(dinp, dweight, dout, inp, weight, rstd, accumulate_dinp=Tru
                                int(accumulate_dw), _stream()), "llmc_rmsnorm_bwd")
 
 
-def rope_forward(packed, raw, freqs, T, NH, NKV):
+def rope_forward(packed, raw, freqs, T, NH, NKV, kcache=None, vcache=None):
     """raw (N, (NH + 2 NKV) * HS) -> packed (N, 3, NH, HS): rotary embedding on queries and keys, key / value heads repeated
-    NH / NKV times (reference: apply_rotary_emb + repeat_kv, train_llama3.py:107-117 and :59-68).  freqs: (maxT, HS/2, 2) fp32."""
+    NH / NKV times (reference: apply_rotary_emb + repeat_kv, train_llama3.py:107-117 and :59-68).  freqs: (maxT, HS/2, 2) fp32.
+    kcache, vcache (B, >= T, NKV, HS), contiguous: the rotated keys and the values of the B = N / T sequences also go to their first T entries."""
     global _launches
     N = raw.shape[0]
     HS = raw.shape[1] // (NH + 2 * NKV)
     _launches += 1
+    if kcache is not None:
+        B = N // T
+        if B * T != N or kcache.shape != vcache.shape or tuple(kcache.shape[2:]) != (NKV, HS) or kcache.shape[0] < B or kcache.shape[1] < T \
+                or not (kcache.is_contiguous() and vcache.is_contiguous()):
+            raise ValueError("rope_forward: caches of shape %s do not hold %d tokens of sequences of %d" % (tuple(kcache.shape), N, T))
+        check(_lib.cuda().llmc_rope_fwd_cache(_p(packed), _p(raw), _p(freqs), _p(kcache), _p(vcache), kcache.shape[1], N, T, NH, NKV, HS, _stream()),
+              "llmc_rope_fwd_cache")
+        return
     check(_lib.cuda().llmc_rope_fwd(_p(packed), _p(raw), _p(freqs), N, T, NH, NKV, HS, _stream()), "llmc_rope_fwd")
 
 

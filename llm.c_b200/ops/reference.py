@@ -310,7 +310,7 @@ def _rotate(x, freqs, T, sign):
     return out
 
 
-def rope_forward(packed, raw, freqs, T, NH, NKV):
+def rope_forward(packed, raw, freqs, T, NH, NKV, kcache=None, vcache=None):
     N = raw.shape[0]
     HS = raw.shape[1] // (NH + 2 * NKV)
     rep = NH // NKV
@@ -322,6 +322,9 @@ def rope_forward(packed, raw, freqs, T, NH, NKV):
     out[:, 0].copy_(q)
     out[:, 1].copy_(k.repeat_interleave(rep, dim=1))
     out[:, 2].copy_(v.repeat_interleave(rep, dim=1))
+    if kcache is not None:
+        kcache[:N // T, :T].copy_(k.view(N // T, T, NKV, HS))
+        vcache[:N // T, :T].copy_(v.view(N // T, T, NKV, HS))
 
 
 def rope_backward(draw, dpacked, freqs, T, NH, NKV):
