@@ -234,6 +234,121 @@ stream_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
     if (warp == 1) tmem_dealloc(tmem_base, tmem_cols);
 }
 
+// The same product with so many weight tiles that every CTA gets several (the LM head of a decoding step), K unsplit: CTAs stay and their TMA
+// warp runs on into the next tile while the epilogue warps, on one of two accumulators, finish the one before.  With a CTA per tile the loads of
+// every tile start with the set-up of its CTA and end with its epilogue: 4 x 50304 x 768 17.0 us against 12.8, 100 x 50304 x 768 29 against 16,
+// 16 x 128256 x 2048 86.5 against 83.8, 64 x 128256 x 4096 183 against 173 (6.1 TB/s).  The output leaves from the registers: a lane is an output
+// column.
+__global__ void __launch_bounds__(THREADS, 2)
+stream_wide_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX, const Args g) {
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    const int stage_bytes = W_BYTES + g.nb * (BK * 2);
+    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + g.stages * stage_bytes);
+    uint64_t* full = bars;                       // [MAX_STAGES]
+    uint64_t* empty = bars + MAX_STAGES;         // [MAX_STAGES]
+    uint64_t* acc_full = bars + 2 * MAX_STAGES;  // [2]
+    uint64_t* acc_empty = acc_full + 2;          // [2]
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int tiles = CEIL_DIV(g.N, WR);
+    const int acc_cols = g.nb <= 16 ? 16 : g.nb <= 32 ? 32 : g.nb <= 64 ? 64 : 128;
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < g.stages; s++) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
+        for (int b = 0; b < 2; b++) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], 4); }
+        *abort_flag = 0;
+        mbar_fence_init();
+        tma_prefetch_desc(&tmW); tma_prefetch_desc(&tmX);
+    }
+    if (warp == 1) { tmem_alloc(tmem_slot, 2 * acc_cols); tmem_relinquish(); }
+    if (warp >= 2) {
+        // the first tile's rows into L2 while the kernel before drains
+        const int row = blockIdx.x * WR + (int)threadIdx.x - 64;
+        if (row < g.N) prefetch_l2(g.w + (size_t)row * g.ldw, 2 * min(g.K, PREFETCH_BYTES / 2));
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem_base = *tmem_slot;
+    pdl_wait();
+    pdl_trigger();
+
+    if (warp == 0) {
+        if (lane == 0) {
+            int st = 0; uint32_t ph = 1;
+            bool ok = true;
+            for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
+                for (int kb = 0; kb < g.num_kb; kb++) {
+                    ok = mbar_wait_relaxed(&empty[st], ph, abort_flag, g.status, 0x930);
+                    if (!ok) break;
+                    uint8_t* dst = smem + st * stage_bytes;
+                    mbar_expect_tx(&full[st], stage_bytes);
+                    tma_load_2d(dst, &tmW, &full[st], kb * BK, tile * WR);                    // box {64 k, 128 rows}
+                    tma_load_2d(dst + W_BYTES, &tmX, &full[st], kb * BK, 0);                  // box {64 k, nb rows}
+                    if (++st == g.stages) { st = 0; ph ^= 1; }
+                }
+            }
+        }
+    } else if (warp == 1) {
+        const bool leader = elect_one();
+        const uint32_t idesc = umma_idesc_bf16(WR, 0, 0, 0) | ((uint32_t)(g.nb >> 3) << 17);
+        int st = 0; uint32_t ph = 0;
+        int it = 0;
+        bool ok = true;
+        for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x, it++) {
+            const int buf = it & 1;
+            ok = __all_sync(0xffffffffu, mbar_wait_relaxed(&acc_empty[buf], ((it >> 1) & 1) ^ 1, abort_flag, g.status, 0x938)) != 0;
+            for (int kb = 0; kb < g.num_kb && ok; kb++) {
+                ok = __all_sync(0xffffffffu, mbar_wait_relaxed(&full[st], ph, abort_flag, g.status, 0x931)) != 0;
+                if (!ok) break;
+                tc_fence_after();
+                const uint64_t dw = umma_desc_sw128(smem_u32(smem + st * stage_bytes), 16, 1024);
+                const uint64_t dx = umma_desc_sw128(smem_u32(smem + st * stage_bytes + W_BYTES), 16, 1024);
+                if (leader) {
+                    #pragma unroll
+                    for (int kk = 0; kk < BK / 16; kk++) umma_ss(tmem_base + buf * acc_cols, dw + 2 * kk, dx + 2 * kk, idesc, (kb | kk) > 0);
+                    umma_commit(&empty[st]);
+                    if (kb == g.num_kb - 1) umma_commit(&acc_full[buf]);
+                }
+                if (++st == g.stages) { st = 0; ph ^= 1; }
+            }
+        }
+    } else {
+        int it = 0;
+        bool ok = true;
+        for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x, it++) {
+            const int buf = it & 1;
+            ok = mbar_wait_relaxed(&acc_full[buf], (it >> 1) & 1, abort_flag, g.status, 0x932);
+            ok = __all_sync(0xffffffffu, ok) != 0;
+            tc_fence_after();
+            const int n = tile * WR + (warp & 3) * 32 + lane;
+            const float bias = g.bias != nullptr && n < g.N ? __bfloat162float(g.bias[n]) : 0.f;
+            for (int c = 0; c < g.nb && ok; c += 16) {
+                uint32_t v[16];
+                tmem_ld16(tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + buf * acc_cols + c, v);
+                tmem_ld_wait();
+                #pragma unroll
+                for (int e = 0; e < 16; e++)
+                    if (c + e < g.M && n < g.N) g.out[(size_t)(c + e) * g.ldo + n] = __float2bfloat16_rn(__uint_as_float(v[e]) + bias);
+            }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&acc_empty[buf]);
+        }
+    }
+    __syncthreads();
+    // after an abandoned wait copies may still be on their way into this CTA's shared memory: give them time to land before it is freed
+    if (*abort_flag) {
+        const long long t0 = clock64();
+        while (clock64() - t0 < 2000000ll) { __nanosleep(1000); }
+    }
+    __syncthreads();
+    tc_fence_after();
+    if (warp == 1) tmem_dealloc(tmem_base, 2 * acc_cols);
+}
+
 // CTAs per weight tile: as many as are resident at once and have some K blocks each; the wider the tile, the more blocks a slice must have to
 // be worth its share of the reduction.  A cluster lives in one GPC, so an eighth of the SMs is not counted on: 36 clusters of 4 on 148 SMs ran
 // in two waves.
@@ -275,6 +390,16 @@ int launch_stream(bf16* out, const bf16* x, const bf16* w, const bf16* bias, int
     }
     int sms = llmc_device_sm_count(); if (sms <= 0) sms = 148;
     const int tiles = CEIL_DIV(N, MODE == SWIGLU ? WR / 2 : WR);
+    if (MODE == STORE && !W_MN && mtiles == 1 && two && tiles > 2 * sms) {
+        static bool configured_wide = false;
+        const int smem = g.stages * stage_bytes + 1024 + 256;
+        if (!configured_wide) {
+            CUDA_CHECK(cudaFuncSetAttribute(stream_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_TWO));
+            configured_wide = true;
+        }
+        CUDA_CHECK(launch_pdl(stream_wide_kernel, dim3(2 * sms), dim3(THREADS), smem, stream, 0, tmW, tmX, g));
+        return 0;
+    }
     const int S = pick_split(tiles * mtiles, g.num_kb, g.nb, sms);
     g.kb_per_split = CEIL_DIV(g.num_kb, S);
     const int smem = g.stages * stage_bytes + 1024 + 256;

@@ -90,8 +90,8 @@ def _few_rows(M, N, K, mode, b_mn, device):
     """Whether a plain product goes to the split-K kernel with 128 x 256 tiles of csrc/stream_gemm.cu.  The lines are where it overtakes the other
     two kernels (M from 100 to 2048, fourteen pairs of N and K, us): deep products whose tiles leave at least half of the SMs idle
     (K = 3072: 24 tiles 21 against 27, 36 tiles 33 against 27; K = 7168: 64 tiles 37 to 43 against 53, 96 tiles 61 against 55), and
-    at most 128 rows, unless there are so many tiles that the overlap of tiles on a persistent CTA counts (100 x 50304 x 768:
-    39 against 31) or the product is a shallow input gradient (100 x 768 x 768: 16 against 14).  Forward products of more than 128 rows
+    at most 128 rows, unless the product is a shallow input gradient (100 x 768 x 768: 16 against 14); with more weight tiles than resident CTAs
+    the CTAs stay for several (100 x 50304 x 768 16 against 22, 128 x 128256 x 2048 96 against 108).  Forward products of more than 128 rows
     below a depth of 6144 keep their one sum over K: at 8 us each (256 x 768 x 3072: 18 against 27) they are not worth another order of
     summation in the loss.  At most 128 rows are summed in slices from K = 512 on, in fp32 and in slice order."""
     if mode != MODE_STORE:
@@ -102,7 +102,7 @@ def _few_rows(M, N, K, mode, b_mn, device):
         return True
     if b_mn:
         return M <= STREAM_MAX_ROWS and K >= 2048 and wtiles <= 2 * sm_count(device)
-    return M <= 64 or (M <= STREAM_MAX_ROWS and wtiles <= 2 * sm_count(device))
+    return M <= STREAM_MAX_ROWS
 
 
 def gemm(a, b, d, M, N, K, lda, ldb, ldd, a_mn, b_mn, mode, bias=None, aux=None, accumulate=False, splits=1, max_ctas=0, ready=None):
