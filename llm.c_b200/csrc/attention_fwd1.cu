@@ -11,7 +11,9 @@
 //                (no shared-memory round trip, no proxy fence); O accumulates in tensor memory across the key tiles and is
 //                rescaled by its own row's thread only when the running maximum grows by more than 2^8 (the stale maximum
 //                is a valid reference point for the exponentials in between, the final division by the row sum cancels it).
-//                The two groups are half a tile out of phase: one group's exponentials run under the other's products.
+//                The two groups take turns at the exponentials (common.cuh, turn_wait), so that one group's run under the other's
+//                loads, maxima and products; without turns they drift into step and compete for the unit (64 x 1024 x 12 heads
+//                233 us instead of 216, 2 x 4096 x 32 258 instead of 240).
 //
 // TMEM columns: S_A [0,128)  S_B [128,256)  O_A [256,320)  O_B [320,384)  P_A [384,448)  P_B [448,512)   (P: 128 bf16 per row)
 //
@@ -35,7 +37,7 @@ constexpr int KVSTAGES = 3;
 constexpr int THREADS = 384;                        // TMA warp, issuer warp, two idle warps, 2 x 4 softmax warps
 constexpr int TMEM_COLS = 512;
 constexpr int SMEM = QBUF * 2 * TILE_BYTES + KVSTAGES * 2 * TILE_BYTES + 2 * TILE_BYTES + 256;      // Q, K/V ring, two output tiles
-constexpr long long SKEW_CYCLES = 1200;
+constexpr int TURN_BAR = 3;                         // named barriers 3..10: [scheduler][slot] turns at the exponentials
 constexpr float RESCALE_LOG2 = 8.0f;                // the running maximum may lag by this much (in log2 units of the scaled scores)
 
 struct Args {
@@ -206,7 +208,7 @@ attn_fwd1_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constan
             if (w + (int)gridDim.x < total) { int b2, h2; decode(w + gridDim.x, np_, b2, h2); next_item = true; }
             // The order inside a step is the order in which the events arrive when slot B runs half a tile behind slot A:
             //   S_A(j+1) [A holds S_A(j)],  O_B += P_B(j-1) V,  S_B(j+1) [B holds S_B(j)],  O_A += P_A(j) V.
-            // With this order a lagging slot B never holds up slot A, so the skew (see the softmax warps) survives.
+            // With this order a lagging slot B never holds up slot A.
             for (int j = 0; j <= nkv && ok; j++) {
                 const uint32_t pos = kabs + j;
                 const int st_prev = (pos + KVSTAGES - 1) % KVSTAGES, st_cur = pos % KVSTAGES, st_next = (pos + 1) % KVSTAGES;
@@ -245,21 +247,21 @@ attn_fwd1_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constan
         const float c = a.scale_log2e;
         bool ok = true;
         bool staged = false;
+        if (x == 1) turn_pass(TURN_BAR + 2 * q4);          // slot A has the first turn
         uint32_t t = 0;                                    // tiles of this slot so far
         int it = 0;
         for (int w = blockIdx.x; w < total; w += gridDim.x, it++) {
             int p, b, h; decode(w, p, b, h);
             const int qi = 2 * p + x;                      // this slot's query tile
-            if (qi >= nq) continue;                        // (uniform for the slot) no second tile in this item
+            const int turns = min(2 * p + 2, nq);          // of either slot in this item
+            if (qi >= nq) {                                // (uniform for the slot) no second tile in this item
+                for (int j = 0; j < turns; j++) { turn_wait(TURN_BAR + 2 * q4 + x); turn_pass(TURN_BAR + 2 * q4 + (x ^ 1)); }
+                continue;
+            }
             float m = -INFINITY, l = 0.f;                  // reference maximum (raw score units) and row sum relative to it
-            // The two slots share the special-function unit: started together (their first S products are issued together) they
-            // would run their exponentials at the same time, at half rate each, and their loads, maxima and waits at the same
-            // time, with the unit idle.  Half a tile of skew (slot B pauses once its first S of the item is there) puts one slot's
-            // exponentials under the other's remaining work.
             for (int j = 0; j <= qi; j++, t++) {
                 if (r == 0) TRACE(1 + x, 0, t);
                 ok = mbar_wait(&s_full[x], t & 1, abort_flag, a.status, 0x520 + x) && ok;
-                if (x == 1 && j == 0) { const long long t0 = clock64(); while (clock64() - t0 < SKEW_CYCLES) { } }
                 tc_fence_after();
                 if (r == 0) TRACE(1 + x, 1, t);
                 uint32_t sv[128];
@@ -295,7 +297,8 @@ attn_fwd1_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constan
                     m = m_new;
                 }
                 if (r == 0) TRACE(1 + x, 3, t);
-                const float moff = m * c;
+                float moff = m * c;
+                turn_wait(TURN_BAR + 2 * q4 + x, moff);
                 float rs0 = 0.f, rs1 = 0.f;
                 uint32_t pk[64];
                 #pragma unroll
@@ -306,6 +309,7 @@ attn_fwd1_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constan
                     pk[e >> 1] = pack_bf16x2(p0, p1);
                 }
                 l += rs0 + rs1;
+                turn_pass(TURN_BAR + 2 * q4 + (x ^ 1), l);
                 if (r == 0) TRACE(1 + x, 5, t);
                 // the previous product has read P_X(t-1) and finished adding to O_X: only now is it waited for, so that it ran
                 // under the exponentials above
@@ -334,6 +338,7 @@ attn_fwd1_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constan
                 if (lane == 0) mbar_arrive(&p_ready[x]);
                 if (r == 0) TRACE(1 + x, 6, t);
             }
+            if (qi + 1 < turns) { turn_wait(TURN_BAR + 2 * q4 + x); turn_pass(TURN_BAR + 2 * q4 + (x ^ 1)); }      // slot A has a tile less
             // ---- item epilogue: O_X / l -> bf16 tile in the layout of a 128-byte-swizzled TMA box -> one bulk store
             ok = mbar_wait(&pv_done[x], (t - 1) & 1, abort_flag, a.status, 0x528 + x) && ok;
             tc_fence_after();
@@ -368,6 +373,7 @@ attn_fwd1_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constan
             const int trow = qi * BT + r;
             if (trow < a.T && ok) a.lse[((size_t)b * a.NH + h) * a.T + trow] = m * a.scale + logf(l);
         }
+        if (x == 0) turn_wait(TURN_BAR + 2 * q4);          // the last turn passed on by slot B
         if (issuer) tma_store_wait<0>();
     }
     tc_fence_before();

@@ -433,6 +433,14 @@ DEVINL void tmem_st32(uint32_t taddr, const uint32_t* r) {
 }
 DEVINL void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
+// Turns at a unit that two warps of a scheduler share (the special-function unit in softmax loops): started together they would run their
+// exponentials at the same time, at half rate each, and everything else at the same time, with the unit idle.  turn_wait(mine) waits until the other
+// warp has called turn_pass(mine); either names a barrier of 64 threads.  The float keeps the work between the two calls between them.
+DEVINL void turn_wait(int bar) { asm volatile("bar.sync %0, 64;" ::"r"(bar) : "memory"); }
+DEVINL void turn_wait(int bar, float& dep) { asm volatile("bar.sync %1, 64;" : "+f"(dep) : "r"(bar) : "memory"); }
+DEVINL void turn_pass(int bar) { asm volatile("bar.arrive %0, 64;" ::"r"(bar) : "memory"); }
+DEVINL void turn_pass(int bar, float& dep) { asm volatile("bar.arrive %1, 64;" : "+f"(dep) : "r"(bar) : "memory"); }
+
 DEVINL bool elect_one() {
     uint32_t pred;
     asm volatile(

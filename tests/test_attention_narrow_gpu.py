@@ -1,0 +1,37 @@
+"""64-wide heads at the sizes where their sequences of tiles change: one and an odd number of tiles, ragged lengths, more heads than CTAs."""
+import pytest
+import torch
+
+from llmc_b200 import _lib
+from llmc_b200.ops import kernels as KN
+from llmc_b200.ops import reference as R
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+@pytest.mark.parametrize("B,T,NH", [(2, 100, 3), (1, 129, 2), (25, 257, 6), (13, 300, 12), (4, 640, 38), (1, 2048, 5), (150, 200, 1)])
+def test_forward_and_backward(B, T, NH):
+    g = torch.Generator().manual_seed(B * T + NH)
+    qkv, dout = torch.randn(B, T, 3 * NH * 64, generator=g).bfloat16(), torch.randn(B, T, NH * 64, generator=g).bfloat16()
+    ro, rl, rd = torch.empty(B, T, NH * 64), torch.empty(B, NH, T), torch.empty(B, T, 3 * NH * 64)
+    R.attention_forward(ro, rl, qkv, B, T, NH)
+    R.attention_backward(rd, dout, qkv, ro, rl, B, T, NH)
+    rel = lambda a, r: float((a.float().cpu() - r).norm() / r.norm())
+    got = []
+    for _ in range(2):
+        out = torch.full((B + 1, T, NH * 64), 7.0, dtype=torch.bfloat16, device=DEV)
+        lse = torch.empty(B, NH, T, device=DEV)
+        buf = torch.full((B + 1, T, 3 * NH * 64), 7.0, dtype=torch.bfloat16, device=DEV)
+        KN.attention_forward(out[:B], lse, qkv.to(DEV), B, T, NH)
+        KN.attention_backward(buf[:B], dout.to(DEV), qkv.to(DEV), out[:B], lse, B, T, NH)
+        got.append((out, lse, buf))
+    assert _lib.read_status() == 0
+    assert all(torch.equal(x, y) for x, y in zip(*got))
+    out, lse, buf = got[0]
+    assert (out[B:] == 7.0).all() and (buf[B:] == 7.0).all()
+    # P, dS, O (through delta) and the result are each rounded to bf16 once, 2^-9 / sqrt(3) = 0.0011 in the mean square: 0.0023 together
+    assert rel(out[:B], ro) < 4e-3 and float((lse.cpu() - rl).abs().max()) < 1e-4
+    for c in range(3):
+        s = slice(c * NH * 64, (c + 1) * NH * 64)
+        assert rel(buf[:B, :, s], rd[..., s]) < 5e-3, c
