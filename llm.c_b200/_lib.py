@@ -54,6 +54,8 @@ def cuda():
         "llmc_free_device_or_managed": (I, [P]),
         "llmc_gemm": (I, [P, P, P, P, P, I, I, I, I, I, I, I, I, I, I, I, P, P, I, S]),
         "llmc_gemm_tiled": (I, [P, P, P, P, P, I, I, I, I, I, I, I, I, I, I, I, P, P, I, I, S]),
+        "llmc_gemm2t": (I, [P, P, P, P, I, I, I, I, I, I, I, S]),
+        "llmc_gemm2t_swiglu": (I, [P, P, P, I, I, I, I, I, I, I, S]),
         "llmc_gemm2": (I, [P, P, P, P, P, I, I, I, I, I, I, I, I, I, I, I, P, P, S]),
         "llmc_gemm2_after_flags": (I, [P, P, P, P, P, I, I, I, I, I, I, I, I, I, I, I, P, P, P, I, U64, S]),
         "llmc_gemm2_workspace": (None, [I, I, I, POINTER(c_longlong), POINTER(c_int)]),

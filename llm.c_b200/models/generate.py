@@ -111,6 +111,8 @@ class CachedDecoder:
             ops.rmsnorm_fused_residual_forward(a["res"][:N], ln[:N], rstd[:N], x[:N], a["proj"][:N], p["ln2w"][l], eps)
             if N <= min(self.skinny_rows, 128) and cfg.hidden_dim % 64 == 0:
                 ops.matmul_swiglu(a["h"][:N], ln[:N], p["fc12w"][l])
+            elif self.skinny_rows and N > 128 and cfg.hidden_dim % 128 == 0:
+                ops.matmul_swiglu_prompt(a["h"][:N], ln[:N], p["fc12w"][l])
             else:
                 mm(a["fc12"], ln, p["fc12w"][l], N)
                 ops.swiglu_forward(a["h"][:N], a["fc12"][:N])

@@ -24,6 +24,7 @@ _NAMES = [
     "params_from_master", "master_from_params", "sum_scaled",
     "rmsnorm_forward", "rmsnorm_fused_residual_forward", "rmsnorm_backward", "rope_forward", "rope_backward",
     "swiglu_forward", "swiglu_backward", "rope_cache", "cached_attention", "matmul_skinny", "matmul_swiglu",
+    "matmul_swiglu_prompt",
 ]
 
 

@@ -393,3 +393,6 @@ def swiglu_backward(dx12, dh, x12):
     sg = torch.sigmoid(x2)
     dx12[:, :H].copy_(dy * x2 * sg)
     dx12[:, H:].copy_(dy * x1 * sg * (1.0 + x2 * (1.0 - sg)))
+
+
+matmul_swiglu_prompt = matmul_swiglu
