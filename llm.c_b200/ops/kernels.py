@@ -89,47 +89,58 @@ def sm_count(device):
 def _few_rows(M, N, K, mode, b_mn, device):
     """Whether a plain product goes to the split-K kernel with 128 x 256 tiles of csrc/stream_gemm.cu.  The lines are where it overtakes the other
     two kernels (M from 100 to 2048, fourteen pairs of N and K, us): deep products whose tiles leave at least half of the SMs idle
-    (input gradients, K = 3072: 24 tiles 21 against 27, 36 tiles 33 against 27; forward 300 x 2048 x 7168 20 against 33, 300 x 4096 x 14336 47 against 51,
-    but 500 x 4096 x 14336 60 against 57 and 777 x 2048 x 7168 32 against 29), and
-    at most 128 rows, unless the product is a shallow input gradient (100 x 768 x 768: 16 against 14); with more weight tiles than resident CTAs
-    the CTAs stay for several (100 x 50304 x 768 16 against 22, 128 x 128256 x 2048 96 against 108).  Forward products of more than 128 rows
+    (K = 3072: 24 tiles 21 against 27, 36 tiles 33 against 27; K = 7168: 64 tiles 37 to 43 against 53, 96 tiles 61 against 55), and
+    at most 128 rows, unless there are more weight tiles than resident CTAs (64 rows and more, _wide) or the product is a shallow input gradient
+    (100 x 768 x 768: 16 against 14).  Forward products of more than 128 rows
     below a depth of 6144 keep their one sum over K: at 8 us each (256 x 768 x 3072: 18 against 27) they are not worth another order of
     summation in the loss.  At most 128 rows are summed in slices from K = 512 on, in fp32 and in slice order."""
     if mode != MODE_STORE:
         return False
     wtiles = (N + 127) // 128
     tiles = (M + 255) // 256 * wtiles
-    if K >= 6144 and (tiles <= 32 or (tiles <= 64 and (b_mn or M <= 384))) or (b_mn and K >= 3072 and tiles <= 32):
+    if (K >= 6144 and tiles <= 64) or (b_mn and K >= 3072 and tiles <= 32):
         return True
     if b_mn:
         return M <= STREAM_MAX_ROWS and K >= 2048 and wtiles <= 2 * sm_count(device)
-    return M <= STREAM_MAX_ROWS
+    return M <= 64 or (M <= STREAM_MAX_ROWS and wtiles <= 2 * sm_count(device))
+
+
+def _wide(M, N, device):
+    """Whether a plain forward product goes to the CTAs of csrc/stream_gemm.cu that stay for several weight tiles: at most 128 rows and more tiles
+    than resident CTAs (100 x 50304 x 768 16 us against 22 in 256-column tiles, 128 x 128256 x 2048 96 against 108)."""
+    return M <= STREAM_MAX_ROWS and (N + 127) // 128 > 2 * sm_count(device)
 
 
 def _swapped(M, N, K, device):
     """Whether a plain forward product goes to the two-SM kernel with swapped operand roles (csrc/gemm2t.cu), whose row tiles fit the rows: as long as
     the tiles fill few rounds of the CTA pairs and K is deep enough to hide its epilogue in pieces of 16 rows.  Same bits as the other two kernels.
     us, theirs in brackets: 777 x 3072 x 2048 12.7 (18.5), 777 x 14336 x 2048 40 (49), 500 x 6144 x 4096 23 (30), 3072 x 2048 x 2048 21.5 (26.6),
-    8192 x 2048 x 2048 60 (63), 256 x 2304 x 768 6.5 (6.8), 256 x 50304 x 768 25.5 (28.0); 512 x 1152 x 384 5.5 (5.1), 3001 x 28672 x 4096 522 (491)."""
-    tiles = (M + 255) // 256 * ((N + 255) // 256)
-    return 128 < M <= 8192 and K >= 768 and K % 8 == 0 and tiles <= 5 * sm_count(device)
+    8192 x 2048 x 2048 60 (63), 256 x 2304 x 768 6.5 (6.8), 256 x 50304 x 768 25.5 (28.0); 512 x 1152 x 384 5.5 (5.1), 3001 x 28672 x 4096 522 (491).
+    Deep products with few tiles are left to the split-K kernel: 300 x 2048 x 7168 33 against 20, 300 x 4096 x 14336 51 against 47, but
+    500 x 4096 x 14336 57 against 60 and 777 x 2048 x 7168 29 against 32."""
+    mt = (M + 255) // 256
+    if not (128 < M <= 8192 and K >= 768 and K % 8 == 0 and mt * ((N + 255) // 256) <= 5 * sm_count(device)):
+        return False
+    split = mt * ((N + 127) // 128)
+    return K < 6144 or split > 64 or (split > 32 and M > 384)
 
 
 def gemm(a, b, d, M, N, K, lda, ldb, ldd, a_mn, b_mn, mode, bias=None, aux=None, accumulate=False, splits=1, max_ctas=0, ready=None):
-    """Dispatches to the split-K kernel for plain products with few tiles (``_few_rows``), to one of the two-SM kernels (``_swapped``; 256 x 256 tiles on
+    """Dispatches to the split-K kernel for plain products with few tiles (``_few_rows``, ``_wide``), to one of the two-SM kernels (``_swapped``; 256 x 256 tiles on
     CTA pairs) for problems with enough tiles, else to the single-CTA one.
     ``ready`` (an object with flags_ptr, n, seq and wait()) marks the B operand as the target of an all-gather in flight: the
     two-SM kernel polls the peers' flags itself before its first load; the single-CTA kernel runs after ``ready.wait()``."""
     global _launches
     lib = _lib.cuda()
     _launches += 1
-    if not a_mn and _few_rows(M, N, K, mode, b_mn, d.device):
+    plain_forward = mode == MODE_STORE and not a_mn and not b_mn
+    if plain_forward and ready is None and TWO_SM_MIN_TILES > 0 and _swapped(M, N, K, d.device):
+        check(lib.llmc_gemm2t(_p(d), _p(a), _p(b), _p(bias), M, N, K, lda, ldb, ldd, 0, _stream()), "llmc_gemm2t")
+        return
+    if not a_mn and (_few_rows(M, N, K, mode, b_mn, d.device) or (plain_forward and _wide(M, N, d.device))):
         if ready is not None:
             ready.wait()
         check(lib.llmc_stream_gemm(_p(d), _p(a), _p(b), _p(bias), M, N, K, lda, ldb, ldd, int(b_mn), _stream()), "llmc_stream_gemm")
-        return
-    if mode == MODE_STORE and not a_mn and not b_mn and ready is None and TWO_SM_MIN_TILES > 0 and _swapped(M, N, K, d.device):
-        check(lib.llmc_gemm2t(_p(d), _p(a), _p(b), _p(bias), M, N, K, lda, ldb, ldd, 0, _stream()), "llmc_gemm2t")
         return
     tiles256 = ((M + 255) // 256) * ((N + 255) // 256)
     if mode == MODE_ACCUM:
