@@ -23,6 +23,15 @@ class TensorTable(Structure):
     _fields_ = [("t", TensorView * 16), ("count", c_int)]
 
 
+class DecoderCall(Structure):
+    """Argument of llmc_decoder_forward (csrc/decoder.cu): addresses, then sizes."""
+    _fields_ = [(n, c_void_p) for n in (
+        "wte", "ln1w", "qkvw", "attprojw", "ln2w", "fc12w", "fcprojw", "lnfw", "lmhead", "freqs", "kcache", "vcache", "x", "ln", "raw", "q", "atty",
+        "proj", "res", "fc12", "h", "last", "logits", "rstd", "packed", "lse", "attention_ws", "tokens", "pos")] + [(n, c_int) for n in (
+            "L", "C", "H", "NH", "NKV", "HS", "vocab_rows", "logit_cols", "freqs_len", "max_batch", "cache_len", "B", "Tq", "start",
+            "how_qkv", "how_attproj", "how_fc12", "how_fcproj", "how_head", "mlp")] + [("eps", c_float)]
+
+
 def _load(name, builder):
     path = os.path.join(LIBDIR, name)
     from . import build as _b
@@ -56,6 +65,7 @@ def cuda():
         "llmc_gemm_tiled": (I, [P, P, P, P, P, I, I, I, I, I, I, I, I, I, I, I, P, P, I, I, S]),
         "llmc_gemm2t": (I, [P, P, P, P, I, I, I, I, I, I, I, S]),
         "llmc_gemm2t_swiglu": (I, [P, P, P, I, I, I, I, I, I, I, S]),
+        "llmc_decoder_forward": (I, [POINTER(DecoderCall), POINTER(c_int), S]),
         "llmc_gemm2": (I, [P, P, P, P, P, I, I, I, I, I, I, I, I, I, I, I, P, P, S]),
         "llmc_gemm2_after_flags": (I, [P, P, P, P, P, I, I, I, I, I, I, I, I, I, I, I, P, P, P, I, U64, S]),
         "llmc_gemm2_workspace": (None, [I, I, I, POINTER(c_longlong), POINTER(c_int)]),

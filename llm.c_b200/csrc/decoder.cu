@@ -1,0 +1,111 @@
+// The launches of one pass of a LLaMA decoder with a key / value cache (models/generate.py, CachedDecoder.forward), issued from native code: embedding,
+// per layer RMSNorm, QKV projection, rotary embedding into the cache, attention, projection, RMSNorm with residual, the SwiGLU MLP, at the end
+// the LM head of the last positions.  No kernel of its own.  Issued from Python, a launch took the host 15 to 20 us: a prompt of 777 tokens in four layers
+// was bound by the host (740 us against about 600 on the GPU).
+#include "common.cuh"
+
+extern "C" {
+int llmc_encoder_fwd(bf16* out, const int* tokens, const bf16* wte, const bf16* wpe, int B, int T, int C, int V, cudaStream_t stream);
+int llmc_rmsnorm_fwd(bf16* out, float* rstd, const bf16* inp, const bf16* weight, int N, int C, float eps, cudaStream_t stream);
+int llmc_rmsnorm_fused_residual_fwd(bf16* residual, bf16* normed, float* rstd, const bf16* inp1, const bf16* inp2, const bf16* weight, int N, int C,
+                                    float eps, cudaStream_t stream);
+int llmc_rope_fwd_cache(bf16* packed, const bf16* raw, const float* freqs, bf16* kcache, bf16* vcache, int cache_len, long long N, int T, int NH, int NKV,
+                        int HS, cudaStream_t stream);
+int llmc_rope_cache(bf16* q, bf16* kcache, bf16* vcache, const bf16* raw, const float* freqs, int freqs_len, int B, int Tq, int Tmax, int start_pos,
+                    int NH, int NKV, int HS, const int* pos_ptr, cudaStream_t stream);
+int llmc_attention_fwd(bf16* out, float* lse, const bf16* qkv, int B, int T, int NH, int hs, cudaStream_t stream);
+int llmc_cached_attention(bf16* out, const bf16* q, const bf16* kcache, const bf16* vcache, int B, int Tq, int Tmax, int start_pos, int NH, int NKV,
+                          int HS, const int* pos_ptr, float* ws, cudaStream_t stream);
+int llmc_swiglu_fwd(bf16* h, const bf16* x12, long long N, int H, cudaStream_t stream);
+int llmc_stream_gemm_chained(bf16* out, const bf16* x, const bf16* w, int M, int N, int K, int ldx, int ldw, int ldo, cudaStream_t stream);
+int llmc_stream_gemm_swiglu_chained(bf16* out, const bf16* x, const bf16* w, int M, int N, int K, int ldx, int ldw, int ldo, cudaStream_t stream);
+int llmc_gemm2t_chained(bf16* out, const bf16* x, const bf16* w, int M, int N, int K, int ldx, int ldw, int ldo, cudaStream_t stream);
+int llmc_gemm2t_swiglu_chained(bf16* out, const bf16* x, const bf16* w, int M, int N, int K, int ldx, int ldw, int ldo, cudaStream_t stream);
+int llmc_gemm2(const bf16* A, const bf16* B, bf16* D, const bf16* bias, bf16* aux, int M, int N, int K, int lda, int ldb, int ldd, int a_mn_major,
+               int b_mn_major, int mode, int accumulate, int splits, float* workspace, unsigned int* counters, cudaStream_t stream);
+int llmc_gemm(const bf16* A, const bf16* B, bf16* D, const bf16* bias, bf16* aux, int M, int N, int K, int lda, int ldb, int ldd, int a_mn_major,
+              int b_mn_major, int mode, int accumulate, int splits, float* workspace, unsigned int* counters, int max_ctas, cudaStream_t stream);
+}
+
+// Kernel of a forward product, chosen by the caller (ops/kernels.py, forward_kernel)
+enum Product : int { GEMM = 0, GEMM2 = 1, STREAM = 2, GEMM2T = 3 };
+// MLP: up-projections and activation in two launches, or one of the two fused forms
+enum Mlp : int { MLP_TWO = 0, MLP_STREAM = 1, MLP_GEMM2T = 2 };
+
+// Mirrored field by field by DecoderCall in _lib.py.
+struct DecoderCall {
+    // model: weights of layer l follow those of layer l - 1
+    const bf16 *wte, *ln1w, *qkvw, *attprojw, *ln2w, *fc12w, *fcprojw, *lnfw, *lmhead;
+    const float* freqs;
+    // caches (L, max_batch, cache_len, NKV, HS)
+    bf16 *kcache, *vcache;
+    // activations, at least B * Tq rows (last, logits: B)
+    bf16 *x, *ln, *raw, *q, *atty, *proj, *res, *fc12, *h, *last, *logits;
+    float* rstd;
+    bf16* packed; float* lse;             // dense prompts only (null: attention over the cache)
+    float* attention_ws;                  // of llmc_cached_attention, null where it needs none
+    const int* tokens; const int* pos;    // pos: position on the device (null: start)
+    int L, C, H, NH, NKV, HS, vocab_rows, logit_cols, freqs_len, max_batch, cache_len;
+    int B, Tq, start;
+    int how_qkv, how_attproj, how_fc12, how_fcproj, how_head, mlp;
+    float eps;
+};
+
+namespace {
+// In this chain the kernel in front of a product never writes weights, so that those that can do it read them while it drains.
+int product(int how, bf16* out, const bf16* x, const bf16* w, int M, int N, int K, cudaStream_t s) {
+    switch (how) {
+        case GEMM2T: return llmc_gemm2t_chained(out, x, w, M, N, K, K, K, N, s);
+        case STREAM: return llmc_stream_gemm_chained(out, x, w, M, N, K, K, K, N, s);
+        case GEMM2: return llmc_gemm2(x, w, out, nullptr, nullptr, M, N, K, K, K, N, 0, 0, 0, 0, 1, nullptr, nullptr, s);
+        case GEMM: return llmc_gemm(x, w, out, nullptr, nullptr, M, N, K, K, K, N, 0, 0, 0, 0, 1, nullptr, nullptr, 0, s);
+    }
+    return -1;
+}
+}  // namespace
+
+// launches: number of kernels issued
+extern "C" int llmc_decoder_forward(const DecoderCall* c, int* launches, cudaStream_t s) {
+    const int N = c->B * c->Tq, C = c->C, H = c->H, QR = (c->NH + 2 * c->NKV) * c->HS;
+    const size_t cache = (size_t)c->max_batch * c->cache_len * c->NKV * c->HS;
+    const bool dense = c->packed != nullptr;
+    int rc, n = 0;
+#define GO(call) do { if ((rc = (call))) return rc; n++; } while (0)
+    GO(llmc_encoder_fwd(c->x, c->tokens, c->wte, nullptr, c->B, c->Tq, C, c->vocab_rows, s));
+    GO(llmc_rmsnorm_fwd(c->ln, c->rstd, c->x, c->ln1w, N, C, c->eps, s));
+    for (int l = 0; l < c->L; l++) {
+        bf16 *kc = c->kcache + l * cache, *vc = c->vcache + l * cache;
+        GO(product(c->how_qkv, c->raw, c->ln, c->qkvw + (size_t)l * QR * C, N, QR, C, s));
+        if (dense) {
+            GO(llmc_rope_fwd_cache(c->packed, c->raw, c->freqs, kc, vc, c->cache_len, N, c->Tq, c->NH, c->NKV, c->HS, s));
+            GO(llmc_attention_fwd(c->atty, c->lse, c->packed, c->B, c->Tq, c->NH, c->HS, s));
+        } else {
+            GO(llmc_rope_cache(c->q, kc, vc, c->raw, c->freqs, c->freqs_len, c->B, c->Tq, c->cache_len, c->start, c->NH, c->NKV, c->HS, c->pos, s));
+            GO(llmc_cached_attention(c->atty, c->q, kc, vc, c->B, c->Tq, c->cache_len, c->start, c->NH, c->NKV, c->HS, c->pos, c->attention_ws, s));
+            if (c->attention_ws) n++;
+        }
+        GO(product(c->how_attproj, c->proj, c->atty, c->attprojw + (size_t)l * C * C, N, C, C, s));
+        GO(llmc_rmsnorm_fused_residual_fwd(c->res, c->ln, c->rstd, c->x, c->proj, c->ln2w + (size_t)l * C, N, C, c->eps, s));
+        const bf16* w12 = c->fc12w + (size_t)l * 2 * H * C;
+        if (c->mlp == MLP_STREAM) {
+            GO(llmc_stream_gemm_swiglu_chained(c->h, c->ln, w12, N, H, C, C, C, H, s));
+        } else if (c->mlp == MLP_GEMM2T) {
+            GO(llmc_gemm2t_swiglu_chained(c->h, c->ln, w12, N, H, C, C, C, H, s));
+        } else {
+            GO(product(c->how_fc12, c->fc12, c->ln, w12, N, 2 * H, C, s));
+            GO(llmc_swiglu_fwd(c->h, c->fc12, N, H, s));
+        }
+        GO(product(c->how_fcproj, c->proj, c->h, c->fcprojw + (size_t)l * C * H, N, C, H, s));
+        GO(llmc_rmsnorm_fused_residual_fwd(c->x, c->ln, c->rstd, c->res, c->proj, l + 1 < c->L ? c->ln1w + (size_t)(l + 1) * C : c->lnfw, N, C, c->eps, s));
+    }
+    const bf16* last = c->ln;                           // one token per row: the last positions are the rows themselves
+    if (c->Tq > 1) {
+        CUDA_CHECK(cudaMemcpy2DAsync(c->last, (size_t)C * 2, c->ln + (size_t)(c->Tq - 1) * C, (size_t)c->Tq * C * 2, (size_t)C * 2, c->B,
+                                     cudaMemcpyDeviceToDevice, s));
+        last = c->last;
+    }
+    GO(product(c->how_head, c->logits, last, c->lmhead, c->B, c->logit_cols, C, s));
+#undef GO
+    *launches = n;
+    return 0;
+}

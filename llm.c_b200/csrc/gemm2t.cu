@@ -34,6 +34,7 @@ struct Args {
     const bf16* bias;          // N entries or null
     int M, N, K;
     int nb, m_tiles, n_tiles, num_kb, stages;
+    int early_w;               // no kernel directly in front of this one writes the weights: they are read before it has completed
     unsigned int* status;
 };
 
@@ -70,12 +71,28 @@ gemm2t_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ C
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
-    pdl_wait();
 
     // output columns of a pair's tile and of a CTA's share; the row tiles of one weight tile run side by side, so that it is read from DRAM once
     constexpr int COLS = SWIGLU ? 128 : 256, CTA_COLS = COLS / 2;
     auto col0 = [&](int w) { return (w / g.m_tiles) * COLS + (int)rank * CTA_COLS; };
     auto row0 = [&](int w) { return (w % g.m_tiles) * g.nb; };
+
+    auto load_w = [&](int n0, int kb, int stage) {
+        uint8_t* dst = smem + stage * stage_bytes;
+        const uint32_t lead_full = map_to_cta(smem_u32(&full[stage]), 0);
+        if (rank == 0) mbar_expect_tx(&full[stage], 2 * stage_bytes);              // bytes of both CTAs
+        if (SWIGLU) {
+            tma_load_2d_2sm(dst, &tmW, lead_full, kb * BK, n0);                    // boxes {64 k, 64 rows}
+            tma_load_2d_2sm(dst + W_BYTES / 2, &tmW, lead_full, kb * BK, g.N + n0);
+        } else {
+            tma_load_2d_2sm(dst, &tmW, lead_full, kb * BK, n0);                    // box {64 k, 128 rows}
+        }
+    };
+    int early = g.early_w && pair < total ? min(g.stages, g.num_kb) : 0;          // stages filled with weights while the kernel before drains
+    if (warp == 0 && lane == 0)
+        for (int kb = 0; kb < early; kb++) load_w(col0(pair), kb, kb);
+    __syncwarp();
+    pdl_wait();
 
     if (warp == 0) {
         if (lane == 0) {
@@ -84,19 +101,14 @@ gemm2t_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ C
             for (int w = pair; w < total && !fail; w += npairs) {
                 const int n0 = col0(w), m0 = row0(w) + (int)rank * (g.nb / 2);
                 for (int kb = 0; kb < g.num_kb; kb++) {
-                    if (!mbar_wait(&empty[stage], phase ^ 1, abort_flag, g.status, 0xD00 + stage)) { fail = true; break; }
-                    uint8_t* dst = smem + stage * stage_bytes;
-                    const uint32_t lead_full = map_to_cta(smem_u32(&full[stage]), 0);
-                    if (rank == 0) mbar_expect_tx(&full[stage], 2 * stage_bytes);              // bytes of both CTAs
-                    if (SWIGLU) {
-                        tma_load_2d_2sm(dst, &tmW, lead_full, kb * BK, n0);                    // boxes {64 k, 64 rows}
-                        tma_load_2d_2sm(dst + W_BYTES / 2, &tmW, lead_full, kb * BK, g.N + n0);
-                    } else {
-                        tma_load_2d_2sm(dst, &tmW, lead_full, kb * BK, n0);                    // box {64 k, 128 rows}
+                    if (kb >= early) {
+                        if (!mbar_wait(&empty[stage], phase ^ 1, abort_flag, g.status, 0xD00 + stage)) { fail = true; break; }
+                        load_w(n0, kb, stage);
                     }
-                    tma_load_2d_2sm(dst + W_BYTES, &tmX, lead_full, kb * BK, m0);              // box {64 k, nb / 2 rows}
+                    tma_load_2d_2sm(smem + stage * stage_bytes + W_BYTES, &tmX, map_to_cta(smem_u32(&full[stage]), 0), kb * BK, m0);    // box {64 k, nb / 2 rows}
                     if (++stage == g.stages) { stage = 0; phase ^= 1; }
                 }
+                early = 0;
             }
         }
     } else if (warp == 1) {
@@ -213,12 +225,14 @@ void pick_rows(int M, int n_tiles, int pairs, int& m_tiles, int& nb) {
 }
 
 template <bool SWIGLU>
-int launch_gemm2t(bf16* out, const bf16* x, const bf16* w, const bf16* bias, int M, int N, int K, int ldx, int ldw, int ldo, int rows, cudaStream_t stream) {
+int launch_gemm2t(bf16* out, const bf16* x, const bf16* w, const bf16* bias, int M, int N, int K, int ldx, int ldw, int ldo, int rows, int early_w,
+                  cudaStream_t stream) {
     if (M <= 0 || N <= 0 || K <= 0) return 0;
     if ((K % 8) || (N % 8) || (ldx % 8) || (ldw % 8) || (ldo % 8) || ldx < K || ldw < K || ldo < N) return -1;
     if (SWIGLU && (N % 128)) return -1;
     int sms = llmc_device_sm_count(); if (sms <= 0) sms = 148;
     Args g;
+    g.early_w = early_w;
     g.bias = bias; g.M = M; g.N = N; g.K = K; g.status = llmc_status_ptr();
     g.n_tiles = CEIL_DIV(N, SWIGLU ? 128 : 256);
     g.num_kb = CEIL_DIV(K, BK);
@@ -262,10 +276,19 @@ int launch_gemm2t(bf16* out, const bf16* x, const bf16* w, const bf16* bias, int
 // multiple of 16 up to 256 (0: pick_rows).
 extern "C" int llmc_gemm2t(bf16* out, const bf16* x, const bf16* w, const bf16* bias, int M, int N, int K, int ldx, int ldw, int ldo, int rows,
                            cudaStream_t stream) {
-    return launch_gemm2t<false>(out, x, w, bias, M, N, K, ldx, ldw, ldo, rows, stream);
+    return launch_gemm2t<false>(out, x, w, bias, M, N, K, ldx, ldw, ldo, rows, 0, stream);
+}
+
+// The same behind a kernel that does not write w (csrc/decoder.cu): an early launch fills the stages with weights while that kernel drains.  What other
+// kernels before it wrote is complete: it triggers the launch after its own wait (pdl.cuh).
+extern "C" int llmc_gemm2t_chained(bf16* out, const bf16* x, const bf16* w, int M, int N, int K, int ldx, int ldw, int ldo, cudaStream_t stream) {
+    return launch_gemm2t<false>(out, x, w, nullptr, M, N, K, ldx, ldw, ldo, 0, 1, stream);
 }
 
 // out (M, N) = (x . w1^T) * silu(x . w2^T) with w = [w1; w2] of 2 N rows; N a multiple of 128
 extern "C" int llmc_gemm2t_swiglu(bf16* out, const bf16* x, const bf16* w, int M, int N, int K, int ldx, int ldw, int ldo, int rows, cudaStream_t stream) {
-    return launch_gemm2t<true>(out, x, w, nullptr, M, N, K, ldx, ldw, ldo, rows, stream);
+    return launch_gemm2t<true>(out, x, w, nullptr, M, N, K, ldx, ldw, ldo, rows, 0, stream);
+}
+extern "C" int llmc_gemm2t_swiglu_chained(bf16* out, const bf16* x, const bf16* w, int M, int N, int K, int ldx, int ldw, int ldo, cudaStream_t stream) {
+    return launch_gemm2t<true>(out, x, w, nullptr, M, N, K, ldx, ldw, ldo, 0, 1, stream);
 }

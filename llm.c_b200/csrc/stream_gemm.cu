@@ -46,6 +46,7 @@ struct Args {
     int nb;                    // activation rows of a tile, a multiple of 16
     int stages, num_kb, kb_per_split;
     int vec_out;               // rows of out start on 8-byte boundaries
+    int early_w;               // no kernel directly in front of this one writes the weights: they are read before it has completed
     unsigned int* status;
 };
 
@@ -126,6 +127,23 @@ stream_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    auto load_w = [&](int kb, int st) {
+        uint8_t* dst = smem + st * stage_bytes;
+        mbar_expect_tx(&full[st], stage_bytes);
+        if (W_MN) {
+            tma_load_2d(dst, &tmW, &full[st], n0, kb * BK);                                   // boxes {64 n, 64 k}
+            tma_load_2d(dst + W_BYTES / 2, &tmW, &full[st], n0 + 64, kb * BK);
+        } else if (MODE == SWIGLU) {
+            tma_load_2d(dst, &tmW, &full[st], kb * BK, n0);                                   // boxes {64 k, 64 rows}
+            tma_load_2d(dst + W_BYTES / 2, &tmW, &full[st], kb * BK, g.N + n0);
+        } else {
+            tma_load_2d(dst, &tmW, &full[st], kb * BK, n0);                                   // box {64 k, 128 rows}
+        }
+    };
+    const int early = g.early_w ? min(g.stages, kb1 - kb0) : 0;       // stages filled with weights while the kernel before drains
+    if (warp == 0 && lane == 0)
+        for (int it = 0; it < early; it++) load_w(kb0 + it, it);
+    __syncwarp();
     pdl_wait();
     pdl_trigger();
 
@@ -133,19 +151,11 @@ stream_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
         if (lane == 0) {
             for (int kb = kb0; kb < kb1; kb++) {
                 const int it = kb - kb0, st = it % g.stages;
-                if (!mbar_wait_relaxed(&empty[st], ((it / g.stages) & 1) ^ 1, abort_flag, g.status, 0x900)) break;
-                uint8_t* dst = smem + st * stage_bytes;
-                mbar_expect_tx(&full[st], stage_bytes);
-                if (W_MN) {
-                    tma_load_2d(dst, &tmW, &full[st], n0, kb * BK);                                   // boxes {64 n, 64 k}
-                    tma_load_2d(dst + W_BYTES / 2, &tmW, &full[st], n0 + 64, kb * BK);
-                } else if (MODE == SWIGLU) {
-                    tma_load_2d(dst, &tmW, &full[st], kb * BK, n0);                                   // boxes {64 k, 64 rows}
-                    tma_load_2d(dst + W_BYTES / 2, &tmW, &full[st], kb * BK, g.N + n0);
-                } else {
-                    tma_load_2d(dst, &tmW, &full[st], kb * BK, n0);                                   // box {64 k, 128 rows}
+                if (it >= early) {
+                    if (!mbar_wait_relaxed(&empty[st], ((it / g.stages) & 1) ^ 1, abort_flag, g.status, 0x900)) break;
+                    load_w(kb, st);
                 }
-                tma_load_2d(dst + W_BYTES, &tmX, &full[st], kb * BK, m0);                             // box {64 k, nb rows}
+                tma_load_2d(smem + st * stage_bytes + W_BYTES, &tmX, &full[st], kb * BK, m0);         // box {64 k, nb rows}
             }
         }
     } else if (warp == 1) {
@@ -272,6 +282,14 @@ stream_wide_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    auto load_w = [&](int tile, int kb, int st) {
+        mbar_expect_tx(&full[st], stage_bytes);
+        tma_load_2d(smem + st * stage_bytes, &tmW, &full[st], kb * BK, tile * WR);            // box {64 k, 128 rows}
+    };
+    int early = g.early_w ? min(g.stages, g.num_kb) : 0;              // stages filled with weights while the kernel before drains
+    if (warp == 0 && lane == 0)
+        for (int kb = 0; kb < early; kb++) load_w(blockIdx.x, kb, kb);
+    __syncwarp();
     pdl_wait();
     pdl_trigger();
 
@@ -281,14 +299,15 @@ stream_wide_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
             bool ok = true;
             for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
                 for (int kb = 0; kb < g.num_kb; kb++) {
-                    ok = mbar_wait_relaxed(&empty[st], ph, abort_flag, g.status, 0x930);
-                    if (!ok) break;
-                    uint8_t* dst = smem + st * stage_bytes;
-                    mbar_expect_tx(&full[st], stage_bytes);
-                    tma_load_2d(dst, &tmW, &full[st], kb * BK, tile * WR);                    // box {64 k, 128 rows}
-                    tma_load_2d(dst + W_BYTES, &tmX, &full[st], kb * BK, 0);                  // box {64 k, nb rows}
+                    if (kb >= early) {
+                        ok = mbar_wait_relaxed(&empty[st], ph, abort_flag, g.status, 0x930);
+                        if (!ok) break;
+                        load_w(tile, kb, st);
+                    }
+                    tma_load_2d(smem + st * stage_bytes + W_BYTES, &tmX, &full[st], kb * BK, 0);       // box {64 k, nb rows}
                     if (++st == g.stages) { st = 0; ph ^= 1; }
                 }
+                early = 0;
             }
         }
     } else if (warp == 1) {
@@ -360,10 +379,11 @@ int pick_split(int tiles, int num_kb, int nb, int sms) {
 }
 
 template <int MODE, bool W_MN>
-int launch_stream(bf16* out, const bf16* x, const bf16* w, const bf16* bias, int M, int N, int K, int ldx, int ldw, int ldo, cudaStream_t stream) {
+int launch_stream(bf16* out, const bf16* x, const bf16* w, const bf16* bias, int M, int N, int K, int ldx, int ldw, int ldo, int early_w, cudaStream_t stream) {
     if (M <= 0 || N <= 0 || K <= 0 || (K % 8) || (ldx % 8) || (ldw % 8) || ldx < K || ldw < (W_MN ? N : K) || ldo < N) return -1;
     if (W_MN && (N % 8)) return -1;
     Args g;
+    g.early_w = early_w;
     g.out = out; g.bias = bias; g.w = w; g.M = M; g.N = N; g.K = K; g.ldo = ldo; g.ldw = ldw;
     const int mtiles = CEIL_DIV(M, MAX_NB);
     g.nb = (CEIL_DIV(M, mtiles) + 15) & ~15;             // M spread evenly over its tiles
@@ -418,12 +438,23 @@ int launch_stream(bf16* out, const bf16* x, const bf16* w, const bf16* bias, int
 extern "C" int llmc_stream_gemm(bf16* out, const bf16* x, const bf16* w, const bf16* bias, int M, int N, int K, int ldx, int ldw, int ldo, int w_mn,
                                 cudaStream_t stream) {
     if (M <= 0 || N <= 0 || K <= 0) return 0;        // an empty product leaves out as it is, like the other two kernels'
-    if (w_mn) return launch_stream<STORE, true>(out, x, w, bias, M, N, K, ldx, ldw, ldo, stream);
-    return launch_stream<STORE, false>(out, x, w, bias, M, N, K, ldx, ldw, ldo, stream);
+    if (w_mn) return launch_stream<STORE, true>(out, x, w, bias, M, N, K, ldx, ldw, ldo, 0, stream);
+    return launch_stream<STORE, false>(out, x, w, bias, M, N, K, ldx, ldw, ldo, 0, stream);
+}
+
+// The same behind a kernel that does not write w (csrc/decoder.cu): an early launch fills the stages with weights while that kernel drains.  What other
+// kernels before it wrote is complete: it triggers the launch after its own wait (pdl.cuh).
+extern "C" int llmc_stream_gemm_chained(bf16* out, const bf16* x, const bf16* w, int M, int N, int K, int ldx, int ldw, int ldo, cudaStream_t stream) {
+    if (M <= 0 || N <= 0 || K <= 0) return 0;
+    return launch_stream<STORE, false>(out, x, w, nullptr, M, N, K, ldx, ldw, ldo, 1, stream);
 }
 
 // out (M, N) = (x . w1^T) * silu(x . w2^T) with w = [w1; w2] of 2 N rows, M <= 128; N a multiple of 64
 extern "C" int llmc_stream_gemm_swiglu(bf16* out, const bf16* x, const bf16* w, int M, int N, int K, int ldx, int ldw, int ldo, cudaStream_t stream) {
     if (N % 64 || M > 128) return -1;
-    return launch_stream<SWIGLU, false>(out, x, w, nullptr, M, N, K, ldx, ldw, ldo, stream);
+    return launch_stream<SWIGLU, false>(out, x, w, nullptr, M, N, K, ldx, ldw, ldo, 0, stream);
+}
+extern "C" int llmc_stream_gemm_swiglu_chained(bf16* out, const bf16* x, const bf16* w, int M, int N, int K, int ldx, int ldw, int ldo, cudaStream_t stream) {
+    if (N % 64 || M > 128) return -1;
+    return launch_stream<SWIGLU, false>(out, x, w, nullptr, M, N, K, ldx, ldw, ldo, 1, stream);
 }

@@ -45,7 +45,7 @@ class CachedDecoder:
         self.whole_tiles = model.device.type == "cuda"
         # steps of at most this many rows run their products on exactly their rows (split-K weight streaming, csrc/stream_gemm.cu), the MLP's
         # up-projections with the activation in the same launch, instead of on rows padded to whole 128-row tiles (0: never)
-        self.skinny_rows = 128 if model.device.type == "cuda" and model.dtype == torch.bfloat16 else 0
+        self.skinny_rows = kernels.STREAM_MAX_ROWS if model.device.type == "cuda" and model.dtype == torch.bfloat16 else 0
 
     def cache_bytes(self):
         return 2 * self.kcache.numel() * self.kcache.element_size()
@@ -83,6 +83,19 @@ class CachedDecoder:
         L, NH, NKV, eps, C = cfg.num_layers, cfg.num_heads, cfg.num_kv_heads, cfg.norm_eps, cfg.channels
         x, ln, rstd = a["x"], a["ln"], a["rstd"]
 
+        # a long prompt from position 0 is the training forward pass: its attention kernel (tensor cores, one pass over the
+        # keys per 128 queries) replaces the per-query scan of the cache, and the rotary kernel writes keys / values to the cache too
+        dense = pos is None and start_pos == 0 and Tq >= self.dense_prefill_from
+        packed = lse = None
+        if dense:
+            if self._dense is None or self._dense[0].shape[0] < N or self._dense[1].numel() < B * NH * Tq:
+                self._dense = (torch.zeros(rows, 3 * C, dtype=m.dtype, device=m.device),
+                               torch.zeros(B * NH * Tq, dtype=torch.float32, device=m.device))
+            packed, lse = self._dense[0][:N], self._dense[1][:B * NH * Tq].view(B, NH, Tq)
+        if self.skinny_rows == kernels.STREAM_MAX_ROWS:
+            kernels.decoder_forward(self, a, (packed, lse) if dense else None, tokens, start_pos, pos)
+            return a["logits"][:B, :cfg.vocab_size].float()
+
         def mm(out, inp, weight, n):
             if self.whole_tiles and n > self.skinny_rows:
                 n = _whole_tiles(n)                             # the rows beyond n are never read
@@ -91,14 +104,6 @@ class CachedDecoder:
 
         ops.encoder_forward(x[:N].view(B, Tq, C), tokens, p["wte"], None)
         ops.rmsnorm_forward(ln[:N], rstd[:N], x[:N], p["ln1w"][0], eps)
-        # a long prompt from position 0 is the training forward pass: its attention kernel (tensor cores, one pass over the
-        # keys per 128 queries) replaces the per-query scan of the cache, and the rotary kernel writes keys / values to the cache too
-        dense = pos is None and start_pos == 0 and Tq >= self.dense_prefill_from
-        if dense:
-            if self._dense is None or self._dense[0].shape[0] < N or self._dense[1].numel() < B * NH * Tq:
-                self._dense = (torch.zeros(rows, 3 * C, dtype=m.dtype, device=m.device),
-                               torch.zeros(B * NH * Tq, dtype=torch.float32, device=m.device))
-            packed, lse = self._dense[0][:N], self._dense[1][:B * NH * Tq].view(B, NH, Tq)
         for l in range(L):
             mm(a["raw"], ln, p["qkvw"][l], N)
             if dense:

@@ -114,15 +114,30 @@ def _wide(M, N, device):
 def _swapped(M, N, K, device):
     """Whether a plain forward product goes to the two-SM kernel with swapped operand roles (csrc/gemm2t.cu), whose row tiles fit the rows: as long as
     the tiles fill few rounds of the CTA pairs and K is deep enough to hide its epilogue in pieces of 16 rows.  Same bits as the other two kernels.
-    us, theirs in brackets: 777 x 3072 x 2048 12.7 (18.5), 777 x 14336 x 2048 40 (49), 500 x 6144 x 4096 23 (30), 3072 x 2048 x 2048 21.5 (26.6),
-    8192 x 2048 x 2048 60 (63), 256 x 2304 x 768 6.5 (6.8), 256 x 50304 x 768 25.5 (28.0); 512 x 1152 x 384 5.5 (5.1), 3001 x 28672 x 4096 522 (491).
+    us, theirs in brackets: 777 x 3072 x 2048 12.7 (18.5), 777 x 14336 x 2048 40 (49), 500 x 6144 x 4096 23 (30),
+    256 x 2304 x 768 6.5 (6.8), 256 x 50304 x 768 25.5 (28.0); 512 x 1152 x 384 5.5 (5.1), 3001 x 28672 x 4096 522 (491).  Above 2048 rows, where a chain
+    of products runs at the power limit, the larger loads count: the MLP of 3001 rows of 4096 channels takes 2683 instead of 2663 us with its
+    down-projection here, although that alone is faster (267 against 294).
     Deep products with few tiles are left to the split-K kernel: 300 x 2048 x 7168 33 against 20, 300 x 4096 x 14336 51 against 47, but
     500 x 4096 x 14336 57 against 60 and 777 x 2048 x 7168 29 against 32."""
     mt = (M + 255) // 256
-    if not (128 < M <= 8192 and K >= 768 and K % 8 == 0 and mt * ((N + 255) // 256) <= 5 * sm_count(device)):
+    if not (128 < M <= 2048 and K >= 768 and K % 8 == 0 and mt * ((N + 255) // 256) <= 5 * sm_count(device)):
         return False
     split = mt * ((N + 127) // 128)
     return K < 6144 or split > 64 or (split > 32 and M > 384)
+
+
+FORWARD_GEMM, FORWARD_GEMM2, FORWARD_STREAM, FORWARD_SWAPPED = range(4)        # csrc/decoder.cu, Product
+
+
+def forward_kernel(M, N, K, device):
+    """The kernel of a plain forward product without flags to wait for."""
+    if TWO_SM_MIN_TILES > 0 and _swapped(M, N, K, device):
+        return FORWARD_SWAPPED
+    if _few_rows(M, N, K, MODE_STORE, False, device) or _wide(M, N, device):
+        return FORWARD_STREAM
+    tiles256 = ((M + 255) // 256) * ((N + 255) // 256)
+    return FORWARD_GEMM2 if TWO_SM_MIN_TILES > 0 and tiles256 >= TWO_SM_MIN_TILES else FORWARD_GEMM
 
 
 def gemm(a, b, d, M, N, K, lda, ldb, ldd, a_mn, b_mn, mode, bias=None, aux=None, accumulate=False, splits=1, max_ctas=0, ready=None):
@@ -133,11 +148,11 @@ def gemm(a, b, d, M, N, K, lda, ldb, ldd, a_mn, b_mn, mode, bias=None, aux=None,
     global _launches
     lib = _lib.cuda()
     _launches += 1
-    plain_forward = mode == MODE_STORE and not a_mn and not b_mn
-    if plain_forward and ready is None and TWO_SM_MIN_TILES > 0 and _swapped(M, N, K, d.device):
+    plain = forward_kernel(M, N, K, d.device) if mode == MODE_STORE and not a_mn and not b_mn else None
+    if plain == FORWARD_SWAPPED and ready is None:
         check(lib.llmc_gemm2t(_p(d), _p(a), _p(b), _p(bias), M, N, K, lda, ldb, ldd, 0, _stream()), "llmc_gemm2t")
         return
-    if not a_mn and (_few_rows(M, N, K, mode, b_mn, d.device) or (plain_forward and _wide(M, N, d.device))):
+    if plain == FORWARD_STREAM or (not a_mn and _few_rows(M, N, K, mode, b_mn, d.device)):
         if ready is not None:
             ready.wait()
         check(lib.llmc_stream_gemm(_p(d), _p(a), _p(b), _p(bias), M, N, K, lda, ldb, ldd, int(b_mn), _stream()), "llmc_stream_gemm")
@@ -488,6 +503,37 @@ def matmul_swiglu_prompt(h, inp, weight12):
     _launches += 1
     check(_lib.cuda().llmc_gemm2t_swiglu(_p(h), _p(inp), _p(weight12), M, H, C, inp.stride(0), weight12.stride(0), h.stride(0), 0, _stream()),
           "llmc_gemm2t_swiglu")
+
+
+def decoder_forward(decoder, bufs, dense, tokens, start_pos, pos):
+    """The launches of ``models.generate.CachedDecoder.forward`` for a bf16 model, from native code (csrc/decoder.cu).  ``bufs``: the decoder's activation
+    buffers; ``dense``: (packed QKV, LSE) buffers for a prompt from position 0, or None."""
+    m = decoder.model
+    cfg, p, dev = m.cfg, m.params, m.device
+    B, Tq = tokens.shape
+    N, C, H, NH, NKV, HS = B * Tq, cfg.channels, cfg.hidden_dim, cfg.num_heads, cfg.num_kv_heads, cfg.head_size
+    cache_len, heads = decoder.kcache.shape[2], NH + 2 * NKV
+    logit_cols = p["lmhead"].shape[0]
+    if N <= 128 and H % 64 == 0:
+        mlp = 1
+    else:
+        mlp = 2 if N > 128 and H % 128 == 0 else 0
+    lib = _lib.cuda()
+    words = 0 if dense else lib.llmc_cached_attention_workspace(B, Tq, cache_len, NH, NKV, HS)
+    ws = _scratch.get("cached_attention", words, torch.float32, dev) if words > 0 else None
+    a = lambda t: None if t is None else t.data_ptr()
+    call = _lib.DecoderCall(
+        **{n: p[n].data_ptr() for n in ("wte", "ln1w", "qkvw", "attprojw", "ln2w", "fc12w", "fcprojw", "lnfw", "lmhead")},
+        **{n: bufs[n].data_ptr() for n in ("x", "ln", "raw", "q", "atty", "proj", "res", "fc12", "h", "last", "logits", "rstd")},
+        freqs=m.freqs.data_ptr(), kcache=decoder.kcache.data_ptr(), vcache=decoder.vcache.data_ptr(), packed=a(dense and dense[0]), lse=a(dense and dense[1]),
+        attention_ws=a(ws), tokens=tokens.data_ptr(), pos=a(pos),
+        L=cfg.num_layers, C=C, H=H, NH=NH, NKV=NKV, HS=HS, vocab_rows=p["wte"].shape[0], logit_cols=logit_cols, freqs_len=m.freqs.shape[0],
+        max_batch=decoder.kcache.shape[1], cache_len=cache_len, B=B, Tq=Tq, start=0 if pos is not None else start_pos,
+        how_qkv=forward_kernel(N, heads * HS, C, dev), how_attproj=forward_kernel(N, C, C, dev), how_fc12=forward_kernel(N, 2 * H, C, dev),
+        how_fcproj=forward_kernel(N, C, H, dev), how_head=forward_kernel(B, logit_cols, C, dev), mlp=mlp, eps=cfg.norm_eps)
+    launches = ctypes.c_int(0)
+    check(lib.llmc_decoder_forward(ctypes.byref(call), ctypes.byref(launches), _stream()), "llmc_decoder_forward")
+    count_launches(launches.value)
 
 
 def make_table(views):

@@ -42,7 +42,7 @@ def test_swiglu(rows, M, H, K):
     assert (out[M:] == 7.0).all() and _lib.read_status() == 0
 
 
-@pytest.mark.parametrize("M,K,N", [(300, 1024, 264), (777, 2048, 520), (4000, 1032, 136)])
+@pytest.mark.parametrize("M,K,N", [(300, 1024, 264), (777, 2048, 520), (2000, 1032, 136)])
 def test_forward_products_take_it(M, K, N):
     """The launcher sends them there with the caller's own tensors: out may have more rows, the bias is added."""
     x, w, b = rnd(M, K), rnd(N, K, scale=0.05, seed=1), rnd(N, seed=2)
