@@ -15,19 +15,30 @@
 // traffic and all of the P stores.
 //
 // A work item is (batch, head, g) with the two key tiles {g, nt-1-g}: nt + 1 pairs whatever g, so a static round-robin over
-// the persistent CTAs is balanced.  dK_j / dV_j leave the CTA once per key tile.  The contribution of pair (j, i) to dQ_i is
-// written as fp32 to its own slot of a workspace; a second kernel adds the slots of a query tile in the order j = 0..i and
-// rounds once.  No atomics, no ordering between CTAs: the gradients are bit-reproducible, which the reference also demands of
-// cuDNN (llmc/cudnn_att.cpp:186-191), and no CTA ever waits for another one.
+// the persistent CTAs is balanced.  dK_j / dV_j leave the CTA once per key tile.  What item g contributes to dQ_i is written as
+// fp32 to a slot of its own in a workspace (the second key tile is added to what the first left there by a reducing bulk copy
+// of the same CTA, ordered after the first); a second kernel adds the slots of a query tile in the order of g and rounds once.
+// No atomics, no ordering between CTAs: the gradients are bit-reproducible, which the reference also demands of cuDNN
+// (llmc/cudnn_att.cpp:186-191), and no CTA ever waits for another one.
+//
+// What bounds it: the chain S^T -> exponentials -> dP^T -> dS^T -> dK, dQ of one pair, about 2900 cycles, of which the tensor
+// pipe works 1450; three things keep the chain short.  S^T(t+1) is issued before dV(t), so that its 64 columns are there when a
+// softmax warp returns for them; the two warps of a scheduler take turns at the exponentials, so that one of them loads, packs
+// and stores while the other has the unit to itself; and accumulators are read into registers and handed back before the
+// staging buffer is waited for.  64 x 1024 x 12 heads: 632 us before, 603 with those, 556 with one slot per item instead of
+// one per pair (a quarter less workspace to write and to add; tiles of one sequence alone need no second kernel).
+// Fetching K_j / V_j of later key tiles into L2 ahead of their loads was slower (566): the loads of 148 CTAs that change
+// their head together wait for memory bandwidth, not for latency.
 //
 // Roles inside a CTA (512 threads):
 //   warp 0       TMA producer: K_j, V_j resident (double buffered across key tiles); Q_i, dO_i through a 3-stage ring.
-//   warp 1       issuer of all five products, in the order dV(t), S^T(t+1), dK(t), dQ(t), dP^T(t+1): program order is what
+//   warp 1       issuer of all five products, in the order S^T(t+1), dV(t), dK(t), dQ(t), dP^T(t+1): program order is what
 //                keeps dP^T of the next pair from overwriting the bf16 dS^T operand that aliases its TMEM columns.
+//   warps 2-3    producers of the per-query statistics table.
 //   warps 4-11   softmax: thread = key row x 64-query half.  Nothing is exchanged between threads (the row statistics of the
 //                forward pass are per query = per column, read from a small shared table).
 //   warps 12-15  drain: the pair's dQ contribution from TMEM to the workspace, and at the end of a key tile dV_j / dK_j to
-//                global memory through a staging buffer and TMA stores; also producers of the per-query statistics table.
+//                global memory through a staging buffer and TMA stores.
 //
 // TMEM columns: S^T [0,128)  dP^T [128,256) (dS^T bf16 aliases the first 32 columns of each 64-column half)
 //               dV [256,320)  dK [320,384)  dQ [384,448)  P^T bf16 [448,512).
@@ -55,14 +66,17 @@ constexpr int THREADS = 512;
 constexpr int TMEM_COLS = 512;
 constexpr int STAT_BYTES = 2 * 2 * BT * 4;          // [2 buffers][lse, delta][128 queries]
 constexpr int SMEM = RB * PAIR_BYTES + XSTAGES * PAIR_BYTES + DS_BYTES + PAIR_BYTES + STAT_BYTES + 256;
+constexpr int TURN_BAR = 3;                         // named barriers 3..10: [scheduler][query half] turns at the exponentials
 constexpr int SLOT_FLOATS = BT * HS;                // one dQ contribution
 static_assert(SMEM <= 232448, "shared memory of one CTA");
 
 struct Args {
     bf16* dqkv;          // (B, T, 3, NH, 64)
-    float* dq_ws;        // [B*NH][nt*(nt+1)/2][16 column groups][128 rows][4] fp32: slot of pair (j, i) = i*(i+1)/2 + j
+    float* dq_ws;        // [B*NH][slots][16 column groups][128 rows][4] fp32: slot_of(i) + g holds what unit g adds to query tile i
     const float* lse;    // (B, NH, T)
-    const float* delta;  // (B, NH, T)
+    const float* delta;  // (B, NH, T); null (one tile per sequence): computed here from out and dout
+    const bf16* out;     // (B, T, NH, 64)
+    const bf16* dout;
     int B, T, NH;
     float scale, scale_log2e;
     unsigned int* status;
@@ -84,6 +98,9 @@ DEVINL void tmem_st8(uint32_t taddr, const uint32_t* r) {
         "tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
         ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]) : "memory");
 }
+
+// Slots of the query tiles before i: tile k has one per unit g <= min(k, G - 1) that reaches it.
+__host__ __device__ inline int slot_of(int i, int G) { return i <= G ? i * (i + 1) / 2 : G * (G + 1) / 2 + (i - G) * G; }
 
 // The sequence of pairs of one CTA: items w (round-robin), their one or two key tiles, the query tiles i >= j of each.
 struct Walk {
@@ -131,7 +148,7 @@ attn_bwd1_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constan
     uint64_t* dq_empty = bars + 18;   // the drain warps hold dQ(t) in registers     (4 arrivals)
     uint64_t* acc_full = bars + 19;   // dV_j, dK_j complete                         (1 commit)
     uint64_t* acc_empty = bars + 20;  // the drain warps hold them                   (4 arrivals)
-    uint64_t* st_full = bars + 21;    // [2] statistics table of a pair written      (4 arrivals)
+    uint64_t* st_full = bars + 21;    // [2] statistics table of a pair written      (2 arrivals)
     uint64_t* st_empty = bars + 23;   // [2] ... and read by every softmax warp      (8 arrivals)
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 25);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
@@ -140,11 +157,11 @@ attn_bwd1_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constan
     const int nt = CEIL_DIV(a.T, BT);
     const int G = (nt + 1) >> 1;                      // key-tile groups {g, nt-1-g}
     const int total = a.B * a.NH * G;
-    const int npairs = nt * (nt + 1) / 2;
+    const int nslots = slot_of(nt, G);
 
     if (threadIdx.x == 0) {
         if ((smem_u32(smem) & 1023u) != 0) record_error(a.status, ST_BAD_ARG, 0x28);
-        for (int i = 0; i < 2; i++) { mbar_init(&res_full[i], 1); mbar_init(&res_empty[i], 1); mbar_init(&st_full[i], 4); mbar_init(&st_empty[i], 8); }
+        for (int i = 0; i < 2; i++) { mbar_init(&res_full[i], 1); mbar_init(&res_empty[i], 1); mbar_init(&st_full[i], 2); mbar_init(&st_empty[i], 8); }
         for (int i = 0; i < XSTAGES; i++) { mbar_init(&x_full[i], 1); mbar_init(&x_empty[i], 1); }
         mbar_init(s_full, 1); mbar_init(s_empty, 8); mbar_init(dp_full, 1); mbar_init(p_ready, 8); mbar_init(p_empty, 1);
         mbar_init(ds_ready, 8); mbar_init(ds_empty, 1); mbar_init(dq_full, 1); mbar_init(dq_empty, 4);
@@ -245,8 +262,17 @@ attn_bwd1_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constan
                 const int nkvt = have_next && nx.first_of_tile() ? kvt + 1 : kvt;
                 const int nrb = nkvt & 1;
                 const uint32_t acc = wk.first_of_tile() ? 0u : 1u;
-                // ---- dV(t) += P^T dO_i : A = P^T in TMEM (16 queries = 8 columns per step), B = dO_i N-major (16 rows = 2048 bytes)
+                // ---- S^T(t+1), as soon as the second half's warps hold S^T(t): the first half's are through with pair t by then
                 if (leader) TRACE(0, 0);
+                if (have_next) {
+                    if (nx.first_of_tile()) ok = WAIT_ALL(&res_full[nrb], (nkvt >> 1) & 1, 0x694);
+                    ok = ok && WAIT_ALL(&x_full[nst], nph, 0x695);
+                    ok = ok && WAIT_ALL(s_empty, t & 1, 0x696);
+                    if (!ok) break;
+                    tc_fence_after();
+                    issue_s(nrb, nst);
+                }
+                // ---- dV(t) += P^T dO_i : A = P^T in TMEM (16 queries = 8 columns per step), B = dO_i N-major (16 rows = 2048 bytes)
                 ok = WAIT_ALL(p_ready, t & 1, 0x692);
                 if (ok && wk.first_of_tile() && kvt > 0) ok = WAIT_ALL(acc_empty, (kvt - 1) & 1, 0x693);
                 if (!ok) break;
@@ -259,15 +285,6 @@ attn_bwd1_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constan
                         for (int kk = 0; kk < BT / 16; kk++) umma_ts(tdV, tP + kk * 8, ob + 128 * kk, idesc_ts, acc | (kk > 0));
                         umma_commit(p_empty);
                     }
-                }
-                // ---- S^T(t+1): its TMEM tile was read into registers before P^T(t) could be written
-                if (have_next) {
-                    if (nx.first_of_tile()) ok = WAIT_ALL(&res_full[nrb], (nkvt >> 1) & 1, 0x694);
-                    ok = ok && WAIT_ALL(&x_full[nst], nph, 0x695);
-                    ok = ok && WAIT_ALL(s_empty, t & 1, 0x696);
-                    if (!ok) break;
-                    tc_fence_after();
-                    issue_s(nrb, nst);
                 }
                 if (leader) TRACE(0, 2);
                 // ---- dK(t) += dS^T Q_i (A = dS^T in TMEM: queries 0..63 in columns [0,32) of the dP^T tile, 64..127 in [64,96));
@@ -283,12 +300,13 @@ attn_bwd1_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constan
                         #pragma unroll
                         for (int kk = 0; kk < BT / 16; kk++)
                             umma_ts(tdK, tdP + (kk >> 2) * 64 + (kk & 3) * 8, qb + 128 * kk, idesc_ts, acc | (kk > 0));
+                        if (wk.last_of_tile()) umma_commit(acc_full);
                         #pragma unroll
                         for (int kk = 0; kk < BT / 16; kk++) umma_ss(tdQ, dSm + 128 * kk, kb + 128 * kk, idesc_q, kk > 0);
                         umma_commit(dq_full);
                         umma_commit(ds_empty);
                         umma_commit(&x_empty[st]);
-                        if (wk.last_of_tile()) { umma_commit(acc_full); umma_commit(&res_empty[rb]); }
+                        if (wk.last_of_tile()) umma_commit(&res_empty[rb]);
                     }
                 }
                 // ---- dP^T(t+1): after dK(t) in program order, so it cannot overwrite dS^T(t) early
@@ -299,67 +317,108 @@ attn_bwd1_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constan
             }
 #undef WAIT_ALL
         }
-    } else if (warp >= 4 && warp < 12) {
+    } else if (warp < 4) {
+        // ---------------------------------------------------------------- statistics of a pair's 128 queries -> table (t & 1), 64 by each of the
+        // two warps: the LSE in log2 units and delta = sum_d O dO times the scale; queries past the end of the sequence get LSE = +inf, so
+        // that their P^T column is zero
+        const float log2e = 1.4426950408889634f;
+        const int w0 = (warp - 2) * 64;                 // the warp's queries of the tile
+        bool ok = true;
+        uint32_t t = 0;
+        for (; wk.valid() && ok; wk.next(), t++) {
+            const int tq0 = wk.i * BT + w0;
+            float l[2], d[16];
+            const size_t row = (size_t)wk.bh * a.T + tq0 + lane;
+            #pragma unroll
+            for (int k = 0; k < 2; k++) l[k] = tq0 + k * 32 + lane < a.T ? a.lse[row + k * 32] * log2e : INFINITY;
+            if (a.delta != nullptr) {
+                #pragma unroll
+                for (int k = 0; k < 2; k++) d[k] = tq0 + k * 32 + lane < a.T ? a.delta[row + k * 32] * a.scale : 0.f;
+            } else {
+                // 8 lanes per query, 4 queries per step; no branch around the loads, so that they are on their way at once
+                #pragma unroll
+                for (int part = 0; part < 4; part++) {
+                    bf16x8 o[4], g[4];
+                    #pragma unroll
+                    for (int k = 0; k < 4; k++) {
+                        const int tq = min(tq0 + part * 16 + k * 4 + (lane >> 3), a.T - 1);
+                        const size_t at = (((size_t)wk.b * a.T + tq) * a.NH + wk.h) * HS + (lane & 7) * 8;
+                        o[k] = ld128cs(a.out + at); g[k] = ld128(a.dout + at);
+                    }
+                    #pragma unroll
+                    for (int k = 0; k < 4; k++) {
+                        float acc = 0.f;
+                        #pragma unroll
+                        for (int e = 0; e < 8; e++) acc += __bfloat162float(o[k][e]) * __bfloat162float(g[k][e]);
+                        acc += __shfl_xor_sync(0xffffffffu, acc, 1);
+                        acc += __shfl_xor_sync(0xffffffffu, acc, 2);
+                        acc += __shfl_xor_sync(0xffffffffu, acc, 4);
+                        d[part * 4 + k] = tq0 + part * 16 + k * 4 + (lane >> 3) < a.T ? acc * a.scale : 0.f;
+                    }
+                }
+            }
+            ok = __all_sync(0xffffffffu, mbar_wait_relaxed(&st_empty[t & 1], ((t >> 1) & 1) ^ 1, abort_flag, a.status, 0x6b0)) != 0;
+            float* tab = sStat + (t & 1) * (2 * BT) + w0;
+            tab[lane] = l[0]; tab[32 + lane] = l[1];
+            if (a.delta != nullptr) {
+                tab[BT + lane] = d[0]; tab[BT + 32 + lane] = d[1];
+            } else if ((lane & 7) == 0) {
+                #pragma unroll
+                for (int k = 0; k < 16; k++) tab[BT + k * 4 + (lane >> 3)] = d[k];
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&st_full[t & 1]);
+        }
+    } else if (warp < 12) {
         // ---------------------------------------------------------------- softmax: thread = key row r x query half hf
         const int q = warp & 3;                        // TMEM lane quarter
         const int hf = (warp - 4) >> 2;                // query half
         const int r = q * 32 + lane;                   // key row of the tile
         const uint32_t lane_off = (uint32_t)(q * 32) << 16;
         bool ok = true;
+        if (hf == 1) turn_pass(TURN_BAR + 2 * q);      // the first half has the first turn
         uint32_t t = 0;
         for (; wk.valid(); wk.next(), t++) {
             const int i = wk.i, j = wk.j;
-            const bool row_ok = j * BT + r < a.T;
             const float* stat = sStat + (t & 1) * (2 * BT) + hf * 64;       // lse * log2(e) of this half's queries; delta * scale 128 floats further
             if (threadIdx.x == 128) TRACE(1, 0);
             ok = mbar_wait(s_full, t & 1, abort_flag, a.status, 0x6a0) && ok;
             tc_fence_after();
             if (threadIdx.x == 128) TRACE(1, 1);
             ok = mbar_wait(&st_full[t & 1], (t >> 1) & 1, abort_flag, a.status, 0x6a1) && ok;
-            if (t > 0) ok = mbar_wait(p_empty, (t - 1) & 1, abort_flag, a.status, 0x6a2) && ok;      // dV(t-1) has read P^T(t-1)
-            if (threadIdx.x == 128) TRACE(1, 7);
-            // ---- P^T = exp2(S^T * scale * log2(e) - LSE * log2(e)); causal: query >= key.  Two passes of 32 queries: with all 64
-            //      scores in registers next to the 64 results the register file is so full that the compiler reuses registers
-            //      across the exponentials, and every one then waits for its predecessor (measured: 34 cycles per element).
+            // ---- P^T = exp2(S^T * scale * log2(e) - LSE * log2(e)); causal: query >= key
             float p[64];
             // only the diagonal tile and a ragged last key tile need masks; both conditions are the same for the whole warp
             const bool masked = (i == j) || (j * BT + BT > a.T);
-            #pragma unroll
-            for (int h2 = 0; h2 < 2; h2++) {
-                uint32_t sv[32];
-                tmem_ld32(tS + lane_off + hf * 64 + h2 * 32, sv);
+            {
+                uint32_t sv[64];
+                tmem_ld32(tS + lane_off + hf * 64, sv);
+                tmem_ld32(tS + lane_off + hf * 64 + 32, sv + 32);
                 tmem_ld_wait();
-                if (h2 == 1) {
-                    tc_fence_before();
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(s_empty);
-                    if (threadIdx.x == 128) TRACE(1, 6);
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(s_empty);
+                float sl = a.scale_log2e;
+                turn_wait(TURN_BAR + 2 * q + hf, sl);
+                if (threadIdx.x == 128) TRACE(1, 6);
+                const uint64_t sl2 = f2_pack(sl, sl);
+                #pragma unroll
+                for (int e = 0; e < 64; e += 4) {
+                    const float4 l4 = *reinterpret_cast<const float4*>(stat + e);
+                    const float2 x0 = f2_unpack(f2_fma(f2_pack_u(sv[e], sv[e + 1]), sl2, f2_pack(-l4.x, -l4.y)));
+                    const float2 x1 = f2_unpack(f2_fma(f2_pack_u(sv[e + 2], sv[e + 3]), sl2, f2_pack(-l4.z, -l4.w)));
+                    p[e] = ex2_fast(x0.x); p[e + 1] = ex2_fast(x0.y); p[e + 2] = ex2_fast(x1.x); p[e + 3] = ex2_fast(x1.y);
                 }
-                if (!masked) {
-                    #pragma unroll
-                    for (int e4 = 0; e4 < 8; e4++) {
-                        const float4 l4 = *reinterpret_cast<const float4*>(stat + h2 * 32 + e4 * 4);
-                        p[h2 * 32 + e4 * 4 + 0] = ex2_fast(fmaf(__uint_as_float(sv[e4 * 4 + 0]), a.scale_log2e, -l4.x));
-                        p[h2 * 32 + e4 * 4 + 1] = ex2_fast(fmaf(__uint_as_float(sv[e4 * 4 + 1]), a.scale_log2e, -l4.y));
-                        p[h2 * 32 + e4 * 4 + 2] = ex2_fast(fmaf(__uint_as_float(sv[e4 * 4 + 2]), a.scale_log2e, -l4.z));
-                        p[h2 * 32 + e4 * 4 + 3] = ex2_fast(fmaf(__uint_as_float(sv[e4 * 4 + 3]), a.scale_log2e, -l4.w));
-                    }
-                } else {
-                    const bool diag = (i == j);
-                    #pragma unroll
-                    for (int e4 = 0; e4 < 8; e4++) {
-                        const float4 l4 = *reinterpret_cast<const float4*>(stat + h2 * 32 + e4 * 4);
-                        const float lv[4] = {l4.x, l4.y, l4.z, l4.w};
-                        #pragma unroll
-                        for (int k = 0; k < 4; k++) {
-                            const int e = h2 * 32 + e4 * 4 + k;
-                            float v = ex2_fast(fmaf(__uint_as_float(sv[e4 * 4 + k]), a.scale_log2e, -lv[k]));
-                            if (diag && hf * 64 + e < r) v = 0.f;
-                            p[e] = row_ok ? v : 0.f;
-                        }
-                    }
-                }
+                turn_pass(TURN_BAR + 2 * q + (hf ^ 1), p[63]);
             }
+            if (masked) {
+                const int lo = j * BT + r >= a.T ? 64 : (i == j ? r - hf * 64 : 0);      // first query of this half that counts for this key
+                #pragma unroll
+                for (int e = 0; e < 64; e++) p[e] = e < lo ? 0.f : p[e];
+            }
+            if (t > 0) ok = mbar_wait(p_empty, (t - 1) & 1, abort_flag, a.status, 0x6a2) && ok;      // dV(t-1) has read P^T(t-1)
+            tc_fence_after();
+            if (threadIdx.x == 128) TRACE(1, 7);
             {
                 uint32_t pk[32];
                 #pragma unroll
@@ -380,21 +439,20 @@ attn_bwd1_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constan
             tc_fence_after();
             if (threadIdx.x == 128) TRACE(1, 4);
             uint8_t* drow = sdS + hf * (BT * 128) + r * 128;
+            const uint64_t sc2 = f2_pack(a.scale, a.scale);
+            uint32_t dv[2][16];
+            tmem_ld16(tdP + lane_off + hf * 64, dv[0]);
             #pragma unroll
             for (int c = 0; c < 4; c++) {
-                uint32_t dv[16];
-                tmem_ld16(tdP + lane_off + hf * 64 + c * 16, dv);
                 tmem_ld_wait();
+                if (c < 3) tmem_ld16(tdP + lane_off + hf * 64 + (c + 1) * 16, dv[(c + 1) & 1]);
+                const uint32_t* dc = dv[c & 1];
                 uint32_t dd[8];
                 #pragma unroll
-                for (int e4 = 0; e4 < 4; e4++) {
-                    const float4 d4 = *reinterpret_cast<const float4*>(stat + BT + c * 16 + e4 * 4);
-                    const float dl[4] = {d4.x, d4.y, d4.z, d4.w};
-                    float ds[4];
-                    #pragma unroll
-                    for (int k = 0; k < 4; k++) ds[k] = p[c * 16 + e4 * 4 + k] * fmaf(__uint_as_float(dv[e4 * 4 + k]), a.scale, -dl[k]);
-                    dd[e4 * 2] = pack_bf16x2(ds[0], ds[1]);
-                    dd[e4 * 2 + 1] = pack_bf16x2(ds[2], ds[3]);
+                for (int e = 0; e < 16; e += 4) {
+                    const float4 d4 = *reinterpret_cast<const float4*>(stat + BT + c * 16 + e);
+                    dd[e / 2] = pack_bf16x2(f2_mul(f2_pack(p[c * 16 + e], p[c * 16 + e + 1]), f2_fma(f2_pack_u(dc[e], dc[e + 1]), sc2, f2_pack(-d4.x, -d4.y))));
+                    dd[e / 2 + 1] = pack_bf16x2(f2_mul(f2_pack(p[c * 16 + e + 2], p[c * 16 + e + 3]), f2_fma(f2_pack_u(dc[e + 2], dc[e + 3]), sc2, f2_pack(-d4.z, -d4.w))));
                 }
                 tmem_st8(tdP + lane_off + hf * 64 + c * 8, dd);
                 // 16 queries = 32 bytes = two 16-byte units 2c, 2c+1 of this row, 128-byte swizzle
@@ -408,59 +466,72 @@ attn_bwd1_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constan
             if (lane == 0) { mbar_arrive(ds_ready); mbar_arrive(&st_empty[t & 1]); }
             if (threadIdx.x == 128) TRACE(1, 5);
         }
-    } else if (warp >= 12) {
+        if (hf == 0) turn_wait(TURN_BAR + 2 * q);      // the last turn passed on by the second half
+    } else {
         // ---------------------------------------------------------------- drain warps (128 threads): thread = row rr of a tile
         const int q = warp & 3;
         const int rr = q * 32 + lane;
         const uint32_t lane_off = (uint32_t)(q * 32) << 16;
-        const float log2e = 1.4426950408889634f;
         const bool issuer = warp == 12 && lane == 0;
         bool ok = true;
         bool staged = false;
         uint32_t t = 0;
         int kvt = 0;
-        // statistics of query rr of a pair's query tile -> table (tt & 1): LSE in log2 units, delta pre-multiplied by the scale;
-        // queries past the end of the sequence get LSE = +inf, so that their P^T column is zero
-        auto put_stats = [&](const Walk& pr, uint32_t tt) {
-            const int tq = pr.i * BT + rr;
-            float l = INFINITY, d = 0.f;
-            if (tq < a.T) { l = a.lse[(size_t)pr.bh * a.T + tq] * log2e; d = a.delta[(size_t)pr.bh * a.T + tq] * a.scale; }
-            ok = mbar_wait_relaxed(&st_empty[tt & 1], ((tt >> 1) & 1) ^ 1, abort_flag, a.status, 0x6b0) && ok;
-            float* tab = sStat + (tt & 1) * (2 * BT);
-            tab[rr] = l; tab[BT + rr] = d;
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&st_full[tt & 1]);
-        };
-        if (wk.valid()) put_stats(wk, 0);
         for (; wk.valid(); t++) {
             const int bh = wk.bh, b = wk.b, h = wk.h, i = wk.i, j = wk.j;
             const bool last = wk.last_of_tile();
+            const int g = wk.g, seg = wk.seg;
             wk.next();
-            if (wk.valid()) put_stats(wk, t + 1);        // the next pair's table, one pair ahead
-            // ---- the pair's dQ contribution: 64 fp32 of query row rr, slot order [group of 4 columns][row][4 floats],
+            // ---- the pair's dQ contribution: 64 fp32 of query row rr, slot order [group of 4 columns][row][4 floats].  The second key tile of a unit
+            //      is added to what the first left in the slot, nt - j pairs ago, by a copy that reduces in L2.  (All contributions of a head summed
+            //      that way, without the fold kernel, took longer: reductions of 32 KB per pair and SM run at 1.4 TB/s.)
             if (threadIdx.x == 384) TRACE(2, 0);
             ok = mbar_wait_relaxed(dq_full, t & 1, abort_flag, a.status, 0x6b1) && ok;
             tc_fence_after();
             if (threadIdx.x == 384) TRACE(2, 1);
             // through the staging buffer and one bulk copy: 16 global stores per thread and pair through the load/store unit held up
             // the shared-memory reads of the softmax warps for about a thousand cycles per pair (measured)
-            float* slot = a.dq_ws + ((size_t)bh * npairs + (size_t)(i * (i + 1) / 2 + j)) * SLOT_FLOATS;
-            if (staged) { if (issuer) tma_store_wait_read<0>(); asm volatile("bar.sync 1, 128;" ::: "memory"); }      // the previous copy has read the buffer
-            #pragma unroll
-            for (int c = 0; c < 2; c++) {
-                uint32_t v[32];
-                tmem_ld32(tdQ + lane_off + c * 32, v);
+            float* slot = a.dq_ws + ((size_t)bh * nslots + slot_of(i, G) + g) * SLOT_FLOATS;
+            if (seg == 1 && issuer) {
+                if (nt - j == 1) tma_store_wait<0>(); else if (nt - j == 2) tma_store_wait<1>(); else tma_store_wait<2>();
+            }
+            {
+                uint32_t v[64];
+                tmem_ld32(tdQ + lane_off, v);
+                tmem_ld32(tdQ + lane_off + 32, v + 32);
                 tmem_ld_wait();
-                if (c == 1) { tc_fence_before(); __syncwarp(); if (lane == 0) mbar_arrive(dq_empty); }
-                #pragma unroll
-                for (int e = 0; e < 8; e++)
-                    *reinterpret_cast<uint4*>(sOut + (c * 8 + e) * (BT * 16) + rr * 16) = make_uint4(v[4 * e], v[4 * e + 1], v[4 * e + 2], v[4 * e + 3]);
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(dq_empty);
+                if (staged) { if (issuer) tma_store_wait_read<0>(); asm volatile("bar.sync 1, 128;" ::: "memory"); }      // the previous copy has read the buffer
+                if (nt > 1) {
+                    #pragma unroll
+                    for (int e = 0; e < 16; e++)
+                        *reinterpret_cast<uint4*>(sOut + e * (BT * 16) + rr * 16) = make_uint4(v[4 * e], v[4 * e + 1], v[4 * e + 2], v[4 * e + 3]);
+                } else {
+                    // a single tile: dQ is finished
+                    #pragma unroll
+                    for (int u = 0; u < 8; u++) {
+                        uint4 o;
+                        o.x = pack_bf16x2(__uint_as_float(v[8 * u]), __uint_as_float(v[8 * u + 1]));
+                        o.y = pack_bf16x2(__uint_as_float(v[8 * u + 2]), __uint_as_float(v[8 * u + 3]));
+                        o.z = pack_bf16x2(__uint_as_float(v[8 * u + 4]), __uint_as_float(v[8 * u + 5]));
+                        o.w = pack_bf16x2(__uint_as_float(v[8 * u + 6]), __uint_as_float(v[8 * u + 7]));
+                        *reinterpret_cast<uint4*>(sOut + rr * 128 + ((u ^ (rr & 7)) * 16)) = o;
+                    }
+                }
             }
             fence_async_smem();
             asm volatile("bar.sync 1, 128;" ::: "memory");
             if (issuer && ok) {
-                asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;"
-                             ::"l"(slot), "r"(smem_u32(sOut)), "r"(SLOT_FLOATS * 4) : "memory");
+                if (nt == 1)
+                    tma_store_4d(&tmDQKV, sOut, 0, h, i * BT, b);
+                else if (seg == 0)
+                    asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;"
+                                 ::"l"(slot), "r"(smem_u32(sOut)), "r"(SLOT_FLOATS * 4) : "memory");
+                else
+                    asm volatile("cp.reduce.async.bulk.global.shared::cta.bulk_group.add.f32 [%0], [%1], %2;"
+                                 ::"l"(slot), "r"(smem_u32(sOut)), "r"(SLOT_FLOATS * 4) : "memory");
                 tma_store_commit();
             }
             staged = true;
@@ -470,29 +541,23 @@ attn_bwd1_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constan
                 //      each (rows past T are clipped by TMA); a warp writing rows itself would touch 32 cache lines per instruction
                 ok = mbar_wait_relaxed(acc_full, kvt & 1, abort_flag, a.status, 0x6b2) && ok;
                 tc_fence_after();
-                if (staged) { if (issuer) tma_store_wait_read<0>(); asm volatile("bar.sync 1, 128;" ::: "memory"); }
+                // (first into registers: the next tile's products wait for the accumulators, not for the staging buffer)
+                uint32_t pk[64];
                 #pragma unroll
-                for (int which = 0; which < 2; which++) {
-                    uint8_t* orow = sOut + which * TILE_BYTES + rr * 128;
+                for (int c = 0; c < 4; c++) {
+                    uint32_t v[32];
+                    tmem_ld32((c < 2 ? tdV : tdK) + lane_off + (c & 1) * 32, v);
+                    tmem_ld_wait();
                     #pragma unroll
-                    for (int c = 0; c < 2; c++) {
-                        uint32_t v[32];
-                        tmem_ld32((which == 0 ? tdV : tdK) + lane_off + c * 32, v);
-                        tmem_ld_wait();
-                        #pragma unroll
-                        for (int u = 0; u < 4; u++) {
-                            uint4 o;
-                            o.x = pack_bf16x2(__uint_as_float(v[8 * u]), __uint_as_float(v[8 * u + 1]));
-                            o.y = pack_bf16x2(__uint_as_float(v[8 * u + 2]), __uint_as_float(v[8 * u + 3]));
-                            o.z = pack_bf16x2(__uint_as_float(v[8 * u + 4]), __uint_as_float(v[8 * u + 5]));
-                            o.w = pack_bf16x2(__uint_as_float(v[8 * u + 6]), __uint_as_float(v[8 * u + 7]));
-                            *reinterpret_cast<uint4*>(orow + (((c * 4 + u) ^ (rr & 7)) * 16)) = o;
-                        }
-                    }
+                    for (int e = 0; e < 16; e++) pk[c * 16 + e] = pack_bf16x2(__uint_as_float(v[2 * e]), __uint_as_float(v[2 * e + 1]));
                 }
                 tc_fence_before();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(acc_empty);
+                if (staged) { if (issuer) tma_store_wait_read<0>(); asm volatile("bar.sync 1, 128;" ::: "memory"); }
+                #pragma unroll
+                for (int u = 0; u < 16; u++)
+                    *reinterpret_cast<uint4*>(sOut + (u >> 3) * TILE_BYTES + rr * 128 + (((u & 7) ^ (rr & 7)) * 16)) = make_uint4(pk[4 * u], pk[4 * u + 1], pk[4 * u + 2], pk[4 * u + 3]);
                 fence_async_smem();
                 asm volatile("bar.sync 1, 128;" ::: "memory");
                 if (issuer && ok) {
@@ -518,7 +583,7 @@ attn_bwd1_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constan
     if (warp == 1) tmem_dealloc(tmem_base, TMEM_COLS);
 }
 
-// dQ[b, t, h, :] = bf16( sum over j = 0..i of slot(j, i)[r, :] ), i = t / 128, r = t % 128, added in the order of j.
+// dQ[b, t, h, :] = bf16( sum over the units g of slot(i, g)[r, :] ), i = t / 128, r = t % 128, added in the order of g.
 // One CTA per (batch, head, query tile), heaviest tiles first.  A slot is read as it was written (order [group of 4 columns][row]
 // [4 floats]): a warp reads 512 contiguous bytes per instruction, every thread has 16 loads of 16 bytes in flight (two slots);
 // the sums are transposed through shared memory so that the 8 lanes of a row store its 128 bytes together.
@@ -528,16 +593,16 @@ dq_fold_kernel(bf16* __restrict__ dqkv, const float* __restrict__ ws, int B, int
     const int nbh = B * NH;
     const int i = nt - 1 - (int)(blockIdx.x / nbh);
     const int bh = (int)(blockIdx.x % nbh);
-    const int npairs = nt * (nt + 1) / 2;
+    const int G = (nt + 1) >> 1, n = min(i, G - 1) + 1;
     const int t = threadIdx.x;
-    const float* src = ws + ((size_t)bh * npairs + (size_t)(i * (i + 1) / 2)) * SLOT_FLOATS + t * 4;
+    const float* src = ws + ((size_t)bh * slot_of(nt, G) + slot_of(i, G)) * SLOT_FLOATS + t * 4;
     f32x4 acc[8];
     #pragma unroll
     for (int k = 0; k < 8; k++)
         #pragma unroll
         for (int e = 0; e < 4; e++) acc[k][e] = 0.f;
-    for (int j = 0; j <= i; j += 2) {
-        const bool two = j + 1 <= i;
+    for (int j = 0; j < n; j += 2) {
+        const bool two = j + 1 < n;
         f32x4 a0[8], a1[8];
         #pragma unroll
         for (int k = 0; k < 8; k++) a0[k] = ld128cs(src + (size_t)j * SLOT_FLOATS + k * 1024);
@@ -591,7 +656,7 @@ extern "C" long long llmc_attention_bwd_workspace(int B, int T, int NH, int hs) 
     words = (words + 63) & ~63ll;
     if (hs == HS) {
         const long long nt = CEIL_DIV(T, BT);
-        words += (long long)B * NH * (nt * (nt + 1) / 2) * SLOT_FLOATS;
+        words += (long long)B * NH * slot_of((int)nt, (int)(nt + 1) / 2) * SLOT_FLOATS;
     }
     return words;
 }
@@ -613,14 +678,15 @@ extern "C" int llmc_attention_bwd(bf16* dqkv, float* ws, const bf16* dout, const
         if ((rc = llmc_get_tensormap(&tmDO, dout, 2, 4, dims, strides, box, 3))) return rc;
     }
     if ((rc = llmc_attn_qkv_map(&tmDQKV, dqkv, B, T, NH, hs))) return rc;
-    if ((rc = llmc_attention_delta(delta, out, dout, B, T, NH, hs, stream))) return rc;
+    const int nt = CEIL_DIV(T, BT);
+    // one tile per sequence: delta and the finished dQ come from the same launch (4 x 64 x 12 heads 19.5 -> 13.4 us)
+    if (nt > 1 && (rc = llmc_attention_delta(delta, out, dout, B, T, NH, hs, stream))) return rc;
     Args a;
-    a.dqkv = dqkv; a.dq_ws = dq_ws; a.lse = lse; a.delta = delta; a.B = B; a.T = T; a.NH = NH;
+    a.dqkv = dqkv; a.dq_ws = dq_ws; a.lse = lse; a.delta = nt > 1 ? delta : nullptr; a.out = out; a.dout = dout; a.B = B; a.T = T; a.NH = NH;
     a.scale = 1.0f / sqrtf((float)hs);
     a.scale_log2e = a.scale * 1.4426950408889634f;
     a.status = llmc_status_ptr();
     a.trace = g_trace;
-    const int nt = CEIL_DIV(T, BT);
     const int total = B * NH * ((nt + 1) / 2);
     int sms = llmc_device_sm_count(); if (sms <= 0) sms = 148;
     const int grid = total < sms ? total : sms;
@@ -631,7 +697,11 @@ extern "C" int llmc_attention_bwd(bf16* dqkv, float* ws, const bf16* dout, const
     }
     attn_bwd1_kernel<<<grid, THREADS, SMEM, stream>>>(tmQKV, tmDO, tmDQKV, a);
     CUDA_CHECK(cudaGetLastError());
+    if (nt == 1) return 0;
     dq_fold_kernel<<<(unsigned)(B * NH * nt), 256, 0, stream>>>(dqkv, dq_ws, B, T, NH, nt);
     CUDA_CHECK(cudaGetLastError());
     return 0;
 }
+
+// kernels that llmc_attention_bwd launches
+extern "C" int llmc_attention_bwd_launches(int T, int hs) { return hs == HS && T <= BT ? 1 : 3; }
