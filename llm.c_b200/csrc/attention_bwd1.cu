@@ -47,6 +47,7 @@
 //
 // Capability parity: attention_backward_cudnn (llmc/cudnn_att.cpp:256-288) and attention_backward of llmc/attention.cuh.
 #include "common.cuh"
+#include "pdl.cuh"
 
 int llmc_attn_qkv_map(CUtensorMap* tm, const bf16* qkv, int B, int T, int NH, int hs);   // attention_fwd.cu
 int llmc_attention_bwd_two_pass(bf16* dqkv, float* delta, const bf16* dout, const bf16* qkv, const bf16* out, const float* lse,
@@ -79,6 +80,7 @@ struct Args {
     const bf16* dout;
     int B, T, NH;
     float scale, scale_log2e;
+    int early;           // the next kernel may start while this one runs
     unsigned int* status;
     long long* trace;    // optional: [4 roles][8 events][TRACE_PAIRS] clock64() stamps of CTA 0 (null in normal runs)
 };
@@ -177,6 +179,8 @@ attn_bwd1_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constan
     const uint32_t tmem_base = *tmem_slot;
     const uint32_t tS = tmem_base, tdP = tmem_base + 128, tdV = tmem_base + 256, tdK = tmem_base + 320, tdQ = tmem_base + 384,
                    tP = tmem_base + 448;
+    pdl_wait();
+    if (a.early) pdl_trigger();
 
     // time stamps of CTA 0's first TRACE_PAIRS pairs, one thread per role, for the timeline tool (llmc_attention_bwd_set_trace)
 #define TRACE(role, ev) do { if (a.trace != nullptr && blockIdx.x == 0 && t < TRACE_PAIRS) a.trace[((role) * 8 + (ev)) * TRACE_PAIRS + t] = clock64(); } while (0)
@@ -694,6 +698,11 @@ extern "C" int llmc_attention_bwd(bf16* dqkv, float* ws, const bf16* dout, const
     if (!configured) {
         CUDA_CHECK(cudaFuncSetAttribute(attn_bwd1_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM));
         configured = true;
+    }
+    a.early = nt == 1 && grid < sms;       // as in the forward pass; with more tiles the kernels before and after are launched plainly
+    if (a.early) {
+        CUDA_CHECK(launch_pdl(attn_bwd1_kernel, dim3(grid), dim3(THREADS), SMEM, stream, 0, tmQKV, tmDO, tmDQKV, a));
+        return 0;
     }
     attn_bwd1_kernel<<<grid, THREADS, SMEM, stream>>>(tmQKV, tmDO, tmDQKV, a);
     CUDA_CHECK(cudaGetLastError());

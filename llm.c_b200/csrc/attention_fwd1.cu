@@ -23,6 +23,7 @@
 //
 // Capability parity: attention_forward_cudnn (llmc/cudnn_att.cpp:222-254) and attention_forward of llmc/attention.cuh.
 #include "common.cuh"
+#include "pdl.cuh"
 
 int llmc_attn_qkv_map(CUtensorMap* tm, const bf16* qkv, int B, int T, int NH, int hs);   // attention_fwd.cu
 int llmc_attention_fwd_general(bf16* out, float* lse, const bf16* qkv, int B, int T, int NH, int hs, cudaStream_t stream);
@@ -45,6 +46,7 @@ struct Args {
     int B, T, NH;
     float scale_log2e; // (1/sqrt(HS)) * log2(e)
     float scale;
+    int early;           // the next kernel may start while this one runs
     unsigned int* status;
     long long* trace;  // optional: [3 roles][8 events][64 tiles] clock64() stamps of CTA 0 (null in normal runs)
 };
@@ -110,6 +112,8 @@ attn_fwd1_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constan
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    pdl_wait();
+    if (a.early) pdl_trigger();
 
     if (warp == 0) {
         // ---------------------------------------------------------------- TMA producer
@@ -421,6 +425,13 @@ extern "C" int llmc_attention_fwd(bf16* out, float* lse, const bf16* qkv, int B,
     if (!configured) {
         CUDA_CHECK(cudaFuncSetAttribute(attn_fwd1_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM));
         configured = true;
+    }
+    // early launch (pdl.cuh) only where SMs stay free: 4 x 64 GPT-2 step 1566 -> 1513 us; otherwise the blocks of the next kernel sit beside
+    // this one's for all of its run: 64 x 1024 x 12 938 -> 986 us
+    a.early = grid < sms;
+    if (a.early) {
+        CUDA_CHECK(launch_pdl(attn_fwd1_kernel, dim3(grid), dim3(THREADS), SMEM, stream, 0, tmQKV, tmOut, a));
+        return 0;
     }
     attn_fwd1_kernel<<<grid, THREADS, SMEM, stream>>>(tmQKV, tmOut, a);
     CUDA_CHECK(cudaGetLastError());
