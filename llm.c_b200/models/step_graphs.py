@@ -9,6 +9,7 @@ before), all scalar arguments are part of the key, and the addresses of every pa
 table are compared.  The scratch buffers of the operators are shared by all callers and replaced when one needs a larger one, so a graph keeps those that its own operators took.
 """
 import contextlib
+import gc
 
 import torch
 
@@ -100,14 +101,21 @@ class StepGraphs:
         graph, side = torch.cuda.CUDAGraph(), torch.cuda.Stream(device=model.device)
         before = kernels.launch_count()
         with torch.cuda.stream(side), kernels.scratch_taken() as scratch:
-            # other threads (watchdog, data loader) may use the device meanwhile
-            graph.capture_begin(capture_error_mode="thread_local")
-            model.step_graphs.side = Side(torch.cuda.Stream(device=model.device))
+            # a collection inside the capture could find a dropped model, and the graphs it held cannot be freed by a thread that captures
+            collects = gc.isenabled()
+            gc.disable()
             try:
-                fn()
+                # other threads (watchdog, data loader) may use the device meanwhile
+                graph.capture_begin(capture_error_mode="thread_local")
+                model.step_graphs.side = Side(torch.cuda.Stream(device=model.device))
+                try:
+                    fn()
+                finally:
+                    model.step_graphs.side = Inline()
+                    graph.capture_end()
             finally:
-                model.step_graphs.side = Inline()
-                graph.capture_end()
+                if collects:
+                    gc.enable()
         e["launches"] = kernels.launch_count() - before
         kernels.count_launches(-e["launches"])                 # captured, not launched
         e["scratch"] = scratch
