@@ -277,7 +277,8 @@ DEVINL bf16x8 rotate_pack(const bf16x8& a, const float4& cs0, const float4& cs1,
 // its index cost as much as the memory took: 16384 rows of 32 + 2 x 8 heads of 128 forward 98 us (128), backward 102 us (166).
 constexpr int ROPE_THREADS = 256;
 
-template <int REP>
+// CACHE: keys and values also go to the cache; calls without one have no branch and no division for it
+template <int REP, bool CACHE>
 __global__ void __launch_bounds__(ROPE_THREADS)
 rope_fwd_kernel(bf16* __restrict__ packed, const bf16* __restrict__ raw, const float2* __restrict__ freqs, bf16* __restrict__ kcache,
                 bf16* __restrict__ vcache, int cache_len, int T, int NH, int NKV, int HS) {
@@ -302,7 +303,7 @@ rope_fwd_kernel(bf16* __restrict__ packed, const bf16* __restrict__ raw, const f
             #pragma unroll
             for (int r = 0; r < (REP ? REP : 1); r++) st128(d + r * HS, a);
             if (REP == 0) for (int r = 1; r < rep; r++) st128(d + r * HS, a);
-            if (kcache != nullptr) {
+            if (CACHE) {
                 const size_t at = (((size_t)(blockIdx.x / (unsigned)T) * cache_len + blockIdx.x % (unsigned)T) * NKV + hk) * HS + p * 8;
                 st128((which == 1 ? kcache : vcache) + at, a);
             }
@@ -488,7 +489,7 @@ extern "C" int llmc_rope_fwd_cache(bf16* packed, const bf16* raw, const float* f
                                    int NKV, int HS, cudaStream_t stream) {
     if (rope_check(NH, NKV, HS)) return -1;
     if (N <= 0) return 0;
-#define ROPE_GO(R) CUDA_CHECK(launch_pdl(rope_fwd_kernel<R>, dim3((unsigned)N), dim3(ROPE_THREADS), 0, stream, 0, packed, raw, reinterpret_cast<const float2*>(freqs), kcache, vcache, cache_len, T, NH, NKV, HS))
+#define ROPE_GO(R) CUDA_CHECK(launch_pdl(kcache != nullptr ? rope_fwd_kernel<R, true> : rope_fwd_kernel<R, false>, dim3((unsigned)N), dim3(ROPE_THREADS), 0, stream, 0, packed, raw, reinterpret_cast<const float2*>(freqs), kcache, vcache, cache_len, T, NH, NKV, HS))
     const int rep = NH / NKV;
     if (rep == 1) ROPE_GO(1);
     else if (rep == 2) ROPE_GO(2);
