@@ -157,7 +157,7 @@ DEVINL float bf16hi(uint32_t u) { return __uint_as_float(u & 0xffff0000u); }
 
 template <bool ACCUM_DINP, int MAXP, bool COLSUM, bool CACHE>
 __global__ void __launch_bounds__(LNB_MAX_THREADS)
-ln_bwd_col_kernel(bf16* __restrict__ dinp, float* __restrict__ partials, const bf16* __restrict__ dout,
+ln_bwd_col_kernel(bf16* dinp, const bf16* dold, float* __restrict__ partials, const bf16* __restrict__ dout,
                   const bf16* __restrict__ inp, const bf16* __restrict__ weight,
                   const float* __restrict__ mean, const float* __restrict__ rstd, int N, int C, int rows_per_cta) {
     pdl_wait();
@@ -194,7 +194,7 @@ ln_bwd_col_kernel(bf16* __restrict__ dinp, float* __restrict__ partials, const b
             if (p < npack) {
                 dq_[i] = __ldcs(reinterpret_cast<const uint4*>(dout + rb + p * 8));
                 xq_[i] = __ldcs(reinterpret_cast<const uint4*>(inp + rb + p * 8));
-                if (ACCUM_DINP) oq_[i] = __ldcs(reinterpret_cast<const uint4*>(dinp + rb + p * 8));
+                if (ACCUM_DINP) oq_[i] = __ldcs(reinterpret_cast<const uint4*>(dold + rb + p * 8));
             }
         }
         rs_ = rstd[row];
@@ -378,7 +378,7 @@ namespace {
 struct LnbLaunch { int threads, ctas, rows_per_cta; };
 
 template <bool ACC, int MAXP, bool COL>
-int lnb_launch(bf16* dinp, float* scratch, const bf16* dout, const bf16* inp, const bf16* weight, const float* mean, const float* rstd,
+int lnb_launch(bf16* dinp, const bf16* dold, float* scratch, const bf16* dout, const bf16* inp, const bf16* weight, const float* mean, const float* rstd,
                int N, int C, int threads, bool rows, int* ctas_out, cudaStream_t stream) {
     constexpr bool CACHE = MAXP <= 2;
     static int occ_cache[LNB_MAX_THREADS / 32 + 1] = {0};
@@ -392,18 +392,18 @@ int lnb_launch(bf16* dinp, float* scratch, const bf16* dout, const bf16* inp, co
     int ctas = occ * sms;
     int rows_per_cta = CEIL_DIV(N, ctas);
     ctas = CEIL_DIV(N, rows_per_cta);
-    if (rows) CUDA_CHECK(launch_pdl(ln_bwd_col_kernel<ACC, MAXP, COL, CACHE>, dim3(ctas), dim3(threads), 0, stream, 0, dinp, scratch, dout, inp, weight, mean, rstd, N, C, rows_per_cta));
+    if (rows) CUDA_CHECK(launch_pdl(ln_bwd_col_kernel<ACC, MAXP, COL, CACHE>, dim3(ctas), dim3(threads), 0, stream, 0, dinp, dold, scratch, dout, inp, weight, mean, rstd, N, C, rows_per_cta));
     *ctas_out = ctas;
     return 0;
 }
 
 template <int MAXP>
-int lnb_dispatch(bool acc, bool col, bf16* dinp, float* scratch, const bf16* dout, const bf16* inp, const bf16* weight,
+int lnb_dispatch(bool acc, bool col, bf16* dinp, const bf16* dold, float* scratch, const bf16* dout, const bf16* inp, const bf16* weight,
                  const float* mean, const float* rstd, int N, int C, int threads, bool rows, int* ctas_out, cudaStream_t stream) {
-    if (acc) return col ? lnb_launch<true, MAXP, true>(dinp, scratch, dout, inp, weight, mean, rstd, N, C, threads, rows, ctas_out, stream)
-                        : lnb_launch<true, MAXP, false>(dinp, scratch, dout, inp, weight, mean, rstd, N, C, threads, rows, ctas_out, stream);
-    return col ? lnb_launch<false, MAXP, true>(dinp, scratch, dout, inp, weight, mean, rstd, N, C, threads, rows, ctas_out, stream)
-               : lnb_launch<false, MAXP, false>(dinp, scratch, dout, inp, weight, mean, rstd, N, C, threads, rows, ctas_out, stream);
+    if (acc) return col ? lnb_launch<true, MAXP, true>(dinp, dold, scratch, dout, inp, weight, mean, rstd, N, C, threads, rows, ctas_out, stream)
+                        : lnb_launch<true, MAXP, false>(dinp, dold, scratch, dout, inp, weight, mean, rstd, N, C, threads, rows, ctas_out, stream);
+    return col ? lnb_launch<false, MAXP, true>(dinp, dold, scratch, dout, inp, weight, mean, rstd, N, C, threads, rows, ctas_out, stream)
+               : lnb_launch<false, MAXP, false>(dinp, dold, scratch, dout, inp, weight, mean, rstd, N, C, threads, rows, ctas_out, stream);
 }
 }  // namespace
 
@@ -411,28 +411,23 @@ int lnb_dispatch(bool acc, bool col, bf16* dinp, float* scratch, const bf16* dou
 // If dcolsum is given it receives (+)= the column sums of the final dinp: when dinp is the residual-stream gradient, that
 // is the bias gradient of the projection that wrote into the residual stream, obtained without another pass.  C <= 16384.
 // parts: 1 the kernel over the rows, 2 the sums over its CTAs (dweight, dbias, dcolsum), which nothing of a backward pass reads: they may follow in
-// another stream; 3 both.
+// another stream; 3 both.  dold: what dinp adds to, where that stays as it is for readers in another stream (null: dinp itself).
 extern "C" int llmc_layernorm_bwd_parts(bf16* dinp, bf16* dweight, bf16* dbias, float* scratch, const bf16* dout, const bf16* inp,
                                   const bf16* weight, const float* mean, const float* rstd, int N, int C,
-                                  int accumulate_dinp, int accumulate_dwdb, bf16* dcolsum, int accumulate_dcol, int parts, cudaStream_t stream) {
+                                  int accumulate_dinp, int accumulate_dwdb, bf16* dcolsum, int accumulate_dcol, const bf16* dold, int parts,
+                                  cudaStream_t stream) {
     if (C % 8 || C > LNB_MAX_THREADS * 8 * 8) return -1;
+    if (dold == nullptr) dold = dinp;
     const int npack = C / 8;
     const int threads = npack <= LNB_MAX_THREADS ? CEIL_DIV(npack, 32) * 32 : LNB_MAX_THREADS;
     const int packs = CEIL_DIV(npack, threads);
     const bool acc = accumulate_dinp != 0, col = dcolsum != nullptr;
     int ctas = 0, rc;
-    if (packs <= 1) rc = lnb_dispatch<1>(acc, col, dinp, scratch, dout, inp, weight, mean, rstd, N, C, threads, parts & 1, &ctas, stream);
-    else if (packs <= 2) rc = lnb_dispatch<2>(acc, col, dinp, scratch, dout, inp, weight, mean, rstd, N, C, threads, parts & 1, &ctas, stream);
-    else if (packs <= 4) rc = lnb_dispatch<4>(acc, col, dinp, scratch, dout, inp, weight, mean, rstd, N, C, threads, parts & 1, &ctas, stream);
-    else rc = lnb_dispatch<8>(acc, col, dinp, scratch, dout, inp, weight, mean, rstd, N, C, threads, parts & 1, &ctas, stream);
+    if (packs <= 1) rc = lnb_dispatch<1>(acc, col, dinp, dold, scratch, dout, inp, weight, mean, rstd, N, C, threads, parts & 1, &ctas, stream);
+    else if (packs <= 2) rc = lnb_dispatch<2>(acc, col, dinp, dold, scratch, dout, inp, weight, mean, rstd, N, C, threads, parts & 1, &ctas, stream);
+    else if (packs <= 4) rc = lnb_dispatch<4>(acc, col, dinp, dold, scratch, dout, inp, weight, mean, rstd, N, C, threads, parts & 1, &ctas, stream);
+    else rc = lnb_dispatch<8>(acc, col, dinp, dold, scratch, dout, inp, weight, mean, rstd, N, C, threads, parts & 1, &ctas, stream);
     if (rc) return rc;
     if (parts & 2) CUDA_CHECK(launch_pdl(ln_bwd_fold_kernel, dim3(CEIL_DIV(C, 16)), dim3(4 * LNB_FOLD_SLICES), 0, stream, 0, dweight, dbias, dcolsum, scratch, ctas, C, accumulate_dwdb, accumulate_dcol));
     return 0;
-}
-
-extern "C" int llmc_layernorm_bwd(bf16* dinp, bf16* dweight, bf16* dbias, float* scratch, const bf16* dout, const bf16* inp,
-                                  const bf16* weight, const float* mean, const float* rstd, int N, int C,
-                                  int accumulate_dinp, int accumulate_dwdb, bf16* dcolsum, int accumulate_dcol, cudaStream_t stream) {
-    return llmc_layernorm_bwd_parts(dinp, dweight, dbias, scratch, dout, inp, weight, mean, rstd, N, C, accumulate_dinp, accumulate_dwdb, dcolsum,
-                                    accumulate_dcol, 3, stream);
 }

@@ -10,7 +10,7 @@
 // 64-wide heads with a block on every SM are launched plainly and trigger nothing: attention at 64 x 1024 x 12 x 64 forward and backward took
 // 986 us with the attribute and 938 without, on one GPU in turn; the classifier's figures stand with it.  Where 64-wide heads leave SMs free
 // the attribute pays: forward + backward of 4 x 64 tokens 1566 us without and 1513 with it, a prefill of 777 tokens 628 and 619.  (The bracketed
-// comparisons were made when the plain launch was the only other thing that differed; those passes take 1513, 273 and 619 us now.)
+// comparisons were made when the plain launch was the only other thing that differed; those passes take 1498, 274 and 618 us now.)
 #pragma once
 #include "common.cuh"
 

@@ -16,8 +16,8 @@
 // 32 x 6144 x 4096 23 us (38), 32 x 28672 x 4096 58 us (69), 100 x 2048 x 7168 23 us (52).  Inside a replayed decoding step (4 rows, 4 layers
 // of 2048 channels, LM head of 128256 rows) this kernel takes the step to 277 us; a weight-streaming kernel on warp-level MMAs with the same
 // early launch and prefetch, used for the products of at most 8 rows, left it at 290 us (at 284 us for the LM head alone), although launched
-// by itself it is faster (4 x 28672 x 4096 50 us against 59; skinny_gemm_kernel in decode.cu).  More rows: 256 x 768 x 50304 (an input gradient)
-// 60 us (291), 777 x 2048 x 7168 37 us (53), 256 x 768 x 3072 18 us (27).
+// by itself it is faster (4 x 28672 x 4096 50 us against 59; skinny_gemm_kernel in decode.cu).  More rows (input gradients, in a chain, the training GEMM's tiles in
+// brackets): 256 x 768 x 768 4.9 us (6.3), 256 x 768 x 3072 7.9 us (16.3), 256 x 768 x 50304 44 us (291 after an L2 flush).
 //
 // Warps of a CTA: 0 TMA producer, 1 MMA issuer, 2-5 epilogue.  Two CTAs fit an SM.
 #include "common.cuh"
@@ -378,6 +378,20 @@ int pick_split(int tiles, int num_kb, int nb, int sms) {
     return s;
 }
 
+// Input gradients of more than 128 rows: row tiles of 64 rows and more, as many as leave room for four slices of K each.  What a CTA waits for is its own
+// loads (128 + rows per k-block) and its share of the reduction, and both shrink with the tile.  Rows x slices, us, in a chain (M x N x K):
+// 256 x 768 x 768 256x4 9.3, 128x4 6.4, 64x4 5.0; 256 x 768 x 2304 11.4, 8.5, 7.1 (64x8 7.4); 256 x 768 x 3072 12.5, 9.5, 8.2 (64x8 7.9);
+// 512 x 1024 x 4096 14.2, 11.9, 12.0; 1024 x 768 x 3072 13.3, 12.5, 96x4 11.7, 64x4 in two rounds 18.0.
+void pick_rows_and_split(int M, int tiles, int num_kb, int sms, int& mtiles, int& S) {
+    const int slots = 2 * (sms * 7 / 8);
+    int t = CEIL_DIV(M, 64);
+    while (t > 1 && tiles * t * 4 > slots) t--;
+    mtiles = t; S = 0;
+    if (CEIL_DIV(M, t) > 128) { mtiles = CEIL_DIV(M, MAX_NB); return; }      // wide tiles: pick_split
+    for (S = 1; S < 4 && num_kb >= S * 2 * 3; ) S *= 2;
+    if (S == 4 && tiles * t * 8 <= slots && num_kb >= 48) S = 8;
+}
+
 template <int MODE, bool W_MN>
 int launch_stream(bf16* out, const bf16* x, const bf16* w, const bf16* bias, int M, int N, int K, int ldx, int ldw, int ldo, int early_w, cudaStream_t stream) {
     if (M <= 0 || N <= 0 || K <= 0 || (K % 8) || (ldx % 8) || (ldw % 8) || ldx < K || ldw < (W_MN ? N : K) || ldo < N) return -1;
@@ -385,8 +399,12 @@ int launch_stream(bf16* out, const bf16* x, const bf16* w, const bf16* bias, int
     Args g;
     g.early_w = early_w;
     g.out = out; g.bias = bias; g.w = w; g.M = M; g.N = N; g.K = K; g.ldo = ldo; g.ldw = ldw;
-    const int mtiles = CEIL_DIV(M, MAX_NB);
+    int sms = llmc_device_sm_count(); if (sms <= 0) sms = 148;
+    const int tiles = CEIL_DIV(N, MODE == SWIGLU ? WR / 2 : WR);
+    int mtiles = CEIL_DIV(M, MAX_NB), S = 0;
+    if (W_MN && M > 128) pick_rows_and_split(M, tiles, CEIL_DIV(K, BK), sms, mtiles, S);
     g.nb = (CEIL_DIV(M, mtiles) + 15) & ~15;             // M spread evenly over its tiles
+    mtiles = CEIL_DIV(M, g.nb);
     g.num_kb = CEIL_DIV(K, BK);
     const int stage_bytes = W_BYTES + g.nb * (BK * 2);
     const bool two = g.nb <= 128;
@@ -408,8 +426,6 @@ int launch_stream(bf16* out, const bf16* x, const bf16* w, const bf16* bias, int
         rc = llmc_get_tensormap(&tmX, x, 2, 2, dimx, strx, boxx, 3);
         if (rc) return rc;
     }
-    int sms = llmc_device_sm_count(); if (sms <= 0) sms = 148;
-    const int tiles = CEIL_DIV(N, MODE == SWIGLU ? WR / 2 : WR);
     if (MODE == STORE && !W_MN && mtiles == 1 && two && tiles > 2 * sms) {
         static bool configured_wide = false;
         const int smem = g.stages * stage_bytes + 1024 + 256;
@@ -420,7 +436,7 @@ int launch_stream(bf16* out, const bf16* x, const bf16* w, const bf16* bias, int
         CUDA_CHECK(launch_pdl(stream_wide_kernel, dim3(2 * sms), dim3(THREADS), smem, stream, 0, tmW, tmX, g));
         return 0;
     }
-    const int S = pick_split(tiles * mtiles, g.num_kb, g.nb, sms);
+    if (S == 0) S = pick_split(tiles * mtiles, g.num_kb, g.nb, sms);
     g.kb_per_split = CEIL_DIV(g.num_kb, S);
     const int smem = g.stages * stage_bytes + 1024 + 256;
     static bool configured = false;

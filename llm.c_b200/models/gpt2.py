@@ -312,7 +312,8 @@ class GPT:
         dres, dl_btc, dl_bt4c, dqkv = a["dresidual"], a["scratch_btc"], a["scratch_bt4c"], a["dqkv"]
         dlogits = a["logits"]
         # gradients of weights and biases are read by nothing in this pass: in a captured graph they run beside the chain of input gradients, joined
-        # before a buffer that they read is overwritten (dres and the partial sums by the next LayerNorm backward, the others by the next layer)
+        # before a buffer that they read is overwritten (the partial sums by the next LayerNorm backward, dres by the one after it, since they take turns
+        # at two buffers, the others by the next layer).  4 x 64 tokens, us: one buffer 1512, two 1528, two and input gradients in slices of K 1498.
         side = self.step_graphs.side
 
         with side.fork():
@@ -322,6 +323,7 @@ class GPT:
         # bias gradient of the projection (fcproj / attproj) whose output was added to the stream just before that LayerNorm
         ops.layernorm_backward(dres, g["lnfw"], g["lnfb"], dl_btc, a["residual3"][L - 1], p["lnfw"], a["lnf_mean"], a["lnf_rstd"],
                                accumulate_dinp=False, accumulate_dwdb=acc, dcolsum=g["fcprojb"][L - 1], accumulate_dcol=acc, sums_in=side.fork)
+        sums = side.mark()
         nvtx = self.device.type == "cuda"
         for l in reversed(range(L)):
           with _Range("backward layer %d" % l, nvtx):
@@ -332,7 +334,6 @@ class GPT:
                 ops.gelu_forward(a["fch_gelu"][lg], a["fch"][l])
             with side.fork():
                 ops.matmul_wgrad(g["fcprojw"][l], dres, a["fch_gelu"][lg], accumulate=acc)
-            dres_read = side.mark()
             ops.matmul_dgrad(dl_bt4c, dres, p["fcprojw"][l], pre_gelu=a["fch"][l])
             if self.recompute >= 2:
                 ops.layernorm_forward(a["ln2"][lln], None, None, a["residual2"][l], p["ln2w"][l], p["ln2b"][l])
@@ -340,13 +341,14 @@ class GPT:
                 ops.bias_grad(g["fcb"][l], dl_bt4c, accumulate=acc)
                 ops.matmul_wgrad(g["fcw"][l], dl_bt4c, a["ln2"][lln], accumulate=acc)
             ops.matmul_dgrad(dl_btc, dl_bt4c, p["fcw"][l])
-            side.join(dres_read)
+            side.join(sums)
+            old, dres = dres, side.other(dres)
             ops.layernorm_backward(dres, g["ln2w"][l], g["ln2b"][l], dl_btc, a["residual2"][l], p["ln2w"][l], a["ln2_mean"][l],
                                    a["ln2_rstd"][l], accumulate_dinp=True, accumulate_dwdb=acc, dcolsum=g["attprojb"][l], accumulate_dcol=acc,
-                                   sums_in=side.fork)
+                                   sums_in=side.fork, dinp_old=old)
+            sums = side.mark()
             with side.fork():
                 ops.matmul_wgrad(g["attprojw"][l], dres, a["atty"][l], accumulate=acc)
-            dres_read = side.mark()
             ops.matmul_dgrad(dl_btc, dres, p["attprojw"][l])
             ops.attention_backward(dqkv, dl_btc, a["qkv"][l], a["atty"][l], a["lse"][l], B, T, NH)
             if self.recompute >= 2:
@@ -355,10 +357,12 @@ class GPT:
                 ops.bias_grad(g["qkvb"][l], dqkv, accumulate=acc)
                 ops.matmul_wgrad(g["qkvw"][l], dqkv, a["ln1"][lln], accumulate=acc)
             ops.matmul_dgrad(dl_btc, dqkv, p["qkvw"][l])
-            side.join(dres_read)
+            side.join(sums)
+            old, dres = dres, side.other(dres)
             ops.layernorm_backward(dres, g["ln1w"][l], g["ln1b"][l], dl_btc, residual, p["ln1w"][l], a["ln1_mean"][l],
                                    a["ln1_rstd"][l], accumulate_dinp=True, accumulate_dwdb=acc,
-                                   dcolsum=(g["fcprojb"][l - 1] if l > 0 else None), accumulate_dcol=acc, sums_in=side.refork)
+                                   dcolsum=(g["fcprojb"][l - 1] if l > 0 else None), accumulate_dcol=acc, sums_in=side.refork, dinp_old=old)
+            sums = side.mark()
             if hook is not None:
                 hook(l)
         side.join()

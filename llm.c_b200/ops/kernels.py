@@ -91,7 +91,10 @@ def _few_rows(M, N, K, mode, b_mn, device):
     two kernels (M from 100 to 2048, fourteen pairs of N and K, us): deep products whose tiles leave at least half of the SMs idle
     (K = 3072: 24 tiles 21 against 27, 36 tiles 33 against 27; K = 7168: 64 tiles 37 to 43 against 53, 96 tiles 61 against 55), and
     at most 128 rows, unless there are more weight tiles than resident CTAs (64 rows and more, _wide) or the product is a shallow input gradient
-    (100 x 768 x 768: 16 against 14).  Forward products of more than 128 rows
+    (100 x 768 x 768: 16 against 14).  Input gradients of more than 128 rows go there as long as four slices of K of row tiles of at most 128
+    rows are resident at once and K pays for the reduction, which grows with the number of tiles (in a chain, theirs in brackets: 130 x 512 x 768
+    4.4 (6.3), 256 x 768 x 768 4.9 (6.3), x 2304 7.0 (13.0), x 3072 7.9 (16.3), 512 x 768 x 768 6.1 (6.4), 1024 x 768 x 1600 9.8 (10.4),
+    1024 x 1024 x 2304 11.7 (13.9); 384 x 2048 x 1024 8.3 (7.8), 1024 x 768 x 1024 8.5 (7.8), 512 x 1600 x 1600 10.7 (10.4)).  Forward products of more than 128 rows
     below a depth of 6144 keep their one sum over K: at 8 us each (256 x 768 x 3072: 18 against 27) they are not worth another order of
     summation in the loss.  At most 128 rows are summed in slices from K = 512 on, in fp32 and in slice order."""
     if mode != MODE_STORE:
@@ -100,8 +103,11 @@ def _few_rows(M, N, K, mode, b_mn, device):
     tiles = (M + 255) // 256 * wtiles
     if (K >= 6144 and tiles <= 64) or (b_mn and K >= 3072 and tiles <= 32):
         return True
+    if b_mn and M > STREAM_MAX_ROWS:
+        narrow = (M + 127) // 128 * wtiles
+        return K >= max(768, 32 * narrow) and narrow * 4 <= 2 * (sm_count(device) * 7 // 8)
     if b_mn:
-        return M <= STREAM_MAX_ROWS and K >= 2048 and wtiles <= 2 * sm_count(device)
+        return K >= 2048 and wtiles <= 2 * sm_count(device)
     return M <= 64 or (M <= STREAM_MAX_ROWS and wtiles <= 2 * sm_count(device))
 
 
@@ -299,8 +305,8 @@ def fused_residual_forward(residual, normed, mean, rstd, inp1, inp2, weight, bia
 
 
 def layernorm_backward(dinp, dweight, dbias, dout, inp, weight, mean, rstd, accumulate_dinp=True, accumulate_dwdb=True,
-                       dcolsum=None, accumulate_dcol=True, sums_in=None):
-    """dinp (+)= dLN(dout); dweight/dbias (+)= their gradients.  ``dcolsum`` (+)= column sums of the final dinp: the bias
+                       dcolsum=None, accumulate_dcol=True, sums_in=None, dinp_old=None):
+    """dinp (+)= dLN(dout), added to ``dinp_old`` if that is given; dweight/dbias (+)= their gradients.  ``dcolsum`` (+)= column sums of the final dinp: the bias
     gradient of the projection that wrote into the residual stream, at no extra pass over memory.  ``sums_in()`` may give a
     context (another stream) in which the three column sums are finished; the next call has to follow them."""
     global _launches
@@ -311,11 +317,11 @@ def layernorm_backward(dinp, dweight, dbias, dout, inp, weight, mean, rstd, accu
     args = (_p(dinp), _p(dweight), _p(dbias), _p(s), _p(dout), _p(inp), _p(weight), _p(mean), _p(rstd),
             N, C, int(accumulate_dinp), int(accumulate_dwdb), _p(dcolsum), int(accumulate_dcol))
     if sums_in is None:
-        check(lib.llmc_layernorm_bwd(*args, _stream()), "llmc_layernorm_bwd")
+        check(lib.llmc_layernorm_bwd_parts(*args, _p(dinp_old), 3, _stream()), "llmc_layernorm_bwd_parts")
         return
-    check(lib.llmc_layernorm_bwd_parts(*args, 1, _stream()), "llmc_layernorm_bwd_parts")
+    check(lib.llmc_layernorm_bwd_parts(*args, _p(dinp_old), 1, _stream()), "llmc_layernorm_bwd_parts")
     with sums_in():
-        check(lib.llmc_layernorm_bwd_parts(*args, 2, _stream()), "llmc_layernorm_bwd_parts")
+        check(lib.llmc_layernorm_bwd_parts(*args, _p(dinp_old), 2, _stream()), "llmc_layernorm_bwd_parts")
 
 
 def attention_forward(out, lse, qkv, B, T, NH):

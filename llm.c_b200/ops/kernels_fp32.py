@@ -79,7 +79,9 @@ def fused_residual_forward(residual, normed, mean, rstd, inp1, inp2, weight, bia
 
 
 def layernorm_backward(dinp, dweight, dbias, dout, inp, weight, mean, rstd, accumulate_dinp=True, accumulate_dwdb=True,
-                       dcolsum=None, accumulate_dcol=True, sums_in=None):
+                       dcolsum=None, accumulate_dcol=True, sums_in=None, dinp_old=None):
+    if accumulate_dinp and dinp_old is not None and dinp_old is not dinp:
+        dinp.copy_(dinp_old)
     lib = _lib_()
     C = inp.shape[-1]
     rows = inp.numel() // C

@@ -130,7 +130,7 @@ def fused_residual_forward(residual, normed, mean, rstd, inp1, inp2, weight, bia
 
 
 def layernorm_backward(dinp, dweight, dbias, dout, inp, weight, mean, rstd, accumulate_dinp=True, accumulate_dwdb=True,
-                       dcolsum=None, accumulate_dcol=True, sums_in=None):
+                       dcolsum=None, accumulate_dcol=True, sums_in=None, dinp_old=None):
     dy, x, w = _f(dout), _f(inp), _f(weight)
     norm = (x - mean.unsqueeze(-1)) * rstd.unsqueeze(-1)
     dnorm = dy * w
@@ -138,7 +138,7 @@ def layernorm_backward(dinp, dweight, dbias, dout, inp, weight, mean, rstd, accu
     dw = (dy * norm).sum(0)
     db = dy.sum(0)
     if accumulate_dinp:
-        dx = dx + _f(dinp)
+        dx = dx + _f(dinp if dinp_old is None else dinp_old)
     if accumulate_dwdb:
         dw, db = dw + _f(dweight), db + _f(dbias)
     dinp.copy_(dx)
