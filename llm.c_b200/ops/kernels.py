@@ -136,9 +136,10 @@ def _swapped(M, N, K, device):
 FORWARD_GEMM, FORWARD_GEMM2, FORWARD_STREAM, FORWARD_SWAPPED = range(4)        # csrc/decoder.cu, Product
 
 
-def forward_kernel(M, N, K, device):
-    """The kernel of a plain forward product without flags to wait for."""
-    if TWO_SM_MIN_TILES > 0 and _swapped(M, N, K, device):
+def forward_kernel(M, N, K, device, aligned=True):
+    """The kernel of a plain forward product without flags to wait for.  ``aligned``: the output starts on a 16-byte boundary.  The swapped kernel stores
+    with TMA, which needs that and rows of whole 16 bytes; the split-K kernel takes any number of columns and any alignment."""
+    if TWO_SM_MIN_TILES > 0 and N % 8 == 0 and aligned and _swapped(M, N, K, device):
         return FORWARD_SWAPPED
     if _few_rows(M, N, K, MODE_STORE, False, device) or _wide(M, N, device):
         return FORWARD_STREAM
@@ -154,7 +155,7 @@ def gemm(a, b, d, M, N, K, lda, ldb, ldd, a_mn, b_mn, mode, bias=None, aux=None,
     global _launches
     lib = _lib.cuda()
     _launches += 1
-    plain = forward_kernel(M, N, K, d.device) if mode == MODE_STORE and not a_mn and not b_mn else None
+    plain = forward_kernel(M, N, K, d.device, d.data_ptr() % 16 == 0) if mode == MODE_STORE and not a_mn and not b_mn else None
     if plain == FORWARD_SWAPPED and ready is None:
         check(lib.llmc_gemm2t(_p(d), _p(a), _p(b), _p(bias), M, N, K, lda, ldb, ldd, 0, _stream()), "llmc_gemm2t")
         return

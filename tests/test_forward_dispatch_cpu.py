@@ -1,0 +1,21 @@
+"""Which kernel a plain forward product goes to, by sizes alone (148 SMs)."""
+import pytest
+import torch
+
+from llmc_b200.ops import kernels as KN
+
+DEV = torch.device("cuda", 0)
+
+
+@pytest.fixture(autouse=True)
+def sms(monkeypatch):
+    monkeypatch.setattr(KN, "sm_count", lambda device: 148)
+
+
+# deep products that both the swapped and the split-K kernel can do: the swapped one has conditions on the output that the other does not have
+@pytest.mark.parametrize("M,N,K", [(500, 2056, 14336), (385, 2056, 6144), (2048, 1000, 6144)])
+def test_ragged_outputs_stay_with_the_split_k_kernel(M, N, K):
+    assert KN.forward_kernel(M, N, K, DEV) == KN.FORWARD_SWAPPED
+    assert KN.forward_kernel(M, N + 4, K, DEV) == KN.FORWARD_STREAM
+    assert KN.forward_kernel(M, N - 7, K, DEV) == KN.FORWARD_STREAM
+    assert KN.forward_kernel(M, N, K, DEV, aligned=False) == KN.FORWARD_STREAM

@@ -53,6 +53,20 @@ def test_forward_products_take_it(M, K, N):
     assert (out[M:] == 7.0).all()
 
 
+@pytest.mark.parametrize("M,N,K,offset", [(500, 2052, 14336, 0), (385, 2052, 6144, 0), (2048, 1004, 6144, 0), (385, 2049, 6144, 0), (500, 2056, 6144, 4), (500, 2056, 6144, 1)])
+def test_outputs_it_cannot_store(M, N, K, offset):
+    """Rows that are not whole 16 bytes, or an output that does not start on a 16-byte boundary."""
+    x, w, b = rnd(M, K), rnd(N, K, scale=0.05, seed=1), rnd(N, seed=2)
+    flat = torch.full((M * N + 16,), 7.0, dtype=torch.bfloat16, device=DEV)
+    out = flat[offset:offset + M * N].view(M, N)
+    KN.matmul_forward(out, x, w, b)
+    want = x.double() @ w.double().t() + b.double()
+    # one rounding to bf16 of an fp32 sum whose own error is below K * 2^-24 times the sum of the magnitudes
+    bound = 2 ** -8 * want.abs() + K * 2 ** -24 * (x.double().abs() @ w.double().abs().t()) + 1e-3
+    assert not ((out.double() - want).abs() > bound).any()
+    assert (flat[:offset] == 7.0).all() and (flat[offset + M * N:] == 7.0).all()
+
+
 def test_refuses_what_it_cannot_do():
     x, w, out = rnd(32, 64), rnd(64, 64), torch.empty(32, 64, dtype=torch.bfloat16, device=DEV)
     lib, p, s = _lib.cuda(), KN._p, KN._stream()
