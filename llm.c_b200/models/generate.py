@@ -92,7 +92,7 @@ class CachedDecoder:
                 self._dense = (torch.zeros(rows, 3 * C, dtype=m.dtype, device=m.device),
                                torch.zeros(B * NH * Tq, dtype=torch.float32, device=m.device))
             packed, lse = self._dense[0][:N], self._dense[1][:B * NH * Tq].view(B, NH, Tq)
-        if self.skinny_rows == kernels.STREAM_MAX_ROWS:
+        if self.skinny_rows == kernels.STREAM_MAX_ROWS and kernels.decoder_layout_ok(self):
             kernels.decoder_forward(self, a, (packed, lse) if dense else None, tokens, start_pos, pos)
             return a["logits"][:B, :cfg.vocab_size].float()
 

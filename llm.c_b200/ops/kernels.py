@@ -512,6 +512,19 @@ def matmul_swiglu_prompt(h, inp, weight12):
           "llmc_gemm2t_swiglu")
 
 
+def decoder_layout_ok(decoder):
+    """Whether ``decoder_forward`` can take this decoder's tensors: it finds a layer's weights and cache by their distance from the first layer's and
+    none of the operators' size checks stands between it and the kernels.  Called operator by operator every layer may lie anywhere."""
+    cfg, p = decoder.model.cfg, decoder.model.params
+    L, C, H, QR = cfg.num_layers, cfg.channels, cfg.hidden_dim, (cfg.num_heads + 2 * cfg.num_kv_heads) * cfg.head_size
+    k, v = decoder.kcache, decoder.vcache
+    shapes = (("ln1w", (L, C)), ("qkvw", (L, QR, C)), ("attprojw", (L, C, C)), ("ln2w", (L, C)), ("fc12w", (L, 2 * H, C)), ("fcprojw", (L, C, H)),
+              ("lnfw", (C,)), ("lmhead", (cfg.padded_vocab_size, C)))
+    return all(p[n].shape == s and p[n].is_contiguous() for n, s in shapes) and p["wte"].shape[1] == C and p["wte"].is_contiguous() \
+        and k.dim() == 5 and k.shape == v.shape and k.shape[0] == L and k.shape[3:] == (cfg.num_kv_heads, cfg.head_size) \
+        and k.is_contiguous() and v.is_contiguous()
+
+
 def decoder_forward(decoder, bufs, dense, tokens, start_pos, pos):
     """The launches of ``models.generate.CachedDecoder.forward`` for a bf16 model, from native code (csrc/decoder.cu).  ``bufs``: the decoder's activation
     buffers; ``dense``: (packed QKV, LSE) buffers for a prompt from position 0, or None."""

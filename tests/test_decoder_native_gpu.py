@@ -32,3 +32,21 @@ def test_same_logits_and_cache(desc, B, chunks):
             # the same kernels but for products of exactly 128 rows and row tiles: bf16 roundings of two layers apart
             assert float((x.float() - y.float()).norm() / y.float().norm()) < 1e-2
     assert min(called) > 0
+
+
+def test_layers_that_lie_apart():
+    """Caches and weights with a gap behind every layer are read one layer at a time."""
+    m = llama3.Llama(llama3.config_from_descriptor("llama3:l=2,c=256,h=4,kv=2,t=512,v=500"), DEV, torch.bfloat16)
+    m.init_random(3)
+    tok = torch.randint(0, 500, (2, 9), generator=torch.Generator().manual_seed(1), dtype=torch.int32).to(DEV)
+    plain, apart = generate.CachedDecoder(m, 2, 64), generate.CachedDecoder(m, 2, 64)
+    want = plain.forward(tok, 0)
+    around = torch.zeros(2, 4, *apart.kcache.shape[2:], dtype=torch.bfloat16, device=DEV)
+    apart.kcache = around[:, :2]
+    weights = torch.zeros(2, m.params["qkvw"].shape[1] + 8, 256, dtype=torch.bfloat16, device=DEV)
+    weights[:, :-8] = m.params["qkvw"]
+    m.params["qkvw"] = weights[:, :-8]
+    got = apart.forward(tok, 0)
+    for x, y in ((got, want), (apart.kcache, plain.kcache), (apart.vcache, plain.vcache)):
+        assert float((x.float() - y.float()).norm() / y.float().norm()) < 1e-2
+    assert not around[:, 2:].any()

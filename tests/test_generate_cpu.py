@@ -163,3 +163,38 @@ def test_an_empty_product_of_few_rows_is_no_error(M, N, K):
     assert lib.llmc_stream_gemm(None, None, None, None, M, N, K, 64, 64, 64, 0, None) == 0
     assert lib.llmc_gemm(None, None, None, None, None, M, N, K, 64, 64, 64, 0, 0, KN.MODE_STORE, 0, 1, None, None, 0, None) == 0
     assert lib.llmc_gemm2(None, None, None, None, None, M, N, K, 64, 64, 64, 0, 0, KN.MODE_STORE, 0, 1, None, None, None) == 0
+
+
+def spread(t, dim):
+    """The same values with a gap behind every slice of ``dim``."""
+    shape = list(t.shape)
+    shape[dim] += 3
+    big = torch.zeros(shape, dtype=t.dtype)
+    out = big.narrow(dim, 0, t.shape[dim])
+    out.copy_(t)
+    assert not out.is_contiguous()
+    return out
+
+
+@pytest.mark.parametrize("what", ["plain", "kcache", "vcache", "qkvw", "fcprojw", "short lmhead"])
+def test_the_natively_issued_pass_gets_only_layers_at_equal_distances(monkeypatch, what):
+    m = small_model()
+    tok = torch.arange(14, dtype=torch.int32).view(2, 7)
+    want = G.CachedDecoder(m, 2, 32).forward(tok, 0)
+    dec, issued = G.CachedDecoder(m, 2, 32), []
+    dec.skinny_rows = KN.STREAM_MAX_ROWS                       # as for a bf16 model on the GPU
+    dec.whole_tiles = False
+    monkeypatch.setattr(KN, "decoder_forward", lambda *a: issued.append(a))
+    if what.endswith("cache"):
+        setattr(dec, what, spread(getattr(dec, what), 1))
+    elif what == "short lmhead":                               # fewer rows than the buffer of logits has columns
+        m.params["lmhead"] = m.params["lmhead"][:-8]
+    elif what != "plain":
+        m.params[what] = spread(m.params[what], m.params[what].dim() - 2)
+    if what == "short lmhead":
+        with pytest.raises((RuntimeError, ValueError)):
+            dec.forward(tok, 0)
+    else:
+        got = dec.forward(tok, 0)
+        assert what == "plain" or torch.allclose(got, want, atol=1e-5, rtol=1e-5)
+    assert len(issued) == (what == "plain")
