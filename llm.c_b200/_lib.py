@@ -65,6 +65,7 @@ def cuda():
         "llmc_gemm_tiled": (I, [P, P, P, P, P, I, I, I, I, I, I, I, I, I, I, I, P, P, I, I, S]),
         "llmc_gemm2t": (I, [P, P, P, P, I, I, I, I, I, I, I, S]),
         "llmc_gemm2t_swiglu": (I, [P, P, P, I, I, I, I, I, I, I, S]),
+        "llmc_decoder_call_size": (I, []),
         "llmc_decoder_forward": (I, [POINTER(DecoderCall), POINTER(c_int), S]),
         "llmc_gemm2": (I, [P, P, P, P, P, I, I, I, I, I, I, I, I, I, I, I, P, P, S]),
         "llmc_gemm2_after_flags": (I, [P, P, P, P, P, I, I, I, I, I, I, I, I, I, I, I, P, P, P, I, U64, S]),
@@ -136,6 +137,8 @@ def cuda():
             fn = getattr(lib, name)
             fn.restype = res
             fn.argtypes = args
+    if lib.llmc_decoder_call_size() != ctypes.sizeof(DecoderCall):
+        raise KernelError("DecoderCall has %d bytes here and %d in csrc/decoder.cu" % (ctypes.sizeof(DecoderCall), lib.llmc_decoder_call_size()))
     _cuda = lib
     return lib
 

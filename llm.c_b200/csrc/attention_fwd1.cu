@@ -23,6 +23,7 @@
 //
 // Capability parity: attention_forward_cudnn (llmc/cudnn_att.cpp:222-254) and attention_forward of llmc/attention.cuh.
 #include "common.cuh"
+#include "decoder_ops.h"
 #include "pdl.cuh"
 
 int llmc_attn_qkv_map(CUtensorMap* tm, const bf16* qkv, int B, int T, int NH, int hs);   // attention_fwd.cu

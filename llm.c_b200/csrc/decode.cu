@@ -12,6 +12,7 @@
 // replayed with the position advanced on the device.  A device position that would leave the cache or the rotary table makes
 // the kernel record ST_BAD_ARG in the status word and return without touching memory.
 #include "common.cuh"
+#include "decoder_ops.h"
 #include "pdl.cuh"
 
 namespace {

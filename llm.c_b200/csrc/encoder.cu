@@ -10,6 +10,7 @@
 //
 // Capability parity: llmc/encoder.cuh (encoder_forward, encoder_backward) of the reference.
 #include "common.cuh"
+#include "decoder_ops.h"
 #include "pdl.cuh"
 
 namespace {

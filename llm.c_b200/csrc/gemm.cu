@@ -21,6 +21,7 @@
 //               tile's MMAs overlap.
 // No TMA load uses cluster multicast. All waits are bounded (see common.cuh).
 #include "common.cuh"
+#include "decoder_ops.h"
 #include "pdl.cuh"
 
 namespace {

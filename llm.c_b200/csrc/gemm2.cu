@@ -13,6 +13,7 @@
 // Epilogue: sixteen warps per CTA in four groups of four, each group owning 64 columns of the CTA's 128 x 256 half tile
 // (staging in shared memory, TMA stores).
 #include "common.cuh"
+#include "decoder_ops.h"
 #include "pdl.cuh"
 #include "two_sm.cuh"
 

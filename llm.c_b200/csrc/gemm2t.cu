@@ -13,6 +13,7 @@
 // output column and a column is a row of the output, so an epilogue warp turns 32 columns x 16 rows round through its own shared memory (one
 // 2-byte store per value, 64 contiguous bytes per warp) and one TMA store.
 #include "common.cuh"
+#include "decoder_ops.h"
 #include "pdl.cuh"
 #include "two_sm.cuh"
 

@@ -6,6 +6,7 @@
 // Capability parity: the reference has these only as PyTorch modules (train_llama3.py: RMSNorm :133-146,
 // apply_rotary_emb :107-117, repeat_kv :59-68, MLP :205-226); there is no CUDA counterpart to compare against.
 #include "common.cuh"
+#include "decoder_ops.h"
 #include "pdl.cuh"
 
 namespace {

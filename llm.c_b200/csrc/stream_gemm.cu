@@ -21,6 +21,7 @@
 //
 // Warps of a CTA: 0 TMA producer, 1 MMA issuer, 2-5 epilogue.  Two CTAs fit an SM.
 #include "common.cuh"
+#include "decoder_ops.h"
 #include "pdl.cuh"
 
 namespace {
