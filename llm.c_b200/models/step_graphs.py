@@ -10,10 +10,35 @@ table are compared.  The scratch buffers of the operators are shared by all call
 """
 import contextlib
 import gc
+import threading
 
 import torch
 
 from ..ops import kernels
+
+
+class _NoCollection:
+    """Garbage collection is off while any thread is inside (the switch is the process's, captures are each thread's); the last one out puts back
+    what the first one found."""
+
+    def __init__(self):
+        self._lock, self._inside, self._was_on = threading.Lock(), 0, False
+
+    def __enter__(self):
+        with self._lock:
+            if self._inside == 0:
+                self._was_on = gc.isenabled()
+                gc.disable()
+            self._inside += 1
+
+    def __exit__(self, *exc):
+        with self._lock:
+            self._inside -= 1
+            if self._inside == 0 and self._was_on:
+                gc.enable()
+
+
+_no_collection = _NoCollection()
 
 
 class Inline:
@@ -112,22 +137,16 @@ class StepGraphs:
     def _capture(model, e, fn):
         graph, side = torch.cuda.CUDAGraph(), torch.cuda.Stream(device=model.device)
         before = kernels.launch_count()
-        with torch.cuda.stream(side), kernels.scratch_taken() as scratch:
-            # a collection inside the capture could find a dropped model, and the graphs it held cannot be freed by a thread that captures
-            collects = gc.isenabled()
-            gc.disable()
+        # a collection inside the capture could find a dropped model, and the graphs it held cannot be freed by a thread that captures
+        with torch.cuda.stream(side), kernels.scratch_taken() as scratch, _no_collection:
+            # other threads (watchdog, data loader) may use the device meanwhile
+            graph.capture_begin(capture_error_mode="thread_local")
+            model.step_graphs.side = Side(torch.cuda.Stream(device=model.device))
             try:
-                # other threads (watchdog, data loader) may use the device meanwhile
-                graph.capture_begin(capture_error_mode="thread_local")
-                model.step_graphs.side = Side(torch.cuda.Stream(device=model.device))
-                try:
-                    fn()
-                finally:
-                    model.step_graphs.side = Inline()
-                    graph.capture_end()
+                fn()
             finally:
-                if collects:
-                    gc.enable()
+                model.step_graphs.side = Inline()
+                graph.capture_end()
         e["launches"] = kernels.launch_count() - before
         kernels.count_launches(-e["launches"])                 # captured, not launched
         e["scratch"] = scratch

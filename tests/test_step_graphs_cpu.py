@@ -1,6 +1,9 @@
 """When a micro-step may be replayed: every buffer that its launches read or write is the one they were captured with."""
+import contextlib
 import copy
+import gc
 import pickle
+import threading
 from types import SimpleNamespace
 
 import pytest
@@ -60,3 +63,38 @@ def test_a_model_with_captured_steps_can_be_copied_and_pickled():
         c.forward(tok, tok)
         m.forward(tok, tok)
         assert torch.equal(c.loss(), m.loss())
+
+
+@pytest.mark.parametrize("enabled", [True, False])
+def test_no_collection_in_a_capture_while_another_thread_ends_its_own(monkeypatch, enabled):
+    graph = SimpleNamespace(capture_begin=lambda capture_error_mode: None, capture_end=lambda: None)
+    monkeypatch.setattr(torch.cuda, "CUDAGraph", lambda: graph)
+    monkeypatch.setattr(torch.cuda, "Stream", lambda device: None)
+    monkeypatch.setattr(torch.cuda, "stream", lambda s: contextlib.nullcontext())
+    both_inside, first_out, seen = threading.Barrier(2), threading.Event(), []
+
+    def model():
+        return SimpleNamespace(device=None, step_graphs=step_graphs.StepGraphs())
+
+    def first():
+        step_graphs.StepGraphs._capture(model(), {}, lambda: both_inside.wait(20))
+        first_out.set()
+
+    def second():
+        def launches():
+            both_inside.wait(20)
+            first_out.wait(20)
+            seen.append(gc.isenabled())
+        step_graphs.StepGraphs._capture(model(), {}, launches)
+
+    before = gc.isenabled()
+    try:
+        (gc.enable if enabled else gc.disable)()
+        threads = [threading.Thread(target=f) for f in (first, second)]
+        for t in threads:
+            t.start()
+        for t in threads:
+            t.join()
+        assert seen == [False] and gc.isenabled() == enabled
+    finally:
+        (gc.enable if before else gc.disable)()
