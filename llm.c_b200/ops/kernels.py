@@ -133,6 +133,17 @@ def _swapped(M, N, K, device):
     return K < 6144 or split > 64 or (split > 32 and M > 384)
 
 
+def _wgrad_two_sm(tiles256, K, accumulate, device):
+    """Whether a weight gradient over K rows goes to the two-SM kernel.  Over few rows it is mostly its output: where 256 x 256 tiles leave half of the
+    CTA pairs idle, narrower tiles of single SMs keep more of them busy (us on pairs, single SMs in brackets: 2304 x 768 x 256 7.4 (6.2), x 1024 13.3
+    (10.0), 3072 x 768 x 256 7.5 (6.4); with more tiles 1600 x 1600 x 256 7.6 (9.0), 3072 x 1024 x 1024 11.4 (12.8), 4096 x 1024 x 64 7.1 (7.3)).  Where it
+    adds to what is there the pairs fetch that by TMA before the sum is ready, single SMs a row per thread in the epilogue (2304 x 768 x 256 8.0
+    (10.6), 1600 x 1600 x 256 8.3 (15.8))."""
+    if tiles256 < 8:
+        return False
+    return K > 1024 or bool(accumulate) or tiles256 * 4 > sm_count(device)
+
+
 FORWARD_GEMM, FORWARD_GEMM2, FORWARD_STREAM, FORWARD_SWAPPED = range(4)        # csrc/decoder.cu, Product
 
 
@@ -166,9 +177,7 @@ def gemm(a, b, d, M, N, K, lda, ldb, ldd, a_mn, b_mn, mode, bias=None, aux=None,
         return
     tiles256 = ((M + 255) // 256) * ((N + 255) // 256)
     if mode == MODE_ACCUM:
-        # a weight gradient over few rows is mostly its output: 256 x 256 tiles leave the pairs idle that narrower tiles of single SMs keep busy
-        # (2304 x 768 x 256 7.0 against 5.9 us, x 1024 13.7 against 9.9; 50304 x 768 x 256 has 591 tiles: 36 against 52)
-        two_sm = TWO_SM_MIN_TILES > 0 and a_mn and b_mn and tiles256 >= 8 and (K > 1024 or tiles256 >= TWO_SM_MIN_TILES)
+        two_sm = TWO_SM_MIN_TILES > 0 and a_mn and b_mn and _wgrad_two_sm(tiles256, K, accumulate, d.device)
         if not two_sm and K <= 1024:
             splits = 1
     else:
