@@ -93,6 +93,7 @@ def cuda():
         "llmc_swiglu_bwd": (I, [P, P, P, L, I, S]),
         "llmc_rope_cache": (I, [P, P, P, P, P, I, I, I, I, I, I, I, I, P, S]),
         "llmc_skinny_gemm": (I, [P, P, P, I, I, I, I, I, I, S]),
+        "llmc_stream_gemm_plan": (None, [I, I, I, I, POINTER(c_int), POINTER(c_int)]),
         "llmc_stream_gemm": (I, [P, P, P, P, I, I, I, I, I, I, I, S]),
         "llmc_stream_gemm_swiglu": (I, [P, P, P, I, I, I, I, I, I, S]),
         "llmc_cached_attention": (I, [P, P, P, P, I, I, I, I, I, I, I, P, P, S]),

@@ -379,18 +379,46 @@ int pick_split(int tiles, int num_kb, int nb, int sms) {
     return s;
 }
 
-// Input gradients of more than 128 rows: row tiles of 64 rows and more, as many as leave room for four slices of K each.  What a CTA waits for is its own
-// loads (128 + rows per k-block) and its share of the reduction, and both shrink with the tile.  Rows x slices, us, in a chain (M x N x K):
-// 256 x 768 x 768 256x4 9.3, 128x4 6.4, 64x4 5.0; 256 x 768 x 2304 11.4, 8.5, 7.1 (64x8 7.4); 256 x 768 x 3072 12.5, 9.5, 8.2 (64x8 7.9);
-// 512 x 1024 x 4096 14.2, 11.9, 12.0; 1024 x 768 x 3072 13.3, 12.5, 96x4 11.7, 64x4 in two rounds 18.0.
-void pick_rows_and_split(int M, int tiles, int num_kb, int sms, int& mtiles, int& S) {
+// How a product is cut: row tiles of nb rows, K in S slices.
+struct Plan { int nb, mtiles, S; };
+int rows_of(int M, int mtiles) { return (CEIL_DIV(M, mtiles) + 15) & ~15; }       // M spread evenly over its tiles
+
+Plan wide_plan(int M, int tiles, int num_kb, int sms) {
+    const int nb = rows_of(M, CEIL_DIV(M, MAX_NB)), mtiles = CEIL_DIV(M, nb);
+    return {nb, mtiles, pick_split(tiles * mtiles, num_kb, nb, sms)};
+}
+
+// Input gradients of more than 128 rows: tiles of about 64 rows (48 at M = 129) or more, as many as leave room for four slices of K each, or as few as
+// the 256 rows of a tile allow.  With the small ones a CTA's share of the reduction and its set-up are short; with the large ones fewer CTAs read the same
+// weights and K can be cut into more slices.  So shallow products take the small ones and deep ones the large ones.  Estimated in ns from the k-blocks of
+// a slice and the rows of a tile, coefficients fitted to 536 products (M 129 to 1024, N 384 to 4096, K 768 to 128256, each way of cutting), 5 and 8 %
+// rms off; the way taken is at most 9 % behind the other, by more than 3 % in 16 of them.  CTAs of small tiles take longer where two share an SM; 13 clusters of 8 large tiles fit
+// the chip at once, 16 do not.  us, small / large tiles: 256 x 768 x 768 5.0 / 9.3, 256 x 768 x 3072 7.9 / 12.5, 1024 x 768 x 3072 11.7 / 13.3,
+// 384 x 768 x 6144 14.9 / 13.1, 256 x 1600 x 14336 27.5 / 21.9, 512 x 2048 x 14336 33 / 31, 384 x 768 x 50304 79 / 43, 512 x 2048 x 128256 304 / 245,
+// but 256 x 2048 x 14336 28 / 40 (16 clusters of 8).
+Plan gradient_plan(int M, int tiles, int num_kb, int sms) {
     const int slots = 2 * (sms * 7 / 8);
+    const Plan wide = wide_plan(M, tiles, num_kb, sms);
     int t = CEIL_DIV(M, 64);
     while (t > 1 && tiles * t * 4 > slots) t--;
-    mtiles = t; S = 0;
-    if (CEIL_DIV(M, t) > 128) { mtiles = CEIL_DIV(M, MAX_NB); return; }      // wide tiles: pick_split
-    for (S = 1; S < 4 && num_kb >= S * 2 * 3; ) S *= 2;
+    if (CEIL_DIV(M, t) > 128) return wide;
+    int S = 1;
+    while (S < 4 && num_kb >= S * 2 * 3) S *= 2;
     if (S == 4 && tiles * t * 8 <= slots && num_kb >= 48) S = 8;
+    Plan narrow = {rows_of(M, t), 0, S};
+    narrow.mtiles = CEIL_DIV(M, narrow.nb);
+    const long long kb_n = CEIL_DIV(num_kb, S), kb_w = CEIL_DIV(num_kb, wide.S);
+    const bool shared_sms = tiles * narrow.mtiles * S > sms * 7 / 8;
+    const long long cost_n = kb_n * (295 + (shared_sms ? 63 + narrow.nb * 87 / 100 : 0)) + 44 * narrow.nb + 2300;
+    const int rounds = wide.S == 8 && tiles * wide.mtiles * 10 > sms ? 2 : 1;
+    const long long cost_w = rounds * (kb_w * (297 + wide.nb * 31 / 100) + 24 * wide.nb + 4200);
+    return cost_n <= cost_w ? narrow : wide;
+}
+
+Plan make_plan(int M, int N, int K, bool swiglu, bool w_mn) {
+    int sms = llmc_device_sm_count(); if (sms <= 0) sms = 148;
+    const int tiles = CEIL_DIV(N, swiglu ? WR / 2 : WR), num_kb = CEIL_DIV(K, BK);
+    return w_mn && M > 128 ? gradient_plan(M, tiles, num_kb, sms) : wide_plan(M, tiles, num_kb, sms);
 }
 
 template <int MODE, bool W_MN>
@@ -400,12 +428,10 @@ int launch_stream(bf16* out, const bf16* x, const bf16* w, const bf16* bias, int
     Args g;
     g.early_w = early_w;
     g.out = out; g.bias = bias; g.w = w; g.M = M; g.N = N; g.K = K; g.ldo = ldo; g.ldw = ldw;
+    const Plan plan = make_plan(M, N, K, MODE == SWIGLU, W_MN);
+    const int tiles = CEIL_DIV(N, MODE == SWIGLU ? WR / 2 : WR), mtiles = plan.mtiles, S = plan.S;
     int sms = llmc_device_sm_count(); if (sms <= 0) sms = 148;
-    const int tiles = CEIL_DIV(N, MODE == SWIGLU ? WR / 2 : WR);
-    int mtiles = CEIL_DIV(M, MAX_NB), S = 0;
-    if (W_MN && M > 128) pick_rows_and_split(M, tiles, CEIL_DIV(K, BK), sms, mtiles, S);
-    g.nb = (CEIL_DIV(M, mtiles) + 15) & ~15;             // M spread evenly over its tiles
-    mtiles = CEIL_DIV(M, g.nb);
+    g.nb = plan.nb;
     g.num_kb = CEIL_DIV(K, BK);
     const int stage_bytes = W_BYTES + g.nb * (BK * 2);
     const bool two = g.nb <= 128;
@@ -437,7 +463,6 @@ int launch_stream(bf16* out, const bf16* x, const bf16* w, const bf16* bias, int
         CUDA_CHECK(launch_pdl(stream_wide_kernel, dim3(2 * sms), dim3(THREADS), smem, stream, 0, tmW, tmX, g));
         return 0;
     }
-    if (S == 0) S = pick_split(tiles * mtiles, g.num_kb, g.nb, sms);
     g.kb_per_split = CEIL_DIV(g.num_kb, S);
     const int smem = g.stages * stage_bytes + 1024 + 256;
     static bool configured = false;
@@ -450,6 +475,12 @@ int launch_stream(bf16* out, const bf16* x, const bf16* w, const bf16* bias, int
 }
 
 }  // namespace
+
+// How a plain product of these sizes is cut
+extern "C" void llmc_stream_gemm_plan(int M, int N, int K, int w_mn, int* rows, int* slices) {
+    const Plan p = make_plan(M, N, K, false, w_mn != 0);
+    *rows = p.nb; *slices = p.S;
+}
 
 // out (M, N) = x (M, K) . w (N, K)^T (+ bias), or x . w (K, N) with w_mn.  K, the row strides of x and w and, with w_mn, N are multiples of 8.
 extern "C" int llmc_stream_gemm(bf16* out, const bf16* x, const bf16* w, const bf16* bias, int M, int N, int K, int ldx, int ldw, int ldo, int w_mn,

@@ -1,4 +1,4 @@
-"""Input gradients of some hundred rows through the split-K kernel (csrc/stream_gemm.cu): row tiles of 64 rows and more, two, four and eight slices of K, ragged
+"""Input gradients of some hundred rows through the split-K kernel (csrc/stream_gemm.cu): row tiles of 48 to 128 rows and, for deep products, of up to 256, two, four and eight slices of K, ragged
 rows, columns and depths, and either side of the line where the dispatch takes it."""
 import pytest
 import torch
@@ -10,7 +10,7 @@ pytestmark = pytest.mark.gpu
 DEV = "cuda"
 
 
-@pytest.mark.parametrize("M,N,K", [(129, 8, 8), (130, 136, 200), (256, 768, 768), (257, 264, 392), (300, 768, 2304), (400, 2048, 776), (256, 1000, 3080), (1024, 768, 3072),
+@pytest.mark.parametrize("M,N,K", [(129, 8, 8), (130, 136, 200), (256, 768, 768), (257, 264, 392), (300, 768, 2304), (400, 2048, 776), (256, 1000, 3080), (1024, 768, 3072), (384, 768, 6152), (200, 1600, 8200),
                                    (500, 2056, 768), (1000, 2048, 768)])
 def test_product(M, N, K):
     g = torch.Generator().manual_seed(M + N + K)
