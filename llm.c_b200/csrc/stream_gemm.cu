@@ -141,6 +141,7 @@ stream_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
             tma_load_2d(dst, &tmW, &full[st], kb * BK, n0);                                   // box {64 k, 128 rows}
         }
     };
+    auto load_x = [&](int kb, int st) { tma_load_2d(smem + st * stage_bytes + W_BYTES, &tmX, &full[st], kb * BK, m0); };       // box {64 k, nb rows}
     const int early = g.early_w ? min(g.stages, kb1 - kb0) : 0;       // stages filled with weights while the kernel before drains
     if (warp == 0 && lane == 0)
         for (int it = 0; it < early; it++) load_w(kb0 + it, it);
@@ -150,13 +151,12 @@ stream_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
 
     if (warp == 0) {
         if (lane == 0) {
-            for (int kb = kb0; kb < kb1; kb++) {
+            for (int it = 0; it < early; it++) load_x(kb0 + it, it);
+            for (int kb = kb0 + early; kb < kb1; kb++) {
                 const int it = kb - kb0, st = it % g.stages;
-                if (it >= early) {
-                    if (!mbar_wait_relaxed(&empty[st], ((it / g.stages) & 1) ^ 1, abort_flag, g.status, 0x900)) break;
-                    load_w(kb, st);
-                }
-                tma_load_2d(smem + st * stage_bytes + W_BYTES, &tmX, &full[st], kb * BK, m0);         // box {64 k, nb rows}
+                if (!mbar_wait_relaxed(&empty[st], ((it / g.stages) & 1) ^ 1, abort_flag, g.status, 0x900)) break;
+                load_w(kb, st);
+                load_x(kb, st);
             }
         }
     } else if (warp == 1) {
