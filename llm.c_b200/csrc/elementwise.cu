@@ -119,7 +119,12 @@ bias_grad_few_kernel(bf16* __restrict__ dbias, const bf16* __restrict__ dout, in
     const int oc = blockIdx.x * 32 + c;
     if (part == 0 && oc < OC) dbias[oc] = __float2bfloat16_rn(accumulate ? s + __bfloat162float(dbias[oc]) : s);
 }
-constexpr int BG_FEW_ROWS = 1024;
+// Its lines: the sums of 1024 rows still take less than a second launch; its CTAs read 64 bytes of a row at a time, which beyond about 80 MB no longer come
+// from L2 (us, two launches in brackets: 1024 x 2304 4.6 (5.6), 1024 x 28672 7.7 (13.8), 777 x 50304 14.1 (15.2), 1024 x 50304 24.8 (18.7), 384 x 128256
+// 22.9 (18.3)); and of a few thousand CTAs each has little to do (1 x 128256 5.5 (3.1)).
+constexpr int BG_FEW_ROWS = 1024, BG_FEW_COLS = 65536;
+constexpr long long BG_FEW_VALUES = 40ll << 20;
+bool bg_few(int rows, int OC) { return rows <= BG_FEW_ROWS && OC <= BG_FEW_COLS && (long long)rows * OC <= BG_FEW_VALUES; }
 
 int bg_strips(int rows, int OC) {
     int sms = llmc_device_sm_count(); if (sms <= 0) sms = 148;
@@ -147,11 +152,11 @@ extern "C" int llmc_residual_add(bf16* out, const bf16* a, const bf16* b, long l
     CUDA_CHECK(launch_pdl(residual_add_kernel, dim3((unsigned)CEIL_DIV(n / 8, 256)), dim3(256), 0, stream, 0, out, a, b, n / 8));
     return 0;
 }
-extern "C" long long llmc_bias_grad_scratch(int rows, int OC) { return rows <= BG_FEW_ROWS ? 0 : (long long)bg_strips(rows, OC) * OC; }
+extern "C" long long llmc_bias_grad_scratch(int rows, int OC) { return bg_few(rows, OC) ? 0 : (long long)bg_strips(rows, OC) * OC; }
 // dbias[c] (+)= sum_r dout[r, c]; scratch: llmc_bias_grad_scratch floats (none for few rows)
 extern "C" int llmc_bias_grad(bf16* dbias, float* scratch, const bf16* dout, int rows, int OC, int accumulate, cudaStream_t stream) {
     if (OC % 8) return -1;
-    if (rows <= BG_FEW_ROWS) {
+    if (bg_few(rows, OC)) {
         CUDA_CHECK(launch_pdl(bias_grad_few_kernel, dim3(CEIL_DIV(OC, 32)), dim3(4 * BGF_SLOTS), 0, stream, 0, dbias, dout, rows, OC, accumulate));
         return 0;
     }

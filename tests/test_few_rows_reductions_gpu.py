@@ -25,6 +25,15 @@ def test_bias_grad(rows, OC, accumulate):
     assert (buf[OC:] == 7.0).all()
 
 
+@pytest.mark.parametrize("rows,OC", [(3, 65536), (3, 65544), (834, 50304), (833, 50304)])
+def test_bias_grad_of_wide_outputs(rows, OC):
+    g = torch.Generator(device=DEV).manual_seed(rows + OC)
+    d, out = torch.randn(rows, OC, generator=g, device=DEV).bfloat16(), torch.full((OC + 8,), 7.0, dtype=torch.bfloat16, device=DEV)
+    KN.bias_grad(out[:OC], d, accumulate=False)
+    want = d.double().sum(0)
+    assert not ((out[:OC].double() - want).abs() > 1e-3 + want.abs() * 2 ** -8).any() and (out[OC:] == 7.0).all()
+
+
 def test_layernorm_backward_in_two_streams():
     N, C = 300, 384
     g = torch.Generator(device=DEV).manual_seed(1)
