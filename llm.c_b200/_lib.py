@@ -62,6 +62,7 @@ def cuda():
         "llmc_alloc_device_or_managed": (I, [POINTER(c_void_p), ctypes.c_size_t, I, POINTER(c_int)]),
         "llmc_free_device_or_managed": (I, [P]),
         "llmc_gemm": (I, [P, P, P, P, P, I, I, I, I, I, I, I, I, I, I, I, P, P, I, S]),
+        "llmc_gemm_pick_width": (I, [I, I, I, I]),
         "llmc_gemm_tiled": (I, [P, P, P, P, P, I, I, I, I, I, I, I, I, I, I, I, P, P, I, I, S]),
         "llmc_gemm2t": (I, [P, P, P, P, I, I, I, I, I, I, I, S]),
         "llmc_gemm2t_swiglu": (I, [P, P, P, I, I, I, I, I, I, I, S]),

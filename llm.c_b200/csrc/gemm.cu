@@ -464,9 +464,12 @@ int launch(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tm
 // arrive: 128 + BN of them) and of an epilogue.  Measured, us per launch with 256 / 128 / 64 columns (M x N x K): 256 x 2304 x 768 8.8 / 7.5 / 6.8,
 // 256 x 3072 x 768 with GELU 11.5 / 9.0 / 7.8, with dGELU 10.6 / 8.2 / 7.3, 256 x 768 x 3072 19.0 / 17.0 / 16.5, 1024 x 2304 x 768 10.0 / 8.3 / 11.0,
 // 896 x 3072 x 2048 18.2 / 23.2 / 31.3; weight gradients 768 x 768 x 256 8.8 / 5.8 / 4.7, 2304 x 768 x 256 8.9 / 5.9 / 6.7.
-int pick_bn(int m_tiles, int N, int num_kb, int sms, int mode) {
+// Of less than 64 rows most of a tile's 128 do not exist and all CTAs read the same few lines of A: more tiles than half the SMs only add readers
+// (4 rows with GELU: 6144 x 4096 25.1 / 23.5 / 29.9, 8192 x 2048 16.3 / 16.3 / 18.2, 14336 x 2048 21.2 / 22.5 / 32.5; 48 rows of an input gradient 14336 x 768 8.1 / 8.7 / 12.2).
+int pick_bn(int M, int m_tiles, int N, int num_kb, int sms, int mode) {
     int best = 256; long long best_cost = -1;
     for (int bn = 256; bn >= 64; bn >>= 1) {
+        if (mode != EPI_ACCUM && M < 64 && bn < 256 && 2 * CEIL_DIV(N, bn) > sms) break;
         const long long waves = CEIL_DIV(m_tiles * CEIL_DIV(N, bn), sms);
         const long long cost = waves * (num_kb * (bn == 256 ? 560 : bn == 128 ? 370 : 290) + (mode == EPI_ACCUM ? 18 : 6) * bn + 600);
         if (best_cost < 0 || cost < best_cost) { best = bn; best_cost = cost; }
@@ -475,6 +478,12 @@ int pick_bn(int m_tiles, int N, int num_kb, int sms, int mode) {
 }
 
 }  // namespace
+
+// Width of the tiles that llmc_gemm takes for a product without split-K
+extern "C" int llmc_gemm_pick_width(int M, int N, int K, int mode) {
+    int sms = llmc_device_sm_count(); if (sms <= 0) sms = 148;
+    return pick_bn(M, CEIL_DIV(M, BM), N, CEIL_DIV(K, BK), sms, mode);
+}
 
 // Number of fp32 workspace elements and counters llmc_gemm needs for a given problem
 extern "C" void llmc_gemm_workspace(int M, int N, int splits, long long* ws_floats, int* num_counters) {
@@ -523,7 +532,7 @@ extern "C" int llmc_gemm_tiled(const bf16* A, const bf16* B, bf16* D, const bf16
     int sms = llmc_device_sm_count(); if (sms <= 0) sms = 148;
     if (max_ctas > 0 && max_ctas < sms) sms = max_ctas;
     if (splits > 1) bn = 256;
-    if (bn == 0) bn = pick_bn(g.num_m_tiles, N, g.num_kb, sms, mode);
+    if (bn == 0) bn = pick_bn(M, g.num_m_tiles, N, g.num_kb, sms, mode);
     if (bn != 64 && bn != 128 && bn != 256) return -1;
     g.num_n_tiles = CEIL_DIV(N, bn);
     if (splits > 1 && (workspace == nullptr || counters == nullptr)) { fprintf(stderr, "[llmc_b200] gemm: split-K needs workspace\n"); return -1; }
