@@ -101,6 +101,8 @@ DEVINL void tmem_st8(uint32_t taddr, const uint32_t* r) {
         ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]) : "memory");
 }
 
+template <int N> struct Groups { static constexpr int value = N; };
+
 // Slots of the query tiles before i: tile k has one per unit g <= min(k, G - 1) that reaches it.
 __host__ __device__ inline int slot_of(int i, int G) { return i <= G ? i * (i + 1) / 2 : G * (G + 1) / 2 + (i - G) * G; }
 
@@ -125,6 +127,11 @@ struct Walk {
     }
 };
 
+// SHORT: one tile of at most 96 queries, whose row sums wait for as many loads as there are queries.  (In one kernel the second loop costs the
+// registers of the first: 5 % of every size.)  us, the other form first: 128 sequences of 16 x 25 heads 107, 79, 64 of 40 x 25 heads 57, 46, 4 of 64 x 12
+// heads 7.7, 7.4.  Three loads save too little of four unless the CTAs have several items each: 128 of 80 x 25 heads 116, 107, 4 of 80 x 12 heads 7.9, 8.4.
+constexpr int SHORT_T = 64, SHORT_T_MANY = 96;
+template <bool SHORT>
 __global__ void __launch_bounds__(THREADS, 1)
 attn_bwd1_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant__ CUtensorMap tmDO,
                  const __grid_constant__ CUtensorMap tmDQKV, const Args a) {
@@ -326,52 +333,103 @@ attn_bwd1_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constan
         // two warps: the LSE in log2 units and delta = sum_d O dO times the scale; queries past the end of the sequence get LSE = +inf, so
         // that their P^T column is zero
         const float log2e = 1.4426950408889634f;
-        const int w0 = (warp - 2) * 64;                 // the warp's queries of the tile
-        bool ok = true;
-        uint32_t t = 0;
-        for (; wk.valid() && ok; wk.next(), t++) {
-            const int tq0 = wk.i * BT + w0;
-            float l[2], d[16];
-            const size_t row = (size_t)wk.bh * a.T + tq0 + lane;
-            #pragma unroll
-            for (int k = 0; k < 2; k++) l[k] = tq0 + k * 32 + lane < a.T ? a.lse[row + k * 32] * log2e : INFINITY;
-            if (a.delta != nullptr) {
-                #pragma unroll
-                for (int k = 0; k < 2; k++) d[k] = tq0 + k * 32 + lane < a.T ? a.delta[row + k * 32] * a.scale : 0.f;
-            } else {
-                // 8 lanes per query, 4 queries per step; no branch around the loads, so that they are on their way at once
-                #pragma unroll
-                for (int part = 0; part < 4; part++) {
-                    bf16x8 o[4], g[4];
+        if constexpr (SHORT) {
+            // at most 96 queries: each warp takes every other group of 16, and none that the sequence does not have
+            auto few = [&](auto groups) {
+                constexpr int NG = decltype(groups)::value;
+                const int w0 = (warp - 2) * 16;
+                bool ok = true;
+                uint32_t t = 0;
+                for (; wk.valid() && ok; wk.next(), t++) {
+                    float l[2], d[16];
                     #pragma unroll
-                    for (int k = 0; k < 4; k++) {
-                        const int tq = min(tq0 + part * 16 + k * 4 + (lane >> 3), a.T - 1);
-                        const size_t at = (((size_t)wk.b * a.T + tq) * a.NH + wk.h) * HS + (lane & 7) * 8;
-                        o[k] = ld128cs(a.out + at); g[k] = ld128(a.dout + at);
+                    for (int k = 0; k < 2; k++) {
+                        const int q = w0 + (2 * k + (lane >> 4)) * 32 + (lane & 15);
+                        l[k] = q < a.T ? a.lse[(size_t)wk.bh * a.T + q] * log2e : INFINITY;
                     }
                     #pragma unroll
-                    for (int k = 0; k < 4; k++) {
-                        float acc = 0.f;
+                    for (int part = 0; part < NG; part++) {
+                        bf16x8 o[4], g[4];
                         #pragma unroll
-                        for (int e = 0; e < 8; e++) acc += __bfloat162float(o[k][e]) * __bfloat162float(g[k][e]);
-                        acc += __shfl_xor_sync(0xffffffffu, acc, 1);
-                        acc += __shfl_xor_sync(0xffffffffu, acc, 2);
-                        acc += __shfl_xor_sync(0xffffffffu, acc, 4);
-                        d[part * 4 + k] = tq0 + part * 16 + k * 4 + (lane >> 3) < a.T ? acc * a.scale : 0.f;
+                        for (int k = 0; k < 4; k++) {
+                            const int q = min(w0 + part * 32 + k * 4 + (lane >> 3), a.T - 1);
+                            const size_t at = (((size_t)wk.b * a.T + q) * a.NH + wk.h) * HS + (lane & 7) * 8;
+                            o[k] = ld128cs(a.out + at); g[k] = ld128(a.dout + at);
+                        }
+                        #pragma unroll
+                        for (int k = 0; k < 4; k++) {
+                            float acc = 0.f;
+                            #pragma unroll
+                            for (int e = 0; e < 8; e++) acc += __bfloat162float(o[k][e]) * __bfloat162float(g[k][e]);
+                            acc += __shfl_xor_sync(0xffffffffu, acc, 1);
+                            acc += __shfl_xor_sync(0xffffffffu, acc, 2);
+                            acc += __shfl_xor_sync(0xffffffffu, acc, 4);
+                            d[part * 4 + k] = w0 + part * 32 + k * 4 + (lane >> 3) < a.T ? acc * a.scale : 0.f;
+                        }
+                    }
+                    #pragma unroll
+                    for (int k = NG * 4; k < 16; k++) d[k] = 0.f;
+                    ok = __all_sync(0xffffffffu, mbar_wait_relaxed(&st_empty[t & 1], ((t >> 1) & 1) ^ 1, abort_flag, a.status, 0x6b0)) != 0;
+                    float* tab = sStat + (t & 1) * (2 * BT) + w0;
+                    #pragma unroll
+                    for (int k = 0; k < 2; k++) tab[(2 * k + (lane >> 4)) * 32 + (lane & 15)] = l[k];
+                    if ((lane & 7) == 0) {
+                        #pragma unroll
+                        for (int k = 0; k < 16; k++) tab[BT + (k >> 2) * 32 + (k & 3) * 4 + (lane >> 3)] = d[k];
+                    }
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&st_full[t & 1]);
+                }
+            };
+            if (a.T <= 32) few(Groups<1>()); else if (a.T <= 64) few(Groups<2>()); else few(Groups<3>());
+        } else {
+            const int w0 = (warp - 2) * 64;                 // the warp's queries of the tile
+            bool ok = true;
+            uint32_t t = 0;
+            for (; wk.valid() && ok; wk.next(), t++) {
+                const int tq0 = wk.i * BT + w0;
+                float l[2], d[16];
+                const size_t row = (size_t)wk.bh * a.T + tq0 + lane;
+                #pragma unroll
+                for (int k = 0; k < 2; k++) l[k] = tq0 + k * 32 + lane < a.T ? a.lse[row + k * 32] * log2e : INFINITY;
+                if (a.delta != nullptr) {
+                    #pragma unroll
+                    for (int k = 0; k < 2; k++) d[k] = tq0 + k * 32 + lane < a.T ? a.delta[row + k * 32] * a.scale : 0.f;
+                } else {
+                    // 8 lanes per query, 4 queries per step; no branch around the loads, so that they are on their way at once
+                    #pragma unroll
+                    for (int part = 0; part < 4; part++) {
+                        bf16x8 o[4], g[4];
+                        #pragma unroll
+                        for (int k = 0; k < 4; k++) {
+                            const int tq = min(tq0 + part * 16 + k * 4 + (lane >> 3), a.T - 1);
+                            const size_t at = (((size_t)wk.b * a.T + tq) * a.NH + wk.h) * HS + (lane & 7) * 8;
+                            o[k] = ld128cs(a.out + at); g[k] = ld128(a.dout + at);
+                        }
+                        #pragma unroll
+                        for (int k = 0; k < 4; k++) {
+                            float acc = 0.f;
+                            #pragma unroll
+                            for (int e = 0; e < 8; e++) acc += __bfloat162float(o[k][e]) * __bfloat162float(g[k][e]);
+                            acc += __shfl_xor_sync(0xffffffffu, acc, 1);
+                            acc += __shfl_xor_sync(0xffffffffu, acc, 2);
+                            acc += __shfl_xor_sync(0xffffffffu, acc, 4);
+                            d[part * 4 + k] = tq0 + part * 16 + k * 4 + (lane >> 3) < a.T ? acc * a.scale : 0.f;
+                        }
                     }
                 }
+                ok = __all_sync(0xffffffffu, mbar_wait_relaxed(&st_empty[t & 1], ((t >> 1) & 1) ^ 1, abort_flag, a.status, 0x6b0)) != 0;
+                float* tab = sStat + (t & 1) * (2 * BT) + w0;
+                tab[lane] = l[0]; tab[32 + lane] = l[1];
+                if (a.delta != nullptr) {
+                    tab[BT + lane] = d[0]; tab[BT + 32 + lane] = d[1];
+                } else if ((lane & 7) == 0) {
+                    #pragma unroll
+                    for (int k = 0; k < 16; k++) tab[BT + k * 4 + (lane >> 3)] = d[k];
+                }
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&st_full[t & 1]);
             }
-            ok = __all_sync(0xffffffffu, mbar_wait_relaxed(&st_empty[t & 1], ((t >> 1) & 1) ^ 1, abort_flag, a.status, 0x6b0)) != 0;
-            float* tab = sStat + (t & 1) * (2 * BT) + w0;
-            tab[lane] = l[0]; tab[32 + lane] = l[1];
-            if (a.delta != nullptr) {
-                tab[BT + lane] = d[0]; tab[BT + 32 + lane] = d[1];
-            } else if ((lane & 7) == 0) {
-                #pragma unroll
-                for (int k = 0; k < 16; k++) tab[BT + k * 4 + (lane >> 3)] = d[k];
-            }
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&st_full[t & 1]);
         }
     } else if (warp < 12) {
         // ---------------------------------------------------------------- softmax: thread = key row r x query half hf
@@ -694,17 +752,19 @@ extern "C" int llmc_attention_bwd(bf16* dqkv, float* ws, const bf16* dout, const
     const int total = B * NH * ((nt + 1) / 2);
     int sms = llmc_device_sm_count(); if (sms <= 0) sms = 148;
     const int grid = total < sms ? total : sms;
-    static bool configured = false;
-    if (!configured) {
-        CUDA_CHECK(cudaFuncSetAttribute(attn_bwd1_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM));
-        configured = true;
+    const bool few = T <= SHORT_T || (T <= SHORT_T_MANY && total > 2 * sms);
+    auto kernel = few ? attn_bwd1_kernel<true> : attn_bwd1_kernel<false>;
+    static bool configured[2] = {false, false};
+    if (!configured[few]) {
+        CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM));
+        configured[few] = true;
     }
     a.early = nt == 1 && grid < sms;       // as in the forward pass; with more tiles the kernels before and after are launched plainly
     if (a.early) {
-        CUDA_CHECK(launch_pdl(attn_bwd1_kernel, dim3(grid), dim3(THREADS), SMEM, stream, 0, tmQKV, tmDO, tmDQKV, a));
+        CUDA_CHECK(launch_pdl(kernel, dim3(grid), dim3(THREADS), SMEM, stream, 0, tmQKV, tmDO, tmDQKV, a));
         return 0;
     }
-    attn_bwd1_kernel<<<grid, THREADS, SMEM, stream>>>(tmQKV, tmDO, tmDQKV, a);
+    kernel<<<grid, THREADS, SMEM, stream>>>(tmQKV, tmDO, tmDQKV, a);
     CUDA_CHECK(cudaGetLastError());
     if (nt == 1) return 0;
     dq_fold_kernel<<<(unsigned)(B * NH * nt), 256, 0, stream>>>(dqkv, dq_ws, B, T, NH, nt);
