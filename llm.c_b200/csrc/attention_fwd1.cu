@@ -11,7 +11,7 @@
 //                (no shared-memory round trip, no proxy fence); O accumulates in tensor memory across the key tiles and is
 //                rescaled by its own row's thread only when the running maximum grows by more than 2^8 (the stale maximum
 //                is a valid reference point for the exponentials in between, the final division by the row sum cancels it).
-//                The two groups take turns at the exponentials (common.cuh, turn_wait), so that one group's run under the other's
+//                In sequences of six tiles and more the two groups take turns at the exponentials (common.cuh, turn_wait), so that one group's run under the other's
 //                loads, maxima and products; without turns they drift into step and compete for the unit (64 x 1024 x 12 heads
 //                233 us instead of 216, 2 x 4096 x 32 258 instead of 240).
 //
@@ -63,6 +63,11 @@ DEVINL void tmem_st16(uint32_t taddr, const uint32_t* r) {
         : "memory");
 }
 
+// TURNS: the slots take turns at the exponentials.  Of sequences of few tiles most work has no partner to take turns with: the last item has one slot when
+// the number of tiles is odd, and slot B's last tile runs alone.  us without / with: 8 x 300 x 12 heads 14.0 / 14.3, 64 x 256 x 12 32.5 / 33.6, 32 x 640 x 12
+// 59.9 / 61.7, but 32 x 768 x 12 73.1 / 71.4, 32 x 1024 x 12 115.1 / 109.6.  (Turns decided per item instead cost 8 % at 1024: a branch in the loop over the tiles.)
+constexpr int TURNS_FROM_TILES = 6;
+template <bool TURNS>
 __global__ void __launch_bounds__(THREADS, 1)
 attn_fwd1_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant__ CUtensorMap tmOut, const Args a) {
     extern __shared__ __align__(1024) uint8_t smem[];
@@ -252,7 +257,7 @@ attn_fwd1_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constan
         const float c = a.scale_log2e;
         bool ok = true;
         bool staged = false;
-        if (x == 1) turn_pass(TURN_BAR + 2 * q4);          // slot A has the first turn
+        if (TURNS && x == 1) turn_pass(TURN_BAR + 2 * q4); // slot A has the first turn
         uint32_t t = 0;                                    // tiles of this slot so far
         int it = 0;
         for (int w = blockIdx.x; w < total; w += gridDim.x, it++) {
@@ -260,7 +265,7 @@ attn_fwd1_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constan
             const int qi = 2 * p + x;                      // this slot's query tile
             const int turns = min(2 * p + 2, nq);          // of either slot in this item
             if (qi >= nq) {                                // (uniform for the slot) no second tile in this item
-                for (int j = 0; j < turns; j++) { turn_wait(TURN_BAR + 2 * q4 + x); turn_pass(TURN_BAR + 2 * q4 + (x ^ 1)); }
+                for (int j = 0; TURNS && j < turns; j++) { turn_wait(TURN_BAR + 2 * q4 + x); turn_pass(TURN_BAR + 2 * q4 + (x ^ 1)); }
                 continue;
             }
             float m = -INFINITY, l = 0.f;                  // reference maximum (raw score units) and row sum relative to it
@@ -303,7 +308,7 @@ attn_fwd1_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constan
                 }
                 if (r == 0) TRACE(1 + x, 3, t);
                 float moff = m * c;
-                turn_wait(TURN_BAR + 2 * q4 + x, moff);
+                if (TURNS) turn_wait(TURN_BAR + 2 * q4 + x, moff);
                 float rs0 = 0.f, rs1 = 0.f;
                 uint32_t pk[64];
                 #pragma unroll
@@ -314,7 +319,7 @@ attn_fwd1_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constan
                     pk[e >> 1] = pack_bf16x2(p0, p1);
                 }
                 l += rs0 + rs1;
-                turn_pass(TURN_BAR + 2 * q4 + (x ^ 1), l);
+                if (TURNS) turn_pass(TURN_BAR + 2 * q4 + (x ^ 1), l);
                 if (r == 0) TRACE(1 + x, 5, t);
                 // the previous product has read P_X(t-1) and finished adding to O_X: only now is it waited for, so that it ran
                 // under the exponentials above
@@ -343,7 +348,7 @@ attn_fwd1_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constan
                 if (lane == 0) mbar_arrive(&p_ready[x]);
                 if (r == 0) TRACE(1 + x, 6, t);
             }
-            if (qi + 1 < turns) { turn_wait(TURN_BAR + 2 * q4 + x); turn_pass(TURN_BAR + 2 * q4 + (x ^ 1)); }      // slot A has a tile less
+            if (TURNS && qi + 1 < turns) { turn_wait(TURN_BAR + 2 * q4 + x); turn_pass(TURN_BAR + 2 * q4 + (x ^ 1)); }      // slot A has a tile less
             // ---- item epilogue: O_X / l -> bf16 tile in the layout of a 128-byte-swizzled TMA box -> one bulk store
             ok = mbar_wait(&pv_done[x], (t - 1) & 1, abort_flag, a.status, 0x528 + x) && ok;
             tc_fence_after();
@@ -378,7 +383,7 @@ attn_fwd1_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constan
             const int trow = qi * BT + r;
             if (trow < a.T && ok) a.lse[((size_t)b * a.NH + h) * a.T + trow] = m * a.scale + logf(l);
         }
-        if (x == 0) turn_wait(TURN_BAR + 2 * q4);          // the last turn passed on by slot B
+        if (TURNS && x == 0) turn_wait(TURN_BAR + 2 * q4); // the last turn passed on by slot B
         if (issuer) tma_store_wait<0>();
     }
     tc_fence_before();
@@ -422,19 +427,21 @@ extern "C" int llmc_attention_fwd(bf16* out, float* lse, const bf16* qkv, int B,
     const int total = B * NH * ((nq + 1) / 2);
     int sms = llmc_device_sm_count(); if (sms <= 0) sms = 148;
     const int grid = total < sms ? total : sms;
-    static bool configured = false;
-    if (!configured) {
-        CUDA_CHECK(cudaFuncSetAttribute(attn_fwd1_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM));
-        configured = true;
+    const bool turns = nq >= TURNS_FROM_TILES;
+    auto kernel = turns ? attn_fwd1_kernel<true> : attn_fwd1_kernel<false>;
+    static bool configured[2] = {false, false};
+    if (!configured[turns]) {
+        CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM));
+        configured[turns] = true;
     }
     // early launch (pdl.cuh) only where SMs stay free: 4 x 64 GPT-2 step 1566 -> 1513 us; otherwise the blocks of the next kernel sit beside
     // this one's for all of its run: 64 x 1024 x 12 938 -> 986 us
     a.early = grid < sms;
     if (a.early) {
-        CUDA_CHECK(launch_pdl(attn_fwd1_kernel, dim3(grid), dim3(THREADS), SMEM, stream, 0, tmQKV, tmOut, a));
+        CUDA_CHECK(launch_pdl(kernel, dim3(grid), dim3(THREADS), SMEM, stream, 0, tmQKV, tmOut, a));
         return 0;
     }
-    attn_fwd1_kernel<<<grid, THREADS, SMEM, stream>>>(tmQKV, tmOut, a);
+    kernel<<<grid, THREADS, SMEM, stream>>>(tmQKV, tmOut, a);
     CUDA_CHECK(cudaGetLastError());
     return 0;
 }
