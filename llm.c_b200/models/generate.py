@@ -6,11 +6,11 @@ part of every row is forced, each step runs only the tokens that are new since t
 sampling is nucleus (top-p) at a temperature, or greedy at temperature 0.
 
 The decoder works on the parameter tensors of a ``models.llama3.Llama`` (it never copies them), with its own small activation
-set and the caches ``(L, max_batch, max_len, NKV, HS)``.  On a GPU every step is a chain of this library's kernels: the GEMMs
-of training for prompts (rows padded to whole 128-row tiles) or split-K weight streaming for steps of at most 128 rows (csrc/stream_gemm.cu,
-SwiGLU in its epilogue), RMSNorm, and the two decoding kernels of csrc/decode.cu (rotary
-embedding written straight into the cache; attention of the new queries over the cached keys with grouped heads read in
-place).  A one-token step issues about nine small launches per layer and is bound by launch latency, so on a GPU it is
+set and the caches ``(L, max_batch, max_len, NKV, HS)``.  On a GPU every step is a chain of this library's kernels, for a bf16 model issued
+from native code (csrc/decoder.cu) on exactly the rows that there are: products in row tiles that fit a prompt (csrc/gemm2t.cu) or split-K weight
+streaming for steps of at most 128 rows (csrc/stream_gemm.cu), either with SwiGLU in its epilogue, RMSNorm, and the training attention kernel for whole
+prompts or the two decoding kernels of csrc/decode.cu (rotary embedding written straight into the cache; attention of the new queries over the cached keys
+with grouped heads read in place).  An fp32 model, or one whose layers do not lie at equal distances, takes the operators one by one.  A one-token step issues about nine small launches per layer and is bound by launch latency, so on a GPU it is
 captured once in a CUDA graph and replayed (``GraphStep``): the position lives in device memory, the graph advances it itself,
 and the kernels refuse a position outside the cache through the library's status word.  On the CPU the same chain runs on
 the fp32 restatement of the operators.
@@ -41,18 +41,19 @@ class CachedDecoder:
         self._dense = None
         # prompts of at least this many tokens per row, starting at position 0, run through the training attention kernel
         self.dense_prefill_from = 128
-        # products run on rows padded to whole 128-row tiles
+        # a bf16 model's pass is issued from native code; without it, with another line for exact rows than the kernels' own (skinny_rows), or
+        # where its layout does not allow that, operator by operator
+        self.native = model.device.type == "cuda" and model.dtype == torch.bfloat16
+        # operator by operator: steps of at most this many rows run their products on exactly their rows (0: never), larger ones on rows padded to
+        # whole 128-row tiles
+        self.skinny_rows = kernels.STREAM_MAX_ROWS if self.native else 0
         self.whole_tiles = model.device.type == "cuda"
-        # steps of at most this many rows run their products on exactly their rows (split-K weight streaming, csrc/stream_gemm.cu), the MLP's
-        # up-projections with the activation in the same launch, instead of on rows padded to whole 128-row tiles (0: never)
-        self.skinny_rows = kernels.STREAM_MAX_ROWS if model.device.type == "cuda" and model.dtype == torch.bfloat16 else 0
 
     def cache_bytes(self):
         return 2 * self.kcache.numel() * self.kcache.element_size()
 
     def _buffers(self, N, B):
-        """Activation rows are padded to a multiple of 128 so that every product is made of whole tiles; the rows beyond N
-        stay zero and are never read back.  The rows of the last positions (``last``, ``logits``) grow with the batch on their own."""
+        """Activation rows are a multiple of 128, for the products that run on whole tiles; the rows beyond N are never read back.  The rows of the last positions (``last``, ``logits``) grow with the batch on their own."""
         rows, last_rows = _whole_tiles(max(N, B)), _whole_tiles(B)
         m, cfg = self.model, self.model.cfg
         C, H, Vp = cfg.channels, cfg.hidden_dim, cfg.padded_vocab_size
@@ -92,7 +93,7 @@ class CachedDecoder:
                 self._dense = (torch.zeros(rows, 3 * C, dtype=m.dtype, device=m.device),
                                torch.zeros(B * NH * Tq, dtype=torch.float32, device=m.device))
             packed, lse = self._dense[0][:N], self._dense[1][:B * NH * Tq].view(B, NH, Tq)
-        if self.skinny_rows == kernels.STREAM_MAX_ROWS and kernels.decoder_layout_ok(self):
+        if self.native and self.skinny_rows == kernels.STREAM_MAX_ROWS and kernels.decoder_layout_ok(self):
             kernels.decoder_forward(self, a, (packed, lse) if dense else None, tokens, start_pos, pos)
             return a["logits"][:B, :cfg.vocab_size].float()
 

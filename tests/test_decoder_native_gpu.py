@@ -10,28 +10,29 @@ pytestmark = pytest.mark.gpu
 DEV = torch.device("cuda", 0)
 
 
-# hidden widths 1024 (either fused MLP), 224 (neither) and 576 (the streamed one only)
-@pytest.mark.parametrize("desc", ["llama3:l=2,c=256,h=4,kv=2,t=512,v=500", "llama3:l=2,c=256,h=4,kv=4,t=512,v=500,m=32,f=0.3", "llama3:l=1,c=256,h=2,kv=1,t=512,v=500,m=32,f=0.8"])
-@pytest.mark.parametrize("B,chunks", [(1, [7, 1, 1]), (3, [40, 1, 5]), (2, [70, 3]), (1, [128, 1]), (2, [200, 130]), (130, [2, 1])])
+# hidden widths 1024 (either fused MLP), 224 (neither) and 576 (the streamed one only), channels from which the swapped products start
+@pytest.mark.parametrize("desc", ["llama3:l=2,c=256,h=4,kv=2,t=2048,v=500", "llama3:l=2,c=256,h=4,kv=4,t=2048,v=500,m=32,f=0.3",
+                                  "llama3:l=1,c=256,h=2,kv=1,t=2048,v=500,m=32,f=0.8", "llama3:l=2,c=768,h=12,kv=4,t=2048,v=500"])
+@pytest.mark.parametrize("B,chunks", [(1, [7, 1, 1]), (3, [40, 1, 5]), (2, [70, 3]), (1, [128, 1]), (2, [200, 130]), (130, [2, 1]), (3, [777, 1])])
 def test_same_logits_and_cache(desc, B, chunks):
     m = llama3.Llama(llama3.config_from_descriptor(desc), DEV, torch.bfloat16)
     m.init_random(3)
-    fast, slow = generate.CachedDecoder(m, B, 400), generate.CachedDecoder(m, B, 400)
-    called = []
-    slow.skinny_rows = 127                                    # not the default: the operators one by one
+    # 20 instead of 800 positions for 130 rows: neither is more than a few hundred MB
+    fast, slow = (generate.CachedDecoder(m, B, 800 if B < 100 else 20) for _ in range(2))
+    slow.native, slow.whole_tiles = False, False               # the operators one by one, on exactly the same rows
     g = torch.Generator().manual_seed(1)
     at = 0
     for n in chunks:
         tok = torch.randint(0, 500, (B, n), generator=g, dtype=torch.int32).to(DEV)
         before = KN.launch_count()
         a = fast.forward(tok, at)
-        called.append(KN.launch_count() - before)
+        issued = KN.launch_count() - before
         b = slow.forward(tok, at)
+        assert issued == KN.launch_count() - before - issued
         at += n
-        for x, y in ((a, b), (fast.kcache, slow.kcache), (fast.vcache, slow.vcache)):
-            # the same kernels but for products of exactly 128 rows and row tiles: bf16 roundings of two layers apart
-            assert float((x.float() - y.float()).norm() / y.float().norm()) < 1e-2
-    assert min(called) > 0
+        # the same kernels on the same rows: the same bits
+        assert torch.equal(a, b) and torch.equal(fast.kcache, slow.kcache) and torch.equal(fast.vcache, slow.vcache)
+        assert torch.isfinite(a).all() and a.abs().max() > 0
 
 
 def test_layers_that_lie_apart():
@@ -47,6 +48,5 @@ def test_layers_that_lie_apart():
     weights[:, :-8] = m.params["qkvw"]
     m.params["qkvw"] = weights[:, :-8]
     got = apart.forward(tok, 0)
-    for x, y in ((got, want), (apart.kcache, plain.kcache), (apart.vcache, plain.vcache)):
-        assert float((x.float() - y.float()).norm() / y.float().norm()) < 1e-2
+    assert torch.equal(got, want) and torch.equal(apart.kcache, plain.kcache) and torch.equal(apart.vcache, plain.vcache)
     assert not around[:, 2:].any()

@@ -182,8 +182,7 @@ def test_the_natively_issued_pass_gets_only_layers_at_equal_distances(monkeypatc
     tok = torch.arange(14, dtype=torch.int32).view(2, 7)
     want = G.CachedDecoder(m, 2, 32).forward(tok, 0)
     dec, issued = G.CachedDecoder(m, 2, 32), []
-    dec.skinny_rows = KN.STREAM_MAX_ROWS                       # as for a bf16 model on the GPU
-    dec.whole_tiles = False
+    dec.native, dec.skinny_rows = True, KN.STREAM_MAX_ROWS     # as for a bf16 model on the GPU
     monkeypatch.setattr(KN, "decoder_forward", lambda *a: issued.append(a))
     if what.endswith("cache"):
         setattr(dec, what, spread(getattr(dec, what), 1))
