@@ -53,3 +53,34 @@ def test_replayed_steps_equal_launched_steps(family):
     graphs = [e for e in m.step_graphs._entries.values() if e["graph"] is not None]
     assert graphs
     assert all(len(e["scratch"]) > 0 and not any(t is other for t in e["scratch"]) for k, e in m.step_graphs._entries.items() if k[0] == "backward" and e["graph"])
+
+
+# 256 rows of 768 channels: input gradients in slices of K beside the weight gradients; 1280 rows: bias gradients through a scratch buffer, on the side
+# branch; every recompute level shares other buffers between the layers
+@pytest.mark.parametrize("recompute", [0, 1, 2])
+@pytest.mark.parametrize("B,T,C,L", [(4, 64, 768, 3), (5, 256, 256, 4)])
+@pytest.mark.parametrize("family", ["gpt2", "llama3"])
+def test_both_branches_of_the_backward_pass(family, B, T, C, L, recompute):
+    def build(graphs):
+        if family == "gpt2":
+            m = gpt2.GPT(gpt2.GPTConfig(T, 1000, 1024, L, C // 64, C), DEV, torch.bfloat16, recompute=recompute)
+        else:
+            m = llama3.Llama(llama3.config_from_descriptor("llama3:l=%d,c=%d,h=%d,kv=%d,t=%d,v=1000,m=64,f=1.0" % (L, C, C // 64, C // 128, T)), DEV, torch.bfloat16,
+                             recompute=recompute)
+        m.init_random(3)
+        m.use_graphs = graphs
+        return m
+
+    replayed, launched = build(True), build(False)
+    g = torch.Generator().manual_seed(0)
+    for step in range(8):
+        for micro in range(2):
+            tok = torch.randint(0, 1000, (B, T + 1), generator=g, dtype=torch.int32)
+            x, y = tok[:, :-1].contiguous().to(DEV), tok[:, 1:].contiguous().to(DEV)
+            for m in (replayed, launched):
+                m.forward(x, y, 2, micro)
+                m.backward(micro, micro == 1)
+            assert torch.equal(replayed.grads_flat, launched.grads_flat), (step, micro)
+            assert torch.equal(replayed.acts["dresidual"], launched.acts["dresidual"])
+        assert torch.equal(replayed.loss(2), launched.loss(2)) and torch.isfinite(launched.loss(2))
+    assert sum(e["graph"] is not None for e in replayed.step_graphs._entries.values()) == 4
