@@ -11,6 +11,7 @@
 // Why two passes with S and dP formed twice and not one: with 128 channels a tile pair's dQ contribution is 64 KB of fp32.  Summing
 // these in a fixed order through memory (what attention_bwd1.cu does at 64 channels) would write and read them at the rate of
 // HBM, which takes longer than the two extra products; and dV, dK, dQ and both score tiles together do not fit 512 TMEM columns.
+// Neither holds at 72 and 80 channels (2 x 128 + 3 x 80 = 496 columns, 40 KB a pair): one pass is possible there and is not built.
 //
 // Both passes are bound by the softmax warps (16 exponentials per clock and SM: 1024 cycles for a 128 x 128 tile, plus the TMEM
 // loads and stores around them) with the tensor pipe close behind (2048 / 1536 cycles a pair).  So nothing but that is left to the

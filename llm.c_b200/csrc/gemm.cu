@@ -465,7 +465,8 @@ int launch(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tm
 // 256 x 3072 x 768 with GELU 11.5 / 9.0 / 7.8, with dGELU 10.6 / 8.2 / 7.3, 256 x 768 x 3072 19.0 / 17.0 / 16.5, 1024 x 2304 x 768 10.0 / 8.3 / 11.0,
 // 896 x 3072 x 2048 18.2 / 23.2 / 31.3; weight gradients 768 x 768 x 256 8.8 / 5.8 / 4.7, 2304 x 768 x 256 8.9 / 5.9 / 6.7.
 // Of less than 64 rows most of a tile's 128 do not exist and all CTAs read the same few lines of A: more tiles than half the SMs only add readers
-// (4 rows with GELU: 6144 x 4096 25.1 / 23.5 / 29.9, 8192 x 2048 16.3 / 16.3 / 18.2, 14336 x 2048 21.2 / 22.5 / 32.5; 48 rows of an input gradient 14336 x 768 8.1 / 8.7 / 12.2).
+// (4 rows with GELU: 6144 x 4096 25.1 / 23.5 / 29.9, 8192 x 2048 16.3 / 16.3 / 18.2, 14336 x 2048 21.2 / 22.5 / 32.5; 48 rows of an input gradient
+// 14336 x 768 8.1 / 8.7 / 12.2).
 int pick_bn(int M, int m_tiles, int N, int num_kb, int sms, int mode) {
     int best = 256; long long best_cost = -1;
     for (int bn = 256; bn >= 64; bn >>= 1) {

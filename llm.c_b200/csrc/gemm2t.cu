@@ -7,7 +7,8 @@
 // 256 nb products, so that small nb cost more per product; the rule weighs both.  Measured figures stand with the dispatch (ops/kernels.py, _swapped).
 //
 // SwiGLU: w holds 2 N rows, out = (x . w1^T) * silu(x . w2^T).  Lanes 0..63 of a CTA are rows of w1, lanes 64..127 the same rows of w2; the two warps that
-// hold the factors of an output exchange half of them through shared memory and finish half of the rows each.
+// hold the factors of an output exchange half of them through shared memory and finish half of the rows each.  Unlike the plain product it is taken for
+// any number of rows, since the launch and the pass over the factors that it saves grow with them (ops/kernels.py, decoder_forward).
 //
 // Structure as in gemm2.cu: warp 0 TMA producer, warp 1 MMA issuer (leader CTA), sixteen epilogue warps, double-buffered accumulator.  A tensor memory lane is an
 // output column and a column is a row of the output, so an epilogue warp turns 32 columns x 16 rows round through its own shared memory (one

@@ -10,11 +10,12 @@
 // in the order of the slices: deterministic, no workspace, no second launch.
 //
 // The kernel is launched with programmatic stream serialization: while the kernel before it drains, its CTAs set up and ask for the
-// first kilobyte of each weight row of their slice in L2 (a hint only: nothing is read before the predecessor has completed).
+// first kilobyte of each weight row of their slice in L2 (a hint only).  Behind a kernel that does not write the weights (the chained entry
+// points) they fill their stages with them; nothing else is read before the predecessor has completed.
 //
 // Alone, after an L2 flush, the 128 x 256 tiles of the training GEMM in brackets: 32 x 4096 x 14336 (M x N x K) 36 us (101),
 // 32 x 6144 x 4096 23 us (38), 32 x 28672 x 4096 58 us (69), 100 x 2048 x 7168 23 us (52).  Inside a replayed decoding step (4 rows, 4 layers
-// of 2048 channels, LM head of 128256 rows) this kernel takes the step to 277 us; a weight-streaming kernel on warp-level MMAs with the same
+// of 2048 channels, LM head of 128256 rows) this kernel took the step to 277 us; a weight-streaming kernel on warp-level MMAs with the same
 // early launch and prefetch, used for the products of at most 8 rows, left it at 290 us (at 284 us for the LM head alone), although launched
 // by itself it is faster (4 x 28672 x 4096 50 us against 59; skinny_gemm_kernel in decode.cu).  More rows (input gradients, in a chain, the training GEMM's tiles in
 // brackets): 256 x 768 x 768 4.9 us (6.3), 256 x 768 x 3072 7.9 us (16.3), 256 x 768 x 50304 44 us (291 after an L2 flush).

@@ -2,7 +2,7 @@
 
     ncu --set full --clock-control none -k regex:<kernel> -s <skip> -c <n> -o out python -m llmc_b200.profile_kernels <op>
 
-Cases are larger than the 126 MB L2 but hold well under 2 GB on the device, so a capture ends by itself within a minute
+Cases are larger than the 126 MB L2 (but for those that stand for small micro-steps and prompts) and hold well under 2 GB on the device, so a capture ends by itself within a minute
 or two.  ``python -m llmc_b200.profile_kernels list`` prints the operators.  With ``--time`` the operator is timed
 with CUDA events instead (L2 flushed between iterations) and its achieved bandwidth / FLOP rate is printed.
 (Counterpart of the reference's profile_gpt2.cu / dev/cuda benchmark mains.)
@@ -48,13 +48,30 @@ def case(op):
         d32 = torch.empty(Mt, Nt, device=DEV)
         return (lambda: K.gemm_tf32(d32, a32, b32, bias32)), 4.0 * (Mt * Kt + Nt * Kt + Mt * Nt), 2.0 * Mt * Nt * Kt
     if op == "gemm_fwd_1cta":
-        # a problem with too few 256 x 256 tiles for the two-SM kernel: runs on the single-CTA kernel (128 x 256 tiles)
-        Ms, Ns, Ks = 2048, 2304, 768
+        # too few 256 x 256 tiles for the two-SM kernel and not deep enough for the swapped one: runs on the single-CTA kernel (128 x 256 tiles)
+        Ms, Ns, Ks = 2048, 2304, 704
         a, w, b = _bf(Ms, Ks), _bf(Ns, Ks, scale=0.02), _bf(Ns)
         out = torch.empty(Ms, Ns, device=DEV, dtype=torch.bfloat16)
         return (lambda: K.matmul_forward(out, a, w, b)), 2.0 * (Ms * Ks + Ns * Ks + Ms * Ns), 2.0 * Ms * Ns * Ks
-    if op in ("attn_fwd", "attn_bwd", "attn_fwd_wide", "attn_bwd_wide"):
-        B, T, NH, HS = (16, 2048, 8, 128) if op.endswith("wide") else (16, 1024, 12, 64)
+    if op in ("gemm_gelu_narrow", "gemm_wgrad_narrow", "gemm_dgrad_slices"):
+        # a micro-step of 4 x 64 tokens: 64- and 128-column tiles of the single-CTA kernel, input gradient with K in slices
+        Ms, Ns, Ks = 256, 3072, 768
+        a, w, b, pre, dout = _bf(Ms, Ks), _bf(Ns, Ks, scale=0.02), _bf(Ns), _bf(Ms, Ns), _bf(Ms, Ns)
+        out, dw, dinp = torch.empty(Ms, Ns, device=DEV, dtype=torch.bfloat16), _bf(Ns, Ks), torch.empty(Ms, Ks, device=DEV, dtype=torch.bfloat16)
+        fns = {"gemm_gelu_narrow": (lambda: K.matmul_forward(out, a, w, b, pre_gelu=pre), Ms * Ks + Ns * Ks + 2 * Ms * Ns),
+               "gemm_wgrad_narrow": (lambda: K.matmul_wgrad(dw, dout, a, False), Ms * Ks + Ns * Ks + Ms * Ns),
+               "gemm_dgrad_slices": (lambda: K.matmul_dgrad(dinp, dout, w), Ms * Ks + Ns * Ks + Ms * Ns)}
+        return fns[op][0], 2.0 * fns[op][1], 2.0 * Ms * Ns * Ks
+    if op in ("gemm_swapped", "gemm_swapped_swiglu"):
+        # a prompt of 777 tokens: down-projection, up-projections with activation
+        Ms, Cs, Hs = 777, 2048, 7168
+        x, h, w12, w3 = _bf(Ms, Cs), _bf(Ms, Hs), _bf(2 * Hs, Cs, scale=0.02), _bf(Cs, Hs, scale=0.02)
+        out = torch.empty(Ms, Cs, device=DEV, dtype=torch.bfloat16)
+        if op == "gemm_swapped":
+            return (lambda: K.matmul_forward(out, h, w3, None)), 2.0 * (Ms * Hs + Cs * Hs + Ms * Cs), 2.0 * Ms * Cs * Hs
+        return (lambda: K.matmul_swiglu_prompt(h, x, w12)), 2.0 * (Ms * Cs + 2 * Cs * Hs + Ms * Hs), 4.0 * Ms * Cs * Hs
+    if op in ("attn_fwd", "attn_bwd", "attn_fwd_wide", "attn_bwd_wide", "attn_fwd_short", "attn_bwd_short"):
+        B, T, NH, HS = (16, 2048, 8, 128) if op.endswith("wide") else (64, 64, 25, 64) if op.endswith("short") else (16, 1024, 12, 64)
         qkv, dout = _bf(B, T, 3 * NH * HS), _bf(B, T, NH * HS)
         out = torch.empty(B, T, NH * HS, device=DEV, dtype=torch.bfloat16)
         lse = torch.empty(B, NH, T, device=DEV)
@@ -140,6 +157,10 @@ def case(op):
         if op == "swiglu_fwd":
             return (lambda: K.swiglu_forward(h, x12)), 2.0 * 3 * N * H, 0.0
         return (lambda: K.swiglu_backward(dx12, dh, x12)), 2.0 * 5 * N * H, 0.0
+    if op == "stream_wide":
+        # the LM head of LLaMA-3 over a decoding step of 4 rows (525 MB of weights)
+        x, w, out = _bf(4, 2048), _bf(128256, 2048, scale=0.02), torch.empty(4, 128256, device=DEV, dtype=torch.bfloat16)
+        return (lambda: K.matmul_forward(out, x, w, None)), 2.0 * (128256 * 2048 + 4 * 2048 + 4 * 128256), 8.0 * 128256 * 2048
     if op in ("skinny_gemm", "skinny_gemm_wide", "stream_gemm"):
         # a decoding step of LLaMA-3 8B: 4 rows against the fused MLP up-projection (235 MB of weights) or the QKV projection
         Mr, Kd, Nw = 4, 4096, (6144 * 8 if op == "skinny_gemm_wide" else 28672)
@@ -158,7 +179,8 @@ def case(op):
 
 OPS = ["gemm_fwd", "gemm_gelu", "gemm_dgrad", "gemm_dgelu", "gemm_wgrad", "attn_fwd", "attn_bwd", "attn_fwd_wide", "attn_bwd_wide", "ln_fwd", "fused_residual", "ln_bwd", "ln_bwd_colsum",
        "classifier", "encoder_fwd", "encoder_bwd", "adamw", "norm", "bias_grad", "gelu", "rms_fwd", "rms_fused_residual", "rms_bwd", "rope_fwd",
-       "rope_bwd", "swiglu_fwd", "swiglu_bwd", "gemm_tf32", "gemm_fwd_1cta", "skinny_gemm", "skinny_gemm_wide", "stream_gemm", "cached_attention"]
+       "rope_bwd", "swiglu_fwd", "swiglu_bwd", "gemm_tf32", "gemm_fwd_1cta", "skinny_gemm", "skinny_gemm_wide", "stream_gemm", "cached_attention",
+       "gemm_gelu_narrow", "gemm_wgrad_narrow", "gemm_dgrad_slices", "gemm_swapped", "gemm_swapped_swiglu", "stream_wide", "attn_fwd_short", "attn_bwd_short"]
 
 
 def main(argv):
