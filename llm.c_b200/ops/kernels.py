@@ -124,8 +124,8 @@ def _swapped(M, N, K, device):
     256 x 2304 x 768 6.5 (6.8), 256 x 50304 x 768 25.5 (28.0); 512 x 1152 x 384 5.5 (5.1), 3001 x 28672 x 4096 522 (491).  Above 2048 rows, where a chain
     of products runs at the power limit, the larger loads count: the MLP of 3001 rows of 4096 channels takes 2683 instead of 2663 us with its
     down-projection here, although that alone is faster (267 against 294).
-    Deep products with few tiles are left to the split-K kernel: 300 x 2048 x 7168 33 against 20, 300 x 4096 x 14336 51 against 47, but
-    500 x 4096 x 14336 57 against 60 and 777 x 2048 x 7168 29 against 32."""
+    Deep products with few tiles are left to the split-K kernel: 300 x 2048 x 7168 33 against 20, 300 x 4096 x 14336 51 against 47.  At the line the two
+    are level: 500 x 4096 x 14336 57 to 78 against 60 to 75, 777 x 2048 x 7168 29 to 37 against 32 to 35, whole prompts of 500 to 1024 tokens within 1 %."""
     mt = (M + 255) // 256
     if not (128 < M <= 2048 and K >= 768 and K % 8 == 0 and mt * ((N + 255) // 256) <= 5 * sm_count(device)):
         return False
