@@ -38,7 +38,7 @@
 // reference, which also demands reproducible gradients of cuDNN (llmc/cudnn_att.cpp:186-191).
 #include "common.cuh"
 
-int llmc_attn_qkv_map(CUtensorMap* tm, const bf16* qkv, int B, int T, int NH, int hs);   // attention_fwd.cu
+int llmc_attn_qkv_map(CUtensorMap* tm, const bf16* qkv, int B, int T, int NH, int hs, int rows);   // attention_fwd.cu
 
 namespace {
 
@@ -86,15 +86,6 @@ __global__ void delta_kernel(float* __restrict__ delta, const bf16* __restrict__
     }
 }
 
-DEVINL void tmem_st16(uint32_t taddr, const uint32_t* r) {
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
-        "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
-        ::"r"(taddr),
-          "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
-          "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
-        : "memory");
-}
 DEVINL void tmem_st8(uint32_t taddr, const uint32_t* r) {
     asm volatile(
         "tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
@@ -500,7 +491,7 @@ int llmc_attention_bwd_two_pass(bf16* dqkv, float* delta, const bf16* dout, cons
                                 int B, int T, int NH, int hs, cudaStream_t stream) {
     if (hs <= 64 || hs > 128 || (hs % 8)) { fprintf(stderr, "[llmc_b200] attention backward: head size %d not supported (multiples of 8 from 64 to 128)\n", hs); return -1; }
     CUtensorMap tmQKV, tmDO, tmDQKV;
-    int rc = llmc_attn_qkv_map(&tmQKV, qkv, B, T, NH, hs);
+    int rc = llmc_attn_qkv_map(&tmQKV, qkv, B, T, NH, hs, BT);
     if (rc) return rc;
     {
         uint64_t dims[4] = {(uint64_t)hs, (uint64_t)NH, (uint64_t)T, (uint64_t)B};
@@ -508,7 +499,7 @@ int llmc_attention_bwd_two_pass(bf16* dqkv, float* delta, const bf16* dout, cons
         uint32_t box[4] = {64, 1, 128, 1};
         if ((rc = llmc_get_tensormap(&tmDO, dout, 2, 4, dims, strides, box, 3))) return rc;
     }
-    if ((rc = llmc_attn_qkv_map(&tmDQKV, dqkv, B, T, NH, hs))) return rc;
+    if ((rc = llmc_attn_qkv_map(&tmDQKV, dqkv, B, T, NH, hs, BT))) return rc;
     if ((rc = llmc_attention_delta(delta, out, dout, B, T, NH, hs, stream))) return rc;
     Args a;
     a.lse = lse; a.delta = delta; a.T = T; a.NH = NH; a.BH = B * NH;

@@ -49,7 +49,7 @@
 #include "common.cuh"
 #include "pdl.cuh"
 
-int llmc_attn_qkv_map(CUtensorMap* tm, const bf16* qkv, int B, int T, int NH, int hs);   // attention_fwd.cu
+int llmc_attn_qkv_map(CUtensorMap* tm, const bf16* qkv, int B, int T, int NH, int hs, int rows);   // attention_fwd.cu
 int llmc_attention_bwd_two_pass(bf16* dqkv, float* delta, const bf16* dout, const bf16* qkv, const bf16* out, const float* lse,
                                 int B, int T, int NH, int hs, cudaStream_t stream);      // attention_bwd.cu
 int llmc_attention_delta(float* delta, const bf16* out, const bf16* dout, int B, int T, int NH, int hs, cudaStream_t stream);
@@ -86,15 +86,6 @@ struct Args {
 };
 constexpr int TRACE_PAIRS = 64;
 
-DEVINL void tmem_st16(uint32_t taddr, const uint32_t* r) {
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
-        "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
-        ::"r"(taddr),
-          "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
-          "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
-        : "memory");
-}
 DEVINL void tmem_st8(uint32_t taddr, const uint32_t* r) {
     asm volatile(
         "tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
@@ -731,7 +722,7 @@ extern "C" int llmc_attention_bwd(bf16* dqkv, float* ws, const bf16* dout, const
     float* delta = ws;
     float* dq_ws = ws + ((((long long)B * NH * T) + 63) & ~63ll);
     CUtensorMap tmQKV, tmDO, tmDQKV;
-    int rc = llmc_attn_qkv_map(&tmQKV, qkv, B, T, NH, hs);
+    int rc = llmc_attn_qkv_map(&tmQKV, qkv, B, T, NH, hs, BT);
     if (rc) return rc;
     {
         uint64_t dims[4] = {(uint64_t)hs, (uint64_t)NH, (uint64_t)T, (uint64_t)B};
@@ -739,7 +730,7 @@ extern "C" int llmc_attention_bwd(bf16* dqkv, float* ws, const bf16* dout, const
         uint32_t box[4] = {64, 1, 128, 1};
         if ((rc = llmc_get_tensormap(&tmDO, dout, 2, 4, dims, strides, box, 3))) return rc;
     }
-    if ((rc = llmc_attn_qkv_map(&tmDQKV, dqkv, B, T, NH, hs))) return rc;
+    if ((rc = llmc_attn_qkv_map(&tmDQKV, dqkv, B, T, NH, hs, BT))) return rc;
     const int nt = CEIL_DIV(T, BT);
     // one tile per sequence: delta and the finished dQ come from the same launch (4 x 64 x 12 heads 19.5 -> 13.4 us)
     if (nt > 1 && (rc = llmc_attention_delta(delta, out, dout, B, T, NH, hs, stream))) return rc;

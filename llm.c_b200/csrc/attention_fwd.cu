@@ -46,16 +46,6 @@ struct Args {
     unsigned int* status;
 };
 
-DEVINL void tmem_st16(uint32_t taddr, const uint32_t* r) {
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
-        "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
-        ::"r"(taddr),
-          "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
-          "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
-        : "memory");
-}
-
 // The items of one CTA: query-tile pair p of a head, late (heavy) pairs first.
 struct Items {
     int round, cta, grid, total, BH, np, NH, nq;
@@ -370,11 +360,11 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
 
 }  // namespace
 
-// Tensor map over a packed (B, T, 3, NH, HS) tensor seen as 4-D {HS, 3*NH, T, B} with a 128-row box.
-int llmc_attn_qkv_map(CUtensorMap* tm, const bf16* qkv, int B, int T, int NH, int hs) {
+// Tensor map over a packed (B, T, 3, NH, HS) tensor seen as 4-D {HS, 3*NH, T, B} with a box of `rows` rows.
+int llmc_attn_qkv_map(CUtensorMap* tm, const bf16* qkv, int B, int T, int NH, int hs, int rows) {
     uint64_t dims[4] = {(uint64_t)hs, (uint64_t)(3 * NH), (uint64_t)T, (uint64_t)B};
     uint64_t strides[4] = {2, (uint64_t)hs * 2, (uint64_t)3 * NH * hs * 2, (uint64_t)T * 3 * NH * hs * 2};
-    uint32_t box[4] = {64, 1, 128, 1};
+    uint32_t box[4] = {64, 1, (uint32_t)rows, 1};
     return llmc_get_tensormap(tm, qkv, 2, 4, dims, strides, box, 3);
 }
 
@@ -383,7 +373,7 @@ int llmc_attn_qkv_map(CUtensorMap* tm, const bf16* qkv, int B, int T, int NH, in
 int llmc_attention_fwd_general(bf16* out, float* lse, const bf16* qkv, int B, int T, int NH, int hs, cudaStream_t stream) {
     if (hs <= 64 || hs > 128 || (hs % 8)) { fprintf(stderr, "[llmc_b200] attention: head size %d not supported (multiples of 8 from 64 to 128)\n", hs); return -1; }
     CUtensorMap tmQKV, tmOut;
-    int rc = llmc_attn_qkv_map(&tmQKV, qkv, B, T, NH, hs);
+    int rc = llmc_attn_qkv_map(&tmQKV, qkv, B, T, NH, hs, BT);
     if (rc) return rc;
     {
         uint64_t dims[4] = {(uint64_t)hs, (uint64_t)NH, (uint64_t)T, (uint64_t)B};

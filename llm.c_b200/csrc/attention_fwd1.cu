@@ -1,21 +1,33 @@
 // Causal flash attention forward for sm_100a, head size 64, on the packed (B, T, 3, NH, HS) QKV layout.
 //
-// A CTA works on TWO adjacent 128-row query tiles (A = 2p, B = 2p + 1) of one (batch, head) at a time and streams the key /
-// value tiles 0..2p+1 past both (B takes one tile more than A), so every K / V tile is loaded once for 256 queries.
+// A CTA works on TWO adjacent 128-row query tiles (slots A = 2p, B = 2p + 1) of one (batch, head) at a time and streams key / value tiles of 64 rows
+// past both, so every K / V tile is loaded once for 256 queries.  TWO CTAs share an SM.
 //
-//   warp 0       TMA producer: the two Q tiles of an item (double buffered across items), then K_j, V_j through a 3-stage ring.
-//   warp 1       issuer of S_X = Q_X K_j^T (SS) and O_X += P_X V_j (TS: A = P_X in tensor memory), X in {A, B}; the warp runs in
-//                uniform control flow with one elected lane executing the tcgen05 instructions.
-//   warps 4-7    softmax of tile A, warps 8-11 softmax of tile B: ONE THREAD PER QUERY ROW holding the row's 128 scores in
+//   warp 0       TMA producer: the Q tiles of an item, each loaded again as soon as its slot's last score product is done, and K_0 V_0 K_1 V_1 ... through
+//                a ring of six.
+//   warps 1, 2   issuers of S_X = Q_X K_j^T (SS) and O_X += P_X V_j (TS: A = P_X in tensor memory), one warp for each slot X, with one elected lane
+//                executing the tcgen05 instructions.
+//   warps 4-7    softmax of tile A, warps 8-11 softmax of tile B: ONE THREAD PER QUERY ROW holding the row's 64 scores in
 //                registers.  Row maximum and row sum need no exchange between threads; P goes back to tensor memory as bf16
-//                (no shared-memory round trip, no proxy fence); O accumulates in tensor memory across the key tiles and is
+//                (no shared-memory round trip, no proxy fence) over the scores it came from; S_X(j+1) is issued directly behind O_X += P_X(j) V, whose
+//                completion it thereby reports.  O accumulates in tensor memory across the key tiles and is
 //                rescaled by its own row's thread only when the running maximum grows by more than 2^8 (the stale maximum
 //                is a valid reference point for the exponentials in between, the final division by the row sum cancels it).
-//                In sequences of six tiles and more the two groups take turns at the exponentials (common.cuh, turn_wait), so that one group's run under the other's
-//                loads, maxima and products; without turns they drift into step and compete for the unit (64 x 1024 x 12 heads
-//                233 us instead of 216, 2 x 4096 x 32 258 instead of 240).
 //
-// TMEM columns: S_A [0,128)  S_B [128,256)  O_A [256,320)  O_B [320,384)  P_A [384,448)  P_B [448,512)   (P: 128 bf16 per row)
+// A slot is bound by its own chain: scores from tensor memory, maxima, exponentials (8 cycles of the special-function unit a warp), conversion, P back, two
+// products, about 2000 cycles for 64 keys, of which the unit is busy for 450.  So four slots share an SM, each with an issuer of its own (one issuer for both
+// slots took 1200 cycles a step), an item's Q tile arrives under the item before, and its output leaves from its own Q buffer.  Key tiles of 64 and the P-over-S
+// overlay are what lets four slots into tensor memory and two CTAs into shared memory; the softmax loop is short enough for the instruction caches (with
+// 128-column tiles and every branch unrolled a warp waited for instructions longer than for anything else).  A part of the exponentials runs on the
+// FMA pipe (ex2_poly2): one pair of eight in the ordinary kernel (none / one / two: 187 / 178 / 186 us at 64 x 1024 x 12), two in DUO (13.8 / 13.2 us for two
+// and one at 1 x 777 x 32).
+//
+// DUO: where the query tiles are so few that SMs would get one chain only, a CTA works on ONE query tile, its slots on alternate key tiles, and adds the two
+// at the end.  us, with the kernel this one replaces (one CTA of two slots per SM, tiles of 128 keys, slots taking turns at the exponentials) in brackets, B x T x heads:
+// 64 x 1024 x 12 178 (205), 2 x 4096 x 32 197 (226), 64 x 256 x 12 25.7 (32.7), 8 x 1024 x 12 29.4 (34.4); DUO 1 x 777 x 32 13.2 (14.8), 4 x 512 x 12 10.4 (11.2),
+// 3 x 1000 x 16 19.6 (23.3), 1 x 2048 x 25 27.7 (41.3), 1 x 129 x 32 5.9 (7.1).
+//
+// TMEM columns of a CTA: S_A [0,64)  O_A [64,128)  S_B [128,192)  O_B [192,256); P_X: the first 32 columns of S_X (64 bf16 per row)
 //
 // Statistics are written as natural-log LSE per (b, h, t), the layout cuDNN's SDPA uses in the reference
 // (llmc/cudnn_att.cpp:105-113).  Output tiles leave through shared memory and TMA stores (rows past T are clipped).
@@ -26,92 +38,86 @@
 #include "decoder_ops.h"
 #include "pdl.cuh"
 
-int llmc_attn_qkv_map(CUtensorMap* tm, const bf16* qkv, int B, int T, int NH, int hs);   // attention_fwd.cu
+int llmc_attn_qkv_map(CUtensorMap* tm, const bf16* qkv, int B, int T, int NH, int hs, int rows);   // attention_fwd.cu
 int llmc_attention_fwd_general(bf16* out, float* lse, const bf16* qkv, int B, int T, int NH, int hs, cudaStream_t stream);
 
 namespace {
 
-constexpr int BT = 128;
+constexpr int BT = 128;                             // query rows of a tile
+constexpr int KT = 64;                              // keys of a tile
 constexpr int HS = 64;
 constexpr int TILE_BYTES = BT * HS * 2;             // 16 KB: one 128-byte-swizzled TMA box
-constexpr int QBUF = 2;                             // Q pair buffers (current / next item)
-constexpr int KVSTAGES = 3;
-constexpr int THREADS = 384;                        // TMA warp, issuer warp, two idle warps, 2 x 4 softmax warps
-constexpr int TMEM_COLS = 512;
-constexpr int SMEM = QBUF * 2 * TILE_BYTES + KVSTAGES * 2 * TILE_BYTES + 2 * TILE_BYTES + 256;      // Q, K/V ring, two output tiles
-constexpr int TURN_BAR = 3;                         // named barriers 3..10: [scheduler][slot] turns at the exponentials
+constexpr int KV_BYTES = KT * HS * 2;               // 8 KB
+constexpr int PAIRS = 3;                            // K / V tile pairs in flight
+constexpr int RING = 2 * PAIRS;
+constexpr int THREADS = 384;                        // TMA warp, two issuer warps, an idle one, 2 x 4 softmax warps
+constexpr int REGS_LOW = 48, REGS_HIGH = 96;        // of 80 at launch (two CTAs): 4 x 48 + 8 x 96 = 12 x 80
+constexpr int TMEM_COLS = 256;
+constexpr int SMEM = 4 * TILE_BYTES + RING * KV_BYTES + 256;      // two Q / output tiles of each slot, K/V ring
+static_assert(2 * (SMEM + 1024) <= 228 * 1024, "two CTAs share an SM");
 constexpr float RESCALE_LOG2 = 8.0f;                // the running maximum may lag by this much (in log2 units of the scaled scores)
 
 struct Args {
     float* lse;        // (B, NH, T)
-    int B, T, NH;
+    int T, NH, BH;
     float scale_log2e; // (1/sqrt(HS)) * log2(e)
     float scale;
     int early;           // the next kernel may start while this one runs
     unsigned int* status;
-    long long* trace;  // optional: [3 roles][8 events][64 tiles] clock64() stamps of CTA 0 (null in normal runs)
 };
-#define TRACE(role, ev, tt) do { if (a.trace != nullptr && blockIdx.x == 0 && (tt) < 64) a.trace[((role) * 8 + (ev)) * 64 + (tt)] = clock64(); } while (0)
 
-DEVINL void tmem_st16(uint32_t taddr, const uint32_t* r) {
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
-        "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
-        ::"r"(taddr),
-          "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
-          "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
-        : "memory");
-}
+// The items of one CTA.  Ordinarily query-tile pair p of a head, late (heavy) pairs first; the slots take the longer tile of a pair in turn.  DUO: one query
+// tile (p) for both slots, slot 0 with its even key tiles and slot 1 with the odd ones.
+template <bool DUO>
+struct Items {
+    int w, grid, total, BH, np, NH, nq, nk;
+    int p, b, h, flip;
+    DEVINL Items(int cta, int grid_, const Args& a) : w(cta), grid(grid_), BH(a.BH), NH(a.NH) {
+        nq = CEIL_DIV(a.T, BT); nk = CEIL_DIV(a.T, KT); np = DUO ? nq : (nq + 1) >> 1; total = BH * np;
+        p = b = h = flip = 0;
+        if (w < total) item();
+    }
+    DEVINL bool valid() const { return w < total; }
+    DEVINL void item() { const int rank = w / BH, bh = w - rank * BH; p = np - 1 - rank; b = bh / NH; h = bh - b * NH; }
+    DEVINL void next() { w += grid; flip ^= 1; if (w < total) item(); }
+    DEVINL int qtile(int x) const { return DUO ? p : 2 * p + (x ^ flip); }                             // query tile of slot x
+    DEVINL int kv_tiles() const { return min(2 * (DUO ? p : min(2 * p + 1, nq - 1)) + 2, nk); }        // key tiles of the item
+    DEVINL int tiles(int x) const {                                                                    // and of slot x: STEP * i + (DUO ? x : 0)
+        return DUO ? (kv_tiles() + 1 - x) >> 1 : qtile(x) < nq ? min(2 * qtile(x) + 2, nk) : 0;
+    }
+    static constexpr int STEP = DUO ? 2 : 1;
+};
 
-// TURNS: the slots take turns at the exponentials.  Of sequences of few tiles most work has no partner to take turns with: the last item has one slot when
-// the number of tiles is odd, and slot B's last tile runs alone.  us without / with: 8 x 300 x 12 heads 14.0 / 14.3, 64 x 256 x 12 32.5 / 33.6, 32 x 640 x 12
-// 59.9 / 61.7, but 32 x 768 x 12 73.1 / 71.4, 32 x 1024 x 12 115.1 / 109.6.  (Turns decided per item instead cost 8 % at 1024: a branch in the loop over the tiles.)
-constexpr int TURNS_FROM_TILES = 6;
-template <bool TURNS>
-__global__ void __launch_bounds__(THREADS, 1)
-attn_fwd1_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant__ CUtensorMap tmOut, const Args a) {
+template <bool DUO>
+__global__ void __launch_bounds__(THREADS, 2)
+attn_fwd1_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmKV, const __grid_constant__ CUtensorMap tmOut, const Args a) {
     extern __shared__ __align__(1024) uint8_t smem[];
-    uint8_t* sQ = smem;                                   // [QBUF][A, B]
-    uint8_t* sK = sQ + QBUF * 2 * TILE_BYTES;             // [KVSTAGES]
-    uint8_t* sV = sK + KVSTAGES * TILE_BYTES;             // [KVSTAGES]
-    uint8_t* sO = sV + KVSTAGES * TILE_BYTES;             // [A, B] output tiles on their way out
-    uint64_t* bars = reinterpret_cast<uint64_t*>(sO + 2 * TILE_BYTES);
-    uint64_t* q_full = bars + 0;      // [2]
-    uint64_t* q_empty = bars + 2;     // [2]
-    uint64_t* k_full = bars + 4;      // [3]
-    uint64_t* k_empty = bars + 7;     // [3]
-    uint64_t* v_full = bars + 10;     // [3]
-    uint64_t* v_empty = bars + 13;    // [3]
-    uint64_t* s_full = bars + 16;     // [2 slots] S_X(t) complete                            (1 commit)
-    uint64_t* s_empty = bars + 18;    // [2] the slot's warps hold S_X(t) in registers          (4 arrivals)
-    uint64_t* p_ready = bars + 20;    // [2] P_X(t) is in TMEM (and O_X rescaled if needed)     (4 arrivals)
-    uint64_t* pv_done = bars + 22;    // [2] O_X += P_X(t) V complete                           (1 commit)
-    uint64_t* o_free = bars + 24;     // [2] the slot's warps hold the item's O_X in registers  (4 arrivals)
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 26);
+    uint8_t* sQ = smem;                                   // [A, B][2]: Q of an item, then its output on the way out; the next item's Q meanwhile in the other
+    uint8_t* sKV = sQ + 4 * TILE_BYTES;                   // [RING]
+    uint64_t* bars = reinterpret_cast<uint64_t*>(sKV + RING * KV_BYTES);
+    uint64_t* q_full = bars + 0;      // [2 slots][2 buffers]
+    uint64_t* q_empty = bars + 4;     // [2][2] the output has left the buffer                  (1 arrival)
+    uint64_t* s_full = bars + 8;      // [2] S_X(t) complete, and with it every earlier product (1 commit)
+    uint64_t* p_ready = bars + 10;    // [2] P_X(t) is in TMEM (and O_X rescaled if needed)     (4 arrivals)
+    uint64_t* o_full = bars + 12;     // [2] the item's O_X is complete                         (1 commit)
+    uint64_t* o_free = bars + 14;     // [2] the slot's warps have read O_X                     (4 arrivals)
+    uint64_t* kv_full = bars + 16;    // [RING] K_0 V_0 K_1 V_1 ...
+    uint64_t* kv_empty = kv_full + RING;      // both slots are done with the tile, or have no use for it
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(kv_empty + RING);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int nq = CEIL_DIV(a.T, BT);
-    const int np = (nq + 1) >> 1;                         // query-tile pairs per (batch, head)
-    const int BH = a.B * a.NH;
-    const int total = BH * np;
-    // work item w -> (pair p, batch, head); late (heavy) pairs first
-    auto decode = [&](int w, int& p, int& b, int& h) {
-        const int rank = w / BH, bh = w - rank * BH;
-        p = np - 1 - rank;
-        b = bh / a.NH; h = bh - b * a.NH;
-    };
 
     if (threadIdx.x == 0) {
         if ((smem_u32(smem) & 1023u) != 0) record_error(a.status, ST_BAD_ARG, 0x18);
+        for (int i = 0; i < 4; i++) { mbar_init(&q_full[i], 1); mbar_init(&q_empty[i], 1); }
         for (int i = 0; i < 2; i++) {
-            mbar_init(&q_full[i], 1); mbar_init(&q_empty[i], 1);
-            mbar_init(&s_full[i], 1); mbar_init(&s_empty[i], 4); mbar_init(&p_ready[i], 4); mbar_init(&pv_done[i], 1); mbar_init(&o_free[i], 4);
+            mbar_init(&s_full[i], 1); mbar_init(&p_ready[i], 4); mbar_init(&o_full[i], 1); mbar_init(&o_free[i], 4);
         }
-        for (int i = 0; i < KVSTAGES; i++) { mbar_init(&k_full[i], 1); mbar_init(&k_empty[i], 1); mbar_init(&v_full[i], 1); mbar_init(&v_empty[i], 1); }
+        for (int i = 0; i < RING; i++) { mbar_init(&kv_full[i], 1); mbar_init(&kv_empty[i], 2); }
         *abort_flag = 0;
         mbar_fence_init();
-        tma_prefetch_desc(&tmQKV); tma_prefetch_desc(&tmOut);
+        tma_prefetch_desc(&tmQ); tma_prefetch_desc(&tmKV); tma_prefetch_desc(&tmOut);
     }
     if (warp == 1) { tmem_alloc(tmem_slot, TMEM_COLS); tmem_relinquish(); }
     tc_fence_before();
@@ -121,245 +127,236 @@ attn_fwd1_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constan
     pdl_wait();
     if (a.early) pdl_trigger();
 
-    if (warp == 0) {
-        // ---------------------------------------------------------------- TMA producer
+    Items<DUO> im(blockIdx.x, gridDim.x, a);
+
+    if (warp < 4) {
+        regs_shrink<REGS_LOW>();
+        if (warp == 0) {
+        // ---------------------------------------------------------------- TMA producer, per item: Q_A Q_B K_0 V_0 K_1 V_1 ...
         if (lane == 0) {
-            int kst = 0; uint32_t kph = 0;
-            int it = 0;
-            bool fail = false;
-            for (int w = blockIdx.x; w < total && !fail; w += gridDim.x, it++) {
-                int p, b, h; decode(w, p, b, h);
-                const int qb = it & 1;
-                if (!mbar_wait_relaxed(&q_empty[qb], ((it >> 1) & 1) ^ 1, abort_flag, a.status, 0x502)) break;
-                mbar_expect_tx(&q_full[qb], 2 * TILE_BYTES);
-                tma_load_4d(sQ + qb * 2 * TILE_BYTES, &tmQKV, &q_full[qb], 0, h, 2 * p * BT, b);                       // Q_A
-                tma_load_4d(sQ + qb * 2 * TILE_BYTES + TILE_BYTES, &tmQKV, &q_full[qb], 0, h, (2 * p + 1) * BT, b);    // Q_B (zeros past T)
-                const int nkv = min(2 * p + 2, nq);
-                for (int j = 0; j < nkv; j++) {
-                    if (!mbar_wait_relaxed(&k_empty[kst], kph ^ 1, abort_flag, a.status, 0x500)) { fail = true; break; }
-                    mbar_expect_tx(&k_full[kst], TILE_BYTES);
-                    tma_load_4d(sK + kst * TILE_BYTES, &tmQKV, &k_full[kst], 0, a.NH + h, j * BT, b);
-                    if (!mbar_wait_relaxed(&v_empty[kst], kph ^ 1, abort_flag, a.status, 0x501)) { fail = true; break; }
-                    mbar_expect_tx(&v_full[kst], TILE_BYTES);
-                    tma_load_4d(sV + kst * TILE_BYTES, &tmQKV, &v_full[kst], 0, 2 * a.NH + h, j * BT, b);
-                    if (++kst == KVSTAGES) { kst = 0; kph ^= 1; }
+            uint32_t st = 0, ph = 1;
+            uint32_t nx[2] = {0, 0};           // items of each slot so far
+            bool ok = true;
+            for (; im.valid() && ok; im.next()) {
+                const int nkv = im.kv_tiles();
+                #pragma unroll
+                for (int x = 0; x < 2; x++) {
+                    if (!ok || im.tiles(x) == 0) continue;
+                    const uint32_t q = 2 * x + (nx[x] & 1);
+                    ok = mbar_wait_relaxed(&q_empty[q], ((nx[x] >> 1) & 1) ^ 1, abort_flag, a.status, 0x502);
+                    if (!ok) break;
+                    mbar_expect_tx(&q_full[q], TILE_BYTES);
+                    tma_load_4d(sQ + q * TILE_BYTES, &tmQ, &q_full[q], 0, im.h, im.qtile(x) * BT, im.b);       // zeros past T
+                    nx[x]++;
+                }
+                for (int j = 0; j < 2 * nkv && ok; j++) {
+                    ok = mbar_wait_relaxed(&kv_empty[st], ph, abort_flag, a.status, 0x500);
+                    if (!ok) break;
+                    mbar_expect_tx(&kv_full[st], KV_BYTES);
+                    tma_load_4d(sKV + st * KV_BYTES, &tmKV, &kv_full[st], 0, (1 + (j & 1)) * a.NH + im.h, (j >> 1) * KT, im.b);
+                    if (++st == RING) { st = 0; ph ^= 1; }
                 }
             }
         }
-    } else if (warp == 1) {
-        // ---------------------------------------------------------------- issuer
-        // Per item and key tile j, in this order:  S_A(j+1),  S_B(j+1),  O_A += P_A(j) V_j,  O_B += P_B(j) V_j;  tile A stops one
-        // key tile before tile B.  The first S of the next item is issued at the end of the current one.
+        } else if (warp < 3) {
+        // ---------------------------------------------------------------- issuer of slot x, per item: S(0), then for every key tile j  O += P(j) V_j, S(j+1).
+        // A chain of short waits and few instructions; one warp for both slots left each waiting for the other's (1200 cycles a step).
+        const int x = warp - 1;
         const bool leader = elect_one();
-#define WAIT_ALL(bar, parity, code) (__all_sync(0xffffffffu, mbar_wait_relaxed(bar, parity, abort_flag, a.status, code)) != 0)
-        constexpr uint32_t idesc_s = umma_idesc_bf16(BT, BT, 0, 0);      // Q (K-major) x K (K-major)
+        constexpr uint32_t idesc_s = umma_idesc_bf16(BT, KT, 0, 0);      // Q (K-major) x K (K-major)
         constexpr uint32_t idesc_o = umma_idesc_bf16(BT, HS, 0, 1);      // P (TMEM) x V (N-major)
-        constexpr uint32_t TILE_UNITS = TILE_BYTES / 16;
-        const uint64_t dQ0 = umma_desc_sw128(smem_u32(sQ), 16, 1024), dK0 = umma_desc_sw128(smem_u32(sK), 16, 1024);
-        const uint64_t dV0 = umma_desc_sw128(smem_u32(sV), TILE_BYTES, 1024);
-        uint32_t ts[2] = {0, 0};          // tiles issued per slot (S products), for the parities of s_empty
-        uint32_t tp[2] = {0, 0};          // tiles whose P V product has been issued per slot
-        uint32_t items[2] = {0, 0};       // items started per slot, for o_free
-        int kst = 0; uint32_t kph = 0;    // ring position of key tile j of the current item
+        constexpr uint32_t KV_UNITS = KV_BYTES / 16;
+        const uint64_t dQ0 = umma_desc_sw128(smem_u32(sQ + 2 * x * TILE_BYTES), 16, 1024);
+        const uint64_t dK0 = umma_desc_sw128(smem_u32(sKV), 16, 1024), dV0 = umma_desc_sw128(smem_u32(sKV + KV_BYTES), KV_BYTES, 1024);
+        const uint32_t tS = tmem_base + x * 128, tO = tS + 64;
+        uint32_t st = 0, ph = 0;          // of the K / V pair j
+        uint32_t t = 0, it = 0;           // tiles and items of this slot so far
         bool ok = true;
-        // S_X of the key tile at ring stage st with the Q tile of buffer qb; the slot that reads a K tile (a Q pair) last releases it
-        auto issue_s = [&](int x, int qb, int st, bool release_k, bool release_q) {
-            const uint64_t q = dQ0 + (uint32_t)(qb * 2 + x) * TILE_UNITS, k = dK0 + (uint32_t)st * TILE_UNITS;
-            if (leader) {
-                #pragma unroll
-                for (int kk = 0; kk < HS / 16; kk++) umma_ss(tmem_base + x * 128, q + 2 * kk, k + 2 * kk, idesc_s, kk > 0);
-                umma_commit(&s_full[x]);
-                TRACE(0, x * 2 + 1, ts[x]);
-                if (release_k) umma_commit(&k_empty[st]);
-                if (release_q) umma_commit(&q_empty[qb]);
+        auto issue_s = [&](uint64_t q, uint32_t st) {
+            const uint64_t k = dK0 + st * (2 * KV_UNITS);
+            #pragma unroll
+            for (int kk = 0; kk < HS / 16; kk++) umma_ss(tS, q + 2 * kk, k + 2 * kk, idesc_s, kk > 0);
+            umma_commit(&s_full[x]);
+            umma_commit(&kv_empty[2 * st]);
+        };
+        for (; im.valid() && ok; im.next()) {
+            const int n = im.tiles(x), nkv = im.kv_tiles();
+            const uint64_t q = dQ0 + (it & 1) * (TILE_BYTES / 16);
+            int i = 0;                    // tiles of this slot in the item so far
+            for (int j = 0; j < nkv && ok; j++) {
+                if (j == (DUO ? x : 0) && n > 0) {
+                    ok = mbar_wait_relaxed(&q_full[2 * x + (it & 1)], (it >> 1) & 1, abort_flag, a.status, 0x510) && mbar_wait_relaxed(&kv_full[2 * st], ph, abort_flag, a.status, 0x511);
+                    if (!ok) break;
+                    tc_fence_after();
+                    if (leader) issue_s(q, st);
+                }
+                if (DUO ? (j & 1) == x : j < n) {
+                    const uint32_t sn = st + Items<DUO>::STEP, st1 = sn >= PAIRS ? sn - PAIRS : sn, ph1 = sn >= PAIRS ? ph ^ 1 : ph;      // of this slot's next tile
+                    // the tiles first, P last: what follows its arrival is the chain of the slot
+                    ok = mbar_wait_relaxed(&kv_full[2 * st + 1], ph, abort_flag, a.status, 0x515);
+                    if (ok && i + 1 < n) ok = mbar_wait_relaxed(&kv_full[2 * st1], ph1, abort_flag, a.status, 0x516);
+                    if (ok && i == 0 && it > 0) ok = mbar_wait_relaxed(&o_free[x], (it - 1) & 1, abort_flag, a.status, 0x517);
+                    ok = ok && mbar_wait_relaxed(&p_ready[x], t & 1, abort_flag, a.status, 0x514);
+                    if (!ok) break;
+                    tc_fence_after();
+                    const uint64_t v = dV0 + st * (2 * KV_UNITS);
+                    if (leader) {
+                        // A = P in TMEM (16 keys = 8 columns per step), B = V N-major (16 rows = 2048 bytes per step)
+                        #pragma unroll
+                        for (int kk = 0; kk < KT / 16; kk++) umma_ts(tO, tS + kk * 8, v + 128 * kk, idesc_o, i > 0 || kk > 0);
+                        if (i + 1 < n) issue_s(q, st1); else umma_commit(&o_full[x]);
+                        umma_commit(&kv_empty[2 * st + 1]);
+                    }
+                    t++; i++;
+                } else {
+                    // a tile that only the other slot reads; its buffer is not given back before it has been filled
+                    ok = mbar_wait_relaxed(&kv_full[2 * st], ph, abort_flag, a.status, 0x512);
+                    if (ok && leader) mbar_arrive(&kv_empty[2 * st]);
+                    ok = ok && mbar_wait_relaxed(&kv_full[2 * st + 1], ph, abort_flag, a.status, 0x513);
+                    if (ok && leader) mbar_arrive(&kv_empty[2 * st + 1]);
+                }
+                if (++st == PAIRS) { st = 0; ph ^= 1; }
             }
-            ts[x]++;
-        };
-        // first S products of an item (key tile 0 at stage st): slot A, and slot B if the item has a second query tile
-        auto issue_first = [&](int p_, int qb, int st) {
-            const bool hb = 2 * p_ + 1 < nq;
-            issue_s(0, qb, st, !hb, !hb && p_ == 0);
-            if (hb) issue_s(1, qb, st, true, false);
-        };
-        // O_X += P_X(jj) V_jj : A = P_X in TMEM (16 keys = 8 columns per step), B = V_jj N-major (16 rows = 2048 bytes)
-        auto issue_pv = [&](int x, int jj, int st, uint32_t ph, bool release_v) {
-            bool good = WAIT_ALL(&v_full[st], ph, 0x515) && WAIT_ALL(&p_ready[x], tp[x] & 1, 0x514);
-            if (good && jj == 0 && items[x] > 0) good = WAIT_ALL(&o_free[x], (items[x] - 1) & 1, 0x517);
-            if (!good) return false;
-            tc_fence_after();
-            const uint64_t v = dV0 + (uint32_t)st * TILE_UNITS;
-            if (leader) {
-                #pragma unroll
-                for (int kk = 0; kk < BT / 16; kk++)
-                    umma_ts(tmem_base + 256 + x * 64, tmem_base + 384 + x * 64 + kk * 8, v + 128 * kk, idesc_o, (jj > 0 || kk > 0));
-                umma_commit(&pv_done[x]);
-                if (release_v) umma_commit(&v_empty[st]);
-                TRACE(0, x * 2, tp[x]);
-            }
-            tp[x]++;
-            if (jj == 0) items[x]++;
-            return true;
-        };
-        int it = 0;
-        uint32_t kabs = 0;                // key tiles of earlier items: tile jj of the current item sits at ring position kabs + jj
-        if ((int)blockIdx.x < total) {
-            int p, b, h; decode(blockIdx.x, p, b, h);
-            ok = WAIT_ALL(&q_full[0], 0, 0x510) && WAIT_ALL(&k_full[0], 0, 0x511);
-            tc_fence_after();
-            if (ok) issue_first(p, 0, 0);
+            if (n > 0) it++;
         }
-        for (int w = blockIdx.x; w < total && ok; w += gridDim.x, it++) {
-            int p, b, h; decode(w, p, b, h);
-            const int qb = it & 1;
-            const bool hasB = 2 * p + 1 < nq;
-            const int nA = 2 * p + 1, nB = hasB ? 2 * p + 2 : 0;
-            const int nkv = hasB ? nB : nA;
-            bool next_item = false; int np_ = 0;
-            if (w + (int)gridDim.x < total) { int b2, h2; decode(w + gridDim.x, np_, b2, h2); next_item = true; }
-            // The order inside a step is the order in which the events arrive when slot B runs half a tile behind slot A:
-            //   S_A(j+1) [A holds S_A(j)],  O_B += P_B(j-1) V,  S_B(j+1) [B holds S_B(j)],  O_A += P_A(j) V.
-            // With this order a lagging slot B never holds up slot A.
-            for (int j = 0; j <= nkv && ok; j++) {
-                const uint32_t pos = kabs + j;
-                const int st_prev = (pos + KVSTAGES - 1) % KVSTAGES, st_cur = pos % KVSTAGES, st_next = (pos + 1) % KVSTAGES;
-                const uint32_t ph_prev = ((pos - 1) / KVSTAGES) & 1, ph_cur = (pos / KVSTAGES) & 1, ph_next = ((pos + 1) / KVSTAGES) & 1;
-                if (j + 1 < nkv) ok = WAIT_ALL(&k_full[st_next], ph_next, 0x512);
-                if (ok && j + 1 < nA) {
-                    ok = WAIT_ALL(&s_empty[0], (ts[0] - 1) & 1, 0x513);
-                    if (ok) { tc_fence_after(); issue_s(0, qb, st_next, !hasB, !hasB && j + 1 == nA - 1); }
-                }
-                if (ok && j >= 1 && j - 1 < nB) ok = issue_pv(1, j - 1, st_prev, ph_prev, true);
-                if (ok && j + 1 < nB) {
-                    ok = WAIT_ALL(&s_empty[1], (ts[1] - 1) & 1, 0x513);
-                    if (ok) { tc_fence_after(); issue_s(1, qb, st_next, true, j + 1 == nB - 1); }
-                }
-                // ---- first S products of the next item, once both slots hold their last S of this one
-                if (ok && next_item && j == nkv - 1) {
-                    ok = WAIT_ALL(&q_full[qb ^ 1], ((it + 1) >> 1) & 1, 0x516) && WAIT_ALL(&k_full[(kabs + nkv) % KVSTAGES], ((kabs + nkv) / KVSTAGES) & 1, 0x51a);
-                    if (ok && ts[0] > 0) ok = WAIT_ALL(&s_empty[0], (ts[0] - 1) & 1, 0x518);
-                    if (ok && ts[1] > 0 && 2 * np_ + 1 < nq) ok = WAIT_ALL(&s_empty[1], (ts[1] - 1) & 1, 0x519);
-                    if (ok) { tc_fence_after(); issue_first(np_, qb ^ 1, (kabs + nkv) % KVSTAGES); }
-                }
-                if (ok && j < nA) ok = issue_pv(0, j, st_cur, ph_cur, !hasB);
-            }
-            kabs += nkv;
+        __syncwarp();
         }
-#undef WAIT_ALL
-    }
-    else if (warp >= 4) {
+    } else {
+        regs_grow<REGS_HIGH>();
         // ---------------------------------------------------------------- softmax of slot x: thread = query row r of the slot's tile
         const int x = (warp - 4) >> 2;
-        const int q4 = warp & 3;
+        const int q4 = warp & 3;                           // the warp's quarter of the tensor memory lanes
         const int r = q4 * 32 + lane;
         const uint32_t lane_off = (uint32_t)(q4 * 32) << 16;
-        const uint32_t tS = tmem_base + x * 128, tO = tmem_base + 256 + x * 64, tP = tmem_base + 384 + x * 64;
+        const uint32_t tS = tmem_base + x * 128 + lane_off, tO = tS + 64;
         const bool issuer = q4 == 0 && lane == 0;          // the thread of the slot that issues its output store
         const float c = a.scale_log2e;
         bool ok = true;
-        bool staged = false;
-        if (TURNS && x == 1) turn_pass(TURN_BAR + 2 * q4); // slot A has the first turn
         uint32_t t = 0;                                    // tiles of this slot so far
-        int it = 0;
-        for (int w = blockIdx.x; w < total; w += gridDim.x, it++) {
-            int p, b, h; decode(w, p, b, h);
-            const int qi = 2 * p + x;                      // this slot's query tile
-            const int turns = min(2 * p + 2, nq);          // of either slot in this item
-            if (qi >= nq) {                                // (uniform for the slot) no second tile in this item
-                for (int j = 0; TURNS && j < turns; j++) { turn_wait(TURN_BAR + 2 * q4 + x); turn_pass(TURN_BAR + 2 * q4 + (x ^ 1)); }
-                continue;
-            }
+        uint32_t it = 0;                                   // items of this slot so far
+        for (; im.valid(); im.next()) {
+            const int nj = im.tiles(x);
+            if (!DUO && nj == 0) continue;                 // (uniform for the slot) no second tile in this item
+            const int qi = im.qtile(x);                    // this slot's query tile
+            const int jd = 2 * qi + (q4 >> 1);             // the key tile on this warp's diagonal: none of the later ones is seen
             float m = -INFINITY, l = 0.f;                  // reference maximum (raw score units) and row sum relative to it
-            for (int j = 0; j <= qi; j++, t++) {
-                if (r == 0) TRACE(1 + x, 0, t);
+            #pragma unroll 1
+            for (int i = 0; i < nj; i++, t++) {
+                const int j = Items<DUO>::STEP * i + (DUO ? x : 0);
                 ok = mbar_wait(&s_full[x], t & 1, abort_flag, a.status, 0x520 + x) && ok;
                 tc_fence_after();
-                if (r == 0) TRACE(1 + x, 1, t);
-                uint32_t sv[128];
-                tmem_ld32(tS + lane_off, sv);
-                tmem_ld32(tS + lane_off + 32, sv + 32);
-                tmem_ld32(tS + lane_off + 64, sv + 64);
-                tmem_ld32(tS + lane_off + 96, sv + 96);
-                tmem_ld_wait();
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&s_empty[x]);       // S_X of the next key tile may be issued
-                if (r == 0) TRACE(1 + x, 2, t);
-                if (j == qi) {
-                    #pragma unroll
-                    for (int e = 0; e < 128; e++) if (e > r) sv[e] = 0xff800000u;      // -inf above the diagonal
-                }
-                float mx0 = -INFINITY, mx1 = -INFINITY, mx2 = -INFINITY, mx3 = -INFINITY;
-                #pragma unroll
-                for (int e = 0; e < 128; e += 4) {
-                    mx0 = fmaxf(mx0, __uint_as_float(sv[e])); mx1 = fmaxf(mx1, __uint_as_float(sv[e + 1]));
-                    mx2 = fmaxf(mx2, __uint_as_float(sv[e + 2])); mx3 = fmaxf(mx3, __uint_as_float(sv[e + 3]));
-                }
-                const float mx = fmaxf(fmaxf(mx0, mx1), fmaxf(mx2, mx3));
-                // move the reference maximum only when it lags by more than 2^RESCALE_LOG2 (decided per warp, so that the
-                // TMEM accesses stay warp-wide); a moved maximum rescales the row sum now and the row of O_X below
-                const bool grow = (mx - m) * c > RESCALE_LOG2 || j == 0;
-                const bool moved = __any_sync(0xffffffffu, grow) != 0;
-                float alpha = 1.0f;
-                if (moved) {
-                    const float m_new = fmaxf(m, mx);
-                    alpha = ex2_fast((m - m_new) * c);      // 0 on the first tile (m = -inf)
-                    l *= alpha;
-                    m = m_new;
-                }
-                if (r == 0) TRACE(1 + x, 3, t);
-                float moff = m * c;
-                if (TURNS) turn_wait(TURN_BAR + 2 * q4 + x, moff);
-                float rs0 = 0.f, rs1 = 0.f;
-                uint32_t pk[64];
-                #pragma unroll
-                for (int e = 0; e < 128; e += 2) {
-                    const float p0 = ex2_fast(fmaf(__uint_as_float(sv[e]), c, -moff));
-                    const float p1 = ex2_fast(fmaf(__uint_as_float(sv[e + 1]), c, -moff));
-                    rs0 += p0; rs1 += p1;
-                    pk[e >> 1] = pack_bf16x2(p0, p1);
-                }
-                l += rs0 + rs1;
-                if (TURNS) turn_pass(TURN_BAR + 2 * q4 + (x ^ 1), l);
-                if (r == 0) TRACE(1 + x, 5, t);
-                // the previous product has read P_X(t-1) and finished adding to O_X: only now is it waited for, so that it ran
-                // under the exponentials above
-                if (j > 0) ok = mbar_wait(&pv_done[x], (t - 1) & 1, abort_flag, a.status, 0x524 + x) && ok;
-                tc_fence_after();
-                if (r == 0) TRACE(1 + x, 4, t);
-                if (moved && j > 0) {
-                    #pragma unroll
-                    for (int half = 0; half < 2; half++) {
-                        uint32_t ov[32];
-                        tmem_ld32(tO + lane_off + half * 32, ov);
-                        tmem_ld_wait();
-                        #pragma unroll
-                        for (int e = 0; e < 32; e++) ov[e] = __float_as_uint(__uint_as_float(ov[e]) * alpha);
-                        tmem_st16(tO + lane_off + half * 32, ov);
-                        tmem_st16(tO + lane_off + half * 32 + 16, ov + 16);
+                uint32_t pk[32];
+                if (j <= jd) {
+                    uint32_t sv[64];
+                    tmem_ld32(tS, sv);
+                    tmem_ld32(tS + 32, sv + 32);
+                    tmem_ld_wait();
+                    if (j == jd) {
+                        // -inf above the diagonal, which crosses the first 32 columns for even quarters and the others for odd ones
+                        if (q4 & 1) {
+                            #pragma unroll
+                            for (int e = 0; e < 32; e++) if (e > lane) sv[32 + e] = 0xff800000u;
+                        } else {
+                            #pragma unroll
+                            for (int e = 0; e < 32; e++) { if (e > lane) sv[e] = 0xff800000u; sv[32 + e] = 0xff800000u; }
+                        }
                     }
+                    float mx4[4];
+                    #pragma unroll
+                    for (int e = 0; e < 4; e++) mx4[e] = fmaxf(__uint_as_float(sv[2 * e]), __uint_as_float(sv[2 * e + 1]));
+                    #pragma unroll
+                    for (int e = 8; e < 64; e += 2) mx4[(e >> 1) & 3] = max3(mx4[(e >> 1) & 3], __uint_as_float(sv[e]), __uint_as_float(sv[e + 1]));
+                    const float mx = max3(fmaxf(mx4[0], mx4[1]), mx4[2], mx4[3]);
+                    // move the reference maximum only when it lags by more than 2^RESCALE_LOG2 (decided per warp, so that the
+                    // TMEM accesses stay warp-wide); a moved maximum rescales the row sum and the row of O_X
+                    const bool grow = (mx - m) * c > RESCALE_LOG2 || i == 0;
+                    if (__any_sync(0xffffffffu, grow)) {
+                        const float m_new = fmaxf(m, mx);
+                        const float alpha = ex2_fast((m - m_new) * c);      // 0 on the first tile (m = -inf)
+                        l *= alpha;
+                        m = m_new;
+                        if (i > 0) {                       // O_X(t-1) is complete: its product was issued ahead of S_X(t)
+                            #pragma unroll 1
+                            for (int g = 0; g < 64; g += 16) {
+                                uint32_t ov[16];
+                                tmem_ld16(tO + g, ov);
+                                tmem_ld_wait();
+                                #pragma unroll
+                                for (int e = 0; e < 16; e++) ov[e] = __float_as_uint(__uint_as_float(ov[e]) * alpha);
+                                tmem_st16(tO + g, ov);
+                            }
+                        }
+                    }
+                    const float moff = m * c;
+                    const uint64_t c2 = f2_both(c), off2 = f2_both(-moff);
+                    uint64_t rs0 = 0, rs1 = 0;
+                    #pragma unroll
+                    for (int e = 0; e < 64; e += 2) {
+                        const uint64_t x2 = f2_fma(f2_pack_u(sv[e], sv[e + 1]), c2, off2);
+                        float2 p;
+                        if (((e >> 1) & 7) < (DUO ? 2 : 1)) {              // one or two of eight pairs on the FMA pipe
+                            p = ex2_poly2(x2);
+                        } else {
+                            p = f2_unpack(x2);
+                            p.x = ex2_fast(p.x); p.y = ex2_fast(p.y);
+                        }
+                        if (e & 2) rs1 = f2_add(rs1, f2_pack(p.x, p.y)); else rs0 = f2_add(rs0, f2_pack(p.x, p.y));
+                        pk[e >> 1] = pack_bf16x2(p.x, p.y);
+                    }
+                    const float2 rs = f2_unpack(f2_add(rs0, rs1));
+                    l += rs.x + rs.y;
+                } else {
+                    #pragma unroll
+                    for (int e = 0; e < 32; e++) pk[e] = 0;
                 }
-                tmem_st16(tP + lane_off, pk);
-                tmem_st16(tP + lane_off + 16, pk + 16);
-                tmem_st16(tP + lane_off + 32, pk + 32);
-                tmem_st16(tP + lane_off + 48, pk + 48);
+                tmem_st32(tS, pk);                          // over this row's own scores
                 tmem_st_wait();
                 tc_fence_before();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&p_ready[x]);
-                if (r == 0) TRACE(1 + x, 6, t);
+                // the output of the item before has left its buffer long ago: the Q tile of the next item may come
+                if (!DUO && i == 0 && it > 0 && issuer) { tma_store_wait_read<0>(); mbar_arrive(&q_empty[2 * x + ((it - 1) & 1)]); }
             }
-            if (TURNS && qi + 1 < turns) { turn_wait(TURN_BAR + 2 * q4 + x); turn_pass(TURN_BAR + 2 * q4 + (x ^ 1)); }      // slot A has a tile less
             // ---- item epilogue: O_X / l -> bf16 tile in the layout of a 128-byte-swizzled TMA box -> one bulk store
-            ok = mbar_wait(&pv_done[x], (t - 1) & 1, abort_flag, a.status, 0x528 + x) && ok;
+            if (nj > 0) ok = mbar_wait(&o_full[x], it & 1, abort_flag, a.status, 0x528 + x) && ok;
             tc_fence_after();
-            if (staged) { if (issuer) tma_store_wait_read<0>(); asm volatile("bar.sync %0, 128;" ::"r"(1 + x) : "memory"); }
+            // DUO: slot 1 leaves its sums, its maximum and its row sum in shared memory (over its own Q buffers and slot 0's second one, which a
+            // block of one item does not use); slot 0 adds them to its own
+            float* other = reinterpret_cast<float*>(sQ + 2 * TILE_BYTES);               // [channel][row]
+            float* other_ml = reinterpret_cast<float*>(sQ + TILE_BYTES);                // [max, sum][row]
+            float mine = 1.0f, theirs = 0.0f;
+            if (DUO) {
+                if (x == 1) {
+                    #pragma unroll 1
+                    for (int g = 0; g < 64; g += 16) {
+                        uint32_t ov[16];
+                        if (nj > 0) { tmem_ld16(tO + g, ov); tmem_ld_wait(); }
+                        #pragma unroll
+                        for (int e = 0; e < 16; e++) other[(g + e) * BT + r] = nj > 0 ? __uint_as_float(ov[e]) : 0.f;
+                    }
+                    other_ml[r] = m;
+                    other_ml[BT + r] = l;
+                }
+                asm volatile("bar.sync 3, 256;" ::: "memory");
+                if (x == 1) break;
+                const float mo = other_ml[r], m_new = fmaxf(m, mo);      // slot 0 has seen key 0: m is finite; slot 1 may have seen none of this row's keys
+                mine = ex2_fast((m - m_new) * c);
+                theirs = ex2_fast((mo - m_new) * c);
+                l = l * mine + other_ml[BT + r] * theirs;
+                m = m_new;
+            }
             const float inv = 1.0f / l;
-            uint8_t* orow = sO + x * TILE_BYTES + r * 128;
-            #pragma unroll
+            uint8_t* otile = sQ + (2 * x + (it & 1)) * TILE_BYTES;     // over the item's Q tile, which its last score product has read
+            uint8_t* orow = otile + r * 128;
+            #pragma unroll 1
             for (int half = 0; half < 2; half++) {
                 uint32_t ov[32];
-                tmem_ld32(tO + lane_off + half * 32, ov);
+                tmem_ld32(tO + half * 32, ov);
                 tmem_ld_wait();
+                if (DUO) {
+                    #pragma unroll
+                    for (int e = 0; e < 32; e++) ov[e] = __float_as_uint(__uint_as_float(ov[e]) * mine + other[(half * 32 + e) * BT + r] * theirs);
+                }
                 #pragma unroll
                 for (int u = 0; u < 4; u++) {
                     uint4 o;
@@ -376,14 +373,13 @@ attn_fwd1_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constan
             fence_async_smem();
             asm volatile("bar.sync %0, 128;" ::"r"(1 + x) : "memory");
             if (issuer && ok) {
-                tma_store_4d(&tmOut, sO + x * TILE_BYTES, 0, h, qi * BT, b);
+                tma_store_4d(&tmOut, otile, 0, im.h, qi * BT, im.b);
                 tma_store_commit();
             }
-            staged = true;
+            it++;
             const int trow = qi * BT + r;
-            if (trow < a.T && ok) a.lse[((size_t)b * a.NH + h) * a.T + trow] = m * a.scale + logf(l);
+            if (trow < a.T && ok) a.lse[((size_t)im.b * a.NH + im.h) * a.T + trow] = m * a.scale + logf(l);
         }
-        if (TURNS && x == 0) turn_wait(TURN_BAR + 2 * q4); // the last turn passed on by slot B
         if (issuer) tma_store_wait<0>();
     }
     tc_fence_before();
@@ -397,19 +393,14 @@ attn_fwd1_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constan
     if (warp == 1) tmem_dealloc(tmem_base, TMEM_COLS);
 }
 
-#undef TRACE
 }  // namespace
-
-// Profiling aid: with a device buffer of 3 * 8 * 64 int64 set here, CTA 0 of every later launch records clock64() stamps of its
-// first 64 tiles per slot (role 0 = issuer, 1 / 2 = first thread of the softmax group of tile A / B).  Null switches it off.
-static long long* g_fwd_trace = nullptr;
-extern "C" int llmc_attention_fwd_set_trace(long long* buf) { g_fwd_trace = buf; return 0; }
 
 // out (B,T,NH,HS) = causal softmax(Q K^T / sqrt(HS)) V ; lse (B,NH,T) fp32.  Head sizes: multiples of 8 from 64 to 128.
 extern "C" int llmc_attention_fwd(bf16* out, float* lse, const bf16* qkv, int B, int T, int NH, int hs, cudaStream_t stream) {
     if (hs != HS) return llmc_attention_fwd_general(out, lse, qkv, B, T, NH, hs, stream);
-    CUtensorMap tmQKV, tmOut;
-    int rc = llmc_attn_qkv_map(&tmQKV, qkv, B, T, NH, hs);
+    CUtensorMap tmQ, tmKV, tmOut;
+    int rc = llmc_attn_qkv_map(&tmQ, qkv, B, T, NH, hs, BT);
+    if (!rc) rc = llmc_attn_qkv_map(&tmKV, qkv, B, T, NH, hs, KT);
     if (rc) return rc;
     {
         uint64_t dims[4] = {(uint64_t)hs, (uint64_t)NH, (uint64_t)T, (uint64_t)B};
@@ -418,30 +409,31 @@ extern "C" int llmc_attention_fwd(bf16* out, float* lse, const bf16* qkv, int B,
         if ((rc = llmc_get_tensormap(&tmOut, out, 2, 4, dims, strides, box, 3))) return rc;
     }
     Args a;
-    a.lse = lse; a.B = B; a.T = T; a.NH = NH;
+    a.lse = lse; a.T = T; a.NH = NH; a.BH = B * NH;
     a.scale = 1.0f / sqrtf((float)hs);
     a.scale_log2e = a.scale * 1.4426950408889634f;
     a.status = llmc_status_ptr();
-    a.trace = g_fwd_trace;
     const int nq = CEIL_DIV(T, BT);
-    const int total = B * NH * ((nq + 1) / 2);
     int sms = llmc_device_sm_count(); if (sms <= 0) sms = 148;
-    const int grid = total < sms ? total : sms;
-    const bool turns = nq >= TURNS_FROM_TILES;
-    auto kernel = turns ? attn_fwd1_kernel<true> : attn_fwd1_kernel<false>;
+    // us, pairs / DUO, query tiles per SM in brackets: 8 x 300 x 12 (1.9) 10.3 / 9.8, 3 x 1000 x 16 (2.6) 23.0 / 19.6, 1 x 2048 x 25 (2.7) 39.3 / 27.7, but
+    // 16 x 256 x 16 (3.5) 11.1 / 17.1, 8 x 1024 x 12 (5.2) 29.4 / 37.1
+    const bool duo = (long long)B * NH * nq <= 3 * sms && T > KT;
+    const int total = B * NH * (duo ? nq : (nq + 1) / 2);
+    const int grid = duo || total < 2 * sms ? total : 2 * sms;
+    auto kernel = duo ? attn_fwd1_kernel<true> : attn_fwd1_kernel<false>;
     static bool configured[2] = {false, false};
-    if (!configured[turns]) {
+    if (!configured[duo]) {
         CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM));
-        configured[turns] = true;
+        configured[duo] = true;
     }
-    // early launch (pdl.cuh) only where SMs stay free: 4 x 64 GPT-2 step 1566 -> 1513 us; otherwise the blocks of the next kernel sit beside
-    // this one's for all of its run: 64 x 1024 x 12 938 -> 986 us
-    a.early = grid < sms;
+    // early launch (pdl.cuh) only where SMs have room for another block: a prefill of 777 tokens (224 blocks) 617 -> 607 us; otherwise the blocks of the next
+    // kernel sit beside this one's for all of its run (64 x 1024 x 12, forward and backward, in the kernels before this one: 938 -> 986 us)
+    a.early = grid < 2 * sms;
     if (a.early) {
-        CUDA_CHECK(launch_pdl(kernel, dim3(grid), dim3(THREADS), SMEM, stream, 0, tmQKV, tmOut, a));
+        CUDA_CHECK(launch_pdl(kernel, dim3(grid), dim3(THREADS), SMEM, stream, 0, tmQ, tmKV, tmOut, a));
         return 0;
     }
-    kernel<<<grid, THREADS, SMEM, stream>>>(tmQKV, tmOut, a);
+    kernel<<<grid, THREADS, SMEM, stream>>>(tmQ, tmKV, tmOut, a);
     CUDA_CHECK(cudaGetLastError());
     return 0;
 }

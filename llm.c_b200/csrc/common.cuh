@@ -180,13 +180,35 @@ DEVINL float gelu_tanh_grad(float x) {
 DEVINL float ex2_fast(float x) { float y; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
 DEVINL float tanh_fast(float x) { float y; asm("tanh.approx.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
 // Two fp32 operations in one instruction (each half rounds like the scalar operation, so results do not change): for loops that are bound by
-// the issue of their arithmetic.  The forward attention kernels and the 64-wide backward, measured with it, are not (no change).
+// the issue of their arithmetic.  The wide forward attention kernel and the 64-wide backward, measured with it, are not (no change).
 DEVINL uint64_t f2_pack(float lo, float hi) { uint64_t r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi)); return r; }
 DEVINL uint64_t f2_pack_u(uint32_t lo, uint32_t hi) { uint64_t r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(lo), "r"(hi)); return r; }
 DEVINL float2 f2_unpack(uint64_t v) { float2 r; asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v)); return r; }
 DEVINL uint64_t f2_fma(uint64_t a, uint64_t b, uint64_t c) { uint64_t r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c)); return r; }
 DEVINL uint64_t f2_mul(uint64_t a, uint64_t b) { uint64_t r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
 DEVINL uint64_t f2_add(uint64_t a, uint64_t b) { uint64_t r; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
+DEVINL uint64_t f2_both(float v) { return f2_pack(v, v); }
+// The larger of three in one instruction (two cycles of a scheduler, like the larger of two); a NaN loses, as in fmaxf
+DEVINL float max3(float a, float b, float c) { float r; asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c)); return r; }
+// 2^x of two numbers on the FMA pipe, for loops that keep the special-function unit busy (ex2 takes 8 cycles of a scheduler there, these two 9 each
+// here).  Cody and Waite's reduction: x = n + f with n the nearest integer, read from the low bits of x + 1.5 * 2^23; 2^f by a polynomial of degree 5 with
+// 2^0 = 1, fitted for the least relative error on [-1/2, 1/2] (linear programme: 7e-8 in exact arithmetic); n is added to the exponent.  Error against 64 bits on [-30, 0]
+// 2.2e-7 at most, 8e-8 rms.  For x < 64; below -125 the result is that of -125 (2.4e-38), a NaN becomes a value that is no smaller than 2^127.
+DEVINL float2 ex2_poly2(uint64_t x) {
+    float2 v = f2_unpack(x);
+    asm("max.NaN.f32 %0, %0, %1;" : "+f"(v.x) : "f"(-125.0f));
+    asm("max.NaN.f32 %0, %0, %1;" : "+f"(v.y) : "f"(-125.0f));
+    x = f2_pack(v.x, v.y);
+    const uint64_t t = f2_add(x, f2_both(12582912.0f));
+    const uint64_t f = f2_add(x, f2_fma(t, f2_both(-1.0f), f2_both(12582912.0f)));
+    uint64_t p = f2_fma(f, f2_both(0.0013202981790527701f), f2_both(0.009674952365458012f));
+    p = f2_fma(p, f, f2_both(0.055510472506284714f));
+    p = f2_fma(p, f, f2_both(0.24022166430950165f));
+    p = f2_fma(p, f, f2_both(0.6931465864181519f));
+    p = f2_fma(p, f, f2_both(1.0f));
+    const float2 r = f2_unpack(p), n = f2_unpack(t);
+    return make_float2(__uint_as_float(__float_as_uint(r.x) + (__float_as_uint(n.x) << 23)), __uint_as_float(__float_as_uint(r.y) + (__float_as_uint(n.y) << 23)));
+}
 
 // GELU with the tanh approximation, 0.5 x (1 + tanh(k (x + 0.044715 x^3))), and its derivative, scalar and in pairs.  Both forms evaluate
 // the same operations in the same order, so an element gives the same bits through either.  In the GEMM epilogues, which sit behind a
@@ -431,6 +453,15 @@ DEVINL void tmem_st32(uint32_t taddr, const uint32_t* r) {
           "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
         : "memory");
 }
+DEVINL void tmem_st16(uint32_t taddr, const uint32_t* r) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
+        "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
+        ::"r"(taddr),
+          "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
+          "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+        : "memory");
+}
 DEVINL void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
 // Turns at a unit that two warps of a scheduler share (the special-function unit in softmax loops): started together they would run their
@@ -440,6 +471,11 @@ DEVINL void turn_wait(int bar) { asm volatile("bar.sync %0, 64;" ::"r"(bar) : "m
 DEVINL void turn_wait(int bar, float& dep) { asm volatile("bar.sync %1, 64;" : "+f"(dep) : "r"(bar) : "memory"); }
 DEVINL void turn_pass(int bar) { asm volatile("bar.arrive %0, 64;" ::"r"(bar) : "memory"); }
 DEVINL void turn_pass(int bar, float& dep) { asm volatile("bar.arrive %1, 64;" : "+f"(dep) : "r"(bar) : "memory"); }
+
+// Moves registers between the warpgroups of a block (all four warps of a group call it): the shares of all groups may add up to what the block was launched
+// with and no more.
+template <int N> DEVINL void regs_shrink() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
+template <int N> DEVINL void regs_grow() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
 
 DEVINL bool elect_one() {
     uint32_t pred;

@@ -38,3 +38,27 @@ def test_forward_and_backward(B, T, NH):
     for c in range(3):
         s = slice(c * NH * 64, (c + 1) * NH * 64)
         assert rel(buf[:B, :, s], rd[..., s]) < 5e-3, c
+
+
+@pytest.mark.parametrize("B,T,NH,ramp", [
+    # both slots of a block on one query tile: two key tiles, ragged and whole last ones, as many query tiles as three per SM (148 SMs); then more
+    (1, 66, 2, 0), (1, 191, 3, 0), (1, 192, 3, 0), (1, 193, 3, 0), (2, 450, 7, 0), (37, 200, 6, 0), (223, 129, 1, 0),
+    # scores that grow along the keys: the reference maximum moves in most tiles
+    (1, 900, 3, 1), (40, 300, 6, 1)])
+def test_forward_slots(B, T, NH, ramp):
+    g = torch.Generator().manual_seed(B + T + NH)
+    qkv = torch.randn(B, T, 3 * NH * 64, generator=g)
+    if ramp:
+        q, k = qkv[..., :NH * 64], qkv[..., NH * 64:2 * NH * 64]
+        q.copy_(q.abs())
+        k.copy_(k.abs() * torch.linspace(0.1, 4.0, T).view(1, T, 1))
+    qkv = qkv.bfloat16()
+    ro, rl = torch.empty(B, T, NH * 64), torch.empty(B, NH, T)
+    R.attention_forward(ro, rl, qkv, B, T, NH)
+    out = torch.full((B + 1, T, NH * 64), 7.0, dtype=torch.bfloat16, device=DEV)
+    lse = torch.empty(B, NH, T, device=DEV)
+    KN.attention_forward(out[:B], lse, qkv.to(DEV), B, T, NH)
+    assert _lib.read_status() == 0 and (out[B:] == 7.0).all()
+    # P and O rounded to bf16 once each: 0.0016 together; LSE of up to 200 in fp32
+    assert float((out[:B].float().cpu() - ro).norm() / ro.norm()) < 4e-3
+    assert float((lse.cpu() - rl).abs().max()) < 1e-4 + 2e-6 * float(rl.abs().max())
