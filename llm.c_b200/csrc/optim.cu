@@ -29,38 +29,65 @@ struct TensorTable {
 
 namespace {
 
+struct alignas(8) Pack64 { bf16 v[4]; };
+
+// The elements of a table's views as one list of chunks of at most `per` elements, none across a slice: view by view, slice by slice.  Blocks take chunks,
+// not views: most views of a transformer are small, and a block for every view and place in it came to thousands that found nothing to do.
+struct Chunks {
+    TensorTable tab;
+    int first[17];         // number of chunks in front of view i
+    int per;
+    Chunks(const TensorTable& t, int per_) : tab(t), per(per_) {
+        first[0] = 0;
+        for (int i = 0; i < 16; i++) first[i + 1] = first[i] + (i < t.count ? (int)CEIL_DIV(t.t[i].n, (long long)per_) * t.t[i].L : 0);
+    }
+    int total() const { return first[16]; }
+};
+// Walks from chunk to chunk in increasing order.
+struct ChunkAt {
+    int view = 0, per_slice = 0, l = 0, c = 0;
+    DEVINL void seek(const Chunks& k, int i) {
+        while (i >= k.first[view + 1]) { view++; per_slice = 0; }
+        if (per_slice == 0) per_slice = (int)CEIL_DIV(k.tab.t[view].n, (long long)k.per);
+        const int j = i - k.first[view];
+        l = j / per_slice; c = j - l * per_slice;
+    }
+};
+
 constexpr int OPT_THREADS = 512;
 
-__global__ void __launch_bounds__(OPT_THREADS)
-norm_sq_kernel(float* __restrict__ partials, const bf16* __restrict__ grads, const TensorTable tab) {
+// Bound by reading the gradients once; 124 million elements, with its sum of the partials, 46 us, 30 million 33 us (59 and 34 with a grid of every SM times every view; alone
+// between other passes: the time the host takes for the two launches is about 30 us).
+constexpr int NORM_THREADS = 256;
+constexpr int NORM_PACKS = 4;            // 128-bit loads of a thread in flight
+constexpr int NORM_BLOCKS = 16;          // per SM
+
+__global__ void __launch_bounds__(NORM_THREADS)
+norm_sq_kernel(float* __restrict__ partials, const bf16* __restrict__ grads, const __grid_constant__ Chunks k) {
     __shared__ float red[32];
-    const TensorView tv = tab.t[blockIdx.y];
-    const long long packs_per_slice = tv.n >> 3;
-    // slice by slice (no division per pack), four independent 128-bit loads in flight per thread; the order of the additions is
-    // fixed by the launch geometry, which the host derives from the device alone: the same sum on every run
-    float a0 = 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f;
-    const long long stride = (long long)gridDim.x * OPT_THREADS;
-    for (int l = 0; l < tv.L; l++) {
-        const bf16* base = grads + tv.p_base + (long long)l * tv.p_stride;
-        long long i = (long long)blockIdx.x * OPT_THREADS + threadIdx.x;
-        for (; i + 3 * stride < packs_per_slice; i += 4 * stride) {
-            const bf16x8 g0 = ld128cs(base + i * 8), g1 = ld128cs(base + (i + stride) * 8), g2 = ld128cs(base + (i + 2 * stride) * 8),
-                         g3 = ld128cs(base + (i + 3 * stride) * 8);
+    // the order of the additions is fixed by the launch geometry, which the host derives from the device alone: the same sum on every run
+    float a[NORM_PACKS];
+    #pragma unroll
+    for (int u = 0; u < NORM_PACKS; u++) a[u] = 0.f;
+    ChunkAt at;
+    for (int i = blockIdx.x; i < k.first[16]; i += gridDim.x) {
+        at.seek(k, i);
+        const TensorView& tv = k.tab.t[at.view];
+        const bf16* base = grads + tv.p_base + (long long)at.l * tv.p_stride;
+        const long long packs = tv.n >> 3, p0 = (long long)at.c * (NORM_PACKS * NORM_THREADS) + threadIdx.x;
+        bf16x8 g[NORM_PACKS];
+        #pragma unroll
+        for (int u = 0; u < NORM_PACKS; u++) g[u] = p0 + u * NORM_THREADS < packs ? ld128(base + (p0 + u * NORM_THREADS) * 8) : bf16x8::zeros();
+        #pragma unroll
+        for (int u = 0; u < NORM_PACKS; u++)
             #pragma unroll
-            for (int e = 0; e < 8; e++) {
-                const float f0 = __bfloat162float(g0[e]), f1 = __bfloat162float(g1[e]), f2 = __bfloat162float(g2[e]), f3 = __bfloat162float(g3[e]);
-                a0 = fmaf(f0, f0, a0); a1 = fmaf(f1, f1, a1); a2 = fmaf(f2, f2, a2); a3 = fmaf(f3, f3, a3);
-            }
-        }
-        for (; i < packs_per_slice; i += stride) {
-            const bf16x8 g = ld128cs(base + i * 8);
-            #pragma unroll
-            for (int e = 0; e < 8; e++) { const float f = __bfloat162float(g[e]); a0 = fmaf(f, f, a0); }
-        }
+            for (int e = 0; e < 8; e++) { const float f = __bfloat162float(g[u][e]); a[u] = fmaf(f, f, a[u]); }
     }
-    float acc = (a0 + a1) + (a2 + a3);
+    float acc = 0.f;
+    #pragma unroll
+    for (int u = 0; u < NORM_PACKS; u++) acc += a[u];
     acc = block_sum(acc, red);
-    if (threadIdx.x == 0) partials[blockIdx.y * gridDim.x + blockIdx.x] = acc;
+    if (threadIdx.x == 0) partials[blockIdx.x] = acc;
 }
 
 // out[0] = scale * sum(partials[0..n)) in index order with a fixed tree: deterministic
@@ -110,12 +137,23 @@ adamw_kernel(bf16* __restrict__ params, float* __restrict__ master, const bf16* 
     }
 }
 
-// The same update on 8-element packs (128-bit accesses): every tensor slice of a transformer is a multiple of 8 elements, and so
-// are its ZeRO shards (the sharding rule demands it); the element-wise kernel above stays as the fallback for odd layouts.
+// The same update on packs (every tensor slice of a transformer is a multiple of 8 elements, and so
+// are its ZeRO shards: the sharding rule demands it); the element-wise kernel above stays as the fallback for odd layouts.
+// Bound by memory: 14 bytes read and 14 written per element.  A thread has groups of four elements whose neighbours belong to its neighbours in the warp, so that each
+// instruction covers whole sectors (with 8 elements, two 16-byte accesses side by side, every sector of the fp32 streams was asked for and written in two
+// halves); blocks are small, and there are many times more of them than fit at once, so that at any time a narrow range of each stream is read
+// and written.  Norm and update of 124 / 30 / 355 million parameters 576 / 154 / 1636 us (713 / 210 / 1942 before; 571 is the copy rate's time for the first), with as many
+// blocks as fit 650 / 170 / 1870, groups of eight elements 690 / - / 1890, one group per thread 639 / 178 / 1761.
+constexpr int PACK_THREADS = 128;
+constexpr int PACK_BLOCKS = 8;           // per SM
+constexpr int PACK_WAVES = 64;           // times as many blocks at most
+constexpr int PACK_QUADS = 2;            // groups of four elements of a thread
+DEVINL uint2 ld64cs(const bf16* p) { return __ldcs(reinterpret_cast<const uint2*>(p)); }
+
 template <bool HAS_MASTER>
-__global__ void __launch_bounds__(OPT_THREADS)
+__global__ void __launch_bounds__(PACK_THREADS, PACK_BLOCKS)
 adamw_pack_kernel(bf16* __restrict__ params, float* __restrict__ master, const bf16* __restrict__ grads,
-                  float* __restrict__ m_buf, float* __restrict__ v_buf, const TensorTable tab,
+                  float* __restrict__ m_buf, float* __restrict__ v_buf, const __grid_constant__ Chunks k,
                   float lr, float beta1, float beta2, float bc1, float bc2, float eps,
                   float grad_scale, const float* __restrict__ norm_sq, float grad_clip) {
     float scale = grad_scale;
@@ -125,39 +163,53 @@ adamw_pack_kernel(bf16* __restrict__ params, float* __restrict__ master, const b
         const float nrm = sqrtf(nsq);
         scale = (nrm > grad_clip) ? grad_scale * grad_clip / nrm : grad_scale;
     }
-    const TensorView tv = tab.t[blockIdx.y];
-    const long long packs_per_slice = tv.n >> 3;
-    const long long total = packs_per_slice * tv.L;
-    for (long long i = (long long)blockIdx.x * OPT_THREADS + threadIdx.x; i < total; i += (long long)gridDim.x * OPT_THREADS) {
-        const long long l = i / packs_per_slice, pk = i - l * packs_per_slice;
-        const long long pi = tv.p_base + l * tv.p_stride + pk * 8;
-        const long long oi = tv.o_base + l * tv.o_stride + pk * 8;
-        const bf16x8 g = ld128cs(grads + pi);
-        f32x4 m0 = ld128cs(m_buf + oi), m1 = ld128cs(m_buf + oi + 4), v0 = ld128cs(v_buf + oi), v1 = ld128cs(v_buf + oi + 4);
-        f32x4 w0, w1;
-        if (HAS_MASTER) { w0 = ld128cs(master + oi); w1 = ld128cs(master + oi + 4); }
-        else {
-            const bf16x8 pw = ld128(params + pi);
-            #pragma unroll
-            for (int e = 0; e < 4; e++) { w0[e] = __bfloat162float(pw[e]); w1[e] = __bfloat162float(pw[e + 4]); }
-        }
-        bf16x8 out;
+    constexpr int U = PACK_QUADS;
+    ChunkAt at;
+    for (int i = blockIdx.x; i < k.first[16]; i += gridDim.x) {
+        at.seek(k, i);
+        const TensorView& tv = k.tab.t[at.view];
+        const int l = at.l, c = at.c;
+        const long long quads = tv.n >> 2;
+        const long long pb = tv.p_base + l * tv.p_stride, ob = tv.o_base + l * tv.o_stride;
+        const float wd = tv.wd;
+        const unsigned int seed = tv.seed;
+        const int layer = l + tv.pad;
+        uint2 g[U];
+        f32x4 m[U], v[U], w[U];
         #pragma unroll
-        for (int e = 0; e < 8; e++) {
-            float& mm = e < 4 ? m0[e] : m1[e - 4];
-            float& vv = e < 4 ? v0[e] : v1[e - 4];
-            float& ww = e < 4 ? w0[e] : w1[e - 4];
-            const float gg = scale * __bfloat162float(g[e]);
-            mm = fmaf(beta1, mm, (1.0f - beta1) * gg);
-            vv = fmaf(beta2, vv, (1.0f - beta2) * gg * gg);
-            // the same expressions as the element-wise kernel (division by the bias corrections included), so both give the same bits
-            const float mh = mm / bc1, vh = vv / bc2;
-            ww = ww - lr * (mh / (sqrtf(vh) + eps) + tv.wd * ww);
-            out[e] = stochastic_round_bf16(ww, squirrel_noise5(sr_position(pk * 8 + e, (int)l + tv.pad), tv.seed));
+        for (int u = 0; u < U; u++) {
+            const long long q = (long long)(c * U + u) * PACK_THREADS + threadIdx.x;
+            if (q >= quads) continue;
+            g[u] = ld64cs(grads + pb + q * 4);
+            m[u] = ld128(m_buf + ob + q * 4); v[u] = ld128(v_buf + ob + q * 4);
+            if (HAS_MASTER) w[u] = ld128(master + ob + q * 4);
+            else {
+                const uint2 pw = *reinterpret_cast<const uint2*>(params + pb + q * 4);
+                const float2 a = unpack_bf16x2(pw.x), b = unpack_bf16x2(pw.y);
+                w[u][0] = a.x; w[u][1] = a.y; w[u][2] = b.x; w[u][3] = b.y;
+            }
         }
-        st128cs(m_buf + oi, m0); st128cs(m_buf + oi + 4, m1); st128cs(v_buf + oi, v0); st128cs(v_buf + oi + 4, v1);
-        if (HAS_MASTER) { st128cs(master + oi, w0); st128cs(master + oi + 4, w1); }
-        st128(params + pi, out);
+        #pragma unroll
+        for (int u = 0; u < U; u++) {
+            const long long q = (long long)(c * U + u) * PACK_THREADS + threadIdx.x;
+            if (q >= quads) continue;
+            const float2 ga = unpack_bf16x2(g[u].x), gb = unpack_bf16x2(g[u].y);
+            const float gf[4] = {ga.x, ga.y, gb.x, gb.y};
+            Pack64 out;
+            #pragma unroll
+            for (int e = 0; e < 4; e++) {
+                const float gg = scale * gf[e];
+                m[u][e] = fmaf(beta1, m[u][e], (1.0f - beta1) * gg);
+                v[u][e] = fmaf(beta2, v[u][e], (1.0f - beta2) * gg * gg);
+                // the same expressions as the element-wise kernel (division by the bias corrections included), so both give the same bits
+                const float mh = m[u][e] / bc1, vh = v[u][e] / bc2;
+                w[u][e] = w[u][e] - lr * (mh / (sqrtf(vh) + eps) + wd * w[u][e]);
+                out.v[e] = stochastic_round_bf16(w[u][e], squirrel_noise5(sr_position(q * 4 + e, layer), seed));
+            }
+            st128(m_buf + ob + q * 4, m[u]); st128(v_buf + ob + q * 4, v[u]);
+            if (HAS_MASTER) st128(master + ob + q * 4, w[u]);
+            *reinterpret_cast<uint2*>(params + pb + q * 4) = *reinterpret_cast<const uint2*>(&out);
+        }
     }
 }
 
@@ -196,15 +248,17 @@ extern "C" int llmc_sum_f32(float* out, const float* in, int n, float scale, cud
     return 0;
 }
 
-extern "C" int llmc_norm_sq_scratch() { return 16 * opt_grid_x(); }
+extern "C" int llmc_norm_sq_scratch() { return NORM_BLOCKS * opt_grid_x(); }
 
 // out[0] = sum of squares of the gradient elements covered by the table. `partials`: llmc_norm_sq_scratch floats.
 extern "C" int llmc_global_norm_sq(float* out, float* partials, const bf16* grads, const TensorTable* tab, cudaStream_t stream) {
-    const int gx = opt_grid_x();
+    if (tab->count < 1 || tab->count > 16) return -1;
     for (int i = 0; i < tab->count; i++) if (tab->t[i].n % 8 || tab->t[i].p_base % 8 || tab->t[i].p_stride % 8) return -1;
-    norm_sq_kernel<<<dim3(gx, tab->count), OPT_THREADS, 0, stream>>>(partials, grads, *tab);
+    const Chunks k(*tab, NORM_PACKS * NORM_THREADS * 8);
+    const int grid = llmc_norm_sq_scratch();
+    norm_sq_kernel<<<grid, NORM_THREADS, 0, stream>>>(partials, grads, k);
     CUDA_CHECK(cudaGetLastError());
-    final_sum_kernel<<<1, 1024, 0, stream>>>(out, partials, gx * tab->count);
+    final_sum_kernel<<<1, 1024, 0, stream>>>(out, partials, grid);
     CUDA_CHECK(cudaGetLastError());
     return 0;
 }
@@ -215,6 +269,7 @@ extern "C" int llmc_global_norm_sq(float* out, float* partials, const bf16* grad
 extern "C" int llmc_adamw(bf16* params, float* master, const bf16* grads, float* m, float* v, const TensorTable* tab,
                           float lr, float beta1, float beta2, float eps, int t, float grad_scale,
                           const float* norm_sq, float grad_clip, cudaStream_t stream) {
+    if (tab->count < 1 || tab->count > 16) return -1;
     const float bc1 = 1.0f - powf(beta1, (float)t), bc2 = 1.0f - powf(beta2, (float)t);
     dim3 grid(opt_grid_x() * 2, tab->count);
     bool packs = true;
@@ -223,8 +278,12 @@ extern "C" int llmc_adamw(bf16* params, float* master, const bf16* grads, float*
         if (tv.n % 8 || tv.p_base % 8 || tv.p_stride % 8 || tv.o_base % 8 || tv.o_stride % 8) packs = false;
     }
     if (packs) {
-        if (master) adamw_pack_kernel<true><<<grid, OPT_THREADS, 0, stream>>>(params, master, grads, m, v, *tab, lr, beta1, beta2, bc1, bc2, eps, grad_scale, norm_sq, grad_clip);
-        else adamw_pack_kernel<false><<<grid, OPT_THREADS, 0, stream>>>(params, master, grads, m, v, *tab, lr, beta1, beta2, bc1, bc2, eps, grad_scale, norm_sq, grad_clip);
+        const Chunks k(*tab, PACK_QUADS * PACK_THREADS * 4);
+        const int most = opt_grid_x() * PACK_BLOCKS * PACK_WAVES;
+        grid = dim3(k.total() < most ? k.total() : most);
+        if (k.total() == 0) return 0;
+        if (master) adamw_pack_kernel<true><<<grid, PACK_THREADS, 0, stream>>>(params, master, grads, m, v, k, lr, beta1, beta2, bc1, bc2, eps, grad_scale, norm_sq, grad_clip);
+        else adamw_pack_kernel<false><<<grid, PACK_THREADS, 0, stream>>>(params, master, grads, m, v, k, lr, beta1, beta2, bc1, bc2, eps, grad_scale, norm_sq, grad_clip);
     } else if (master) adamw_kernel<true><<<grid, OPT_THREADS, 0, stream>>>(params, master, grads, m, v, *tab, lr, beta1, beta2, bc1, bc2, eps, grad_scale, norm_sq, grad_clip);
     else adamw_kernel<false><<<grid, OPT_THREADS, 0, stream>>>(params, master, grads, m, v, *tab, lr, beta1, beta2, bc1, bc2, eps, grad_scale, norm_sq, grad_clip);
     CUDA_CHECK(cudaGetLastError());
