@@ -5,7 +5,7 @@
 #include "decoder_ops.h"
 
 // Kernel of a forward product, chosen by the caller (ops/kernels.py, forward_kernel)
-enum Product : int { GEMM = 0, GEMM2 = 1, STREAM = 2, GEMM2T = 3 };
+enum Product : int { GEMM = 0, GEMM2 = 1, STREAM = 2, GEMM2T = 3, SLICED = 4 };
 // MLP: up-projections and activation in two launches, or one of the two fused forms
 enum Mlp : int { MLP_TWO = 0, MLP_STREAM = 1, MLP_GEMM2T = 2 };
 
@@ -33,7 +33,7 @@ namespace {
 int product(int how, bf16* out, const bf16* x, const bf16* w, int M, int N, int K, cudaStream_t s) {
     switch (how) {
         case GEMM2T: return llmc_gemm2t_chained(out, x, w, M, N, K, K, K, N, s);
-        case STREAM: return llmc_stream_gemm_chained(out, x, w, M, N, K, K, K, N, s);
+        case STREAM: case SLICED: return llmc_stream_gemm_chained(out, x, w, M, N, K, K, K, N, how == SLICED ? 2 : 0, s);
         case GEMM2: return llmc_gemm2(x, w, out, nullptr, nullptr, M, N, K, K, K, N, 0, 0, 0, 0, 1, nullptr, nullptr, s);
         case GEMM: return llmc_gemm(x, w, out, nullptr, nullptr, M, N, K, K, K, N, 0, 0, 0, 0, 1, nullptr, nullptr, 0, s);
     }

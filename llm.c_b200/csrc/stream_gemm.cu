@@ -18,7 +18,8 @@
 // of 2048 channels, LM head of 128256 rows) this kernel took the step to 277 us; a weight-streaming kernel on warp-level MMAs with the same
 // early launch and prefetch, used for the products of at most 8 rows, left it at 290 us (at 284 us for the LM head alone), although launched
 // by itself it is faster (4 x 28672 x 4096 50 us against 59; skinny_gemm_kernel in decode.cu).  More rows (input gradients, in a chain, the training GEMM's tiles in
-// brackets): 256 x 768 x 768 4.9 us (6.3), 256 x 768 x 3072 7.9 us (16.3), 256 x 768 x 50304 44 us (291 after an L2 flush).
+// brackets): 256 x 768 x 768 4.9 us (6.3), 256 x 768 x 3072 7.9 us (16.3), 256 x 768 x 50304 44 us (291 after an L2 flush).  Forward products of some hundred rows
+// cut the same way against the tiles of gemm2t.cu: 256 x 768 x 768 5.1 us (6.2), 256 x 768 x 3072 7.9 (14.1), 512 x 2048 x 2048 11.2 (11.7).
 //
 // Warps of a CTA: 0 TMA producer, 1 MMA issuer, 2-5 epilogue.  Two CTAs fit an SM.
 #include "common.cuh"
@@ -389,7 +390,7 @@ Plan wide_plan(int M, int tiles, int num_kb, int sms) {
     return {nb, mtiles, pick_split(tiles * mtiles, num_kb, nb, sms)};
 }
 
-// Input gradients of more than 128 rows: tiles of about 64 rows (48 at M = 129) or more, as many as leave room for four slices of K each, or as few as
+// Input gradients of more than 128 rows, and forward products cut like them: tiles of about 64 rows (48 at M = 129) or more, as many as leave room for four slices of K each, or as few as
 // the 256 rows of a tile allow.  With the small ones a CTA's share of the reduction and its set-up are short; with the large ones fewer CTAs read the same
 // weights and K can be cut into more slices.  So shallow products take the small ones and deep ones the large ones.  Estimated in ns from the k-blocks of
 // a slice and the rows of a tile, coefficients fitted to 536 products (M 129 to 1024, N 384 to 4096, K 768 to 128256, each way of cutting), 5 and 8 %
@@ -416,20 +417,22 @@ Plan gradient_plan(int M, int tiles, int num_kb, int sms) {
     return cost_n <= cost_w ? narrow : wide;
 }
 
-Plan make_plan(int M, int N, int K, bool swiglu, bool w_mn) {
+// form: 0 a forward product, 1 an input gradient, 2 a forward product cut like one
+Plan make_plan(int M, int N, int K, bool swiglu, int form) {
     int sms = llmc_device_sm_count(); if (sms <= 0) sms = 148;
     const int tiles = CEIL_DIV(N, swiglu ? WR / 2 : WR), num_kb = CEIL_DIV(K, BK);
-    return w_mn && M > 128 ? gradient_plan(M, tiles, num_kb, sms) : wide_plan(M, tiles, num_kb, sms);
+    return form && M > 128 ? gradient_plan(M, tiles, num_kb, sms) : wide_plan(M, tiles, num_kb, sms);
 }
 
 template <int MODE, bool W_MN>
-int launch_stream(bf16* out, const bf16* x, const bf16* w, const bf16* bias, int M, int N, int K, int ldx, int ldw, int ldo, int early_w, cudaStream_t stream) {
+int launch_stream(bf16* out, const bf16* x, const bf16* w, const bf16* bias, int M, int N, int K, int ldx, int ldw, int ldo, int early_w, cudaStream_t stream,
+                  bool sliced = false) {
     if (M <= 0 || N <= 0 || K <= 0 || (K % 8) || (ldx % 8) || (ldw % 8) || ldx < K || ldw < (W_MN ? N : K) || ldo < N) return -1;
     if (W_MN && (N % 8)) return -1;
     Args g;
     g.early_w = early_w;
     g.out = out; g.bias = bias; g.w = w; g.M = M; g.N = N; g.K = K; g.ldo = ldo; g.ldw = ldw;
-    const Plan plan = make_plan(M, N, K, MODE == SWIGLU, W_MN);
+    const Plan plan = make_plan(M, N, K, MODE == SWIGLU, W_MN ? 1 : sliced ? 2 : 0);
     const int tiles = CEIL_DIV(N, MODE == SWIGLU ? WR / 2 : WR), mtiles = plan.mtiles, S = plan.S;
     int sms = llmc_device_sm_count(); if (sms <= 0) sms = 148;
     g.nb = plan.nb;
@@ -478,24 +481,25 @@ int launch_stream(bf16* out, const bf16* x, const bf16* w, const bf16* bias, int
 }  // namespace
 
 // How a plain product of these sizes is cut
-extern "C" void llmc_stream_gemm_plan(int M, int N, int K, int w_mn, int* rows, int* slices) {
-    const Plan p = make_plan(M, N, K, false, w_mn != 0);
+extern "C" void llmc_stream_gemm_plan(int M, int N, int K, int form, int* rows, int* slices) {
+    const Plan p = make_plan(M, N, K, false, form);
     *rows = p.nb; *slices = p.S;
 }
 
-// out (M, N) = x (M, K) . w (N, K)^T (+ bias), or x . w (K, N) with w_mn.  K, the row strides of x and w and, with w_mn, N are multiples of 8.
-extern "C" int llmc_stream_gemm(bf16* out, const bf16* x, const bf16* w, const bf16* bias, int M, int N, int K, int ldx, int ldw, int ldo, int w_mn,
+// out (M, N) = x (M, K) . w (N, K)^T (+ bias), form 0 or 2 (make_plan), or x . w (K, N), form 1.  K, the row strides of x and w and, in form 1, N are multiples of 8.
+extern "C" int llmc_stream_gemm(bf16* out, const bf16* x, const bf16* w, const bf16* bias, int M, int N, int K, int ldx, int ldw, int ldo, int form,
                                 cudaStream_t stream) {
     if (M <= 0 || N <= 0 || K <= 0) return 0;        // an empty product leaves out as it is, like the other two kernels'
-    if (w_mn) return launch_stream<STORE, true>(out, x, w, bias, M, N, K, ldx, ldw, ldo, 0, stream);
-    return launch_stream<STORE, false>(out, x, w, bias, M, N, K, ldx, ldw, ldo, 0, stream);
+    if (form == 1) return launch_stream<STORE, true>(out, x, w, bias, M, N, K, ldx, ldw, ldo, 0, stream);
+    return launch_stream<STORE, false>(out, x, w, bias, M, N, K, ldx, ldw, ldo, 0, stream, form == 2);
 }
 
 // The same behind a kernel that does not write w (csrc/decoder.cu): an early launch fills the stages with weights while that kernel drains.  What other
 // kernels before it wrote is complete: it triggers the launch after its own wait (pdl.cuh).
-extern "C" int llmc_stream_gemm_chained(bf16* out, const bf16* x, const bf16* w, int M, int N, int K, int ldx, int ldw, int ldo, cudaStream_t stream) {
+extern "C" int llmc_stream_gemm_chained(bf16* out, const bf16* x, const bf16* w, int M, int N, int K, int ldx, int ldw, int ldo, int form,
+                                        cudaStream_t stream) {
     if (M <= 0 || N <= 0 || K <= 0) return 0;
-    return launch_stream<STORE, false>(out, x, w, nullptr, M, N, K, ldx, ldw, ldo, 1, stream);
+    return launch_stream<STORE, false>(out, x, w, nullptr, M, N, K, ldx, ldw, ldo, 1, stream, form == 2);
 }
 
 // out (M, N) = (x . w1^T) * silu(x . w2^T) with w = [w1; w2] of 2 N rows, M <= 128; N a multiple of 64

@@ -95,8 +95,7 @@ def _few_rows(M, N, K, mode, b_mn, device):
     rows are resident at once and K pays for the reduction, which grows with the number of tiles (in a chain, theirs in brackets: 130 x 512 x 768
     4.4 (6.3), 256 x 768 x 768 4.9 (6.3), x 2304 7.0 (13.0), x 3072 7.9 (16.3), 512 x 768 x 768 6.1 (6.4), 1024 x 768 x 1600 9.8 (10.4),
     1024 x 1024 x 2304 11.7 (13.9); 384 x 2048 x 1024 8.3 (7.8), 1024 x 768 x 1024 8.5 (7.8), 512 x 1600 x 1600 10.7 (10.4)).  Forward products of more than 128 rows
-    below a depth of 6144 keep their one sum over K: at 8 us each (256 x 768 x 3072: 18 against 27) they are not worth another order of
-    summation in the loss.  At most 128 rows are summed in slices from K = 512 on, in fp32 and in slice order."""
+    that are cut into small row tiles too have a rule of their own (``_sliced``).  At most 128 rows are summed in slices from K = 512 on, in fp32 and in slice order."""
     if mode != MODE_STORE:
         return False
     wtiles = (N + 127) // 128
@@ -104,11 +103,24 @@ def _few_rows(M, N, K, mode, b_mn, device):
     if (K >= 6144 and tiles <= 64) or (b_mn and K >= 3072 and tiles <= 32):
         return True
     if b_mn and M > STREAM_MAX_ROWS:
-        narrow = (M + 127) // 128 * wtiles
-        return K >= max(768, 32 * narrow) and narrow * 4 <= 2 * (sm_count(device) * 7 // 8)
+        return _slices_pay(M, wtiles, K, device)
     if b_mn:
         return K >= 2048 and wtiles <= 2 * sm_count(device)
     return M <= 64 or (M <= STREAM_MAX_ROWS and wtiles <= 2 * sm_count(device))
+
+
+def _slices_pay(M, wtiles, K, device):
+    narrow = (M + 127) // 128 * wtiles
+    return K >= max(768, 32 * narrow) and narrow * 4 <= 2 * (sm_count(device) * 7 // 8)
+
+
+def _sliced(M, N, K, device):
+    """Whether a forward product of more than 128 rows goes to the split-K kernel with row tiles and slices like an input gradient's.  The line is the input
+    gradients' one: below it (fewer tiles, deeper) the slices win over the swapped kernel's one sum over K, above it they lose.  us in a chain, the swapped
+    kernel in brackets: 129 x 768 x 768 4.7 (6.0), 256 x 768 x 768 5.1 (6.2), 512 x 768 x 768 6.3 (6.3), 256 x 768 x 3072 7.9 (14.1), 1024 x 768 x 3072 12.1
+    (15.1), 256 x 384 x 1536 5.9 (8.8), 512 x 1024 x 1024 7.0 (7.3), 1024 x 1024 x 4096 14.7 (18.7), 512 x 2048 x 2048 11.2 (11.7), 300 x 2048 x 7168 16 (28; 20 in
+    row tiles of up to 256); beyond it 256 x 2304 x 768 7.6 (6.4), 777 x 1024 x 1024 8.7 (8.0), 2048 x 768 x 3072 21 (15).  The sums are fp32 and added in slice order."""
+    return M > STREAM_MAX_ROWS and K % 8 == 0 and _slices_pay(M, (N + 127) // 128, K, device)
 
 
 def _wide(M, N, device):
@@ -144,12 +156,14 @@ def _wgrad_two_sm(tiles256, K, accumulate, device):
     return K > 1024 or bool(accumulate) or tiles256 * 4 > sm_count(device)
 
 
-FORWARD_GEMM, FORWARD_GEMM2, FORWARD_STREAM, FORWARD_SWAPPED = range(4)        # csrc/decoder.cu, Product
+FORWARD_GEMM, FORWARD_GEMM2, FORWARD_STREAM, FORWARD_SWAPPED, FORWARD_SLICED = range(5)        # csrc/decoder.cu, Product
 
 
 def forward_kernel(M, N, K, device, aligned=True):
     """The kernel of a plain forward product without flags to wait for.  ``aligned``: the output starts on a 16-byte boundary.  The swapped kernel stores
     with TMA, which needs that and rows of whole 16 bytes; the split-K kernel takes any number of columns and any alignment."""
+    if TWO_SM_MIN_TILES > 0 and _sliced(M, N, K, device):
+        return FORWARD_SLICED
     if TWO_SM_MIN_TILES > 0 and N % 8 == 0 and aligned and _swapped(M, N, K, device):
         return FORWARD_SWAPPED
     if _few_rows(M, N, K, MODE_STORE, False, device) or _wide(M, N, device):
@@ -169,6 +183,9 @@ def gemm(a, b, d, M, N, K, lda, ldb, ldd, a_mn, b_mn, mode, bias=None, aux=None,
     plain = forward_kernel(M, N, K, d.device, d.data_ptr() % 16 == 0) if mode == MODE_STORE and not a_mn and not b_mn else None
     if plain == FORWARD_SWAPPED and ready is None:
         check(lib.llmc_gemm2t(_p(d), _p(a), _p(b), _p(bias), M, N, K, lda, ldb, ldd, 0, _stream()), "llmc_gemm2t")
+        return
+    if plain == FORWARD_SLICED and ready is None:
+        check(lib.llmc_stream_gemm(_p(d), _p(a), _p(b), _p(bias), M, N, K, lda, ldb, ldd, 2, _stream()), "llmc_stream_gemm")
         return
     if plain == FORWARD_STREAM or (not a_mn and _few_rows(M, N, K, mode, b_mn, d.device)):
         if ready is not None:

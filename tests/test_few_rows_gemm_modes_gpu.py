@@ -58,3 +58,16 @@ def test_dispatch(M, N, K, forward, gradient):
     assert KN._few_rows(M, N, K, KN.MODE_STORE, False, dev) == forward
     assert KN._few_rows(M, N, K, KN.MODE_STORE, True, dev) == gradient
     assert not KN._few_rows(M, N, K, KN.MODE_GELU, False, dev) and not KN._few_rows(M, N, K, KN.MODE_DGELU, True, dev)
+
+
+# forward products cut like input gradients: row tiles that do not divide the rows, ragged columns, a K tail, one row tile and many
+@pytest.mark.parametrize("M,N,K", [(129, 768, 768), (200, 130, 1000), (257, 999, 3080), (1000, 384, 1536), (300, 2048, 7168), (1024, 1024, 4096)])
+def test_sliced_forward(M, N, K):
+    assert KN.forward_kernel(M, N, K, torch.device(DEV, 0)) == KN.FORWARD_SLICED
+    x, w, b = rnd(M, K), rnd(N, K, scale=0.05, seed=1), rnd(N, seed=2)
+    buf = torch.full((M + 16, N), 7.0, dtype=torch.bfloat16, device=DEV)
+    KN.matmul_forward(buf[:M], x.to(DEV), w.to(DEV), b.to(DEV))
+    # against 64 bits: one rounding to bf16 (2^-9) of the sum and of nothing before it
+    ref = (x.double() @ w.double().t() + b.double()).float()
+    close(buf[:M], ref, 1e-3, 2.0 ** -8)
+    assert (buf[M:] == 7.0).all()
