@@ -148,6 +148,7 @@ class GPT:
         self.grad_hook = None
         # set by a communication backend whose all-gather may still be in flight when forward starts (parallel/p2p.py)
         self.step_graphs = StepGraphs()
+        self.chain_first_tokens = 1536         # captured passes of up to so many tokens (models/step_graphs.py, _capture)
         self.use_graphs = True          # replay small micro-steps from CUDA graphs (off: launch every kernel, for per-operator measurements)
         self.param_sync = None          # called as grad_hook(layer or -1 for the embeddings/final LN) on the last micro-step
 
@@ -311,9 +312,9 @@ class GPT:
         acc = micro_step > 0
         dres, dl_btc, dl_bt4c, dqkv = a["dresidual"], a["scratch_btc"], a["scratch_bt4c"], a["dqkv"]
         dlogits = a["logits"]
-        # gradients of weights and biases are read by nothing in this pass: in a captured graph they run beside the chain of input gradients, joined
-        # before a buffer that they read is overwritten (the partial sums by the next LayerNorm backward, dres by the one after it, since they take turns
-        # at two buffers, the others by the next layer).  4 x 64 tokens, us: one buffer 1512, two 1528, two and input gradients in slices of K 1498.
+        # gradients of weights and biases are read by nothing in this pass: in a captured graph they run beside the chain of input gradients, each joined
+        # before a buffer that it reads is written again (the partial sums by the next LayerNorm backward, dres by the one after it, since they take turns
+        # at two buffers, the others by the next layer)
         side = self.step_graphs.side
 
         with side.fork():
@@ -322,8 +323,8 @@ class GPT:
         # every LayerNorm backward also emits the column sums of the residual-stream gradient it leaves behind: that is the
         # bias gradient of the projection (fcproj / attproj) whose output was added to the stream just before that LayerNorm
         ops.layernorm_backward(dres, g["lnfw"], g["lnfb"], dl_btc, a["residual3"][L - 1], p["lnfw"], a["lnf_mean"], a["lnf_rstd"],
-                               accumulate_dinp=False, accumulate_dwdb=acc, dcolsum=g["fcprojb"][L - 1], accumulate_dcol=acc, sums_in=side.fork)
-        sums = side.mark()
+                               accumulate_dinp=False, accumulate_dwdb=acc, dcolsum=g["fcprojb"][L - 1], accumulate_dcol=acc, sums_in=side.fork_sums)
+        sums = side.mark_sums()
         nvtx = self.device.type == "cuda"
         for l in reversed(range(L)):
           with _Range("backward layer %d" % l, nvtx):
@@ -331,38 +332,51 @@ class GPT:
             lln = 0 if self.recompute >= 2 else l
             lg = 0 if self.recompute >= 1 else l
             if self.recompute >= 1:
+                side.free(a["fch_gelu"][lg])
                 ops.gelu_forward(a["fch_gelu"][lg], a["fch"][l])
             with side.fork():
                 ops.matmul_wgrad(g["fcprojw"][l], dres, a["fch_gelu"][lg], accumulate=acc)
+            side.read(dres, a["fch_gelu"][lg])
+            side.free(dl_bt4c)
             ops.matmul_dgrad(dl_bt4c, dres, p["fcprojw"][l], pre_gelu=a["fch"][l])
             if self.recompute >= 2:
+                side.free(a["ln2"][lln])
                 ops.layernorm_forward(a["ln2"][lln], None, None, a["residual2"][l], p["ln2w"][l], p["ln2b"][l])
-            with side.fork():
+            with side.fork_sums():
                 ops.bias_grad(g["fcb"][l], dl_bt4c, accumulate=acc)
+            with side.fork():
                 ops.matmul_wgrad(g["fcw"][l], dl_bt4c, a["ln2"][lln], accumulate=acc)
+            side.read(dl_bt4c, a["ln2"][lln])
             ops.matmul_dgrad(dl_btc, dl_bt4c, p["fcw"][l])
             side.join(sums)
             old, dres = dres, side.other(dres)
+            side.free(dres)
             ops.layernorm_backward(dres, g["ln2w"][l], g["ln2b"][l], dl_btc, a["residual2"][l], p["ln2w"][l], a["ln2_mean"][l],
                                    a["ln2_rstd"][l], accumulate_dinp=True, accumulate_dwdb=acc, dcolsum=g["attprojb"][l], accumulate_dcol=acc,
-                                   sums_in=side.fork, dinp_old=old)
-            sums = side.mark()
+                                   sums_in=side.fork_sums, dinp_old=old)
+            sums = side.mark_sums()
             with side.fork():
                 ops.matmul_wgrad(g["attprojw"][l], dres, a["atty"][l], accumulate=acc)
+            side.read(dres)
             ops.matmul_dgrad(dl_btc, dres, p["attprojw"][l])
+            side.free(dqkv)
             ops.attention_backward(dqkv, dl_btc, a["qkv"][l], a["atty"][l], a["lse"][l], B, T, NH)
             if self.recompute >= 2:
+                side.free(a["ln1"][lln])
                 ops.layernorm_forward(a["ln1"][lln], None, None, residual, p["ln1w"][l], p["ln1b"][l])
-            with side.fork():
+            with side.fork_sums():
                 ops.bias_grad(g["qkvb"][l], dqkv, accumulate=acc)
+            with side.fork():
                 ops.matmul_wgrad(g["qkvw"][l], dqkv, a["ln1"][lln], accumulate=acc)
+            side.read(dqkv, a["ln1"][lln])
             ops.matmul_dgrad(dl_btc, dqkv, p["qkvw"][l])
             side.join(sums)
             old, dres = dres, side.other(dres)
+            side.free(dres)
             ops.layernorm_backward(dres, g["ln1w"][l], g["ln1b"][l], dl_btc, residual, p["ln1w"][l], a["ln1_mean"][l],
                                    a["ln1_rstd"][l], accumulate_dinp=True, accumulate_dwdb=acc,
-                                   dcolsum=(g["fcprojb"][l - 1] if l > 0 else None), accumulate_dcol=acc, sums_in=side.refork, dinp_old=old)
-            sums = side.mark()
+                                   dcolsum=(g["fcprojb"][l - 1] if l > 0 else None), accumulate_dcol=acc, sums_in=side.fork_sums, dinp_old=old)
+            sums = side.mark_sums()
             if hook is not None:
                 hook(l)
         side.join()
