@@ -27,8 +27,8 @@ class DecoderCall(Structure):
     """Argument of llmc_decoder_forward (csrc/decoder.cu): addresses, then sizes."""
     _fields_ = [(n, c_void_p) for n in (
         "wte", "ln1w", "qkvw", "attprojw", "ln2w", "fc12w", "fcprojw", "lnfw", "lmhead", "freqs", "kcache", "vcache", "x", "ln", "raw", "q", "atty",
-        "proj", "res", "fc12", "h", "last", "logits", "rstd", "packed", "lse", "attention_ws", "tokens", "pos")] + [(n, c_int) for n in (
-            "L", "C", "H", "NH", "NKV", "HS", "vocab_rows", "logit_cols", "freqs_len", "max_batch", "cache_len", "B", "Tq", "start",
+        "proj", "res", "fc12", "h", "last", "logits", "logits32", "advance", "rstd", "packed", "lse", "attention_ws", "tokens", "pos")] + [(n, c_int) for n in (
+            "L", "C", "H", "NH", "NKV", "HS", "vocab_rows", "logit_cols", "vocab", "freqs_len", "max_batch", "cache_len", "B", "Tq", "start",
             "how_qkv", "how_attproj", "how_fc12", "how_fcproj", "how_head", "mlp")] + [("eps", c_float)]
 
 
@@ -98,6 +98,7 @@ def cuda():
         "llmc_stream_gemm": (I, [P, P, P, P, I, I, I, I, I, I, I, S]),
         "llmc_stream_gemm_swiglu": (I, [P, P, P, I, I, I, I, I, I, S]),
         "llmc_cached_attention": (I, [P, P, P, P, I, I, I, I, I, I, I, P, P, S]),
+        "llmc_cached_attention_rope": (I, [P, P, P, I, P, P, I, I, I, I, I, I, I, P, P, I, S]),
         "llmc_cached_attention_workspace": (L, [I, I, I, I, I, I]),
         "llmc_gelu_bwd_inplace": (I, [P, P, L, S]),
         "llmc_residual_add": (I, [P, P, P, L, S]),

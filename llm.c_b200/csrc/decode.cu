@@ -8,6 +8,8 @@
 //   cached_attention  out (N, NH, HS) = softmax(q . K[0 .. pos] / sqrt(HS)) V[0 .. pos] per (batch row, new token, head);
 //                     grouped queries read the cache head h / (NH / NKV) directly, nothing is expanded.
 //
+// llmc_cached_attention_rope does both in one launch where the fast kernel of the second is taken.
+//
 // start_pos comes from the host or, when `pos_ptr` is given, from device memory: a decoding step captured in a CUDA graph is
 // replayed with the position advanced on the device.  A device position that would leave the cache or the rotary table makes
 // the kernel record ST_BAD_ARG in the status word and return without touching memory.
@@ -17,6 +19,8 @@
 
 namespace {
 
+// one rotary pair
+DEVINL float2 rotate(float re, float im, float c, float s) { return make_float2(re * c - im * s, re * s + im * c); }
 DEVINL bf16x8 rotate8(const bf16x8& a, const float4& cs0, const float4& cs1) {
     bf16x8 r;
     const float c[4] = {cs0.x, cs0.z, cs1.x, cs1.z};
@@ -24,8 +28,9 @@ DEVINL bf16x8 rotate8(const bf16x8& a, const float4& cs0, const float4& cs1) {
     #pragma unroll
     for (int j = 0; j < 4; j++) {
         const float re = __bfloat162float(a[2 * j]), im = __bfloat162float(a[2 * j + 1]);
-        r[2 * j] = __float2bfloat16_rn(re * c[j] - im * s[j]);
-        r[2 * j + 1] = __float2bfloat16_rn(re * s[j] + im * c[j]);
+        const float2 t = rotate(re, im, c[j], s[j]);
+        r[2 * j] = __float2bfloat16_rn(t.x);
+        r[2 * j + 1] = __float2bfloat16_rn(t.y);
     }
     return r;
 }
@@ -214,18 +219,29 @@ template <int HS_> __host__ __device__ constexpr int ca_ring_bytes() { return CA
 template <int HS_> __host__ __device__ constexpr int ca_part_floats() { return CA_MAX_R * (HS_ + 2); }                                 // acc, max, sum of 8 rows
 template <int HS_> __host__ __device__ constexpr int ca_smem_bytes() { return CA_WARPS * ca_ring_bytes<HS_>() + ca_part_floats<HS_>() * 4; }
 
+// Where the queries and the new keys and values come from when they are not in q and the caches yet (ROPE): the output of the QKV projection
+struct Fresh {
+    const bf16* raw;           // (N, NH + 2 NKV, HS), not rotated
+    const float2* freqs;       // (freqs_len, HS / 2) cos, sin
+    int freqs_len;
+    int early;                 // no kernel directly in front of this one writes the caches or the position: cached keys are read before it has completed
+};
+
 // CLUSTER: the gridDim.x slices of a head are one cluster and `out` receives the result; otherwise the slice's partial goes to ws.
-template <int HS_, bool CLUSTER>
+// ROPE: the queries are rotated in registers; the warp whose tile a new key falls into rotates it, puts it and its value into the tile and writes both
+// to the caches.  A launch of its own for that (rope_cache_kernel) costs a decoding step 3 to 4 us in every layer.
+template <int HS_, bool CLUSTER, bool ROPE>
 __global__ void __launch_bounds__(CA_THREADS)
-cached_attention_split_kernel(bf16* __restrict__ out, float* __restrict__ ws, const bf16* __restrict__ q, const bf16* __restrict__ kcache,
-                              const bf16* __restrict__ vcache, int Tq, int Tmax, int start_pos, int NH, int NKV, float scale,
+cached_attention_split_kernel(bf16* __restrict__ out, float* __restrict__ ws, const bf16* __restrict__ q, const Fresh fresh, bf16* kcache,
+                              bf16* vcache, int Tq, int Tmax, int start_pos, int NH, int NKV, float scale,
                               const int* __restrict__ pos_ptr, unsigned int* status, int keys_per_slice, int rows) {
-    pdl_wait();
-    pdl_trigger();
+    const bool early = ROPE && fresh.early;
+    if (!early) { pdl_wait(); pdl_trigger(); }
     if (pos_ptr) {
         start_pos = *pos_ptr;
-        if (start_pos < 0 || start_pos + Tq > Tmax) {           // the same for every CTA of a cluster
-            if (threadIdx.x == 0 && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0) record_error(status, ST_BAD_ARG, 0x32);
+        if (start_pos < 0 || start_pos + Tq > Tmax || (ROPE && start_pos + Tq > fresh.freqs_len)) {           // the same for every CTA of a cluster
+            if (early) pdl_wait();             // the kernel behind this one relies on what is before it
+            if (threadIdx.x == 0 && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0) record_error(status, ST_BAD_ARG, ROPE ? 0x30 : 0x32);
             return;
         }
     }
@@ -246,8 +262,9 @@ cached_attention_split_kernel(bf16* __restrict__ out, float* __restrict__ ws, co
     const int k0 = min(nkeys, slice * keys_per_slice), k1 = min(nkeys, k0 + keys_per_slice);
 
     const long long row_stride = (long long)NKV * HS_;
-    const bf16* kbase = kcache + ((b * Tmax) * NKV + g) * HS_;
-    const bf16* vbase = vcache + ((b * Tmax) * NKV + g) * HS_;
+    bf16* kbase = kcache + ((b * Tmax) * NKV + g) * HS_;
+    bf16* vbase = vcache + ((b * Tmax) * NKV + g) * HS_;
+    const int cached = ROPE ? min(k1, start_pos) : k1;         // keys below are in the cache
     // K and V rows kt .. kt + 15 -> stage st; rows past the slice are zero, and so are their probabilities
     auto fetch = [&](int kt, int st) {
         if (kt < k1) {
@@ -257,8 +274,8 @@ cached_attention_split_kernel(bf16* __restrict__ out, float* __restrict__ ws, co
                 const int id = i * 32 + lane, row = id / CHUNKS, c = id % CHUNKS;
                 const long long src = min(kt + row, k1 - 1) * row_stride + c * 8;
                 const int off = row * ROWB + ((c ^ (row & 7)) * 16);
-                cp_async16_or_zero(dst + off, kbase + src, kt + row < k1);
-                cp_async16_or_zero(dst + CA_TILE * ROWB + off, vbase + src, kt + row < k1);
+                cp_async16_or_zero(dst + off, kbase + src, kt + row < cached);
+                cp_async16_or_zero(dst + CA_TILE * ROWB + off, vbase + src, kt + row < cached);
             }
         }
         cp_async_commit();                                     // possibly empty: the group count per tile stays one
@@ -267,17 +284,30 @@ cached_attention_split_kernel(bf16* __restrict__ out, float* __restrict__ ws, co
     const int kt0 = k0 + warp * CA_TILE;
     #pragma unroll
     for (int s = 0; s < CA_STAGES - 1; s++) fetch(kt0 + s * TSTEP, s);
+    if (early) { pdl_wait(); pdl_trigger(); }
 
     // query rows r -> token r / G, head g * G + r % G; the A operand of S: lane holds channels 2 tq4, 2 tq4 + 1 and + 8, + 9 of row gq.
     // Rows past `rows` are zero and dropped at the end.
     uint32_t qa[KS][2];
     {
         const int r = gq < rows ? gq : 0;
-        const bf16* qr = q + ((b * Tq + r / G) * NH + g * G + r % G) * HS_ + 2 * tq4;
+        const bf16* qr = ROPE ? fresh.raw + ((b * Tq + r / G) * (NH + 2 * NKV) + g * G + r % G) * HS_ + 2 * tq4
+                              : q + ((b * Tq + r / G) * NH + g * G + r % G) * HS_ + 2 * tq4;
         #pragma unroll
         for (int kk = 0; kk < KS; kk++) {
             qa[kk][0] = gq < rows ? *reinterpret_cast<const uint32_t*>(qr + kk * 16) : 0u;
             qa[kk][1] = gq < rows ? *reinterpret_cast<const uint32_t*>(qr + kk * 16 + 8) : 0u;
+        }
+        if (ROPE) {
+            // the two channels of a word are a rotary pair
+            const float2* fr = fresh.freqs + (size_t)(start_pos + r / G) * (HS_ / 2) + tq4;
+            #pragma unroll
+            for (int kk = 0; kk < KS; kk++)
+                #pragma unroll
+                for (int i = 0; i < 2; i++) {
+                    const float2 x = unpack_bf16x2(qa[kk][i]), f = fr[kk * 8 + i * 4], y = rotate(x.x, x.y, f.x, f.y);
+                    qa[kk][i] = pack_bf16x2(y.x, y.y);
+                }
         }
     }
     const int limit = min(k1, start_pos + (gq < rows ? gq : 0) / G + 1);      // keys [0, limit) are visible to this lane's row
@@ -294,6 +324,22 @@ cached_attention_split_kernel(bf16* __restrict__ out, float* __restrict__ ws, co
         cp_async_wait<CA_STAGES - 1>();
         __syncwarp();
         const uint32_t kb = smem_u32(ring + st * STAGE), vb = kb + CA_TILE * ROWB;
+        if (ROPE && kt + CA_TILE > start_pos) {
+            // new rows of this tile: 16 bytes of a key or of its value per lane
+            const int t0 = max(0, kt - start_pos), t1 = min(min(kt + CA_TILE, k1) - start_pos, Tq);
+            for (int id = lane; id < (t1 - t0) * 2 * CHUNKS; id += 32) {
+                const int t = t0 + id / (2 * CHUNKS), c = id % CHUNKS, row = start_pos + t - kt;
+                const bool value = (id / CHUNKS) & 1;
+                bf16x8 x = ld128(fresh.raw + ((b * Tq + t) * (NH + 2 * NKV) + NH + (value ? NKV : 0) + g) * HS_ + c * 8);
+                if (!value) {
+                    const float4* f = reinterpret_cast<const float4*>(fresh.freqs + (size_t)(start_pos + t) * (HS_ / 2) + c * 4);
+                    x = rotate8(x, f[0], f[1]);
+                }
+                st128((value ? vbase : kbase) + (kt + row) * row_stride + c * 8, x);
+                *reinterpret_cast<bf16x8*>(ring + st * STAGE + (value ? CA_TILE * ROWB : 0) + row * ROWB + ((c ^ (row & 7)) * 16)) = x;
+            }
+            __syncwarp();
+        }
         // ---- S (row gq, keys 2 tq4 + {0,1} of each group of 8 keys)
         float s[2][4];
         #pragma unroll
@@ -550,22 +596,33 @@ int ca_keys_per_slice(int B, int Tmax, int NKV) {
 int ca_slices(int B, int Tmax, int NKV) { return CEIL_DIV(Tmax, ca_keys_per_slice(B, Tmax, NKV)); }
 bool ca_fast(int Tq, int NH, int NKV, int HS) { return (HS == 64 || HS == 128) && (NH / NKV) * Tq <= CA_MAX_R; }
 
-template <int HS_, bool CLUSTER>
-int ca_launch(bf16* out, float* ws, const bf16* q, const bf16* kcache, const bf16* vcache, int B, int Tq, int Tmax, int start_pos, int NH,
+template <int HS_, bool CLUSTER, bool ROPE>
+int ca_launch(bf16* out, float* ws, const bf16* q, const Fresh& fresh, bf16* kcache, bf16* vcache, int B, int Tq, int Tmax, int start_pos, int NH,
               int NKV, const int* pos_ptr, cudaStream_t stream) {
     const int rows = (NH / NKV) * Tq, slices = ca_slices(B, Tmax, NKV);
     constexpr int smem = ca_smem_bytes<HS_>();
     static bool configured = false;
     if (!configured) {
-        CUDA_CHECK(cudaFuncSetAttribute(cached_attention_split_kernel<HS_, CLUSTER>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        CUDA_CHECK(cudaFuncSetAttribute(cached_attention_split_kernel<HS_, CLUSTER, ROPE>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
         configured = true;
     }
-    CUDA_CHECK(launch_pdl(cached_attention_split_kernel<HS_, CLUSTER>, dim3(slices, NKV, B), dim3(CA_THREADS), smem, stream, CLUSTER ? slices : 0,
-                          out, ws, q, kcache, vcache, Tq, Tmax, start_pos, NH, NKV, rsqrtf((float)HS_), pos_ptr, llmc_status_ptr(),
+    CUDA_CHECK(launch_pdl(cached_attention_split_kernel<HS_, CLUSTER, ROPE>, dim3(slices, NKV, B), dim3(CA_THREADS), smem, stream, CLUSTER ? slices : 0,
+                          out, ws, q, fresh, kcache, vcache, Tq, Tmax, start_pos, NH, NKV, rsqrtf((float)HS_), pos_ptr, llmc_status_ptr(),
                           ca_keys_per_slice(B, Tmax, NKV), rows));
     if (!CLUSTER)
         CUDA_CHECK(launch_pdl(cached_attention_combine_kernel<HS_>, dim3(rows, NKV, B), dim3(HS_), 0, stream, 0, out, (const float*)ws, Tq, NH, NKV, slices));
     return 0;
+}
+
+template <bool ROPE>
+int ca_dispatch(bf16* out, float* ws, const bf16* q, const Fresh& fresh, bf16* kcache, bf16* vcache, int B, int Tq, int Tmax, int start_pos, int NH,
+                int NKV, int HS, const int* pos_ptr, cudaStream_t stream) {
+    const bool cluster = ca_slices(B, Tmax, NKV) <= CA_MAX_CLUSTER;
+#define CA_GO(H, CL) return ca_launch<H, CL, ROPE>(out, ws, q, fresh, kcache, vcache, B, Tq, Tmax, start_pos, NH, NKV, pos_ptr, stream)
+    if (HS == 64) { if (cluster) CA_GO(64, true); CA_GO(64, false); }
+    if (cluster) CA_GO(128, true);
+    CA_GO(128, false);
+#undef CA_GO
 }
 }  // namespace
 
@@ -583,17 +640,27 @@ extern "C" int llmc_cached_attention(bf16* out, const bf16* q, const bf16* kcach
     const bool cluster = ca_fast(Tq, NH, NKV, HS) && ca_slices(B, Tmax, NKV) <= CA_MAX_CLUSTER;
     if (ca_fast(Tq, NH, NKV, HS) && (cluster || ws != nullptr)) {
         if ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(kcache) | reinterpret_cast<uintptr_t>(vcache)) & 15) return -5;
-#define CA_GO(H, CL) return ca_launch<H, CL>(out, ws, q, kcache, vcache, B, Tq, Tmax, start_pos, NH, NKV, pos_ptr, stream)
-        if (HS == 64) { if (cluster) CA_GO(64, true); CA_GO(64, false); }
-        if (cluster) CA_GO(128, true);
-        CA_GO(128, false);
-#undef CA_GO
+        return ca_dispatch<false>(out, ws, q, Fresh{}, const_cast<bf16*>(kcache), const_cast<bf16*>(vcache), B, Tq, Tmax, start_pos, NH, NKV, HS, pos_ptr, stream);
     }
     const dim3 grid(NH, Tq, B);
     cached_attention_kernel<<<grid, DEC_THREADS, 0, stream>>>(out, q, kcache, vcache, Tq, Tmax, start_pos, NH, NKV, HS, rsqrtf((float)HS),
                                                               pos_ptr, llmc_status_ptr());
     CUDA_CHECK(cudaGetLastError());
     return 0;
+}
+
+// llmc_rope_cache and llmc_cached_attention in one launch, from the output of the QKV projection; the same bits.  For what the fast path of the
+// second takes (head width 64 or 128, at most 8 query rows per cached head, a workspace where it needs one); otherwise -6, and nothing is done.
+// early: the kernel in front writes neither the caches nor the position (csrc/decoder.cu); what others before it wrote is complete (pdl.cuh).
+extern "C" int llmc_cached_attention_rope(bf16* out, const bf16* raw, const float* freqs, int freqs_len, bf16* kcache, bf16* vcache, int B, int Tq, int Tmax,
+                                          int start_pos, int NH, int NKV, int HS, const int* pos_ptr, float* ws, int early, cudaStream_t stream) {
+    const int rc = decode_check(B, Tq, Tmax, start_pos, NH, NKV, HS, pos_ptr != nullptr);
+    if (rc) return rc;
+    if (!pos_ptr && start_pos + Tq > freqs_len) return -4;
+    if (!ca_fast(Tq, NH, NKV, HS) || (ca_slices(B, Tmax, NKV) > CA_MAX_CLUSTER && ws == nullptr)) return -6;
+    if ((reinterpret_cast<uintptr_t>(raw) | reinterpret_cast<uintptr_t>(kcache) | reinterpret_cast<uintptr_t>(vcache) | reinterpret_cast<uintptr_t>(freqs)) & 15) return -6;
+    const Fresh fresh = {raw, reinterpret_cast<const float2*>(freqs), freqs_len, early};
+    return ca_dispatch<true>(out, ws, nullptr, fresh, kcache, vcache, B, Tq, Tmax, start_pos, NH, NKV, HS, pos_ptr, stream);
 }
 
 // out (M, N) = x (M, K) . w (N, K)^T for M <= 8; K and the row strides of x and w are multiples of 8 elements.

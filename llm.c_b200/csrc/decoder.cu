@@ -18,11 +18,13 @@ struct DecoderCall {
     bf16 *kcache, *vcache;
     // activations, at least B * Tq rows (last, logits: B)
     bf16 *x, *ln, *raw, *q, *atty, *proj, *res, *fc12, *h, *last, *logits;
+    float* logits32;                      // (B, vocab) logits as the caller wants them, for the streamed head (null: bf16 in logits)
+    int* advance;                         // position to add 1 to, with logits32 (null: none)
     float* rstd;
     bf16* packed; float* lse;             // dense prompts only (null: attention over the cache)
     float* attention_ws;                  // of llmc_cached_attention, null where it needs none
     const int* tokens; const int* pos;    // pos: position on the device (null: start)
-    int L, C, H, NH, NKV, HS, vocab_rows, logit_cols, freqs_len, max_batch, cache_len;
+    int L, C, H, NH, NKV, HS, vocab_rows, logit_cols, vocab, freqs_len, max_batch, cache_len;
     int B, Tq, start;
     int how_qkv, how_attproj, how_fc12, how_fcproj, how_head, mlp;
     float eps;
@@ -59,6 +61,10 @@ extern "C" int llmc_decoder_forward(const DecoderCall* c, int* launches, cudaStr
         if (dense) {
             GO(llmc_rope_fwd_cache(c->packed, c->raw, c->freqs, kc, vc, c->cache_len, N, c->Tq, c->NH, c->NKV, c->HS, s));
             GO(llmc_attention_fwd(c->atty, c->lse, c->packed, c->B, c->Tq, c->NH, c->HS, s));
+        } else if ((rc = llmc_cached_attention_rope(c->atty, c->raw, c->freqs, c->freqs_len, kc, vc, c->B, c->Tq, c->cache_len, c->start, c->NH, c->NKV, c->HS,
+                                                    c->pos, c->attention_ws, 1, s)) != -6) {
+            if (rc) return rc;
+            n += c->attention_ws ? 2 : 1;
         } else {
             GO(llmc_rope_cache(c->q, kc, vc, c->raw, c->freqs, c->freqs_len, c->B, c->Tq, c->cache_len, c->start, c->NH, c->NKV, c->HS, c->pos, s));
             GO(llmc_cached_attention(c->atty, c->q, kc, vc, c->B, c->Tq, c->cache_len, c->start, c->NH, c->NKV, c->HS, c->pos, c->attention_ws, s));
@@ -84,7 +90,8 @@ extern "C" int llmc_decoder_forward(const DecoderCall* c, int* launches, cudaStr
                                      cudaMemcpyDeviceToDevice, s));
         last = c->last;
     }
-    GO(product(c->how_head, c->logits, last, c->lmhead, c->B, c->logit_cols, C, s));
+    if (c->logits32) GO(llmc_stream_gemm_logits(c->logits32, c->vocab, last, c->lmhead, c->B, c->logit_cols, C, C, C, c->advance, s));
+    else GO(product(c->how_head, c->logits, last, c->lmhead, c->B, c->logit_cols, C, s));
 #undef GO
     *launches = n;
     return 0;

@@ -15,8 +15,11 @@ int llmc_rope_cache(bf16* q, bf16* kcache, bf16* vcache, const bf16* raw, const 
 int llmc_attention_fwd(bf16* out, float* lse, const bf16* qkv, int B, int T, int NH, int hs, cudaStream_t stream);
 int llmc_cached_attention(bf16* out, const bf16* q, const bf16* kcache, const bf16* vcache, int B, int Tq, int Tmax, int start_pos, int NH, int NKV,
                           int HS, const int* pos_ptr, float* ws, cudaStream_t stream);
+int llmc_cached_attention_rope(bf16* out, const bf16* raw, const float* freqs, int freqs_len, bf16* kcache, bf16* vcache, int B, int Tq, int Tmax,
+                               int start_pos, int NH, int NKV, int HS, const int* pos_ptr, float* ws, int early, cudaStream_t stream);
 int llmc_swiglu_fwd(bf16* h, const bf16* x12, long long N, int H, cudaStream_t stream);
 int llmc_stream_gemm_chained(bf16* out, const bf16* x, const bf16* w, int M, int N, int K, int ldx, int ldw, int ldo, int form, cudaStream_t stream);
+int llmc_stream_gemm_logits(float* out, int cols, const bf16* x, const bf16* w, int M, int N, int K, int ldx, int ldw, int* advance, cudaStream_t stream);
 int llmc_stream_gemm_swiglu_chained(bf16* out, const bf16* x, const bf16* w, int M, int N, int K, int ldx, int ldw, int ldo, cudaStream_t stream);
 int llmc_gemm2t_chained(bf16* out, const bf16* x, const bf16* w, int M, int N, int K, int ldx, int ldw, int ldo, cudaStream_t stream);
 int llmc_gemm2t_swiglu_chained(bf16* out, const bf16* x, const bf16* w, int M, int N, int K, int ldx, int ldw, int ldo, cudaStream_t stream);

@@ -43,6 +43,8 @@ enum Mode : int { STORE = 0, SWIGLU = 1 };
 
 struct Args {
     bf16* out;
+    float* out32; int cols32;  // in place of out (null: out): the bf16 results as fp32, the first cols32 columns, in rows of as many
+    int* advance;              // a counter to add 1 to (null: none)
     const bf16* bias;          // N entries or null (STORE)
     const bf16* w;             // for the prefetch
     int M, N, K, ldo, ldw;
@@ -74,6 +76,7 @@ DEVINL void sum_peers(float (&f)[4], uint32_t addr, uint32_t S) {
     #pragma unroll
     for (uint32_t s = 1; s < MAX_SPLIT; s++) if (s < S) { f[0] += p[s].x; f[1] += p[s].y; f[2] += p[s].z; f[3] += p[s].w; }
 }
+DEVINL float round_bf16(float v) { return __bfloat162float(__float2bfloat16_rn(v)); }
 DEVINL void prefetch_l2(const void* p, uint32_t bytes) {
     asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
 }
@@ -150,6 +153,7 @@ stream_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
     __syncwarp();
     pdl_wait();
     pdl_trigger();
+    if (g.advance != nullptr && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 64) *g.advance += 1;
 
     if (warp == 0) {
         if (lane == 0) {
@@ -228,7 +232,10 @@ stream_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
                 #pragma unroll
                 for (int e = 0; e < 4; e++) f[e] += bias[e];
             }
-            if (vec) {
+            if (MODE == STORE && g.out32 != nullptr) {
+                #pragma unroll
+                for (int e = 0; e < 4; e++) if (n + e < g.cols32) g.out32[(size_t)(m0 + m) * g.cols32 + n + e] = round_bf16(f[e]);
+            } else if (vec) {
                 *reinterpret_cast<uint2*>(g.out + at) = make_uint2(pack_bf16x2(f[0], f[1]), pack_bf16x2(f[2], f[3]));
             } else {
                 #pragma unroll
@@ -295,6 +302,7 @@ stream_wide_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
     __syncwarp();
     pdl_wait();
     pdl_trigger();
+    if (g.advance != nullptr && blockIdx.x == 0 && threadIdx.x == 64) *g.advance += 1;
 
     if (warp == 0) {
         if (lane == 0) {
@@ -351,9 +359,15 @@ stream_wide_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
                 uint32_t v[16];
                 tmem_ld16(tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + buf * acc_cols + c, v);
                 tmem_ld_wait();
-                #pragma unroll
-                for (int e = 0; e < 16; e++)
-                    if (c + e < g.M && n < g.N) g.out[(size_t)(c + e) * g.ldo + n] = __float2bfloat16_rn(__uint_as_float(v[e]) + bias);
+                if (g.out32 != nullptr) {
+                    #pragma unroll
+                    for (int e = 0; e < 16; e++)
+                        if (c + e < g.M && n < g.cols32) g.out32[(size_t)(c + e) * g.cols32 + n] = round_bf16(__uint_as_float(v[e]) + bias);
+                } else {
+                    #pragma unroll
+                    for (int e = 0; e < 16; e++)
+                        if (c + e < g.M && n < g.N) g.out[(size_t)(c + e) * g.ldo + n] = __float2bfloat16_rn(__uint_as_float(v[e]) + bias);
+                }
             }
             tc_fence_before();
             __syncwarp();
@@ -426,11 +440,12 @@ Plan make_plan(int M, int N, int K, bool swiglu, int form) {
 
 template <int MODE, bool W_MN>
 int launch_stream(bf16* out, const bf16* x, const bf16* w, const bf16* bias, int M, int N, int K, int ldx, int ldw, int ldo, int early_w, cudaStream_t stream,
-                  bool sliced = false) {
+                  bool sliced = false, float* out32 = nullptr, int cols32 = 0, int* advance = nullptr) {
     if (M <= 0 || N <= 0 || K <= 0 || (K % 8) || (ldx % 8) || (ldw % 8) || ldx < K || ldw < (W_MN ? N : K) || ldo < N) return -1;
     if (W_MN && (N % 8)) return -1;
     Args g;
     g.early_w = early_w;
+    g.out32 = out32; g.cols32 = cols32; g.advance = advance;
     g.out = out; g.bias = bias; g.w = w; g.M = M; g.N = N; g.K = K; g.ldo = ldo; g.ldw = ldw;
     const Plan plan = make_plan(M, N, K, MODE == SWIGLU, W_MN ? 1 : sliced ? 2 : 0);
     const int tiles = CEIL_DIV(N, MODE == SWIGLU ? WR / 2 : WR), mtiles = plan.mtiles, S = plan.S;
@@ -510,4 +525,11 @@ extern "C" int llmc_stream_gemm_swiglu(bf16* out, const bf16* x, const bf16* w, 
 extern "C" int llmc_stream_gemm_swiglu_chained(bf16* out, const bf16* x, const bf16* w, int M, int N, int K, int ldx, int ldw, int ldo, cudaStream_t stream) {
     if (N % 64 || M > 128) return -1;
     return launch_stream<SWIGLU, false>(out, x, w, nullptr, M, N, K, ldx, ldw, ldo, 1, stream);
+}
+
+// The last product of a decoding pass: its bf16 results as fp32, the first `cols` columns in rows of as many, and, where a counter is given, 1 added to it (the
+// position of a replayed step).  In launches of their own the conversion and the addition took 7 us of a step of 4 rows and 15 of one of 32 (128256 columns).
+extern "C" int llmc_stream_gemm_logits(float* out, int cols, const bf16* x, const bf16* w, int M, int N, int K, int ldx, int ldw, int* advance, cudaStream_t stream) {
+    if (M <= 0 || N <= 0 || K <= 0 || cols <= 0 || cols > N) return -1;
+    return launch_stream<STORE, false>(nullptr, x, w, nullptr, M, N, K, ldx, ldw, N, 1, stream, false, out, cols, advance);
 }

@@ -72,6 +72,10 @@ class CachedDecoder:
         """tokens (B, Tq) int32 on the model's device: the tokens at positions start_pos .. start_pos + Tq - 1 of every row.
         Returns the fp32 logits (B, vocab_size) of the last of them; keys and values of all of them enter the cache.
         With ``pos`` (one int32 on the device) the position is read by the kernels when they run and start_pos is ignored."""
+        return self._forward(tokens, start_pos, pos, False)[0]
+
+    def _forward(self, tokens, start_pos, pos, advance):
+        """``forward``, and whether 1 has been added to ``pos``, which ``advance`` asks for."""
         m = self.model
         cfg, p = m.cfg, m.params
         B, Tq = tokens.shape
@@ -94,8 +98,10 @@ class CachedDecoder:
                                torch.zeros(B * NH * Tq, dtype=torch.float32, device=m.device))
             packed, lse = self._dense[0][:N], self._dense[1][:B * NH * Tq].view(B, NH, Tq)
         if self.native and self.skinny_rows == kernels.STREAM_MAX_ROWS and kernels.decoder_layout_ok(self):
-            kernels.decoder_forward(self, a, (packed, lse) if dense else None, tokens, start_pos, pos)
-            return a["logits"][:B, :cfg.vocab_size].float()
+            logits = kernels.decoder_forward(self, a, (packed, lse) if dense else None, tokens, start_pos, pos, **({"advance": True} if advance else {}))
+            if logits is not None:
+                return logits, advance
+            return a["logits"][:B, :cfg.vocab_size].float(), False
 
         def mm(out, inp, weight, n):
             if self.whole_tiles and n > self.skinny_rows:
@@ -111,8 +117,7 @@ class CachedDecoder:
                 ops.rope_forward(packed, a["raw"][:N], m.freqs, Tq, NH, NKV, self.kcache[l], self.vcache[l])
                 ops.attention_forward(a["atty"][:N], lse, packed, B, Tq, NH)
             else:
-                ops.rope_cache(a["q"][:N], self.kcache[l], self.vcache[l], a["raw"][:N], m.freqs, Tq, start_pos, NH, NKV, pos)
-                ops.cached_attention(a["atty"][:N], a["q"][:N], self.kcache[l], self.vcache[l], Tq, start_pos, NH, NKV, pos)
+                ops.rope_cached_attention(a["atty"][:N], a["q"][:N], self.kcache[l], self.vcache[l], a["raw"][:N], m.freqs, Tq, start_pos, NH, NKV, pos)
             mm(a["proj"], a["atty"], p["attprojw"][l], N)
             ops.rmsnorm_fused_residual_forward(a["res"][:N], ln[:N], rstd[:N], x[:N], a["proj"][:N], p["ln2w"][l], eps)
             if N <= min(self.skinny_rows, 128) and cfg.hidden_dim % 64 == 0:
@@ -130,7 +135,7 @@ class CachedDecoder:
             last = a["last"]
             last[:B].copy_(ln[:N].view(B, Tq, C)[:, -1])
         mm(a["logits"], last, p["lmhead"], B)
-        return a["logits"][:B, :cfg.vocab_size].float()
+        return a["logits"][:B, :cfg.vocab_size].float(), False
 
 
 class GraphStep:
@@ -150,8 +155,9 @@ class GraphStep:
         torch.cuda.current_stream(dev).wait_stream(side)       # what it wrote at start_pos is overwritten by the first real step
         self.graph = torch.cuda.CUDAGraph()
         with kernels.scratch_taken() as scratch, torch.cuda.graph(self.graph):
-            self.logits = decoder.forward(self.tokens, 0, pos=self.pos)
-            self.pos.add_(1)
+            self.logits, advanced = decoder._forward(self.tokens, 0, self.pos, True)
+            if not advanced:
+                self.pos.add_(1)
         # the graph holds addresses: a longer prompt replaces the decoder's activation buffers, another caller the scratch buffers
         self._held = (scratch, decoder._bufs, decoder.kcache, decoder.vcache, decoder.model.freqs)
 

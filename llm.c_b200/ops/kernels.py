@@ -499,6 +499,24 @@ def cached_attention(out, q, kcache, vcache, Tq, start_pos, NH, NKV, pos=None):
           "llmc_cached_attention")
 
 
+def rope_cached_attention(out, q, kcache, vcache, raw, freqs, Tq, start_pos, NH, NKV, pos=None):
+    """``rope_cache`` and ``cached_attention`` on its results; ``q`` is scratch.  Decoding steps run in one launch, with the same bits (16 rows of 4 layers of 2048 channels:
+    279 us a step in two launches per layer, see csrc/decode.cu)."""
+    global _launches
+    lib = _lib.cuda()
+    N, HS = raw.shape[0], kcache.shape[-1]
+    B, Tmax = N // Tq, kcache.shape[1]
+    words = lib.llmc_cached_attention_workspace(B, Tq, Tmax, NH, NKV, HS)
+    ws = _scratch.get("cached_attention", words, torch.float32, raw.device) if words > 0 else None
+    rc = lib.llmc_cached_attention_rope(_p(out), _p(raw), _p(freqs), freqs.shape[0], _p(kcache), _p(vcache), B, Tq, Tmax, start_pos, NH, NKV, HS, _p(pos), _p(ws), 0, _stream())
+    if rc != -6:
+        check(rc, "llmc_cached_attention_rope")
+        _launches += 2 if words > 0 else 1
+        return
+    rope_cache(q, kcache, vcache, raw, freqs, Tq, start_pos, NH, NKV, pos)
+    cached_attention(out, q, kcache, vcache, Tq, start_pos, NH, NKV, pos)
+
+
 def matmul_skinny(out, inp, weight):
     """out[M,OC] = inp[M,C] @ weight[OC,C]^T for at most 8 rows on warp-level MMAs (csrc/decode.cu); ``matmul_forward`` takes such products too, faster
     behind another kernel of this library and slower alone."""
@@ -551,9 +569,10 @@ def decoder_layout_ok(decoder):
         and k.is_contiguous() and v.is_contiguous()
 
 
-def decoder_forward(decoder, bufs, dense, tokens, start_pos, pos):
+def decoder_forward(decoder, bufs, dense, tokens, start_pos, pos, advance=False):
     """The launches of ``models.generate.CachedDecoder.forward`` for a bf16 model, from native code (csrc/decoder.cu).  ``bufs``: the decoder's activation
-    buffers; ``dense``: (packed QKV, LSE) buffers for a prompt from position 0, or None."""
+    buffers; ``dense``: (packed QKV, LSE) buffers for a prompt from position 0, or None.  Returns the fp32 logits (B, vocab_size) where the head's kernel writes
+    them, after adding 1 to ``pos`` if ``advance`` asks for it, else None: bf16 logits are in ``bufs``."""
     m = decoder.model
     cfg, p, dev = m.cfg, m.params, m.device
     B, Tq = tokens.shape
@@ -570,18 +589,23 @@ def decoder_forward(decoder, bufs, dense, tokens, start_pos, pos):
     words = 0 if dense else lib.llmc_cached_attention_workspace(B, Tq, cache_len, NH, NKV, HS)
     ws = _scratch.get("cached_attention", words, torch.float32, dev) if words > 0 else None
     a = lambda t: None if t is None else t.data_ptr()
+    # the streamed head writes the logits as they are returned; other heads (more than 128 rows) bf16
+    how_head = forward_kernel(B, logit_cols, C, dev)
+    logits32 = torch.empty(B, cfg.vocab_size, dtype=torch.float32, device=dev) if how_head == FORWARD_STREAM else None
     call = _lib.DecoderCall(
         **{n: p[n].data_ptr() for n in ("wte", "ln1w", "qkvw", "attprojw", "ln2w", "fc12w", "fcprojw", "lnfw", "lmhead")},
         **{n: bufs[n].data_ptr() for n in ("x", "ln", "raw", "q", "atty", "proj", "res", "fc12", "h", "last", "logits", "rstd")},
         freqs=m.freqs.data_ptr(), kcache=decoder.kcache.data_ptr(), vcache=decoder.vcache.data_ptr(), packed=a(dense and dense[0]), lse=a(dense and dense[1]),
         attention_ws=a(ws), tokens=tokens.data_ptr(), pos=a(pos),
-        L=cfg.num_layers, C=C, H=H, NH=NH, NKV=NKV, HS=HS, vocab_rows=p["wte"].shape[0], logit_cols=logit_cols, freqs_len=m.freqs.shape[0],
+        logits32=a(logits32), advance=a(pos) if advance and logits32 is not None else None,
+        L=cfg.num_layers, C=C, H=H, NH=NH, NKV=NKV, HS=HS, vocab_rows=p["wte"].shape[0], logit_cols=logit_cols, vocab=cfg.vocab_size, freqs_len=m.freqs.shape[0],
         max_batch=decoder.kcache.shape[1], cache_len=cache_len, B=B, Tq=Tq, start=0 if pos is not None else start_pos,
         how_qkv=forward_kernel(N, heads * HS, C, dev), how_attproj=forward_kernel(N, C, C, dev), how_fc12=forward_kernel(N, 2 * H, C, dev),
-        how_fcproj=forward_kernel(N, C, H, dev), how_head=forward_kernel(B, logit_cols, C, dev), mlp=mlp, eps=cfg.norm_eps)
+        how_fcproj=forward_kernel(N, C, H, dev), how_head=how_head, mlp=mlp, eps=cfg.norm_eps)
     launches = ctypes.c_int(0)
     check(lib.llmc_decoder_forward(ctypes.byref(call), ctypes.byref(launches), _stream()), "llmc_decoder_forward")
     count_launches(launches.value)
+    return logits32
 
 
 def make_table(views):

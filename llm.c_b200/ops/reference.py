@@ -370,6 +370,11 @@ def cached_attention(out, q, kcache, vcache, Tq, start_pos, NH, NKV, pos=None):
     out.view(B, Tq, NH, HS).copy_(y.transpose(1, 2))
 
 
+def rope_cached_attention(out, q, kcache, vcache, raw, freqs, Tq, start_pos, NH, NKV, pos=None):
+    rope_cache(q, kcache, vcache, raw, freqs, Tq, start_pos, NH, NKV, pos)
+    cached_attention(out, q, kcache, vcache, Tq, start_pos, NH, NKV, pos)
+
+
 def matmul_skinny(out, inp, weight):
     out.copy_(_f(inp) @ _f(weight).t())
 

@@ -1,0 +1,52 @@
+"""Rotary embedding, cache and attention of a decoding step in one launch against the two launches it replaces: the same bits."""
+import pytest
+import torch
+
+from llmc_b200 import _lib
+from llmc_b200.ops import kernels as KN
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+# the first key, new keys at both ends of a tile of 16 and across two, of a slice and across two, several slices, more slices than a cluster holds,
+# a cache with more rows than the batch
+@pytest.mark.parametrize("B,Tq,start,Tmax,NH,NKV,HS", [
+    (1, 1, 0, 8, 2, 2, 64), (2, 1, 15, 192, 8, 2, 64), (2, 1, 16, 192, 8, 2, 64), (3, 8, 12, 64, 2, 2, 128), (1, 2, 127, 1024, 8, 2, 128), (1, 2, 128, 1024, 8, 2, 128),
+    (3, 1, 1500, 1600, 4, 1, 128), (1, 1, 9000, 9100, 2, 1, 64), (40, 1, 77, 300, 16, 8, 64), (1, 8, 250, 258, 2, 2, 128), (32, 1, 2000, 2048, 32, 8, 128)])
+@pytest.mark.parametrize("device_pos", [False, True])
+def test_same_bits(B, Tq, start, Tmax, NH, NKV, HS, device_pos):
+    g = torch.Generator(device=DEV).manual_seed(start + B)
+    rnd = lambda *s: torch.randn(*s, generator=g, device=DEV).bfloat16()
+    raw, k, v = rnd(B * Tq, (NH + 2 * NKV) * HS), rnd(B + 1, Tmax, NKV, HS), rnd(B + 1, Tmax, NKV, HS)
+    k[:, start:], v[:, start:] = float("nan"), float("nan")             # what no query may see
+    freqs = torch.randn(Tmax + 3, HS // 2, 2, generator=g, device=DEV)
+    pos = torch.tensor([start], dtype=torch.int32, device=DEV) if device_pos else None
+    got = []
+    for fused in (True, False):
+        kc, vc, q = k.clone(), v.clone(), torch.zeros(B * Tq, NH * HS, dtype=torch.bfloat16, device=DEV)
+        out = torch.full((B * Tq + 1, NH * HS), 7.0, dtype=torch.bfloat16, device=DEV)
+        before = KN.launch_count()
+        if fused:
+            KN.rope_cached_attention(out[:-1], q, kc, vc, raw, freqs, Tq, 0 if device_pos else start, NH, NKV, pos)
+            launches = KN.launch_count() - before
+        else:
+            KN.rope_cache(q, kc, vc, raw, freqs, Tq, 0 if device_pos else start, NH, NKV, pos)
+            KN.cached_attention(out[:-1], q, kc, vc, Tq, 0 if device_pos else start, NH, NKV, pos)
+            assert KN.launch_count() - before == launches + 1
+        got.append((out, kc, vc))
+    assert _lib.read_status() == 0
+    for a, b in zip(*got):
+        assert torch.equal(torch.nan_to_num(a, 1e4), torch.nan_to_num(b, 1e4))
+    assert torch.isfinite(got[0][0]).all() and torch.equal(got[0][1][B:].isnan(), k[B:].isnan())
+
+
+def test_position_outside_the_cache_or_the_table():
+    raw, out = torch.zeros(1, 4 * 64, dtype=torch.bfloat16, device=DEV), torch.full((1, 128), 7.0, dtype=torch.bfloat16, device=DEV)
+    k, v = torch.zeros(1, 40, 1, 64, dtype=torch.bfloat16, device=DEV), torch.zeros(1, 40, 1, 64, dtype=torch.bfloat16, device=DEV)
+    for rows, at in ((40, 40), (30, 30), (40, -1)):
+        freqs = torch.zeros(rows, 32, 2, device=DEV)
+        KN.rope_cached_attention(out, out.clone(), k, v, raw, freqs, 1, 0, 2, 1, torch.tensor([at], dtype=torch.int32, device=DEV))
+        assert _lib.read_status() != 0 and (out == 7.0).all()
+    with pytest.raises(_lib.KernelError):
+        KN.rope_cached_attention(out, out.clone(), k, v, raw, torch.zeros(30, 32, 2, device=DEV), 1, 30, 2, 1)
