@@ -168,7 +168,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 27);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_index(), lane = threadIdx.x & 31;
     const int nt = CEIL_DIV(a.T, BT);
 
     if (threadIdx.x == 0) {

@@ -153,7 +153,7 @@ attn_bwd1_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constan
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 25);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_index(), lane = threadIdx.x & 31;
     const int nt = CEIL_DIV(a.T, BT);
     const int G = (nt + 1) >> 1;                      // key-tile groups {g, nt-1-g}
     const int total = a.B * a.NH * G;

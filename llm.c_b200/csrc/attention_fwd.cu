@@ -12,10 +12,10 @@
 //     score product: the next item's Q tile arrives while that slot finishes its last softmax and its epilogue.
 // Bound by the softmax of the two slots (1024 exponential cycles per 128 x 128 tile each) with the tensor pipe right behind (2 x 1024
 // cycles per key tile).  Measured, with the kernel this one replaces (16 softmax warps exchanging row statistics, P through shared
-// memory) in brackets: B=16 T=2048 NH=8 HS=128 178 us (256), B=2 T=4096 NH=32 HS=128 296 us (422), B=3 T=1000 NH=32 HS=80 47 us (68).
-// Letting the maximum lag by up to 2^8, as the 64-wide kernel does, takes 167 / 274 / 44 us, but then the largest probability of a row is not 1
+// memory) in brackets: B=16 T=2048 NH=8 HS=128 166 us (256), B=2 T=4096 NH=32 HS=128 280 us (422), B=3 T=1000 NH=32 HS=80 39 us (68).
+// Letting the maximum lag by up to 2^8, as the 64-wide kernel does, took 167 / 274 / 44 us where this took 178 / 296 / 47, but then the largest probability of a row is not 1
 // and is rounded to bf16 like the others: the error against 64 bits grows by 1 % (0.00200 -> 0.00204 on the last case).
-// Handing P over in two halves, so that the product starts under the second half's exponentials, was slower (174 / 281 us).
+// Handing P over in two halves, so that the product starts under the second half's exponentials, was slower than that (174 / 281 us).
 //
 // Items are dealt to the persistent CTAs heaviest first in alternating direction, which evens out their decreasing lengths.
 //
@@ -86,7 +86,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 18);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_index(), lane = threadIdx.x & 31;
     const int nq = CEIL_DIV(a.T, BT);
 
     if (threadIdx.x == 0) {

@@ -19,13 +19,13 @@
 // slots took 1200 cycles a step), an item's Q tile arrives under the item before, and its output leaves from its own Q buffer.  Key tiles of 64 and the P-over-S
 // overlay are what lets four slots into tensor memory and two CTAs into shared memory; the softmax loop is short enough for the instruction caches (with
 // 128-column tiles and every branch unrolled a warp waited for instructions longer than for anything else).  A part of the exponentials runs on the
-// FMA pipe (ex2_poly2): one pair of eight in the ordinary kernel (none / one / two: 187 / 178 / 186 us at 64 x 1024 x 12), two in DUO (13.8 / 13.2 us for two
-// and one at 1 x 777 x 32).
+// FMA pipe (ex2_poly2): one pair of eight in the ordinary kernel (none / one / two: 177 / 171 / 175 us at 64 x 1024 x 12), two in DUO (none / one / two: 16.1 /
+// 16.0 / 14.9 us at 1 x 777 x 32).
 //
 // DUO: where the query tiles are so few that SMs would get one chain only, a CTA works on ONE query tile, its slots on alternate key tiles, and adds the two
 // at the end.  us, with the kernel this one replaces (one CTA of two slots per SM, tiles of 128 keys, slots taking turns at the exponentials) in brackets, B x T x heads:
-// 64 x 1024 x 12 178 (205), 2 x 4096 x 32 197 (226), 64 x 256 x 12 25.7 (32.7), 8 x 1024 x 12 29.4 (34.4); DUO 1 x 777 x 32 13.2 (14.8), 4 x 512 x 12 10.4 (11.2),
-// 3 x 1000 x 16 19.6 (23.3), 1 x 2048 x 25 27.7 (41.3), 1 x 129 x 32 5.9 (7.1).
+// 64 x 1024 x 12 171 (205), 2 x 4096 x 32 192 (225), 64 x 256 x 12 24.0 (32.8), 8 x 1024 x 12 28.7 (34.4); DUO 1 x 777 x 32 14.7 (14.7), 4 x 512 x 12 10.4 (11.1),
+// 3 x 1000 x 16 19.2 (23.2), 1 x 2048 x 25 27.0 (41.2), 1 x 129 x 32 5.6 (7.1).
 //
 // TMEM columns of a CTA: S_A [0,64)  O_A [64,128)  S_B [128,192)  O_B [192,256); P_X: the first 32 columns of S_X (64 bf16 per row)
 //
@@ -106,7 +106,7 @@ attn_fwd1_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(kv_empty + RING);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_index(), lane = threadIdx.x & 31;
 
     if (threadIdx.x == 0) {
         if ((smem_u32(smem) & 1023u) != 0) record_error(a.status, ST_BAD_ARG, 0x18);

@@ -190,10 +190,10 @@ DEVINL uint64_t f2_add(uint64_t a, uint64_t b) { uint64_t r; asm("add.rn.f32x2 %
 DEVINL uint64_t f2_both(float v) { return f2_pack(v, v); }
 // The larger of three in one instruction (two cycles of a scheduler, like the larger of two); a NaN loses, as in fmaxf
 DEVINL float max3(float a, float b, float c) { float r; asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c)); return r; }
-// 2^x of two numbers on the FMA pipe, for loops that keep the special-function unit busy (ex2 takes 8 cycles of a scheduler there, these two 9 each
+// 2^x of two numbers on the FMA pipe, for loops that keep the special-function unit busy (ex2 takes 8 cycles of a scheduler there, these two 10 each
 // here).  Cody and Waite's reduction: x = n + f with n the nearest integer, read from the low bits of x + 1.5 * 2^23; 2^f by a polynomial of degree 5 with
-// 2^0 = 1, fitted for the least relative error on [-1/2, 1/2] (linear programme: 7e-8 in exact arithmetic); n is added to the exponent.  Error against 64 bits on [-30, 0]
-// 2.2e-7 at most, 8e-8 rms.  For x < 64; below -125 the result is that of -125 (2.4e-38), a NaN becomes a value that is no smaller than 2^127.
+// 2^0 = 1, fitted for the least relative error on [-1/2, 1/2] (linear programme: 7e-8 in exact arithmetic).  Error against 64 bits on [-30, 0]
+// 2.2e-7 at most, 8e-8 rms.  For x < 64; below -125 the result is that of -125 (2.4e-38).
 DEVINL float2 ex2_poly2(uint64_t x) {
     float2 v = f2_unpack(x);
     asm("max.NaN.f32 %0, %0, %1;" : "+f"(v.x) : "f"(-125.0f));
@@ -206,8 +206,9 @@ DEVINL float2 ex2_poly2(uint64_t x) {
     p = f2_fma(p, f, f2_both(0.24022166430950165f));
     p = f2_fma(p, f, f2_both(0.6931465864181519f));
     p = f2_fma(p, f, f2_both(1.0f));
-    const float2 r = f2_unpack(p), n = f2_unpack(t);
-    return make_float2(__uint_as_float(__float_as_uint(r.x) + (__float_as_uint(n.x) << 23)), __uint_as_float(__float_as_uint(r.y) + (__float_as_uint(n.y) << 23)));
+    // times 2^n by a multiplication: a NaN stays one
+    const float2 n = f2_unpack(t);
+    return f2_unpack(f2_mul(p, f2_pack_u((__float_as_uint(n.x) << 23) + 0x3f800000u, (__float_as_uint(n.y) << 23) + 0x3f800000u)));
 }
 
 // GELU with the tanh approximation, 0.5 x (1 + tanh(k (x + 0.044715 x^3))), and its derivative, scalar and in pairs.  Both forms evaluate
@@ -477,6 +478,11 @@ DEVINL void turn_pass(int bar, float& dep) { asm volatile("bar.arrive %1, 64;" :
 template <int N> DEVINL void regs_shrink() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
 template <int N> DEVINL void regs_grow() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
 
+// The warp's index in its block, by a shuffle that makes it known to be the same in all lanes: what follows from it (a role's barriers, tiles and descriptors) goes
+// to uniform registers, which the tensor and TMA instructions want, instead of being moved there at each use.  That counts where an issuer's instructions lie on the
+// chain of every tile.  Attention, us without / with: 64 x 1024 x 12 heads of 64 forward 212 / 177, backward 391 / 369, 2 x 4096 x 32 of 128 forward 289 / 280.
+// The matrix products, whose issuer runs ahead of its accumulators, take the same time with either.
+DEVINL int warp_index() { return __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0); }
 DEVINL bool elect_one() {
     uint32_t pred;
     asm volatile(

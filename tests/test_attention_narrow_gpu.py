@@ -62,3 +62,18 @@ def test_forward_slots(B, T, NH, ramp):
     # P and O rounded to bf16 once each: 0.0016 together; LSE of up to 200 in fp32
     assert float((out[:B].float().cpu() - ro).norm() / ro.norm()) < 4e-3
     assert float((lse.cpu() - rl).abs().max()) < 1e-4 + 2e-6 * float(rl.abs().max())
+
+
+@pytest.mark.parametrize("B", [1, 40])                # one / two query tiles to a CTA
+def test_a_nan_key_reaches_its_queries(B):
+    """Head h has a NaN in key 3 h: every place of a group of exponentials, whichever unit takes it."""
+    T, NH = 130, 24
+    qkv = torch.randn(B, T, 3, NH, 64, generator=torch.Generator().manual_seed(B)).bfloat16()
+    for h in range(NH):
+        qkv[:, 3 * h, 1, h, 5] = float("nan")
+    out, lse = torch.empty(B, T, NH * 64, dtype=torch.bfloat16, device=DEV), torch.empty(B, NH, T, device=DEV)
+    KN.attention_forward(out, lse, qkv.view(B, T, -1).to(DEV), B, T, NH)
+    assert _lib.read_status() == 0
+    seen = torch.arange(T)[None, :] >= 3 * torch.arange(NH)[:, None]                     # (NH, T)
+    assert torch.equal(lse.isnan().cpu(), seen.expand(B, -1, -1))
+    assert torch.equal(out.view(B, T, NH, 64).isnan().cpu(), seen.t()[None, :, :, None].expand(B, -1, -1, 64))
