@@ -113,7 +113,7 @@ def cuda():
         "llmc_attention_fwd": (I, [P, P, P, I, I, I, I, S]),
         "llmc_attention_bwd": (I, [P, P, P, P, P, P, I, I, I, I, S]),
         "llmc_attention_bwd_workspace": (L, [I, I, I, I]),
-        "llmc_attention_bwd_launches": (I, [I, I]),
+        "llmc_attention_bwd_launches": (I, [I, I, I, I]),
         # full-precision operator set (csrc/fp32_ops.cu)
         "llmc_f32_gelu_fwd": (I, [P, P, L, S]),
         "llmc_f32_gelu_bwd": (I, [P, P, L, S]),

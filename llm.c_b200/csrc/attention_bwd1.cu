@@ -18,6 +18,8 @@
 // the persistent CTAs is balanced.  dK_j / dV_j leave the CTA once per key tile.  What item g contributes to dQ_i is written as
 // fp32 to a slot of its own in a workspace (the second key tile is added to what the first left there by a reducing bulk copy
 // of the same CTA, ordered after the first); a second kernel adds the slots of a query tile in the order of g and rounds once.
+// With many heads of few tiles (whole_heads) a CTA takes all units of a head instead and sums dQ_i in one slot: what the slot holds is fetched into the
+// staging buffer behind the pair before, the drain warps add to it there, and the last key tile's sum is rounded and written for good.
 // No atomics, no ordering between CTAs: the gradients are bit-reproducible, which the reference also demands of cuDNN
 // (llmc/cudnn_att.cpp:186-191), and no CTA ever waits for another one.
 //
@@ -73,12 +75,13 @@ static_assert(SMEM <= 232448, "shared memory of one CTA");
 
 struct Args {
     bf16* dqkv;          // (B, T, 3, NH, 64)
-    float* dq_ws;        // [B*NH][slots][16 column groups][128 rows][4] fp32: slot_of(i) + g holds what unit g adds to query tile i
+    float* dq_ws;        // [B*NH][slots][16 column groups][128 rows][4] fp32: slot_of(i) + g holds what unit g adds to query tile i; WHOLE: [CTAs][nt] such slots
     const float* lse;    // (B, NH, T)
     const float* delta;  // (B, NH, T); null (one tile per sequence): computed here from out and dout
     const bf16* out;     // (B, T, NH, 64)
     const bf16* dout;
-    int B, T, NH;
+    int T, NH;
+    int item0, items;    // this launch takes items item0 .. items - 1
     float scale, scale_log2e;
     int early;           // the next kernel may start while this one runs
     unsigned int* status;
@@ -98,6 +101,8 @@ template <int N> struct Groups { static constexpr int value = N; };
 __host__ __device__ inline int slot_of(int i, int G) { return i <= G ? i * (i + 1) / 2 : G * (G + 1) / 2 + (i - G) * G; }
 
 // The sequence of pairs of one CTA: items w (round-robin), their one or two key tiles, the query tiles i >= j of each.
+// WHOLE: an item is a head, all its units in the order of g.
+template <bool WHOLE>
 struct Walk {
     int w, total, G, nt, stride, NH;
     int bh, b, h, g, seg, j, i;
@@ -107,12 +112,16 @@ struct Walk {
         if (w < total) item();
     }
     DEVINL bool valid() const { return w < total; }
-    DEVINL void item() { bh = w / G; g = w - bh * G; b = bh / NH; h = bh - b * NH; seg = 0; j = g; i = j; }
+    DEVINL void item() {
+        if (WHOLE) { bh = w; g = 0; } else { bh = w / G; g = w - bh * G; }
+        b = bh / NH; h = bh - b * NH; seg = 0; j = g; i = j;
+    }
     DEVINL bool first_of_tile() const { return i == j; }
     DEVINL bool last_of_tile() const { return i == nt - 1; }
     DEVINL void next() {                      // valid() turns false past the last pair
         if (++i < nt) return;
         if (seg == 0 && 2 * g != nt - 1) { seg = 1; j = nt - 1 - g; i = j; return; }
+        if (WHOLE && ++g < G) { seg = 0; j = g; i = j; return; }
         w += stride;
         if (w < total) item();
     }
@@ -122,10 +131,12 @@ struct Walk {
 // registers of the first: 5 % of every size.)  us, the other form first: 128 sequences of 16 x 25 heads 107, 79, 64 of 40 x 25 heads 57, 46, 4 of 64 x 12
 // heads 7.7, 7.4.  Three loads save too little of four unless the CTAs have several items each: 128 of 80 x 25 heads 116, 107, 4 of 80 x 12 heads 7.9, 8.4.
 constexpr int SHORT_T = 64, SHORT_T_MANY = 96;
-template <bool SHORT>
+enum { SPLIT = 0, SHORT_SPLIT = 1, WHOLE_HEADS = 2 };
+template <int MODE>
 __global__ void __launch_bounds__(THREADS, 1)
 attn_bwd1_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant__ CUtensorMap tmDO,
                  const __grid_constant__ CUtensorMap tmDQKV, const Args a) {
+    constexpr bool SHORT = MODE == SHORT_SPLIT, WHOLE = MODE == WHOLE_HEADS;
     extern __shared__ __align__(1024) uint8_t smem[];
     uint8_t* sRes = smem;                              // [RB][K_j, V_j]
     uint8_t* sStr = sRes + RB * PAIR_BYTES;            // [XSTAGES][Q_i, dO_i]
@@ -150,13 +161,13 @@ attn_bwd1_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constan
     uint64_t* acc_empty = bars + 20;  // the drain warps hold them                   (4 arrivals)
     uint64_t* st_full = bars + 21;    // [2] statistics table of a pair written      (2 arrivals)
     uint64_t* st_empty = bars + 23;   // [2] ... and read by every softmax warp      (8 arrivals)
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 25);
+    uint64_t* part_full = bars + 25;  // WHOLE: what a query tile has so far is in the staging buffer
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 26);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
     const int warp = warp_index(), lane = threadIdx.x & 31;
     const int nt = CEIL_DIV(a.T, BT);
     const int G = (nt + 1) >> 1;                      // key-tile groups {g, nt-1-g}
-    const int total = a.B * a.NH * G;
     const int nslots = slot_of(nt, G);
 
     if (threadIdx.x == 0) {
@@ -165,7 +176,7 @@ attn_bwd1_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constan
         for (int i = 0; i < XSTAGES; i++) { mbar_init(&x_full[i], 1); mbar_init(&x_empty[i], 1); }
         mbar_init(s_full, 1); mbar_init(s_empty, 8); mbar_init(dp_full, 1); mbar_init(p_ready, 8); mbar_init(p_empty, 1);
         mbar_init(ds_ready, 8); mbar_init(ds_empty, 1); mbar_init(dq_full, 1); mbar_init(dq_empty, 4);
-        mbar_init(acc_full, 1); mbar_init(acc_empty, 4);
+        mbar_init(acc_full, 1); mbar_init(acc_empty, 4); mbar_init(part_full, 1);
         *abort_flag = 0;
         mbar_fence_init();
         tma_prefetch_desc(&tmQKV); tma_prefetch_desc(&tmDO); tma_prefetch_desc(&tmDQKV);
@@ -183,8 +194,8 @@ attn_bwd1_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constan
     // time stamps of CTA 0's first TRACE_PAIRS pairs, one thread per role, for the timeline tool (llmc_attention_bwd_set_trace)
 #define TRACE(role, ev) do { if (a.trace != nullptr && blockIdx.x == 0 && t < TRACE_PAIRS) a.trace[((role) * 8 + (ev)) * TRACE_PAIRS + t] = clock64(); } while (0)
 
-    Walk wk;
-    wk.start(blockIdx.x, total, G, nt, gridDim.x, a.NH);
+    Walk<WHOLE> wk;
+    wk.start(a.item0 + blockIdx.x, a.items, G, nt, gridDim.x, a.NH);
 
     if (warp == 0) {
         // ---------------------------------------------------------------- TMA producer
@@ -256,7 +267,7 @@ attn_bwd1_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constan
             if (ok) { issue_s(0, 0); issue_dp(0, 0); }
             while (ok) {
                 // pair t = wk; the pair after it, if any
-                Walk nx = wk; nx.next();
+                Walk<WHOLE> nx = wk; nx.next();
                 const bool have_next = nx.valid();
                 const int rb = kvt & 1;
                 const int nst = st + 1 == XSTAGES ? 0 : st + 1;
@@ -528,7 +539,7 @@ attn_bwd1_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constan
         const bool issuer = warp == 12 && lane == 0;
         bool ok = true;
         bool staged = false;
-        uint32_t t = 0;
+        uint32_t t = 0, parts = 0;
         int kvt = 0;
         for (; wk.valid(); t++) {
             const int bh = wk.bh, b = wk.b, h = wk.h, i = wk.i, j = wk.j;
@@ -544,8 +555,11 @@ attn_bwd1_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constan
             if (threadIdx.x == 384) TRACE(2, 1);
             // through the staging buffer and one bulk copy: 16 global stores per thread and pair through the load/store unit held up
             // the shared-memory reads of the softmax warps for about a thousand cycles per pair (measured)
-            float* slot = a.dq_ws + ((size_t)bh * nslots + slot_of(i, G) + g) * SLOT_FLOATS;
-            if (seg == 1 && issuer) {
+            // WHOLE: one slot per query tile, of the CTA.  What it holds was fetched into the staging buffer behind the pair before; the last key tile's sum is
+            // rounded and leaves for good.
+            float* slot = a.dq_ws + (WHOLE ? (size_t)blockIdx.x * nt + i : (size_t)bh * nslots + slot_of(i, G) + g) * SLOT_FLOATS;
+            const bool more = WHOLE && j > 0, done = WHOLE ? j == min(i, nt >> 1) : nt == 1;
+            if (!WHOLE && seg == 1 && issuer) {
                 if (nt - j == 1) tma_store_wait<0>(); else if (nt - j == 2) tma_store_wait<1>(); else tma_store_wait<2>();
             }
             {
@@ -556,13 +570,26 @@ attn_bwd1_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constan
                 tc_fence_before();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(dq_empty);
-                if (staged) { if (issuer) tma_store_wait_read<0>(); asm volatile("bar.sync 1, 128;" ::: "memory"); }      // the previous copy has read the buffer
-                if (nt > 1) {
+                if (more) {
+                    ok = mbar_wait_relaxed(part_full, parts & 1, abort_flag, a.status, 0x6b3) && ok;
+                    parts++;
+                    #pragma unroll
+                    for (int e = 0; e < 16; e++) {
+                        const float4 s4 = *reinterpret_cast<const float4*>(sOut + e * (BT * 16) + rr * 16);
+                        v[4 * e] = __float_as_uint(s4.x + __uint_as_float(v[4 * e])); v[4 * e + 1] = __float_as_uint(s4.y + __uint_as_float(v[4 * e + 1]));
+                        v[4 * e + 2] = __float_as_uint(s4.z + __uint_as_float(v[4 * e + 2])); v[4 * e + 3] = __float_as_uint(s4.w + __uint_as_float(v[4 * e + 3]));
+                    }
+                    if (done) asm volatile("bar.sync 1, 128;" ::: "memory");        // all have read what the rounded rows go over
+                } else if (staged) {
+                    if (issuer) tma_store_wait_read<0>();                           // the previous copy has read the buffer
+                    asm volatile("bar.sync 1, 128;" ::: "memory");
+                }
+                if (!done) {
                     #pragma unroll
                     for (int e = 0; e < 16; e++)
                         *reinterpret_cast<uint4*>(sOut + e * (BT * 16) + rr * 16) = make_uint4(v[4 * e], v[4 * e + 1], v[4 * e + 2], v[4 * e + 3]);
                 } else {
-                    // a single tile: dQ is finished
+                    // dQ is finished
                     #pragma unroll
                     for (int u = 0; u < 8; u++) {
                         uint4 o;
@@ -577,9 +604,9 @@ attn_bwd1_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constan
             fence_async_smem();
             asm volatile("bar.sync 1, 128;" ::: "memory");
             if (issuer && ok) {
-                if (nt == 1)
+                if (done)
                     tma_store_4d(&tmDQKV, sOut, 0, h, i * BT, b);
-                else if (seg == 0)
+                else if (WHOLE || seg == 0)
                     asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;"
                                  ::"l"(slot), "r"(smem_u32(sOut)), "r"(SLOT_FLOATS * 4) : "memory");
                 else
@@ -621,6 +648,14 @@ attn_bwd1_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constan
                 staged = true;
                 kvt++;
             }
+            if (WHOLE && wk.valid() && wk.j > 0 && issuer && ok) {
+                // what the next pair's query tile has so far.  Its last addition left nt - j pairs ago or more.
+                if (nt - wk.j == 1) tma_store_wait<0>(); else if (nt - wk.j == 2) tma_store_wait<1>(); else tma_store_wait<2>();
+                tma_store_wait_read<0>();
+                mbar_expect_tx(part_full, SLOT_FLOATS * 4);
+                asm volatile("cp.async.bulk.shared::cta.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                             ::"r"(smem_u32(sOut)), "l"(a.dq_ws + ((size_t)blockIdx.x * nt + wk.i) * SLOT_FLOATS), "r"(SLOT_FLOATS * 4), "r"(smem_u32(part_full)) : "memory");
+            }
         }
         if (issuer) tma_store_wait<0>();
     }
@@ -641,11 +676,11 @@ attn_bwd1_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constan
 // [4 floats]): a warp reads 512 contiguous bytes per instruction, every thread has 16 loads of 16 bytes in flight (two slots);
 // the sums are transposed through shared memory so that the 8 lanes of a row store its 128 bytes together.
 __global__ void __launch_bounds__(256)
-dq_fold_kernel(bf16* __restrict__ dqkv, const float* __restrict__ ws, int B, int T, int NH, int nt) {
+dq_fold_kernel(bf16* __restrict__ dqkv, const float* __restrict__ ws, int bh0, int T, int NH, int nt) {
     __shared__ __align__(16) bf16 tile[BT][HS + 8];
-    const int nbh = B * NH;
+    const int nbh = gridDim.x / nt;
     const int i = nt - 1 - (int)(blockIdx.x / nbh);
-    const int bh = (int)(blockIdx.x % nbh);
+    const int bh = bh0 + (int)(blockIdx.x % nbh);
     const int G = (nt + 1) >> 1, n = min(i, G - 1) + 1;
     const int t = threadIdx.x;
     const float* src = ws + ((size_t)bh * slot_of(nt, G) + slot_of(i, G)) * SLOT_FLOATS + t * 4;
@@ -697,6 +732,22 @@ dq_fold_kernel(bf16* __restrict__ dqkv, const float* __restrict__ ws, int B, int
 
 }  // namespace
 
+// How many heads, the first ones, are dealt to CTAs whole (WHOLE_HEADS); the others are split into units over the CTAs and folded.
+// Whole up to 10 tiles: the CTAs' slots, 32 KB a tile, then stay in L2 (47 MB of its 126), so that dQ costs no memory traffic before its last rounding.  us of the
+// three or four launches, split in brackets, B x T x heads: 64 x 1024 x 12 459 (523), 128 x 384 x 12 177 (278), 64 x 256 x 12 63 (85), 40 x 1152 x 12 390 (437),
+// 32 x 1280 x 12 379 (396), 20 x 1536 x 12 345 (336), 16 x 2048 x 12 484 (459).
+// Heads that do not fill the CTAs once more are split if that is shorter by more than what it costs: the fold, 4 pairs (1 x 384 x 12 23.6 whole, 25.3 split,
+// 1 x 512 x 12 30.3, 25.9), and next to whole heads a kernel of their own as well, 6 pairs (16 x 512 x 12 56.9 whole, 63.8 split).  With one full round of
+// heads only, the split slots still fit into L2: 13 x 1024 x 12 127.5 in two kernels, 126.3 all split, 13 x 768 x 12 87.1, 85.2.
+constexpr int WHOLE_TILES = 10, SPLIT_GAIN = 4, SPLIT_GAIN_BESIDE = 6;
+static int whole_heads(int heads, int nt, int sms) {
+    if (nt < 2 || nt > WHOLE_TILES) return 0;
+    const int rest = heads % sms, full = heads - rest, G = (nt + 1) / 2;
+    const int gain = nt * (nt + 1) / 2 - CEIL_DIV(rest * G, sms) * (nt + 1);
+    if (rest == 0 || gain < (full ? SPLIT_GAIN_BESIDE : SPLIT_GAIN)) return heads;
+    return full >= 2 * sms ? full : 0;
+}
+
 // Profiling aid: with a device buffer of 4 * 8 * 64 int64 set here, CTA 0 of every later single-pass launch records clock64()
 // stamps of its first 64 tile pairs (role 0 = issuer, 1 = first softmax warp, 2 = first drain warp; events in program
 // order).  Null (the default) switches it off.
@@ -735,33 +786,41 @@ extern "C" int llmc_attention_bwd(bf16* dqkv, float* ws, const bf16* dout, const
     // one tile per sequence: delta and the finished dQ come from the same launch (4 x 64 x 12 heads 19.5 -> 13.4 us)
     if (nt > 1 && (rc = llmc_attention_delta(delta, out, dout, B, T, NH, hs, stream))) return rc;
     Args a;
-    a.dqkv = dqkv; a.dq_ws = dq_ws; a.lse = lse; a.delta = nt > 1 ? delta : nullptr; a.out = out; a.dout = dout; a.B = B; a.T = T; a.NH = NH;
+    a.dqkv = dqkv; a.dq_ws = dq_ws; a.lse = lse; a.delta = nt > 1 ? delta : nullptr; a.out = out; a.dout = dout; a.T = T; a.NH = NH;
     a.scale = 1.0f / sqrtf((float)hs);
     a.scale_log2e = a.scale * 1.4426950408889634f;
     a.status = llmc_status_ptr();
     a.trace = g_trace;
-    const int total = B * NH * ((nt + 1) / 2);
     int sms = llmc_device_sm_count(); if (sms <= 0) sms = 148;
-    const int grid = total < sms ? total : sms;
-    const bool few = T <= SHORT_T || (T <= SHORT_T_MANY && total > 2 * sms);
-    auto kernel = few ? attn_bwd1_kernel<true> : attn_bwd1_kernel<false>;
-    static bool configured[2] = {false, false};
-    if (!configured[few]) {
-        CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM));
-        configured[few] = true;
-    }
-    a.early = nt == 1 && grid < sms;       // as in the forward pass; with more tiles the kernels before and after are launched plainly
-    if (a.early) {
-        CUDA_CHECK(launch_pdl(kernel, dim3(grid), dim3(THREADS), SMEM, stream, 0, tmQKV, tmDO, tmDQKV, a));
+    const int G = (nt + 1) / 2;
+    static bool configured[3] = {false, false, false};
+    auto launch = [&](auto kernel, int mode, int item0, int items) {
+        if (!configured[mode]) { CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM)); configured[mode] = true; }
+        const int grid = items - item0 < sms ? items - item0 : sms;
+        a.item0 = item0; a.items = items;
+        a.early = nt == 1 && grid < sms;       // as in the forward pass; with more tiles the kernels before and after are launched plainly
+        if (a.early) { CUDA_CHECK(launch_pdl(kernel, dim3(grid), dim3(THREADS), SMEM, stream, 0, tmQKV, tmDO, tmDQKV, a)); return 0; }
+        kernel<<<grid, THREADS, SMEM, stream>>>(tmQKV, tmDO, tmDQKV, a);
+        CUDA_CHECK(cudaGetLastError());
         return 0;
-    }
-    kernel<<<grid, THREADS, SMEM, stream>>>(tmQKV, tmDO, tmDQKV, a);
-    CUDA_CHECK(cudaGetLastError());
-    if (nt == 1) return 0;
-    dq_fold_kernel<<<(unsigned)(B * NH * nt), 256, 0, stream>>>(dqkv, dq_ws, B, T, NH, nt);
+    };
+    const int whole = whole_heads(B * NH, nt, sms), rest = B * NH - whole;
+    if (whole && (rc = launch(attn_bwd1_kernel<WHOLE_HEADS>, WHOLE_HEADS, 0, whole))) return rc;
+    if (rest == 0) return 0;
+    if (T <= SHORT_T || (T <= SHORT_T_MANY && rest > 2 * sms)) rc = launch(attn_bwd1_kernel<SHORT_SPLIT>, SHORT_SPLIT, whole * G, B * NH * G);
+    else rc = launch(attn_bwd1_kernel<SPLIT>, SPLIT, whole * G, B * NH * G);
+    if (rc || nt == 1) return rc;
+    dq_fold_kernel<<<(unsigned)(rest * nt), 256, 0, stream>>>(dqkv, dq_ws, whole, T, NH, nt);
     CUDA_CHECK(cudaGetLastError());
     return 0;
 }
 
 // kernels that llmc_attention_bwd launches
-extern "C" int llmc_attention_bwd_launches(int T, int hs) { return hs == HS && T <= BT ? 1 : 3; }
+extern "C" int llmc_attention_bwd_launches(int B, int T, int NH, int hs) {
+    if (hs != HS) return 3;
+    const int nt = CEIL_DIV(T, BT);
+    if (nt <= 1) return 1;
+    int sms = llmc_device_sm_count(); if (sms <= 0) sms = 148;
+    const int whole = whole_heads(B * NH, nt, sms);
+    return 1 + (whole > 0) + (whole < B * NH ? 2 : 0);
+}

@@ -366,7 +366,7 @@ def attention_backward(dqkv, dout, qkv, out, lse, B, T, NH):
     lib = _lib.cuda()
     # row statistics and, for 64-wide heads, the dQ contributions of the single-pass kernel's units (csrc/attention_bwd1.cu)
     ws = _scratch.get("attn_bwd", lib.llmc_attention_bwd_workspace(B, T, NH, hs), torch.float32, qkv.device)
-    _launches += lib.llmc_attention_bwd_launches(T, hs)
+    _launches += lib.llmc_attention_bwd_launches(B, T, NH, hs)
     check(lib.llmc_attention_bwd(_p(dqkv), _p(ws), _p(dout), _p(qkv), _p(out), _p(lse), B, T, NH, hs, _stream()),
           "llmc_attention_bwd")
 
