@@ -7,11 +7,11 @@
 // launch itself run under the tail of the kernel before.  The same kernels launched without the attribute in brackets: forward + backward of 4 x 64
 // tokens of GPT-2 124M 2.39 ms (2.58), a decoding step of 4 rows 280 us (312), a prefill of 777 tokens 740 us (819), residual + LayerNorm forward
 // and backward at 65536 x 768 153 us (157).  The classifier, the attention kernels of wide heads and those of
-// 64-wide heads with a block on every SM are launched plainly and trigger nothing: attention at 64 x 1024 x 12 x 64 forward and backward took
+// 64-wide heads with a block on every SM (the forward: two) are launched plainly and trigger nothing: attention at 64 x 1024 x 12 x 64 forward and backward took
 // 986 us with the attribute and 938 without, on one GPU in turn, with the trigger right behind the wait (at the end of a CTA, where gemm2_kernel has
 // its own, it was not tried there); the classifier's figures stand with it.  Where 64-wide heads leave SMs free
 // the attribute pays: forward + backward of 4 x 64 tokens 1566 us without and 1513 with it.  (The bracketed comparisons were made when the plain launch
-// was the only other thing that differed; those passes take 1502, 274 and 619 us now, 3 % more or less from one GPU to another.)
+// was the only other thing that differed; those passes take 1310, 262 and 605 us now, 3 % more or less from one GPU to another.)
 #pragma once
 #include "common.cuh"
 

@@ -9,8 +9,8 @@ The decoder works on the parameter tensors of a ``models.llama3.Llama`` (it neve
 set and the caches ``(L, max_batch, max_len, NKV, HS)``.  On a GPU every step is a chain of this library's kernels, for a bf16 model issued
 from native code (csrc/decoder.cu) on exactly the rows that there are: products in row tiles that fit a prompt (csrc/gemm2t.cu) or split-K weight
 streaming for steps of at most 128 rows (csrc/stream_gemm.cu), either with SwiGLU in its epilogue, RMSNorm, and the training attention kernel for whole
-prompts or the two decoding kernels of csrc/decode.cu (rotary embedding written straight into the cache; attention of the new queries over the cached keys
-with grouped heads read in place).  An fp32 model, or one whose layers do not lie at equal distances, takes the operators one by one.  A one-token step issues about nine small launches per layer and is bound by launch latency, so on a GPU it is
+prompts or the kernels of csrc/decode.cu (rotary embedding written straight into the cache; attention of the new queries over the cached keys
+with grouped heads read in place; one launch for both in decoding steps).  An fp32 model, or one whose layers do not lie at equal distances, takes the operators one by one.  A one-token step issues about seven small launches per layer and is bound by launch latency, so on a GPU it is
 captured once in a CUDA graph and replayed (``GraphStep``): the position lives in device memory, the graph advances it itself,
 and the kernels refuse a position outside the cache through the library's status word.  On the CPU the same chain runs on
 the fp32 restatement of the operators.

@@ -1,7 +1,7 @@
 """CUDA graphs of a model's forward and backward launches.
 
 A micro-step of a small batch is bound by the host: a 12-layer GPT-2 issues about 260 kernel launches of a few microseconds each, and the
-launcher takes longer than the kernel (forward + backward of 4 x 64 tokens of GPT-2 124M: 4.5 ms launched, 1.5 ms replayed).
+launcher takes longer than the kernel (forward + backward of 4 x 64 tokens of GPT-2 124M: 4.5 ms launched, 1.3 ms replayed).
 ``StepGraphs.run`` executes a launch sequence eagerly the first two times it sees its key and from the third time on replays a graph of it.
 
 What makes a replay equal to the eager call: the sequence only reads and writes buffers that the model owns (inputs are copied into them

@@ -500,8 +500,8 @@ def cached_attention(out, q, kcache, vcache, Tq, start_pos, NH, NKV, pos=None):
 
 
 def rope_cached_attention(out, q, kcache, vcache, raw, freqs, Tq, start_pos, NH, NKV, pos=None):
-    """``rope_cache`` and ``cached_attention`` on its results; ``q`` is scratch.  Decoding steps run in one launch, with the same bits (16 rows of 4 layers of 2048 channels:
-    279 us a step in two launches per layer, see csrc/decode.cu)."""
+    """``rope_cache`` and ``cached_attention`` on its results; ``q`` is scratch.  Decoding steps run in one launch, with the same bits (a step of 4 rows, 4 layers of 2048
+    channels: 266 us, in two launches per layer 271; of 32 rows, 4 layers of 4096 channels: 763, 773)."""
     global _launches
     lib = _lib.cuda()
     N, HS = raw.shape[0], kcache.shape[-1]
