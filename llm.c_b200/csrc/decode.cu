@@ -162,8 +162,10 @@ cached_attention_kernel(bf16* __restrict__ out, const bf16* __restrict__ q, cons
 // Decoding attention, fast path (head width 64 or 128, at most 8 query rows per cached head: the decoding step itself).
 // Reading the cache once is all the work there is, so
 //   * a CTA serves ONE cached head of one batch row for ALL its (NH / NKV) * Tq query rows and a slice of the keys;
-//   * each of its 4 warps walks tiles of 16 keys whose K and V rows arrive by cp.async through a ring of its own (two tiles in
-//     flight per warp, 16-byte chunks of row j XOR-swizzled by j & 7), so that about 100 KB per SM are on the way at any time;
+//   * each of its 4 warps walks tiles of 16 keys whose K and V rows arrive by cp.async through a ring of its own (16-byte chunks of row j XOR-swizzled
+//     by j & 7).  A warp has the next two tiles on their way, or one where the heads are 128 wide and the SMs have more than one CTA: 64 KB of an SM
+//     are in flight then, which memory serves faster than 128 KB (us, two tiles in brackets, with the same CTAs on an SM either way: 32 rows at position
+//     2000 44.1 (47.2), 4095 81.4 (89.5); with a CTA an SM at most, 1 row at position 8000, 16.0 (15.6), with heads of 64, 16 rows at 900, 10.3 (9.8));
 //   * the products run on warp-level MMAs: S = Q K^T with the query rows as the 16-row operand (8 of them used), O += P V with the
 //     probabilities taken from the score registers.  fp32 FMAs with one key per lane (the kernel before this one) were bound by the
 //     shared-memory reads of the queries and the probabilities (187 us for the case below).
@@ -173,12 +175,11 @@ cached_attention_kernel(bf16* __restrict__ out, const bf16* __restrict__ q, cons
 //   * running (max, sum, accumulator) per warp, merged over the warps through shared memory, then over the key slices in slice
 //     order: through distributed shared memory when the slices of a head form one cluster (at most 8), else through a small fp32
 //     workspace and a second kernel.
-// 32 rows at position 4095, 32 heads on 8 cached heads of 128: 109 us (4.9 TB/s); 4 rows at position 160: 10 us against 25.
+// 32 rows at position 4095, 32 heads on 8 cached heads of 128: 81 us (6.6 TB/s), behind one another; 4 rows at position 160, heads of 64: 4.2 us.
 constexpr int CA_WARPS = 4;
 constexpr int CA_THREADS = CA_WARPS * 32;
 constexpr int CA_MAX_R = 8;
 constexpr int CA_TILE = 16;           // keys per tile of a warp
-constexpr int CA_STAGES = 3;
 constexpr int CA_MIN_KEYS = 128;      // a slice is at least this long (unless the cache is shorter)
 constexpr int CA_MAX_CLUSTER = 8;
 constexpr float CA_LOG2E = 1.4426950408889634f;
@@ -215,9 +216,9 @@ DEVINL void cluster_sync() {
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
-template <int HS_> __host__ __device__ constexpr int ca_ring_bytes() { return CA_STAGES * 2 * CA_TILE * HS_ * 2; }                     // of one warp
+template <int HS_, int STAGES> __host__ __device__ constexpr int ca_ring_bytes() { return STAGES * 2 * CA_TILE * HS_ * 2; }             // of one warp
 template <int HS_> __host__ __device__ constexpr int ca_part_floats() { return CA_MAX_R * (HS_ + 2); }                                 // acc, max, sum of 8 rows
-template <int HS_> __host__ __device__ constexpr int ca_smem_bytes() { return CA_WARPS * ca_ring_bytes<HS_>() + ca_part_floats<HS_>() * 4; }
+template <int HS_, int STAGES> __host__ __device__ constexpr int ca_smem_bytes() { return CA_WARPS * ca_ring_bytes<HS_, STAGES>() + ca_part_floats<HS_>() * 4; }
 
 // Where the queries and the new keys and values come from when they are not in q and the caches yet (ROPE): the output of the QKV projection
 struct Fresh {
@@ -230,7 +231,7 @@ struct Fresh {
 // CLUSTER: the gridDim.x slices of a head are one cluster and `out` receives the result; otherwise the slice's partial goes to ws.
 // ROPE: the queries are rotated in registers; the warp whose tile a new key falls into rotates it, puts it and its value into the tile and writes both
 // to the caches.  A launch of its own for that (rope_cache_kernel) costs a decoding step 3 to 4 us in every layer.
-template <int HS_, bool CLUSTER, bool ROPE>
+template <int HS_, int STAGES, bool CLUSTER, bool ROPE>
 __global__ void __launch_bounds__(CA_THREADS)
 cached_attention_split_kernel(bf16* __restrict__ out, float* __restrict__ ws, const bf16* __restrict__ q, const Fresh fresh, bf16* kcache,
                               bf16* vcache, int Tq, int Tmax, int start_pos, int NH, int NKV, float scale,
@@ -253,8 +254,8 @@ cached_attention_split_kernel(bf16* __restrict__ out, float* __restrict__ ws, co
     extern __shared__ __align__(16) uint8_t ca_smem[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int gq = lane >> 2, tq4 = lane & 3;                  // MMA fragment coordinates: row gq, column pair tq4
-    uint8_t* ring = ca_smem + warp * ca_ring_bytes<HS_>();
-    float* part = reinterpret_cast<float*>(ca_smem + CA_WARPS * ca_ring_bytes<HS_>());      // this CTA's merged partial: [8][HS_], max[8], sum[8]
+    uint8_t* ring = ca_smem + warp * ca_ring_bytes<HS_, STAGES>();
+    float* part = reinterpret_cast<float*>(ca_smem + CA_WARPS * ca_ring_bytes<HS_, STAGES>());      // this CTA's merged partial: [8][HS_], max[8], sum[8]
     const int slice = blockIdx.x, g = blockIdx.y, nslices = gridDim.x;
     const long long b = blockIdx.z;
     const int G = NH / NKV;
@@ -283,7 +284,7 @@ cached_attention_split_kernel(bf16* __restrict__ out, float* __restrict__ ws, co
     constexpr int TSTEP = CA_WARPS * CA_TILE;
     const int kt0 = k0 + warp * CA_TILE;
     #pragma unroll
-    for (int s = 0; s < CA_STAGES - 1; s++) fetch(kt0 + s * TSTEP, s);
+    for (int s = 0; s < STAGES - 1; s++) fetch(kt0 + s * TSTEP, s);
     if (early) { pdl_wait(); pdl_trigger(); }
 
     // query rows r -> token r / G, head g * G + r % G; the A operand of S: lane holds channels 2 tq4, 2 tq4 + 1 and + 8, + 9 of row gq.
@@ -320,8 +321,8 @@ cached_attention_split_kernel(bf16* __restrict__ out, float* __restrict__ ws, co
     const int mrow = lane & 7, mid = lane >> 3;
     int st = 0;
     for (int kt = kt0; kt < k1; kt += TSTEP) {
-        fetch(kt + (CA_STAGES - 1) * TSTEP, st == 0 ? CA_STAGES - 1 : st - 1);
-        cp_async_wait<CA_STAGES - 1>();
+        fetch(kt + (STAGES - 1) * TSTEP, st == 0 ? STAGES - 1 : st - 1);
+        cp_async_wait<STAGES - 1>();
         __syncwarp();
         const uint32_t kb = smem_u32(ring + st * STAGE), vb = kb + CA_TILE * ROWB;
         if (ROPE && kt + CA_TILE > start_pos) {
@@ -400,7 +401,7 @@ cached_attention_split_kernel(bf16* __restrict__ out, float* __restrict__ ws, co
             mma_16x8x16(acc[2 * n2 + 1], lo[0], lo[0], lo[1], lo[1], vf[2], vf[3]);
         }
         __syncwarp();                                          // the stage may be refilled
-        st = st + 1 == CA_STAGES ? 0 : st + 1;
+        st = st + 1 == STAGES ? 0 : st + 1;
     }
     cp_async_wait<0>();
     l += __shfl_xor_sync(0xffffffffu, l, 1);
@@ -596,17 +597,17 @@ int ca_keys_per_slice(int B, int Tmax, int NKV) {
 int ca_slices(int B, int Tmax, int NKV) { return CEIL_DIV(Tmax, ca_keys_per_slice(B, Tmax, NKV)); }
 bool ca_fast(int Tq, int NH, int NKV, int HS) { return (HS == 64 || HS == 128) && (NH / NKV) * Tq <= CA_MAX_R; }
 
-template <int HS_, bool CLUSTER, bool ROPE>
+template <int HS_, int STAGES, bool CLUSTER, bool ROPE>
 int ca_launch(bf16* out, float* ws, const bf16* q, const Fresh& fresh, bf16* kcache, bf16* vcache, int B, int Tq, int Tmax, int start_pos, int NH,
               int NKV, const int* pos_ptr, cudaStream_t stream) {
     const int rows = (NH / NKV) * Tq, slices = ca_slices(B, Tmax, NKV);
-    constexpr int smem = ca_smem_bytes<HS_>();
+    constexpr int smem = ca_smem_bytes<HS_, STAGES>();
     static bool configured = false;
     if (!configured) {
-        CUDA_CHECK(cudaFuncSetAttribute(cached_attention_split_kernel<HS_, CLUSTER, ROPE>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        CUDA_CHECK(cudaFuncSetAttribute(cached_attention_split_kernel<HS_, STAGES, CLUSTER, ROPE>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
         configured = true;
     }
-    CUDA_CHECK(launch_pdl(cached_attention_split_kernel<HS_, CLUSTER, ROPE>, dim3(slices, NKV, B), dim3(CA_THREADS), smem, stream, CLUSTER ? slices : 0,
+    CUDA_CHECK(launch_pdl(cached_attention_split_kernel<HS_, STAGES, CLUSTER, ROPE>, dim3(slices, NKV, B), dim3(CA_THREADS), smem, stream, CLUSTER ? slices : 0,
                           out, ws, q, fresh, kcache, vcache, Tq, Tmax, start_pos, NH, NKV, rsqrtf((float)HS_), pos_ptr, llmc_status_ptr(),
                           ca_keys_per_slice(B, Tmax, NKV), rows));
     if (!CLUSTER)
@@ -617,11 +618,15 @@ int ca_launch(bf16* out, float* ws, const bf16* q, const Fresh& fresh, bf16* kca
 template <bool ROPE>
 int ca_dispatch(bf16* out, float* ws, const bf16* q, const Fresh& fresh, bf16* kcache, bf16* vcache, int B, int Tq, int Tmax, int start_pos, int NH,
                 int NKV, int HS, const int* pos_ptr, cudaStream_t stream) {
-    const bool cluster = ca_slices(B, Tmax, NKV) <= CA_MAX_CLUSTER;
-#define CA_GO(H, CL) return ca_launch<H, CL, ROPE>(out, ws, q, fresh, kcache, vcache, B, Tq, Tmax, start_pos, NH, NKV, pos_ptr, stream)
-    if (HS == 64) { if (cluster) CA_GO(64, true); CA_GO(64, false); }
-    if (cluster) CA_GO(128, true);
-    CA_GO(128, false);
+    const int slices = ca_slices(B, Tmax, NKV);
+    const bool cluster = slices <= CA_MAX_CLUSTER;
+    int sms = llmc_device_sm_count(); if (sms <= 0) sms = 148;
+    const bool shared = B * NKV * slices > sms;                // more than one CTA on an SM
+#define CA_GO(H, ST, CL) return ca_launch<H, ST, CL, ROPE>(out, ws, q, fresh, kcache, vcache, B, Tq, Tmax, start_pos, NH, NKV, pos_ptr, stream)
+    if (HS == 64) { if (cluster) CA_GO(64, 3, true); CA_GO(64, 3, false); }
+    if (shared) { if (cluster) CA_GO(128, 2, true); CA_GO(128, 2, false); }
+    if (cluster) CA_GO(128, 3, true);
+    CA_GO(128, 3, false);
 #undef CA_GO
 }
 }  // namespace

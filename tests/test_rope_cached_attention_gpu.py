@@ -50,3 +50,23 @@ def test_position_outside_the_cache_or_the_table():
         assert _lib.read_status() != 0 and (out == 7.0).all()
     with pytest.raises(_lib.KernelError):
         KN.rope_cached_attention(out, out.clone(), k, v, raw, torch.zeros(30, 32, 2, device=DEV), 1, 30, 2, 1)
+
+
+# 128-wide heads with more CTAs than SMs (one tile in flight per warp): one slice per head, slices of a cluster, more slices than one holds; fewer tiles than
+# a CTA has warps, whole and cut tiles, one trip of a warp and several
+@pytest.mark.parametrize("B,start,Tmax,NKV", [(20, 0, 40, 8), (20, 15, 40, 8), (20, 62, 130, 8), (20, 64, 130, 8), (160, 127, 300, 1), (10, 190, 512, 8), (10, 511, 512, 8),
+                                              (2, 8700, 9000, 8)])
+def test_one_tile_in_flight(B, start, Tmax, NKV):
+    g = torch.Generator(device=DEV).manual_seed(start + B)
+    rnd = lambda *s: torch.randn(*s, generator=g, device=DEV).bfloat16()
+    NH, HS = 4 * NKV, 128
+    q, k, v = rnd(B, NH * HS), rnd(B, Tmax, NKV, HS), rnd(B, Tmax, NKV, HS)
+    k[:, start + 1:], v[:, start + 1:] = float("nan"), float("nan")
+    out = torch.empty(B, NH * HS, dtype=torch.bfloat16, device=DEV)
+    KN.cached_attention(out, q, k, v, 1, start, NH, NKV)
+    assert _lib.read_status() == 0
+    kk, vv = (x[:, :start + 1].double().repeat_interleave(4, 2) for x in (k, v))
+    p = torch.softmax(torch.einsum("bhd,bthd->bht", q.view(B, NH, HS).double(), kk) / HS ** 0.5, -1)
+    ref = torch.einsum("bht,bthd->bhd", p, vv).view(B, NH * HS)
+    # fp32 products and probabilities of 24 bits; the result is rounded to bf16 once, 2^-9 at most
+    assert float((out.double() - ref).norm() / ref.norm()) < 2 ** -9
