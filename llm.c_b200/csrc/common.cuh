@@ -193,11 +193,11 @@ DEVINL float max3(float a, float b, float c) { float r; asm("max.f32 %0, %1, %2,
 // 2^x of two numbers on the FMA pipe, for loops that keep the special-function unit busy (ex2 takes 8 cycles of a scheduler there, these two 10 each
 // here).  Cody and Waite's reduction: x = n + f with n the nearest integer, read from the low bits of x + 1.5 * 2^23; 2^f by a polynomial of degree 5 with
 // 2^0 = 1, fitted for the least relative error on [-1/2, 1/2] (linear programme: 7e-8 in exact arithmetic).  Error against 64 bits on [-30, 0]
-// 2.2e-7 at most, 8e-8 rms.  For x < 64; below -125 the result is that of -125 (2.4e-38).
+// 2.2e-7 at most, 8e-8 rms.  For x < 64; 0 below -126.5.
 DEVINL float2 ex2_poly2(uint64_t x) {
     float2 v = f2_unpack(x);
-    asm("max.NaN.f32 %0, %0, %1;" : "+f"(v.x) : "f"(-125.0f));
-    asm("max.NaN.f32 %0, %0, %1;" : "+f"(v.y) : "f"(-125.0f));
+    asm("max.NaN.f32 %0, %0, %1;" : "+f"(v.x) : "f"(-127.0f));
+    asm("max.NaN.f32 %0, %0, %1;" : "+f"(v.y) : "f"(-127.0f));
     x = f2_pack(v.x, v.y);
     const uint64_t t = f2_add(x, f2_both(12582912.0f));
     const uint64_t f = f2_add(x, f2_fma(t, f2_both(-1.0f), f2_both(12582912.0f)));
