@@ -1,7 +1,7 @@
 // Fused softmax + cross-entropy + dlogits over bf16 logits (N rows of Vp columns, the first V valid).
 //
 // One CTA per row.  Pass 1 computes the running maximum and the sum of exponentials (online
-// softmax), pass 2 re-reads the row (it is still in L2: a row is ~100 KB) and overwrites it in place
+// softmax), pass 2 re-reads the row (it is still in L2: a row is 100 to 256 KB) and overwrites it in place
 // with (softmax - onehot(target)) * dloss.  HBM traffic is one read and one write of the logits.
 // Columns V..Vp (vocabulary padding) are set to zero so the weight-gradient GEMM can consume the
 // whole padded row.
@@ -11,9 +11,7 @@
 
 namespace {
 
-constexpr int CLS_THREADS = 512;
-
-template <bool WRITE_DLOGITS>
+template <bool WRITE_DLOGITS, int CLS_THREADS>
 __global__ void __launch_bounds__(CLS_THREADS)
 classifier_kernel(bf16* __restrict__ logits, float* __restrict__ losses, const int* __restrict__ targets,
                   float dloss, int V, int Vp, int accumulate_loss) {
@@ -81,14 +79,20 @@ classifier_kernel(bf16* __restrict__ logits, float* __restrict__ losses, const i
 
 }  // namespace
 
+// Columns from which on a row has 1024 threads instead of 512 where it is read twice: two rows of an SM under way instead of four.  Four of such rows on every
+// SM (73 MB and more) do not stay in L2 between the passes.  8192 rows, us, 512 / 1024 threads: 57344 columns 331 / 344, 65536 393 / 383, 81920 514 / 474,
+// 100352 684 / 590, 128256 columns of 4096 rows 457 / 391, of 700 rows 105 / 76, of 4 18.4 / 16.6; 50304 of 16384 rows 553 / 617.
+constexpr int LONG_ROW = 61440;
+
 // losses[row] (+)= -log softmax(logits[row])[target]; logits[row] <- dlogits (if write_dlogits)
 extern "C" int llmc_fused_classifier(bf16* logits, float* losses, const int* targets, float dloss, int N, int V, int Vp,
                                      int write_dlogits, int accumulate_loss, cudaStream_t stream) {
     if (Vp % 8) return -1;
     // launched plainly, without an early start of its own or of the kernel behind it (pdl.cuh): with both, its blocks share the SMs with the
     // products before and after it, and LM head + classifier + both gradients take 3950 us instead of 3884 at 16384 rows, 120 instead of 116 at 256
-    if (write_dlogits) classifier_kernel<true><<<N, CLS_THREADS, 0, stream>>>(logits, losses, targets, dloss, V, Vp, accumulate_loss);
-    else classifier_kernel<false><<<N, CLS_THREADS, 0, stream>>>(logits, losses, targets, dloss, V, Vp, accumulate_loss);
+    if (write_dlogits && Vp > LONG_ROW) classifier_kernel<true, 1024><<<N, 1024, 0, stream>>>(logits, losses, targets, dloss, V, Vp, accumulate_loss);
+    else if (write_dlogits) classifier_kernel<true, 512><<<N, 512, 0, stream>>>(logits, losses, targets, dloss, V, Vp, accumulate_loss);
+    else classifier_kernel<false, 512><<<N, 512, 0, stream>>>(logits, losses, targets, dloss, V, Vp, accumulate_loss);
     CUDA_CHECK(cudaGetLastError());
     return 0;
 }

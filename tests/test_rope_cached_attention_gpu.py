@@ -68,5 +68,5 @@ def test_one_tile_in_flight(B, start, Tmax, NKV):
     kk, vv = (x[:, :start + 1].double().repeat_interleave(4, 2) for x in (k, v))
     p = torch.softmax(torch.einsum("bhd,bthd->bht", q.view(B, NH, HS).double(), kk) / HS ** 0.5, -1)
     ref = torch.einsum("bht,bthd->bhd", p, vv).view(B, NH * HS)
-    # fp32 products and probabilities of 24 bits; the result is rounded to bf16 once, 2^-9 at most
+    # fp32 products and probabilities of 24 bits; the result is rounded to bf16 once, 2^-8 of an element at most, 0.0016 in the mean square
     assert float((out.double() - ref).norm() / ref.norm()) < 2 ** -9
