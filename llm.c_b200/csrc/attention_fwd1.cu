@@ -276,7 +276,7 @@ attn_fwd1_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                     const bool grow = (mx - m) * c > RESCALE_LOG2 || i < FIRST_TILES;
                     if (__any_sync(0xffffffffu, grow)) {
                         const float m_new = fmaxf(m, mx);
-                        const float alpha = ex2_fast((m - m_new) * c);      // 0 on the first tile (m = -inf)
+                        const float alpha = m == m_new ? 1.0f : ex2_fast((m - m_new) * c);      // (-inf - -inf while a row has seen no score above -inf)
                         l *= alpha;
                         m = m_new;
                         if (i > 0) {                       // O_X(t-1) is complete: its product was issued ahead of S_X(t)
@@ -291,7 +291,7 @@ attn_fwd1_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                             }
                         }
                     }
-                    const float moff = m * c;
+                    const float moff = m == -INFINITY ? 0.f : m * c;         // probabilities of 0, not of -inf - -inf
                     const uint64_t c2 = f2_both(c), off2 = f2_both(-moff);
                     uint64_t rs0 = 0, rs1 = 0;
                     #pragma unroll
@@ -343,12 +343,13 @@ attn_fwd1_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                 }
                 asm volatile("bar.sync 3, 256;" ::: "memory");
                 if (x == 1) break;
-                const float mo = other_ml[r], m_new = fmaxf(m, mo);      // slot 0 has seen key 0: m is finite; slot 1 may have seen none of this row's keys
+                const float mo = other_ml[r], m_new = fmaxf(m, mo);      // slot 1 may have seen none of this row's keys
                 mine = ex2_fast((m - m_new) * c);
                 theirs = ex2_fast((mo - m_new) * c);
                 l = l * mine + other_ml[BT + r] * theirs;
                 m = m_new;
             }
+            if (m == -INFINITY) l = NAN;                   // no score above -inf: no softmax
             const float inv = 1.0f / l;
             uint8_t* otile = sQ + (2 * x + (it & 1)) * TILE_BYTES;     // over the item's Q tile, which its last score product has read
             uint8_t* orow = otile + r * 128;

@@ -102,3 +102,30 @@ def test_error_is_that_of_probabilities_rounded_once(B, T, NH):
         norm += float(exact.square().sum())
     assert _lib.read_status() == 0
     assert err ** 0.5 < 1.002 * rounded ** 0.5, ((err / norm) ** 0.5, (rounded / norm) ** 0.5)
+
+# keys 0 .. 63 (of some heads 0 .. 127: whole tiles that a row sees nothing in) with scores that overflow
+@pytest.mark.parametrize("B", [1, 40])
+def test_infinite_scores_in_the_first_tiles(B):
+    T, NH = 330, 24
+    qkv = torch.randn(B, T, 3, NH, 64, generator=torch.Generator().manual_seed(B)).bfloat16()
+    qkv[:, :, 0, :, 7], qkv[:, :, 1, :, 7] = 1e20, 0.0
+    first = torch.tensor([64, 128, 40, 100, 200, 0]).repeat(NH // 6)       # keys of a head that score -inf
+    for h in range(NH):
+        qkv[:, :first[h], 1, h, 7] = -1e20
+    out, lse = torch.empty(B, T, NH * 64, dtype=torch.bfloat16, device=DEV), torch.empty(B, NH, T, device=DEV)
+    KN.attention_forward(out, lse, qkv.view(B, T, -1).to(DEV), B, T, NH)
+    assert _lib.read_status() == 0
+    q, k, v = qkv.float().permute(2, 0, 3, 1, 4)
+    keys = torch.arange(T)
+    hidden = (keys[None, :] > keys[:, None])[None] | (keys[None, None, :] < first[:, None, None])       # (NH, T, T)
+    q[..., 7] = k[..., 7] = 0.0
+    s = (q @ k.transpose(2, 3) / 8).masked_fill(hidden, -torch.inf)
+    # a row all of whose scores are -inf has no softmax
+    seen = keys[None, :] >= first[:, None]
+    ref = torch.softmax(s, -1) @ v
+    got = out.view(B, T, NH, 64).transpose(1, 2).float().cpu()
+    assert torch.equal(got.isnan().any(-1), ~seen.expand(B, -1, -1)) and torch.equal(got.isnan().all(-1), ~seen.expand(B, -1, -1))
+    assert torch.equal(lse.isnan().cpu(), ~seen.expand(B, -1, -1))
+    got, ref = got[seen.expand(B, -1, -1)], ref[seen.expand(B, -1, -1)]
+    assert float((got - ref).norm() / ref.norm()) < 4e-3                   # P and O rounded to bf16 once each
+    assert torch.allclose(lse.cpu()[seen.expand(B, -1, -1)], torch.logsumexp(s, -1)[seen.expand(B, -1, -1)], atol=1e-4)
