@@ -43,7 +43,7 @@ rope_cache_kernel(bf16* __restrict__ q, bf16* __restrict__ kcache, bf16* __restr
     pdl_trigger();
     if (pos_ptr) {
         start_pos = *pos_ptr;
-        if (start_pos < 0 || start_pos + Tq > Tmax || start_pos + Tq > freqs_len) {
+        if (start_pos < 0 || start_pos > Tmax - Tq || start_pos > freqs_len - Tq) {
             if (threadIdx.x == 0 && blockIdx.x == 0) record_error(status, ST_BAD_ARG, 0x30);
             return;
         }
@@ -83,7 +83,7 @@ cached_attention_kernel(bf16* __restrict__ out, const bf16* __restrict__ q, cons
                         const int* __restrict__ pos_ptr, unsigned int* status) {
     if (pos_ptr) {
         start_pos = *pos_ptr;
-        if (start_pos < 0 || start_pos + Tq > Tmax) {
+        if (start_pos < 0 || start_pos > Tmax - Tq) {
             if (threadIdx.x == 0 && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0) record_error(status, ST_BAD_ARG, 0x31);
             return;
         }
@@ -240,7 +240,7 @@ cached_attention_split_kernel(bf16* __restrict__ out, float* __restrict__ ws, co
     if (!early) { pdl_wait(); pdl_trigger(); }
     if (pos_ptr) {
         start_pos = *pos_ptr;
-        if (start_pos < 0 || start_pos + Tq > Tmax || (ROPE && start_pos + Tq > fresh.freqs_len)) {           // the same for every CTA of a cluster
+        if (start_pos < 0 || start_pos > Tmax - Tq || (ROPE && start_pos > fresh.freqs_len - Tq)) {           // the same for every CTA of a cluster
             if (early) pdl_wait();             // the kernel behind this one relies on what is before it
             if (threadIdx.x == 0 && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0) record_error(status, ST_BAD_ARG, ROPE ? 0x30 : 0x32);
             return;
@@ -559,7 +559,7 @@ skinny_gemm_kernel(bf16* __restrict__ out, const bf16* __restrict__ x, const bf1
 int decode_check(int B, int Tq, int Tmax, int start_pos, int NH, int NKV, int HS, bool device_pos) {
     if (HS % 8 || HS > DEC_MAX_HS || HS < 16 || NKV <= 0 || NH % NKV) return -1;
     if (B <= 0 || Tq <= 0 || Tq > Tmax) return -2;
-    if (!device_pos && (start_pos < 0 || start_pos + Tq > Tmax)) return -2;
+    if (!device_pos && (start_pos < 0 || start_pos > Tmax - Tq)) return -2;      // (their sum may not fit an int)
     if (B > 65535 || Tq > 65535) return -3;
     return 0;
 }
@@ -572,7 +572,7 @@ extern "C" int llmc_rope_cache(bf16* q, bf16* kcache, bf16* vcache, const bf16* 
                                int Tmax, int start_pos, int NH, int NKV, int HS, const int* pos_ptr, cudaStream_t stream) {
     const int rc = decode_check(B, Tq, Tmax, start_pos, NH, NKV, HS, pos_ptr != nullptr);
     if (rc) return rc;
-    if (!pos_ptr && start_pos + Tq > freqs_len) return -4;
+    if (!pos_ptr && start_pos > freqs_len - Tq) return -4;
     const long long N = (long long)B * Tq;
     const long long total = N * (NH + 2 * NKV) * (HS / 8);
     CUDA_CHECK(launch_pdl(rope_cache_kernel, dim3((unsigned)CEIL_DIV(total, 256)), dim3(256), 0, stream, 0, q, kcache, vcache, raw,
@@ -661,7 +661,7 @@ extern "C" int llmc_cached_attention_rope(bf16* out, const bf16* raw, const floa
                                           int start_pos, int NH, int NKV, int HS, const int* pos_ptr, float* ws, int early, cudaStream_t stream) {
     const int rc = decode_check(B, Tq, Tmax, start_pos, NH, NKV, HS, pos_ptr != nullptr);
     if (rc) return rc;
-    if (!pos_ptr && start_pos + Tq > freqs_len) return -4;
+    if (!pos_ptr && start_pos > freqs_len - Tq) return -4;
     if (!ca_fast(Tq, NH, NKV, HS) || (ca_slices(B, Tmax, NKV) > CA_MAX_CLUSTER && ws == nullptr)) return -6;
     if ((reinterpret_cast<uintptr_t>(raw) | reinterpret_cast<uintptr_t>(kcache) | reinterpret_cast<uintptr_t>(vcache) | reinterpret_cast<uintptr_t>(freqs)) & 15) return -6;
     const Fresh fresh = {raw, reinterpret_cast<const float2*>(freqs), freqs_len, early};

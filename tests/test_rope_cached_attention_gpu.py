@@ -65,7 +65,7 @@ def test_rotation_rounds_one_product(HS):
 def test_position_outside_the_cache_or_the_table():
     raw, out = torch.zeros(1, 4 * 64, dtype=torch.bfloat16, device=DEV), torch.full((1, 128), 7.0, dtype=torch.bfloat16, device=DEV)
     k, v = torch.zeros(1, 40, 1, 64, dtype=torch.bfloat16, device=DEV), torch.zeros(1, 40, 1, 64, dtype=torch.bfloat16, device=DEV)
-    for rows, at in ((40, 40), (30, 30), (40, -1)):
+    for rows, at in ((40, 40), (30, 30), (40, -1), (40, 2 ** 31 - 1)):
         freqs = torch.zeros(rows, 32, 2, device=DEV)
         KN.rope_cached_attention(out, out.clone(), k, v, raw, freqs, 1, 0, 2, 1, torch.tensor([at], dtype=torch.int32, device=DEV))
         assert _lib.read_status() != 0 and (out == 7.0).all()
