@@ -254,26 +254,25 @@ class GPT:
         if ps is not None:
             ps.wait(-1)
         ops.encoder_forward(a["encoded"], self.inputs, p["wte"], p["wpe"])
-        ops.layernorm_forward(a["ln1"][0], a["ln1_mean"][0], a["ln1_rstd"][0], a["encoded"], p["ln1w"][0], p["ln1b"][0])
+        residual, ln1 = a["encoded"], a["ln1"][0]
+        ops.layernorm_forward(ln1, a["ln1_mean"][0], a["ln1_rstd"][0], residual, p["ln1w"][0], p["ln1b"][0])
         for l in range(L):
           with _Range("forward layer %d" % l, nvtx):
-            lln = 0 if self.recompute >= 2 else l
-            lg = 0 if self.recompute >= 1 else l
-            residual = a["encoded"] if l == 0 else a["residual3"][l - 1]
-            ops.matmul_forward(a["qkv"][l], a["ln1"][lln], p["qkvw"][l], p["qkvb"][l], ready=(ps.flags(l) if ps is not None else None))
-            ops.attention_forward(a["atty"][l], a["lse"][l], a["qkv"][l], B, T, NH)
-            ops.matmul_forward(a["scratch_btc"], a["atty"][l], p["attprojw"][l], p["attprojb"][l])
-            ops.fused_residual_forward(a["residual2"][l], a["ln2"][lln], a["ln2_mean"][l], a["ln2_rstd"][l], residual,
-                                       a["scratch_btc"], p["ln2w"][l], p["ln2b"][l])
-            ops.matmul_forward(a["fch_gelu"][lg], a["ln2"][lln], p["fcw"][l], p["fcb"][l], pre_gelu=a["fch"][l])
-            ops.matmul_forward(a["scratch_btc"], a["fch_gelu"][lg], p["fcprojw"][l], p["fcprojb"][l])
+            # (a view of a tensor takes the host as long as many lines of Python: one for each buffer)
+            qkv, atty, residual2, gelu = a["qkv"][l], a["atty"][l], a["residual2"][l], a["fch_gelu"][0 if self.recompute >= 1 else l]
+            ln2 = a["ln2"][0 if self.recompute >= 2 else l]
+            ops.matmul_forward(qkv, ln1, p["qkvw"][l], p["qkvb"][l], ready=(ps.flags(l) if ps is not None else None))
+            ops.attention_forward(atty, a["lse"][l], qkv, B, T, NH)
+            ops.matmul_forward(a["scratch_btc"], atty, p["attprojw"][l], p["attprojb"][l])
+            ops.fused_residual_forward(residual2, ln2, a["ln2_mean"][l], a["ln2_rstd"][l], residual, a["scratch_btc"], p["ln2w"][l], p["ln2b"][l])
+            ops.matmul_forward(gelu, ln2, p["fcw"][l], p["fcb"][l], pre_gelu=a["fch"][l])
+            ops.matmul_forward(a["scratch_btc"], gelu, p["fcprojw"][l], p["fcprojb"][l])
+            residual = a["residual3"][l]
             if l + 1 < L:
-                nl = 0 if self.recompute >= 2 else l + 1
-                ops.fused_residual_forward(a["residual3"][l], a["ln1"][nl], a["ln1_mean"][l + 1], a["ln1_rstd"][l + 1],
-                                           a["residual2"][l], a["scratch_btc"], p["ln1w"][l + 1], p["ln1b"][l + 1])
+                ln1 = a["ln1"][0 if self.recompute >= 2 else l + 1]
+                ops.fused_residual_forward(residual, ln1, a["ln1_mean"][l + 1], a["ln1_rstd"][l + 1], residual2, a["scratch_btc"], p["ln1w"][l + 1], p["ln1b"][l + 1])
             else:
-                ops.fused_residual_forward(a["residual3"][l], a["lnf"], a["lnf_mean"], a["lnf_rstd"], a["residual2"][l],
-                                           a["scratch_btc"], p["lnfw"], p["lnfb"])
+                ops.fused_residual_forward(residual, a["lnf"], a["lnf_mean"], a["lnf_rstd"], residual2, a["scratch_btc"], p["lnfw"], p["lnfb"])
         ops.matmul_forward(a["logits"], a["lnf"], p["wte"], None)
         if dloss is not None:
             ops.fused_classifier(a["logits"], a["losses"], self.targets.view(-1), dloss, cfg.vocab_size,
@@ -330,23 +329,23 @@ class GPT:
           with _Range("backward layer %d" % l, nvtx):
             residual = a["encoded"] if l == 0 else a["residual3"][l - 1]
             lln = 0 if self.recompute >= 2 else l
-            lg = 0 if self.recompute >= 1 else l
+            gelu, ln1, ln2, atty = a["fch_gelu"][0 if self.recompute >= 1 else l], a["ln1"][lln], a["ln2"][lln], a["atty"][l]
             if self.recompute >= 1:
-                side.free(a["fch_gelu"][lg])
-                ops.gelu_forward(a["fch_gelu"][lg], a["fch"][l])
+                side.free(gelu)
+                ops.gelu_forward(gelu, a["fch"][l])
             with side.fork():
-                ops.matmul_wgrad(g["fcprojw"][l], dres, a["fch_gelu"][lg], accumulate=acc)
-            side.read(dres, a["fch_gelu"][lg])
+                ops.matmul_wgrad(g["fcprojw"][l], dres, gelu, accumulate=acc)
+            side.read(dres, gelu)
             side.free(dl_bt4c)
             ops.matmul_dgrad(dl_bt4c, dres, p["fcprojw"][l], pre_gelu=a["fch"][l])
             if self.recompute >= 2:
-                side.free(a["ln2"][lln])
-                ops.layernorm_forward(a["ln2"][lln], None, None, a["residual2"][l], p["ln2w"][l], p["ln2b"][l])
+                side.free(ln2)
+                ops.layernorm_forward(ln2, None, None, a["residual2"][l], p["ln2w"][l], p["ln2b"][l])
             with side.fork_sums():
                 ops.bias_grad(g["fcb"][l], dl_bt4c, accumulate=acc)
             with side.fork():
-                ops.matmul_wgrad(g["fcw"][l], dl_bt4c, a["ln2"][lln], accumulate=acc)
-            side.read(dl_bt4c, a["ln2"][lln])
+                ops.matmul_wgrad(g["fcw"][l], dl_bt4c, ln2, accumulate=acc)
+            side.read(dl_bt4c, ln2)
             ops.matmul_dgrad(dl_btc, dl_bt4c, p["fcw"][l])
             side.join(sums)
             old, dres = dres, side.other(dres)
@@ -356,19 +355,19 @@ class GPT:
                                    sums_in=side.fork_sums, dinp_old=old)
             sums = side.mark_sums()
             with side.fork():
-                ops.matmul_wgrad(g["attprojw"][l], dres, a["atty"][l], accumulate=acc)
+                ops.matmul_wgrad(g["attprojw"][l], dres, atty, accumulate=acc)
             side.read(dres)
             ops.matmul_dgrad(dl_btc, dres, p["attprojw"][l])
             side.free(dqkv)
-            ops.attention_backward(dqkv, dl_btc, a["qkv"][l], a["atty"][l], a["lse"][l], B, T, NH)
+            ops.attention_backward(dqkv, dl_btc, a["qkv"][l], atty, a["lse"][l], B, T, NH)
             if self.recompute >= 2:
-                side.free(a["ln1"][lln])
-                ops.layernorm_forward(a["ln1"][lln], None, None, residual, p["ln1w"][l], p["ln1b"][l])
+                side.free(ln1)
+                ops.layernorm_forward(ln1, None, None, residual, p["ln1w"][l], p["ln1b"][l])
             with side.fork_sums():
                 ops.bias_grad(g["qkvb"][l], dqkv, accumulate=acc)
             with side.fork():
-                ops.matmul_wgrad(g["qkvw"][l], dqkv, a["ln1"][lln], accumulate=acc)
-            side.read(dqkv, a["ln1"][lln])
+                ops.matmul_wgrad(g["qkvw"][l], dqkv, ln1, accumulate=acc)
+            side.read(dqkv, ln1)
             ops.matmul_dgrad(dl_btc, dqkv, p["qkvw"][l])
             side.join(sums)
             old, dres = dres, side.other(dres)

@@ -350,39 +350,39 @@ class Llama:
           with _Range("backward layer %d" % l, nvtx):
             residual = a["encoded"] if l == 0 else a["residual3"][l - 1]
             lln = 0 if self.recompute >= 2 else l
-            lg = 0 if self.recompute >= 1 else l
+            h, ln1, ln2, atty = a["h"][0 if self.recompute >= 1 else l], a["ln1"][lln], a["ln2"][lln], a["atty"][l]
             if self.recompute >= 1:
-                side.free(a["h"][lg])
-                ops.swiglu_forward(a["h"][lg], a["fc12"][l])
+                side.free(h)
+                ops.swiglu_forward(h, a["fc12"][l])
             with side.fork():
-                ops.matmul_wgrad(g["fcprojw"][l], dres, a["h"][lg], accumulate=acc)
-            side.read(dres, a["h"][lg])
+                ops.matmul_wgrad(g["fcprojw"][l], dres, h, accumulate=acc)
+            side.read(dres, h)
             ops.matmul_dgrad(dh, dres, p["fcprojw"][l])
             side.free(dfc12)
             ops.swiglu_backward(dfc12, dh, a["fc12"][l])
             if self.recompute >= 2:
-                side.free(a["ln2"][lln])
-                ops.rmsnorm_forward(a["ln2"][lln], None, a["residual2"][l], p["ln2w"][l], eps)
+                side.free(ln2)
+                ops.rmsnorm_forward(ln2, None, a["residual2"][l], p["ln2w"][l], eps)
             with side.fork():
-                ops.matmul_wgrad(g["fc12w"][l], dfc12, a["ln2"][lln], accumulate=acc)
-            side.read(dfc12, a["ln2"][lln])
+                ops.matmul_wgrad(g["fc12w"][l], dfc12, ln2, accumulate=acc)
+            side.read(dfc12, ln2)
             ops.matmul_dgrad(dl_btc, dfc12, p["fc12w"][l])
             side.free(dres)
             ops.rmsnorm_backward(dres, g["ln2w"][l], dl_btc, a["residual2"][l], p["ln2w"][l], a["ln2_rstd"][l], accumulate_dinp=True,
                                  accumulate_dw=acc)
             with side.fork():
-                ops.matmul_wgrad(g["attprojw"][l], dres, a["atty"][l], accumulate=acc)
+                ops.matmul_wgrad(g["attprojw"][l], dres, atty, accumulate=acc)
             side.read(dres)
             ops.matmul_dgrad(dl_btc, dres, p["attprojw"][l])
-            ops.attention_backward(dqkv, dl_btc, a["qkv"][l], a["atty"][l], a["lse"][l], B, T, NH)
+            ops.attention_backward(dqkv, dl_btc, a["qkv"][l], atty, a["lse"][l], B, T, NH)
             side.free(dqkv_raw)
             ops.rope_backward(dqkv_raw, dqkv, self.freqs, T, NH, NKV)
             if self.recompute >= 2:
-                side.free(a["ln1"][lln])
-                ops.rmsnorm_forward(a["ln1"][lln], None, residual, p["ln1w"][l], eps)
+                side.free(ln1)
+                ops.rmsnorm_forward(ln1, None, residual, p["ln1w"][l], eps)
             with side.fork():
-                ops.matmul_wgrad(g["qkvw"][l], dqkv_raw, a["ln1"][lln], accumulate=acc)
-            side.read(dqkv_raw, a["ln1"][lln])
+                ops.matmul_wgrad(g["qkvw"][l], dqkv_raw, ln1, accumulate=acc)
+            side.read(dqkv_raw, ln1)
             ops.matmul_dgrad(dl_btc, dqkv_raw, p["qkvw"][l])
             side.free(dres)
             ops.rmsnorm_backward(dres, g["ln1w"][l], dl_btc, residual, p["ln1w"][l], a["ln1_rstd"][l], accumulate_dinp=True,
