@@ -100,6 +100,7 @@ def cuda():
         "llmc_cached_attention": (I, [P, P, P, P, I, I, I, I, I, I, I, P, P, S]),
         "llmc_cached_attention_rope": (I, [P, P, P, I, P, P, I, I, I, I, I, I, I, P, P, I, S]),
         "llmc_cached_attention_workspace": (L, [I, I, I, I, I, I]),
+        "llmc_cached_attention_stages": (I, [I, I, I, I, I]),
         "llmc_gelu_bwd_inplace": (I, [P, P, L, S]),
         "llmc_residual_add": (I, [P, P, P, L, S]),
         "llmc_bias_grad_scratch": (L, [I, I]),

@@ -163,9 +163,7 @@ cached_attention_kernel(bf16* __restrict__ out, const bf16* __restrict__ q, cons
 // Reading the cache once is all the work there is, so
 //   * a CTA serves ONE cached head of one batch row for ALL its (NH / NKV) * Tq query rows and a slice of the keys;
 //   * each of its 4 warps walks tiles of 16 keys whose K and V rows arrive by cp.async through a ring of its own (16-byte chunks of row j XOR-swizzled
-//     by j & 7).  A warp has the next two tiles on their way, or one where the heads are 128 wide and the SMs have more than one CTA: 64 KB of an SM
-//     are in flight then, which memory serves faster than 128 KB (us, two tiles in brackets, with the same CTAs on an SM either way: 32 rows at position
-//     2000 44.1 (47.2), 4095 81.4 (89.5); with a CTA an SM at most, 1 row at position 8000, 16.0 (15.6), with heads of 64, 16 rows at 900, 10.3 (9.8));
+//     by j & 7).  A warp has the next two tiles on their way, or one (ca_stages);
 //   * the products run on warp-level MMAs: S = Q K^T with the query rows as the 16-row operand (8 of them used), O += P V with the
 //     probabilities taken from the score registers.  fp32 FMAs with one key per lane (the kernel before this one) were bound by the
 //     shared-memory reads of the queries and the probabilities (187 us for the case below).
@@ -597,6 +595,18 @@ int ca_keys_per_slice(int B, int Tmax, int NKV) {
 int ca_slices(int B, int Tmax, int NKV) { return CEIL_DIV(Tmax, ca_keys_per_slice(B, Tmax, NKV)); }
 bool ca_fast(int Tq, int NH, int NKV, int HS) { return (HS == 64 || HS == 128) && (NH / NKV) * Tq <= CA_MAX_R; }
 
+// Stages of a warp's ring.  With two (one tile in flight behind the one that is worked on) a 128-wide CTA asks for 32 KB at a time instead of 64, and two CTAs on an SM
+// stream long slices of keys faster; everywhere else the deeper ring is the better or an equal one.  Whole steps of four layers of 4096 channels, us, three /
+// two stages (rows x position, CTAs): 32 x 2000 (256) 754 / 743, 37 x 3000 (296) 889 / 870, 32 x 4000 (256) 928 / 893, 8 x 8000 (256) 712 / 706; shorter slices
+// 32 x 700 (256) 644 / 644, 8 x 2000 (256) 598 / 602; fewer CTAs 24 x 2000 (192) 709 / 713, 20 x 2000 (160) 696 / 702; more 40 x 1000 (320) 751 / 757,
+// 64 x 2000 (512) 965 / 976; slices without a cluster 1 x 16000 (296) 617 / 643, 4 x 16000 (288) 724 / 752.  Without the rotary embedding the kernel is small
+// enough for three CTAs on an SM and two stages are slower in long slices too: 32 x 2000 46 / 53, 32 x 4000 83 / 111.
+int ca_stages(int B, int Tmax, int NKV, int HS, bool rope) {
+    int sms = llmc_device_sm_count(); if (sms <= 0) sms = 148;
+    const int slices = ca_slices(B, Tmax, NKV), ctas = B * NKV * slices;
+    return rope && HS == 128 && slices <= CA_MAX_CLUSTER && 2 * ctas > 3 * sms && ctas <= 2 * sms && ca_keys_per_slice(B, Tmax, NKV) >= 1024 ? 2 : 3;
+}
+
 template <int HS_, int STAGES, bool CLUSTER, bool ROPE>
 int ca_launch(bf16* out, float* ws, const bf16* q, const Fresh& fresh, bf16* kcache, bf16* vcache, int B, int Tq, int Tmax, int start_pos, int NH,
               int NKV, const int* pos_ptr, cudaStream_t stream) {
@@ -618,18 +628,18 @@ int ca_launch(bf16* out, float* ws, const bf16* q, const Fresh& fresh, bf16* kca
 template <bool ROPE>
 int ca_dispatch(bf16* out, float* ws, const bf16* q, const Fresh& fresh, bf16* kcache, bf16* vcache, int B, int Tq, int Tmax, int start_pos, int NH,
                 int NKV, int HS, const int* pos_ptr, cudaStream_t stream) {
-    const int slices = ca_slices(B, Tmax, NKV);
-    const bool cluster = slices <= CA_MAX_CLUSTER;
-    int sms = llmc_device_sm_count(); if (sms <= 0) sms = 148;
-    const bool shared = B * NKV * slices > sms;                // more than one CTA on an SM
+    const bool cluster = ca_slices(B, Tmax, NKV) <= CA_MAX_CLUSTER;
 #define CA_GO(H, ST, CL) return ca_launch<H, ST, CL, ROPE>(out, ws, q, fresh, kcache, vcache, B, Tq, Tmax, start_pos, NH, NKV, pos_ptr, stream)
     if (HS == 64) { if (cluster) CA_GO(64, 3, true); CA_GO(64, 3, false); }
-    if (shared) { if (cluster) CA_GO(128, 2, true); CA_GO(128, 2, false); }
+    if constexpr (ROPE) if (ca_stages(B, Tmax, NKV, HS, true) == 2) CA_GO(128, 2, true);
     if (cluster) CA_GO(128, 3, true);
     CA_GO(128, 3, false);
 #undef CA_GO
 }
 }  // namespace
+
+// How many tiles of keys a warp of llmc_cached_attention (rope: llmc_cached_attention_rope) has room for, where it takes the fast path
+extern "C" int llmc_cached_attention_stages(int B, int Tmax, int NKV, int HS, int rope) { return ca_stages(B, Tmax, NKV, HS, rope != 0); }
 
 // fp32 words of workspace llmc_cached_attention needs for this problem (0: it runs without one)
 extern "C" long long llmc_cached_attention_workspace(int B, int Tq, int Tmax, int NH, int NKV, int HS) {

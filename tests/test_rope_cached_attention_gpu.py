@@ -13,7 +13,10 @@ DEV = "cuda"
 # a cache with more rows than the batch
 @pytest.mark.parametrize("B,Tq,start,Tmax,NH,NKV,HS", [
     (1, 1, 0, 8, 2, 2, 64), (2, 1, 15, 192, 8, 2, 64), (2, 1, 16, 192, 8, 2, 64), (3, 8, 12, 64, 2, 2, 128), (1, 2, 127, 1024, 8, 2, 128), (1, 2, 128, 1024, 8, 2, 128),
-    (3, 1, 1500, 1600, 4, 1, 128), (1, 1, 9000, 9100, 2, 1, 64), (40, 1, 77, 300, 16, 8, 64), (1, 8, 250, 258, 2, 2, 128), (32, 1, 2000, 2048, 32, 8, 128)])
+    (3, 1, 1500, 1600, 4, 1, 128), (1, 1, 9000, 9100, 2, 1, 64), (40, 1, 77, 300, 16, 8, 64), (1, 8, 250, 258, 2, 2, 128), (32, 1, 2000, 2048, 32, 8, 128),
+    # a ring of two stages in the one launch (of three in the two): fewer tiles than a CTA has warps, one trip of a warp and several, new keys in whole and cut tiles
+    (28, 1, 0, 1100, 16, 8, 128), (28, 1, 15, 1100, 16, 8, 128), (37, 1, 64, 1030, 16, 8, 128), (30, 2, 126, 1030, 16, 8, 128), (28, 1, 1099, 1100, 32, 8, 128),
+    (10, 8, 2040, 3100, 8, 8, 128)])
 @pytest.mark.parametrize("device_pos", [False, True])
 def test_same_bits(B, Tq, start, Tmax, NH, NKV, HS, device_pos):
     g = torch.Generator(device=DEV).manual_seed(start + B)
@@ -73,11 +76,11 @@ def test_position_outside_the_cache_or_the_table():
         KN.rope_cached_attention(out, out.clone(), k, v, raw, torch.zeros(30, 32, 2, device=DEV), 1, 30, 2, 1)
 
 
-# 128-wide heads with more CTAs than SMs (one tile in flight per warp): one slice per head, slices of a cluster, more slices than one holds; fewer tiles than
+# 128-wide heads with more CTAs than SMs: one slice per head, slices of a cluster, more slices than one holds; fewer tiles than
 # a CTA has warps, whole and cut tiles, one trip of a warp and several
 @pytest.mark.parametrize("B,start,Tmax,NKV", [(20, 0, 40, 8), (20, 15, 40, 8), (20, 62, 130, 8), (20, 64, 130, 8), (160, 127, 300, 1), (10, 190, 512, 8), (10, 511, 512, 8),
                                               (2, 8700, 9000, 8)])
-def test_one_tile_in_flight(B, start, Tmax, NKV):
+def test_many_wide_heads(B, start, Tmax, NKV):
     g = torch.Generator(device=DEV).manual_seed(start + B)
     rnd = lambda *s: torch.randn(*s, generator=g, device=DEV).bfloat16()
     NH, HS = 4 * NKV, 128
