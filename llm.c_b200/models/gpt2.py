@@ -148,7 +148,7 @@ class GPT:
         self.grad_hook = None
         # set by a communication backend whose all-gather may still be in flight when forward starts (parallel/p2p.py)
         self.step_graphs = StepGraphs()
-        self.chain_first_tokens = 1536         # captured passes of up to so many tokens (models/step_graphs.py, _capture)
+        self.chain_first_tokens = min(1536, (5 << 29) // cfg.channels ** 2)         # captured passes of up to so many tokens (models/step_graphs.py, _capture)
         self.use_graphs = True          # replay small micro-steps from CUDA graphs (off: launch every kernel, for per-operator measurements)
         self.param_sync = None          # called as grad_hook(layer or -1 for the embeddings/final LN) on the last micro-step
 

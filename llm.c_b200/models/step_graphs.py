@@ -165,8 +165,10 @@ class StepGraphs:
     @staticmethod
     def _capture(model, e, fn):
         # the chain in a stream of higher priority: its blocks come first wherever an SM gets free, those of the side branches take what it leaves.  Pays as long
-        # as the side branches are the smaller part: GPT-2 124M, us, without / with: 64 tokens 1192 / 1171, 256 1335 / 1309, 512 1724 / 1656, 1024 2148 / 2060, 1536 2718 / 2687,
-        # but 2048 2829 / 2868; two LLaMA layers' worth of wide weight gradients over 128 tokens 1279 / 1307
+        # as the side branches are the smaller part, and they grow with the tokens and the square of the channels.  GPT-2's layers, us, without / with the priority, 12 of 768
+        # channels: 64 tokens 1163 / 1147, 512 1581 / 1545, 1024 2375 / 2289, 1536 2671 / 2648; 8 of 1280: 64 1089 / 1042, 1024 2454 / 2395, 1536 2680 / 2651; 4 of 2048: 64
+        # 928 / 884, 512 1390 / 1368, but 768 1791 / 1800; 3 of 2560: 256 1138 / 1124, 384 1324 / 1327, 1536 3240 / 3434; 2 of 4096: 128 1220 / 1208, 256 1359 / 1387, 512 2044 /
+        # 2125; two LLaMA layers' worth of wide weight gradients over 128 tokens 1279 / 1307.  The models say up to how many tokens (LLaMA: none)
         first = 0 < e.get("tokens", 0) <= getattr(model, "chain_first_tokens", 0)
         graph, chain = torch.cuda.CUDAGraph(), torch.cuda.Stream(device=model.device, **({"priority": -1} if first else {}))
         before = kernels.launch_count()

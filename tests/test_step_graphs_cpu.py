@@ -98,3 +98,11 @@ def test_no_collection_in_a_capture_while_another_thread_ends_its_own(monkeypatc
         assert seen == [False] and gc.isenabled() == enabled
     finally:
         (gc.enable if before else gc.disable)()
+
+
+# tokens of a captured pass whose chain gets the priority: fewer for wide layers
+@pytest.mark.parametrize("channels,tokens", [(64, 1536), (768, 1536), (1280, 1536), (1600, 1048), (2048, 640), (2560, 409), (4096, 160)])
+def test_the_chain_comes_first_up_to(channels, tokens):
+    with torch.device("meta"):
+        m = gpt2.GPT(gpt2.GPTConfig(16, 100, 128, 1, channels // 64, channels), "meta", torch.bfloat16)
+    assert m.chain_first_tokens == tokens

@@ -56,9 +56,9 @@ def test_replayed_steps_equal_launched_steps(family):
 
 
 # 256 rows of 768 channels: input gradients in slices of K beside the weight gradients; 1280 rows: bias gradients through a scratch buffer, on the side
-# branch; every recompute level shares other buffers between the layers
+# branch; 2048 rows: the chain without priority over the side branches; every recompute level shares other buffers between the layers
 @pytest.mark.parametrize("recompute", [0, 1, 2])
-@pytest.mark.parametrize("B,T,C,L", [(4, 64, 768, 3), (5, 256, 256, 4)])
+@pytest.mark.parametrize("B,T,C,L", [(4, 64, 768, 3), (5, 256, 256, 4), (8, 256, 256, 3)])
 @pytest.mark.parametrize("family", ["gpt2", "llama3"])
 def test_both_branches_of_the_backward_pass(family, B, T, C, L, recompute):
     def build(graphs):
