@@ -98,7 +98,7 @@ class CachedDecoder:
                                torch.zeros(B * NH * Tq, dtype=torch.float32, device=m.device))
             packed, lse = self._dense[0][:N], self._dense[1][:B * NH * Tq].view(B, NH, Tq)
         if self.native and self.skinny_rows == kernels.STREAM_MAX_ROWS and kernels.decoder_layout_ok(self):
-            logits = kernels.decoder_forward(self, a, (packed, lse) if dense else None, tokens, start_pos, pos, **({"advance": True} if advance else {}))
+            logits = kernels.decoder_forward(self, a, (packed, lse) if dense else None, tokens, start_pos, pos, advance)
             if logits is not None:
                 return logits, advance
             return a["logits"][:B, :cfg.vocab_size].float(), False
