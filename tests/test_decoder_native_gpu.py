@@ -50,3 +50,19 @@ def test_layers_that_lie_apart():
     got = apart.forward(tok, 0)
     assert torch.equal(got, want) and torch.equal(apart.kcache, plain.kcache) and torch.equal(apart.vcache, plain.vcache)
     assert not around[:, 2:].any()
+
+
+# a head of one weight tile per CTA, and of several
+@pytest.mark.parametrize("vocab", [500, 50001])
+def test_replayed_steps(vocab):
+    m = llama3.Llama(llama3.config_from_descriptor("llama3:l=2,c=256,h=4,kv=2,t=256,v=%d" % vocab), DEV, torch.bfloat16)
+    m.init_random(3)
+    replayed, launched = generate.CachedDecoder(m, 3, 64), generate.CachedDecoder(m, 3, 64)
+    tok = torch.randint(0, vocab, (3, 20), generator=torch.Generator().manual_seed(1), dtype=torch.int32).to(DEV)
+    for d in (replayed, launched):
+        d.forward(tok[:, :15].contiguous(), 0)
+    step = generate.GraphStep(replayed, 3, 15)
+    for i in range(15, 20):
+        got, want = step.step(tok[:, i:i + 1].contiguous()), launched.forward(tok[:, i:i + 1].contiguous(), i)
+        assert torch.equal(got, want) and got.shape == (3, vocab) and int(step.pos) == i + 1
+    assert torch.equal(replayed.kcache[:, :, :20], launched.kcache[:, :, :20]) and torch.equal(replayed.vcache[:, :, :20], launched.vcache[:, :, :20])

@@ -1,4 +1,5 @@
-"""Gradient norm and AdamW over lists of chunks: slices shorter than, as long as and longer than a chunk, views of one element group, many layers."""
+"""Gradient norm and AdamW over lists of chunks: slices shorter than, as long as and longer than a chunk, views of one element group, many layers, more chunks than
+blocks."""
 import pytest
 import torch
 
@@ -21,7 +22,10 @@ def _views(sizes, shift):
 
 @pytest.mark.parametrize("sizes", [
     [(8, 1)], [(1016, 3), (1024, 2), (1032, 2)], [(8, 40), (8192, 3), (8200, 2), (768, 12)], [(3 * 1024 * 1024 + 8, 2), (16, 1)],
-    [(8 * (i + 1), 1 + i % 3) for i in range(16)]])
+    [(8 * (i + 1), 1 + i % 3) for i in range(16)],
+    # 16 blocks of an SM share the norm's chunks of 8192 elements, 512 the update's of 1024: on 148 SMs a block takes a second one beyond 19.4 and 77.6
+    # million elements, here in another view with slices of another length
+    [(1000 * 1024 + 8, 30), (768, 40), (8200, 3), (8 * 1024 * 1024 + 16, 7), (1016, 5)]])
 @pytest.mark.parametrize("master", [True, False])
 def test_chunks(sizes, master):
     g = torch.Generator(device=DEV).manual_seed(len(sizes))
