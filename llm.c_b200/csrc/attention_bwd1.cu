@@ -733,18 +733,21 @@ dq_fold_kernel(bf16* __restrict__ dqkv, const float* __restrict__ ws, int bh0, i
 }  // namespace
 
 // How many heads, the first ones, are dealt to CTAs whole (WHOLE_HEADS); the others are split into units over the CTAs and folded.
-// Whole up to 10 tiles: the CTAs' slots, 32 KB a tile, then stay in L2 (47 MB of its 126), so that dQ costs no memory traffic before its last rounding.  us of the
-// three or four launches, split in brackets, B x T x heads: 64 x 1024 x 12 459 (523), 128 x 384 x 12 177 (278), 64 x 256 x 12 63 (85), 40 x 1152 x 12 390 (437),
-// 32 x 1280 x 12 379 (396), 20 x 1536 x 12 345 (336), 16 x 2048 x 12 484 (459).
-// Heads that do not fill the CTAs once more are split if that is shorter by more than what it costs: the fold, 4 pairs (1 x 384 x 12 23.6 whole, 25.3 split,
-// 1 x 512 x 12 30.3, 25.9), and next to whole heads a kernel of their own as well, 6 pairs (16 x 512 x 12 56.9 whole, 63.8 split).  With one full round of
-// heads only, the split slots still fit into L2: 13 x 1024 x 12 127.5 in two kernels, 126.3 all split, 13 x 768 x 12 87.1, 85.2.
-constexpr int WHOLE_TILES = 10, SPLIT_GAIN = 4, SPLIT_GAIN_BESIDE = 6;
+// Whole up to 10 tiles.  The CTAs' slots, 32 KB a tile, share L2 with the streams that pass by them: with 296 heads dQ costs 105 MB of memory traffic at 8 tiles
+// (39 MB of slots), 423 at 10 (48 MB), 945 at 12 and 2377 at 16 (counted: bytes moved beyond the inputs and gradients), the split heads' slots, written
+// and folded, at least 504, 776, 1106 and 1940.  us of all launches, split in brackets, B x T x heads: 64 x 1024 x 12 459 (523), 128 x 384 x 12 177 (278),
+// 64 x 256 x 12 63 (85), 40 x 1152 x 12 390 (437), 32 x 1280 x 12 379 (396), 20 x 1536 x 12 345 (336), 16 x 2048 x 12 484 (459).
+// Heads that do not fill the CTAs once more are split if that is shorter by more than what it costs: the fold, 4 pairs, or 2 where each CTA has one unit at most and the
+// fold is small (12 x 640 x 8 37 whole, 38 split, 1 x 512 x 12 30.3, 25.9, 2 x 300 x 12 18.0, 16.8, 4 x 384 x 12 18.7, 17.9; 8 x 384 x 12, two units, 19.8, 27.0, and with two
+// tiles, where nothing gets shorter, 4 x 256 x 12 13.0, 15.8), and next to whole heads a kernel of their own as well, 6 pairs (16 x 512 x 12 56.9 whole, 63.8 split,
+// 16 x 300 x 12 31.9, 37.7).  With one full round of heads only, the split slots still fit into L2: 13 x 1024 x 12 127.5 in two kernels, 126.3 all split,
+// 13 x 768 x 12 87.1, 85.2.
+constexpr int WHOLE_TILES = 10, SPLIT_GAIN = 4, SPLIT_GAIN_ONCE = 2, SPLIT_GAIN_BESIDE = 6;
 static int whole_heads(int heads, int nt, int sms) {
     if (nt < 2 || nt > WHOLE_TILES) return 0;
     const int rest = heads % sms, full = heads - rest, G = (nt + 1) / 2;
     const int gain = nt * (nt + 1) / 2 - CEIL_DIV(rest * G, sms) * (nt + 1);
-    if (rest == 0 || gain < (full ? SPLIT_GAIN_BESIDE : SPLIT_GAIN)) return heads;
+    if (rest == 0 || gain < (full ? SPLIT_GAIN_BESIDE : rest * G <= sms ? SPLIT_GAIN_ONCE : SPLIT_GAIN)) return heads;
     return full >= 2 * sms ? full : 0;
 }
 

@@ -70,8 +70,9 @@ def case(op):
         if op == "gemm_swapped":
             return (lambda: K.matmul_forward(out, h, w3, None)), 2.0 * (Ms * Hs + Cs * Hs + Ms * Cs), 2.0 * Ms * Cs * Hs
         return (lambda: K.matmul_swiglu_prompt(h, x, w12)), 2.0 * (Ms * Cs + 2 * Cs * Hs + Ms * Hs), 4.0 * Ms * Cs * Hs
-    if op in ("attn_fwd", "attn_bwd", "attn_fwd_wide", "attn_bwd_wide", "attn_fwd_short", "attn_bwd_short"):
-        B, T, NH, HS = (16, 2048, 8, 128) if op.endswith("wide") else (64, 64, 25, 64) if op.endswith("short") else (16, 1024, 12, 64)
+    if op.startswith("attn_"):
+        # heads: three of them for each of 148 SMs, so that every CTA of the backward takes whole ones; few: both slots of a CTA of the forward on one query tile
+        B, T, NH, HS = {"wide": (16, 2048, 8, 128), "short": (64, 64, 25, 64), "heads": (37, 1024, 12, 64), "few": (1, 2048, 25, 64)}.get(op.rsplit("_")[-1], (16, 1024, 12, 64))
         qkv, dout = _bf(B, T, 3 * NH * HS), _bf(B, T, NH * HS)
         out = torch.empty(B, T, NH * HS, device=DEV, dtype=torch.bfloat16)
         lse = torch.empty(B, NH, T, device=DEV)
@@ -97,8 +98,8 @@ def case(op):
         }
         fn, bytes_ = fns[op]
         return fn, bytes_, 0.0
-    if op == "classifier":
-        N, V, Vp = 8192, 50257, 50304
+    if op in ("classifier", "classifier_long"):
+        N, V, Vp = (8192, 50257, 50304) if op == "classifier" else (4096, 128256, 128256)
         logits = _bf(N, Vp)
         losses = torch.zeros(N, device=DEV)
         tgt = torch.randint(0, V, (N,), device=DEV, dtype=torch.int32)
@@ -168,11 +169,14 @@ def case(op):
         out = torch.empty(Mr, Nw, device=DEV, dtype=torch.bfloat16)
         product = (lambda: K.matmul_forward(out, x, w, None)) if op == "stream_gemm" else (lambda: K.matmul_skinny(out, x, w))
         return product, 2.0 * (Nw * Kd + Mr * Kd + Mr * Nw), 2.0 * Mr * Nw * Kd
-    if op == "cached_attention":
-        # 32 rows decoding at position 4095 with 32 query heads over 8 cached heads of width 128 (537 MB of cache read)
+    if op in ("cached_attention", "cached_attention_step"):
+        # 32 rows decoding at position 4095 with 32 query heads over 8 cached heads of width 128 (537 MB of cache read); step: with the rotary embedding in the launch
         B, Tmax, NH, NKV, HS = 32, 4096, 32, 8, 128
         kc, vc = _bf(B, Tmax, NKV, HS), _bf(B, Tmax, NKV, HS)
         q, out = _bf(B, NH * HS), torch.empty(B, NH * HS, device=DEV, dtype=torch.bfloat16)
+        if op == "cached_attention_step":
+            raw, freqs = _bf(B, (NH + 2 * NKV) * HS), torch.randn(Tmax, HS // 2, 2, device=DEV)
+            return (lambda: K.rope_cached_attention(out, q, kc, vc, raw, freqs, 1, Tmax - 1, NH, NKV)), 2.0 * (kc.numel() + vc.numel()), 0.0
         return (lambda: K.cached_attention(out, q, kc, vc, 1, Tmax - 1, NH, NKV)), 2.0 * (kc.numel() + vc.numel()), 0.0
     raise SystemExit("unknown operator %r" % op)
 
@@ -180,7 +184,8 @@ def case(op):
 OPS = ["gemm_fwd", "gemm_gelu", "gemm_dgrad", "gemm_dgelu", "gemm_wgrad", "attn_fwd", "attn_bwd", "attn_fwd_wide", "attn_bwd_wide", "ln_fwd", "fused_residual", "ln_bwd", "ln_bwd_colsum",
        "classifier", "encoder_fwd", "encoder_bwd", "adamw", "norm", "bias_grad", "gelu", "rms_fwd", "rms_fused_residual", "rms_bwd", "rope_fwd",
        "rope_bwd", "swiglu_fwd", "swiglu_bwd", "gemm_tf32", "gemm_fwd_1cta", "skinny_gemm", "skinny_gemm_wide", "stream_gemm", "cached_attention",
-       "gemm_gelu_narrow", "gemm_wgrad_narrow", "gemm_dgrad_slices", "gemm_swapped", "gemm_swapped_swiglu", "stream_wide", "attn_fwd_short", "attn_bwd_short"]
+       "gemm_gelu_narrow", "gemm_wgrad_narrow", "gemm_dgrad_slices", "gemm_swapped", "gemm_swapped_swiglu", "stream_wide", "attn_fwd_short", "attn_bwd_short",
+       "attn_fwd_few", "attn_bwd_heads", "cached_attention_step", "classifier_long"]
 
 
 def main(argv):

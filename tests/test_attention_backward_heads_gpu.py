@@ -11,7 +11,8 @@ DEV = "cuda"
 
 
 @pytest.mark.parametrize("B,T,NH", [
-    (1, 256, 148), (1, 130, 149), (3, 300, 99),              # two and three tiles: always whole
+    (1, 256, 148), (1, 130, 149), (3, 300, 99),              # two and three tiles: whole
+    (2, 300, 37), (1, 384, 75), (1, 257, 1),                 # three tiles of heads whose units a CTA has one of: split; of one head more: whole
     (2, 400, 96), (1, 512, 70), (1, 600, 190),               # four, five: whole beside whole heads / split / one full round only: split
     (1, 640, 300), (1, 1024, 300), (4, 897, 80),             # two rounds whole, the others split
     (2, 1280, 150), (1, 1281, 300),                          # the most tiles; one more
