@@ -408,11 +408,12 @@ Plan wide_plan(int M, int tiles, int num_kb, int sms) {
 // the 256 rows of a tile allow.  With the small ones a CTA's share of the reduction and its set-up are short; with the large ones fewer CTAs read the same
 // weights and K can be cut into more slices.  So shallow products take the small ones and deep ones the large ones.  Estimated in ns from the k-blocks of
 // a slice and the rows of a tile, coefficients fitted to 536 products (M 129 to 1024, N 384 to 4096, K 768 to 128256, each way of cutting), 5 and 8 %
-// rms off; the way taken is at most 9 % behind the other, by more than 3 % in 16 of them.  CTAs of small tiles take longer where two share an SM; 13 clusters of 8 large tiles fit
+// rms off; the way taken is at most 9 % behind the other, by more than 3 % in 16 of them.  CTAs of small tiles take longer where two share an SM; 15 clusters of 8 large tiles fit
 // the chip at once, 16 do not.  us, small / large tiles: 256 x 768 x 768 5.0 / 9.3, 256 x 768 x 3072 7.9 / 12.5, 1024 x 768 x 3072 11.7 / 13.3,
 // 384 x 768 x 6144 14.9 / 13.1, 256 x 1600 x 14336 27.5 / 21.9, 512 x 2048 x 14336 33 / 31, 384 x 768 x 50304 79 / 43, 512 x 2048 x 128256 304 / 245,
-// but 256 x 2048 x 14336 28 / 40 (16 clusters of 8).
-Plan gradient_plan(int M, int tiles, int num_kb, int sms) {
+// but 256 x 2048 x 14336 28 / 40 (16 clusters of 8).  Forward products of K = 6144 and more take small tiles only where the estimate is 4 % ahead: 269 x 448 x 14208 16.5 /
+// 15.6, 521 x 1152 x 7360 17.7 / 17.2 with estimates 3 and 2 % ahead, 561 x 1024 x 6336 16.1 / 16.3 with 7 %; 15 clusters 641 x 576 x 6784 15.6 / 13.5.
+Plan gradient_plan(int M, int tiles, int num_kb, int sms, bool forward) {
     const int slots = 2 * (sms * 7 / 8);
     const Plan wide = wide_plan(M, tiles, num_kb, sms);
     int t = CEIL_DIV(M, 64);
@@ -426,16 +427,16 @@ Plan gradient_plan(int M, int tiles, int num_kb, int sms) {
     const long long kb_n = CEIL_DIV(num_kb, S), kb_w = CEIL_DIV(num_kb, wide.S);
     const bool shared_sms = tiles * narrow.mtiles * S > sms * 7 / 8;
     const long long cost_n = kb_n * (295 + (shared_sms ? 63 + narrow.nb * 87 / 100 : 0)) + 44 * narrow.nb + 2300;
-    const int rounds = wide.S == 8 && tiles * wide.mtiles * 10 > sms ? 2 : 1;
+    const int rounds = wide.S == 8 && tiles * wide.mtiles * 19 > 2 * sms ? 2 : 1;
     const long long cost_w = rounds * (kb_w * (297 + wide.nb * 31 / 100) + 24 * wide.nb + 4200);
-    return cost_n <= cost_w ? narrow : wide;
+    return cost_n + (forward && num_kb >= 96 ? cost_n / 25 : 0) <= cost_w ? narrow : wide;
 }
 
 // form: 0 a forward product, 1 an input gradient, 2 a forward product cut like one
 Plan make_plan(int M, int N, int K, bool swiglu, int form) {
     int sms = llmc_device_sm_count(); if (sms <= 0) sms = 148;
     const int tiles = CEIL_DIV(N, swiglu ? WR / 2 : WR), num_kb = CEIL_DIV(K, BK);
-    return form && M > 128 ? gradient_plan(M, tiles, num_kb, sms) : wide_plan(M, tiles, num_kb, sms);
+    return form && M > 128 ? gradient_plan(M, tiles, num_kb, sms, form == 2) : wide_plan(M, tiles, num_kb, sms);
 }
 
 template <int MODE, bool W_MN>

@@ -1,4 +1,4 @@
-"""How the split-K kernel cuts an input gradient (csrc/stream_gemm.cu): rows of a tile and slices of K on a chip of 148 SMs."""
+"""How the split-K kernel cuts an input gradient, and a forward product like one (csrc/stream_gemm.cu): rows of a tile and slices of K on a chip of 148 SMs."""
 import ctypes
 
 import pytest
@@ -31,3 +31,11 @@ def test_input_gradients(plan, M, N, K, rows, slices):
 def test_few_rows_and_forward_products_are_cut_as_before(plan):
     assert plan(4, 768, 50304) == (16, 8) and plan(100, 2048, 7168) == (112, 8)
     assert plan(300, 2048, 7168, 0) == (160, 4) and plan(128, 768, 3072, 0) == (128, 8)
+
+
+# 15 clusters of eight large tiles fit the chip, 16 do not; deep forward products take small tiles only where the estimate is clearly for them
+@pytest.mark.parametrize("M,N,K,gradient,forward", [
+    (641, 576, 6784, (224, 8), (224, 8)), (768, 640, 6144, (256, 8), (256, 8)), (500, 1024, 8192, (64, 4), (64, 4)), (554, 704, 6400, (64, 4), (64, 4)),
+    (269, 448, 14208, (64, 8), (144, 8)), (521, 1152, 7360, (80, 4), (176, 4)), (561, 1024, 6336, (80, 4), (80, 4)), (256, 768, 3072, (64, 8), (64, 8))])
+def test_large_and_small_tiles(plan, M, N, K, gradient, forward):
+    assert plan(M, N, K) == gradient and plan(M, N, K, 2) == forward
