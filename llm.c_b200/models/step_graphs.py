@@ -71,11 +71,13 @@ class Side:
     the main branch from here on follow the sums given up to the mark, ``join()``: everything the side branches have been given.
     ``read(buffer)`` notes that the launches given to them so far read it, ``free(buffer)`` joins those: before the main branch writes it again.
 
-    Forward and backward of GPT-2 124M at 4 x 64 tokens 1372 us with one branch that is joined at the end of every layer, 1335 us so."""
+    Forward and backward of GPT-2 124M at 4 x 64 tokens 1372 us with one branch that is joined at the end of every layer, 1335 us with two, 1310 with the priority of
+    ``_capture``, 1280 since a join adds no edge that is there already (with everything recomputed and 2 x 64 tokens 1370, -, 1390, 1355)."""
 
     def __init__(self, stream, sums):
         self.stream, self.sums = stream, sums
-        self._used = []                    # of the two, those that have work of this capture
+        self._forks = {}                   # of the two, those that have work of this capture: how often they were given some
+        self._joined = {}                  # and how much of it the main branch follows
         self._others = {}
         self._readers = {}
 
@@ -88,8 +90,7 @@ class Side:
         return self._others[t.data_ptr()]
 
     def _fork(self, stream):
-        if stream not in self._used:
-            self._used.append(stream)
+        self._forks[stream] = self._forks.get(stream, 0) + 1
         stream.wait_event(torch.cuda.current_stream().record_event())
         return torch.cuda.stream(stream)
 
@@ -99,22 +100,29 @@ class Side:
     def fork_sums(self):
         return self._fork(self.sums)
 
-    def mark_sums(self):
-        return self.sums.record_event()
+    def _mark(self, stream):
+        return stream, self._forks[stream], stream.record_event()
 
-    def join(self, mark=None):
-        for m in [s.record_event() for s in self._used] if mark is None else [mark]:
-            torch.cuda.current_stream().wait_event(m)
+    def mark_sums(self):
+        return self._mark(self.sums)
+
+    def join(self, *marks):
+        # a launch with an edge from another branch does not start under the one before it: none for what the main branch follows already
+        for stream, forks, event in marks or [self._mark(s) for s in self._forks]:
+            if self._joined.get(stream, 0) < forks:
+                self._joined[stream] = forks
+                torch.cuda.current_stream().wait_event(event)
 
     def read(self, *buffers):
-        marks = [s.record_event() for s in self._used]
+        marks = [self._mark(s) for s in self._forks]
         for t in buffers:
             self._readers[t.data_ptr()] = marks
 
     def free(self, *buffers):
         for t in buffers:
-            for m in self._readers.pop(t.data_ptr(), ()):
-                torch.cuda.current_stream().wait_event(m)
+            marks = self._readers.pop(t.data_ptr(), None)
+            if marks:
+                self.join(*marks)
 
 
 class StepGraphs:

@@ -22,6 +22,8 @@ class Stream:
         return dict(self.clock)
 
     def wait_event(self, event):
+        if self is self.world.main and all(self.clock.get(s, 0) >= n for s, n in event.items()):
+            self.world.idle_waits += 1
         for s, n in event.items():
             self.clock[s] = max(self.clock.get(s, 0), n)
 
@@ -32,7 +34,7 @@ class World:
     def __init__(self):
         self.main = Stream(self)
         self.now = self.main
-        self.log, self.scratch = [], {}
+        self.log, self.scratch, self.idle_waits = [], {}, 0
 
     # ---- torch.cuda
     def current_stream(self):
@@ -109,6 +111,8 @@ def _run(monkeypatch, family, recompute, spoil=None):
 def test_launches_on_the_same_memory_follow_one_another(monkeypatch, family, recompute):
     world = _run(monkeypatch, family, recompute)
     assert len({s for _, s, *_ in world.log}) == (3 if family == "gpt2" else 2)
+    # and none of the chain waits for what it follows already: a launch with an edge from another branch does not start under the one before it
+    assert world.idle_waits == 0
 
 
 @pytest.mark.parametrize("family", ["gpt2", "llama3"])
