@@ -23,9 +23,10 @@
 // 16.0 / 14.9 us at 1 x 777 x 32).
 //
 // DUO: where the query tiles are so few that SMs would get one chain only, a CTA works on ONE query tile, its slots on alternate key tiles, and adds the two
-// at the end.  us, with the kernel this one replaces (one CTA of two slots per SM, tiles of 128 keys, slots taking turns at the exponentials) in brackets, B x T x heads:
-// 64 x 1024 x 12 171 (205), 2 x 4096 x 32 192 (225), 64 x 256 x 12 24.0 (32.8), 8 x 1024 x 12 28.7 (34.4); DUO 1 x 777 x 32 14.7 (14.7), 4 x 512 x 12 10.4 (11.1),
-// 3 x 1000 x 16 19.2 (23.2), 1 x 2048 x 25 27.0 (41.2), 1 x 129 x 32 5.6 (7.1).
+// at the end.  us, with the kernel this one replaces (one CTA of two slots per SM, tiles of 128 keys, slots taking turns at the exponentials) in brackets, in turn on one
+// GPU, B x T x heads: 64 x 1024 x 12 175 (205), 2 x 4096 x 32 198 (233), 64 x 256 x 12 27.3 (35.9), 8 x 1024 x 12 28.6 (34.5); DUO 4 x 512 x 12 10.3 (11.0),
+// 3 x 1000 x 16 19.1 (22.9), 1 x 2048 x 25 27.3 (41.7), 1 x 129 x 32 5.5 (7.0).  Where about half of the SMs get a second CTA, which then decides, DUO gains
+// nothing: 1 x 777 x 32 14.7 (14.4), 4 x 512 x 16 11.5 (11.3).
 //
 // TMEM columns of a CTA: S_A [0,64)  O_A [64,128)  S_B [128,192)  O_B [192,256); P_X: the first 32 columns of S_X (64 bf16 per row)
 //
@@ -241,8 +242,8 @@ attn_fwd1_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
             const int jd = 2 * qi + (q4 >> 1);             // the key tile on this warp's diagonal: none of the later ones is seen
             float m = -INFINITY, l = 0.f;                  // reference maximum (raw score units) and row sum relative to it
             // Tiles that move the reference however little their maximum is above it.  The largest probability of a row, which alone is exact in bf16 where it is 1,
-            // is more often 1 with a maximum over 128 keys than over 64: error of O against 64 bits at 12 x 700 x 16 0.00202 and 0.00203.  Two slots on a row
-            // have a reference each, 0.00201 with 64 keys.
+            // is more often 1 with a maximum over 128 keys than over 64: error of O against 64 bits at 12 x 700 x 16 0.002010 and 0.002034 (0.002017 in the kernel
+            // before, which took tiles of 128 keys).  Two slots on a row have a reference each: 1 x 777 x 32 0.002006 with 64 keys (0.002022).
             constexpr int FIRST_TILES = DUO ? 1 : 2;
             #pragma unroll 1
             for (int i = 0; i < nj; i++, t++) {

@@ -480,7 +480,8 @@ template <int N> DEVINL void regs_grow() { asm volatile("setmaxnreg.inc.sync.ali
 
 // The warp's index in its block, by a shuffle that makes it known to be the same in all lanes: what follows from it (a role's barriers, tiles and descriptors) goes
 // to uniform registers, which the tensor and TMA instructions want, instead of being moved there at each use.  That counts where an issuer's instructions lie on the
-// chain of every tile.  Attention, us without / with: 64 x 1024 x 12 heads of 64 forward 212 / 177, backward 391 / 369, 2 x 4096 x 32 of 128 forward 289 / 280.
+// chain of every tile.  Attention, us without / with, in turn: 64 x 1024 x 12 heads of 64 forward 187 / 175, backward (all launches) 555 / 500, 16 x 1024 x 16 of 128 forward
+// 136 / 128, 3 x 1000 x 32 of 80 53 / 50; the backward of wide heads gains 0 to 2 %.
 // The matrix products, whose issuer runs ahead of its accumulators, take the same time with either.
 DEVINL int warp_index() { return __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0); }
 DEVINL bool elect_one() {

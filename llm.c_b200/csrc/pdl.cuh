@@ -11,7 +11,7 @@
 // 986 us with the attribute and 938 without, on one GPU in turn, with the trigger right behind the wait (at the end of a CTA, where gemm2_kernel has
 // its own, it was not tried there); the classifier's figures stand with it.  Where 64-wide heads leave SMs free
 // the attribute pays: forward + backward of 4 x 64 tokens 1566 us without and 1513 with it.  (The bracketed comparisons were made when the plain launch
-// was the only other thing that differed; those passes take 1310, 262 and 605 us now, 3 % more or less from one GPU to another.)
+// was the only other thing that differed; those passes take 1284, 260 and 628 us now, 3 % more or less from one GPU to another.)
 #pragma once
 #include "common.cuh"
 

@@ -118,8 +118,9 @@ def _sliced(M, N, K, device):
     """Whether a forward product of more than 128 rows goes to the split-K kernel with row tiles and slices like an input gradient's.  The line is the input
     gradients' one: below it (fewer tiles, deeper) the slices win over the swapped kernel's one sum over K, above it they lose.  us in a chain, the swapped
     kernel in brackets: 129 x 768 x 768 4.7 (6.0), 256 x 768 x 768 5.1 (6.2), 512 x 768 x 768 6.3 (6.3), 256 x 768 x 3072 7.9 (14.1), 1024 x 768 x 3072 12.1
-    (15.1), 256 x 384 x 1536 5.9 (8.8), 512 x 1024 x 1024 7.0 (7.3), 1024 x 1024 x 4096 14.7 (18.7), 512 x 2048 x 2048 11.2 (11.7), 300 x 2048 x 7168 16 (28; 20 in
-    row tiles of up to 256); beyond it 256 x 2304 x 768 7.6 (6.4), 777 x 1024 x 1024 8.7 (8.0), 2048 x 768 x 3072 21 (15).  The sums are fp32 and added in slice order."""
+    (15.1), 256 x 384 x 1536 5.9 (8.8), 512 x 1024 x 1024 7.0 (7.3), 1024 x 1024 x 4096 14.7 (18.7), 512 x 2048 x 2048 11.2 (11.7); from K = 6144 on,
+    where products of few tiles went to the split-K kernel in large row tiles before, in brackets, 220 x 192 x 13312 12.0 (16.1), 554 x 704 x 6400 14.9 (16.4); beyond the line
+    256 x 2304 x 768 7.6 (6.4), 777 x 1024 x 1024 8.7 (8.0), 2048 x 768 x 3072 21 (15).  The sums are fp32 and added in slice order."""
     return M > STREAM_MAX_ROWS and K % 8 == 0 and _slices_pay(M, (N + 127) // 128, K, device)
 
 
