@@ -53,6 +53,8 @@ constexpr int PAIRS = 3;                            // K / V tile pairs in fligh
 constexpr int RING = 2 * PAIRS;
 constexpr int THREADS = 384;                        // TMA warp, two issuer warps, an idle one, 2 x 4 softmax warps
 constexpr int REGS_LOW = 48, REGS_HIGH = 96;        // of 80 at launch (two CTAs): 4 x 48 + 8 x 96 = 12 x 80
+constexpr int REGS_LAUNCH = (4 * REGS_LOW + 8 * REGS_HIGH) / 12;
+static_assert(12 * REGS_LAUNCH == 4 * REGS_LOW + 8 * REGS_HIGH, "the shares of the warps add up to what a block is launched with");
 constexpr int TMEM_COLS = 256;
 constexpr int SMEM = 4 * TILE_BYTES + RING * KV_BYTES + 256;      // two Q / output tiles of each slot, K/V ring
 static_assert(2 * (SMEM + 1024) <= 228 * 1024, "two CTAs share an SM");
@@ -429,6 +431,10 @@ extern "C" int llmc_attention_fwd(bf16* out, float* lse, const bf16* qkv, int B,
     auto kernel = duo ? attn_fwd1_kernel<true> : attn_fwd1_kernel<false>;
     static bool configured[2] = {false, false};
     if (!configured[duo]) {
+        // a block compiled to fewer registers would wait for its larger shares for good
+        cudaFuncAttributes attr;
+        CUDA_CHECK(cudaFuncGetAttributes(&attr, kernel));
+        if (attr.numRegs < REGS_LAUNCH) { fprintf(stderr, "[llmc_b200] attention: compiled to %d registers, %d expected\n", attr.numRegs, REGS_LAUNCH); return -1; }
         CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM));
         configured[duo] = true;
     }
